@@ -11,313 +11,15 @@
 // fused_bias_swiglu_patches.py:21), swiglu_with_probs (primus_turbo.py:1954-1980), clamped SwiGLU
 // (primus/backends/megatron/core/fusions/fused_bias_swiglu.py:25-100), TE cross-entropy fusion
 // and FusedAdam (primus/backends/megatron/patches/torch_fused_adam_patches.py:40-88).
-#include "common.cuh"
+#include "vec.cuh"
 
 namespace {
 
-struct alignas(16) Bf8 {
-  __nv_bfloat162 v[4];
-};
-
-__device__ __forceinline__ void bf8_to_f(const Bf8& b, float* f) {
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    float2 t = __bfloat1622float2(b.v[i]);
-    f[2 * i] = t.x;
-    f[2 * i + 1] = t.y;
-  }
-}
-__device__ __forceinline__ Bf8 f_to_bf8(const float* f) {
-  Bf8 b;
-#pragma unroll
-  for (int i = 0; i < 4; ++i) b.v[i] = __floats2bfloat162_rn(f[2 * i], f[2 * i + 1]);
-  return b;
-}
-
-template <int THREADS>
-__device__ __forceinline__ float block_sum(float v, float* red) {
-  v = pb::warp_sum(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float r = (l < THREADS / 32) ? red[l] : 0.f;
-  r = pb::warp_sum(r);
-  return r;
-}
-template <int THREADS>
-__device__ __forceinline__ float block_max(float v, float* red) {
-  v = pb::warp_max(v);
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  __syncthreads();
-  if (l == 0) red[w] = v;
-  __syncthreads();
-  float r = (l < THREADS / 32) ? red[l] : -INFINITY;
-  r = pb::warp_max(r);
-  return r;
-}
-
-// ------------------------------------------------------------------ RMSNorm forward
-// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream to xsum.
-constexpr int RN_THREADS = 256;
-// One row per CTA; VPT 16-byte vectors per thread stay in registers between the sum-of-squares pass and the scaling
-// pass, so every operand is read from memory exactly once.
-template <int VPT>
-__global__ void __launch_bounds__(RN_THREADS)
-rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
-                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
-                   __nv_bfloat16* __restrict__ xsum, float* __restrict__ rstd_out, int H, long ldx,
-                   long ldy, float eps) {
-  __shared__ float red[32];
-  const long row = blockIdx.x;
-  const Bf8* xr = reinterpret_cast<const Bf8*>(x + row * ldx);
-  const Bf8* rr = res ? reinterpret_cast<const Bf8*>(res + row * ldx) : nullptr;
-  Bf8* sr = xsum ? reinterpret_cast<Bf8*>(xsum + row * ldx) : nullptr;
-  const int nv = H / 8;
-  float f[VPT][8];
-  float ss = 0.f;
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int i = threadIdx.x + k * RN_THREADS;
-    if (i < nv) {
-      bf8_to_f(xr[i], f[k]);
-      if (rr) {
-        float g[8];
-        bf8_to_f(rr[i], g);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) f[k][j] += g[j];
-        Bf8 s = f_to_bf8(f[k]);
-        sr[i] = s;
-        bf8_to_f(s, f[k]);  // normalise exactly what later layers will read
-      }
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[k][j] * f[k][j];
-    }
-  }
-  ss = block_sum<RN_THREADS>(ss, red);
-  const float rstd = rsqrtf(ss / H + eps);
-  if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
-  const Bf8* wr = reinterpret_cast<const Bf8*>(w);
-  Bf8* yr = reinterpret_cast<Bf8*>(y + row * ldy);
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int i = threadIdx.x + k * RN_THREADS;
-    if (i < nv) {
-      float g[8];
-      bf8_to_f(wr[i], g);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[k][j] = f[k][j] * rstd * g[j];
-      yr[i] = f_to_bf8(f[k]);
-    }
-  }
-}
-
-template <typename... Args>
-void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
-  const int vpt = (H / 8 + RN_THREADS - 1) / RN_THREADS;
-  if (vpt <= 1) rmsnorm_fwd_kernel<1><<<(unsigned)rows, RN_THREADS, 0, s>>>(args...);
-  else if (vpt == 2) rmsnorm_fwd_kernel<2><<<(unsigned)rows, RN_THREADS, 0, s>>>(args...);
-  else if (vpt <= 4) rmsnorm_fwd_kernel<4><<<(unsigned)rows, RN_THREADS, 0, s>>>(args...);
-  else rmsnorm_fwd_kernel<8><<<(unsigned)rows, RN_THREADS, 0, s>>>(args...);
-}
-
-// ------------------------------------------------------------------ RMSNorm backward
-// dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x)  (+ dres when given)
-// dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
-// A CTA walks rows blockIdx.x, blockIdx.x + gridDim.x, ...; VPT 16-byte vectors per thread per row.  The next row's
-// operands are fetched into registers before the current row's block reduction, so the reduction's two barriers
-// overlap the loads instead of serialising with them.
-template <int VPT>
-__global__ void __launch_bounds__(RN_THREADS, (VPT <= 2) ? 2 : 1)
-rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                   float* __restrict__ partial, int rows, int H, long ldx, long lddy) {
-  __shared__ float red[32];
-  const int nv = H / 8;
-  float wreg[VPT][8];
-  float dw[VPT][8];
-  const Bf8* wr = reinterpret_cast<const Bf8*>(w);
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int i = threadIdx.x + k * RN_THREADS;
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
-    if (i < nv) bf8_to_f(wr[i], wreg[k]);
-  }
-  Bf8 nx[VPT], ng[VPT], nr[VPT];
-  float nrs = 0.f;
-  auto fetch = [&](long row) {
-    const Bf8* dyr = reinterpret_cast<const Bf8*>(dy + row * lddy);
-    const Bf8* xr = reinterpret_cast<const Bf8*>(x + row * ldx);
-    const Bf8* drr = dres ? reinterpret_cast<const Bf8*>(dres + row * ldx) : nullptr;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-        nx[k] = xr[i];
-        ng[k] = dyr[i];
-        if (drr) nr[k] = drr[i];
-      }
-    }
-    nrs = rstd[row];
-  };
-  long row = blockIdx.x;
-  if (row < rows) fetch(row);
-  for (; row < rows; row += gridDim.x) {
-    float fx[VPT][8], fg[VPT][8], fr[VPT][8];
-    const float rs = nrs;
-    float dot = 0.f;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-        bf8_to_f(nx[k], fx[k]);
-        bf8_to_f(ng[k], fg[k]);
-        if (dres) bf8_to_f(nr[k], fr[k]);
-      }
-    }
-    if (row + gridDim.x < rows) fetch(row + gridDim.x);
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          dw[k][j] += fg[k][j] * fx[k][j] * rs;
-          fg[k][j] *= wreg[k][j];
-          dot += fg[k][j] * fx[k][j];
-        }
-      }
-    }
-    dot = block_sum<RN_THREADS>(dot, red);
-    const float c = dot * rs * rs * rs / H;
-    Bf8* dxr = reinterpret_cast<Bf8*>(dx + row * ldx);
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fg[k][j] * rs - fx[k][j] * c;
-        if (dres) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += fr[k][j];
-        }
-        dxr[i] = f_to_bf8(o);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int i = threadIdx.x + k * RN_THREADS;
-    if (i < nv) {
-      float* p = partial + (long)blockIdx.x * H + (long)i * 8;
-      *reinterpret_cast<float4*>(p) = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
-      *reinterpret_cast<float4*>(p + 4) = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
-    }
-  }
-}
-
-// Rows wider than 8192 elements (up to 16384): 8 vectors per thread; the weight is re-read per row (L1-resident) and
-// nothing is prefetched, which keeps the kernel inside the register file.
-__global__ void __launch_bounds__(RN_THREADS, 1)
-rmsnorm_bwd_wide_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
-                        const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
-                        const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                        float* __restrict__ partial, int rows, int H, long ldx, long lddy) {
-  constexpr int VPT = 8;
-  __shared__ float red[32];
-  const int nv = H / 8;
-  float dw[VPT][8];
-  const Bf8* wr = reinterpret_cast<const Bf8*>(w);
-#pragma unroll
-  for (int k = 0; k < VPT; ++k)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
-  for (long row = blockIdx.x; row < rows; row += gridDim.x) {
-    const Bf8* dyr = reinterpret_cast<const Bf8*>(dy + row * lddy);
-    const Bf8* xr = reinterpret_cast<const Bf8*>(x + row * ldx);
-    const float rs = rstd[row];
-    float fx[VPT][8], fg[VPT][8];
-    float dot = 0.f;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-        float wv[8];
-        bf8_to_f(xr[i], fx[k]);
-        bf8_to_f(dyr[i], fg[k]);
-        bf8_to_f(wr[i], wv);
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          dw[k][j] += fg[k][j] * fx[k][j] * rs;
-          fg[k][j] *= wv[j];
-          dot += fg[k][j] * fx[k][j];
-        }
-      }
-    }
-    dot = block_sum<RN_THREADS>(dot, red);
-    const float c = dot * rs * rs * rs / H;
-    Bf8* dxr = reinterpret_cast<Bf8*>(dx + row * ldx);
-    const Bf8* drr = dres ? reinterpret_cast<const Bf8*>(dres + row * ldx) : nullptr;
-#pragma unroll
-    for (int k = 0; k < VPT; ++k) {
-      const int i = threadIdx.x + k * RN_THREADS;
-      if (i < nv) {
-        float o[8];
-#pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fg[k][j] * rs - fx[k][j] * c;
-        if (drr) {
-          float r[8];
-          bf8_to_f(drr[i], r);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += r[j];
-        }
-        dxr[i] = f_to_bf8(o);
-      }
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < VPT; ++k) {
-    const int i = threadIdx.x + k * RN_THREADS;
-    if (i < nv) {
-      float* p = partial + (long)blockIdx.x * H + (long)i * 8;
-      *reinterpret_cast<float4*>(p) = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
-      *reinterpret_cast<float4*>(p + 4) = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
-    }
-  }
-}
-
-template <typename... Args>
-void launch_rmsnorm_bwd(int P, int H, cudaStream_t s, Args... args) {
-  const int vpt = (H / 8 + RN_THREADS - 1) / RN_THREADS;
-  if (vpt <= 1) rmsnorm_bwd_kernel<1><<<P, RN_THREADS, 0, s>>>(args...);
-  else if (vpt == 2) rmsnorm_bwd_kernel<2><<<P, RN_THREADS, 0, s>>>(args...);
-  else if (vpt <= 4) rmsnorm_bwd_kernel<4><<<P, RN_THREADS, 0, s>>>(args...);
-  else rmsnorm_bwd_wide_kernel<<<P, RN_THREADS, 0, s>>>(args...);
-}
-
-// dw[h] (+)= sum_p partial[p, h].  A CTA owns 32 columns; its 16 thread rows each add every 16th partial (coalesced
-// 128-byte reads) and a fixed-order tree in shared memory folds them, so the result does not depend on scheduling.
-constexpr int DWR_COLS = 32, DWR_ROWS = 16;
-__global__ void __launch_bounds__(DWR_COLS * DWR_ROWS)
-rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, int accumulate) {
-  __shared__ float red[DWR_ROWS][DWR_COLS + 1];
-  const int c = threadIdx.x % DWR_COLS, g = threadIdx.x / DWR_COLS;
-  const int h = blockIdx.x * DWR_COLS + c;
-  float s = 0.f;
-  if (h < H)
-    for (int p = g; p < P; p += DWR_ROWS) s += partial[(long)p * H + h];
-  red[g][c] = s;
-  __syncthreads();
-#pragma unroll
-  for (int step = DWR_ROWS / 2; step > 0; step >>= 1) {
-    if (g < step) red[g][c] += red[g + step][c];
-    __syncthreads();
-  }
-  if (g == 0 && h < H) dw[h] = accumulate ? dw[h] + red[0][c] : red[0][c];
-}
+using pb::Bf8;
+using pb::bf8_to_f;
+using pb::block_max;
+using pb::block_sum;
+using pb::f_to_bf8;
 
 // ------------------------------------------------------------------ logit soft-capping
 // forward: y = cap * tanh(x / cap) (in place when y == x); backward: dx = dy * (1 - (y / cap)^2) from the saved output.
@@ -745,31 +447,6 @@ inline int grid_for(long work_items, int threads, int cap = 148 * 16) {
 
 extern "C" {
 
-int pb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* xsum, float* rstd,
-                   long rows, int H, long ldx, long ldy, float eps, cudaStream_t s) {
-  if (H % 8 || ldx % 8 || ldy % 8 || H > 8 * 8 * RN_THREADS) return -2;
-  if (rows == 0) return 0;
-  launch_rmsnorm_fwd(rows, H, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
-                     (__nv_bfloat16*)y, (__nv_bfloat16*)xsum, rstd, H, ldx, ldy, eps);
-  PB_CHECK_LAUNCH();
-}
-
-// Number of CTAs (= rows of the [P, H] fp32 scratch) the backward uses for a given row count.
-int pb_rmsnorm_bwd_num_partials(long rows) { return (int)(rows < 592 ? (rows < 1 ? 1 : rows) : 592); }
-
-// scratch: fp32 [pb_rmsnorm_bwd_num_partials(rows), H]. dw_accumulate: 1 -> dw += result.
-int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
-                   void* dx, float* dw, float* scratch, long rows, int H, long ldx, long lddy,
-                   int dw_accumulate, cudaStream_t s) {
-  if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L) return -2;   // 32-bit row indices
-  if (rows == 0) return 0;
-  const int P = pb_rmsnorm_bwd_num_partials(rows);
-  launch_rmsnorm_bwd(P, H, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
-                     (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, (int)rows, H, ldx, lddy);
-  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, dw_accumulate);
-  PB_CHECK_LAUNCH();
-}
-
 int pb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, long T, int heads, int d,
             int rot_dim, long ld, int backward, cudaStream_t s) {
   if (rot_dim % 16 || ld % 8 || d % 8) return -2;
@@ -910,49 +587,6 @@ int pb_embedding_bwd(const void* dy, const long* tokens, float* dw, long T, int 
 }
 
 }  // extern "C"
-
-// ------------------------------------------------------------------------------------------------
-// Allocation-free variant of pb_rmsnorm_bwd (declared in primus_b200_noalloc.h).
-//
-// For callers that cannot allocate at the call site (a host application that owns every cudaMalloc,
-// a pre-planned memory arena, a latency-critical loop): the partial weight gradients go to a fixed
-// array in this library's device image rather than to caller-provided scratch.  Host code must not
-// pass the array's name to a kernel (on the host that name is only a stand-in for the symbol); its
-// device address is looked up once per device with cudaGetSymbolAddress, with that device current.
-#include "primus_b200_noalloc.h"
-
-namespace {
-static __device__ __align__(256) float g_noalloc_rmsnorm_partials[(long)PB_NOALLOC_MAX_PARTIALS * PB_NOALLOC_MAX_H];
-constexpr int kMaxDevices = 64;
-float* g_noalloc_scratch_ptr[kMaxDevices] = {nullptr};
-}  // namespace
-
-extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, const float* rstd,
-                                      const void* dres, void* dx, float* dw, long rows, int H, long ldx,
-                                      long lddy, int dw_accumulate, cudaStream_t s) {
-  // the kernels index rows with 32-bit integers: more than INT_MAX rows are rejected rather than truncated
-  if (H <= 0 || H % 8 || ldx % 8 || lddy % 8 || rows < 0 || rows > 2147483647L) return PB_NOALLOC_ERR_BAD_ARG;
-  if (H > PB_NOALLOC_MAX_H) return PB_NOALLOC_ERR_TOO_LARGE;  // the built-in scratch holds rows of <= 8192 floats
-  if (rows == 0) return 0;
-  int dev = -1;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e != cudaSuccess) return (int)e;
-  if (dev < 0 || dev >= kMaxDevices) return PB_NOALLOC_ERR_BAD_ARG;
-  if (!g_noalloc_scratch_ptr[dev]) {
-    // once per device: device address of the scratch array of the image loaded on *this* device
-    float* p = nullptr;
-    e = cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_noalloc_rmsnorm_partials);
-    if (e != cudaSuccess) return (int)e;
-    g_noalloc_scratch_ptr[dev] = p;
-  }
-  float* scratch = g_noalloc_scratch_ptr[dev];
-  const int P = (int)(rows < PB_NOALLOC_MAX_PARTIALS ? rows : PB_NOALLOC_MAX_PARTIALS);
-  // every one of the P partial rows is fully written by its CTA before the reduction reads it
-  launch_rmsnorm_bwd(P, H, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
-                     (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, (int)rows, H, ldx, lddy);
-  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, dw_accumulate);
-  return (int)cudaGetLastError();
-}
 
 // ------------------------------------------------------------------------------------------------
 // MoE token movement.

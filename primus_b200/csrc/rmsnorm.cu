@@ -1,0 +1,480 @@
+// RMSNorm for sm_100a: forward (optional fused residual add) and backward (optional residual gradient).
+//
+// Rows range from 64 channels (per-head norms: hundreds of thousands of rows) to 16384.  A group of LPR lanes owns a row
+// and every lane VPL 16-byte vectors of it, so that short rows share a warp and long ones spread over a CTA, and no lane
+// idles at the widths models use (powers of two; other multiples of 8 leave the last vectors of some lanes empty).
+//
+// Reference call sites these replace: rmsnorm / fused residual norm
+// (primus/backends/megatron/core/extensions/primus_turbo.py:1697-1700, fused_residual_rmsnorm.py).
+#include "vec.cuh"
+
+namespace {
+
+using pb::Bf8;
+using pb::bf8_to_f;
+using pb::f_to_bf8;
+
+// Sum over the LPR lanes of a row group; every lane of the group gets it.  LPR > 32: one slot per warp in `red`, which
+// the caller does not reuse before another barrier.
+template <int LPR>
+__device__ __forceinline__ float group_sum(float v, float* red) {
+  if (LPR <= 32) {
+#pragma unroll
+    for (int o = LPR / 2; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    return v;
+  }
+  v = pb::warp_sum(v);
+  const int warp = threadIdx.x >> 5;
+  if ((threadIdx.x & 31) == 0) red[warp] = v;
+  __syncthreads();
+  const float* r = red + warp / (LPR / 32) * (LPR / 32);
+  float s = 0.f;
+#pragma unroll
+  for (int i = 0; i < LPR / 32; ++i) s += r[i];
+  return s;
+}
+
+// ------------------------------------------------------------------ forward
+// y = (x [+ res]) * rstd * w ; optionally writes the summed residual stream to xsum.  RPG rows per group: their loads
+// are issued together, so a lane has RPG * VPL (about four) 16-byte loads per operand in flight whatever the row length.
+// Values stay packed in registers between the two passes: every operand is read from memory once.
+template <int LPR, int VPL, int RPG, int THREADS>
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                   const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                   __nv_bfloat16* __restrict__ xsum, float* __restrict__ rstd_out, long rows, int H, long ldx,
+                   long ldy, float eps) {
+  __shared__ float red[THREADS / 32];
+  const int lane = threadIdx.x % LPR;
+  const long row0 = (blockIdx.x * (long)(THREADS / LPR) + threadIdx.x / LPR) * RPG;
+  const int nv = H / 8;
+  Bf8 v[RPG][VPL], wv[VPL];
+  float ss[RPG];
+#pragma unroll
+  for (int r = 0; r < RPG; ++r)
+#pragma unroll
+    for (int k = 0; k < VPL; ++k)
+      if (row0 + r < rows && lane + k * LPR < nv)
+        v[r][k] = reinterpret_cast<const Bf8*>(x + (row0 + r) * ldx)[lane + k * LPR];
+  if (res != nullptr) {
+    Bf8 q[RPG][VPL];
+#pragma unroll
+    for (int r = 0; r < RPG; ++r)
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (row0 + r < rows && lane + k * LPR < nv)
+          q[r][k] = reinterpret_cast<const Bf8*>(res + (row0 + r) * ldx)[lane + k * LPR];
+#pragma unroll
+    for (int r = 0; r < RPG; ++r)
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (row0 + r < rows && lane + k * LPR < nv) {
+          float f[8], g[8];
+          bf8_to_f(v[r][k], f);
+          bf8_to_f(q[r][k], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] += g[j];
+          v[r][k] = f_to_bf8(f);  // normalise exactly what later layers will read
+          reinterpret_cast<Bf8*>(xsum + (row0 + r) * ldx)[lane + k * LPR] = v[r][k];
+        }
+  }
+#pragma unroll
+  for (int k = 0; k < VPL; ++k)
+    if (lane + k * LPR < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[lane + k * LPR];
+#pragma unroll
+  for (int r = 0; r < RPG; ++r) {
+    ss[r] = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k)
+      if (row0 + r < rows && lane + k * LPR < nv) {
+        float f[8];
+        bf8_to_f(v[r][k], f);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss[r] += f[j] * f[j];
+      }
+  }
+#pragma unroll
+  for (int r = 0; r < RPG; ++r) {
+    const float rstd = rsqrtf(group_sum<LPR>(ss[r], red) / H + eps);
+    if (row0 + r >= rows) continue;   // (RPG is 1 where group_sum holds a barrier)
+    if (lane == 0 && rstd_out) rstd_out[row0 + r] = rstd;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k)
+      if (lane + k * LPR < nv) {
+        float f[8], g[8];
+        bf8_to_f(v[r][k], f);
+        bf8_to_f(wv[k], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+        reinterpret_cast<Bf8*>(y + (row0 + r) * ldy)[lane + k * LPR] = f_to_bf8(f);
+      }
+  }
+}
+
+template <typename... Args>
+void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
+  const int nv = H / 8;
+#define PB_NORM_FWD(LPR, VPL, RPG, THREADS)                                                             \
+  rmsnorm_fwd_kernel<LPR, VPL, RPG, THREADS>                                                            \
+      <<<(unsigned)((rows + (THREADS / LPR) * RPG - 1) / ((THREADS / LPR) * RPG)), THREADS, 0, s>>>(args...)
+  if (nv <= 8) PB_NORM_FWD(8, 1, 4, 128);
+  else if (nv <= 16) PB_NORM_FWD(16, 1, 4, 128);
+  else if (nv <= 32) PB_NORM_FWD(32, 1, 4, 128);
+  else if (nv <= 64) PB_NORM_FWD(32, 2, 2, 128);
+  else if (nv <= 128) PB_NORM_FWD(32, 4, 1, 128);
+  else if (nv <= 256) PB_NORM_FWD(64, 4, 1, 128);
+  else if (nv <= 512) PB_NORM_FWD(128, 4, 1, 128);
+  else if (nv <= 1024) PB_NORM_FWD(256, 4, 1, 256);
+  else PB_NORM_FWD(512, 4, 1, 512);
+#undef PB_NORM_FWD
+}
+
+// ------------------------------------------------------------------ backward
+// dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x)  (+ dres when given)
+// dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
+
+// Rows of up to 1024 channels: LPR <= 32 lanes per row, no barrier in the loop, RPG rows per group in flight.  The dw
+// sums of a CTA's groups meet in shared memory at the end.
+template <int LPR, int VPL, int RPG>
+__global__ void __launch_bounds__(256, 2)
+rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                         const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
+                         const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                         float* __restrict__ partial, long rows, int H, long ldx, long lddy) {
+  constexpr int GROUPS = 256 / LPR;
+  __shared__ float4 sums[GROUPS][LPR * VPL * 2];
+  const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
+  const int nv = H / 8;
+  Bf8 wv[VPL];
+  float dw[VPL][8];
+#pragma unroll
+  for (int k = 0; k < VPL; ++k) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
+    if (lane + k * LPR < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[lane + k * LPR];
+  }
+  const long stride = (long)gridDim.x * GROUPS * RPG;
+  // the loop bound is the CTA's first row: all lanes of a warp run the same number of iterations (shuffles inside)
+  for (long base = (long)blockIdx.x * GROUPS * RPG; base < rows; base += stride) {
+    const long row0 = base + grp * RPG;
+    Bf8 vx[RPG][VPL], vg[RPG][VPL], vr[RPG][VPL];
+    float rs[RPG];
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) {
+      rs[r] = 0.f;
+      if (row0 + r < rows) rs[r] = rstd[row0 + r];
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (row0 + r < rows && lane + k * LPR < nv) {
+          vx[r][k] = reinterpret_cast<const Bf8*>(x + (row0 + r) * ldx)[lane + k * LPR];
+          vg[r][k] = reinterpret_cast<const Bf8*>(dy + (row0 + r) * lddy)[lane + k * LPR];
+          if (dres) vr[r][k] = reinterpret_cast<const Bf8*>(dres + (row0 + r) * ldx)[lane + k * LPR];
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) {
+      float dot = 0.f;
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (row0 + r < rows && lane + k * LPR < nv) {
+          float fx[8], fg[8], fw[8];
+          bf8_to_f(vx[r][k], fx);
+          bf8_to_f(vg[r][k], fg);
+          bf8_to_f(wv[k], fw);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            dw[k][j] += fg[j] * fx[j] * rs[r];
+            dot += fg[j] * fw[j] * fx[j];
+          }
+        }
+      dot = group_sum<LPR>(dot, nullptr);
+      const float c = dot * rs[r] * rs[r] * rs[r] / H;
+#pragma unroll
+      for (int k = 0; k < VPL; ++k)
+        if (row0 + r < rows && lane + k * LPR < nv) {
+          float fx[8], fg[8], fw[8], o[8];
+          bf8_to_f(vx[r][k], fx);
+          bf8_to_f(vg[r][k], fg);
+          bf8_to_f(wv[k], fw);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] = fg[j] * fw[j] * rs[r] - fx[j] * c;
+          if (dres) {
+            bf8_to_f(vr[r][k], fx);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) o[j] += fx[j];
+          }
+          reinterpret_cast<Bf8*>(dx + (row0 + r) * ldx)[lane + k * LPR] = f_to_bf8(o);
+        }
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < VPL; ++k) {
+    sums[grp][(lane + k * LPR) * 2] = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
+    sums[grp][(lane + k * LPR) * 2 + 1] = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nv * 2; i += 256) {
+    float4 t = sums[0][i];
+#pragma unroll
+    for (int g = 1; g < GROUPS; ++g) {
+      const float4 u = sums[g][i];
+      t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+    }
+    reinterpret_cast<float4*>(partial + (long)blockIdx.x * H)[i] = t;
+  }
+}
+
+// Longer rows: one CTA per row, persistent over rows blockIdx.x, blockIdx.x + gridDim.x, ...  Every thread keeps a ring
+// of STAGES rows of its own vectors in shared memory, filled by its own 16-byte cp.async copies, so loads run several
+// rows ahead of the block reductions without holding registers; the reduction is the only barrier of a row (its slots
+// alternate).
+template <int VPT, int THREADS, bool RES>
+__global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
+rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                   const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
+                   const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
+                   float* __restrict__ partial, long rows, int H, long ldx, long lddy, int stages) {
+  extern __shared__ __align__(16) uint8_t ring_raw[];
+  __shared__ float red[2][THREADS / 32];
+  constexpr int OPS = RES ? 3 : 2;
+  Bf8* ring = reinterpret_cast<Bf8*>(ring_raw);   // [stage][operand][k][thread]
+  const int tid = threadIdx.x;
+  const int nv = H / 8;
+  Bf8 wv[VPT];
+  float dw[VPT][8];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
+    if (tid + k * THREADS < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[tid + k * THREADS];
+  }
+  auto fetch = [&](long row, int st) {
+    if (row < rows) {
+      Bf8* slot = ring + (long)st * OPS * VPT * THREADS + tid;
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int i = tid + k * THREADS;
+        if (i < nv) {
+          pb::cp_async_16(slot + k * THREADS, reinterpret_cast<const Bf8*>(x + row * ldx) + i);
+          pb::cp_async_16(slot + (VPT + k) * THREADS, reinterpret_cast<const Bf8*>(dy + row * lddy) + i);
+          if (RES) pb::cp_async_16(slot + (2 * VPT + k) * THREADS, reinterpret_cast<const Bf8*>(dres + row * ldx) + i);
+        }
+      }
+    }
+    pb::cp_async_commit();   // also when empty: the wait below counts groups
+  };
+  // two ring sizes: the wait needs a constant
+  auto wait_oldest = [&]() {
+    if (stages == 4) pb::cp_async_wait<3>();
+    else pb::cp_async_wait<1>();
+  };
+  long row = blockIdx.x;
+  for (int st = 0; st < stages; ++st) fetch(row + (long)st * gridDim.x, st);
+  float rs = row < rows ? rstd[row] : 0.f;
+  int st = 0, flip = 0;
+  for (; row < rows; row += gridDim.x) {
+    const long next = row + gridDim.x;
+    const float rs_next = next < rows ? rstd[next] : 0.f;
+    wait_oldest();
+    const Bf8* slot = ring + (long)st * OPS * VPT * THREADS + tid;
+    Bf8 vx[VPT], vg[VPT], vr[VPT];
+    float dot = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (tid + k * THREADS < nv) {
+        vx[k] = slot[k * THREADS];
+        vg[k] = slot[(VPT + k) * THREADS];
+        if (RES) vr[k] = slot[(2 * VPT + k) * THREADS];
+        float fx[8], fg[8], fw[8];
+        bf8_to_f(vx[k], fx);
+        bf8_to_f(vg[k], fg);
+        bf8_to_f(wv[k], fw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dw[k][j] += fg[j] * fx[j] * rs;
+          dot += fg[j] * fw[j] * fx[j];
+        }
+      }
+    dot = pb::warp_sum(dot);
+    if ((tid & 31) == 0) red[flip][tid >> 5] = dot;
+    __syncthreads();
+    // the slot's values are in registers (the sum above used them; vr is pinned by the barrier's memory clobber)
+    fetch(row + (long)stages * gridDim.x, st);
+    dot = 0.f;
+#pragma unroll
+    for (int i = 0; i < THREADS / 32; ++i) dot += red[flip][i];
+    const float c = dot * rs * rs * rs / H;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (tid + k * THREADS < nv) {
+        float fx[8], fg[8], fw[8], o[8];
+        bf8_to_f(vx[k], fx);
+        bf8_to_f(vg[k], fg);
+        bf8_to_f(wv[k], fw);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) o[j] = fg[j] * fw[j] * rs - fx[j] * c;
+        if (RES) {
+          bf8_to_f(vr[k], fx);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) o[j] += fx[j];
+        }
+        reinterpret_cast<Bf8*>(dx + row * ldx)[tid + k * THREADS] = f_to_bf8(o);
+      }
+    rs = rs_next;
+    flip ^= 1;
+    if (++st == stages) st = 0;
+  }
+#pragma unroll
+  for (int k = 0; k < VPT; ++k)
+    if (tid + k * THREADS < nv) {
+      float4* p = reinterpret_cast<float4*>(partial + (long)blockIdx.x * H + (long)(tid + k * THREADS) * 8);
+      p[0] = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
+      p[1] = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
+    }
+}
+
+// CTAs (= partial rows) of the backward: two per SM, fewer when there are fewer rows
+constexpr int BWD_MAX_PARTIALS = 296;
+
+template <int VPT, int THREADS, bool RES>
+int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
+                            const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, long rows,
+                            int H, long ldx, long lddy) {
+  constexpr int STAGE = (RES ? 3 : 2) * VPT * THREADS * 16;
+  // four rows ahead where two CTAs of an SM then still fit into its shared memory, else two
+  constexpr int STAGES = 4 * STAGE <= 100 * 1024 ? 4 : 2;
+  auto kern = rmsnorm_bwd_kernel<VPT, THREADS, RES>;
+  static bool attr_set = false;
+  if (!attr_set) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE);
+    if (e != cudaSuccess) return (int)e;
+    attr_set = true;
+  }
+  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy, STAGES);
+  return 0;
+}
+
+int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
+                       const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, long rows, int H,
+                       long ldx, long lddy) {
+  const int nv = H / 8;
+#define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                         \
+  {                                                                                                              \
+    rmsnorm_bwd_short_kernel<LPR, VPL, RPG><<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy); \
+    return 0;                                                                                                    \
+  }
+#define PB_NORM_BWD(VPT, THREADS)                                                                                     \
+  return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy) \
+              : launch_rmsnorm_bwd_ring<VPT, THREADS, false>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy)
+  if (nv <= 8) PB_NORM_BWD_SHORT(8, 1, 4)
+  if (nv <= 16) PB_NORM_BWD_SHORT(16, 1, 4)
+  if (nv <= 32) PB_NORM_BWD_SHORT(32, 1, 4)
+  if (nv <= 64) PB_NORM_BWD_SHORT(32, 2, 2)
+  if (nv <= 128) PB_NORM_BWD_SHORT(32, 4, 1)
+  if (nv <= 256) PB_NORM_BWD(1, 256);
+  if (nv <= 512) PB_NORM_BWD(2, 256);
+  if (nv <= 1024) PB_NORM_BWD(4, 256);
+  PB_NORM_BWD(4, 512);
+#undef PB_NORM_BWD
+#undef PB_NORM_BWD_SHORT
+}
+
+// dw[h] (+)= sum_p partial[p, h].  A CTA owns 32 columns; its 16 thread rows each add every 16th partial (coalesced
+// 128-byte reads, eight in flight) and a fixed-order tree in shared memory folds them, so the result does not depend on
+// scheduling.
+constexpr int DWR_COLS = 32, DWR_ROWS = 16;
+__global__ void __launch_bounds__(DWR_COLS * DWR_ROWS)
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, int accumulate) {
+  __shared__ float red[DWR_ROWS][DWR_COLS + 1];
+  const int c = threadIdx.x % DWR_COLS, g = threadIdx.x / DWR_COLS;
+  const int h = blockIdx.x * DWR_COLS + c;
+  float s = 0.f;
+  if (h < H) {
+#pragma unroll 8
+    for (int p = g; p < P; p += DWR_ROWS) s += partial[(long)p * H + h];
+  }
+  red[g][c] = s;
+  __syncthreads();
+#pragma unroll
+  for (int step = DWR_ROWS / 2; step > 0; step >>= 1) {
+    if (g < step) red[g][c] += red[g + step][c];
+    __syncthreads();
+  }
+  if (g == 0 && h < H) dw[h] = accumulate ? dw[h] + red[0][c] : red[0][c];
+}
+
+int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
+  // every one of the P partial rows is fully written by its CTA before the reduction reads it
+  const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+                                    (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, H, ldx, lddy);
+  if (rc) return rc;
+  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, dw_accumulate);
+  return (int)cudaGetLastError();
+}
+
+}  // namespace
+
+extern "C" {
+
+int pb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* xsum, float* rstd,
+                   long rows, int H, long ldx, long ldy, float eps, cudaStream_t s) {
+  if (H % 8 || ldx % 8 || ldy % 8 || H > 16384) return -2;
+  if (rows == 0) return 0;
+  launch_rmsnorm_fwd(rows, H, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
+                     (__nv_bfloat16*)y, (__nv_bfloat16*)xsum, rstd, rows, H, ldx, ldy, eps);
+  return (int)cudaGetLastError();
+}
+
+// Number of CTAs (= rows of the [P, H] fp32 scratch) the backward uses for a given row count.
+int pb_rmsnorm_bwd_num_partials(long rows) { return (int)(rows < BWD_MAX_PARTIALS ? (rows < 1 ? 1 : rows) : BWD_MAX_PARTIALS); }
+
+// scratch: fp32 [pb_rmsnorm_bwd_num_partials(rows), H]. dw_accumulate: 1 -> dw += result.
+int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
+                   void* dx, float* dw, float* scratch, long rows, int H, long ldx, long lddy,
+                   int dw_accumulate, cudaStream_t s) {
+  if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L) return -2;
+  if (rows == 0) return 0;
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dw, scratch, rows, H, ldx, lddy,
+                     dw_accumulate, s);
+}
+
+}  // extern "C"
+
+// ------------------------------------------------------------------------------------------------
+// Allocation-free variant of pb_rmsnorm_bwd (declared in primus_b200_noalloc.h).
+//
+// For callers that cannot allocate at the call site (a host application that owns every cudaMalloc,
+// a pre-planned memory arena, a latency-critical loop): the partial weight gradients go to a fixed
+// array in this library's device image rather than to caller-provided scratch.  Host code must not
+// pass the array's name to a kernel (on the host that name is only a stand-in for the symbol); its
+// device address is looked up once per device with cudaGetSymbolAddress, with that device current.
+#include "primus_b200_noalloc.h"
+
+namespace {
+static __device__ __align__(256) float g_noalloc_rmsnorm_partials[(long)PB_NOALLOC_MAX_PARTIALS * PB_NOALLOC_MAX_H];
+constexpr int kMaxDevices = 64;
+float* g_noalloc_scratch_ptr[kMaxDevices] = {nullptr};
+}  // namespace
+
+extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, const float* rstd,
+                                      const void* dres, void* dx, float* dw, long rows, int H, long ldx,
+                                      long lddy, int dw_accumulate, cudaStream_t s) {
+  // the kernels index rows with 32-bit integers: more than INT_MAX rows are rejected rather than truncated
+  if (H <= 0 || H % 8 || ldx % 8 || lddy % 8 || rows < 0 || rows > 2147483647L) return PB_NOALLOC_ERR_BAD_ARG;
+  if (H > PB_NOALLOC_MAX_H) return PB_NOALLOC_ERR_TOO_LARGE;  // the built-in scratch holds rows of <= 8192 floats
+  if (rows == 0) return 0;
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  if (dev < 0 || dev >= kMaxDevices) return PB_NOALLOC_ERR_BAD_ARG;
+  if (!g_noalloc_scratch_ptr[dev]) {
+    // once per device: device address of the scratch array of the image loaded on *this* device
+    float* p = nullptr;
+    e = cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_noalloc_rmsnorm_partials);
+    if (e != cudaSuccess) return (int)e;
+    g_noalloc_scratch_ptr[dev] = p;
+  }
+  const int P = (int)(rows < PB_NOALLOC_MAX_PARTIALS ? rows : PB_NOALLOC_MAX_PARTIALS);
+  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate, s);
+}

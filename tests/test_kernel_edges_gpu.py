@@ -1,0 +1,53 @@
+"""Kernels at the edges of their tiles and dispatch rules: row widths around every lane-group size of the norms, GEMM
+shapes around the 256 x 256 CTA-pair tile, permutation maps around the scan step, ragged vocabularies and masked logits.
+
+Tolerances: a bf16 result rounds once (2^-8 relative at most, 2^-9 on average), so elementwise results are compared
+within 2^-7 of their own size plus 2^-9 of the tensor's maximum; fp32 sums of n products of O(1) values within
+n * 2^-24 * sqrt(n) of their size, generously 1e-4."""
+import pytest
+import torch
+
+from primus_b200.ops import _lib, attention, fused, gemm, optim
+from primus_b200.ops import moe as M
+
+pytestmark = pytest.mark.gpu
+
+
+def _gen(seed=0):
+    return torch.Generator(device="cuda").manual_seed(seed)
+
+
+def _close_bf16(got, ref, what):
+    ref = ref.double()
+    err = (got.double() - ref).abs()
+    lim = ref.abs() * 2.0 ** -7 + ref.abs().max() * 2.0 ** -9
+    assert (err <= lim).all(), f"{what}: error {err.max().item()} at value {ref.flatten()[err.argmax()].item()}"
+
+
+def _rms64(x, w, eps=1e-5):
+    return x * torch.rsqrt(x.pow(2).mean(-1, keepdim=True) + eps) * w
+
+
+@pytest.mark.parametrize("H", [8, 64, 72, 128, 136, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("rows,with_res", [(1, True), (13, False), (700, True)])
+def test_rmsnorm_widths(H, rows, with_res):
+    g = _gen(H + rows)
+    x, r, dy, ds = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    xl, wl = x.clone().requires_grad_(), w.clone().requires_grad_()
+    s64 = ((x + r) if with_res else x).double().requires_grad_()
+    w64 = w.double().requires_grad_()
+    y64 = _rms64(s64, w64)
+    if with_res:
+        rl = r.clone().requires_grad_()
+        y, s = fused.rmsnorm(xl, wl, 1e-5, rl)
+        torch.autograd.backward([y, s], [dy, ds])
+        torch.autograd.backward([y64, s64 * 1.0], [dy.double(), ds.double()])
+        assert torch.equal(s.detach(), x + r) and torch.equal(rl.grad, xl.grad)
+    else:
+        y = fused.rmsnorm(xl, wl)
+        y.backward(dy)
+        y64.backward(dy.double())
+    _close_bf16(y.detach(), y64.detach(), "y")
+    _close_bf16(xl.grad, s64.grad, "dx")
+    _close_bf16(wl.grad, w64.grad, "dw")
