@@ -164,7 +164,7 @@ class MoELayer(nn.Module):
             seq = cfg.seq_length if cfg.moe_router_load_balancing_type == "seq_aux_loss" and \
                 y.shape[0] % cfg.seq_length == 0 else None
             aux = moe_ops.load_balancing_loss(full, idx, cfg.num_experts, cfg.moe_router_topk,
-                                              cfg.moe_aux_loss_coeff, seq)
+                                              cfg.moe_aux_loss_coeff, seq, counts)
             probs = AuxLossScaler.apply(probs, aux)
             self.last_aux_loss = aux.detach()
         return probs, idx, counts
@@ -248,12 +248,10 @@ class MoELayer(nn.Module):
     def _forward_local(self, y, probs, flat_e, counts, T, k):
         rows_cap = moe_ops.rows_capacity(T * k, self.e_local)
         sched = moe_ops.build_schedule(counts.to(torch.int32), rows_cap)
-        src, pos = moe_ops.permutation_maps(flat_e, sched)
-        src_token = torch.where(src >= 0, src // k, src)
+        src, pos, src_token = moe_ops.token_maps(flat_e, sched, k)
         inv_pos = pos.view(T, k)
         x_perm = moe_ops.gather_rows(y, src_token, inv_pos)
-        pf = torch.cat([probs.reshape(-1).float(), probs.new_zeros(1, dtype=torch.float32)])
-        probs_perm = pf[src.long()]  # src = -1 picks the appended zero
+        probs_perm = moe_ops.permute_probs(probs, src, pos)
         out_perm = self.experts_forward(x_perm, probs_perm, sched)
         return moe_ops.combine_rows(out_perm, inv_pos, src_token)
 
@@ -293,8 +291,7 @@ class MoELayer(nn.Module):
         sched = moe_ops.build_schedule(counts_local, rows_cap)
         src, pos = moe_ops.permutation_maps(expert_of_row, sched)
         x_perm = moe_ops.gather_rows(recv, src, pos.view(R, 1))
-        pf = torch.cat([recv_probs, recv_probs.new_zeros(1)])
-        probs_perm = pf[src.long()]
+        probs_perm = moe_ops.permute_probs(recv_probs, src, pos)
         out_perm = self.experts_forward(x_perm, probs_perm, sched)
         back = moe_ops.combine_rows(out_perm, pos.view(R, 1), src)       # padded layout -> arrival order
         ret = epc.all_to_all(back, out_splits, in_splits, st.ep_group)   # -> this rank's sorted copies

@@ -128,10 +128,11 @@ def router_scores_ref(logits: torch.Tensor, topk: int, score_function: str = "so
 
 
 def load_balancing_loss(full_scores: torch.Tensor, idx: torch.Tensor, num_experts: int, topk: int, coeff: float,
-                        seq_len: Optional[int] = None) -> torch.Tensor:
+                        seq_len: Optional[int] = None, counts: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Switch-style aux loss ``coeff * E * sum_e f_e * P_e`` with ``f_e`` the fraction of routed tokens and
     ``P_e`` the mean score.  With ``seq_len`` the loss is computed per sequence and averaged
-    (``seq_aux_loss``)."""
+    (``seq_aux_loss``).  ``counts``: the tokens per expert of ``idx`` where the caller has them (counting them here
+    waits for the device)."""
     T, E = full_scores.shape
     if seq_len:
         B = T // seq_len
@@ -141,8 +142,9 @@ def load_balancing_loss(full_scores: torch.Tensor, idx: torch.Tensor, num_expert
         f = onehot.sum(1) / (seq_len * topk)
         P = scores.mean(1)
         return coeff * E * (f * P).sum(-1).mean()
-    counts = torch.bincount(idx.reshape(-1), minlength=E).float()
-    f = counts / (T * topk)
+    if counts is None:
+        counts = torch.bincount(idx.reshape(-1), minlength=E)
+    f = counts.float() / (T * topk)
     P = full_scores.mean(0)
     return coeff * E * (f * P).sum()
 
@@ -189,8 +191,26 @@ def permutation_maps(expert_of_copy: torch.Tensor, sched: Schedule):
     """expert_of_copy: int64 [R] local expert of every routed row (in arrival order).
     Returns (src [rows_cap] int32: arrival row feeding each padded row, -1 for padding;
              pos [R] int32: padded row of every arrival row)."""
+    src, pos, _ = _maps(expert_of_copy, sched, 1, False)
+    return src, pos
+
+
+def token_maps(expert_of_copy: torch.Tensor, sched: Schedule, topk: int):
+    """:func:`permutation_maps` of ``topk`` copies per token: (src, pos, src_token), where ``src_token`` [rows_cap] is the
+    token (``src // topk``) feeding each padded row."""
+    return _maps(expert_of_copy, sched, topk, True)
+
+
+def _maps(expert_of_copy, sched: Schedule, topk: int, tokens: bool):
     R = expert_of_copy.numel()
     dev = expert_of_copy.device
+    if expert_of_copy.is_cuda:
+        src = torch.empty(sched.rows_cap, dtype=torch.int32, device=dev)
+        src_token = torch.empty(sched.rows_cap, dtype=torch.int32, device=dev) if tokens else None
+        pos = torch.empty(R, dtype=torch.int32, device=dev)
+        _lib.call("moe_permutation_maps", expert_of_copy.long().contiguous(), R, topk, sched.row_start.numel(),
+                  sched.row_start, sched.padded, sched.rows_cap, src, src_token, pos)
+        return src, pos, src_token
     order = torch.argsort(expert_of_copy, stable=True)
     sorted_e = expert_of_copy[order]
     cum = torch.cumsum(sched.counts.long(), 0) - sched.counts.long()
@@ -200,7 +220,35 @@ def permutation_maps(expert_of_copy: torch.Tensor, sched: Schedule):
     src[dest] = order.to(torch.int32)
     pos = torch.empty(R, dtype=torch.int32, device=dev)
     pos[order] = dest.to(torch.int32)
-    return src, pos
+    return src, pos, torch.where(src >= 0, src // topk, src) if tokens else None
+
+
+class PermuteProbsFn(torch.autograd.Function):
+    """out[r] = probs[src[r]] (0 for padding rows).  Every copy feeds exactly one row, so the backward is the gather of
+    the rows' gradients by ``pos``."""
+
+    @staticmethod
+    def forward(ctx, probs, src, pos):
+        out = torch.empty(src.numel(), dtype=torch.float32, device=probs.device)
+        _lib.call("gather_f32", probs, src, out, src.numel())
+        ctx.save_for_backward(pos)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        (pos,) = ctx.saved_tensors
+        d = torch.empty(pos.numel(), dtype=torch.float32, device=dout.device)
+        _lib.call("gather_f32", dout.float().contiguous(), pos, d, pos.numel())
+        return d, None, None
+
+
+def permute_probs(probs, src, pos):
+    """Routing probabilities [R] of the copies -> fp32 [rows_cap] of the padded rows they feed (0 for padding)."""
+    probs = probs.reshape(-1).float()
+    if not probs.is_cuda:
+        pf = torch.cat([probs, probs.new_zeros(1)])
+        return pf[src.long()]  # src = -1 picks the appended zero
+    return PermuteProbsFn.apply(probs.contiguous(), src, pos)
 
 
 class GatherRowsFn(torch.autograd.Function):

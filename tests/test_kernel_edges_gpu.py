@@ -51,3 +51,24 @@ def test_rmsnorm_widths(H, rows, with_res):
     _close_bf16(y.detach(), y64.detach(), "y")
     _close_bf16(xl.grad, s64.grad, "dx")
     _close_bf16(wl.grad, w64.grad, "dw")
+
+
+@pytest.mark.parametrize("R,E,topk", [(1, 1, 1), (31, 5, 1), (4095, 8, 3), (4096, 300, 4), (4100, 7, 2), (12289, 64, 1)])
+def test_permutation_maps_match_stable_sort(R, E, topk):
+    e = torch.randint(0, E, (R,), generator=torch.Generator().manual_seed(R))
+    e[e == E // 2] = 0                                     # an expert without copies (except when it is the only one)
+    counts = torch.bincount(e, minlength=E).to(torch.int32)
+    cap = M.rows_capacity(R, E)
+    cpu = M.token_maps(e, M.build_schedule(counts, cap), topk)
+    gpu = M.token_maps(e.cuda(), M.build_schedule(counts.cuda(), cap), topk)
+    for c, g, name in zip(cpu, gpu, ("src", "pos", "src_token")):
+        assert torch.equal(c, g.cpu()), name
+    src, pos = M.permutation_maps(e.cuda(), M.build_schedule(counts.cuda(), cap))
+    assert torch.equal(src.cpu(), cpu[0]) and torch.equal(pos.cpu(), cpu[1])
+    p = torch.rand(R, device="cuda", requires_grad=True)
+    out = M.permute_probs(p, src, pos)
+    ref = torch.where(src >= 0, p.detach()[src.clamp_min(0).long()], torch.zeros((), device="cuda"))
+    assert torch.equal(out.detach(), ref)
+    d = torch.rand(cap, device="cuda")
+    out.backward(d)
+    assert torch.equal(p.grad, d[pos.long()])
