@@ -219,8 +219,15 @@ def gemm(
 
 
 def launch_bf16(a, b, out, M: int, N: int, K: int, a_mn: bool, b_mn: bool, mode: int, block_n: int,
-                max_ctas: int = 0) -> None:
-    """Raw launch of the bf16 tcgen05 GEMM with explicit tile options (the autotuner times candidates through it)."""
+                max_ctas: int = 0, two_cta: bool | None = None) -> None:
+    """Raw launch of the bf16 tcgen05 GEMM with explicit tile options (the autotuner times candidates through it).
+    ``two_cta``: the CTA-pair kernel (None: where both dimensions fill a 256 x 256 tile)."""
+    if two_cta is None:
+        two_cta = block_n == 256 and M >= 256 and N >= 256 and max_ctas != 1
+    if two_cta:
+        _lib.call("gemm_bf16_2cta", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                  int(a_mn), int(b_mn), mode, max_ctas, _lib.status_word(a.device))
+        return
     _lib.call(
         "gemm_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
         int(a_mn), int(b_mn), mode, block_n, max_ctas, _lib.status_word(a.device),

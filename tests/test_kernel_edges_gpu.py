@@ -72,3 +72,27 @@ def test_permutation_maps_match_stable_sort(R, E, topk):
     d = torch.rand(cap, device="cuda")
     out.backward(d)
     assert torch.equal(p.grad, d[pos.long()])
+
+
+@pytest.mark.parametrize("M_,N_,K_", [(256, 256, 64), (256, 264, 72), (264, 256, 200), (520, 1000, 64), (1000, 520, 328),
+                                      (4096, 2048, 136), (8, 136, 2048), (136, 264, 4104), (768, 256, 3208), (256, 512, 2056)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True), (True, False)])
+def test_cta_pair_bf16_gemm(M_, N_, K_, a_mn, b_mn):
+    g = _gen(M_ + N_ + K_)
+    a = torch.randn(*((K_, M_) if a_mn else (M_, K_)), device="cuda", generator=g).bfloat16()
+    b = torch.randn(*((K_, N_) if b_mn else (N_, K_)), device="cuda", generator=g).bfloat16()
+    A, B = (a.t() if a_mn else a).double(), (b if b_mn else b.t()).double()
+    ref = A @ B
+    lim = 2.0 ** -24 * K_ * (A.abs() @ B.abs()).max()     # fp32 accumulation in any order
+    for mode, out in (("bf16", None), ("f32", torch.empty(M_, N_, device="cuda")), ("add", torch.ones(M_, N_, device="cuda"))):
+        got = gemm.gemm(a, b, a_mn, b_mn, out=out, accumulate=mode == "add").double()
+        torch.cuda.synchronize()
+        _lib.check_status()
+        if mode == "bf16":
+            _close_bf16(got, ref, mode)
+        else:
+            err = (got - ref - (1 if mode == "add" else 0)).abs().max()
+            assert err <= lim + 2.0 ** -22 * ref.abs().max(), f"{mode}: {err}"
+        again = gemm.gemm(a, b, a_mn, b_mn, out=torch.empty_like(got, dtype=torch.float32) if mode != "bf16" else None)
+        if mode != "add":
+            assert torch.equal(again.double(), got), "not reproducible"
