@@ -117,12 +117,15 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 #define PB_NORM_FWD(LPR, VPL, RPG, THREADS)                                                             \
   rmsnorm_fwd_kernel<LPR, VPL, RPG, THREADS>                                                            \
       <<<(unsigned)((rows + (THREADS / LPR) * RPG - 1) / ((THREADS / LPR) * RPG)), THREADS, 0, s>>>(args...)
-  if (nv <= 8) PB_NORM_FWD(8, 1, 4, 128);
-  else if (nv <= 16) PB_NORM_FWD(16, 1, 4, 128);
-  else if (nv <= 32) PB_NORM_FWD(32, 1, 4, 128);
-  else if (nv <= 64) PB_NORM_FWD(32, 2, 2, 128);
-  else if (nv <= 128) PB_NORM_FWD(32, 4, 1, 128);
-  else if (nv <= 256) PB_NORM_FWD(64, 4, 1, 128);
+  // a few hundred rows do not fill the SMs with four rows (or four vectors) per lane: spread them (768 rows of 256: 3.0 ->
+  // 2.2 us; at 4096 rows of 2048 the wide form is already the better one, 12.2 against 13.5 us)
+  const bool few = rows * nv < 148 * 2048L;
+  if (nv <= 8) { if (few) PB_NORM_FWD(8, 1, 1, 128); else PB_NORM_FWD(8, 1, 4, 128); }
+  else if (nv <= 16) { if (few) PB_NORM_FWD(16, 1, 1, 128); else PB_NORM_FWD(16, 1, 4, 128); }
+  else if (nv <= 32) { if (few) PB_NORM_FWD(32, 1, 1, 128); else PB_NORM_FWD(32, 1, 4, 128); }
+  else if (nv <= 64) { if (few) PB_NORM_FWD(32, 2, 1, 128); else PB_NORM_FWD(32, 2, 2, 128); }
+  else if (nv <= 128) { if (few) PB_NORM_FWD(128, 1, 1, 128); else PB_NORM_FWD(32, 4, 1, 128); }
+  else if (nv <= 256) { if (few) PB_NORM_FWD(256, 1, 1, 256); else PB_NORM_FWD(64, 4, 1, 128); }
   else if (nv <= 512) PB_NORM_FWD(128, 4, 1, 128);
   else if (nv <= 1024) PB_NORM_FWD(256, 4, 1, 256);
   else PB_NORM_FWD(512, 4, 1, 512);
@@ -366,9 +369,10 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
 #define PB_NORM_BWD(VPT, THREADS)                                                                                     \
   return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy) \
               : launch_rmsnorm_bwd_ring<VPT, THREADS, false>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy)
-  if (nv <= 8) PB_NORM_BWD_SHORT(8, 1, 4)
-  if (nv <= 16) PB_NORM_BWD_SHORT(16, 1, 4)
-  if (nv <= 32) PB_NORM_BWD_SHORT(32, 1, 4)
+  const bool few = rows * nv < 148 * 512L * 4;   // (two CTAs of 256 threads per SM)
+  if (nv <= 8) { if (few) PB_NORM_BWD_SHORT(8, 1, 1) else PB_NORM_BWD_SHORT(8, 1, 4) }
+  if (nv <= 16) { if (few) PB_NORM_BWD_SHORT(16, 1, 1) else PB_NORM_BWD_SHORT(16, 1, 4) }
+  if (nv <= 32) { if (few) PB_NORM_BWD_SHORT(32, 1, 1) else PB_NORM_BWD_SHORT(32, 1, 4) }
   if (nv <= 64) PB_NORM_BWD_SHORT(32, 2, 2)
   if (nv <= 128) PB_NORM_BWD_SHORT(32, 4, 1)
   if (nv <= 256) PB_NORM_BWD(1, 256);
@@ -379,19 +383,152 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
 #undef PB_NORM_BWD_SHORT
 }
 
+// ------------------------------------------------------------------ per-head norms of q and k in a packed QKV tensor
+// qkv [T, (hq + 2 hkv) * d] = [q heads | k heads | v heads]: every q and k head is normalised with its own gain (wq / wk),
+// v heads are copied, and the result is packed the same way, so that nothing is sliced, copied or concatenated around the
+// norms.  A group of LPR lanes owns a head row; RPG head rows of a group are in flight.
+template <int LPR, int RPG>
+__global__ void __launch_bounds__(128)
+qk_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq,
+                   const __nv_bfloat16* __restrict__ wk, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
+                   long rows, int hq, int hkv, int d, long ldx, long ldy, float eps) {
+  const int lane = threadIdx.x % LPR;
+  const long row0 = (blockIdx.x * (long)(128 / LPR) + threadIdx.x / LPR) * RPG;
+  const int heads = hq + 2 * hkv;
+  const bool in = lane < d / 8;
+  Bf8 v[RPG], gq, gk;
+  if (in) {
+    gq = reinterpret_cast<const Bf8*>(wq)[lane];
+    gk = reinterpret_cast<const Bf8*>(wk)[lane];
+  }
+#pragma unroll
+  for (int r = 0; r < RPG; ++r) {
+    const long row = row0 + r;
+    if (row < rows && in) v[r] = reinterpret_cast<const Bf8*>(x + row / heads * ldx + row % heads * d)[lane];
+  }
+#pragma unroll
+  for (int r = 0; r < RPG; ++r) {
+    const long row = row0 + r, t = row / heads;
+    const int h = (int)(row - t * heads);
+    const bool live = row < rows && in;
+    float f[8], ss = 0.f;
+    if (live) {
+      bf8_to_f(v[r], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+    const float rstd = rsqrtf(group_sum<LPR>(ss, nullptr) / d + eps);
+    if (!live) continue;
+    if (h < hq + hkv) {
+      float g[8];
+      bf8_to_f(h < hq ? gq : gk, g);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+      v[r] = f_to_bf8(f);
+      if (lane == 0) rstd_out[t * (hq + hkv) + h] = rstd;
+    }
+    reinterpret_cast<Bf8*>(y + t * ldy + (long)h * d)[lane] = v[r];
+  }
+}
+
+// Backward: dx of the q and k heads, the v gradient copied; gain sums per CTA in partial [gridDim.x, 2 d] (q, then k).
+template <int LPR, int RPG>
+__global__ void __launch_bounds__(256, 2)
+qk_norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
+                   const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
+                   const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, long rows,
+                   int hq, int hkv, int d, long ldx, long lddy, long lddx) {
+  constexpr int GROUPS = 256 / LPR;
+  __shared__ float4 sums[GROUPS][LPR * 2];
+  const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
+  const int heads = hq + 2 * hkv;
+  const bool in = lane < d / 8;
+  Bf8 gq, gk;
+  float dw[2][8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) dw[0][j] = dw[1][j] = 0.f;
+  if (in) {
+    gq = reinterpret_cast<const Bf8*>(wq)[lane];
+    gk = reinterpret_cast<const Bf8*>(wk)[lane];
+  }
+  const long stride = (long)gridDim.x * GROUPS * RPG;
+  for (long base = (long)blockIdx.x * GROUPS * RPG; base < rows; base += stride) {
+    const long row0 = base + grp * RPG;
+    Bf8 vx[RPG], vg[RPG];
+    float rs[RPG];
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) {
+      const long row = row0 + r, t = row / heads;
+      const int h = (int)(row - t * heads);
+      rs[r] = 0.f;
+      if (row < rows && in) {
+        vg[r] = reinterpret_cast<const Bf8*>(dy + t * lddy + (long)h * d)[lane];
+        if (h < hq + hkv) {
+          vx[r] = reinterpret_cast<const Bf8*>(x + t * ldx + (long)h * d)[lane];
+          rs[r] = rstd[t * (hq + hkv) + h];
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RPG; ++r) {
+      const long row = row0 + r, t = row / heads;
+      const int h = (int)(row - t * heads);
+      const bool live = row < rows && in, norm = live && h < hq + hkv;
+      float fx[8], fg[8], dot = 0.f;
+      if (norm) {
+        float fw[8];
+        bf8_to_f(vx[r], fx);
+        bf8_to_f(vg[r], fg);
+        bf8_to_f(h < hq ? gq : gk, fw);
+        const float sq = h < hq ? rs[r] : 0.f, sk = h < hq ? 0.f : rs[r];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          dw[0][j] += fg[j] * fx[j] * sq;
+          dw[1][j] += fg[j] * fx[j] * sk;
+          fg[j] *= fw[j];
+          dot += fg[j] * fx[j];
+        }
+      }
+      dot = group_sum<LPR>(dot, nullptr);
+      if (norm) {
+        const float c = dot * rs[r] * rs[r] * rs[r] / d;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) fg[j] = fg[j] * rs[r] - fx[j] * c;
+        vg[r] = f_to_bf8(fg);
+      }
+      if (live) reinterpret_cast<Bf8*>(dx + t * lddx + (long)h * d)[lane] = vg[r];
+    }
+  }
+#pragma unroll
+  for (int w = 0; w < 2; ++w) {
+    __syncthreads();
+    sums[grp][lane * 2] = make_float4(dw[w][0], dw[w][1], dw[w][2], dw[w][3]);
+    sums[grp][lane * 2 + 1] = make_float4(dw[w][4], dw[w][5], dw[w][6], dw[w][7]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < d / 4; i += 256) {
+      float4 t = sums[0][i];
+      for (int g = 1; g < GROUPS; ++g) {
+        const float4 u = sums[g][i];
+        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
+      }
+      reinterpret_cast<float4*>(partial + (long)blockIdx.x * 2 * d + w * d)[i] = t;
+    }
+  }
+}
+
 // dw[h] (+)= sum_p partial[p, h].  A CTA owns 32 columns; its 16 thread rows each add every 16th partial (coalesced
 // 128-byte reads, eight in flight) and a fixed-order tree in shared memory folds them, so the result does not depend on
 // scheduling.
 constexpr int DWR_COLS = 32, DWR_ROWS = 16;
 __global__ void __launch_bounds__(DWR_COLS * DWR_ROWS)
-rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, int accumulate) {
+rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, long ld, int accumulate) {
   __shared__ float red[DWR_ROWS][DWR_COLS + 1];
   const int c = threadIdx.x % DWR_COLS, g = threadIdx.x / DWR_COLS;
   const int h = blockIdx.x * DWR_COLS + c;
   float s = 0.f;
   if (h < H) {
 #pragma unroll 8
-    for (int p = g; p < P; p += DWR_ROWS) s += partial[(long)p * H + h];
+    for (int p = g; p < P; p += DWR_ROWS) s += partial[p * ld + h];
   }
   red[g][c] = s;
   __syncthreads();
@@ -409,7 +546,7 @@ int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float
   const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                     (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, H, ldx, lddy);
   if (rc) return rc;
-  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, dw_accumulate);
+  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, H, dw_accumulate);
   return (int)cudaGetLastError();
 }
 
@@ -437,6 +574,45 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
   if (rows == 0) return 0;
   return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
+}
+
+// y = qkv with RMSNorm over every q head (gain wq) and k head (gain wk); rstd: fp32 [T, hq + hkv].
+int pb_qk_norm_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, long T, int hq, int hkv, int d,
+                   long ldx, long ldy, float eps, cudaStream_t s) {
+  if (d % 8 || d <= 0 || d > 256 || ldx % 8 || ldy % 8) return -2;
+  const long rows = T * (hq + 2 * hkv);
+  if (rows == 0) return 0;
+#define PB_QK_FWD(LPR)                                                                                                  \
+  qk_norm_fwd_kernel<LPR, 4><<<(unsigned)((rows + 128 / LPR * 4 - 1) / (128 / LPR * 4)), 128, 0, s>>>(                  \
+      (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, (__nv_bfloat16*)y, rstd, rows, hq, hkv, \
+      d, ldx, ldy, eps)
+  if (d <= 64) PB_QK_FWD(8);
+  else if (d <= 128) PB_QK_FWD(16);
+  else PB_QK_FWD(32);
+#undef PB_QK_FWD
+  return (int)cudaGetLastError();
+}
+
+// scratch: fp32 [pb_rmsnorm_bwd_num_partials(T), 2 d]; dwq / dwk: fp32 [d], dw_accumulate: += instead of =.
+int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq,
+                   float* dwk, float* scratch, long T, int hq, int hkv, int d, long ldx, long lddy, long lddx,
+                   int dw_accumulate, cudaStream_t s) {
+  if (d % 8 || d <= 0 || d > 256 || ldx % 8 || lddy % 8 || lddx % 8) return -2;
+  const long rows = T * (hq + 2 * hkv);
+  if (rows == 0) return 0;
+  const int P = pb_rmsnorm_bwd_num_partials(T);
+#define PB_QK_BWD(LPR)                                                                                            \
+  qk_norm_bwd_kernel<LPR, 4><<<P, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                 \
+                                               (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, rstd,          \
+                                               (__nv_bfloat16*)dx, scratch, rows, hq, hkv, d, ldx, lddy, lddx)
+  if (d <= 64) PB_QK_BWD(8);
+  else if (d <= 128) PB_QK_BWD(16);
+  else PB_QK_BWD(32);
+#undef PB_QK_BWD
+  const int blocks = (d + DWR_COLS - 1) / DWR_COLS, threads = DWR_COLS * DWR_ROWS;
+  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate);
+  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate);
+  return (int)cudaGetLastError();
 }
 
 }  // extern "C"

@@ -153,14 +153,8 @@ class SelfAttention(nn.Module):
 
     def _qk_norm(self, qkv, d):
         """Per-head RMSNorm of q and k (Qwen3)."""
-        T = qkv.shape[0]
-        hq, hkv = self.hq, self.hkv
-        q = qkv[:, : hq * d].reshape(T * hq, d)
-        k = qkv[:, hq * d: (hq + hkv) * d].reshape(T * hkv, d)
-        v = qkv[:, (hq + hkv) * d:]
-        qn = fused.rmsnorm(q, self.q_layernorm.weight, self.cfg.norm_epsilon).reshape(T, hq * d)
-        kn = fused.rmsnorm(k, self.k_layernorm.weight, self.cfg.norm_epsilon).reshape(T, hkv * d)
-        return torch.cat([qn, kn, v], dim=1)
+        return fused.qk_norm(qkv, self.q_layernorm.weight, self.k_layernorm.weight, self.hq, self.hkv, d,
+                             self.cfg.norm_epsilon)
 
 
 class MLP(nn.Module):

@@ -124,6 +124,49 @@ def rmsnorm(x, w, eps=1e-5, residual=None):
     return RMSNormFn.apply(x, w, eps, residual)
 
 
+class QKNormFn(torch.autograd.Function):
+    """RMSNorm of every q and k head inside a packed [T, (hq + 2 hkv) d] projection output; v passes through."""
+
+    @staticmethod
+    def forward(ctx, qkv, wq, wk, hq, hkv, d, eps):
+        T = qkv.shape[0]
+        out = torch.empty(T, (hq + 2 * hkv) * d, dtype=qkv.dtype, device=qkv.device)
+        rstd = torch.empty(T, hq + hkv, dtype=torch.float32, device=qkv.device)
+        _lib.call("qk_norm_fwd", qkv, wq, wk, out, rstd, T, hq, hkv, d, qkv.stride(0), out.stride(0), float(eps))
+        ctx.save_for_backward(qkv, wq, wk, rstd)
+        ctx.dims = (hq, hkv, d)
+        ctx.w_refs = (wq, wk)
+        return out
+
+    @staticmethod
+    def backward(ctx, dy):
+        qkv, wq, wk, rstd = ctx.saved_tensors
+        hq, hkv, d = ctx.dims
+        T = qkv.shape[0]
+        if not dy.is_contiguous():
+            dy = dy.contiguous()
+        dx = torch.empty(T, (hq + 2 * hkv) * d, dtype=qkv.dtype, device=qkv.device)
+        main = [getattr(w, "main_grad", None) for w in ctx.w_refs]
+        dw = [g if g is not None else torch.zeros(d, dtype=torch.float32, device=qkv.device) for g in main]
+        P = _lib.call_ret("rmsnorm_bwd_num_partials", T)
+        _lib.call("qk_norm_bwd", dy, qkv, wq, wk, rstd, dx, dw[0], dw[1], scratch(qkv.device, "qk_norm_dw", P * 2 * d),
+                  T, hq, hkv, d, qkv.stride(0), dy.stride(0), dx.stride(0), 1)
+        dwq, dwk = (None if g is not None else t.to(w.dtype) for g, t, w in zip(main, dw, (wq, wk)))
+        return dx, dwq, dwk, None, None, None, None
+
+
+def qk_norm(qkv, wq, wk, hq, hkv, d, eps=1e-5):
+    """Per-head RMSNorm of the q heads (gain ``wq`` [d]) and k heads (``wk``) of a packed tensor
+    ``[q heads | k heads | v heads]`` [T, (hq + 2 hkv) d]; the v heads are unchanged."""
+    T = qkv.shape[0]
+    if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and d % 8 == 0 and d <= 256
+            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
+        return QKNormFn.apply(qkv, gamma(wq), gamma(wk), hq, hkv, d, eps)
+    q = rmsnorm(qkv[:, : hq * d].reshape(T * hq, d), wq, eps).reshape(T, hq * d)
+    k = rmsnorm(qkv[:, hq * d: (hq + hkv) * d].reshape(T * hkv, d), wk, eps).reshape(T, hkv * d)
+    return torch.cat([q, k, qkv[:, (hq + hkv) * d:]], dim=1)
+
+
 # ----------------------------------------------------------------------------------------------
 # RoPE (rotate-half convention, first ``rot_dim`` channels of each head)
 def llama3_scale_frequencies(inv, factor: float, low_freq_factor: float = 1.0, high_freq_factor: float = 4.0,

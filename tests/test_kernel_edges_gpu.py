@@ -96,3 +96,29 @@ def test_cta_pair_bf16_gemm(M_, N_, K_, a_mn, b_mn):
         again = gemm.gemm(a, b, a_mn, b_mn, out=torch.empty_like(got, dtype=torch.float32) if mode != "bf16" else None)
         if mode != "add":
             assert torch.equal(again.double(), got), "not reproducible"
+
+
+@pytest.mark.parametrize("T,hq,hkv,d,pad", [(1, 1, 1, 64, 0), (130, 4, 2, 128, 0), (77, 6, 3, 72, 16), (33, 2, 1, 256, 0),
+                                            (2000, 8, 1, 128, 8)])
+def test_qk_norm_matches_separate_norms(T, hq, hkv, d, pad):
+    g = _gen(d)
+    W = (hq + 2 * hkv) * d
+    buf = torch.randn(T, W + pad, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(T, W, device="cuda", generator=g).bfloat16()
+    wq, wk = ((1 + 0.1 * torch.randn(d, device="cuda", generator=g)).bfloat16().requires_grad_() for _ in range(2))
+    wk.main_grad = torch.ones(d, device="cuda")
+    qkv = buf.requires_grad_()
+    out = fused.qk_norm(qkv[:, :W], wq, wk, hq, hkv, d)
+    out.backward(dy)
+    x64 = buf.detach()[:, :W].double().requires_grad_()
+    q64, k64 = wq.detach().double().requires_grad_(), wk.detach().double().requires_grad_()
+    h = x64.view(T, hq + 2 * hkv, d)
+    ref = torch.cat([_rms64(h[:, :hq], q64), _rms64(h[:, hq:hq + hkv], k64), h[:, hq + hkv:]], 1).reshape(T, W)
+    ref.backward(dy.double())
+    _close_bf16(out.detach(), ref.detach(), "out")
+    assert torch.equal(out.detach()[:, (hq + hkv) * d:], buf.detach()[:, (hq + hkv) * d:W])
+    _close_bf16(qkv.grad[:, :W], x64.grad, "dqkv")
+    _close_bf16(wq.grad, q64.grad, "dwq")
+    assert wk.grad is None
+    err = (wk.main_grad.double() - 1 - k64.grad).abs().max()
+    assert err <= 1e-4 * (1 + k64.grad.abs().max()), f"dwk {err}"
