@@ -19,6 +19,10 @@
 //   tmem_empty[acc] in the even CTA: one arrival per epilogue warp of both CTAs, as soon as the warp has read its part.
 // A cluster barrier closes the kernel so that neither CTA exits while its peer may still touch its memory.
 //
+// Split K: where the output has too few tiles for the SMs and K is long (the data gradient of an output head over few
+// tokens: K is the vocabulary), the K range is cut into `splits` parts whose fp32 partial tiles go to a workspace
+// [splits, M rounded up to 256, N]; a second kernel adds the parts in order, so the result does not depend on scheduling.
+//
 // Operand layouts and output modes as in csrc/gemm_bf16.cu.
 #include "common.cuh"
 
@@ -100,7 +104,8 @@ __device__ __forceinline__ void tile_coords(int tile, int num_m, int num_n, int&
 template <int A_MN, int B_MN, int OUT>
 __global__ void __launch_bounds__(NUM_THREADS, 1)
 gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                      const __grid_constant__ CUtensorMap tmD, int M, int N, int K, int* status) {
+                      const __grid_constant__ CUtensorMap tmD, int M, int N, int K, int splits, int kb_per_split,
+                      int* status) {
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* smem_ab = smem;
@@ -114,7 +119,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   const int num_pairs = gridDim.x >> 1;
   const int num_m = (M + 2 * BM - 1) / (2 * BM);
   const int num_n = (N + BN - 1) / BN;
-  const int num_tiles = num_m * num_n;
+  const int tiles_per_split = num_m * num_n;
+  const int num_tiles = tiles_per_split * splits;
   const int num_kb = (K + BK - 1) / BK;
   volatile int* abort_flag = &bars->abort_flag;
 
@@ -151,10 +157,12 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       bool ok = true;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
         int mb, nb;
-        tile_coords(tile, num_m, num_n, mb, nb);
+        const int split = tile / tiles_per_split;
+        tile_coords(tile - split * tiles_per_split, num_m, num_n, mb, nb);
         const int m0 = (mb * 2 + (int)cta) * BM;         // 128-row block of this CTA
         const int n0 = nb * BN + (int)cta * (BN / 2);    // this CTA's half of the B tile
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int kb_end = min(num_kb, (split + 1) * kb_per_split);
+        for (int kb = split * kb_per_split; kb < kb_end; ++kb) {
           if (!wait_or_abort(&bars->empty[stage], phase ^ 1, abort_flag)) {
             atomicCAS(status, 0, PB_ERR_TIMEOUT_TMA);
             bars->abort_flag = 1;
@@ -201,7 +209,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         }
         pb::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
-        for (int kb = 0; kb < num_kb; ++kb) {
+        const int kb0 = tile / tiles_per_split * kb_per_split, kb_end = min(num_kb, kb0 + kb_per_split);
+        for (int kb = kb0; kb < kb_end; ++kb) {
           if (!wait_or_abort(&bars->full[stage], phase, abort_flag)) {
             atomicCAS(status, 0, PB_ERR_TIMEOUT_MMA);
             bars->abort_flag = 1;
@@ -217,7 +226,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                                      : pb::make_smem_desc(sa + k * (UMMA_K * 2), 0, 1024, 2);
             const uint64_t db = B_MN ? pb::make_smem_desc(sb + k * (UMMA_K * 128), BK * 128, 1024, 2)
                                      : pb::make_smem_desc(sb + k * (UMMA_K * 2), 0, 1024, 2);
-            umma_f16_ss_2cta(d_tmem, da, db, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+            umma_f16_ss_2cta(d_tmem, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           pb::umma_commit_2cta(&bars->empty[stage], 3);
           if (++stage == STAGES) {
@@ -244,8 +253,10 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
     uint32_t acc_phase = 0;
     for (int tile = pair; tile < num_tiles; tile += num_pairs) {
       int mb, nb;
-      tile_coords(tile, num_m, num_n, mb, nb);
+      const int split = tile / tiles_per_split;
+      tile_coords(tile - split * tiles_per_split, num_m, num_n, mb, nb);
       const int m0 = (mb * 2 + (int)cta) * BM + lane_grp * 32, n0 = nb * BN + half * HC;
+      const int row0 = split * num_m * 2 * BM + m0;     // in the output, or in the workspace of the parts
       if (!warp_wait_or_abort(&bars->tmem_full[acc], acc_phase, abort_flag, lane)) {
         atomicCAS(status, 0, PB_ERR_TIMEOUT_EPILOGUE);
         bars->abort_flag = 1;
@@ -260,8 +271,8 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
         pb::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0 && m0 < M && n < N) {
-          if (OUT == OUT_F32_ADD) pb::tma_reduce_add_2d(&tmD, ebuf, n, m0);
-          else pb::tma_store_2d(&tmD, ebuf, n, m0);
+          if (OUT == OUT_F32_ADD) pb::tma_reduce_add_2d(&tmD, ebuf, n, row0);
+          else pb::tma_store_2d(&tmD, ebuf, n, row0);
           pb::tma_store_commit();
           pb::tma_store_wait_read<0>();    // the staging buffer may be overwritten by the next round
         }
@@ -323,7 +334,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
 template <int A_MN, int B_MN, int OUT>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, int M, int N, int K, int* status,
-           int max_ctas, cudaStream_t stream) {
+           int max_ctas, cudaStream_t stream, int splits = 1) {
   auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN, OUT>;
   static bool attr_set = false;
   if (!attr_set) {
@@ -353,14 +364,64 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
     }
     max_pairs = n;
   }
-  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+  const int num_kb = (K + BK - 1) / BK;
+  const int kb_per_split = (num_kb + splits - 1) / splits;
+  const int tiles = ((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN) * splits;
   int pairs = max_pairs;
   if (max_ctas > 0 && max_ctas / 2 < pairs) pairs = max_ctas / 2;
   if (tiles < pairs) pairs = tiles;
   if (pairs < 1) pairs = 1;
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.stream = stream;
-  return (int)cudaLaunchKernelEx(&cfg, kern, tA, tB, tD, M, N, K, status);
+  return (int)cudaLaunchKernelEx(&cfg, kern, tA, tB, tD, M, N, K, splits, kb_per_split, status);
+}
+
+// out[m, n] (=|+=) sum over the parts of ws[s, m, n]; four columns per thread, parts in order
+template <int OUT>
+__global__ void __launch_bounds__(256)
+splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ out, int M, int N, long ldd, int splits, long part) {
+  const int nv = N / 4;
+  const long i = blockIdx.x * 256L + threadIdx.x;
+  const long m = i / nv;
+  if (m >= M) return;
+  const int n = (int)(i - m * nv) * 4;
+  const float4* p = reinterpret_cast<const float4*>(ws + m * N + n);
+  float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 4
+  for (int s = 0; s < splits; ++s) {
+    const float4 v = p[s * (part / 4)];
+    a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+  }
+  if (OUT == OUT_BF16) {
+    uint2 h = make_uint2(pb::pack_bf16x2(a.x, a.y), pb::pack_bf16x2(a.z, a.w));
+    *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(out) + m * ldd + n) = h;
+  } else {
+    float4* o = reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + m * ldd + n);
+    if (OUT == OUT_F32_ADD) {
+      const float4 v = *o;
+      a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+    }
+    *o = a;
+  }
+}
+
+int check_operands(const void* A, const void* B, const void* D, long lda, long ldb, long ldd, int out_mode) {
+  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16) ||
+      (reinterpret_cast<uintptr_t>(D) % 16))
+    return -2;
+  return (out_mode == 0 ? (ldd % 8) : (ldd % 4)) ? -2 : 0;
+}
+
+int operand_maps(CUtensorMap& tA, CUtensorMap& tB, const void* A, const void* B, int M, int N, int K, long lda, long ldb,
+                 int a_mn, int b_mn) {
+  const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
+  int rc;
+  if (!a_mn) rc = pbh::make_tmap_2d(&tA, A, bf, 2, M, K, lda, BM, BK, sw);
+  else rc = pbh::make_tmap_2d(&tA, A, bf, 2, K, M, lda, BK, 64, sw);
+  if (rc) return rc;
+  if (!b_mn) return pbh::make_tmap_2d(&tB, B, bf, 2, N, K, ldb, BN / 2, BK, sw);
+  return pbh::make_tmap_2d(&tB, B, bf, 2, K, N, ldb, BK, 64, sw);
 }
 
 }  // namespace
@@ -369,22 +430,13 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
 extern "C" int pb_gemm_bf16_2cta(const void* A, const void* B, void* D, int M, int N, int K, long lda, long ldb, long ldd,
                                  int a_mn, int b_mn, int out_mode, int max_ctas, int* status, cudaStream_t stream) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if ((lda % 8) || (ldb % 8) || (reinterpret_cast<uintptr_t>(A) % 16) || (reinterpret_cast<uintptr_t>(B) % 16) ||
-      (reinterpret_cast<uintptr_t>(D) % 16))
-    return -2;
-  if (out_mode == 0 ? (ldd % 8) : (ldd % 4)) return -2;
+  int rc = check_operands(A, B, D, lda, ldb, ldd, out_mode);
+  if (rc) return rc;
   CUtensorMap tA, tB, tD;
-  int rc;
-  const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
+  if ((rc = operand_maps(tA, tB, A, B, M, N, K, lda, ldb, a_mn, b_mn))) return rc;
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
-  if (!a_mn) rc = pbh::make_tmap_2d(&tA, A, bf, 2, M, K, lda, BM, BK, sw);
-  else rc = pbh::make_tmap_2d(&tA, A, bf, 2, K, M, lda, BK, 64, sw);
-  if (rc) return rc;
-  if (!b_mn) rc = pbh::make_tmap_2d(&tB, B, bf, 2, N, K, ldb, BN / 2, BK, sw);
-  else rc = pbh::make_tmap_2d(&tB, B, bf, 2, K, N, ldb, BK, 64, sw);
-  if (rc) return rc;
   // output boxes: 32 rows x 128 bytes (64 bf16 / 32 fp32 columns); rows and columns past M, N are clipped by TMA
-  if (out_mode == 0) rc = pbh::make_tmap_2d(&tD, D, bf, 2, M, N, ldd, 32, 64, sw);
+  if (out_mode == 0) rc = pbh::make_tmap_2d(&tD, D, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, M, N, ldd, 32, 64, sw);
   else rc = pbh::make_tmap_2d(&tD, D, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, M, N, ldd, 32, 32, sw);
   if (rc) return rc;
 
@@ -400,4 +452,34 @@ extern "C" int pb_gemm_bf16_2cta(const void* A, const void* B, void* D, int M, i
   else if (a_mn && b_mn) { PB_DISPATCH_OUT(1, 1) }
   else { PB_DISPATCH_OUT(1, 0) }
   return -3;
+}
+
+// The same with K cut into `splits` parts.  ws: fp32 [splits, M rounded up to 256, N] (not initialised); N % 4 == 0 and
+// splits <= ceil(K / 64).  A split count that would leave a part without a K step is lowered.
+extern "C" int pb_gemm_bf16_splitk(const void* A, const void* B, void* D, float* ws, int M, int N, int K, long lda, long ldb,
+                                   long ldd, int a_mn, int b_mn, int out_mode, int splits, int* status,
+                                   cudaStream_t stream) {
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  int rc = check_operands(A, B, D, lda, ldb, ldd, out_mode);
+  if (rc) return rc;
+  const int num_kb = (K + BK - 1) / BK;
+  if (N % 4 || splits < 1 || splits > num_kb || out_mode < 0 || out_mode > 2 || (reinterpret_cast<uintptr_t>(ws) % 16)) return -2;
+  const int per = (num_kb + splits - 1) / splits;
+  splits = (num_kb + per - 1) / per;
+  CUtensorMap tA, tB, tD;
+  if ((rc = operand_maps(tA, tB, A, B, M, N, K, lda, ldb, a_mn, b_mn))) return rc;
+  const long rows = (M + 2 * BM - 1) / (2 * BM) * (2 * BM);
+  if ((rc = pbh::make_tmap_2d(&tD, ws, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, rows * splits, N, N, 32, 32,
+                              CU_TENSOR_MAP_SWIZZLE_128B)))
+    return rc;
+  if (!a_mn && !b_mn) rc = launch<0, 0, OUT_F32>(tA, tB, tD, M, N, K, status, 0, stream, splits);
+  else if (!a_mn && b_mn) rc = launch<0, 1, OUT_F32>(tA, tB, tD, M, N, K, status, 0, stream, splits);
+  else if (a_mn && b_mn) rc = launch<1, 1, OUT_F32>(tA, tB, tD, M, N, K, status, 0, stream, splits);
+  else rc = launch<1, 0, OUT_F32>(tA, tB, tD, M, N, K, status, 0, stream, splits);
+  if (rc) return rc;
+  const unsigned blocks = (unsigned)(((long)M * (N / 4) + 255) / 256);
+  if (out_mode == OUT_BF16) splitk_reduce_kernel<OUT_BF16><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
+  else if (out_mode == OUT_F32) splitk_reduce_kernel<OUT_F32><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
+  else splitk_reduce_kernel<OUT_F32_ADD><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
+  return (int)cudaGetLastError();
 }

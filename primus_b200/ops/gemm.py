@@ -218,11 +218,31 @@ def gemm(
     return out
 
 
+# CTA pairs of a B200, and the K steps (of 64) a part of a split reduction keeps at least: a part of 16 steps takes about as
+# long as adding the parts costs (workspace traffic and one more launch, ~5 us)
+_CTA_PAIRS = 74
+_SPLIT_MIN_STEPS = 16
+
+
+def _split_k(M: int, N: int, K: int) -> int:
+    """Parts to cut the reduction into: as many as fill the idle CTA pairs of a GEMM with few 256 x 256 output tiles."""
+    tiles = -(-M // 256) * -(-N // 256)
+    steps = -(-K // 64)
+    return max(1, min(_CTA_PAIRS // tiles, steps // _SPLIT_MIN_STEPS)) if N % 4 == 0 else 1
+
+
 def launch_bf16(a, b, out, M: int, N: int, K: int, a_mn: bool, b_mn: bool, mode: int, block_n: int,
                 max_ctas: int = 0, two_cta: bool | None = None) -> None:
     """Raw launch of the bf16 tcgen05 GEMM with explicit tile options (the autotuner times candidates through it).
-    ``two_cta``: the CTA-pair kernel (None: where both dimensions fill a 256 x 256 tile)."""
+    ``two_cta``: the CTA-pair kernel (None: where both dimensions fill a 256 x 256 tile, or, with the reduction split,
+    where K is long and the tiles are few)."""
     if two_cta is None:
+        splits = _split_k(M, N, K) if block_n == 256 and max_ctas == 0 else 1
+        if splits > 1:
+            ws = torch.empty(splits * (-(-M // 256) * 256) * N, dtype=torch.float32, device=a.device)
+            _lib.call("gemm_bf16_splitk", a, b, out, ws, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                      int(a_mn), int(b_mn), mode, splits, _lib.status_word(a.device))
+            return
         two_cta = block_n == 256 and M >= 256 and N >= 256 and max_ctas != 1
     if two_cta:
         _lib.call("gemm_bf16_2cta", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
