@@ -21,7 +21,6 @@
 namespace {
 
 constexpr int TILE = 128;
-constexpr int PITCH = TILE + 8;  // bf16 elements per shared-memory row (272 B: conflict-free 16-byte row reads)
 
 __device__ __forceinline__ int e8m0_from_amax(float amax) {
   const float v = amax * (1.0f / 448.0f);
@@ -76,139 +75,155 @@ __device__ __forceinline__ long sf_offset(int mn, int k_blk32, int k_groups) {
   return ((long)(mn >> 7) * k_groups + (k_blk32 >> 2)) * 512 + (mn & 31) * 16 + ((mn & 127) >> 5) * 4 + (k_blk32 & 3);
 }
 
-constexpr int QUANT_SMEM = TILE * PITCH * 2;   // one staged bf16 tile; the fp8 results go from registers to global
-
-// Quantises the 128 x 128 bf16 tile staged in `tile` (row pitch PITCH) whose origin in the [R, C] tensor is
-// (row0, col0).  Called by all threads of a 256-thread CTA after the tile is complete (caller synchronises before).
-// Results are written straight from registers: 64 contiguous bytes per thread in the row direction, 8 bytes per row
-// (64 contiguous bytes per 8 lanes) in the column direction -- whole 32-byte sectors either way.
+// ------------------------------------------------------------------ register quantiser
+// A CTA of four warps quantises a 128 x 128 tile, one warp a strip of 32 rows, one 64-column half after the other.  Lane
+// (cg = lane & 7, sub = lane >> 3) holds columns 8 cg .. 8 cg + 7 of rows 4 i + sub (i < 8) as packed bf16, so that a row's
+// block maximum needs two shuffles inside four lanes, a column's block maximum two shuffles across the four subs, both on
+// packed pairs, and loads, row results and column results are all whole 32-byte sectors.  The elements never pass through
+// shared memory and the warps do not wait for one another (an earlier version staged the tile in shared memory and
+// alternated load / barrier / two compute phases at 0.56 of copy bandwidth); only the 2 x 512 bytes of scales are gathered
+// there, because the operand layout interleaves the bytes of 4 row blocks and 32 rows.
+//
 // MODE selects where a block of 32 takes its scale exponent from:
 //   SCALE_BLOCK32 its own maximum (MXFP8);
 //   SCALE_FIXED   `fixed_e` for every block (one power-of-two scale for the tensor, or for this 128 x 128 tile);
 //   SCALE_VEC128  `e_rowv[r]` for the blocks of tile row r (row direction) and `e_colv[c]` for those of tile column c
 //                 (column direction): one scale per 1 x 128 / 128 x 1 vector, written into its four 32-blocks.
 enum { SCALE_BLOCK32 = 0, SCALE_FIXED = 1, SCALE_VEC128 = 2 };
-template <int MODE = SCALE_BLOCK32, bool FP4 = false>
-__device__ __forceinline__ void quantize_staged_tile(const __nv_bfloat16* tile, int R, int C,
-                                                     int row0, int col0, uint8_t* __restrict__ q_row,
-                                                     uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col,
-                                                     uint8_t* __restrict__ sf_col, int fixed_e = 0,
-                                                     const uint8_t* e_rowv = nullptr, const uint8_t* e_colv = nullptr) {
-  const int tid = threadIdx.x;
+constexpr int QT = 128;                 // threads of a quantising CTA
+
+struct TileScales {
+  uint4 row[32], col[32];               // the tile's two 512-byte scale blocks
+};
+
+__device__ __forceinline__ __nv_bfloat162 as_bf2(uint32_t w) { return *reinterpret_cast<__nv_bfloat162*>(&w); }
+__device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
+__device__ __forceinline__ uint32_t max_pair(uint32_t a, uint32_t b) { return as_u32(__hmax2(as_bf2(a), as_bf2(b))); }
+__device__ __forceinline__ uint32_t abs_pair(uint32_t a) { return a & 0x7fff7fffu; }
+__device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
+__device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
+
+// Quantises part `h` of this warp's strip -- 8 CG columns, held in d[CG] -- into q_row / q_col (either may be null).  CG = 8:
+// the layout above (two halves); CG = 4: quarters, lane (cg = lane & 3, sub = lane >> 2) holds rows 8 i + sub (i < 4), half
+// the registers for one more shuffle per column pair.  p: offset of the lane's first element in the [R, C] tensor.
+template <int MODE = SCALE_BLOCK32, bool FP4 = false, int CG = 8>
+__device__ __forceinline__ void quantize_half(const uint4 (&d)[CG], int h, long p, int C, uint8_t* __restrict__ q_row,
+                                              uint8_t* __restrict__ q_col, TileScales* scales, int fixed_e = 0,
+                                              const uint8_t* e_rowv = nullptr, const uint8_t* e_colv = nullptr) {
+  constexpr int SUBS = 32 / CG;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int cg = lane % CG, sub = lane / CG;
   if (q_row) {
-    // thread -> (row r, two 32-element blocks): 64 contiguous bytes of the row
-    const int r = tid & 127, half = tid >> 7;
+    uint32_t m[CG / 2];                 // block maxima of the lane's rows 2 j, 2 j + 1
+    if (MODE == SCALE_BLOCK32) {
 #pragma unroll
-    for (int jj = 0; jj < 2; ++jj) {
-      const int j = half * 2 + jj;
-      float f[32];
+      for (int j = 0; j < CG / 2; ++j) {
+        uint32_t a[2];
 #pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        const uint4 d = *reinterpret_cast<const uint4*>(&tile[r * PITCH + j * 32 + v * 8]);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&d);
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          const float2 t = __bfloat1622float2(h[u]);
-          f[v * 8 + 2 * u] = t.x;
-          f[v * 8 + 2 * u + 1] = t.y;
+        for (int u = 0; u < 2; ++u) {
+          const uint4& v = d[2 * j + u];
+          a[u] = max_pair(max_pair(abs_pair(v.x), abs_pair(v.y)), max_pair(abs_pair(v.z), abs_pair(v.w)));
         }
+        m[j] = max_pair(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632));
+        m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 1));
+        m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 2));
       }
-      float amax = 0.f;
+    }
 #pragma unroll
-      for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(f[i]));
-      const int e = MODE == SCALE_FIXED ? fixed_e : (MODE == SCALE_VEC128 ? (int)e_rowv[r] : e8m0_sel<FP4>(amax));
+    for (int i = 0; i < CG; ++i) {
+      const int r = SUBS * i + sub;
+      const int e = MODE == SCALE_FIXED ? fixed_e
+                    : MODE == SCALE_VEC128 ? (int)e_rowv[warp * 32 + r]
+                                           : e8m0_sel<FP4>((i & 1) ? hi_f(m[i >> 1]) : lo_f(m[i >> 1]));
       const float inv = inv_scale_from_e8m0(e);
-      uint32_t w[8];
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-        w[i] = (uint32_t)cvt2_sel<FP4>(f[4 * i] * inv, f[4 * i + 1] * inv) |
-               ((uint32_t)cvt2_sel<FP4>(f[4 * i + 2] * inv, f[4 * i + 3] * inv) << 16);
-      uint4* dst = reinterpret_cast<uint4*>(q_row + (long)(row0 + r) * C + col0 + j * 32);
-      dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
-      dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
-      sf_row[sf_offset(row0 + r, (col0 >> 5) + j, C >> 7)] = (uint8_t)e;
+      const uint32_t w0 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].x) * inv, hi_f(d[i].x) * inv) |
+                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].y) * inv, hi_f(d[i].y) * inv) << 16);
+      const uint32_t w1 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].z) * inv, hi_f(d[i].z) * inv) |
+                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].w) * inv, hi_f(d[i].w) * inv) << 16);
+      *reinterpret_cast<uint2*>(q_row + p + (long)(SUBS * i) * C) = make_uint2(w0, w1);
+      if ((cg & 3) == 0) reinterpret_cast<uint8_t*>(scales->row)[r * 16 + warp * 4 + h * (CG / 4) + (cg >> 2)] = (uint8_t)e;
     }
   }
   if (q_col) {
-    // warp -> (64-column half, 32-row block); lane -> (8-column group cg, row subset sub): rows 4*sub + j and
-    // 16 + 4*sub + j (j < 4), so that the two subsets sharing a shared-memory wavefront sit 64 bytes apart in the
-    // banks.  One 16-byte load and one 8-byte store per row; the column maxima are reduced across the four subsets
-    // with two shuffles on packed bf16 pairs.
-    const int lane = tid & 31, warp = tid >> 5;
-    const int cg = lane & 7, sub = lane >> 3;
-    const int cbase = (warp & 1) * 64 + cg * 8;
-    const int ib = warp >> 1;
-    uint4 d[8];
-    __nv_bfloat162 m[4];
+    uint32_t m[4] = {0, 0, 0, 0};       // maxima of column pairs 2 u, 2 u + 1
+    if (MODE == SCALE_BLOCK32) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) m[u] = __floats2bfloat162_rn(0.f, 0.f);
+      for (int i = 0; i < CG; ++i) {
+        m[0] = max_pair(m[0], abs_pair(d[i].x));
+        m[1] = max_pair(m[1], abs_pair(d[i].y));
+        m[2] = max_pair(m[2], abs_pair(d[i].z));
+        m[3] = max_pair(m[3], abs_pair(d[i].w));
+      }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = ib * 32 + (i >> 2) * 16 + sub * 4 + (i & 3);
-      d[i] = *reinterpret_cast<const uint4*>(&tile[r * PITCH + cbase]);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&d[i]);
+      for (int u = 0; u < 4; ++u) {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) m[u] = __hmax2(m[u], __habs2(h[u]));
+        for (int o = CG; o < 32; o <<= 1) m[u] = max_pair(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+      }
     }
+    const int c0 = h * 8 * CG + cg * 8; // first of the lane's columns in the tile
     float inv[8];
-    int e[8];
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-      uint32_t w = *reinterpret_cast<uint32_t*>(&m[u]);
-      uint32_t o = __shfl_xor_sync(0xffffffffu, w, 8);
-      m[u] = __hmax2(m[u], *reinterpret_cast<__nv_bfloat162*>(&o));
-      w = *reinterpret_cast<uint32_t*>(&m[u]);
-      o = __shfl_xor_sync(0xffffffffu, w, 16);
-      m[u] = __hmax2(m[u], *reinterpret_cast<__nv_bfloat162*>(&o));
-      const float2 a = __bfloat1622float2(m[u]);
-      e[2 * u] = MODE == SCALE_FIXED ? fixed_e : (MODE == SCALE_VEC128 ? (int)e_colv[cbase + 2 * u] : e8m0_sel<FP4>(a.x));
-      e[2 * u + 1] =
-          MODE == SCALE_FIXED ? fixed_e : (MODE == SCALE_VEC128 ? (int)e_colv[cbase + 2 * u + 1] : e8m0_sel<FP4>(a.y));
-      inv[2 * u] = inv_scale_from_e8m0(e[2 * u]);
-      inv[2 * u + 1] = inv_scale_from_e8m0(e[2 * u + 1]);
+      const int e0 = MODE == SCALE_FIXED ? fixed_e : MODE == SCALE_VEC128 ? (int)e_colv[c0 + 2 * u] : e8m0_sel<FP4>(lo_f(m[u]));
+      const int e1 = MODE == SCALE_FIXED ? fixed_e : MODE == SCALE_VEC128 ? (int)e_colv[c0 + 2 * u + 1] : e8m0_sel<FP4>(hi_f(m[u]));
+      inv[2 * u] = inv_scale_from_e8m0(e0);
+      inv[2 * u + 1] = inv_scale_from_e8m0(e1);
+      if (sub == u) {                   // every sub holds the 8 exponents; sub u writes those of its two columns
+        const int c = c0 + 2 * u;
+        uint8_t* sf = reinterpret_cast<uint8_t*>(scales->col) + (c & 31) * 16 + (c >> 5) * 4 + warp;
+        sf[0] = (uint8_t)e0;
+        sf[16] = (uint8_t)e1;
+      }
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int r = ib * 32 + (i >> 2) * 16 + sub * 4 + (i & 3);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&d[i]);
-      uint32_t w[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const float2 t0 = __bfloat1622float2(h[2 * u]), t1 = __bfloat1622float2(h[2 * u + 1]);
-        w[u] = (uint32_t)cvt2_sel<FP4>(t0.x * inv[4 * u], t0.y * inv[4 * u + 1]) |
-               ((uint32_t)cvt2_sel<FP4>(t1.x * inv[4 * u + 2], t1.y * inv[4 * u + 3]) << 16);
-      }
-      *reinterpret_cast<uint2*>(q_col + (long)(row0 + r) * C + col0 + cbase) = make_uint2(w[0], w[1]);
-    }
-    // every lane of a column group holds the 8 scales; subset s writes those of columns 2s and 2s + 1
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      if (sub == u) {
-        sf_col[sf_offset(col0 + cbase + 2 * u, (row0 >> 5) + ib, R >> 7)] = (uint8_t)e[2 * u];
-        sf_col[sf_offset(col0 + cbase + 2 * u + 1, (row0 >> 5) + ib, R >> 7)] = (uint8_t)e[2 * u + 1];
-      }
+    for (int i = 0; i < CG; ++i) {
+      const uint32_t w0 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].x) * inv[0], hi_f(d[i].x) * inv[1]) |
+                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].y) * inv[2], hi_f(d[i].y) * inv[3]) << 16);
+      const uint32_t w1 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].z) * inv[4], hi_f(d[i].z) * inv[5]) |
+                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].w) * inv[6], hi_f(d[i].w) * inv[7]) << 16);
+      *reinterpret_cast<uint2*>(q_col + p + (long)(SUBS * i) * C) = make_uint2(w0, w1);
     }
   }
 }
 
+// Writes the gathered scale blocks of the tile at (row0, col0) of an [R, C] tensor (all threads of the CTA).
+__device__ __forceinline__ void store_scales(const TileScales* scales, int R, int C, int row0, int col0,
+                                             uint8_t* __restrict__ sf_row, uint8_t* __restrict__ sf_col) {
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t < 32) {
+    if (sf_row) reinterpret_cast<uint4*>(sf_row + ((long)(row0 >> 7) * (C >> 7) + (col0 >> 7)) * 512)[t] = scales->row[t];
+  } else if (t < 64) {
+    if (sf_col) reinterpret_cast<uint4*>(sf_col + ((long)(col0 >> 7) * (R >> 7) + (row0 >> 7)) * 512)[t - 32] = scales->col[t - 32];
+  }
+}
+
+// element offset of a lane: row `sub` of its warp's strip, first of its 8 columns of part 0
+template <int CG = 8>
+__device__ __forceinline__ long lane_offset(int row0, int col0, long ld) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  return (long)(row0 + warp * 32 + lane / CG) * ld + col0 + (lane % CG) * 8;
+}
+
+__device__ __forceinline__ void load_tile(const __nv_bfloat16* __restrict__ x, long p, int C, uint4 (&d)[2][8]) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) d[h][i] = *reinterpret_cast<const uint4*>(x + p + h * 64 + (long)(4 * i) * C);
+}
+
 template <bool FP4>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(QT, 5)
 quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_t* __restrict__ q_row,
                    uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  extern __shared__ __align__(16) uint8_t smem_q[];
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_q);
+  __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const int tid = threadIdx.x;
-  // load 128 x 128 bf16 (16 vectors of 16 B per row)
+  const long p = lane_offset(row0, col0, C);
+  uint4 d[2][8];
+  load_tile(x, p, C, d);
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int v = tid + it * 256;
-    const int r = v >> 4, c8 = (v & 15) * 8;
-    const uint4 d = *reinterpret_cast<const uint4*>(x + (long)(row0 + r) * C + col0 + c8);
-    *reinterpret_cast<uint4*>(&tile[r * PITCH + c8]) = d;
-  }
-  __syncthreads();
-  quantize_staged_tile<SCALE_BLOCK32, FP4>(tile, R, C, row0, col0, q_row, sf_row, q_col, sf_col);
+  for (int h = 0; h < 2; ++h) quantize_half<SCALE_BLOCK32, FP4>(d[h], h, p + h * 64, C, q_row, q_col, &scales);
+  store_scales(&scales, R, C, row0, col0, sf_row, sf_col);
 }
 
 // Tensor-wise FP8 ("current scaling" with a power-of-two scale): one scale 2^e for the whole tensor,
@@ -216,28 +231,23 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_t* _
 // the MXFP8 layout with that exponent in every block, so the block-scaled GEMM consumes it unchanged.  The behaviour
 // of the reference's tensor-wise quantiser (primus_turbo_cpp_extension::quantize_fp8_tensorwise, called from
 // primus/backends/megatron/core/extensions/primus_turbo_float8_local.py:66-70).
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(QT, 5)
 quant_tensorwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, const float* __restrict__ tensor_amax,
                         const float* __restrict__ fallback_amax, uint8_t* __restrict__ q_row,
                         uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  extern __shared__ __align__(16) uint8_t smem_q[];
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_q);
+  __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const int tid = threadIdx.x;
-#pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int v = tid + it * 256;
-    const int r = v >> 4, c8 = (v & 15) * 8;
-    const uint4 d = *reinterpret_cast<const uint4*>(x + (long)(row0 + r) * C + col0 + c8);
-    *reinterpret_cast<uint4*>(&tile[r * PITCH + c8]) = d;
-  }
+  const long p = lane_offset(row0, col0, C);
+  uint4 d[2][8];
+  load_tile(x, p, C, d);
   // delayed scaling passes the maximum its history predicts as `tensor_amax` and this step's measured maximum as
   // `fallback_amax`, which is used while the history is still empty (0)
   float a = *tensor_amax;
   if (a == 0.f && fallback_amax != nullptr) a = *fallback_amax;
   const int fixed_e = e8m0_from_amax(a);
-  __syncthreads();
-  quantize_staged_tile<SCALE_FIXED>(tile, R, C, row0, col0, q_row, sf_row, q_col, sf_col, fixed_e);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, fixed_e);
+  store_scales(&scales, R, C, row0, col0, sf_row, sf_col);
 }
 
 // Block-wise FP8 (blocks of 128): activations and gradients take one power-of-two scale per 1 x 128 vector along the
@@ -247,55 +257,83 @@ quant_tensorwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, const
 // "blockwise" recipe (primus/backends/megatron/core/extensions/primus_turbo.py: Float8QuantConfig with
 // ScalingGranularity.BLOCKWISE, block_size 128), with scales restricted to powers of two.
 template <bool TILEWISE>
-__global__ void __launch_bounds__(256, 4)
+__global__ void __launch_bounds__(QT, 4)
 quant_blockwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_t* __restrict__ q_row,
                        uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  extern __shared__ __align__(16) uint8_t smem_q[];
+  __shared__ TileScales scales;
   __shared__ uint8_t e_rowv[TILE], e_colv[TILE];
-  __shared__ float warp_max[4];
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_q);
+  __shared__ uint32_t col_max[4][TILE / 2];      // per warp strip: maxima of column pairs
+  __shared__ uint32_t strip_max[4];
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const int tid = threadIdx.x;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, cg = lane & 7, sub = lane >> 3;
+  const long p = lane_offset(row0, col0, C);
+  uint4 d[2][8];
+  load_tile(x, p, C, d);
+  uint32_t rm[4];                                // rows (8 j + sub, 8 j + 4 + sub): maximum over the tile's 128 columns
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int v = tid + it * 256;
-    const int r = v >> 4, c8 = (v & 15) * 8;
-    const uint4 d = *reinterpret_cast<const uint4*>(x + (long)(row0 + r) * C + col0 + c8);
-    *reinterpret_cast<uint4*>(&tile[r * PITCH + c8]) = d;
-  }
-  __syncthreads();
-  // threads 0..127: maximum of tile row tid; threads 128..255: maximum of tile column tid - 128
-  float m = 0.f;
-  if (tid < TILE) {
-    __nv_bfloat162 mm = __floats2bfloat162_rn(0.f, 0.f);
+  for (int j = 0; j < 4; ++j) {
+    uint32_t a[2];
 #pragma unroll
-    for (int v = 0; v < 16; ++v) {
-      const uint4 d = *reinterpret_cast<const uint4*>(&tile[tid * PITCH + v * 8]);
-      const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&d);
+    for (int u = 0; u < 2; ++u) {
+      a[u] = 0;
 #pragma unroll
-      for (int u = 0; u < 4; ++u) mm = __hmax2(mm, __habs2(h[u]));
+      for (int h = 0; h < 2; ++h) {
+        const uint4& v = d[h][2 * j + u];
+        a[u] = max_pair(a[u], max_pair(max_pair(abs_pair(v.x), abs_pair(v.y)), max_pair(abs_pair(v.z), abs_pair(v.w))));
+      }
     }
-    const float2 f = __bfloat1622float2(mm);
-    m = fmaxf(f.x, f.y);
-  } else if (!TILEWISE) {
-    const int c = tid - TILE;
-#pragma unroll 8
-    for (int r = 0; r < TILE; ++r) m = fmaxf(m, fabsf(__bfloat162float(tile[r * PITCH + c])));
+    rm[j] = max_pair(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) rm[j] = max_pair(rm[j], __shfl_xor_sync(0xffffffffu, rm[j], o));
   }
   if (TILEWISE) {
-    float v = m;
+    uint32_t m = max_pair(max_pair(rm[0], rm[1]), max_pair(rm[2], rm[3]));
+    m = max_pair(m, __shfl_xor_sync(0xffffffffu, m, 8));
+    m = max_pair(m, __shfl_xor_sync(0xffffffffu, m, 16));
+    if (lane == 0) strip_max[warp] = m;
+    __syncthreads();
+    m = max_pair(max_pair(strip_max[0], strip_max[1]), max_pair(strip_max[2], strip_max[3]));
+    const int fixed_e = e8m0_from_amax(fmaxf(lo_f(m), hi_f(m)));
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (tid < TILE && (tid & 31) == 0) warp_max[tid >> 5] = v;
-    __syncthreads();
-    const int fixed_e = e8m0_from_amax(fmaxf(fmaxf(warp_max[0], warp_max[1]), fmaxf(warp_max[2], warp_max[3])));
-    quantize_staged_tile<SCALE_FIXED>(tile, R, C, row0, col0, q_row, sf_row, q_col, sf_col, fixed_e);
+    for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, fixed_e);
   } else {
-    if (tid < TILE) e_rowv[tid] = (uint8_t)e8m0_from_amax(m);
-    else e_colv[tid - TILE] = (uint8_t)e8m0_from_amax(m);
+    if (cg == 0) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        e_rowv[warp * 32 + 8 * j + sub] = (uint8_t)e8m0_from_amax(lo_f(rm[j]));
+        e_rowv[warp * 32 + 8 * j + 4 + sub] = (uint8_t)e8m0_from_amax(hi_f(rm[j]));
+      }
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      uint32_t m[4] = {0, 0, 0, 0};
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        m[0] = max_pair(m[0], abs_pair(d[h][i].x));
+        m[1] = max_pair(m[1], abs_pair(d[h][i].y));
+        m[2] = max_pair(m[2], abs_pair(d[h][i].z));
+        m[3] = max_pair(m[3], abs_pair(d[h][i].w));
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        m[u] = max_pair(m[u], __shfl_xor_sync(0xffffffffu, m[u], 8));
+        m[u] = max_pair(m[u], __shfl_xor_sync(0xffffffffu, m[u], 16));
+        if (sub == u) col_max[warp][h * 32 + cg * 4 + u] = m[u];
+      }
+    }
     __syncthreads();
-    quantize_staged_tile<SCALE_VEC128>(tile, R, C, row0, col0, q_row, sf_row, q_col, sf_col, 0, e_rowv, e_colv);
+    if (threadIdx.x < TILE / 2) {
+      const int t = threadIdx.x;
+      const uint32_t m = max_pair(max_pair(col_max[0][t], col_max[1][t]), max_pair(col_max[2][t], col_max[3][t]));
+      e_colv[2 * t] = (uint8_t)e8m0_from_amax(lo_f(m));
+      e_colv[2 * t + 1] = (uint8_t)e8m0_from_amax(hi_f(m));
+    }
+    __syncthreads();
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      quantize_half<SCALE_VEC128>(d[h], h, p + h * 64, C, q_row, q_col, &scales, 0, e_rowv, e_colv);
   }
+  store_scales(&scales, R, C, row0, col0, sf_row, sf_col);
 }
 
 // max |x| over n bf16 values (n a multiple of 8) into *out, which the caller zeroes first (non-negative floats order
@@ -323,15 +361,9 @@ amax_bf16_kernel(const __nv_bfloat16* __restrict__ x, long n8, float* __restrict
   }
 }
 
-__device__ __forceinline__ void bf8_load(const __nv_bfloat16* p, float* f) {
-  const uint4 d = *reinterpret_cast<const uint4*>(p);
-  const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&d);
-#pragma unroll
-  for (int u = 0; u < 4; ++u) {
-    const float2 t = __bfloat1622float2(h[u]);
-    f[2 * u] = t.x;
-    f[2 * u + 1] = t.y;
-  }
+__device__ __forceinline__ void bf8_unpack(const uint4& d, float* f) {
+  f[0] = lo_f(d.x); f[1] = hi_f(d.x); f[2] = lo_f(d.y); f[3] = hi_f(d.y);
+  f[4] = lo_f(d.z); f[5] = hi_f(d.z); f[6] = lo_f(d.w); f[7] = hi_f(d.w);
 }
 __device__ __forceinline__ uint4 bf8_pack(const float* f) {
   uint4 o;
@@ -344,81 +376,101 @@ __device__ __forceinline__ uint4 bf8_pack(const float* f) {
 
 // SwiGLU forward fused with the quantisation of its output: h1 [T, 2I] = [gate | up] -> MXFP8 of
 // act[T, I] = silu(gate) * up (rounded to bf16 first, so the values equal quantising the un-fused kernel's output).
-__global__ void __launch_bounds__(256, 4)
+// Four rows' loads in flight per lane and round keep it at 80 registers: six CTAs (24 warps) per SM hide the two special-
+// function operations per element, which four CTAs did not (132 us at 8192 x 14336).
+__global__ void __launch_bounds__(QT, 6)
 swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, float clamp, uint8_t* __restrict__ q_row,
                           uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  extern __shared__ __align__(16) uint8_t smem_q[];
-  __nv_bfloat16* tile = reinterpret_cast<__nv_bfloat16*>(smem_q);
+  __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const int tid = threadIdx.x;
+  const long pin = lane_offset(row0, col0, 2L * I), p = lane_offset(row0, col0, I);
+#pragma unroll 1
+  for (int h = 0; h < 2; ++h) {
+    uint4 d[8];
 #pragma unroll
-  for (int it = 0; it < 8; ++it) {
-    const int v = tid + it * 256;
-    const int r = v >> 4, c8 = (v & 15) * 8;
-    const __nv_bfloat16* g = h1 + (long)(row0 + r) * 2 * I + col0 + c8;
-    float fg[8], fu[8], o[8];
-    bf8_load(g, fg);
-    bf8_load(g + I, fu);
+    for (int i0 = 0; i0 < 8; i0 += 4) {
+      uint4 up[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float gg = fg[j], uu = fu[j];
-      if (clamp > 0.f) {
-        gg = fminf(gg, clamp);
-        uu = fminf(fmaxf(uu, -clamp), clamp);
+      for (int i = 0; i < 4; ++i) {
+        const __nv_bfloat16* g = h1 + pin + h * 64 + (long)(4 * (i0 + i)) * 2 * I;
+        d[i0 + i] = *reinterpret_cast<const uint4*>(g);
+        up[i] = *reinterpret_cast<const uint4*>(g + I);
       }
-      const float sig = pb::fast_sigmoid(gg);
-      o[j] = gg * sig * uu * 1.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float fg[8], fu[8], o[8];
+        bf8_unpack(d[i0 + i], fg);
+        bf8_unpack(up[i], fu);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          float gg = fg[j], uu = fu[j];
+          if (clamp > 0.f) {
+            gg = fminf(gg, clamp);
+            uu = fminf(fmaxf(uu, -clamp), clamp);
+          }
+          const float sig = pb::fast_sigmoid(gg);
+          o[j] = gg * sig * uu * 1.f;
+        }
+        d[i0 + i] = bf8_pack(o);
+      }
     }
-    *reinterpret_cast<uint4*>(&tile[r * PITCH + c8]) = bf8_pack(o);
+    quantize_half(d, h, p + h * 64, I, q_row, q_col, &scales);
   }
-  __syncthreads();
-  quantize_staged_tile(tile, T, I, row0, col0, q_row, sf_row, q_col, sf_col);
+  store_scales(&scales, T, I, row0, col0, sf_row, sf_col);
 }
 
 // SwiGLU backward fused with the quantisation of its output: (h1 [T, 2I], dact [T, I]) -> MXFP8 (both directions) of
 // dh1 [T, 2I] = [dgate | dup].  One CTA per 128 x 128 tile of the activation: it reads gate, up and dact once, stages
 // the dgate and the dup tile, and quantises one after the other.
-constexpr int QUANT_SMEM_BWD = 2 * TILE * PITCH * 2;
-__global__ void __launch_bounds__(256, 3)
+// A warp computes the dgate and the dup values of its strip by 32 x 32 quarters: the twelve loads of a quarter are in
+// flight per lane, and two results of 16 registers instead of 32 let five CTAs share an SM instead of three.
+__global__ void __launch_bounds__(QT, 5)
 swiglu_bwd_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, const __nv_bfloat16* __restrict__ dact, int T, int I,
                               float clamp, uint8_t* __restrict__ q_row, uint8_t* __restrict__ sf_row,
                               uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  extern __shared__ __align__(16) uint8_t smem_q[];
-  __nv_bfloat16* tile_g = reinterpret_cast<__nv_bfloat16*>(smem_q);
-  __nv_bfloat16* tile_u = tile_g + TILE * PITCH;
+  __shared__ TileScales scales[2];               // of the dgate and of the dup tile
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const int tid = threadIdx.x;
-#pragma unroll 2
-  for (int it = 0; it < 8; ++it) {
-    const int v = tid + it * 256;
-    const int r = v >> 4, c8 = (v & 15) * 8;
-    const __nv_bfloat16* g = h1 + (long)(row0 + r) * 2 * I + col0 + c8;
-    float fg[8], fu[8], fd[8], og[8], ou[8];
-    bf8_load(g, fg);
-    bf8_load(g + I, fu);
-    bf8_load(dact + (long)(row0 + r) * I + col0 + c8, fd);
+  const long pin = lane_offset<4>(row0, col0, 2L * I), pd = lane_offset<4>(row0, col0, I);
+#pragma unroll 1
+  for (int h = 0; h < 4; ++h) {
+    uint4 dg[4], du[4], da[4];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float gg = fg[j], uu = fu[j];
-      float gmask = 1.f, umask = 1.f;
-      if (clamp > 0.f) {
-        if (gg > clamp) { gg = clamp; gmask = 0.f; }
-        if (uu > clamp) { uu = clamp; umask = 0.f; }
-        if (uu < -clamp) { uu = -clamp; umask = 0.f; }
-      }
-      const float sig = pb::fast_sigmoid(gg);
-      const float sl = gg * sig;
-      const float d = fd[j] * 1.f;
-      const float dsl = sig * (1.f + gg * (1.f - sig));
-      og[j] = d * uu * dsl * gmask;
-      ou[j] = d * sl * umask;
+    for (int i = 0; i < 4; ++i) {
+      const __nv_bfloat16* g = h1 + pin + h * 32 + (long)(8 * i) * 2 * I;
+      dg[i] = *reinterpret_cast<const uint4*>(g);
+      du[i] = *reinterpret_cast<const uint4*>(g + I);
+      da[i] = *reinterpret_cast<const uint4*>(dact + pd + h * 32 + (long)(8 * i) * I);
     }
-    *reinterpret_cast<uint4*>(&tile_g[r * PITCH + c8]) = bf8_pack(og);
-    *reinterpret_cast<uint4*>(&tile_u[r * PITCH + c8]) = bf8_pack(ou);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      float fg[8], fu[8], fd[8], og[8], ou[8];
+      bf8_unpack(dg[i], fg);
+      bf8_unpack(du[i], fu);
+      bf8_unpack(da[i], fd);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float gg = fg[j], uu = fu[j];
+        float gmask = 1.f, umask = 1.f;
+        if (clamp > 0.f) {
+          if (gg > clamp) { gg = clamp; gmask = 0.f; }
+          if (uu > clamp) { uu = clamp; umask = 0.f; }
+          if (uu < -clamp) { uu = -clamp; umask = 0.f; }
+        }
+        const float sig = pb::fast_sigmoid(gg);
+        const float sl = gg * sig;
+        const float d = fd[j] * 1.f;
+        const float dsl = sig * (1.f + gg * (1.f - sig));
+        og[j] = d * uu * dsl * gmask;
+        ou[j] = d * sl * umask;
+      }
+      dg[i] = bf8_pack(og);
+      du[i] = bf8_pack(ou);
+    }
+    quantize_half<SCALE_BLOCK32, false, 4>(dg, h, pin + h * 32, 2 * I, q_row, q_col, &scales[0]);
+    quantize_half<SCALE_BLOCK32, false, 4>(du, h, pin + I + h * 32, 2 * I, q_row, q_col, &scales[1]);
   }
-  __syncthreads();
-  quantize_staged_tile(tile_g, T, 2 * I, row0, col0, q_row, sf_row, q_col, sf_col);
-  quantize_staged_tile(tile_u, T, 2 * I, row0, I + col0, q_row, sf_row, q_col, sf_col);
+  store_scales(&scales[0], T, 2 * I, row0, col0, sf_row, sf_col);
+  store_scales(&scales[1], T, 2 * I, row0, I + col0, sf_row, sf_col);
 }
 
 // value [R, C] fp8 + scales (operand layout with MN = R or C) -> fp32 [R, C]; test / debugging helper
@@ -442,14 +494,7 @@ extern "C" {
 int pb_quant_mxfp8(const void* x, int R, int C, void* q_row, void* sf_row, void* q_col, void* sf_col, cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
   dim3 grid(C / TILE, R / TILE);
-  constexpr int SMEM = QUANT_SMEM;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(quant_mxfp8_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  quant_mxfp8_kernel<false><<<grid, 256, SMEM, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), R, C,
+  quant_mxfp8_kernel<false><<<grid, QT, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), R, C,
                                                 reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row),
                                                 reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -460,13 +505,7 @@ int pb_quant_mxfp8(const void* x, int R, int C, void* q_row, void* sf_row, void*
 int pb_quant_mxfp4_as_fp8(const void* x, int R, int C, void* q_row, void* sf_row, void* q_col, void* sf_col,
                           cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(quant_mxfp8_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  quant_mxfp8_kernel<true><<<dim3(C / TILE, R / TILE), 256, QUANT_SMEM, s>>>(
+  quant_mxfp8_kernel<true><<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), R, C, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -476,18 +515,12 @@ int pb_quant_mxfp4_as_fp8(const void* x, int R, int C, void* q_row, void* sf_row
 int pb_quant_fp8_tensorwise(const void* x, int R, int C, float* amax, void* q_row, void* sf_row, void* q_col, void* sf_col,
                             cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(quant_tensorwise_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
   cudaError_t e = cudaMemsetAsync(amax, 0, sizeof(float), s);
   if (e != cudaSuccess) return (int)e;
   const long n8 = (long)R * C / 8;
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax);
-  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), 256, QUANT_SMEM, s>>>(
+  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), R, C, amax, nullptr, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -500,16 +533,10 @@ int pb_quant_fp8_tensorwise(const void* x, int R, int C, float* amax, void* q_ro
 int pb_quant_fp8_delayed(const void* x, int R, int C, float* amax_now, const float* scale_amax, void* q_row,
                          void* sf_row, void* q_col, void* sf_col, cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(quant_tensorwise_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
   const long n8 = (long)R * C / 8;
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax_now);
-  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), 256, QUANT_SMEM, s>>>(
+  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(x), R, C, scale_amax, amax_now, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -520,40 +547,20 @@ int pb_quant_fp8_delayed(const void* x, int R, int C, float* amax_now, const flo
 int pb_quant_fp8_blockwise(const void* x, int R, int C, int tilewise, void* q_row, void* sf_row, void* q_col,
                            void* sf_col, cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(quant_blockwise_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         QUANT_SMEM);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(quant_blockwise_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANT_SMEM);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
   const dim3 grid(C / TILE, R / TILE);
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   uint8_t *qr = reinterpret_cast<uint8_t*>(q_row), *sr = reinterpret_cast<uint8_t*>(sf_row);
   uint8_t *qc = reinterpret_cast<uint8_t*>(q_col), *sc = reinterpret_cast<uint8_t*>(sf_col);
-  if (tilewise) quant_blockwise_kernel<true><<<grid, 256, QUANT_SMEM, s>>>(xp, R, C, qr, sr, qc, sc);
-  else quant_blockwise_kernel<false><<<grid, 256, QUANT_SMEM, s>>>(xp, R, C, qr, sr, qc, sc);
+  if (tilewise) quant_blockwise_kernel<true><<<grid, QT, 0, s>>>(xp, R, C, qr, sr, qc, sc);
+  else quant_blockwise_kernel<false><<<grid, QT, 0, s>>>(xp, R, C, qr, sr, qc, sc);
   return (int)cudaGetLastError();
-}
-
-static int set_quant_smem(const void* kern) {
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, QUANT_SMEM);
-  return (int)e;
 }
 
 // act = silu(gate) * up of h1 [T, 2I] (T, I multiples of 128) quantised to MXFP8; either output pair may be null.
 int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row, void* sf_row, void* q_col,
                           void* sf_col, cudaStream_t s) {
   if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    int rc = set_quant_smem(reinterpret_cast<const void*>(swiglu_quant_mxfp8_kernel));
-    if (rc) return rc;
-    attr_set = true;
-  }
-  swiglu_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), 256, QUANT_SMEM, s>>>(
+  swiglu_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -563,14 +570,7 @@ int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row
 int pb_swiglu_bwd_quant_mxfp8(const void* h1, const void* dact, int T, int I, float clamp, void* q_row, void* sf_row,
                               void* q_col, void* sf_col, cudaStream_t s) {
   if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(swiglu_bwd_quant_mxfp8_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         QUANT_SMEM_BWD);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
-  swiglu_bwd_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), 256, QUANT_SMEM_BWD, s>>>(
+  swiglu_bwd_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
       reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
       reinterpret_cast<uint8_t*>(sf_col));
