@@ -52,41 +52,51 @@ __global__ void softcap_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const _
 // ------------------------------------------------------------------ RoPE (rotate-half), in place
 // x: [T, heads, d] with row pitch ld; rotates the first rot_dim channels of every head.
 // pos[t] selects the row of the cos/sin tables ([max_pos, rot_dim/2] fp32). sign=-1 for backward.
-__global__ void rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ pos,
-                            const float* __restrict__ cos_t, const float* __restrict__ sin_t, long T,
-                            int heads, int d, int rot_dim, long ld, float sign) {
+// A thread owns 8 channel pairs of ROPE_HEADS neighbouring heads of a token: their 2 x ROPE_HEADS 16-byte loads are in
+// flight together and share one read of the cos / sin entries.
+template <int ROPE_HEADS>
+__global__ void __launch_bounds__(256)
+rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ cos_t,
+            const float* __restrict__ sin_t, long T, int heads, int d, int rot_dim, long ld, float sign) {
   const int half = rot_dim / 2;
   const int vec_per_head = half / 8;
-  const long total = T * heads * vec_per_head;
-  for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
-       idx += (long)gridDim.x * blockDim.x) {
-    const int v = idx % vec_per_head;
-    const long th = idx / vec_per_head;
-    const int h = th % heads;
-    const long t = th / heads;
-    const int p = pos ? pos[t] : (int)t;
-    __nv_bfloat16* base = x + t * ld + (long)h * d + v * 8;
-    Bf8 a = *reinterpret_cast<Bf8*>(base);
-    Bf8 b = *reinterpret_cast<Bf8*>(base + half);
-    float fa[8], fb[8], c[8], s[8];
-    bf8_to_f(a, fa);
-    bf8_to_f(b, fb);
-    const float* cp = cos_t + (long)p * half + v * 8;
-    const float* sp = sin_t + (long)p * half + v * 8;
-    *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cp);
-    *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cp + 4);
-    *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sp);
-    *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sp + 4);
-    float oa[8], ob[8];
+  const int per_token = vec_per_head * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
+  const long idx = blockIdx.x * 256L + threadIdx.x;
+  const long t = idx / per_token;
+  if (t >= T) return;
+  const int r = (int)(idx - t * per_token);
+  const int v = r % vec_per_head, h0 = r / vec_per_head * ROPE_HEADS;
+  const int p = pos ? pos[t] : (int)t;
+  __nv_bfloat16* base = x + t * ld + (long)h0 * d + v * 8;
+  Bf8 a[ROPE_HEADS], b[ROPE_HEADS];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float sn = s[j] * sign;
-      oa[j] = fa[j] * c[j] - fb[j] * sn;
-      ob[j] = fb[j] * c[j] + fa[j] * sn;
+  for (int i = 0; i < ROPE_HEADS; ++i)
+    if (h0 + i < heads) {
+      a[i] = *reinterpret_cast<Bf8*>(base + (long)i * d);
+      b[i] = *reinterpret_cast<Bf8*>(base + (long)i * d + half);
     }
-    *reinterpret_cast<Bf8*>(base) = f_to_bf8(oa);
-    *reinterpret_cast<Bf8*>(base + half) = f_to_bf8(ob);
-  }
+  float c[8], s[8];
+  const float* cp = cos_t + (long)p * half + v * 8;
+  const float* sp = sin_t + (long)p * half + v * 8;
+  *reinterpret_cast<float4*>(c) = *reinterpret_cast<const float4*>(cp);
+  *reinterpret_cast<float4*>(c + 4) = *reinterpret_cast<const float4*>(cp + 4);
+  *reinterpret_cast<float4*>(s) = *reinterpret_cast<const float4*>(sp);
+  *reinterpret_cast<float4*>(s + 4) = *reinterpret_cast<const float4*>(sp + 4);
+#pragma unroll
+  for (int i = 0; i < ROPE_HEADS; ++i)
+    if (h0 + i < heads) {
+      float fa[8], fb[8], oa[8], ob[8];
+      bf8_to_f(a[i], fa);
+      bf8_to_f(b[i], fb);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const float sn = s[j] * sign;
+        oa[j] = fa[j] * c[j] - fb[j] * sn;
+        ob[j] = fb[j] * c[j] + fa[j] * sn;
+      }
+      *reinterpret_cast<Bf8*>(base + (long)i * d) = f_to_bf8(oa);
+      *reinterpret_cast<Bf8*>(base + (long)i * d + half) = f_to_bf8(ob);
+    }
 }
 
 // gated-unit activations: kind 0 = SiLU (SwiGLU), 1 = tanh-approximated GELU (GEGLU)
@@ -450,10 +460,16 @@ extern "C" {
 int pb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, long T, int heads, int d,
             int rot_dim, long ld, int backward, cudaStream_t s) {
   if (rot_dim % 16 || ld % 8 || d % 8) return -2;
-  const long total = T * heads * (rot_dim / 16);
-  if (total == 0) return 0;
-  rope_kernel<<<grid_for(total, 256), 256, 0, s>>>((__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads, d,
-                                                  rot_dim, ld, backward ? -1.f : 1.f);
+  // four heads per thread where that still gives every SM 1024 threads, else one head, for the parallelism
+  const long vecs = T * (rot_dim / 16), four = vecs * ((heads + 3) / 4), one = vecs * heads;
+  if (one <= 0) return 0;
+  const float sign = backward ? -1.f : 1.f;
+  if (four >= 148 * 1024L)
+    rope_kernel<4><<<(unsigned)((four + 255) / 256), 256, 0, s>>>((__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads, d, rot_dim,
+                                                                 ld, sign);
+  else
+    rope_kernel<1><<<(unsigned)((one + 255) / 256), 256, 0, s>>>((__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads, d, rot_dim,
+                                                                ld, sign);
   PB_CHECK_LAUNCH();
 }
 

@@ -122,3 +122,18 @@ def test_qk_norm_matches_separate_norms(T, hq, hkv, d, pad):
     assert wk.grad is None
     err = (wk.main_grad.double() - 1 - k64.grad).abs().max()
     assert err <= 1e-4 * (1 + k64.grad.abs().max()), f"dwk {err}"
+
+
+@pytest.mark.parametrize("heads,d,rot,T", [(1, 64, 64, 5), (3, 128, 128, 130), (6, 64, 32, 77), (9, 192, 64, 64)])
+def test_rope_head_groups(heads, d, rot, T):
+    g = _gen(heads)
+    x = torch.randn(T, heads * d + 8, device="cuda", generator=g).bfloat16()
+    before = x.clone()
+    cos, sin = fused.rope_tables(T + 3, rot, 1e4, "cuda")
+    pos = torch.randint(0, T + 3, (T,), device="cuda", generator=g, dtype=torch.int32)
+    view = x[:, :heads * d].view(T, heads, d)
+    fused.rope_inplace_(view, cos, sin, pos, rot)
+    _close_bf16(view, fused.rope_ref(before[:, :heads * d].view(T, heads, d).double(), cos, sin, pos, rot), "rope")
+    assert torch.equal(x[:, heads * d:], before[:, heads * d:])
+    fused.rope_inplace_(view, cos, sin, pos, rot, backward=True)
+    _close_bf16(view, before[:, :heads * d].view(T, heads, d), "inverse")
