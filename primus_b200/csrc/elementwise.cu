@@ -614,9 +614,11 @@ int pb_embedding_bwd(const void* dy, const long* tokens, float* dw, long T, int 
 // primus/backends/transformer_engine/pytorch/common/triton/permutation.py:189-305.
 namespace {
 
-__global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ src,
-                                       const float* __restrict__ scale, __nv_bfloat16* __restrict__ out, long R,
-                                       int H, const int* __restrict__ limit_rows) {
+// MOE_UNROLL vectors of a row per lane are loaded before the first is stored
+constexpr int MOE_UNROLL = 8;
+__global__ void __launch_bounds__(256)
+moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ src, const float* __restrict__ scale,
+                       __nv_bfloat16* __restrict__ out, long R, int H, const int* __restrict__ limit_rows) {
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -625,48 +627,78 @@ __global__ void moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, cons
   for (long r = warp_global; r < R && r < lim; r += num_warps) {
     const int s = src[r];
     Bf8* o = reinterpret_cast<Bf8*>(out + r * H);
-    if (s < 0) {
-      Bf8 z;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) z.v[i] = __floats2bfloat162_rn(0.f, 0.f);
-      for (int v = lane; v < nv; v += 32) o[v] = z;
-      continue;
-    }
     const Bf8* in = reinterpret_cast<const Bf8*>(x + (long)s * H);
-    if (scale) {
-      const float sc = scale[r];
-      for (int v = lane; v < nv; v += 32) {
-        float f[8];
-        bf8_to_f(in[v], f);
+    const float sc = scale && s >= 0 ? scale[r] : 1.f;
+    for (int base = lane; base < nv; base += 32 * MOE_UNROLL) {
+      Bf8 t[MOE_UNROLL];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) f[j] *= sc;
-        o[v] = f_to_bf8(f);
+      for (int u = 0; u < MOE_UNROLL; ++u) {
+        const int v = base + u * 32;
+        if (s < 0) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) t[u].v[i] = __floats2bfloat162_rn(0.f, 0.f);
+        } else if (v < nv) {
+          t[u] = in[v];
+        }
       }
-    } else {
-      for (int v = lane; v < nv; v += 32) o[v] = in[v];
+#pragma unroll
+      for (int u = 0; u < MOE_UNROLL; ++u) {
+        const int v = base + u * 32;
+        if (v >= nv) break;
+        if (scale) {
+          float f[8];
+          bf8_to_f(t[u], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] *= sc;
+          t[u] = f_to_bf8(f);
+        }
+        o[v] = t[u];
+      }
     }
   }
 }
 
-__global__ void moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos,
-                                        __nv_bfloat16* __restrict__ out, long T, int topk, int H) {
+// Two vectors per lane at a time; the rows of four copies (eight loads) are in flight together, summed in copy order.
+__global__ void __launch_bounds__(256)
+moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, __nv_bfloat16* __restrict__ out,
+                        long T, int topk, int H) {
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
   const int nv = H / 8;
   for (long t = warp_global; t < T; t += num_warps) {
     Bf8* o = reinterpret_cast<Bf8*>(out + t * H);
-    for (int v = lane; v < nv; v += 32) {
-      float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      for (int k = 0; k < topk; ++k) {
-        const int p = pos[t * topk + k];
-        if (p < 0) continue;
-        float f[8];
-        bf8_to_f(reinterpret_cast<const Bf8*>(y + (long)p * H)[v], f);
+    for (int v = lane; v < nv; v += 64) {
+      const bool second = v + 32 < nv;
+      float acc[2][8] = {};
+      for (int k0 = 0; k0 < topk; k0 += 4) {
+        int p[4];
+        Bf8 a[4], b[4];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[j] += f[j];
+        for (int k = 0; k < 4; ++k) p[k] = k0 + k < topk ? pos[t * topk + k0 + k] : -1;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (p[k] < 0) continue;
+          const Bf8* row = reinterpret_cast<const Bf8*>(y + (long)p[k] * H);
+          a[k] = row[v];
+          if (second) b[k] = row[v + 32];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          if (p[k] < 0) continue;
+          float f[8];
+          bf8_to_f(a[k], f);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) acc[0][j] += f[j];
+          if (second) {
+            bf8_to_f(b[k], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[1][j] += f[j];
+          }
+        }
       }
-      o[v] = f_to_bf8(acc);
+      o[v] = f_to_bf8(acc[0]);
+      if (second) o[v + 32] = f_to_bf8(acc[1]);
     }
   }
 }
@@ -677,7 +709,7 @@ extern "C" int pb_moe_gather_rows(const void* x, const int* src, const float* sc
                                   const int* limit_rows, cudaStream_t s) {
   if (H % 8) return -2;
   if (R == 0) return 0;
-  moe_gather_rows_kernel<<<grid_for(R * 32, 256), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale,
+  moe_gather_rows_kernel<<<grid_for(R * 32, 256, 1 << 16), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale,
                                                               (__nv_bfloat16*)out, R, H, limit_rows);
   return (int)cudaGetLastError();
 }
@@ -686,7 +718,7 @@ extern "C" int pb_moe_combine_rows(const void* y, const int* pos, void* out, lon
                                    cudaStream_t s) {
   if (H % 8) return -2;
   if (T == 0) return 0;
-  moe_combine_rows_kernel<<<grid_for(T * 32, 256), 256, 0, s>>>((const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T,
+  moe_combine_rows_kernel<<<grid_for(T * 32, 256, 1 << 16), 256, 0, s>>>((const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T,
                                                                topk, H);
   return (int)cudaGetLastError();
 }

@@ -30,6 +30,7 @@ constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
 constexpr int EPI_BUF_BYTES = BM * 128;
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 2 * EPI_BUF_BYTES + 1024 + 256;
 constexpr int TMEM_COLS = 2 * BN;
+constexpr int GROUP_M = 16;
 
 enum { G_FPROP = 0, G_DGRAD = 1, G_WGRAD = 2 };
 
@@ -68,14 +69,20 @@ struct Tile {
   int k_blocks;   // number of reduction blocks
 };
 
-// MODE fprop/dgrad: tiles = max_mblocks x num_n (m fastest inside a group of 8 row blocks)
+// MODE fprop/dgrad: tiles = max_mblocks x num_n, m fastest inside groups of GROUP_M row blocks and all column blocks of a
+//                   group before the next: the CTAs in flight then share a few experts' weights and their rows, which are
+//                   read from memory once.  (Running over all row blocks of a column block first re-read the activations,
+//                   150 MB at 36k rows of 2048, from memory once per column block.)
 // MODE wgrad      : tiles = E x num_m x num_n over D[e][N_out, K_out]
 template <int MODE>
 __device__ __forceinline__ Tile get_tile(int tile, int num_m, int num_n, int K, const int* __restrict__ mblock_expert,
                                          const int* __restrict__ row_start, const int* __restrict__ padded) {
   Tile t;
   if (MODE != G_WGRAD) {
-    const int mb = tile % num_m, nb = tile / num_m;
+    const int per_group = GROUP_M * num_n;
+    const int g = tile / per_group, r = tile - g * per_group;
+    const int gm = min(GROUP_M, num_m - g * GROUP_M);
+    const int mb = g * GROUP_M + r % gm, nb = r / gm;
     const int e = mblock_expert[mb];
     t.valid = e >= 0;
     t.expert = e;
