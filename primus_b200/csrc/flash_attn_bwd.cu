@@ -452,34 +452,79 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 }
 
 // delta[b, h, s] = sum_d dO * O ;  lse2 = lse * log2(e) (so the main kernels need no per-element multiply).
-// One thread per (batch, head, position), position fastest: a thread streams its 2 * dv bf16 values with 16-byte
-// loads (many loads in flight per thread) and the per-row results are written coalesced.
-__global__ void __launch_bounds__(256)
+// A CTA takes 32 positions x 8 heads.  DV / 8 lanes share a (position, head) row, neighbouring rows of the same position
+// are neighbours in memory, so a warp reads whole 128-byte lines; the 32 sums of a head then leave as one 128-byte line.
+constexpr int DL_POS = 32, DL_HEADS = 8, DL_THREADS = 256;
+template <int DV>
+__global__ void __launch_bounds__(DL_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2, int seq, int hq,
-                  int dv, long o_row, long do_row, long total_rows) {
-  const long i = blockIdx.x * (long)blockDim.x + threadIdx.x;
-  if (i >= total_rows * hq) return;
-  const long pos = i % seq;
-  const int h = (int)((i / seq) % hq);
-  const long b = i / ((long)seq * hq);
-  const long t = b * seq + pos;
-  const uint4* op = reinterpret_cast<const uint4*>(o + t * o_row + (long)h * dv);
-  const uint4* dp = reinterpret_cast<const uint4*>(d_o + t * do_row + (long)h * dv);
-  float s = 0.f;
-#pragma unroll 4
-  for (int v = 0; v < dv / 8; ++v) {
-    const uint4 x = op[v], y = dp[v];
-    const __nv_bfloat162* xa = reinterpret_cast<const __nv_bfloat162*>(&x);
-    const __nv_bfloat162* ya = reinterpret_cast<const __nv_bfloat162*>(&y);
+                  long o_row, long do_row) {
+  constexpr int LANES = DV / 8;
+  constexpr int GROUPS = DL_THREADS / LANES;
+  constexpr int ITERS = DL_POS * DL_HEADS / GROUPS;
+  __shared__ float sums[DL_HEADS][DL_POS + 1];
+  const long t0 = (long)blockIdx.x * DL_POS;    // seq is a multiple of 128: the positions lie in one sequence
+  const int h0 = blockIdx.y * DL_HEADS;
+  const int lane = threadIdx.x % LANES, grp = threadIdx.x / LANES;
+#pragma unroll 1
+  for (int i0 = 0; i0 < ITERS; i0 += 4) {
+    uint4 x[4], y[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const float2 a = __bfloat1622float2(xa[u]), c = __bfloat1622float2(ya[u]);
-      s += a.x * c.x + a.y * c.y;
+    for (int i = 0; i < 4; ++i) {
+      const int item = (i0 + i) * GROUPS + grp, p = item / DL_HEADS, h = h0 + item % DL_HEADS;
+      x[i] = y[i] = make_uint4(0, 0, 0, 0);
+      if (h < hq) {
+        x[i] = reinterpret_cast<const uint4*>(o + (t0 + p) * o_row + (long)h * DV)[lane];
+        y[i] = reinterpret_cast<const uint4*>(d_o + (t0 + p) * do_row + (long)h * DV)[lane];
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int item = (i0 + i) * GROUPS + grp;
+      const __nv_bfloat162* xa = reinterpret_cast<const __nv_bfloat162*>(&x[i]);
+      const __nv_bfloat162* ya = reinterpret_cast<const __nv_bfloat162*>(&y[i]);
+      float s = 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const float2 a = __bfloat1622float2(xa[u]), c = __bfloat1622float2(ya[u]);
+        s += a.x * c.x + a.y * c.y;
+      }
+#pragma unroll
+      for (int k = LANES / 2; k > 0; k >>= 1) s += __shfl_xor_sync(0xffffffffu, s, k);
+      if (lane == 0) sums[item % DL_HEADS][item / DL_HEADS] = s;
     }
   }
-  delta[i] = s;
-  lse2[i] = lse[i] * 1.4426950408889634f;
+  __syncthreads();
+  const int h = h0 + threadIdx.x / DL_POS, p = threadIdx.x % DL_POS;
+  if (h < hq) {
+    const long b = t0 / seq;
+    const long off = (b * hq + h) * seq + (t0 - b * seq) + p;
+    delta[off] = sums[threadIdx.x / DL_POS][p];
+    lse2[off] = lse[off] * 1.4426950408889634f;
+  }
+}
+
+// Gradient of the per-head sink logits: dsink[h] = - sum over the head's rows of exp(sink - lse) * delta (the sink has no
+// value vector: it only enters through the softmax normaliser).  One CTA per head, fixed summation order.
+__global__ void __launch_bounds__(1024)
+attn_sink_grad_kernel(const float* __restrict__ delta, const float* __restrict__ lse, const float* __restrict__ sinks,
+                      float* __restrict__ dsinks, int batch, int seq, int hq) {
+  __shared__ float red[32];
+  const int h = blockIdx.x;
+  const float sink = sinks[h];
+  float s = 0.f;
+  for (int b = 0; b < batch; ++b) {
+    const long off = ((long)b * hq + h) * seq;
+    for (int i = threadIdx.x; i < seq; i += 1024) s += expf(sink - lse[off + i]) * delta[off + i];
+  }
+  s = pb::warp_sum(s);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    s = pb::warp_sum(red[threadIdx.x]);
+    if (threadIdx.x == 0) dsinks[h] = -s;
+  }
 }
 
 struct BwdArgs {
@@ -501,13 +546,9 @@ int launch_bwd(const BwdArgs& a) {
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
   const long T = (long)a.batch * a.seq;
-  {
-    const int threads = 256;
-    const long blocks = (T * a.hq + threads - 1) / threads;
-    attn_delta_kernel<<<(unsigned)blocks, threads, 0, a.stream>>>(
-        (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.delta + (long)a.batch * a.hq * a.seq,
-        a.seq, a.hq, DV, a.o_row, a.do_row, T);
-  }
+  attn_delta_kernel<DV><<<dim3((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS), DL_THREADS, 0, a.stream>>>(
+      (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.delta + (long)a.batch * a.hq * a.seq, a.seq,
+      a.hq, a.o_row, a.do_row);
   int rc;
   CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64, dq_m, dk_m, dv_m;
   const long TK = (long)a.batch * a.seq_k;
@@ -600,4 +641,12 @@ extern "C" int pb_flash_attn_bwd(const void* d_o, const void* q, const void* k, 
                                  int* status, cudaStream_t stream) {
   return pb_flash_attn_bwd_ex(d_o, q, k, v, o, lse, delta, dq, dk, dv, batch, seq, seq, 0, hq, hkv, d_qk, d_v, q_row,
                               k_row, v_row, o_row, do_row, dq_row, dk_row, dv_row, scale, causal, status, stream);
+}
+
+// dsinks[h] from the row sums delta [batch, hq, seq] that the backward left in its scratch and the forward's lse.
+extern "C" int pb_attn_sink_grad(const float* delta, const float* lse, const float* sinks, float* dsinks, int batch, int seq,
+                                 int hq, cudaStream_t stream) {
+  if (hq <= 0) return 0;
+  attn_sink_grad_kernel<<<hq, 1024, 0, stream>>>(delta, lse, sinks, dsinks, batch, seq, hq);
+  return (int)cudaGetLastError();
 }

@@ -91,8 +91,9 @@ def flash_attn_fwd(q, k, v, batch: int, causal: bool, scale: float, q_off: int =
 
 
 def flash_attn_bwd(do, q, k, v, o, lse, batch: int, causal: bool, scale: float, dq=None, dk=None, dv=None,
-                   q_off: int = 0, window: int = 0, softcap: float = 0.0):
-    """Returns (dq, dk, dv); optional pre-allocated outputs may be strided views (packed dQKV)."""
+                   q_off: int = 0, window: int = 0, softcap: float = 0.0, sinks=None):
+    """Returns (dq, dk, dv), and the gradient of the ``sinks`` when they are given; optional pre-allocated outputs may be
+    strided views (packed dQKV)."""
     T, hq, dqk = q.shape
     hkv, dvd = k.shape[1], v.shape[2]
     S = T // batch
@@ -109,12 +110,17 @@ def flash_attn_bwd(do, q, k, v, o, lse, batch: int, causal: bool, scale: float, 
               q.stride(0), k.stride(0), v.stride(0), o.stride(0), do.stride(0), dq.stride(0), dk.stride(0),
               dv.stride(0), float(scale), int(causal), int(window or 0), float(softcap or 0.0),
               _lib.status_word(q.device))
-    return dq, dk, dv
+    if sinks is None:
+        return dq, dk, dv
+    dsinks = torch.empty_like(sinks)
+    _lib.call("attn_sink_grad", delta, lse, sinks, dsinks, batch, S, hq)
+    return dq, dk, dv, dsinks
 
 
 def sink_grad(do, o, lse, sinks, batch: int):
-    """Gradient of the per-head sink logits: d sink_h = - sum_rows exp(sink_h - lse_row) * rowsum(dO * O) (the sink has
-    no value vector, so it only enters through the softmax normaliser)."""
+    """Gradient of the per-head sink logits in plain PyTorch (the oracle of what :func:`flash_attn_bwd` returns for them):
+    d sink_h = - sum_rows exp(sink_h - lse_row) * rowsum(dO * O) (the sink has no value vector, so it only enters through
+    the softmax normaliser)."""
     T, hq, _ = o.shape
     S = T // batch
     delta = (do.float() * o.float()).sum(-1).view(batch, S, hq).permute(0, 2, 1)      # [B, Hq, S]
@@ -134,9 +140,9 @@ class FlashAttnFn(torch.autograd.Function):
     def backward(ctx, do):
         q, k, v, o, lse, sinks = ctx.saved_tensors
         batch, causal, scale, q_off, window, has_sinks, softcap = ctx.args
-        dq, dk, dv = flash_attn_bwd(do, q, k, v, o, lse, batch, causal, scale, q_off=q_off, window=window,
-                                    softcap=softcap)
-        ds = sink_grad(do, o, lse, sinks, batch) if has_sinks else None
+        dq, dk, dv, *ds = flash_attn_bwd(do, q, k, v, o, lse, batch, causal, scale, q_off=q_off, window=window,
+                                         softcap=softcap, sinks=sinks if has_sinks else None)
+        ds = ds[0] if has_sinks else None
         return dq, dk, dv, None, None, None, None, None, ds, None
 
 

@@ -343,14 +343,15 @@ class RopeAttentionFn(torch.autograd.Function):
             ds = torch.zeros_like(sinks) if has_sinks else None
             for a, b in segments:
                 lb = lse[:, a:b].unsqueeze(0).contiguous()
-                attention.flash_attn_bwd(do3[a:b], q[a:b], k[a:b], v[a:b], o[a:b], lb, 1, causal, scale, dq=dq[a:b],
-                                         dk=dk[a:b], dv=dv[a:b], window=window, softcap=softcap)
+                grads = attention.flash_attn_bwd(do3[a:b], q[a:b], k[a:b], v[a:b], o[a:b], lb, 1, causal, scale,
+                                                 dq=dq[a:b], dk=dk[a:b], dv=dv[a:b], window=window, softcap=softcap,
+                                                 sinks=sinks if has_sinks else None)
                 if has_sinks:
-                    ds += attention.sink_grad(do3[a:b], o[a:b], lb, sinks, 1)
+                    ds += grads[3]
         else:
-            attention.flash_attn_bwd(do3, q, k, v, o, lse, batch, causal, scale, dq=dq, dk=dk, dv=dv, window=window,
-                                     softcap=softcap)
-            ds = attention.sink_grad(do3, o, lse, sinks, batch) if has_sinks else None
+            grads = attention.flash_attn_bwd(do3, q, k, v, o, lse, batch, causal, scale, dq=dq, dk=dk, dv=dv,
+                                             window=window, softcap=softcap, sinks=sinks if has_sinks else None)
+            ds = grads[3] if has_sinks else None
         if has_rope:
             dqk = dqkv[:, : (hq + hkv) * d].view(T, hq + hkv, d)
             fused.rope_inplace_(dqk, cos, sin, pos if has_pos else None, rot_dim, backward=True)

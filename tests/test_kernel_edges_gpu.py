@@ -137,3 +137,15 @@ def test_rope_head_groups(heads, d, rot, T):
     assert torch.equal(x[:, heads * d:], before[:, heads * d:])
     fused.rope_inplace_(view, cos, sin, pos, rot, backward=True)
     _close_bf16(view, before[:, :heads * d].view(T, heads, d), "inverse")
+
+
+@pytest.mark.parametrize("batch,S,hq,hkv", [(1, 128, 3, 1), (2, 256, 16, 2)])
+def test_sink_gradient_matches_oracle(batch, S, hq, hkv):
+    g = _gen(hq)
+    q, do = (torch.randn(batch * S, hq, 64, device="cuda", generator=g).bfloat16() for _ in range(2))
+    k, v = (torch.randn(batch * S, hkv, 64, device="cuda", generator=g).bfloat16() for _ in range(2))
+    sinks = torch.randn(hq, device="cuda", generator=g)
+    o, lse = attention.flash_attn_fwd(q, k, v, batch, True, 0.125, sinks=sinks)
+    ds = attention.flash_attn_bwd(do, q, k, v, o, lse, batch, True, 0.125, sinks=sinks)[3]
+    ref = attention.sink_grad(do, o, lse, sinks, batch)
+    assert (ds - ref).abs().max() <= 1e-4 * (1 + ref.abs().max())
