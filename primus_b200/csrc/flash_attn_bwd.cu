@@ -1,21 +1,21 @@
 // Flash-attention backward for sm_100a.
 //
-// One templated kernel runs in two modes that share all plumbing:
+// Templated kernels run in two modes that share all plumbing:
 //   MODE_DKDV: a CTA owns 128 KV rows of one KV head (resident tiles X1 = K, X2 = V) and streams
-//              64-row tiles of Q / dO (Y1, Y2) of every query head of the group;
+//              tiles of Q / dO (Y1, Y2) of every query head of the group;
 //              S^T = K Q^T, dP^T = V dO^T  ->  P^T, dS^T  ->  dV += P^T dO,  dK += dS^T Q.
-//   MODE_DQ  : a CTA owns 128 query rows of one head (X1 = Q, X2 = dO) and streams 64-row tiles of
+//   MODE_DQ  : a CTA owns 128 query rows of one head (X1 = Q, X2 = dO) and streams tiles of
 //              K / V;  S = Q K^T, dP = dO V^T  ->  dS  ->  dQ += dS K.
 // In both modes the accumulators live in tensor memory for the whole loop (no atomics, results are
-// bit-reproducible), the S / dP tiles are double-buffered in TMEM where capacity allows, and the
-// streamed tiles are used twice from one shared-memory copy (K-major operand for the first GEMM,
-// MN-major operand for the second).  The softmax threads turn S / dP into bf16 P / dS *in tensor memory*:
-// a thread overwrites the first 8 of its own 16 S (dP) columns with the packed pair values, and the second
-// GEMM takes its A operand from there (`tcgen05.mma` with A in TMEM), one 16-wide K step per column group.
-// Nothing but mbarriers goes through shared memory between the two GEMMs of a step.  The per-step chain of
-// a softmax thread (TMEM load -> exp2 / multiply -> TMEM store -> arrive) is latency bound, so two teams of
-// 128 threads work on alternating steps (each thread owns one row and all 64 columns of its step) while
-// the MMA thread runs two steps ahead.
+// bit-reproducible), and the streamed tiles are used twice from one shared-memory copy (K-major operand for
+// the first GEMM, MN-major operand for the second).  The softmax threads turn S / dP into bf16 P / dS *in tensor
+// memory*, 8 packed columns per 16 values, and the second GEMM takes its A operand from there (`tcgen05.mma` with A in
+// TMEM), one 16-wide K step per column group.  Nothing but mbarriers goes through shared memory between the two GEMMs of
+// a step.
+//   flash_attn_bwd_kernel       64-row steps: the multi-latent head shape (d_qk 192, d_v 128), whose accumulators leave
+//                               too little tensor memory for wider ones.  Two teams of 256 softmax threads work on
+//                               alternating steps while the MMA thread runs ahead.
+//   flash_attn_bwd_wide_kernel  128-row steps: d_qk == d_v.
 //
 // Replaces the backward of `flash_attn_func` (primus/backends/megatron/core/extensions/
 // primus_turbo.py:812-823); deterministic by construction (cf. the `deterministic=` flag there, :805).
@@ -27,9 +27,10 @@ namespace {
 
 constexpr int BR = 128;  // resident rows
 constexpr int BC = 64;   // streamed rows per step
-constexpr int BW_THREADS = 320;   // warp0 TMA, warp1 MMA, warps 2..9: two softmax teams of 128 threads
-constexpr int BW_COMPUTE = 256;
-constexpr int BW_TEAMS = 2;       // team t handles steps i = t (mod 2): one thread per resident row, all 64 columns
+constexpr int BW_THREADS = 576;   // warp0 TMA, warp1 MMA, warps 2..17: two softmax teams of 256 threads
+constexpr int BW_COMPUTE = 512;
+constexpr int BW_TEAMS = 2;       // team t handles steps i = t (mod 2): two threads per resident row, 32 columns each
+constexpr int BW_HALF = BC / 2;   // streamed columns of a step per softmax thread
 constexpr int XATOM = 128 * 128;  // bytes of a [128 rows x 64 bf16] atom
 constexpr int YATOM = 64 * 128;   // bytes of a [64 rows x 64 bf16] atom
 enum { MODE_DKDV = 0, MODE_DQ = 1 };
@@ -37,21 +38,15 @@ enum { MODE_DKDV = 0, MODE_DQ = 1 };
 template <int DQK, int DV, int MODE>
 struct BwCfg {
   static constexpr int ACC_COLS = (MODE == MODE_DKDV) ? (DQK + DV) : DQK;
-  // S / dP buffers in tensor memory: 3 when they fit next to the accumulators and (MODE_DQ) the TMEM copies of the
-  // resident tiles, else 2, else 1.  For the dQ pass of 128-wide heads two buffers + the TMEM operands measured
-  // faster (2.217 ms for the whole backward at seq 8192) than three buffers without them (2.260 ms).
-  static constexpr int XA_COLS = (MODE == MODE_DQ) ? (DQK / 2 + DV / 2) : 0;
-  static constexpr int SBUF = (ACC_COLS + 384 + XA_COLS <= 512) ? 3 : ((ACC_COLS + 256 <= 512) ? 2 : 1);
-  // barrier of step i: one per buffer when there are three (steps i and i + 2 of a team can both be in flight), else
-  // one per softmax team
-  __host__ __device__ static constexpr int bar_idx(int i) { return SBUF == 3 ? i % 3 : (i & 1); }
-  __host__ __device__ static constexpr uint32_t bar_parity(int i) { return SBUF == 3 ? ((i / 3) & 1) : ((i >> 1) & 1); }
-  // MODE_DQ: when tensor memory has room, the resident tiles (Q, dO) are also kept there as packed bf16 and the first
-  // GEMMs of a step (S = Q K^T, dP = dO V^T) take their A operand from tensor memory: a both-operands-in-shared-memory
-  // MMA with a 64-wide N tile re-reads 128 x 16 A elements per 32 clocks, three times what shared memory delivers
-  static constexpr bool XA = (MODE == MODE_DQ) && (ACC_COLS + SBUF * 128 + DQK / 2 + DV / 2 <= 512);
-  static constexpr int XA1_COL = ACC_COLS + SBUF * 128;
-  static constexpr int XA2_COL = XA1_COL + DQK / 2;
+  // S / dP buffers in tensor memory: 2 when they fit next to the accumulators, else 1
+  static constexpr int SBUF = (ACC_COLS + 256 <= 512) ? 2 : 1;
+  // When only one S / dP pair fits next to the accumulators (192 / 128-wide heads, dK / dV pass), the columns are split
+  // into two S buffers and one dP buffer: P and dS are both packed into the step's S columns (8 + 8 of every 16), so the
+  // dP buffer is free again as soon as the softmax threads have *read* it, and the S / dP GEMMs of a step run under the
+  // softmax of the step before instead of after it.
+  static constexpr bool SPLIT = SBUF == 1;
+  static constexpr int DP_COL = SPLIT ? 2 * BC : BC;     // dP columns: of the region / relative to the step's S columns
+  static_assert(!SPLIT || ACC_COLS + 3 * BC <= 512, "tensor memory");
   static constexpr int X1_BYTES = BR * DQK * 2;
   static constexpr int X2_BYTES = BR * DV * 2;
   static constexpr int Y1_BYTES = BC * DQK * 2;
@@ -69,10 +64,10 @@ struct BwCfg {
 struct BwBars {
   uint64_t x_full;
   uint64_t y_full[4], y_empty[4];
-  uint64_t s_full[3];
-  uint64_t p_ready[3]; // per team: P / dS of its current step are in tensor memory (one arrival per warp)
+  uint64_t s_full[2];  // per team
+  uint64_t p_ready[2]; // per team: P / dS of its current step are in tensor memory (one arrival per warp)
   uint64_t acc_done;   // all MMAs of the CTA have completed
-  uint64_t xa_ready;   // resident tiles copied into tensor memory (one arrival per softmax warp)
+  uint64_t dp_free;    // SPLIT: the softmax threads hold the step's dP in registers (one arrival per warp of the team)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -160,10 +155,10 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       pb::mbar_init(&bars->y_full[i], 1);
       pb::mbar_init(&bars->y_empty[i], 1);
     }
-    for (int i = 0; i < 3; ++i) pb::mbar_init(&bars->s_full[i], 1);
-    for (int i = 0; i < 3; ++i) pb::mbar_init(&bars->p_ready[i], BW_COMPUTE / BW_TEAMS / 32);
+    for (int i = 0; i < 2; ++i) pb::mbar_init(&bars->s_full[i], 1);
+    for (int i = 0; i < 2; ++i) pb::mbar_init(&bars->p_ready[i], BW_COMPUTE / BW_TEAMS / 32);
     pb::mbar_init(&bars->acc_done, 1);
-    pb::mbar_init(&bars->xa_ready, BW_COMPUTE / 32);
+    pb::mbar_init(&bars->dp_free, BW_COMPUTE / BW_TEAMS / 32);
     bars->abort_flag = 0;
     pb::fence_barrier_init();
   }
@@ -175,7 +170,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   __syncthreads();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  const uint32_t tmem_sbuf = tmem_base + C::ACC_COLS;  // [buf][S 64 | dP 64]
+  const uint32_t tmem_sbuf = tmem_base + C::ACC_COLS;  // [buf][S 64 | dP 64], SPLIT: [S 64][S 64][dP 64]
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -218,56 +213,52 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
       const uint32_t x1a = pb::smem_u32(x1_smem), x2a = pb::smem_u32(x2_smem);
       bool ok = true;
+      auto s_cols = [&](int i) { return tmem_sbuf + (C::SPLIT ? (i & 1) * BC : (i % C::SBUF) * 128); };
+      auto dp_cols = [&](int i) { return C::SPLIT ? tmem_sbuf + C::DP_COL : s_cols(i) + C::DP_COL; };
+      auto issue_s = [&](int i) {
+        const uint32_t y1a = pb::smem_u32(y1_smem + (i % C::NS) * C::Y1_BYTES);
+#pragma unroll
+        for (int k = 0; k < DQK / 16; ++k)
+          pb::umma_f16_ss(s_cols(i), pb::make_smem_desc(x1a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
+                          pb::make_smem_desc(y1a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s, k > 0 ? 1u : 0u);
+      };
+      auto issue_dp = [&](int i) {
+        const uint32_t y2a = pb::smem_u32(y2_smem + (i % C::NS) * C::Y2_BYTES);
+#pragma unroll
+        for (int k = 0; k < DV / 16; ++k)
+          pb::umma_f16_ss(dp_cols(i), pb::make_smem_desc(x2a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
+                          pb::make_smem_desc(y2a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s, k > 0 ? 1u : 0u);
+      };
       auto issue_sdp = [&](int i) {
-        const int st = i % C::NS;
-        const uint32_t y1a = pb::smem_u32(y1_smem + st * C::Y1_BYTES);
-        const uint32_t y2a = pb::smem_u32(y2_smem + st * C::Y2_BYTES);
-        const uint32_t ts = tmem_sbuf + (i % C::SBUF) * 128;
-        if (C::XA) {
-#pragma unroll
-          for (int k = 0; k < DQK / 16; ++k)
-            pb::umma_f16_ts(ts, tmem_base + C::XA1_COL + 8 * k,
-                            pb::make_smem_desc(y1a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s, k > 0 ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < DV / 16; ++k)
-            pb::umma_f16_ts(ts + 64, tmem_base + C::XA2_COL + 8 * k,
-                            pb::make_smem_desc(y2a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s, k > 0 ? 1u : 0u);
-        } else {
-#pragma unroll
-          for (int k = 0; k < DQK / 16; ++k)
-            pb::umma_f16_ss(ts, pb::make_smem_desc(x1a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
-                            pb::make_smem_desc(y1a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s,
-                            k > 0 ? 1u : 0u);
-#pragma unroll
-          for (int k = 0; k < DV / 16; ++k)
-            pb::umma_f16_ss(ts + 64, pb::make_smem_desc(x2a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
-                            pb::make_smem_desc(y2a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s,
-                            k > 0 ? 1u : 0u);
-        }
-        pb::umma_commit(&bars->s_full[C::bar_idx(i)]);
+        issue_s(i);
+        issue_dp(i);
+        pb::umma_commit(&bars->s_full[i & 1]);
       };
       // The S / dP GEMMs run SBUF steps ahead.  Step i + SBUF reuses the TMEM buffer of step i; it is issued after
       // the second GEMMs of step i (same thread: the tensor pipe keeps the order), which themselves wait for the
       // softmax threads to have replaced S / dP of step i by P / dS.
       do {
         BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_MMA);
-        if (C::XA) {
-          BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_MMA);
-          pb::tc_fence_after();
-        }
-        for (int j = 0; j < C::SBUF && j < n_iter && ok; ++j) {
+        for (int j = 0; j < (C::SPLIT ? 2 : C::SBUF) && j < n_iter && ok; ++j) {
           BW_WAIT(&bars->y_full[j % C::NS], (j / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
-          issue_sdp(j);
+          if (C::SPLIT && j == 1) issue_s(1);
+          else issue_sdp(j);
         }
       } while (false);
       for (int i = 0; i < n_iter && ok; ++i) {
         const int st = i % C::NS;
-        BW_WAIT(&bars->p_ready[C::bar_idx(i)], C::bar_parity(i), PB_ERR_TIMEOUT_MMA);
+        if (C::SPLIT && i + 1 < n_iter) {     // S of step i + 1 is already on its way
+          BW_WAIT(&bars->dp_free, i & 1, PB_ERR_TIMEOUT_MMA);
+          pb::tc_fence_after();
+          issue_dp(i + 1);
+          pb::umma_commit(&bars->s_full[(i + 1) & 1]);
+        }
+        BW_WAIT(&bars->p_ready[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_MMA);
         pb::tc_fence_after();
         const uint32_t y1a = pb::smem_u32(y1_smem + st * C::Y1_BYTES);
         const uint32_t y2a = pb::smem_u32(y2_smem + st * C::Y2_BYTES);
-        const uint32_t ts = tmem_sbuf + (i % C::SBUF) * 128;
+        const uint32_t ts = s_cols(i), tds = C::SPLIT ? ts + 8 : ts + C::DP_COL;
         if (MODE == MODE_DKDV) {
 #pragma unroll
           for (int k = 0; k < BC / 16; ++k)   // acc(DV) += P . Y2, A = packed P of K step k (TMEM columns 16k .. 16k+7)
@@ -276,14 +267,15 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         }
 #pragma unroll
         for (int k = 0; k < BC / 16; ++k)     // acc(DQK) += dS . Y1
-          pb::umma_f16_ts(tmem_base, ts + 64 + 16 * k, pb::make_smem_desc(y1a + k * 2048, YATOM, 1024, 2), idesc_a1,
+          pb::umma_f16_ts(tmem_base, tds + 16 * k, pb::make_smem_desc(y1a + k * 2048, YATOM, 1024, 2), idesc_a1,
                           (i > 0 || k > 0) ? 1u : 0u);
         pb::umma_commit(&bars->y_empty[st]);
-        if (i + C::SBUF < n_iter) {
-          const int in = i + C::SBUF;
+        const int in = i + (C::SPLIT ? 2 : C::SBUF);
+        if (in < n_iter) {
           BW_WAIT(&bars->y_full[in % C::NS], (in / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
-          issue_sdp(in);
+          if (C::SPLIT) issue_s(in);
+          else issue_sdp(in);
         }
       }
       if (ok) pb::umma_commit(&bars->acc_done);
@@ -291,66 +283,48 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   } else {
     // ------------------------------------------------------------------ softmax-gradient threads
     const int wq = warp & 3;              // TMEM lane quarter of this warp
-    const int team = (warp - 2) >> 2;     // 0 / 1: even / odd steps
+    const int team = (warp - 2) >> 3;     // 0 / 1: even / odd steps
+    const int half = ((warp - 2) >> 2) & 1;   // which 32 of a step's 64 columns
     const int row = wq * 32 + lane;
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
     const int row_g = rb * BR + row;
     float lse2_row = 0.f, delta_row = 0.f;
     if (MODE == MODE_DQ) {
       const long off = ((long)batch * hq + xhead) * seq + row_g;
-      lse2_row = lse[off];  // already in log2 units
+      lse2_row = lse[off];  // negated, in log2 units
       delta_row = delta[off];
     }
     bool ok = true;
-    if (C::XA) {
-      // team 0 copies its row of X1 (Q), team 1 its row of X2 (dO) from the 128-byte-swizzled shared tiles into
-      // tensor memory: word w of a row (elements 2w, 2w + 1) goes to column w, the layout of a TMEM A operand
-      do {
-        BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);
-        const uint8_t* xs = team == 0 ? x1_smem : x2_smem;
-        const int natoms = (team == 0 ? DQK : DV) / 64;
-        const uint32_t dst = tmem_base + lane_addr + (team == 0 ? C::XA1_COL : C::XA2_COL);
-        for (int a = 0; a < natoms; ++a) {
-          uint32_t wds[32];
-#pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            const uint4 v = *reinterpret_cast<const uint4*>(xs + a * XATOM + row * 128 + ((c ^ (row & 7)) << 4));
-            wds[4 * c] = v.x; wds[4 * c + 1] = v.y; wds[4 * c + 2] = v.z; wds[4 * c + 3] = v.w;
-          }
-          pb::tmem_st_32x32b_x32(dst + 32 * a, wds);
-        }
-        pb::tmem_wait_st();
-        pb::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) pb::mbar_arrive(&bars->xa_ready);
-      } while (false);
-    }
     for (int i = team; i < n_iter && ok; i += BW_TEAMS) {
-      const int sb = i % C::SBUF;
       const int st = i % C::NS;
       const int cs = c_start + i % n_per_head;
-      BW_WAIT(&bars->s_full[C::bar_idx(i)], C::bar_parity(i), PB_ERR_TIMEOUT_EPILOGUE);
+      BW_WAIT(&bars->s_full[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_EPILOGUE);
       if (MODE == MODE_DKDV) {
         BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
       }
       pb::tc_fence_after();
-      const uint32_t ts = tmem_sbuf + lane_addr + sb * 128;
+      const uint32_t ts = tmem_sbuf + lane_addr + (C::SPLIT ? (i & 1) * BC : (i % C::SBUF) * 128) + half * BW_HALF;
+      const uint32_t tdp = C::SPLIT ? tmem_sbuf + lane_addr + C::DP_COL + half * BW_HALF : ts + C::DP_COL;
+      const uint32_t tds = C::SPLIT ? ts + 8 : tdp;    // where the packed dS goes
       const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
       // largest (query position - key position) inside this tile pair: beyond the window -> element-wise mask
       const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BC + BC - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BC);
       const bool diag = (causal && (cs_rel >= 2 * rb) && (cs_rel <= 2 * rb + 1)) || (window > 0 && max_diff >= window);
-      const float* st_lse = stat_smem + st * 128;
+      const float* st_lse = stat_smem + st * 128 + half * BW_HALF;
       const float* st_delta = st_lse + 64;
-      uint32_t s[BC], dp[BC];
+      uint32_t s[BW_HALF], dp[BW_HALF];
       pb::tmem_ld_32x32b_x32(ts, s);
-      pb::tmem_ld_32x32b_x32(ts + 32, s + 32);
-      pb::tmem_ld_32x32b_x32(ts + 64, dp);
-      pb::tmem_ld_32x32b_x32(ts + 96, dp + 32);
+      pb::tmem_ld_32x32b_x32(tdp, dp);
       pb::tmem_wait_ld();
+      if (C::SPLIT) {
+        pb::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) pb::mbar_arrive(&bars->dp_free);
+      }
       auto body = [&](auto diag_tag) {
         constexpr bool DIAG = decltype(diag_tag)::value;
 #pragma unroll
-        for (int kk = 0; kk < BC / 16; ++kk) {   // one 16-wide K step of the second GEMM at a time
+        for (int kk = 0; kk < BW_HALF / 16; ++kk) {   // one 16-wide K step of the second GEMM at a time
           uint32_t pk[8], dsk[8];
 #pragma unroll
           for (int e4 = 0; e4 < 16; e4 += 4) {
@@ -372,9 +346,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
                 sv = t * cap_b;                  // = softcap * tanh(scale * s / softcap) / scale
                 dcap = 1.f - t * t;              // derivative of the capped score with respect to scale * s
               }
-              float p = pb::fast_exp2(fmaf(sv, sl2, -l2[u]));
+              float p = pb::fast_exp2(fmaf(sv, sl2, l2[u]));   // (lse is stored negated)
               if (DIAG) {
-                const int col_g = cs_rel * BC + c + u;
+                const int col_g = cs_rel * BC + half * BW_HALF + c + u;
                 const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
                 if (diff < 0 || (window > 0 && diff >= window)) p = 0.f;
               }
@@ -386,16 +360,16 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
             dsk[e4 / 2] = pb::pack_bf16x2(dv[0], dv[1]);
             dsk[e4 / 2 + 1] = pb::pack_bf16x2(dv[2], dv[3]);
           }
-          // P / dS (bf16 pairs) replace the first 8 of the 16 S / dP columns of this K step
+          // P / dS (bf16 pairs) replace the first 8 of the 16 S / dP columns of this K step (SPLIT: both go to S columns)
           if (MODE == MODE_DKDV) pb::tmem_st_32x32b_x8(ts + 16 * kk, pk);
-          pb::tmem_st_32x32b_x8(ts + 64 + 16 * kk, dsk);
+          pb::tmem_st_32x32b_x8(tds + 16 * kk, dsk);
         }
       };
       if (diag) body(std::true_type{}); else body(std::false_type{});
       pb::tmem_wait_st();
       pb::tc_fence_before();
       __syncwarp();
-      if (lane == 0) pb::mbar_arrive(&bars->p_ready[C::bar_idx(i)]);   // one arrival per warp
+      if (lane == 0) pb::mbar_arrive(&bars->p_ready[i & 1]);   // one arrival per warp
     }
     // ---- epilogue: accumulators -> bf16 -> (dead) resident tiles -> TMA store
     do {
@@ -404,7 +378,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       pb::tc_fence_after();
       auto drain = [&](uint32_t tcol, int ncols, uint8_t* dst) {
 #pragma unroll 1
-        for (int c = team; c < ncols / 32; c += BW_TEAMS) {
+        for (int c = 2 * team + half; c < ncols / 32; c += 4) {
           uint32_t r[32];
           pb::tmem_ld_32x32b_x32(tmem_base + lane_addr + tcol + c * 32, r);
           pb::tmem_wait_ld();
@@ -451,14 +425,487 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   }
 }
 
-// delta[b, h, s] = sum_d dO * O ;  lse2 = lse * log2(e) (so the main kernels need no per-element multiply).
+// ------------------------------------------------------------------------------------------------
+// 128-wide steps, for d_qk == d_v (64, 128) and the dQ pass of (192, 128).  A tcgen05.mma with N = 64 occupies the tensor pipe about as long as one with
+// N = 128, so the 64-row steps above pay twice for S and dP; and there the two second GEMMs of a step run only after its
+// whole softmax.  Here a step streams 128 rows, and its work is cut so that the tensor pipe always has some of it:
+//   * the softmax threads take P = exp2(S) as soon as S is there, before dP;
+//   * dS and the second GEMMs go by column halves A (64 columns) and B: the GEMMs of half A run while half B is computed;
+//   * what frees a tensor-memory region is the *read* of it.  With two S buffers (64-wide heads) P and dS are packed into
+//     the step's S columns (8 + 8 of every 16) and the next dP starts as soon as this one is in registers; with one S
+//     buffer (128-wide) they are packed into the dP columns and the next S starts instead.
+// Streamed tiles sit in NS buffers of 128 rows, loaded and released by 64-row halves.  In the dQ pass of 128-wide heads the
+// resident tiles (Q, dO) move to tensor memory at the start, as A operands of the first GEMMs; their shared memory is the
+// third buffer.
+template <int DQK, int DV, int MODE>
+struct BwWideCfg {
+  static constexpr int BCW = 128;
+  static constexpr int ACC_COLS = (MODE == MODE_DKDV) ? DQK + DV : DQK;
+  static constexpr int NSB = DQK == 64 ? 2 : 1;                        // S buffers
+  static constexpr bool XA1 = MODE == MODE_DQ && DQK == 128;           // X1 (Q) in tensor memory
+  static constexpr bool XA2 = MODE == MODE_DQ && DV == 128;            // X2 (dO) in tensor memory
+  static constexpr int S_COL = ACC_COLS;
+  static constexpr int DP_COL = ACC_COLS + NSB * BCW;
+  static constexpr int XA1_COL = DP_COL + BCW;
+  static constexpr int XA2_COL = XA1_COL + (XA1 ? DQK / 2 : 0);
+  static constexpr int T1_BYTES = BR * DQK * 2;                        // a [128, DQK] tile (X1, Y1)
+  static constexpr int T2_BYTES = BR * DV * 2;                         // a [128, DV] tile (X2, Y2)
+  static constexpr int STAT_FLOATS = MODE == MODE_DKDV ? 256 : 0;      // per half: 64 lse, 64 delta
+  static constexpr int STAGE_BYTES = T1_BYTES + T2_BYTES + STAT_FLOATS * 4;
+  static constexpr int FIXED_BYTES = (XA1 ? 0 : T1_BYTES) + (XA2 ? 0 : T2_BYTES) + 1024 + 512;
+  static constexpr int NS_FIT = (232448 - FIXED_BYTES) / STAGE_BYTES;
+  static constexpr int NS = NS_FIT >= 4 ? 4 : NS_FIT;
+  static constexpr int SMEM_BYTES = FIXED_BYTES + NS * STAGE_BYTES;
+  static_assert(NS >= 2, "shared memory");
+  static_assert(XA2_COL + (XA2 ? DV / 2 : 0) <= 512, "tensor memory");
+};
+constexpr int BWW_WARPS = 16;                       // softmax warps: thread = one resident row x 16 columns of each half
+constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
+
+struct BwWideBars {
+  uint64_t x_full;
+  uint64_t y_full[4], ya_empty[4], yb_empty[4];
+  uint64_t s_full[2], dp_full;
+  uint64_t freed;          // the softmax threads hold S (one S buffer) or dP (two) of the step in registers
+  uint64_t pa[2], pb[2];   // P / dS of half A / B are in tensor memory; by step parity, because with two S buffers a warp can
+                           // be a step ahead of another
+  uint64_t acc_done;
+  uint64_t xa_ready;       // resident tiles copied into tensor memory
+  uint32_t tmem_base;
+  int abort_flag;
+};
+
+// one look at a barrier, without waiting
+__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.test_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t}"
+      : "=r"(ok)
+      : "r"(pb::smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+// VAR: 0 plain, 1 sliding window, 2 soft-capped scores (with or without a window); a variant carries no code of a later one
+template <int DQK, int DV, int MODE, int VAR>
+__global__ void __launch_bounds__(BWW_THREADS, 1)
+flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
+                           const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
+                           const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmO2,
+                           const float* __restrict__ lse, const float* __restrict__ delta, int seq, int seq_k, int q_off,
+                           int hq, int hkv, float scale, int causal, int window_arg, float softcap_arg, int* status) {
+  using C = BwWideCfg<DQK, DV, MODE>;
+  constexpr int BCW = C::BCW;
+  constexpr bool CAP = VAR == 2;
+  const int window = VAR ? window_arg : 0;
+  const float cap_a = CAP ? scale / softcap_arg : 0.f;
+  const float cap_b = CAP ? softcap_arg / scale : 0.f;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* y1_smem = smem + (C::XA1 ? 0 : C::T1_BYTES) + (C::XA2 ? 0 : C::T2_BYTES);   // NS stages
+  uint8_t* y2_smem = y1_smem + C::NS * C::T1_BYTES;                                     // NS stages
+  // a resident tile that goes to tensor memory passes through the last stage's buffer before its first streamed tile
+  uint8_t* x1_smem = C::XA1 ? y1_smem + (C::NS - 1) * C::T1_BYTES : smem;
+  uint8_t* x2_smem = C::XA2 ? y2_smem + (C::NS - 1) * C::T2_BYTES : smem + (C::XA1 ? 0 : C::T1_BYTES);
+  float* stat_smem = reinterpret_cast<float*>(y2_smem + C::NS * C::T2_BYTES);   // NS x [64 lse A | 64 delta A | lse B | delta B]
+  BwWideBars* bars = reinterpret_cast<BwWideBars*>(stat_smem + C::NS * C::STAT_FLOATS);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int g = hq / hkv;
+  const int seq_x = (MODE == MODE_DKDV) ? seq_k : seq;
+  const int seq_y = (MODE == MODE_DKDV) ? seq : seq_k;
+  const int num_rb = seq_x / BR;
+  const int num_c = seq_y / BCW;
+  const int qo = q_off / BCW;
+  // longest row blocks first, as in the kernel above
+  const int rb = (MODE == MODE_DKDV) ? blockIdx.y : (num_rb - 1 - blockIdx.y);
+  const int nxh = (MODE == MODE_DKDV) ? hkv : hq;
+  const int xhead = blockIdx.x % nxh;
+  const int batch = blockIdx.x / nxh;
+  const int tok0 = batch * seq_x;
+  const int toky0 = batch * seq_y;
+  const int c_start = (MODE == MODE_DKDV) ? (causal ? max(0, rb - qo) : 0)
+                                          : (window > 0 ? max(0, rb * BR + q_off - window + 1) / BCW : 0);
+  const int c_end = (MODE == MODE_DKDV)
+                        ? (window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BCW + 1) : num_c)
+                        : (causal ? min(num_c, rb + 1 + qo) : num_c);
+  const int n_per_head = max(0, c_end - c_start);
+  const int n_iter = (MODE == MODE_DKDV) ? g * n_per_head : n_per_head;
+  volatile int* abort_flag = &bars->abort_flag;
+  const float sl2 = scale * 1.4426950408889634f;
+
+  if (threadIdx.x == 0) {
+    pb::mbar_init(&bars->x_full, 1);
+    for (int i = 0; i < 4; ++i) {
+      pb::mbar_init(&bars->y_full[i], 1);
+      pb::mbar_init(&bars->ya_empty[i], 1);
+      pb::mbar_init(&bars->yb_empty[i], 1);
+    }
+    pb::mbar_init(&bars->s_full[0], 1);
+    pb::mbar_init(&bars->s_full[1], 1);
+    pb::mbar_init(&bars->dp_full, 1);
+    pb::mbar_init(&bars->freed, BWW_WARPS);
+    for (int i = 0; i < 2; ++i) {
+      pb::mbar_init(&bars->pa[i], BWW_WARPS);
+      pb::mbar_init(&bars->pb[i], BWW_WARPS);
+    }
+    pb::mbar_init(&bars->acc_done, 1);
+    pb::mbar_init(&bars->xa_ready, BWW_WARPS);
+    bars->abort_flag = 0;
+    pb::fence_barrier_init();
+  }
+  if (warp == 1) {
+    pb::tmem_alloc<1>(&bars->tmem_base, 512);
+    pb::tmem_relinquish<1>();
+  }
+  pb::tc_fence_before();
+  __syncthreads();
+  pb::tc_fence_after();
+  const uint32_t tmem_base = bars->tmem_base;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (lane == 0) {
+      bool ok = true;
+      pb::mbar_expect_tx(&bars->x_full, C::T1_BYTES + C::T2_BYTES);
+#pragma unroll
+      for (int a = 0; a < DQK / 64; ++a)
+        pb::tma_load_3d(x1_smem + a * XATOM, &tmX1, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
+#pragma unroll
+      for (int a = 0; a < DV / 64; ++a)
+        pb::tma_load_3d(x2_smem + a * XATOM, &tmX2, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
+      for (int i = 0; i < n_iter && ok; ++i) {
+        const int st = i % C::NS;
+        const uint32_t par = ((i / C::NS) & 1) ^ 1;
+        const int yhead = (MODE == MODE_DKDV) ? (xhead * g + i / n_per_head) : (xhead / g);
+        const int cs = c_start + i % n_per_head;
+        if ((C::XA1 || C::XA2) && i == C::NS - 1) {
+          BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
+        }
+        for (int h = 0; h < 2 && ok; ++h) {
+          BW_WAIT(h == 0 ? &bars->ya_empty[st] : &bars->yb_empty[st], par, PB_ERR_TIMEOUT_TMA);
+          if (h == 0)
+            pb::mbar_expect_tx(&bars->y_full[st], C::STAGE_BYTES);
+          const int row = cs * BCW + h * 64;
+#pragma unroll
+          for (int a = 0; a < DQK / 64; ++a)
+            pb::tma_load_3d(y1_smem + st * C::T1_BYTES + a * XATOM + h * YATOM, &tmY1, &bars->y_full[st], a * 64, yhead,
+                            toky0 + row);
+#pragma unroll
+          for (int a = 0; a < DV / 64; ++a)
+            pb::tma_load_3d(y2_smem + st * C::T2_BYTES + a * XATOM + h * YATOM, &tmY2, &bars->y_full[st], a * 64, yhead,
+                            toky0 + row);
+          if (MODE == MODE_DKDV) {
+            const long off = ((long)batch * hq + yhead) * seq + row;
+            float* stat = stat_smem + st * C::STAT_FLOATS + h * 128;
+            bulk_load_1d(stat, lse + off, 256, &bars->y_full[st]);
+            bulk_load_1d(stat + 64, delta + off, 256, &bars->y_full[st]);
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0) {
+      constexpr uint32_t idesc_s = pb::make_idesc_bf16(BR, BCW, 0, 0);
+      constexpr uint32_t idesc_a1 = pb::make_idesc_bf16(BR, DQK, 0, 1);  // acc(DQK) += dS . Y1
+      constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
+      const uint32_t x1a = pb::smem_u32(x1_smem), x2a = pb::smem_u32(x2_smem);
+      bool ok = true;
+      // X . Y^T -> 128 columns, X from shared or from tensor memory
+      auto issue_first = [&](auto dim, auto from_tmem, uint32_t tcol, uint32_t xa, uint32_t xt, uint32_t ya) {
+#pragma unroll
+        for (int k = 0; k < decltype(dim)::value / 16; ++k) {
+          const uint32_t off = (k / 4) * XATOM + (k % 4) * 32;
+          const uint64_t db = pb::make_smem_desc(ya + off, 0, 1024, 2);
+          if (decltype(from_tmem)::value)
+            pb::umma_f16_ts(tmem_base + tcol, tmem_base + xt + 8 * k, db, idesc_s, k > 0 ? 1u : 0u);
+          else
+            pb::umma_f16_ss(tmem_base + tcol, pb::make_smem_desc(xa + off, 0, 1024, 2), db, idesc_s, k > 0 ? 1u : 0u);
+        }
+      };
+      auto issue_s = [&](int i) {
+        issue_first(std::integral_constant<int, DQK>{}, std::bool_constant<C::XA1>{},
+                    C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0), x1a, C::XA1_COL,
+                    pb::smem_u32(y1_smem + (i % C::NS) * C::T1_BYTES));
+        pb::umma_commit(&bars->s_full[C::NSB == 2 ? (i & 1) : 0]);
+      };
+      auto issue_dp = [&](int i) {
+        issue_first(std::integral_constant<int, DV>{}, std::bool_constant<C::XA2>{}, C::DP_COL, x2a, C::XA2_COL,
+                    pb::smem_u32(y2_smem + (i % C::NS) * C::T2_BYTES));
+        pb::umma_commit(&bars->dp_full);
+      };
+      auto issue_second = [&](int i, int half) {                            // accumulators += (P, dS of the half) . Y
+        const int st = i % C::NS;
+        const uint32_t y1a = pb::smem_u32(y1_smem + st * C::T1_BYTES), y2a = pb::smem_u32(y2_smem + st * C::T2_BYTES);
+        const uint32_t tp = tmem_base + (C::NSB == 2 ? C::S_COL + (i & 1) * BCW : C::DP_COL);
+        if (MODE == MODE_DKDV) {
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {
+            const int k = half * 4 + kk;
+            pb::umma_f16_ts(tmem_base + DQK, tp + 16 * k, pb::make_smem_desc(y2a + k * 2048, XATOM, 1024, 2), idesc_a2,
+                            (i > 0 || k > 0) ? 1u : 0u);
+          }
+        }
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk) {
+          const int k = half * 4 + kk;
+          pb::umma_f16_ts(tmem_base, tp + 16 * k + 8, pb::make_smem_desc(y1a + k * 2048, XATOM, 1024, 2), idesc_a1,
+                          (i > 0 || k > 0) ? 1u : 0u);
+        }
+        pb::umma_commit(half == 0 ? &bars->ya_empty[st] : &bars->yb_empty[st]);
+      };
+      do {
+        if (n_iter == 0) break;
+        BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_MMA);
+        if (C::XA1 || C::XA2) {
+          BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_MMA);
+        }
+        BW_WAIT(&bars->y_full[0], 0, PB_ERR_TIMEOUT_MMA);
+        pb::tc_fence_after();
+        issue_s(0);
+        issue_dp(0);
+        if (C::NSB == 2 && n_iter > 1) {
+          BW_WAIT(&bars->y_full[1], 0, PB_ERR_TIMEOUT_MMA);
+          pb::tc_fence_after();
+          issue_s(1);
+        }
+      } while (false);
+      for (int i = 0; i < n_iter && ok; ++i) {
+        // S of the next step (one S buffer) goes out at the first point at which its tile has arrived: the issuing thread
+        // must not wait for a load while P / dS of this step are ready
+        bool s_next = C::NSB == 2 || i + 1 >= n_iter;
+        uint64_t* y_next = &bars->y_full[(i + 1) % C::NS];
+        const uint32_t y_par = ((i + 1) / C::NS) & 1;
+        auto try_s = [&]() {
+          if (!s_next && mbar_test(y_next, y_par)) {
+            pb::tc_fence_after();
+            issue_s(i + 1);
+            s_next = true;
+          }
+        };
+        if (i + 1 < n_iter) {
+          BW_WAIT(&bars->freed, i & 1, PB_ERR_TIMEOUT_MMA);
+          pb::tc_fence_after();
+          if (C::NSB == 2) issue_dp(i + 1);
+          else try_s();
+        }
+        BW_WAIT(&bars->pa[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_MMA);
+        pb::tc_fence_after();
+        issue_second(i, 0);
+        try_s();
+        BW_WAIT(&bars->pb[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_MMA);
+        pb::tc_fence_after();
+        issue_second(i, 1);
+        if (C::NSB == 1) {
+          if (!s_next) {
+            BW_WAIT(y_next, y_par, PB_ERR_TIMEOUT_MMA);
+            pb::tc_fence_after();
+            issue_s(i + 1);
+          }
+          if (i + 1 < n_iter) issue_dp(i + 1);
+        } else if (i + 2 < n_iter) {
+          BW_WAIT(&bars->y_full[(i + 2) % C::NS], ((i + 2) / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
+          pb::tc_fence_after();
+          issue_s(i + 2);
+        }
+      }
+      if (ok) pb::umma_commit(&bars->acc_done);
+    }
+  } else {
+    // ------------------------------------------------------------------ softmax-gradient threads
+    const int wq = warp & 3;                      // TMEM lane quarter of this warp
+    const int qd = (warp - 2) >> 2;               // 16-column group of each half
+    const int row = wq * 32 + lane;
+    const uint32_t lane_addr = uint32_t(wq * 32) << 16;
+    const int row_g = rb * BR + row;
+    float lse2_row = 0.f, delta_row = 0.f;
+    if (MODE == MODE_DQ) {
+      const long off = ((long)batch * hq + xhead) * seq + row_g;
+      lse2_row = lse[off];  // negated, in log2 units
+      delta_row = delta[off];
+    }
+    const uint64_t sl2_2 = pb::pack_f32x2(sl2, sl2), minus_one = pb::pack_f32x2(-1.f, -1.f);
+    const uint64_t row_l2 = pb::pack_f32x2(lse2_row, lse2_row), row_delta = pb::pack_f32x2(delta_row, delta_row);
+    bool ok = true;
+    if (C::XA1 || C::XA2) {
+      // a thread copies 64 channels of its row of Q (groups 0, 1) or dO (groups 2, 3; 0, 1 when Q stays) from the
+      // 128-byte-swizzled tile: word w of a row (elements 2w, 2w + 1) goes to column w, the layout of a TMEM A operand
+      do {
+        BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);
+        const bool q_part = C::XA1 && qd < 2;
+        if (C::XA1 || qd < 2) {
+          const uint8_t* xs = (q_part ? x1_smem : x2_smem) + (qd & 1) * XATOM + row * 128;
+          uint32_t wds[32];
+#pragma unroll
+          for (int c = 0; c < 8; ++c) {
+            const uint4 v = *reinterpret_cast<const uint4*>(xs + ((c ^ (row & 7)) << 4));
+            wds[4 * c] = v.x; wds[4 * c + 1] = v.y; wds[4 * c + 2] = v.z; wds[4 * c + 3] = v.w;
+          }
+          pb::tmem_st_32x32b_x32(tmem_base + lane_addr + (q_part ? C::XA1_COL : C::XA2_COL) + (qd & 1) * 32, wds);
+          pb::tmem_wait_st();
+        }
+        pb::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) pb::mbar_arrive(&bars->xa_ready);
+      } while (false);
+    }
+    for (int i = 0; i < n_iter && ok; ++i) {
+      const int st = i % C::NS;
+      const int cs = c_start + i % n_per_head;
+      if (MODE == MODE_DKDV) {
+        BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
+      }
+      const uint32_t ts = tmem_base + lane_addr + C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0) + 16 * qd;
+      const uint32_t td = tmem_base + lane_addr + C::DP_COL + 16 * qd;
+      const uint32_t tout = C::NSB == 2 ? ts : td;
+      const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
+      const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BCW + BCW - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BCW);
+      const bool diag = (causal && cs_rel == rb) || (window > 0 && max_diff >= window);
+      const float* stat = stat_smem + st * C::STAT_FLOATS + 16 * qd;
+      BW_WAIT(&bars->s_full[C::NSB == 2 ? (i & 1) : 0], C::NSB == 2 ? ((i >> 1) & 1) : (i & 1), PB_ERR_TIMEOUT_EPILOGUE);
+      pb::tc_fence_after();
+      float p[32], dc[CAP ? 32 : 1];
+      {
+        uint32_t sr[32];
+        pb::tmem_ld_32x32b_x16(ts, sr);
+        pb::tmem_ld_32x32b_x16(ts + 64, sr + 16);
+        pb::tmem_wait_ld();
+        if (C::NSB == 1) {
+          pb::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) pb::mbar_arrive(&bars->freed);
+        }
+#pragma unroll
+        for (int e2 = 0; e2 < 32; e2 += 2) {
+          uint64_t l2 = row_l2;
+          if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(stat + (e2 >> 4) * 128 + (e2 & 15));
+          float s0 = __uint_as_float(sr[e2]), s1 = __uint_as_float(sr[e2 + 1]);
+          if (CAP) {
+            // the score is softcap * tanh(scale * s / softcap) / scale; dc: its derivative with respect to scale * s
+            const float t0 = pb::fast_tanh(s0 * cap_a), t1 = pb::fast_tanh(s1 * cap_a);
+            s0 = t0 * cap_b;
+            s1 = t1 * cap_b;
+            dc[e2] = 1.f - t0 * t0;
+            dc[e2 + 1] = 1.f - t1 * t1;
+          }
+          pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
+          p[e2] = pb::fast_exp2(p[e2]);
+          p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
+        }
+        if (diag) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) {
+            const int col_g = cs_rel * BCW + (e >> 4) * 64 + 16 * qd + (e & 15);
+            const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
+            if (diff < 0 || (window > 0 && diff >= window)) p[e] = 0.f;
+          }
+        }
+      }
+      BW_WAIT(&bars->dp_full, i & 1, PB_ERR_TIMEOUT_EPILOGUE);
+      pb::tc_fence_after();
+      uint32_t dp[32];
+      pb::tmem_ld_32x32b_x16(td, dp);
+      pb::tmem_ld_32x32b_x16(td + 64, dp + 16);
+      pb::tmem_wait_ld();
+      if (C::NSB == 2) {
+        pb::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) pb::mbar_arrive(&bars->freed);
+      }
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        uint32_t pk[16];                          // packed P (8), dS (8) of this thread's 16 columns
+#pragma unroll
+        for (int e2 = 0; e2 < 16; e2 += 2) {
+          const int e = half * 16 + e2;
+          uint64_t dl = row_delta;
+          if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(stat + half * 128 + 64 + e2);
+          const uint64_t pp = pb::pack_f32x2(p[e], p[e + 1]);
+          // dS = P (dP - delta), times the score scale, which the epilogue applies
+          uint64_t ds = pb::mul_f32x2(pp, pb::fma_f32x2(dl, minus_one, pb::pack_f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1]))));
+          if (CAP) ds = pb::mul_f32x2(ds, pb::pack_f32x2(dc[e], dc[e + 1]));
+          float d0, d1;
+          pb::unpack_f32x2(ds, d0, d1);
+          pk[e2 / 2] = pb::pack_bf16x2(p[e], p[e + 1]);
+          pk[8 + e2 / 2] = pb::pack_bf16x2(d0, d1);
+        }
+        if (MODE == MODE_DKDV) pb::tmem_st_32x32b_x16(tout + half * 64, pk);
+        else pb::tmem_st_32x32b_x8(tout + half * 64 + 8, pk + 8);
+        pb::tmem_wait_st();
+        pb::tc_fence_before();
+        __syncwarp();
+        if (lane == 0) pb::mbar_arrive(half == 0 ? &bars->pa[i & 1] : &bars->pb[i & 1]);
+      }
+    }
+    // ---- epilogue: accumulators -> bf16 -> (dead) resident tiles -> TMA store
+    do {
+      if (!ok) break;
+      BW_WAIT(&bars->acc_done, 0, PB_ERR_TIMEOUT_EPILOGUE);
+      BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);     // (long past, except for a block without a step)
+      pb::tc_fence_after();
+      uint8_t* o1_smem = C::XA1 ? y1_smem : x1_smem;          // all tiles have been consumed
+      auto drain = [&](uint32_t tcol, int ncols, uint8_t* dst, float mul) {
+#pragma unroll 1
+        for (int c = qd; c < ncols / 32; c += 4) {
+          uint32_t r[32];
+          pb::tmem_ld_32x32b_x32(tmem_base + lane_addr + tcol + c * 32, r);
+          pb::tmem_wait_ld();
+          if (n_iter == 0) {                      // nothing was accumulated: the columns are undefined
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[e] = 0u;
+          }
+          uint8_t* atom = dst + (c >> 1) * XATOM + row * 128;
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint32_t w[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+              w[u] = pb::pack_bf16x2(__uint_as_float(r[8 * q4 + 2 * u]) * mul, __uint_as_float(r[8 * q4 + 2 * u + 1]) * mul);
+            const int chunk = (c & 1) * 4 + q4;
+            *reinterpret_cast<uint4*>(atom + ((chunk ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      };
+      drain(0, DQK, o1_smem, scale);
+      if (MODE == MODE_DKDV) drain(DQK, DV, x2_smem, 1.f);
+      pb::fence_proxy_async_smem();
+      pb::named_bar_sync(1, 32 * BWW_WARPS);
+      if (threadIdx.x == 64) {
+#pragma unroll
+        for (int a = 0; a < DQK / 64; ++a) pb::tma_store_3d(&tmO1, o1_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
+        if (MODE == MODE_DKDV) {
+#pragma unroll
+          for (int a = 0; a < DV / 64; ++a) pb::tma_store_3d(&tmO2, x2_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
+        }
+        pb::tma_store_commit();
+        pb::tma_store_wait_all<0>();
+      }
+    } while (false);
+  }
+
+  if (*abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(2000);
+  }
+  pb::tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    pb::tc_fence_after();
+    pb::tmem_dealloc<1>(tmem_base, 512);
+  }
+}
+
+// delta[b, h, s] = sum_d dO * O ;  neg_lse2 = -lse * log2(e) (the addend of the main kernels' exponent).
 // A CTA takes 32 positions x 8 heads.  DV / 8 lanes share a (position, head) row, neighbouring rows of the same position
 // are neighbours in memory, so a warp reads whole 128-byte lines; the 32 sums of a head then leave as one 128-byte line.
 constexpr int DL_POS = 32, DL_HEADS = 8, DL_THREADS = 256;
 template <int DV>
 __global__ void __launch_bounds__(DL_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                  const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ lse2, int seq, int hq,
+                  const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ neg_lse2, int seq, int hq,
                   long o_row, long do_row) {
   constexpr int LANES = DV / 8;
   constexpr int GROUPS = DL_THREADS / LANES;
@@ -501,7 +948,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
     const long b = t0 / seq;
     const long off = (b * hq + h) * seq + (t0 - b * seq) + p;
     delta[off] = sums[threadIdx.x / DL_POS][p];
-    lse2[off] = lse[off] * 1.4426950408889634f;
+    neg_lse2[off] = lse[off] * -1.4426950408889634f;
   }
 }
 
@@ -561,41 +1008,43 @@ int launch_bwd(const BwdArgs& a) {
   MK(dq_m, a.dq, T, a.hq, DQK, a.dq_row, 128) MK(dk_m, a.dk, TK, a.hkv, DQK, a.dk_row, 128)
   MK(dv_m, a.dv, TK, a.hkv, DV, a.dv_row, 128)
 #undef MK
-  {
-    using C = BwCfg<DQK, DV, MODE_DKDV>;
-    auto kern = (a.window > 0 || a.softcap > 0.f) ? flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, true> : flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, false>;
-    static bool attr_set[2] = {false, false};
-    if (!attr_set[a.window > 0 || a.softcap > 0.f]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-      if (e != cudaSuccess) return (int)e;
-      attr_set[a.window > 0 || a.softcap > 0.f] = true;
-    }
-    dim3 grid(a.hkv * a.batch, a.seq_k / BR, 1);
-    kern<<<grid, BW_THREADS, C::SMEM_BYTES, a.stream>>>(k128, v128, q64, do64, dk_m, dv_m,
-                                                       a.delta + (long)a.batch * a.hq * a.seq, a.delta, a.seq, a.seq_k,
-                                                       a.q_off, a.hq, a.hkv, a.scale, a.causal, a.window, a.softcap, a.status);
+  const int var = a.softcap > 0.f ? 2 : (a.window > 0 ? 1 : 0);
+  const float* lse2 = a.delta + (long)a.batch * a.hq * a.seq;
+  const dim3 grid_kv(a.hkv * a.batch, a.seq_k / BR, 1), grid_q(a.hq * a.batch, a.seq / BR, 1);
+#define PB_BWD(KERN, CFG, THREADS, GRID, X1, X2, Y1, Y2, O1, O2)                                                        \
+  {                                                                                                                     \
+    static bool attr_set[3] = {false, false, false};                                                                    \
+    auto kern = KERN;                                                                                                   \
+    if (!attr_set[var]) {                                                                                               \
+      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES);         \
+      if (e != cudaSuccess) return (int)e;                                                                              \
+      attr_set[var] = true;                                                                                             \
+    }                                                                                                                   \
+    kern<<<GRID, THREADS, CFG::SMEM_BYTES, a.stream>>>(X1, X2, Y1, Y2, O1, O2, lse2, a.delta, a.seq, a.seq_k, a.q_off, a.hq, \
+                                                       a.hkv, a.scale, a.causal, a.window, a.softcap, a.status);        \
   }
-  {
-    using C = BwCfg<DQK, DV, MODE_DQ>;
-    auto kern = (a.window > 0 || a.softcap > 0.f) ? flash_attn_bwd_kernel<DQK, DV, MODE_DQ, true> : flash_attn_bwd_kernel<DQK, DV, MODE_DQ, false>;
-    static bool attr_set[2] = {false, false};
-    if (!attr_set[a.window > 0 || a.softcap > 0.f]) {
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-      if (e != cudaSuccess) return (int)e;
-      attr_set[a.window > 0 || a.softcap > 0.f] = true;
-    }
-    dim3 grid(a.hq * a.batch, a.seq / BR, 1);
-    kern<<<grid, BW_THREADS, C::SMEM_BYTES, a.stream>>>(q128, do128, k64, v64, dq_m, dq_m,
-                                                       a.delta + (long)a.batch * a.hq * a.seq, a.delta, a.seq, a.seq_k,
-                                                       a.q_off, a.hq, a.hkv, a.scale, a.causal, a.window, a.softcap, a.status);
+  if constexpr (DQK == DV) {
+    using CKV = BwWideCfg<DQK, DV, MODE_DKDV>;
+    PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 2>
+            : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 0>),
+           CKV, BWW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
+  } else {
+    using CKV = BwCfg<DQK, DV, MODE_DKDV>;
+    PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, true> : flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, false>), CKV,
+           BW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
   }
+  using CQ = BwWideCfg<DQK, DV, MODE_DQ>;
+  PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 2>
+          : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 0>),
+         CQ, BWW_THREADS, grid_q, q128, do128, k64, v64, dq_m, dq_m)
+#undef PB_BWD
   return (int)cudaGetLastError();
 }
 
 }  // namespace
 
 // Layouts as in pb_flash_attn_fwd_ex (q / o / d_o / dq: batch*seq rows; k / v / dk / dv: batch*seq_k rows).
-// delta: fp32 scratch [2, batch, hq, seq] (written here: row sums of dO*O, then the log-sum-exp in log2 units).
+// delta: fp32 scratch [2, batch, hq, seq] (written here: row sums of dO*O, then minus the log-sum-exp in log2 units).
 extern "C" int pb_flash_attn_bwd_cap(const void* d_o, const void* q, const void* k, const void* v, const void* o,
                                      const float* lse, float* delta, void* dq, void* dk, void* dv, int batch, int seq,
                                      int seq_k, int q_off, int hq, int hkv, int d_qk, int d_v, long q_row, long k_row,
