@@ -325,13 +325,33 @@ __device__ __forceinline__ void store4(__nv_bfloat16* p, const float* o) {
 __device__ __forceinline__ void store1(float* p, float o) { *p = o; }
 __device__ __forceinline__ void store1(__nv_bfloat16* p, float o) { *p = __float2bfloat16(o); }
 
+// a / b for a loop-invariant b whose correctly rounded reciprocal r the host supplies: a quotient estimate, its exact
+// remainder (fma) and one correction give the correctly rounded quotient (P. Markstein, "Computation of elementary functions
+// on the IBM RISC System/6000 processor", 1990).  An infinite estimate is the quotient already.
+__device__ __forceinline__ float div_invariant(float a, float b, float r) {
+  const float q = a * r;
+  const float c = fmaf(fmaf(-q, b, a), r, q);
+  return fabsf(q) < INFINITY ? c : q;
+}
+
+// The two bias corrections are the same for all elements; dividing by them with the general division made the update bound
+// by its three divisions (895 us for 105 M elements, 3.5 TB/s, against 541 us without any).
+__device__ __forceinline__ void adamw_update(float& p, float& m, float& v, float g, float lr, float beta1, float beta2,
+                                             float eps, float wd, float bc1, float bc2, float ic1, float ic2) {
+  m = beta1 * m + (1.f - beta1) * g;
+  v = beta2 * v + (1.f - beta2) * g * g;
+  const float mh = div_invariant(m, bc1, ic1);
+  const float vh = div_invariant(v, bc2, ic2);
+  p = p * (1.f - lr * wd) - lr * mh / (sqrtf(vh) + eps);
+}
+
 // GradT: fp32 or bf16 gradients; StateT: fp32 or bf16 moments (precision-aware optimizer: the moments can be kept in
 // bf16 to halve their memory; the arithmetic is fp32 either way and the master weights stay fp32).
 template <typename GradT, typename StateT>
 __global__ void adamw_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v,
                              const GradT* __restrict__ grad, __nv_bfloat16* __restrict__ param_out,
                              long n, float lr, float beta1, float beta2, float eps, float wd,
-                             float bc1, float bc2, const float* __restrict__ grad_scale,
+                             float bc1, float bc2, float ic1, float ic2, const float* __restrict__ grad_scale,
                              const int* __restrict__ skip) {
   if (skip && *skip) return;
   const float gs = grad_scale ? *grad_scale : 1.f;
@@ -354,14 +374,7 @@ __global__ void adamw_kernel(float* __restrict__ master, StateT* __restrict__ m,
       }
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float gg = g[j] * gs;
-      mm[j] = beta1 * mm[j] + (1.f - beta1) * gg;
-      vv[j] = beta2 * vv[j] + (1.f - beta2) * gg * gg;
-      const float mh = mm[j] / bc1;
-      const float vh = vv[j] / bc2;
-      p[j] = p[j] * (1.f - lr * wd) - lr * mh / (sqrtf(vh) + eps);
-    }
+    for (int j = 0; j < 4; ++j) adamw_update(p[j], mm[j], vv[j], g[j] * gs, lr, beta1, beta2, eps, wd, bc1, bc2, ic1, ic2);
     if (full) {
       store4(master + i, p);
       store4(m + i, mm);
@@ -378,15 +391,107 @@ __global__ void adamw_kernel(float* __restrict__ master, StateT* __restrict__ m,
   }
 }
 
-// partial[b] = sum of squares handled by block b (deterministic two-stage reduction)
+// AdamW over one bucket in one launch.  The bucket is cut into ranges with their own weight-decay multiplier and learning
+// rate (norm gains without decay between matrices with it: one launch per range left the SMs idle around every small one);
+// range r starts at starts[r] (element 0 first, all multiples of 4) and uses wd * mult[r] and lrs.v[group[r]].  A CTA takes
+// a contiguous chunk whose first range the host has looked up; its threads walk on from there, after their loads are issued.
+constexpr int ADAMW_CHUNK = 8192;
+struct AdamWRates {
+  float v[4];
+};
+template <typename GradT, typename StateT>
+__global__ void __launch_bounds__(256, 5)
+adamw_ranges_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v,
+                    const GradT* __restrict__ grad, __nv_bfloat16* __restrict__ param_out, long n,
+                    const int* __restrict__ first, const long* __restrict__ starts, const float* __restrict__ mult,
+                    const int* __restrict__ group, int R, AdamWRates lrs, float beta1, float beta2, float eps, float wd,
+                    float bc1, float bc2, float ic1, float ic2, const float* __restrict__ grad_scale,
+                    const int* __restrict__ skip) {
+  if (skip && *skip) return;
+  const long c0 = (long)blockIdx.x * ADAMW_CHUNK, c1 = min(n, c0 + ADAMW_CHUNK);
+  int r = first[blockIdx.x];
+  const float gs = grad_scale ? *grad_scale : 1.f;
+  long end = r + 1 < R ? starts[r + 1] : n;
+  float lr = lrs.v[group[r]], rwd = wd * mult[r];
+  for (long i = c0 + threadIdx.x * 4; i < c1; i += 256 * 4) {
+    float p[4], mm[4], vv[4], g[4];
+    const bool full = i + 4 <= n;
+    if (full) {
+      load4(master + i, p);
+      load4(m + i, mm);
+      load4(v + i, vv);
+      load4(grad + i, g);
+    } else {
+      for (int j = 0; j < 4; ++j) {
+        const bool in = i + j < n;
+        p[j] = in ? master[i + j] : 0.f;
+        mm[j] = in ? (float)m[i + j] : 0.f;
+        vv[j] = in ? (float)v[i + j] : 0.f;
+        g[j] = in ? (float)grad[i + j] : 0.f;
+      }
+    }
+    if (i >= end) {
+      do {
+        ++r;
+        end = r + 1 < R ? starts[r + 1] : n;
+      } while (i >= end);
+      lr = lrs.v[group[r]];
+      rwd = wd * mult[r];
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) adamw_update(p[j], mm[j], vv[j], g[j] * gs, lr, beta1, beta2, eps, rwd, bc1, bc2, ic1, ic2);
+    if (full) {
+      store4(master + i, p);
+      store4(m + i, mm);
+      store4(v + i, vv);
+      store4(param_out + i, p);
+    } else {
+      for (int j = 0; j < 4 && i + j < n; ++j) {
+        master[i + j] = p[j];
+        store1(m + i + j, mm[j]);
+        store1(v + i + j, vv[j]);
+        param_out[i + j] = __float2bfloat16(p[j]);
+      }
+    }
+  }
+}
+
+// partial[b] = sum of squares handled by block b (deterministic two-stage reduction).  Four 16-byte loads per thread and
+// step; the elements in front of the first 16-byte boundary and behind the last go to block 0.
 template <typename T>
 __global__ void __launch_bounds__(512) sumsq_partial_kernel(const T* __restrict__ x, long n,
                                                            float* __restrict__ partial) {
   __shared__ float red[32];
-  float s = 0.f;
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
-    const float f = (float)x[i];
-    s += f * f;
+  constexpr int PER = 16 / sizeof(T);
+  const long mis = (long)((reinterpret_cast<uintptr_t>(x) & 15) / sizeof(T));
+  const long head = min(mis ? PER - mis : 0L, n);
+  const long nv = (n - head) / PER, tail0 = head + nv * PER;
+  const uint4* xv = reinterpret_cast<const uint4*>(x + head);
+  float a[4] = {0.f, 0.f, 0.f, 0.f};
+  auto add = [&](const uint4& q, float& s) {
+    if (sizeof(T) == 4) {
+      const float f[4] = {__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s += f[j] * f[j];
+    } else {
+      float f[8];
+      bf8_to_f(*reinterpret_cast<const Bf8*>(&q), f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) s += f[j] * f[j];
+    }
+  };
+  const long stride = (long)gridDim.x * 512;
+  for (long i = blockIdx.x * 512L + threadIdx.x; i < nv; i += 4 * stride) {
+    uint4 q[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) q[u] = i + u * stride < nv ? xv[i + u * stride] : make_uint4(0, 0, 0, 0);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) add(q[u], a[u]);
+  }
+  float s = (a[0] + a[1]) + (a[2] + a[3]);
+  if (blockIdx.x == 0) {
+    for (long j = threadIdx.x; j < head; j += 512) s += (float)x[j] * (float)x[j];
+    for (long j = tail0 + threadIdx.x; j < n; j += 512) s += (float)x[j] * (float)x[j];
   }
   s = block_sum<512>(s, red);
   if (threadIdx.x == 0) partial[blockIdx.x] = s;
@@ -542,7 +647,32 @@ int pb_adamw_ex(float* master, void* m, void* v, const void* grad, int grad_is_b
   __nv_bfloat16* po = (__nv_bfloat16*)param_out;
 #define PB_ADAMW(GT, ST)                                                                                          \
   adamw_kernel<GT, ST><<<g, 256, 0, s>>>(master, (ST*)m, (ST*)v, (const GT*)grad, po, n, lr, beta1, beta2, eps, wd, \
-                                         bc1, bc2, grad_scale, skip)
+                                         bc1, bc2, (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
+  if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
+  else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
+  else if (state_is_bf16) PB_ADAMW(float, __nv_bfloat16);
+  else PB_ADAMW(float, float);
+#undef PB_ADAMW
+  PB_CHECK_LAUNCH();
+}
+
+// One bucket: ranges r = 0 .. R - 1 start at starts[r] (device, int64; starts[0] = 0, ascending multiples of 4) and use
+// weight decay wd * mult[r] and learning rate lr[group[r]] (four rates); first[c]: the range that element
+// c * pb_adamw_ranges_chunk() lies in.  param_out: bf16.
+int pb_adamw_ranges_chunk() { return ADAMW_CHUNK; }
+
+int pb_adamw_ranges(float* master, void* m, void* v, const void* grad, int grad_is_bf16, int state_is_bf16,
+                    void* param_out, long n, const int* first, const long* starts, const float* mult, const int* group, int R, float lr0,
+                    float lr1, float lr2, float lr3, float beta1, float beta2, float eps, float wd, float bc1, float bc2,
+                    const float* grad_scale, const int* skip, cudaStream_t s) {
+  if (n == 0) return 0;
+  if (R <= 0 || param_out == nullptr) return -2;
+  const AdamWRates lrs{{lr0, lr1, lr2, lr3}};
+  const unsigned g = (unsigned)((n + ADAMW_CHUNK - 1) / ADAMW_CHUNK);
+  __nv_bfloat16* po = (__nv_bfloat16*)param_out;
+#define PB_ADAMW(GT, ST)                                                                                                  \
+  adamw_ranges_kernel<GT, ST><<<g, 256, 0, s>>>(master, (ST*)m, (ST*)v, (const GT*)grad, po, n, first, starts, mult, group, R, lrs, \
+                                                beta1, beta2, eps, wd, bc1, bc2, (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
   if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
   else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
   else if (state_is_bf16) PB_ADAMW(float, __nv_bfloat16);

@@ -50,6 +50,31 @@ def adamw_step_(master, exp_avg, exp_avg_sq, grad, param_out, *, lr, beta1, beta
               grad_scale, skip)
 
 
+def range_table(ranges, start: int, n: int, device):
+    """Device table of a bucket of ``n`` elements with the ranges ``[(lo, hi, weight-decay multiplier, learning-rate
+    group)]`` (consecutive, from ``start``; ``lo`` multiples of 4 relative to it) for :func:`adamw_ranges_`."""
+    starts = torch.tensor([r[0] - start for r in ranges], dtype=torch.int64)
+    chunk = _lib.call_ret("adamw_ranges_chunk")
+    first = torch.searchsorted(starts, torch.arange(0, n, chunk), right=True) - 1
+    return (first.to(torch.int32).to(device), starts.to(device),
+            torch.tensor([float(r[2]) for r in ranges], dtype=torch.float32).to(device),
+            torch.tensor([int(r[3]) for r in ranges], dtype=torch.int32).to(device))
+
+
+def adamw_ranges_(master, exp_avg, exp_avg_sq, grad, param_out, table, *, lrs, beta1, beta2, eps, weight_decay, step,
+                  grad_scale=None, skip=None):
+    """:func:`adamw_step_` of a whole bucket whose ranges differ in weight decay and learning rate, in one launch (CUDA
+    tensors, bf16 ``param_out``).  ``table``: see :func:`range_table`; ``lrs``: the rates of groups 0 to 3."""
+    n = master.numel()
+    assert master.dtype == torch.float32 and master.is_contiguous() and master.data_ptr() % 16 == 0
+    assert grad.numel() == n and grad.is_contiguous() and exp_avg.dtype == exp_avg_sq.dtype
+    assert param_out.dtype == torch.bfloat16 and param_out.numel() == n and len(lrs) == 4
+    _lib.call("adamw_ranges", master, exp_avg, exp_avg_sq, grad, int(grad.dtype == torch.bfloat16),
+              int(exp_avg.dtype == torch.bfloat16), param_out, n, *table, table[1].numel(), *[float(x) for x in lrs],
+              float(beta1), float(beta2), float(eps), float(weight_decay), float(1.0 - beta1 ** step),
+              float(1.0 - beta2 ** step), grad_scale, skip)
+
+
 def sumsq_(x, out, accumulate=False, nonfinite=None):
     """out[0] (+)= sum(x^2) in fp32 (deterministic two-stage reduction)."""
     if not x.is_cuda:

@@ -412,6 +412,7 @@ class DistributedOptimizer:
                 self.state.append(dict(buf=buf, bucket=b, s=s, e=e, master=master,
                                        m=torch.zeros_like(master, dtype=state_dtype),
                                        v=torch.zeros_like(master, dtype=state_dtype), wd_ranges=wd_ranges,
+                                       range_table=self._range_table(buf, s, e, wd_ranges),
                                        dup_ranges=self._tp_duplicate_ranges(buf, b, s, e) if self.tp_size > 1 else []))
         self.sumsq = torch.zeros(1, dtype=torch.float32, device=dev)
         self.sumsq_part = torch.zeros(1, dtype=torch.float32, device=dev)
@@ -447,6 +448,15 @@ class DistributedOptimizer:
             else:
                 merged.append(r)
         return merged
+
+    @staticmethod
+    def _range_table(buf, s, e, ranges):
+        """Device table for the one-launch update of a shard; None where a range does not fit it."""
+        if buf.device.type != "cuda" or buf.param_dtype != torch.bfloat16 or not ranges:
+            return None
+        if any(not 0 <= grp < 4 or (lo - s) % 4 for lo, _, _, grp in ranges):
+            return None
+        return optim_ops.range_table(ranges, s, e - s, buf.device)
 
     @staticmethod
     def _tp_duplicate_ranges(buf, b, s, e):
@@ -608,7 +618,15 @@ class DistributedOptimizer:
         base_lr = lr
         for st in self.state:
             buf = st["buf"]
-            for lo, hi, mult, grp in st["wd_ranges"]:
+            ranges = st["wd_ranges"]
+            if st.get("range_table") is not None:
+                optim_ops.adamw_ranges_(st["master"], st["m"], st["v"], buf.grad_data[st["s"]:st["e"]],
+                                        buf.param_data[st["s"]:st["e"]], st["range_table"],
+                                        lrs=[self._group_lr.get(g, base_lr) for g in range(4)], beta1=self.betas[0],
+                                        beta2=self.betas[1], eps=self.eps, weight_decay=wd, step=self.step_count,
+                                        grad_scale=self.coef, skip=self.skip)
+                continue
+            for lo, hi, mult, grp in ranges:
                 lr = self._group_lr.get(grp, base_lr)
                 a, b_ = lo - st["s"], hi - st["s"]
                 out = buf.param_data[lo:hi] if buf.param_dtype == torch.bfloat16 else None

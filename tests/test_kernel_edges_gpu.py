@@ -149,3 +149,67 @@ def test_sink_gradient_matches_oracle(batch, S, hq, hkv):
     ds = attention.flash_attn_bwd(do, q, k, v, o, lse, batch, True, 0.125, sinks=sinks)[3]
     ref = attention.sink_grad(do, o, lse, sinks, batch)
     assert (ds - ref).abs().max() <= 1e-4 * (1 + ref.abs().max())
+
+
+@pytest.mark.parametrize("n,off", [(1, 0), (3, 1), (4099, 3), (2 ** 20 + 5, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_sumsq_ragged_and_misaligned(n, off, dtype):
+    x = torch.randn(n + off, device="cuda", generator=_gen(n)).to(dtype)[off:]
+    out = torch.zeros(1, device="cuda")
+    optim.sumsq_(x, out)
+    ref = x.double().pow(2).sum().item()
+    assert abs(out.item() - ref) <= 1e-5 * ref
+
+
+@pytest.mark.parametrize("cuts", [[0], [0, 4, 8, 8192, 8196, 20000], [0, 8188, 16384]])
+@pytest.mark.parametrize("state", [torch.float32, torch.bfloat16])
+def test_adamw_ranges_match_one_launch_per_range(cuts, state):
+    n, g = 24604, _gen(len(cuts))
+    ranges = [(100 + a, 100 + b, float(i % 2), i % 4) for i, (a, b) in enumerate(zip(cuts, cuts[1:] + [n]))]
+    lrs = [1e-2, 2e-3, 5e-3, 1e-3]
+    hyper = dict(beta1=0.9, beta2=0.95, eps=1e-8, step=3, grad_scale=torch.full((1,), 0.7, device="cuda"))
+
+    def fresh():
+        g.manual_seed(1)
+        t = [torch.randn(n, device="cuda", generator=g) for _ in range(3)]
+        v = torch.rand(n, device="cuda", generator=g)
+        return t[0], t[1].to(state), v.to(state), t[2], torch.zeros(n, device="cuda", dtype=torch.bfloat16)
+
+    p, m, v, grad, out = fresh()
+    p64, m64, v64, g64 = p.double(), m.double(), v.double(), grad.double() * 0.7
+    optim.adamw_ranges_(p, m, v, grad, out, optim.range_table(ranges, 100, n, "cuda"), lrs=lrs, weight_decay=0.1, **hyper)
+    p2, m2, v2, grad, out2 = fresh()
+    upd = torch.zeros_like(p64)
+    for lo, hi, mult, grp in ranges:
+        sl = slice(lo - 100, hi - 100)
+        optim.adamw_step_(p2[sl], m2[sl], v2[sl], grad[sl], out2[sl], lr=lrs[grp], weight_decay=0.1 * mult, **hyper)
+        mm, vv = 0.9 * m64[sl] + 0.1 * g64[sl], 0.95 * v64[sl] + 0.05 * g64[sl] ** 2
+        upd[sl] = lrs[grp] * (mm / (1 - 0.9 ** 3)) / ((vv / (1 - 0.95 ** 3)).sqrt() + 1e-8)
+        p64[sl] = p64[sl] * (1 - lrs[grp] * 0.1 * mult) - upd[sl]
+    for a, b in ((p, p2), (m, m2), (v, v2), (out, out2)):
+        assert torch.equal(a, b)
+    # fp32 rounding of p and of the update: a few ulp of either; m is a sum that may cancel (0.1 |m| + 0.1 |g| in fp32)
+    scale = upd.abs() + max(lrs) * (m64.abs() + g64.abs()) / v64.sqrt().clamp_min(1e-3)
+    assert ((p.double() - p64).abs() <= 2.0 ** -22 * (p64.abs() + scale)).all()
+
+
+@pytest.mark.parametrize("V", [8, 4088, 16384, 16392, 53248, 53256, 106504, 128256])
+def test_cross_entropy_masked_and_ragged(V):
+    """Rows with -inf and lowest-value masks (a row of nothing but the lowest value has no fp32 log-sum-exp)."""
+    g = _gen(V)
+    T = 9
+    x = (torch.randn(T, V, device="cuda", generator=g) * 4).bfloat16()
+    low = torch.finfo(torch.bfloat16).min
+    x[1, 1:] = float("-inf")
+    x[2, : V - 1] = low
+    x[4, V // 2:] = low
+    lab = torch.randint(0, V, (T,), device="cuda", generator=g)
+    lab[1], lab[2], lab[4] = 0, V - 1, 0
+    ref = x.double().requires_grad_()
+    loss64 = torch.nn.functional.cross_entropy(ref, lab, reduction="none")
+    loss64.sum().backward()
+    xl = x.clone().requires_grad_()
+    loss = fused.cross_entropy(xl * 1.0, lab)
+    loss.sum().backward()
+    assert (loss.double() - loss64).abs().max() <= 1e-5 * (1 + loss64.abs().max())
+    _close_bf16(xl.grad, ref.grad, "dlogits")
