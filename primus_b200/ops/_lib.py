@@ -54,22 +54,34 @@ def require():
 _PTR = ctypes.c_void_p
 
 
-def _conv(a):
-    if a is None:
-        return _PTR(0)
-    if isinstance(a, torch.Tensor):
-        return _PTR(a.data_ptr())
-    if isinstance(a, bool):
-        return ctypes.c_int(int(a))
-    if isinstance(a, int):
-        return ctypes.c_long(a)
-    if isinstance(a, float):
-        return ctypes.c_float(a)
-    return a
-
-
 def stream_ptr() -> ctypes.c_void_p:
     return _PTR(torch.cuda.current_stream().cuda_stream)
+
+
+def _ctype(a):
+    """C type an argument travels as: tensors and None are pointers, integers 64-bit (a launcher's 32-bit parameter reads
+    the low half of the register), floats single precision; ctypes instances keep their own type."""
+    if a is None or isinstance(a, torch.Tensor):
+        return _PTR
+    if isinstance(a, int):
+        return ctypes.c_long
+    if isinstance(a, float):
+        return ctypes.c_float
+    return type(a)
+
+
+# Launchers bound so far: name -> (function with its argument types set from the first call, kernels per call).  ctypes then
+# converts plain integers and floats itself; wrapping every argument of every call in a ctypes object cost more than the
+# launch for the 20-argument launchers.
+_BOUND: dict = {}
+
+
+def _bind(name: str, args, stream: bool):
+    fn = load()["pb_" + name]       # an object of its own: argument types set here are not seen by other users
+    fn.restype = ctypes.c_int
+    fn.argtypes = [_ctype(a) for a in args] + ([_PTR] if stream else [])
+    _BOUND[name, stream] = bound = (fn, _KERNELS_PER_CALL.get(name, 1))
+    return bound
 
 
 # Number of device kernels each launcher enqueues (default 1); used for the launch counter below.
@@ -81,19 +93,18 @@ LAUNCH_COUNT = 0
 def call(name: str, *args) -> None:
     """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended."""
     global LAUNCH_COUNT
-    fn = getattr(load(), "pb_" + name)
-    fn.restype = ctypes.c_int
-    LAUNCH_COUNT += _KERNELS_PER_CALL.get(name, 1)
-    rc = fn(*[_conv(a) for a in args], stream_ptr())
+    fn, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
+    LAUNCH_COUNT += kernels
+    rc = fn(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args],
+            torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
     if rc != 0:
         raise NativeLibraryError(f"pb_{name} failed with code {rc}")
 
 
 def call_ret(name: str, *args) -> int:
     """Invoke a host-only helper that returns a value (no stream appended)."""
-    fn = getattr(load(), "pb_" + name)
-    fn.restype = ctypes.c_int
-    return fn(*[_conv(a) for a in args])
+    fn, _ = _BOUND.get((name, False)) or _bind(name, args, False)
+    return fn(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args])
 
 
 class I32(int):
