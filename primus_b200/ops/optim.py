@@ -8,6 +8,7 @@ trainer_base.yaml:72-118).
 """
 from __future__ import annotations
 
+import numpy as np
 import torch
 
 from . import _lib
@@ -53,12 +54,14 @@ def adamw_step_(master, exp_avg, exp_avg_sq, grad, param_out, *, lr, beta1, beta
 def range_table(ranges, start: int, n: int, device):
     """Device table of a bucket of ``n`` elements with the ranges ``[(lo, hi, weight-decay multiplier, learning-rate
     group)]`` (consecutive, from ``start``; ``lo`` multiples of 4 relative to it) for :func:`adamw_ranges_`."""
-    starts = torch.tensor([r[0] - start for r in ranges], dtype=torch.int64)
-    chunk = _lib.call_ret("adamw_ranges_chunk")
-    first = torch.searchsorted(starts, torch.arange(0, n, chunk), right=True) - 1
-    return (first.to(torch.int32).to(device), starts.to(device),
-            torch.tensor([float(r[2]) for r in ranges], dtype=torch.float32).to(device),
-            torch.tensor([int(r[3]) for r in ranges], dtype=torch.int32).to(device))
+    R, chunk = len(ranges), _lib.call_ret("adamw_ranges_chunk")
+    starts = np.array([r[0] - start for r in ranges], dtype=np.int64)
+    first = np.searchsorted(starts, np.arange(0, n, chunk), side="right") - 1
+    # one buffer, one copy to the device: starts (8 bytes each), multipliers, groups, first ranges (4 bytes each)
+    buf = np.concatenate([starts.view(np.int32), np.array([r[2] for r in ranges], dtype=np.float32).view(np.int32),
+                          np.array([r[3] for r in ranges], dtype=np.int32), first.astype(np.int32)])
+    t = torch.from_numpy(buf).to(device)
+    return t[4 * R:], t[:2 * R].view(torch.int64), t[2 * R:3 * R].view(torch.float32), t[3 * R:4 * R]
 
 
 def adamw_ranges_(master, exp_avg, exp_avg_sq, grad, param_out, table, *, lrs, beta1, beta2, eps, weight_decay, step,
