@@ -1,13 +1,11 @@
-// Memory-bound training ops for sm_100a: RMSNorm (fwd/bwd, optional fused residual add), RoPE,
-// SwiGLU (plain / routing-prob weighted / clamped), cross-entropy (fused softmax + gradient,
-// vocab-parallel capable), AdamW on flat buffers, L2-norm / scale helpers.
+// Memory-bound training ops for sm_100a: RoPE, SwiGLU (plain / routing-prob weighted / clamped), cross-entropy (fused
+// softmax + gradient, vocab-parallel capable), AdamW on flat buffers, L2-norm / scale helpers, MoE row movement.  (RMSNorm:
+// csrc/rmsnorm.cu.)
 //
 // All kernels move 16 bytes per thread per access and keep fp32 math in registers; each is one
 // pass over its operands except where a row statistic forces a second read (which hits L1/L2).
 //
-// Reference call sites these replace: rmsnorm / fused residual norm
-// (primus/backends/megatron/core/extensions/primus_turbo.py:1697-1700, fused_residual_rmsnorm.py),
-// TE fused RoPE and bias-SwiGLU (primus/backends/megatron/patches/te_patches/
+// Reference call sites these replace: TE fused RoPE and bias-SwiGLU (primus/backends/megatron/patches/te_patches/
 // fused_bias_swiglu_patches.py:21), swiglu_with_probs (primus_turbo.py:1954-1980), clamped SwiGLU
 // (primus/backends/megatron/core/fusions/fused_bias_swiglu.py:25-100), TE cross-entropy fusion
 // and FusedAdam (primus/backends/megatron/patches/torch_fused_adam_patches.py:40-88).

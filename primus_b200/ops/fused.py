@@ -1,4 +1,4 @@
-"""Autograd wrappers of the memory-bound sm_100a kernels in ``csrc/elementwise.cu``:
+"""Autograd wrappers of the memory-bound sm_100a kernels in ``csrc/elementwise.cu`` and ``csrc/rmsnorm.cu``:
 RMSNorm (optionally fused with the residual add), RoPE, SwiGLU (plain / probs-weighted / clamped),
 cross-entropy (fused forward+gradient, vocab-parallel) and the embedding gradient.
 
