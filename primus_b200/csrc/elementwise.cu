@@ -454,45 +454,72 @@ adamw_ranges_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* 
   }
 }
 
-// partial[b] = sum of squares handled by block b (deterministic two-stage reduction).  Four 16-byte loads per thread and
-// step; the elements in front of the first 16-byte boundary and behind the last go to block 0.
-template <typename T>
-__global__ void __launch_bounds__(512) sumsq_partial_kernel(const T* __restrict__ x, long n,
-                                                           float* __restrict__ partial) {
-  __shared__ float red[32];
-  constexpr int PER = 16 / sizeof(T);
-  const long mis = (long)((reinterpret_cast<uintptr_t>(x) & 15) / sizeof(T));
-  const long head = min(mis ? PER - mis : 0L, n);
-  const long nv = (n - head) / PER, tail0 = head + nv * PER;
-  const uint4* xv = reinterpret_cast<const uint4*>(x + head);
-  float a[4] = {0.f, 0.f, 0.f, 0.f};
-  auto add = [&](const uint4& q, float& s) {
-    if (sizeof(T) == 4) {
-      const float f[4] = {__uint_as_float(q.x), __uint_as_float(q.y), __uint_as_float(q.z), __uint_as_float(q.w)};
+// partial[b] = sum of squares handled by block b (deterministic two-stage reduction).  The order of the additions is fixed
+// and part of the result (the clip coefficient, and with it the whole optimizer state, moves with the last bit of the norm):
+// SUMSQ_CHAINS serial sums, chain j over the elements j, j + SUMSQ_CHAINS, ... in turn; the 512 chains of a block meet in
+// a butterfly over 32 neighbours (distances 16, 8, 4, 2, 1) and one over the 16 results.
+// What bounds it is the bytes in flight.  A thread therefore owns PER neighbouring chains, whose elements are one 16-byte
+// load, with U of them issued before the first is added, and a block is 512 / PER threads; the butterfly steps whose
+// distance is below PER are additions inside a thread.  A start off a 16-byte boundary takes element loads, in the same
+// order.
+constexpr int SUMSQ_BLOCKS = 1184, SUMSQ_BLOCK_CHAINS = 512;
+constexpr long SUMSQ_CHAINS = (long)SUMSQ_BLOCKS * SUMSQ_BLOCK_CHAINS;
+
+__device__ __forceinline__ void sumsq_unpack(const float* p, float (&f)[4]) {
+  const float4 q = *reinterpret_cast<const float4*>(p);
+  f[0] = q.x; f[1] = q.y; f[2] = q.z; f[3] = q.w;
+}
+__device__ __forceinline__ void sumsq_unpack(const __nv_bfloat16* p, float (&f)[8]) {
+  bf8_to_f(*reinterpret_cast<const Bf8*>(p), f);
+}
+
+template <typename T, bool ALIGNED>
+__global__ void __launch_bounds__(SUMSQ_BLOCK_CHAINS * sizeof(T) / 16)
+sumsq_partial_kernel(const T* __restrict__ x, long n, float* __restrict__ partial) {
+  constexpr int PER = 16 / sizeof(T), THREADS = SUMSQ_BLOCK_CHAINS / PER, LANES = 32 / PER, U = 8;
+  __shared__ float red[16];
+  const long j0 = (long)blockIdx.x * SUMSQ_BLOCK_CHAINS + threadIdx.x * PER;
+  float s[PER] = {};
+  long i = j0;
+  if (ALIGNED) {
+    for (; i + (U - 1) * SUMSQ_CHAINS + PER <= n; i += U * SUMSQ_CHAINS) {
+      float f[U][PER];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) s += f[j] * f[j];
-    } else {
-      float f[8];
-      bf8_to_f(*reinterpret_cast<const Bf8*>(&q), f);
+      for (int u = 0; u < U; ++u) sumsq_unpack(x + i + u * SUMSQ_CHAINS, f[u]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) s += f[j] * f[j];
+      for (int u = 0; u < U; ++u)
+#pragma unroll
+        for (int e = 0; e < PER; ++e) s[e] += f[u][e] * f[u][e];
     }
-  };
-  const long stride = (long)gridDim.x * 512;
-  for (long i = blockIdx.x * 512L + threadIdx.x; i < nv; i += 4 * stride) {
-    uint4 q[4];
+    for (; i + PER <= n; i += SUMSQ_CHAINS) {
+      float f[PER];
+      sumsq_unpack(x + i, f);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) q[u] = i + u * stride < nv ? xv[i + u * stride] : make_uint4(0, 0, 0, 0);
+      for (int e = 0; e < PER; ++e) s[e] += f[e] * f[e];
+    }
+  }
+  for (; i < n; i += SUMSQ_CHAINS) {
 #pragma unroll
-    for (int u = 0; u < 4; ++u) add(q[u], a[u]);
+    for (int e = 0; e < PER; ++e)
+      if (i + e < n) {
+        const float f = (float)x[i + e];
+        s[e] += f * f;
+      }
   }
-  float s = (a[0] + a[1]) + (a[2] + a[3]);
-  if (blockIdx.x == 0) {
-    for (long j = threadIdx.x; j < head; j += 512) s += (float)x[j] * (float)x[j];
-    for (long j = tail0 + threadIdx.x; j < n; j += 512) s += (float)x[j] * (float)x[j];
+#pragma unroll
+  for (int o = LANES / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < PER; ++e) s[e] += __shfl_xor_sync(0xffffffffu, s[e], o);
+#pragma unroll
+  for (int o = PER / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int e = 0; e < o; ++e) s[e] += s[e + o];
+  if (threadIdx.x % LANES == 0) red[threadIdx.x / LANES] = s[0];
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    const float r = pb::warp_sum(threadIdx.x < 16 ? red[threadIdx.x] : 0.f);
+    if (threadIdx.x == 0) partial[blockIdx.x] = r;
   }
-  s = block_sum<512>(s, red);
-  if (threadIdx.x == 0) partial[blockIdx.x] = s;
 }
 // out[0] (+)= sum(partial); nonfinite[0] |= !isfinite(sum)
 __global__ void __launch_bounds__(512) sumsq_final_kernel(const float* __restrict__ partial, int P,
@@ -686,16 +713,18 @@ int pb_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf
                      skip, s);
 }
 
-int pb_sumsq_num_partials() { return 1184; }
+int pb_sumsq_num_partials() { return SUMSQ_BLOCKS; }
 
 // out[0] (+)= sum(x^2). scratch: fp32 [pb_sumsq_num_partials()].
 int pb_sumsq(const void* x, int is_bf16, long n, float* scratch, float* out, int accumulate,
              int* nonfinite, cudaStream_t s) {
   const int P = pb_sumsq_num_partials();
-  if (is_bf16)
-    sumsq_partial_kernel<__nv_bfloat16><<<P, 512, 0, s>>>((const __nv_bfloat16*)x, n, scratch);
-  else
-    sumsq_partial_kernel<float><<<P, 512, 0, s>>>((const float*)x, n, scratch);
+  const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
+#define PB_SUMSQ(T, A) \
+  sumsq_partial_kernel<T, A><<<P, SUMSQ_BLOCK_CHAINS * sizeof(T) / 16, 0, s>>>((const T*)x, n, scratch)
+  if (is_bf16) { if (aligned) PB_SUMSQ(__nv_bfloat16, true); else PB_SUMSQ(__nv_bfloat16, false); }
+  else { if (aligned) PB_SUMSQ(float, true); else PB_SUMSQ(float, false); }
+#undef PB_SUMSQ
   sumsq_final_kernel<<<1, 512, 0, s>>>(scratch, P, out, accumulate, nonfinite);
   PB_CHECK_LAUNCH();
 }
