@@ -59,20 +59,22 @@ def stream_ptr() -> ctypes.c_void_p:
 
 
 def _ctype(a):
-    """C type an argument travels as: tensors and None are pointers, integers 64-bit (a launcher's 32-bit parameter reads
-    the low half of the register), floats single precision; ctypes instances keep their own type."""
-    if a is None or isinstance(a, torch.Tensor):
-        return _PTR
-    if isinstance(a, int):
-        return ctypes.c_long
+    """C type an argument travels as: floats single precision, integers 64-bit (a launcher's 32-bit parameter reads the low
+    half of the register), single ctypes values their own type.  All else is a pointer: tensors, None, and ctypes arrays,
+    which as their own class would admit no other length."""
     if isinstance(a, float):
         return ctypes.c_float
-    return type(a)
+    if isinstance(a, int):
+        return ctypes.c_long
+    if isinstance(a, ctypes._SimpleCData):
+        return type(a)
+    return _PTR
 
 
 # Launchers bound so far: name -> (function with its argument types set from the first call, kernels per call).  ctypes then
 # converts plain integers and floats itself; wrapping every argument of every call in a ctypes object cost more than the
-# launch for the 20-argument launchers.
+# launch for the 20-argument launchers.  A later call may bring an argument of another kind (None after an integer, a ctypes
+# integer after a plain one): ctypes refuses it before anything is called, and the launcher is bound anew.
 _BOUND: dict = {}
 
 
@@ -82,6 +84,14 @@ def _bind(name: str, args, stream: bool):
     fn.argtypes = [_ctype(a) for a in args] + ([_PTR] if stream else [])
     _BOUND[name, stream] = bound = (fn, _KERNELS_PER_CALL.get(name, 1))
     return bound
+
+
+def _run(name: str, fn, args, *stream) -> int:
+    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+    try:
+        return fn(*plain, *stream)
+    except ctypes.ArgumentError:
+        return _bind(name, args, bool(stream))[0](*plain, *stream)
 
 
 # Number of device kernels each launcher enqueues (default 1); used for the launch counter below.
@@ -95,8 +105,7 @@ def call(name: str, *args) -> None:
     global LAUNCH_COUNT
     fn, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
     LAUNCH_COUNT += kernels
-    rc = fn(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args],
-            torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    rc = _run(name, fn, args, torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
     if rc != 0:
         raise NativeLibraryError(f"pb_{name} failed with code {rc}")
 
@@ -104,7 +113,7 @@ def call(name: str, *args) -> None:
 def call_ret(name: str, *args) -> int:
     """Invoke a host-only helper that returns a value (no stream appended)."""
     fn, _ = _BOUND.get((name, False)) or _bind(name, args, False)
-    return fn(*[a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args])
+    return _run(name, fn, args)
 
 
 class I32(int):

@@ -1,6 +1,13 @@
-"""Host-side parts of the native library, on a machine without a GPU."""
+"""Host-side parts of the native library and of its binding, on a machine without a GPU."""
+import contextlib
+import ctypes
 import subprocess
 from pathlib import Path
+
+import pytest
+import torch
+
+from primus_b200.ops import _lib
 
 ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "primus_b200" / "csrc"
@@ -55,3 +62,56 @@ def test_division_by_an_invariant_is_the_division(tmp_path):
     awkward = [1.0, 1 - 2 ** -24, 1 - 2 ** -23, 0.5 + 2 ** -24, 0.75, 1e-6, 2 ** -40, 0.0]
     out = subprocess.run([exe, *(f"{b:.17g}" for b in corrections + awkward)], capture_output=True, text=True, check=True)
     assert not out.stdout, out.stdout
+
+
+LAUNCHERS = r"""
+extern "C" {
+int pb_last_peer(const long* peers, int n, void* stream) { return (int)peers[n - 1] - (int)(long)stream; }
+int pb_half(float x, void* stream) { return (int)(2 * x) - (int)(long)stream; }
+int pb_is_null(const void* p, int n, void* stream) { return (p == nullptr) + 10 * n - (int)(long)stream; }
+int pb_first_byte(const char* text) { return text[0]; }
+int pb_next_peer(const long* peers, int n) { return (int)peers[n - 1] + 1; }
+}
+"""
+
+
+@pytest.fixture
+def launchers(tmp_path, monkeypatch):
+    """A library of host functions in the place of the kernels' launchers; the current stream is 7."""
+    lib = ctypes.CDLL(str(_compile(tmp_path, "launchers", LAUNCHERS, "-shared", "-fPIC")))
+    monkeypatch.setattr(_lib, "_LIB", lib)
+    monkeypatch.setattr(_lib, "_BOUND", {})
+    monkeypatch.setattr(_lib, "LAUNCH_COUNT", 0)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 7)
+
+
+def _table(*values):
+    return (ctypes.c_long * len(values))(*values)
+
+
+def test_launcher_takes_peer_tables_of_any_length(launchers):
+    for n in (2, 8, 4):
+        _lib.call("last_peer", _table(*range(n - 1), 7), n)
+        assert _lib.call_ret("next_peer", _table(*range(n)), n) == n
+    assert _lib.LAUNCH_COUNT == 3
+
+
+@pytest.mark.parametrize("first,second", [((None, 0), (torch.zeros(1), 1)), ((torch.zeros(1), 1), (None, 0)),
+                                          ((0, 0), (None, 0)), ((0, ctypes.c_int(0)), (torch.zeros(1), 1)),
+                                          ((_table(1), 1), (None, ctypes.c_long(0)))])
+def test_launcher_takes_other_kinds_than_on_its_first_call(launchers, first, second):
+    """A null pointer (None or 0) and a tensor, plain and ctypes integers, in either order."""
+    for _ in range(2):
+        for p, n in (first, second):
+            with pytest.raises(_lib.NativeLibraryError, match=f"code {-6 if not getattr(n, 'value', n) else 3}"):
+                _lib.call("is_null", p, n)
+    assert _lib.LAUNCH_COUNT == 4
+
+
+def test_launcher_takes_floats_after_an_integer(launchers):
+    with contextlib.suppress(_lib.NativeLibraryError):
+        _lib.call("half", 1)             # (an integer in a float's place is not converted on the first call)
+    _lib.call("half", 3.5)
+    _lib.call("half", 3.5)
+    assert _lib.call_ret("first_byte", b"a") == ord("a")
