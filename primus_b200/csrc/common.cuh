@@ -13,6 +13,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+
 #ifndef PB_WAIT_CYCLES
 #define PB_WAIT_CYCLES (3000000000LL)  // ~1.5-2 s at B200 clocks
 #endif
@@ -465,6 +467,20 @@ inline int sm_count() {
     if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n <= 0) n = 148;
   }
   return n;
+}
+
+// Raises a kernel's dynamic shared memory limit on the current device, once per device; `done`: the kernel's own static flags.
+constexpr int MAX_DEVICES = 64;
+template <typename Kernel>
+int allow_shared_memory(Kernel kern, int bytes, std::atomic<bool> (&done)[MAX_DEVICES]) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return (int)e;
+  const bool known = dev >= 0 && dev < MAX_DEVICES;
+  if (known && done[dev].load(std::memory_order_relaxed)) return 0;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess && known) done[dev].store(true, std::memory_order_relaxed);
+  return (int)e;
 }
 
 inline EncodeTiledFn get_encode_fn() {

@@ -347,12 +347,9 @@ int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, cons
   // four rows ahead where two CTAs of an SM then still fit into its shared memory, else two
   constexpr int STAGES = 4 * STAGE <= 100 * 1024 ? 4 : 2;
   auto kern = rmsnorm_bwd_kernel<VPT, THREADS, RES>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, STAGES * STAGE);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, STAGES * STAGE, allowed);
+  if (rc) return rc;
   kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy, STAGES);
   return 0;
 }

@@ -2,6 +2,7 @@
 import contextlib
 import ctypes
 import subprocess
+import sys
 from pathlib import Path
 
 import pytest
@@ -115,3 +116,67 @@ def test_launcher_takes_floats_after_an_integer(launchers):
     _lib.call("half", 3.5)
     _lib.call("half", 3.5)
     assert _lib.call_ret("first_byte", b"a") == ord("a")
+
+
+# Stands in for the CUDA runtime: launches are recorded as "device <d> shared <bytes>", and refused where a kernel asks for more
+# than 48 KB without having been given the attribute on that device, or when `fail_next` says so.
+RUNTIME = r"""
+#include <cstdio>
+#include <map>
+#include <utility>
+struct dim3_ { unsigned x, y, z; };
+static int device, error, fail_next;
+static std::map<std::pair<int, const void*>, int> limit;
+static char log_[1 << 16];
+static int used;
+extern "C" {
+void fake_device(int d) { device = d; }
+void fake_fail_next(int n) { fail_next = n; }
+const char* fake_log() { return log_; }
+int cudaGetDevice(int* d) { *d = device; return 0; }
+int cudaFuncSetAttribute(const void* f, int, int value) { limit[{device, f}] = value; return 0; }
+int cudaGetLastError() { int e = error; error = 0; return e; }
+int cudaLaunchKernel(const void* f, dim3_, dim3_, void**, size_t shared, void*) {
+  used += snprintf(log_ + used, sizeof log_ - used, "device %d shared %zu\n", device, shared);
+  if (shared > 48 * 1024 && (int)shared > limit[{device, f}]) error = 1;
+  if (fail_next > 0 && --fail_next == 0) error = 700;
+  return error;
+}
+}
+"""
+
+BACKWARD = """
+import ctypes, sys
+fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)      # its names come before the runtime's
+lib = ctypes.CDLL(sys.argv[2])
+fake.fake_log.restype = ctypes.c_char_p
+p, n = ctypes.c_void_p(4096), ctypes.c_long
+rows, H, residual = int(sys.argv[3]), int(sys.argv[4]), int(sys.argv[5])
+def backward():
+    return lib.pb_rmsnorm_bwd(p, p, p, p, p if residual else None, p, p, p, n(rows), H, n(H), n(H), 1, None)
+for step in sys.argv[6:]:
+    what, value = step.split("=")
+    if what == "device":
+        fake.fake_device(int(value))
+        print("rc", backward())
+    else:
+        fake.fake_fail_next(int(value))
+print(fake.fake_log().decode())
+"""
+
+
+def _norm_backward(tmp_path, rows, H, residual, *steps):
+    """Return codes and launches of RMSNorm backward calls on a stand-in for the CUDA runtime."""
+    fake = _compile(tmp_path, "runtime", RUNTIME, "-shared", "-fPIC")
+    out = subprocess.run([sys.executable, "-c", BACKWARD, fake, _lib.lib_path(), str(rows), str(H), str(int(residual)), *steps],
+                         capture_output=True, text=True, check=True).stdout.split("\n")
+    return [int(line.split()[1]) for line in out if line.startswith("rc")], [line for line in out if line.startswith("device")]
+
+
+@pytest.mark.skipif(not _lib.available(), reason="the native library is not built")
+@pytest.mark.parametrize("H", [1032, 2048, 4096, 8192, 16384])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_backward_on_several_devices(tmp_path, H, residual):
+    codes, launches = _norm_backward(tmp_path, 1000, H, residual, "device=0", "device=1", "device=0", "device=3")
+    assert codes == [0, 0, 0, 0]
+    assert [line.split()[1] for line in launches] == list("00110033")       # each the rows' kernel and the reduction
