@@ -351,7 +351,7 @@ int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, cons
   const int rc = pbh::allow_shared_memory(kern, STAGES * STAGE, allowed);
   if (rc) return rc;
   kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy, STAGES);
-  return 0;
+  return (int)cudaGetLastError();
 }
 
 int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
@@ -361,7 +361,7 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
 #define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                         \
   {                                                                                                              \
     rmsnorm_bwd_short_kernel<LPR, VPL, RPG><<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy); \
-    return 0;                                                                                                    \
+    return (int)cudaGetLastError();                                                                              \
   }
 #define PB_NORM_BWD(VPT, THREADS)                                                                                     \
   return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy) \
@@ -606,6 +606,8 @@ int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk
   else if (d <= 128) PB_QK_BWD(16);
   else PB_QK_BWD(32);
 #undef PB_QK_BWD
+  const int rc = (int)cudaGetLastError();
+  if (rc) return rc;                                 // no gain sums from partial rows that nothing wrote
   const int blocks = (d + DWR_COLS - 1) / DWR_COLS, threads = DWR_COLS * DWR_ROWS;
   rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate);
   rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate);

@@ -153,6 +153,8 @@ fake.fake_log.restype = ctypes.c_char_p
 p, n = ctypes.c_void_p(4096), ctypes.c_long
 rows, H, residual = int(sys.argv[3]), int(sys.argv[4]), int(sys.argv[5])
 def backward():
+    if H <= 256 and residual:                                 # norms of H-channel heads inside a packed tensor
+        return lib.pb_qk_norm_bwd(p, p, p, p, p, p, p, p, p, n(rows), 2, 1, H, n(4 * H), n(4 * H), n(4 * H), 1, None)
     return lib.pb_rmsnorm_bwd(p, p, p, p, p if residual else None, p, p, p, n(rows), H, n(H), n(H), 1, None)
 for step in sys.argv[6:]:
     what, value = step.split("=")
@@ -180,3 +182,12 @@ def test_norm_backward_on_several_devices(tmp_path, H, residual):
     codes, launches = _norm_backward(tmp_path, 1000, H, residual, "device=0", "device=1", "device=0", "device=3")
     assert codes == [0, 0, 0, 0]
     assert [line.split()[1] for line in launches] == list("00110033")       # each the rows' kernel and the reduction
+
+
+@pytest.mark.skipif(not _lib.available(), reason="the native library is not built")
+@pytest.mark.parametrize("H", [64, 256, 512, 1024, 2048, 8192, 16384])
+@pytest.mark.parametrize("residual", [False, True])
+def test_norm_backward_stops_after_a_refused_launch(tmp_path, H, residual):
+    """The weight gradient is not added up from partial sums that were never written."""
+    codes, launches = _norm_backward(tmp_path, 1000, H, residual, "fail=1", "device=0", "device=0")
+    assert codes == [700, 0] and len(launches) == 1 + (3 if H <= 256 and residual else 2)
