@@ -124,7 +124,8 @@ __device__ __forceinline__ void quantize_half(const uint4 (&d)[CG], int h, long 
           const uint4& v = d[2 * j + u];
           a[u] = max_pair(max_pair(abs_pair(v.x), abs_pair(v.y)), max_pair(abs_pair(v.z), abs_pair(v.w)));
         }
-        m[j] = max_pair(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632));
+        // (a block of nothing but NaN counts as zero, as in the column direction: the maximum ignores a NaN operand)
+        m[j] = max_pair(0u, max_pair(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632)));
         m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 1));
         m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 2));
       }
