@@ -124,6 +124,13 @@ def rmsnorm(x, w, eps=1e-5, residual=None):
     return RMSNormFn.apply(x, w, eps, residual)
 
 
+def dense_rows(t):
+    """``t`` itself where it is contiguous and starts on a 16-byte boundary, else a copy that does: what a kernel may read in
+    16-byte vectors without a row pitch."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class QKNormFn(torch.autograd.Function):
     """RMSNorm of every q and k head inside a packed [T, (hq + 2 hkv) d] projection output; v passes through."""
 
@@ -143,8 +150,7 @@ class QKNormFn(torch.autograd.Function):
         qkv, wq, wk, rstd = ctx.saved_tensors
         hq, hkv, d = ctx.dims
         T = qkv.shape[0]
-        if not dy.is_contiguous():
-            dy = dy.contiguous()
+        dy = dense_rows(dy)
         dx = torch.empty(T, (hq + 2 * hkv) * d, dtype=qkv.dtype, device=qkv.device)
         main = [getattr(w, "main_grad", None) for w in ctx.w_refs]
         dw = [g if g is not None else torch.zeros(d, dtype=torch.float32, device=qkv.device) for g in main]

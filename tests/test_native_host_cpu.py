@@ -8,7 +8,7 @@ from pathlib import Path
 import pytest
 import torch
 
-from primus_b200.ops import _lib
+from primus_b200.ops import _lib, attention, fused
 
 ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "primus_b200" / "csrc"
@@ -191,3 +191,15 @@ def test_norm_backward_stops_after_a_refused_launch(tmp_path, H, residual):
     """The weight gradient is not added up from partial sums that were never written."""
     codes, launches = _norm_backward(tmp_path, 1000, H, residual, "fail=1", "device=0", "device=0")
     assert codes == [700, 0] and len(launches) == 1 + (3 if H <= 256 and residual else 2)
+
+
+@pytest.mark.parametrize("off,rows", [(0, 4), (1, 4), (3, 1), (8, 2)])
+def test_gradient_of_packed_heads_is_read_from_an_aligned_start(off, rows):
+    """The kernels read 16 bytes at a time: a contiguous view that starts in between is copied, any other is not."""
+    g = torch.arange(off + rows * 64, dtype=torch.float32).bfloat16()[off:].view(rows, 64)
+    got = fused.dense_rows(g)
+    assert torch.equal(got, g) and got.is_contiguous() and got.data_ptr() % 16 == 0
+    assert (got.data_ptr() == g.data_ptr()) == (g.data_ptr() % 16 == 0)
+    wide = torch.arange(rows * 128, dtype=torch.float32).bfloat16().view(rows, 128)
+    got = fused.dense_rows(wide[:, 8:72])
+    assert torch.equal(got, wide[:, 8:72]) and got.is_contiguous() and got.data_ptr() % 16 == 0
