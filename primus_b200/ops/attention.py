@@ -72,6 +72,10 @@ def _check_view(t, d):
     assert t.data_ptr() % 16 == 0
 
 
+def _check_sinks(sinks, hq):
+    assert sinks.dtype == torch.float32 and sinks.numel() == hq and sinks.is_contiguous()
+
+
 def flash_attn_fwd(q, k, v, batch: int, causal: bool, scale: float, q_off: int = 0, window: int = 0, sinks=None,
                    softcap: float = 0.0):
     T, hq, dqk = q.shape
@@ -83,7 +87,7 @@ def flash_attn_fwd(q, k, v, batch: int, causal: bool, scale: float, q_off: int =
     o = torch.empty(T, hq, dv, dtype=q.dtype, device=q.device)
     lse = torch.empty(batch, hq, S, dtype=torch.float32, device=q.device)
     if sinks is not None:
-        assert sinks.dtype == torch.float32 and sinks.numel() == hq and sinks.is_contiguous()
+        _check_sinks(sinks, hq)
     _lib.call("flash_attn_fwd_cap", q, k, v, o, lse, batch, S, SK, int(q_off), hq, hkv, dqk, dv, q.stride(0), k.stride(0),
               v.stride(0), o.stride(0), float(scale), int(causal), int(window or 0), sinks, float(softcap or 0.0),
               _lib.status_word(q.device))
@@ -105,6 +109,8 @@ def flash_attn_bwd(do, q, k, v, o, lse, batch: int, causal: bool, scale: float, 
     do = do if (do.stride(2) == 1 and do.stride(1) == dvd) else do.contiguous()
     for t, d in ((q, dqk), (k, dqk), (v, dvd), (o, dvd), (do, dvd), (dq, dqk), (dk, dqk), (dv, dvd)):
         _check_view(t, d)
+    if sinks is not None:
+        _check_sinks(sinks, hq)
     delta = torch.empty(2, batch, hq, S, dtype=torch.float32, device=q.device)  # [rowsum(dO*O), lse*log2e]
     _lib.call("flash_attn_bwd_cap", do, q, k, v, o, lse, delta, dq, dk, dv, batch, S, SK, int(q_off), hq, hkv, dqk, dvd,
               q.stride(0), k.stride(0), v.stride(0), o.stride(0), do.stride(0), dq.stride(0), dk.stride(0),

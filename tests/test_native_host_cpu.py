@@ -203,3 +203,17 @@ def test_gradient_of_packed_heads_is_read_from_an_aligned_start(off, rows):
     wide = torch.arange(rows * 128, dtype=torch.float32).bfloat16().view(rows, 128)
     got = fused.dense_rows(wide[:, 8:72])
     assert torch.equal(got, wide[:, 8:72]) and got.is_contiguous() and got.data_ptr() % 16 == 0
+
+
+@pytest.mark.parametrize("sinks", [torch.zeros(2, dtype=torch.bfloat16), torch.zeros(3), torch.zeros(4)[::2]])
+def test_attention_backward_refuses_sinks_the_kernel_cannot_read(sinks, monkeypatch):
+    """The gradient kernel reads one contiguous fp32 logit per head, as the forward checks: nothing is launched for others."""
+    q = torch.zeros(128, 2, 64, dtype=torch.bfloat16)
+    launched = []
+    monkeypatch.setattr(_lib, "call", lambda name, *args: launched.append(name))
+    monkeypatch.setattr(_lib, "status_word", lambda device: None)
+    with pytest.raises(AssertionError):
+        attention.flash_attn_bwd(q, q, q, q, q, torch.zeros(1, 2, 128), 1, True, 0.125, sinks=sinks)
+    assert not launched
+    attention.flash_attn_bwd(q, q, q, q, q, torch.zeros(1, 2, 128), 1, True, 0.125, sinks=torch.zeros(2))
+    assert launched == ["flash_attn_bwd_cap", "attn_sink_grad"]
