@@ -13,6 +13,8 @@ and the fused main-grad accumulation of primus/backends/megatron/core/tensor_par
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _lib, autotune
@@ -219,40 +221,58 @@ def gemm(
     return out
 
 
-# CTA pairs of a B200, and the K steps (of 64) a part of a split reduction keeps at least: a part of 16 steps takes about as
-# long as adding the parts costs (workspace traffic and one more launch, ~5 us)
-_CTA_PAIRS = 74
-_SPLIT_MIN_STEPS = 16
+_SMS = 148
+_ONE_CTA, _CTA_PAIR = 0, 1          # routes of a bf16 GEMM; s > 1: CTA pairs with the reduction cut into s parts
 
 
-def _split_k(M: int, N: int, K: int) -> int:
-    """Parts to cut the reduction into: as many as fill the idle CTA pairs of a GEMM with few 256 x 256 output tiles."""
-    tiles = -(-M // 256) * -(-N // 256)
+@functools.lru_cache(maxsize=4096)
+def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, max_ctas: int) -> int:
+    """The route that takes the least time by a model of the three (microseconds, fitted to 190 shapes of 64 to 16384 in three
+    layouts, each route timed; the choice is within 1 % of the best one on average, where the pair kernel for every output of
+    at least 256 x 256 was 20 % slower than the one-CTA kernel on outputs of one wave and up to 50 % on ragged ones).
+
+    A wave takes as long per K step (64) on either kernel, about 0.28 us, but the pair's tile is 256 rows instead of 128, and a
+    launch of clusters costs 1.1 us more (2048 x 2048 x 512: 9.0 against 7.9 us).  What the one-CTA tile pays for is its
+    operand traffic per product, a third above the pair's: 15 % in the layout whose operands both need a transposed read, 4
+    and 14 % with two and more waves (8192 x 4096 x 4096: 194 against 180 us), and far more where the rows of B start off a
+    64-byte boundary and every 128-byte row of a box touches another sector or line (3152 x 584 x 8656, K-major A: 73 against
+    50 us).
+    Parts of a split reduction fill CTA pairs that few tiles leave idle; they pay 3.2 us for the second kernel and the trip of
+    their fp32 sums (1024 x 1024: K = 4096 24 -> 16 us in four parts, K = 1024 9.8 -> 12.7 us in two)."""
+    step, ctas = 0.28, max_ctas or _SMS
+    pairs = ctas // 2
     steps = -(-K // 64)
-    return max(1, min(_CTA_PAIRS // tiles, steps // _SPLIT_MIN_STEPS)) if N % 4 == 0 else 1
+    one_tiles, pair_tiles = -(-M // 128) * -(-N // 256), -(-M // 256) * -(-N // 256)
+    waves = -(-one_tiles // ctas)
+    off_64, off_32 = ldb % 32 != 0, ldb % 16 != 0
+    pair_step = step * (1.3 if off_32 else 1.0)
+    one_step = step * (1.15 if both_mn else 1.0) * (1.0, 1.04, 1.14)[min(waves, 3) - 1] * (1.8 if off_32 else 1.25 if off_64 else 1.0)
+    best = (waves * steps * one_step, _ONE_CTA)
+    if M >= 256 and N >= 256 and pairs:
+        best = min(best, (1.1 + -(-pair_tiles // pairs) * steps * pair_step, _CTA_PAIR))
+    if N % 4 == 0 and max_ctas == 0:      # (a caller that leaves SMs to other work does not get a second kernel)
+        for parts in range(2, min(pairs // pair_tiles, steps // 8) + 1):
+            best = min(best, (3.2 + -(-steps // parts) * pair_step + 8 * parts * M * N / 12e6, parts))
+    return best[1]
 
 
 def launch_bf16(a, b, out, M: int, N: int, K: int, a_mn: bool, b_mn: bool, mode: int, block_n: int,
                 max_ctas: int = 0, two_cta: bool | None = None) -> None:
     """Raw launch of the bf16 tcgen05 GEMM with explicit tile options (the autotuner times candidates through it).
-    ``two_cta``: the CTA-pair kernel (None: where both dimensions fill a 256 x 256 tile, or, with the reduction split,
-    where K is long and the tiles are few)."""
-    if two_cta is None:
-        splits = _split_k(M, N, K) if block_n == 256 and max_ctas == 0 else 1
-        if splits > 1:
-            ws = torch.empty(splits * (-(-M // 256) * 256) * N, dtype=torch.float32, device=a.device)
-            _lib.call("gemm_bf16_splitk", a, b, out, ws, M, N, K, a.stride(0), b.stride(0), out.stride(0),
-                      int(a_mn), int(b_mn), mode, splits, _lib.status_word(a.device))
-            return
-        two_cta = block_n == 256 and M >= 256 and N >= 256 and max_ctas != 1
-    if two_cta:
+    ``two_cta``: the CTA-pair kernel (None: chosen by the sizes, a split reduction among the choices)."""
+    route = int(two_cta or 0)
+    if two_cta is None and block_n == 256:
+        route = _bf16_route(M, N, K, a_mn and b_mn, b.stride(0), max_ctas)
+    if route > _CTA_PAIR:
+        ws = torch.empty(route * (-(-M // 256) * 256) * N, dtype=torch.float32, device=a.device)
+        _lib.call("gemm_bf16_splitk", a, b, out, ws, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                  int(a_mn), int(b_mn), mode, route, _lib.status_word(a.device))
+    elif route == _CTA_PAIR:
         _lib.call("gemm_bf16_2cta", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
                   int(a_mn), int(b_mn), mode, max_ctas, _lib.status_word(a.device))
-        return
-    _lib.call(
-        "gemm_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
-        int(a_mn), int(b_mn), mode, block_n, max_ctas, _lib.status_word(a.device),
-    )
+    else:
+        _lib.call("gemm_bf16", a, b, out, M, N, K, a.stride(0), b.stride(0), out.stride(0),
+                  int(a_mn), int(b_mn), mode, block_n, max_ctas, _lib.status_word(a.device))
 
 
 class LinearFn(torch.autograd.Function):
