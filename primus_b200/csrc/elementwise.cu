@@ -761,55 +761,107 @@ int pb_embedding_bwd(const void* dy, const long* tokens, float* dw, long T, int 
 //   moe_combine_rows: out[t, :] = sum_k y[pos[t, k], :]        (pos < 0 skipped)  -- the un-weighted top-k
 //                     combine (routing probabilities are applied inside the expert activation) and, read
 //                     the other way round, the backward of the gather.
-// One warp moves one row with 16-byte accesses.  Replaces the permutation kernels of
+// A warp moves rows with 16-byte accesses.  Replaces the permutation kernels of
 // primus/backends/transformer_engine/pytorch/common/triton/permutation.py:189-305.
 namespace {
 
-// MOE_UNROLL vectors of a row per lane are loaded before the first is stored
-constexpr int MOE_UNROLL = 8;
+// What bounds both is the loads in flight, and those are a matter of the warps on an SM as much as of the vectors that a lane
+// asks for: eight vectors per lane at 64 and more registers were slower than two at 32 to 40.  A warp takes ROWS neighbouring
+// rows (tokens) at a time, several where a row is a vector per lane or less, and VECS vectors of each per lane.
+template <int ROWS, int VECS>
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ src, const float* __restrict__ scale,
                        __nv_bfloat16* __restrict__ out, long R, int H, const int* __restrict__ limit_rows) {
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
-  const long lim = limit_rows ? (long)limit_rows[0] : R;
   const int nv = H / 8;
-  for (long r = warp_global; r < R && r < lim; r += num_warps) {
-    const int s = src[r];
-    Bf8* o = reinterpret_cast<Bf8*>(out + r * H);
-    const Bf8* in = reinterpret_cast<const Bf8*>(x + (long)s * H);
-    const float sc = scale && s >= 0 ? scale[r] : 1.f;
-    for (int base = lane; base < nv; base += 32 * MOE_UNROLL) {
-      Bf8 t[MOE_UNROLL];
+  const long end = limit_rows ? min(R, (long)*limit_rows) : R;
+  for (long r0 = warp_global * ROWS; r0 < end; r0 += num_warps * ROWS) {
+    int s[ROWS];
+    float sc[ROWS];
 #pragma unroll
-      for (int u = 0; u < MOE_UNROLL; ++u) {
-        const int v = base + u * 32;
-        if (s < 0) {
+    for (int i = 0; i < ROWS; ++i) s[i] = r0 + i < end ? src[r0 + i] : -1;
 #pragma unroll
-          for (int i = 0; i < 4; ++i) t[u].v[i] = __floats2bfloat162_rn(0.f, 0.f);
-        } else if (v < nv) {
-          t[u] = in[v];
+    for (int i = 0; i < ROWS; ++i) sc[i] = scale && s[i] >= 0 ? scale[r0 + i] : 1.f;
+    for (int base = lane; base < nv; base += 32 * VECS) {
+      Bf8 t[ROWS][VECS];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int u = 0; u < VECS; ++u) {
+          const int v = base + u * 32;
+          if (s[i] < 0) {
+#pragma unroll
+            for (int j = 0; j < 4; ++j) t[i][u].v[j] = __floats2bfloat162_rn(0.f, 0.f);
+          } else if (v < nv) {
+            t[i][u] = reinterpret_cast<const Bf8*>(x + (long)s[i] * H)[v];
+          }
         }
-      }
 #pragma unroll
-      for (int u = 0; u < MOE_UNROLL; ++u) {
-        const int v = base + u * 32;
-        if (v >= nv) break;
-        if (scale) {
-          float f[8];
-          bf8_to_f(t[u], f);
+      for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) f[j] *= sc;
-          t[u] = f_to_bf8(f);
+        for (int u = 0; u < VECS; ++u) {
+          const int v = base + u * 32;
+          if (v >= nv || r0 + i >= end) continue;
+          if (scale) {
+            float f[8];
+            bf8_to_f(t[i][u], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) f[j] *= sc[i];
+            t[i][u] = f_to_bf8(f);
+          }
+          reinterpret_cast<Bf8*>(out + (r0 + i) * H)[v] = t[i][u];
         }
-        o[v] = t[u];
-      }
     }
   }
 }
 
-// Two vectors per lane at a time; the rows of four copies (eight loads) are in flight together, summed in copy order.
+// All COPIES copies of a token at once, summed in copy order: a vector's sum needs its registers only while it is stored.
+template <int COPIES, int ROWS, int VECS, int CTAS>
+__global__ void __launch_bounds__(256, CTAS)
+moe_combine_all_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, __nv_bfloat16* __restrict__ out, long T, int H) {
+  const int lane = threadIdx.x & 31;
+  const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
+  const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
+  const int nv = H / 8;
+  for (long t0 = warp_global * ROWS; t0 < T; t0 += num_warps * ROWS) {
+    int p[ROWS][COPIES];
+#pragma unroll
+    for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+      for (int k = 0; k < COPIES; ++k) p[i][k] = t0 + i < T ? pos[(t0 + i) * COPIES + k] : -1;
+    for (int base = lane; base < nv; base += 32 * VECS) {
+      Bf8 a[ROWS][VECS][COPIES];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int u = 0; u < VECS; ++u)
+#pragma unroll
+          for (int k = 0; k < COPIES; ++k)
+            if (p[i][k] >= 0 && base + u * 32 < nv) a[i][u][k] = reinterpret_cast<const Bf8*>(y + (long)p[i][k] * H)[base + u * 32];
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int u = 0; u < VECS; ++u) {
+          if (t0 + i >= T || base + u * 32 >= nv) continue;
+          float acc[8] = {};
+#pragma unroll
+          for (int k = 0; k < COPIES; ++k) {
+            if (p[i][k] < 0) continue;
+            float f[8];
+            bf8_to_f(a[i][u][k], f);
+#pragma unroll
+            for (int j = 0; j < 8; ++j) acc[j] += f[j];
+          }
+          reinterpret_cast<Bf8*>(out + (t0 + i) * H)[base + u * 32] = f_to_bf8(acc);
+        }
+    }
+  }
+}
+
+// COPIES of a token's topk copies at a time, summed in copy order.
+template <int COPIES, int ROWS, int VECS>
 __global__ void __launch_bounds__(256)
 moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, __nv_bfloat16* __restrict__ out,
                         long T, int topk, int H) {
@@ -817,42 +869,49 @@ moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restri
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
   const int nv = H / 8;
-  for (long t = warp_global; t < T; t += num_warps) {
-    Bf8* o = reinterpret_cast<Bf8*>(out + t * H);
-    for (int v = lane; v < nv; v += 64) {
-      const bool second = v + 32 < nv;
-      float acc[2][8] = {};
-      for (int k0 = 0; k0 < topk; k0 += 4) {
-        int p[4];
-        Bf8 a[4], b[4];
+  for (long t0 = warp_global * ROWS; t0 < T; t0 += num_warps * ROWS) {
+    for (int base = lane; base < nv; base += 32 * VECS) {
+      float acc[ROWS][VECS][8] = {};
+      for (int k0 = 0; k0 < topk; k0 += COPIES) {
+        int p[ROWS][COPIES];
+        Bf8 a[ROWS][COPIES][VECS];
 #pragma unroll
-        for (int k = 0; k < 4; ++k) p[k] = k0 + k < topk ? pos[t * topk + k0 + k] : -1;
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (p[k] < 0) continue;
-          const Bf8* row = reinterpret_cast<const Bf8*>(y + (long)p[k] * H);
-          a[k] = row[v];
-          if (second) b[k] = row[v + 32];
-        }
+          for (int k = 0; k < COPIES; ++k) p[i][k] = k0 + k < topk && t0 + i < T ? pos[(t0 + i) * topk + k0 + k] : -1;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          if (p[k] < 0) continue;
-          float f[8];
-          bf8_to_f(a[k], f);
+        for (int i = 0; i < ROWS; ++i)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) acc[0][j] += f[j];
-          if (second) {
-            bf8_to_f(b[k], f);
+          for (int k = 0; k < COPIES; ++k)
 #pragma unroll
-            for (int j = 0; j < 8; ++j) acc[1][j] += f[j];
-          }
-        }
+            for (int u = 0; u < VECS; ++u)
+              if (p[i][k] >= 0 && base + u * 32 < nv)
+                a[i][k][u] = reinterpret_cast<const Bf8*>(y + (long)p[i][k] * H)[base + u * 32];
+#pragma unroll
+        for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+          for (int k = 0; k < COPIES; ++k)
+#pragma unroll
+            for (int u = 0; u < VECS; ++u)
+              if (p[i][k] >= 0 && base + u * 32 < nv) {
+                float f[8];
+                bf8_to_f(a[i][k][u], f);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[i][u][j] += f[j];
+              }
       }
-      o[v] = f_to_bf8(acc[0]);
-      if (second) o[v + 32] = f_to_bf8(acc[1]);
+#pragma unroll
+      for (int i = 0; i < ROWS; ++i)
+#pragma unroll
+        for (int u = 0; u < VECS; ++u)
+          if (t0 + i < T && base + u * 32 < nv)
+            reinterpret_cast<Bf8*>(out + (t0 + i) * H)[base + u * 32] = f_to_bf8(acc[i][u]);
     }
   }
 }
+
+// CTAs of eight warps for `warps` warps' work (one pass over most layers; more loop)
+inline unsigned moe_grid(long warps) { return (unsigned)grid_for(warps * 32, 256, 1 << 16); }
 
 }  // namespace
 
@@ -860,8 +919,12 @@ extern "C" int pb_moe_gather_rows(const void* x, const int* src, const float* sc
                                   const int* limit_rows, cudaStream_t s) {
   if (H % 8) return -2;
   if (R == 0) return 0;
-  moe_gather_rows_kernel<<<grid_for(R * 32, 256, 1 << 16), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale,
-                                                              (__nv_bfloat16*)out, R, H, limit_rows);
+#define PB_GATHER(ROWS, VECS)                                                                                        \
+  moe_gather_rows_kernel<ROWS, VECS><<<moe_grid((R + ROWS - 1) / ROWS), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale, \
+                                                                                     (__nv_bfloat16*)out, R, H, limit_rows)
+  // (us, B200, before and now: 4096 tokens of 2048, 64 experts, eight copies 51 -> 43; 65536 of 256, two copies 44 -> 22)
+  if (H <= 256) PB_GATHER(4, 1); else PB_GATHER(1, 2);
+#undef PB_GATHER
   return (int)cudaGetLastError();
 }
 
@@ -869,7 +932,21 @@ extern "C" int pb_moe_combine_rows(const void* y, const int* pos, void* out, lon
                                    cudaStream_t s) {
   if (H % 8) return -2;
   if (T == 0) return 0;
-  moe_combine_rows_kernel<<<grid_for(T * 32, 256, 1 << 16), 256, 0, s>>>((const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T,
-                                                               topk, H);
+#define PB_COMBINE_ALL(COPIES, ROWS, VECS, CTAS)                                                  \
+  moe_combine_all_kernel<COPIES, ROWS, VECS, CTAS><<<moe_grid((T + ROWS - 1) / ROWS), 256, 0, s>>>( \
+      (const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T, H)
+#define PB_COMBINE(COPIES, ROWS, VECS)                                                            \
+  moe_combine_rows_kernel<COPIES, ROWS, VECS><<<moe_grid((T + ROWS - 1) / ROWS), 256, 0, s>>>(    \
+      (const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T, topk, H)
+  // (us, B200, before and now: 16384 tokens of 2048, one copy 31 -> 24; 65536 of 256, two copies 35 -> 17; 4096 of 2048,
+  // eight copies 35 -> 29).  Fewer than 148 x 16 warps leave the SMs short of loads unless each asks for more of them: 1024
+  // tokens of 4096, eight copies 18 us against 23.
+  if (topk == 1) PB_COMBINE_ALL(1, 1, 4, 6);
+  else if (topk == 2) { if (H <= 512) PB_COMBINE_ALL(2, 2, 1, 6); else PB_COMBINE_ALL(2, 1, 4, 4); }
+  else if (T < 148 * 16) PB_COMBINE(4, 1, 2);
+  else if (H <= 256) { if (T < 16384) PB_COMBINE(4, 1, 1); else PB_COMBINE(1, 1, 1); }
+  else PB_COMBINE(2, 1, 2);
+#undef PB_COMBINE_ALL
+#undef PB_COMBINE
   return (int)cudaGetLastError();
 }
