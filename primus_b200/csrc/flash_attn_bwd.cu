@@ -768,7 +768,19 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       const float* stat = stat_smem + st * C::STAT_FLOATS + 16 * qd;
       BW_WAIT(&bars->s_full[C::NSB == 2 ? (i & 1) : 0], C::NSB == 2 ? ((i >> 1) & 1) : (i & 1), PB_ERR_TIMEOUT_EPILOGUE);
       pb::tc_fence_after();
-      float p[32], dc[CAP ? 32 : 1];
+      auto masked = [&](int e) {
+        const int col_g = cs_rel * BCW + (e >> 4) * 64 + 16 * qd + (e & 15);
+        const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
+        return diff < 0 || (window > 0 && diff >= window);
+      };
+      float p[32];      // CAP: tanh(scale * s / softcap) until dP is there, so that no element needs two registers
+      auto probabilities = [&](int e2, float s0, float s1) {      // p[e2], p[e2 + 1] of two scores
+        uint64_t l2 = row_l2;
+        if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(stat + (e2 >> 4) * 128 + (e2 & 15));
+        pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
+        p[e2] = pb::fast_exp2(p[e2]);
+        p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
+      };
       {
         uint32_t sr[32];
         pb::tmem_ld_32x32b_x16(ts, sr);
@@ -781,28 +793,18 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         }
 #pragma unroll
         for (int e2 = 0; e2 < 32; e2 += 2) {
-          uint64_t l2 = row_l2;
-          if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(stat + (e2 >> 4) * 128 + (e2 & 15));
-          float s0 = __uint_as_float(sr[e2]), s1 = __uint_as_float(sr[e2 + 1]);
+          const float s0 = __uint_as_float(sr[e2]), s1 = __uint_as_float(sr[e2 + 1]);
           if (CAP) {
-            // the score is softcap * tanh(scale * s / softcap) / scale; dc: its derivative with respect to scale * s
-            const float t0 = pb::fast_tanh(s0 * cap_a), t1 = pb::fast_tanh(s1 * cap_a);
-            s0 = t0 * cap_b;
-            s1 = t1 * cap_b;
-            dc[e2] = 1.f - t0 * t0;
-            dc[e2 + 1] = 1.f - t1 * t1;
+            p[e2] = pb::fast_tanh(s0 * cap_a);
+            p[e2 + 1] = pb::fast_tanh(s1 * cap_a);
+          } else {
+            probabilities(e2, s0, s1);
           }
-          pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
-          p[e2] = pb::fast_exp2(p[e2]);
-          p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
         }
-        if (diag) {
+        if (!CAP && diag) {
 #pragma unroll
-          for (int e = 0; e < 32; ++e) {
-            const int col_g = cs_rel * BCW + (e >> 4) * 64 + 16 * qd + (e & 15);
-            const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
-            if (diff < 0 || (window > 0 && diff >= window)) p[e] = 0.f;
-          }
+          for (int e = 0; e < 32; ++e)
+            if (masked(e)) p[e] = 0.f;
         }
       }
       BW_WAIT(&bars->dp_full, i & 1, PB_ERR_TIMEOUT_EPILOGUE);
@@ -822,12 +824,24 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
 #pragma unroll
         for (int e2 = 0; e2 < 16; e2 += 2) {
           const int e = half * 16 + e2;
+          float dc0 = 1.f, dc1 = 1.f;
+          if (CAP) {
+            // the score is softcap * tanh(scale * s / softcap) / scale; dc: its derivative with respect to scale * s
+            const float t0 = p[e], t1 = p[e + 1];
+            dc0 = fmaf(-t0, t0, 1.f);
+            dc1 = fmaf(-t1, t1, 1.f);
+            probabilities(e, t0 * cap_b, t1 * cap_b);
+            if (diag) {
+              if (masked(e)) p[e] = 0.f;
+              if (masked(e + 1)) p[e + 1] = 0.f;
+            }
+          }
           uint64_t dl = row_delta;
           if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(stat + half * 128 + 64 + e2);
           const uint64_t pp = pb::pack_f32x2(p[e], p[e + 1]);
           // dS = P (dP - delta), times the score scale, which the epilogue applies
           uint64_t ds = pb::mul_f32x2(pp, pb::fma_f32x2(dl, minus_one, pb::pack_f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1]))));
-          if (CAP) ds = pb::mul_f32x2(ds, pb::pack_f32x2(dc[e], dc[e + 1]));
+          if (CAP) ds = pb::mul_f32x2(ds, pb::pack_f32x2(dc0, dc1));
           float d0, d1;
           pb::unpack_f32x2(ds, d0, d1);
           pk[e2 / 2] = pb::pack_bf16x2(p[e], p[e + 1]);
