@@ -117,18 +117,20 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 #define PB_NORM_FWD(LPR, VPL, RPG, THREADS)                                                             \
   rmsnorm_fwd_kernel<LPR, VPL, RPG, THREADS>                                                            \
       <<<(unsigned)((rows + (THREADS / LPR) * RPG - 1) / ((THREADS / LPR) * RPG)), THREADS, 0, s>>>(args...)
-  // a few hundred rows do not fill the SMs with four rows (or four vectors) per lane: spread them (768 rows of 256: 3.0 ->
-  // 2.2 us; at 4096 rows of 2048 the wide form is already the better one, 12.2 against 13.5 us)
+  // Few rows do not fill the SMs with four rows (or two, or a row per warp) per group: spread them (768 rows of 256: 3.0 -> 2.2
+  // us).  The lines lie where both forms take the same time; 64 lanes of four vectors hold for 1032 to 2048 channels at any
+  // number of rows (500 rows of 2048 3.2 us, with 256 lanes of one vector 3.5), 256 lanes of eight above 8192 (4096 rows of
+  // 12288 76 us, with 512 lanes of four 85).
   const bool few = rows * nv < 148 * 2048L;
   if (nv <= 8) { if (few) PB_NORM_FWD(8, 1, 1, 128); else PB_NORM_FWD(8, 1, 4, 128); }
   else if (nv <= 16) { if (few) PB_NORM_FWD(16, 1, 1, 128); else PB_NORM_FWD(16, 1, 4, 128); }
   else if (nv <= 32) { if (few) PB_NORM_FWD(32, 1, 1, 128); else PB_NORM_FWD(32, 1, 4, 128); }
   else if (nv <= 64) { if (few) PB_NORM_FWD(32, 2, 1, 128); else PB_NORM_FWD(32, 2, 2, 128); }
-  else if (nv <= 128) { if (few) PB_NORM_FWD(128, 1, 1, 128); else PB_NORM_FWD(32, 4, 1, 128); }
-  else if (nv <= 256) { if (few) PB_NORM_FWD(256, 1, 1, 256); else PB_NORM_FWD(64, 4, 1, 128); }
+  else if (nv <= 128 && rows * nv >= 148 * 256L) PB_NORM_FWD(32, 4, 1, 128);
+  else if (nv <= 256) PB_NORM_FWD(64, 4, 1, 128);
   else if (nv <= 512) PB_NORM_FWD(128, 4, 1, 128);
   else if (nv <= 1024) PB_NORM_FWD(256, 4, 1, 256);
-  else PB_NORM_FWD(512, 4, 1, 512);
+  else PB_NORM_FWD(256, 8, 1, 256);
 #undef PB_NORM_FWD
 }
 
@@ -339,6 +341,17 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // CTAs (= partial rows) of the backward: two per SM, fewer when there are fewer rows
 constexpr int BWD_MAX_PARTIALS = 296;
 
+// CTAs that `rows` rows of H channels keep busy, out of at most P.  Every CTA's partial row costs the reduction as much as a row
+// of the CTA's own, so few rows take one CTA per SM, and short ones (a warp or less per row) one per eight rows: 200 rows of
+// 128 4.5 us instead of 5.9, 290 of 1536 5.5 instead of 6.4.
+inline bool bwd_row_per_warp(long rows, int H) { return H <= 512 || (H <= 1024 && rows >= 148 * 16); }
+inline int bwd_ctas(int P, long rows, int H) {
+  long n = P;
+  if (bwd_row_per_warp(rows, H)) { if (rows < 148 * 16) n = (rows + 7) / 8 < 148 ? (rows + 7) / 8 : 148; }
+  else if (rows <= 148 * 4) n = 148;
+  return (int)(n < P ? n : P);
+}
+
 template <int VPT, int THREADS, bool RES>
 int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
                             const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, long rows,
@@ -371,7 +384,9 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
   if (nv <= 16) { if (few) PB_NORM_BWD_SHORT(16, 1, 1) else PB_NORM_BWD_SHORT(16, 1, 4) }
   if (nv <= 32) { if (few) PB_NORM_BWD_SHORT(32, 1, 1) else PB_NORM_BWD_SHORT(32, 1, 4) }
   if (nv <= 64) PB_NORM_BWD_SHORT(32, 2, 2)
-  if (nv <= 128) PB_NORM_BWD_SHORT(32, 4, 1)
+  // (a row per warp leaves most warps without one up to some two thousand rows: 40 rows of 1024 4.8 us with a row per CTA, 6.7
+  // with a row per warp, 1500 rows 8.3 and 9.7 us, 8192 rows 19.4 and 18.8 us)
+  if (bwd_row_per_warp(rows, H)) PB_NORM_BWD_SHORT(32, 4, 1)
   if (nv <= 256) PB_NORM_BWD(1, 256);
   if (nv <= 512) PB_NORM_BWD(2, 256);
   if (nv <= 1024) PB_NORM_BWD(4, 256);
@@ -539,7 +554,8 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
 
 int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                 float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
-  // every one of the P partial rows is fully written by its CTA before the reduction reads it
+  // every one of the partial rows is fully written by its CTA before the reduction reads it
+  P = bwd_ctas(P, rows, H);
   const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
                                     (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, H, ldx, lddy);
   if (rc) return rc;
