@@ -103,6 +103,9 @@ __device__ __forceinline__ uint32_t abs_pair(uint32_t a) { return a & 0x7fff7fff
 __device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
+// strip of 32 rows of this warp (a CTA of more than four warps has several on every strip, which share its parts)
+__device__ __forceinline__ int strip() { return (threadIdx.x >> 5) & 3; }
+
 // Quantises part `h` of this warp's strip -- 8 CG columns, held in d[CG] -- into q_row / q_col (either may be null).  CG = 8:
 // the layout above (two halves); CG = 4: quarters, lane (cg = lane & 3, sub = lane >> 2) holds rows 8 i + sub (i < 4), half
 // the registers for one more shuffle per column pair.  p: offset of the lane's first element in the [R, C] tensor.
@@ -111,7 +114,7 @@ __device__ __forceinline__ void quantize_half(const uint4 (&d)[CG], int h, long 
                                               uint8_t* __restrict__ q_col, TileScales* scales, int fixed_e = 0,
                                               const uint8_t* e_rowv = nullptr, const uint8_t* e_colv = nullptr) {
   constexpr int SUBS = 32 / CG;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = strip();
   const int cg = lane % CG, sub = lane / CG;
   if (q_row) {
     uint32_t m[CG / 2];                 // block maxima of the lane's rows 2 j, 2 j + 1
@@ -202,8 +205,8 @@ __device__ __forceinline__ void store_scales(const TileScales* scales, int R, in
 // element offset of a lane: row `sub` of its warp's strip, first of its 8 columns of part 0
 template <int CG = 8>
 __device__ __forceinline__ long lane_offset(int row0, int col0, long ld) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  return (long)(row0 + warp * 32 + lane / CG) * ld + col0 + (lane % CG) * 8;
+  const int lane = threadIdx.x & 31;
+  return (long)(row0 + strip() * 32 + lane / CG) * ld + col0 + (lane % CG) * 8;
 }
 
 __device__ __forceinline__ void load_tile(const __nv_bfloat16* __restrict__ x, long p, int C, uint4 (&d)[2][8]) {
@@ -378,15 +381,18 @@ __device__ __forceinline__ uint4 bf8_pack(const float* f) {
 // SwiGLU forward fused with the quantisation of its output: h1 [T, 2I] = [gate | up] -> MXFP8 of
 // act[T, I] = silu(gate) * up (rounded to bf16 first, so the values equal quantising the un-fused kernel's output).
 // Four rows' loads in flight per lane and round keep it at 80 registers: six CTAs (24 warps) per SM hide the two special-
-// function operations per element, which four CTAs did not (132 us at 8192 x 14336).
-__global__ void __launch_bounds__(QT, 6)
+// function operations per element, which four CTAs did not (132 us at 8192 x 14336).  WIDE: as many warps per strip as it has
+// parts, for tensors of at most a tile per SM, where a warp's parts one after the other are the time (1024 x 1408: 5.4 -> 4.9
+// us, backward 10.4 -> 7.2); with several CTAs per SM the parts' registers are better spent on more CTAs.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 2 * QT : QT, WIDE ? 2 : 6)
 swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, float clamp, uint8_t* __restrict__ q_row,
                           uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
   __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
   const long pin = lane_offset(row0, col0, 2L * I), p = lane_offset(row0, col0, I);
 #pragma unroll 1
-  for (int h = 0; h < 2; ++h) {
+  for (int h = WIDE ? threadIdx.x / QT : 0; h < 2; h += WIDE ? 2 : 1) {
     uint4 d[8];
 #pragma unroll
     for (int i0 = 0; i0 < 8; i0 += 4) {
@@ -421,11 +427,11 @@ swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, fl
 }
 
 // SwiGLU backward fused with the quantisation of its output: (h1 [T, 2I], dact [T, I]) -> MXFP8 (both directions) of
-// dh1 [T, 2I] = [dgate | dup].  One CTA per 128 x 128 tile of the activation: it reads gate, up and dact once, stages
-// the dgate and the dup tile, and quantises one after the other.
+// dh1 [T, 2I] = [dgate | dup].  One CTA per 128 x 128 tile of the activation, which reads gate, up and dact once.
 // A warp computes the dgate and the dup values of its strip by 32 x 32 quarters: the twelve loads of a quarter are in
-// flight per lane, and two results of 16 registers instead of 32 let five CTAs share an SM instead of three.
-__global__ void __launch_bounds__(QT, 5)
+// flight per lane, and two results of 16 registers instead of 32 let five CTAs share an SM instead of three.  WIDE: as above.
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 4 * QT : QT, WIDE ? 1 : 5)
 swiglu_bwd_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, const __nv_bfloat16* __restrict__ dact, int T, int I,
                               float clamp, uint8_t* __restrict__ q_row, uint8_t* __restrict__ sf_row,
                               uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
@@ -433,7 +439,7 @@ swiglu_bwd_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, const __nv_b
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
   const long pin = lane_offset<4>(row0, col0, 2L * I), pd = lane_offset<4>(row0, col0, I);
 #pragma unroll 1
-  for (int h = 0; h < 4; ++h) {
+  for (int h = WIDE ? threadIdx.x / QT : 0; h < 4; h += WIDE ? 4 : 1) {
     uint4 dg[4], du[4], da[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -561,7 +567,9 @@ int pb_quant_fp8_blockwise(const void* x, int R, int C, int tilewise, void* q_ro
 int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row, void* sf_row, void* q_col,
                           void* sf_col, cudaStream_t s) {
   if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
-  swiglu_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), QT, 0, s>>>(
+  const dim3 grid(I / TILE, T / TILE);
+  const bool wide = (long)grid.x * grid.y <= 148;
+  (wide ? swiglu_quant_mxfp8_kernel<true> : swiglu_quant_mxfp8_kernel<false>)<<<grid, wide ? 2 * QT : QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -571,7 +579,9 @@ int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row
 int pb_swiglu_bwd_quant_mxfp8(const void* h1, const void* dact, int T, int I, float clamp, void* q_row, void* sf_row,
                               void* q_col, void* sf_col, cudaStream_t s) {
   if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
-  swiglu_bwd_quant_mxfp8_kernel<<<dim3(I / TILE, T / TILE), QT, 0, s>>>(
+  const dim3 grid(I / TILE, T / TILE);
+  const bool wide = (long)grid.x * grid.y <= 148;
+  (wide ? swiglu_bwd_quant_mxfp8_kernel<true> : swiglu_bwd_quant_mxfp8_kernel<false>)<<<grid, wide ? 4 * QT : QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
       reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
       reinterpret_cast<uint8_t*>(sf_col));
