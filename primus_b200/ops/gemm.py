@@ -226,7 +226,7 @@ _ONE_CTA, _CTA_PAIR = 0, 1          # routes of a bf16 GEMM; s > 1: CTA pairs wi
 
 
 @functools.lru_cache(maxsize=4096)
-def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, max_ctas: int) -> int:
+def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, out_bytes: int, max_ctas: int) -> int:
     """The route that takes the least time by a model of the three (microseconds, fitted to 190 shapes of 64 to 16384 in three
     layouts, each route timed; the choice is within 1 % of the best one on average, where the pair kernel for every output of
     at least 256 x 256 was 20 % slower than the one-CTA kernel on outputs of one wave and up to 50 % on ragged ones).
@@ -236,7 +236,8 @@ def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, max_ctas: int) 
     operand traffic per product, a third above the pair's: 15 % in the layout whose operands both need a transposed read, 4
     and 14 % with two and more waves (8192 x 4096 x 4096: 194 against 180 us), and far more where the rows of B start off a
     64-byte boundary and every 128-byte row of a box touches another sector or line (3152 x 584 x 8656, K-major A: 73 against
-    50 us).
+    50 us).  Where writing the output (``out_bytes`` an element, 8 when it is added to) outlasts the products there is nothing to
+    gain from fewer operand bytes (768 x 32000 x 256, accumulating: 39 us, 41 in pairs).
     Parts of a split reduction fill CTA pairs that few tiles leave idle; they pay 3.2 us for the second kernel and the trip of
     their fp32 sums (1024 x 1024: K = 4096 24 -> 16 us in four parts, K = 1024 9.8 -> 12.7 us in two)."""
     step, ctas = 0.28, max_ctas or _SMS
@@ -249,7 +250,9 @@ def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, max_ctas: int) 
     one_step = step * (1.15 if both_mn else 1.0) * (1.0, 1.04, 1.14)[min(waves, 3) - 1] * (1.8 if off_32 else 1.25 if off_64 else 1.0)
     best = (waves * steps * one_step, _ONE_CTA)
     if M >= 256 and N >= 256 and pairs:
-        best = min(best, (1.1 + -(-pair_tiles // pairs) * steps * pair_step, _CTA_PAIR))
+        products = -(-pair_tiles // pairs) * steps * pair_step
+        if products >= 0.6 * out_bytes * M * N / 6.5e6:
+            best = min(best, (1.1 + products, _CTA_PAIR))
     if N % 4 == 0 and max_ctas == 0:      # (a caller that leaves SMs to other work does not get a second kernel)
         for parts in range(2, min(pairs // pair_tiles, steps // 8) + 1):
             best = min(best, (3.2 + -(-steps // parts) * pair_step + 8 * parts * M * N / 12e6, parts))
@@ -262,7 +265,7 @@ def launch_bf16(a, b, out, M: int, N: int, K: int, a_mn: bool, b_mn: bool, mode:
     ``two_cta``: the CTA-pair kernel (None: chosen by the sizes, a split reduction among the choices)."""
     route = int(two_cta or 0)
     if two_cta is None and block_n == 256:
-        route = _bf16_route(M, N, K, a_mn and b_mn, b.stride(0), max_ctas)
+        route = _bf16_route(M, N, K, a_mn and b_mn, b.stride(0), (2, 4, 8)[mode], max_ctas)
     if route > _CTA_PAIR:
         ws = torch.empty(route * (-(-M // 256) * 256) * N, dtype=torch.float32, device=a.device)
         _lib.call("gemm_bf16_splitk", a, b, out, ws, M, N, K, a.stride(0), b.stride(0), out.stride(0),

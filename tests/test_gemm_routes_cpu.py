@@ -15,18 +15,23 @@ ONE, PAIR = gemm._ONE_CTA, gemm._CTA_PAIR
     (128, 256, 512, ONE), (100, 100, 100, ONE),
 ])
 def test_route_of_a_size(M, N, K, route):
-    assert gemm._bf16_route(M, N, K, False, K, 0) == route
+    assert gemm._bf16_route(M, N, K, False, K, 2, 0) == route
 
 
 def test_route_splits_long_reductions_of_few_tiles():
     for M, N, K in ((768, 256, 32000), (100, 2048, 8192), (16, 4096, 4096), (1536, 1536, 8192)):
-        parts = gemm._bf16_route(M, N, K, False, K, 0)
+        parts = gemm._bf16_route(M, N, K, False, K, 2, 0)
         assert 1 < parts <= -(-K // 64)
         assert parts * -(-M // 256) * -(-N // 256) <= 74
-        assert gemm._bf16_route(M, N - 2, K, False, K, 0) < 2          # the sums are added four columns at a time
-        assert gemm._bf16_route(M, N, K, False, K, 64) < 2             # SMs left to other work
+        assert gemm._bf16_route(M, N - 2, K, False, K, 2, 0) < 2          # the sums are added four columns at a time
+        assert gemm._bf16_route(M, N, K, False, K, 2, 64) < 2             # SMs left to other work
 
 
 def test_route_leaves_the_pair_kernel_to_calls_with_two_ctas():
-    assert gemm._bf16_route(8192, 8192, 8192, False, 8192, 1) == ONE
-    assert gemm._bf16_route(8192, 8192, 8192, False, 8192, 32) == PAIR
+    assert gemm._bf16_route(8192, 8192, 8192, False, 8192, 2, 1) == ONE
+    assert gemm._bf16_route(8192, 8192, 8192, False, 8192, 2, 32) == PAIR
+
+
+def test_route_of_a_gemm_that_its_output_bounds():
+    assert gemm._bf16_route(768, 32000, 256, True, 32000, 8, 0) == ONE
+    assert gemm._bf16_route(8192, 4096, 1024, True, 4096, 8, 0) == PAIR
