@@ -923,7 +923,7 @@ extern "C" int pb_moe_gather_rows(const void* x, const int* src, const float* sc
   moe_gather_rows_kernel<ROWS, VECS><<<moe_grid((R + ROWS - 1) / ROWS), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale, \
                                                                                      (__nv_bfloat16*)out, R, H, limit_rows)
   // (us, B200, before and now: 4096 tokens of 2048, 64 experts, eight copies 51 -> 43; 65536 of 256, two copies 44 -> 22)
-  if (H <= 256) PB_GATHER(4, 1); else PB_GATHER(1, 2);
+  if (H <= 256 && R >= 8192) PB_GATHER(4, 1); else PB_GATHER(1, 2);
 #undef PB_GATHER
   return (int)cudaGetLastError();
 }
