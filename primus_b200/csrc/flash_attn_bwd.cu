@@ -1,21 +1,20 @@
-// Flash-attention backward for sm_100a.
-//
-// Templated kernels run in two modes that share all plumbing:
+// Flash-attention backward for sm_100a: two passes that share all plumbing.
 //   MODE_DKDV: a CTA owns 128 KV rows of one KV head (resident tiles X1 = K, X2 = V) and streams
 //              tiles of Q / dO (Y1, Y2) of every query head of the group;
 //              S^T = K Q^T, dP^T = V dO^T  ->  P^T, dS^T  ->  dV += P^T dO,  dK += dS^T Q.
 //   MODE_DQ  : a CTA owns 128 query rows of one head (X1 = Q, X2 = dO) and streams tiles of
 //              K / V;  S = Q K^T, dP = dO V^T  ->  dS  ->  dQ += dS K.
-// In both modes the accumulators live in tensor memory for the whole loop (no atomics, results are
+// In both the accumulators live in tensor memory for the whole loop (no atomics, results are
 // bit-reproducible), and the streamed tiles are used twice from one shared-memory copy (K-major operand for
 // the first GEMM, MN-major operand for the second).  The softmax threads turn S / dP into bf16 P / dS *in tensor
 // memory*, 8 packed columns per 16 values, and the second GEMM takes its A operand from there (`tcgen05.mma` with A in
 // TMEM), one 16-wide K step per column group.  Nothing but mbarriers goes through shared memory between the two GEMMs of
 // a step.
-//   flash_attn_bwd_kernel       64-row steps: the multi-latent head shape (d_qk 192, d_v 128), whose accumulators leave
-//                               too little tensor memory for wider ones.  Two teams of 256 softmax threads work on
-//                               alternating steps while the MMA thread runs ahead.
-//   flash_attn_bwd_wide_kernel  128-row steps: d_qk == d_v.
+//   flash_attn_bwd_wide_kernel  128-row steps: both passes of the heads with d_qk == d_v, the dQ pass of the multi-latent
+//                               head shape (d_qk 192, d_v 128).
+//   flash_attn_bwd_kernel       64-row steps: the dK / dV pass of the multi-latent shape, whose accumulators leave too little
+//                               tensor memory for wider ones.  Two teams of 256 softmax threads work on alternating
+//                               steps while the MMA thread runs ahead.
 //
 // Replaces the backward of `flash_attn_func` (primus/backends/megatron/core/extensions/
 // primus_turbo.py:812-823); deterministic by construction (cf. the `deterministic=` flag there, :805).
@@ -35,18 +34,14 @@ constexpr int XATOM = 128 * 128;  // bytes of a [128 rows x 64 bf16] atom
 constexpr int YATOM = 64 * 128;   // bytes of a [64 rows x 64 bf16] atom
 enum { MODE_DKDV = 0, MODE_DQ = 1 };
 
-template <int DQK, int DV, int MODE>
+template <int DQK, int DV>
 struct BwCfg {
-  static constexpr int ACC_COLS = (MODE == MODE_DKDV) ? (DQK + DV) : DQK;
-  // S / dP buffers in tensor memory: 2 when they fit next to the accumulators, else 1
-  static constexpr int SBUF = (ACC_COLS + 256 <= 512) ? 2 : 1;
-  // When only one S / dP pair fits next to the accumulators (192 / 128-wide heads, dK / dV pass), the columns are split
-  // into two S buffers and one dP buffer: P and dS are both packed into the step's S columns (8 + 8 of every 16), so the
-  // dP buffer is free again as soon as the softmax threads have *read* it, and the S / dP GEMMs of a step run under the
-  // softmax of the step before instead of after it.
-  static constexpr bool SPLIT = SBUF == 1;
-  static constexpr int DP_COL = SPLIT ? 2 * BC : BC;     // dP columns: of the region / relative to the step's S columns
-  static_assert(!SPLIT || ACC_COLS + 3 * BC <= 512, "tensor memory");
+  static constexpr int ACC_COLS = DQK + DV;
+  // Next to the accumulators there is room for three 64-column buffers: two of S and one of dP.  P and dS are both packed
+  // into the step's S columns (8 + 8 of every 16), so the dP buffer is free again as soon as the softmax threads have *read*
+  // it, and the S / dP GEMMs of a step run under the softmax of the step before instead of after it.
+  static constexpr int DP_COL = 2 * BC;                  // dP columns of the region behind the accumulators
+  static_assert(ACC_COLS + 3 * BC <= 512, "tensor memory");
   static constexpr int X1_BYTES = BR * DQK * 2;
   static constexpr int X2_BYTES = BR * DV * 2;
   static constexpr int Y1_BYTES = BC * DQK * 2;
@@ -67,7 +62,7 @@ struct BwBars {
   uint64_t s_full[2];  // per team
   uint64_t p_ready[2]; // per team: P / dS of its current step are in tensor memory (one arrival per warp)
   uint64_t acc_done;   // all MMAs of the CTA have completed
-  uint64_t dp_free;    // SPLIT: the softmax threads hold the step's dP in registers (one arrival per warp of the team)
+  uint64_t dp_free;    // the softmax threads hold the step's dP in registers (one arrival per warp of the team)
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -97,7 +92,7 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
       : "memory");
 }
 
-template <int DQK, int DV, int MODE, bool WIN>
+template <int DQK, int DV, bool WIN>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                       const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
@@ -111,7 +106,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   const float cap_b = (WIN && softcap > 0.f) ? softcap / scale : 0.f;
   // seq: query rows per sequence, seq_k: key rows per sequence, q_off: key position of query row 0 (multiple of 128);
   // window > 0 (causal self-attention only): a query sees its last `window` keys, itself included
-  using C = BwCfg<DQK, DV, MODE>;
+  using C = BwCfg<DQK, DV>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint8_t* x1_smem = smem;
@@ -124,28 +119,20 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int g = hq / hkv;
-  const int seq_x = (MODE == MODE_DKDV) ? seq_k : seq;   // stationary operand (K, V | Q, dO)
-  const int seq_y = (MODE == MODE_DKDV) ? seq : seq_k;   // streamed operand (Q, dO | K, V)
-  const int num_rb = seq_x / BR;
-  const int num_c = seq_y / BC;
+  const int num_c = seq / BC;
   const int qo = q_off / BC;                              // offset in streamed-tile units
   // grid (heads * batch, row blocks): blocks are issued x-fastest, so all heads of the longest row block start
   // first and the short ones fill the tail (work per block is proportional to the number of streamed tiles)
-  const int rb = (MODE == MODE_DKDV) ? blockIdx.y : (num_rb - 1 - blockIdx.y);
-  const int nxh = (MODE == MODE_DKDV) ? hkv : hq;
-  const int xhead = blockIdx.x % nxh;  // MODE_DKDV: kv head; MODE_DQ: query head
-  const int batch = blockIdx.x / nxh;
-  const int tok0 = batch * seq_x;
-  const int toky0 = batch * seq_y;
-  // streamed-tile schedule: MODE_DKDV streams the query tiles at or after this key block, MODE_DQ the key tiles at or
-  // before this query block (query row i sits at key position q_off + i)
-  const int c_start = (MODE == MODE_DKDV) ? (causal ? max(0, 2 * rb - qo) : 0)
-                                          : (window > 0 ? max(0, rb * BR + q_off - window + 1) / BC : 0);
-  const int c_end = (MODE == MODE_DKDV)
-                        ? (window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BC + 1) : num_c)
-                        : (causal ? min(num_c, 2 * rb + 2 + qo) : num_c);
+  const int rb = blockIdx.y;
+  const int xhead = blockIdx.x % hkv;
+  const int batch = blockIdx.x / hkv;
+  const int tok0 = batch * seq_k;
+  const int toky0 = batch * seq;
+  // streamed-tile schedule: the query tiles at or after this key block (query row i sits at key position q_off + i)
+  const int c_start = causal ? max(0, 2 * rb - qo) : 0;
+  const int c_end = window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BC + 1) : num_c;
   const int n_per_head = max(0, c_end - c_start);
-  const int n_iter = (MODE == MODE_DKDV) ? g * n_per_head : n_per_head;
+  const int n_iter = g * n_per_head;
   volatile int* abort_flag = &bars->abort_flag;
   const float sl2 = scale * 1.4426950408889634f;
 
@@ -170,7 +157,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   __syncthreads();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-  const uint32_t tmem_sbuf = tmem_base + C::ACC_COLS;  // [buf][S 64 | dP 64], SPLIT: [S 64][S 64][dP 64]
+  const uint32_t tmem_sbuf = tmem_base + C::ACC_COLS;  // [S 64][S 64][dP 64]
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
@@ -185,11 +172,10 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         pb::tma_load_3d(x2_smem + a * XATOM, &tmX2, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
       for (int i = 0; i < n_iter && ok; ++i) {
         const int st = i % C::NS;
-        const int yhead = (MODE == MODE_DKDV) ? (xhead * g + i / n_per_head) : (xhead / g);
+        const int yhead = xhead * g + i / n_per_head;
         const int cs = c_start + i % n_per_head;
         BW_WAIT(&bars->y_empty[st], ((i / C::NS) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
-        const uint32_t bytes = C::Y1_BYTES + C::Y2_BYTES + (MODE == MODE_DKDV ? C::STAT_BYTES : 0);
-        pb::mbar_expect_tx(&bars->y_full[st], bytes);
+        pb::mbar_expect_tx(&bars->y_full[st], C::STAGE_BYTES);
 #pragma unroll
         for (int a = 0; a < DQK / 64; ++a)
           pb::tma_load_3d(y1_smem + st * C::Y1_BYTES + a * YATOM, &tmY1, &bars->y_full[st], a * 64, yhead,
@@ -198,11 +184,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         for (int a = 0; a < DV / 64; ++a)
           pb::tma_load_3d(y2_smem + st * C::Y2_BYTES + a * YATOM, &tmY2, &bars->y_full[st], a * 64, yhead,
                           toky0 + cs * BC);
-        if (MODE == MODE_DKDV) {
-          const long off = ((long)batch * hq + yhead) * seq + cs * BC;
-          bulk_load_1d(stat_smem + st * 128, lse + off, 256, &bars->y_full[st]);
-          bulk_load_1d(stat_smem + st * 128 + 64, delta + off, 256, &bars->y_full[st]);
-        }
+        const long off = ((long)batch * hq + yhead) * seq + cs * BC;
+        bulk_load_1d(stat_smem + st * 128, lse + off, 256, &bars->y_full[st]);
+        bulk_load_1d(stat_smem + st * 128 + 64, delta + off, 256, &bars->y_full[st]);
       }
     }
   } else if (warp == 1) {
@@ -213,8 +197,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
       const uint32_t x1a = pb::smem_u32(x1_smem), x2a = pb::smem_u32(x2_smem);
       bool ok = true;
-      auto s_cols = [&](int i) { return tmem_sbuf + (C::SPLIT ? (i & 1) * BC : (i % C::SBUF) * 128); };
-      auto dp_cols = [&](int i) { return C::SPLIT ? tmem_sbuf + C::DP_COL : s_cols(i) + C::DP_COL; };
+      auto s_cols = [&](int i) { return tmem_sbuf + (i & 1) * BC; };
       auto issue_s = [&](int i) {
         const uint32_t y1a = pb::smem_u32(y1_smem + (i % C::NS) * C::Y1_BYTES);
 #pragma unroll
@@ -226,29 +209,27 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         const uint32_t y2a = pb::smem_u32(y2_smem + (i % C::NS) * C::Y2_BYTES);
 #pragma unroll
         for (int k = 0; k < DV / 16; ++k)
-          pb::umma_f16_ss(dp_cols(i), pb::make_smem_desc(x2a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
+          pb::umma_f16_ss(tmem_sbuf + C::DP_COL, pb::make_smem_desc(x2a + (k / 4) * XATOM + (k % 4) * 32, 0, 1024, 2),
                           pb::make_smem_desc(y2a + (k / 4) * YATOM + (k % 4) * 32, 0, 1024, 2), idesc_s, k > 0 ? 1u : 0u);
       };
-      auto issue_sdp = [&](int i) {
-        issue_s(i);
-        issue_dp(i);
-        pb::umma_commit(&bars->s_full[i & 1]);
-      };
-      // The S / dP GEMMs run SBUF steps ahead.  Step i + SBUF reuses the TMEM buffer of step i; it is issued after
-      // the second GEMMs of step i (same thread: the tensor pipe keeps the order), which themselves wait for the
-      // softmax threads to have replaced S / dP of step i by P / dS.
+      // S runs two steps ahead of the second GEMMs, dP one.  S of step i + 2 reuses the columns of step i; it is issued
+      // after the second GEMMs of step i (same thread: the tensor pipe keeps the order), which themselves wait for the
+      // softmax threads to have replaced S of step i by P / dS.
       do {
         BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_MMA);
-        for (int j = 0; j < (C::SPLIT ? 2 : C::SBUF) && j < n_iter && ok; ++j) {
+        for (int j = 0; j < 2 && j < n_iter && ok; ++j) {
           BW_WAIT(&bars->y_full[j % C::NS], (j / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
-          if (C::SPLIT && j == 1) issue_s(1);
-          else issue_sdp(j);
+          issue_s(j);
+          if (j == 0) {
+            issue_dp(0);
+            pb::umma_commit(&bars->s_full[0]);
+          }
         }
       } while (false);
       for (int i = 0; i < n_iter && ok; ++i) {
         const int st = i % C::NS;
-        if (C::SPLIT && i + 1 < n_iter) {     // S of step i + 1 is already on its way
+        if (i + 1 < n_iter) {                 // S of step i + 1 is already on its way
           BW_WAIT(&bars->dp_free, i & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
           issue_dp(i + 1);
@@ -258,24 +239,21 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         pb::tc_fence_after();
         const uint32_t y1a = pb::smem_u32(y1_smem + st * C::Y1_BYTES);
         const uint32_t y2a = pb::smem_u32(y2_smem + st * C::Y2_BYTES);
-        const uint32_t ts = s_cols(i), tds = C::SPLIT ? ts + 8 : ts + C::DP_COL;
-        if (MODE == MODE_DKDV) {
+        const uint32_t ts = s_cols(i);
 #pragma unroll
-          for (int k = 0; k < BC / 16; ++k)   // acc(DV) += P . Y2, A = packed P of K step k (TMEM columns 16k .. 16k+7)
-            pb::umma_f16_ts(tmem_base + DQK, ts + 16 * k, pb::make_smem_desc(y2a + k * 2048, YATOM, 1024, 2), idesc_a2,
-                            (i > 0 || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < BC / 16; ++k)     // acc(DV) += P . Y2, A = packed P of K step k (TMEM columns 16k .. 16k+7)
+          pb::umma_f16_ts(tmem_base + DQK, ts + 16 * k, pb::make_smem_desc(y2a + k * 2048, YATOM, 1024, 2), idesc_a2,
+                          (i > 0 || k > 0) ? 1u : 0u);
 #pragma unroll
         for (int k = 0; k < BC / 16; ++k)     // acc(DQK) += dS . Y1
-          pb::umma_f16_ts(tmem_base, tds + 16 * k, pb::make_smem_desc(y1a + k * 2048, YATOM, 1024, 2), idesc_a1,
+          pb::umma_f16_ts(tmem_base, ts + 8 + 16 * k, pb::make_smem_desc(y1a + k * 2048, YATOM, 1024, 2), idesc_a1,
                           (i > 0 || k > 0) ? 1u : 0u);
         pb::umma_commit(&bars->y_empty[st]);
-        const int in = i + (C::SPLIT ? 2 : C::SBUF);
+        const int in = i + 2;
         if (in < n_iter) {
           BW_WAIT(&bars->y_full[in % C::NS], (in / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
-          if (C::SPLIT) issue_s(in);
-          else issue_sdp(in);
+          issue_s(in);
         }
       }
       if (ok) pb::umma_commit(&bars->acc_done);
@@ -288,27 +266,18 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
     const int row = wq * 32 + lane;
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
     const int row_g = rb * BR + row;
-    float lse2_row = 0.f, delta_row = 0.f;
-    if (MODE == MODE_DQ) {
-      const long off = ((long)batch * hq + xhead) * seq + row_g;
-      lse2_row = lse[off];  // negated, in log2 units
-      delta_row = delta[off];
-    }
     bool ok = true;
     for (int i = team; i < n_iter && ok; i += BW_TEAMS) {
       const int st = i % C::NS;
       const int cs = c_start + i % n_per_head;
       BW_WAIT(&bars->s_full[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_EPILOGUE);
-      if (MODE == MODE_DKDV) {
-        BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
-      }
+      BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
       pb::tc_fence_after();
-      const uint32_t ts = tmem_sbuf + lane_addr + (C::SPLIT ? (i & 1) * BC : (i % C::SBUF) * 128) + half * BW_HALF;
-      const uint32_t tdp = C::SPLIT ? tmem_sbuf + lane_addr + C::DP_COL + half * BW_HALF : ts + C::DP_COL;
-      const uint32_t tds = C::SPLIT ? ts + 8 : tdp;    // where the packed dS goes
-      const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
+      const uint32_t ts = tmem_sbuf + lane_addr + (i & 1) * BC + half * BW_HALF;
+      const uint32_t tdp = tmem_sbuf + lane_addr + C::DP_COL + half * BW_HALF;
+      const int cs_rel = cs + qo;   // streamed tile index in the stationary block's frame
       // largest (query position - key position) inside this tile pair: beyond the window -> element-wise mask
-      const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BC + BC - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BC);
+      const int max_diff = cs_rel * BC + BC - 1 - rb * BR;
       const bool diag = (causal && (cs_rel >= 2 * rb) && (cs_rel <= 2 * rb + 1)) || (window > 0 && max_diff >= window);
       const float* st_lse = stat_smem + st * 128 + half * BW_HALF;
       const float* st_delta = st_lse + 64;
@@ -316,11 +285,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       pb::tmem_ld_32x32b_x32(ts, s);
       pb::tmem_ld_32x32b_x32(tdp, dp);
       pb::tmem_wait_ld();
-      if (C::SPLIT) {
-        pb::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) pb::mbar_arrive(&bars->dp_free);
-      }
+      pb::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) pb::mbar_arrive(&bars->dp_free);
       auto body = [&](auto diag_tag) {
         constexpr bool DIAG = decltype(diag_tag)::value;
 #pragma unroll
@@ -329,12 +296,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 #pragma unroll
           for (int e4 = 0; e4 < 16; e4 += 4) {
             const int c = kk * 16 + e4;
-            float4 l4 = make_float4(lse2_row, lse2_row, lse2_row, lse2_row);
-            float4 d4 = make_float4(delta_row, delta_row, delta_row, delta_row);
-            if (MODE == MODE_DKDV) {
-              l4 = *reinterpret_cast<const float4*>(st_lse + c);
-              d4 = *reinterpret_cast<const float4*>(st_delta + c);
-            }
+            const float4 l4 = *reinterpret_cast<const float4*>(st_lse + c);
+            const float4 d4 = *reinterpret_cast<const float4*>(st_delta + c);
             const float l2[4] = {l4.x, l4.y, l4.z, l4.w}, dl[4] = {d4.x, d4.y, d4.z, d4.w};
             float pv[4], dv[4];
 #pragma unroll
@@ -349,7 +312,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
               float p = pb::fast_exp2(fmaf(sv, sl2, l2[u]));   // (lse is stored negated)
               if (DIAG) {
                 const int col_g = cs_rel * BC + half * BW_HALF + c + u;
-                const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
+                const int diff = col_g - row_g;   // query - key position
                 if (diff < 0 || (window > 0 && diff >= window)) p = 0.f;
               }
               pv[u] = p;
@@ -360,9 +323,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
             dsk[e4 / 2] = pb::pack_bf16x2(dv[0], dv[1]);
             dsk[e4 / 2 + 1] = pb::pack_bf16x2(dv[2], dv[3]);
           }
-          // P / dS (bf16 pairs) replace the first 8 of the 16 S / dP columns of this K step (SPLIT: both go to S columns)
-          if (MODE == MODE_DKDV) pb::tmem_st_32x32b_x8(ts + 16 * kk, pk);
-          pb::tmem_st_32x32b_x8(tds + 16 * kk, dsk);
+          // P and dS (bf16 pairs) replace the 16 S columns of this K step
+          pb::tmem_st_32x32b_x8(ts + 16 * kk, pk);
+          pb::tmem_st_32x32b_x8(ts + 8 + 16 * kk, dsk);
         }
       };
       if (diag) body(std::true_type{}); else body(std::false_type{});
@@ -396,18 +359,16 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         }
       };
       drain(0, DQK, x1_smem);
-      if (MODE == MODE_DKDV) drain(DQK, DV, x2_smem);
+      drain(DQK, DV, x2_smem);
       pb::fence_proxy_async_smem();
       pb::named_bar_sync(1, BW_COMPUTE);
       if (threadIdx.x == 64) {
 #pragma unroll
         for (int a = 0; a < DQK / 64; ++a)
           pb::tma_store_3d(&tmO1, x1_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
-        if (MODE == MODE_DKDV) {
 #pragma unroll
-          for (int a = 0; a < DV / 64; ++a)
-            pb::tma_store_3d(&tmO2, x2_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
-        }
+        for (int a = 0; a < DV / 64; ++a)
+          pb::tma_store_3d(&tmO2, x2_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
         pb::tma_store_commit();
         pb::tma_store_wait_all<0>();
       }
@@ -426,8 +387,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 }
 
 // ------------------------------------------------------------------------------------------------
-// 128-wide steps, for d_qk == d_v (64, 128) and the dQ pass of (192, 128).  A tcgen05.mma with N = 64 occupies the tensor pipe about as long as one with
-// N = 128, so the 64-row steps above pay twice for S and dP; and there the two second GEMMs of a step run only after its
+// 128-wide steps, for d_qk == d_v (64, 128) and the dQ pass of (192, 128).  A tcgen05.mma with N = 64 occupies the tensor
+// pipe about as long as one with N = 128, so the 64-row steps above pay twice for S and dP; and there the two second GEMMs of a step run only after its
 // whole softmax.  Here a step streams 128 rows, and its work is cut so that the tensor pipe always has some of it:
 //   * the softmax threads take P = exp2(S) as soon as S is there, before dP;
 //   * dS and the second GEMMs go by column halves A (64 columns) and B: the GEMMs of half A run while half B is computed;
@@ -1043,8 +1004,8 @@ int launch_bwd(const BwdArgs& a) {
             : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 0>),
            CKV, BWW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
   } else {
-    using CKV = BwCfg<DQK, DV, MODE_DKDV>;
-    PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, true> : flash_attn_bwd_kernel<DQK, DV, MODE_DKDV, false>), CKV,
+    using CKV = BwCfg<DQK, DV>;
+    PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, true> : flash_attn_bwd_kernel<DQK, DV, false>), CKV,
            BW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
   }
   using CQ = BwWideCfg<DQK, DV, MODE_DQ>;

@@ -74,13 +74,12 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, vo
 }
 
 // Warp-collective wait: lane 0 polls, the other lanes park at the shuffle (no issue slots, no shared-memory traffic).
-__device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int lane,
-                                                   unsigned backoff_ns) {
+__device__ __forceinline__ bool warp_wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int lane) {
   int got = 1;
   if (lane == 0 && !pb::mbar_try_wait(bar, parity)) {
     const long long t0 = clock64();
     while (!pb::mbar_try_wait(bar, parity)) {
-      if (backoff_ns) __nanosleep(backoff_ns);
+      __nanosleep(32);
       if (*abort_flag || clock64() - t0 > PB_WAIT_CYCLES) {
         got = 0;
         break;
@@ -257,7 +256,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       int mb, nb;
       tile_coords(tile, num_m, num_n, mb, nb);
       const int m0 = (mb * 2 + (int)cta) * BM + lane_grp * 32, n0 = nb * BN + half * HC;
-      if (!warp_wait_or_abort(&bars->tmem_full, acc_phase, abort_flag, lane, 32)) {
+      if (!warp_wait_or_abort(&bars->tmem_full, acc_phase, abort_flag, lane)) {
         atomicCAS(status, 0, PB_ERR_TIMEOUT_EPILOGUE);
         bars->abort_flag = 1;
         ok = false;

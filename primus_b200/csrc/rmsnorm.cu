@@ -651,7 +651,7 @@ float* g_noalloc_scratch_ptr[kMaxDevices] = {nullptr};
 extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void* w, const float* rstd,
                                       const void* dres, void* dx, float* dw, long rows, int H, long ldx,
                                       long lddy, int dw_accumulate, cudaStream_t s) {
-  // the kernels index rows with 32-bit integers: more than INT_MAX rows are rejected rather than truncated
+  // more than INT_MAX rows are outside the interface, as they are for pb_rmsnorm_bwd
   if (H <= 0 || H % 8 || ldx % 8 || lddy % 8 || rows < 0 || rows > 2147483647L) return PB_NOALLOC_ERR_BAD_ARG;
   if (H > PB_NOALLOC_MAX_H) return PB_NOALLOC_ERR_TOO_LARGE;  // the built-in scratch holds rows of <= 8192 floats
   if (rows == 0) return 0;
