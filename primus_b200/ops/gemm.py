@@ -237,7 +237,9 @@ def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, out_bytes: int,
     and 14 % with two and more waves (8192 x 4096 x 4096: 194 against 180 us), and far more where the rows of B start off a
     64-byte boundary and every 128-byte row of a box touches another sector or line (3152 x 584 x 8656, K-major A: 73 against
     50 us).  Where writing the output (``out_bytes`` an element, 8 when it is added to) outlasts the products there is nothing to
-    gain from fewer operand bytes (768 x 32000 x 256, accumulating: 39 us, 41 in pairs).
+    gain from fewer operand bytes (768 x 32000 x 256, accumulating: 39 us, 41 in pairs).  And over reductions of 512 and more
+    steps, in more than two waves, the pairs drift apart until they read most operands from memory instead of L2, 27 GB instead
+    of 16 for 8192 x 4096 x 128256: 7.1 against 6.4 ms, 7.4 against 7.0 at the power cap (K = 28672: 1.34 and 1.32, 1.50 and 1.50).
     Parts of a split reduction fill CTA pairs that few tiles leave idle; they pay 3.2 us for the second kernel and the trip of
     their fp32 sums (1024 x 1024: K = 4096 24 -> 16 us in four parts, K = 1024 9.8 -> 12.7 us in two)."""
     step, ctas = 0.28, max_ctas or _SMS
@@ -250,8 +252,9 @@ def _bf16_route(M: int, N: int, K: int, both_mn: bool, ldb: int, out_bytes: int,
     one_step = step * (1.15 if both_mn else 1.0) * (1.0, 1.04, 1.14)[min(waves, 3) - 1] * (1.8 if off_32 else 1.25 if off_64 else 1.0)
     best = (waves * steps * one_step, _ONE_CTA)
     if M >= 256 and N >= 256 and pairs:
-        products = -(-pair_tiles // pairs) * steps * pair_step
-        if products >= 0.6 * out_bytes * M * N / 6.5e6:
+        pair_waves = -(-pair_tiles // pairs)
+        products = pair_waves * steps * pair_step
+        if products >= 0.6 * out_bytes * M * N / 6.5e6 and (steps < 512 or pair_waves <= 2):
             best = min(best, (1.1 + products, _CTA_PAIR))
     if N % 4 == 0 and max_ctas == 0:      # (a caller that leaves SMs to other work does not get a second kernel)
         for parts in range(2, min(pairs // pair_tiles, steps // 8) + 1):

@@ -13,6 +13,7 @@ ONE, PAIR = gemm._ONE_CTA, gemm._CTA_PAIR
     (2048, 1024, 2048, ONE), (1536, 1536, 2048, ONE),      # half the pairs idle, but the parts' sums would cost more
     (4096, 4096, 4096, PAIR), (8192, 14336, 4096, PAIR), (4096, 128256, 2048, PAIR),
     (128, 256, 512, ONE), (100, 100, 100, ONE),
+    (8192, 4096, 128256, ONE), (8192, 4096, 28672, PAIR), (4096, 2048, 128256, PAIR),      # pairs drift apart over long K
 ])
 def test_route_of_a_size(M, N, K, route):
     assert gemm._bf16_route(M, N, K, False, K, 2, 0) == route
