@@ -86,14 +86,6 @@ def _bind(name: str, args, stream: bool):
     return bound
 
 
-def _run(name: str, fn, args, *stream) -> int:
-    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
-    try:
-        return fn(*plain, *stream)
-    except ctypes.ArgumentError:
-        return _bind(name, args, bool(stream))[0](*plain, *stream)
-
-
 # Number of device kernels each launcher enqueues (default 1); used for the launch counter below.
 _KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "sumsq": 2, "flash_attn_bwd": 3, "quant_fp8_tensorwise": 2, "quant_fp8_delayed": 2,
                      "gemm_bf16_splitk": 2, "qk_norm_bwd": 3}
@@ -105,7 +97,12 @@ def call(name: str, *args) -> None:
     global LAUNCH_COUNT
     fn, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
     LAUNCH_COUNT += kernels
-    rc = _run(name, fn, args, torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+    plain.append(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
+    try:
+        rc = fn(*plain)
+    except ctypes.ArgumentError:
+        rc = _bind(name, args, True)[0](*plain)
     if rc != 0:
         raise NativeLibraryError(f"pb_{name} failed with code {rc}")
 
@@ -113,7 +110,11 @@ def call(name: str, *args) -> None:
 def call_ret(name: str, *args) -> int:
     """Invoke a host-only helper that returns a value (no stream appended)."""
     fn, _ = _BOUND.get((name, False)) or _bind(name, args, False)
-    return _run(name, fn, args)
+    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+    try:
+        return fn(*plain)
+    except ctypes.ArgumentError:
+        return _bind(name, args, False)[0](*plain)
 
 
 class I32(int):
