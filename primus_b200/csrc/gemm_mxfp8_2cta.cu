@@ -11,8 +11,8 @@
 // The block scales travel with the operands: per K step a CTA loads the 512-byte scale block of its rows of A and the two of
 // the tile's 256 columns of B beside the operand stage, and the MMA thread copies them to tensor memory (`tcgen05.cp`, the
 // pair form: every CTA from its own shared memory) right in front of the stage's MMAs; the tensor pipe keeps the order, so
-// scales need no barrier of their own.  (Four warps per CTA that wrote them with `tcgen05.st`, handed over across the pair,
-// cost a quarter of the kernel: 714 us of 8192 x 28672 x 4096 against 544 us with the hand-over switched off.)
+// scales need no barrier of their own.  (Four warps per CTA that wrote them with `tcgen05.st`, handed over
+// across the pair, cost 3 to 5 % on random normal operands: 823 against 797 us for one launch of 8192 x 28672 x 4096.)
 //
 // Warp roles in both CTAs: warp 0 TMA producer, warp 1 MMA issuer (even CTA only), warps 2..9 epilogue (each CTA drains its
 // 128 rows through swizzled staging boxes and TMA stores / reduce-adds).

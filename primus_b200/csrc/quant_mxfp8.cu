@@ -381,7 +381,7 @@ __device__ __forceinline__ uint4 bf8_pack(const float* f) {
 // SwiGLU forward fused with the quantisation of its output: h1 [T, 2I] = [gate | up] -> MXFP8 of
 // act[T, I] = silu(gate) * up (rounded to bf16 first, so the values equal quantising the un-fused kernel's output).
 // Four rows' loads in flight per lane and round keep it at 80 registers: six CTAs (24 warps) per SM hide the two special-
-// function operations per element, which four CTAs did not (132 us at 8192 x 14336).  WIDE: as many warps per strip as it has
+// function operations per element (8192 x 14336, row direction: 107 us, 127 with the tile staged in shared memory).  WIDE: as many warps per strip as it has
 // parts, for tensors of at most a tile per SM, where a warp's parts one after the other are the time (1024 x 1408: 5.4 -> 4.9
 // us, backward 10.4 -> 7.2); with several CTAs per SM the parts' registers are better spent on more CTAs.
 template <bool WIDE>

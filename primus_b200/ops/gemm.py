@@ -1,5 +1,5 @@
-"""bf16 GEMM on the tcgen05 kernels (``csrc/gemm_bf16_2cta.cu``, CTA pairs; ``csrc/gemm_bf16.cu`` for small outputs) and the
-autograd linear built on them.
+"""bf16 GEMM on the tcgen05 kernels (``csrc/gemm_bf16_2cta.cu``, CTA pairs and split reductions; ``csrc/gemm_bf16.cu``, single
+CTAs) and the autograd linear built on them.
 
 ``gemm(a, b, a_mn, b_mn, out=..., accumulate=...)`` computes ``D = A . B^T`` where the logical
 operands are A[M,K] and B[N,K]; ``a_mn`` / ``b_mn`` say that the *stored* matrix is the transpose
