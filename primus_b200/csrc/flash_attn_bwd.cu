@@ -4,6 +4,8 @@
 //              S^T = K Q^T, dP^T = V dO^T  ->  P^T, dS^T  ->  dV += P^T dO,  dK += dS^T Q.
 //   MODE_DQ  : a CTA owns 128 query rows of one head (X1 = Q, X2 = dO) and streams tiles of
 //              K / V;  S = Q K^T, dP = dO V^T  ->  dS  ->  dQ += dS K.
+// Where the blocks are few or uneven, the CTAs of a cluster share a block's steps and add up their sums over distributed
+// shared memory, in the order of their ranks (bwd_cluster_size).
 // In both the accumulators live in tensor memory for the whole loop (no atomics, results are
 // bit-reproducible), and the streamed tiles are used twice from one shared-memory copy (K-major operand for
 // the first GEMM, MN-major operand for the second).  The softmax threads turn S / dP into bf16 P / dS *in tensor
@@ -54,6 +56,7 @@ struct BwCfg {
   // step, so at least three stages are needed to keep a load in flight behind the running step
   static constexpr int NS = NS_FIT >= 4 ? 4 : (NS_FIT >= 3 ? 3 : 2);
   static constexpr int SMEM_BYTES = FIXED_BYTES + NS * STAGE_BYTES;
+  static_assert(ACC_COLS * 4 * BR <= FIXED_BYTES - 1536 + NS * (Y1_BYTES + Y2_BYTES), "sums of a shared block");
 };
 
 struct BwBars {
@@ -92,13 +95,64 @@ __device__ __forceinline__ void bulk_load_1d(void* smem_dst, const void* gsrc, u
       : "memory");
 }
 
+// What a launch adds for blocks whose steps are shared by the CTAs of a cluster: the outputs as plain pointers.
+struct BwOut {
+  __nv_bfloat16 *p1, *p2;
+  long ld1, ld2;
+};
+
+__device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr) : "memory");
+  return v;
+}
+
+// Accumulators of a block whose steps were shared by the CTAs of a cluster: every CTA has left its fp32 sums in its shared
+// memory ([128 rows][C1 + C2], 16-byte chunks of a row XORed with row & 7); this CTA adds up a share of the rows, always in
+// the order of the ranks, and stores them.
+template <int C1, int C2>
+__device__ __forceinline__ void cluster_sum_rows(const uint8_t* stage, int rank, int csize, int tid, int nthreads, long row0,
+                                                 int head, const BwOut& out, float mul1) {
+  constexpr int GROUPS = (C1 + C2) / 8;
+  const int rows = BR / csize;
+  for (int it = tid; it < rows * GROUPS; it += nthreads) {
+    const int row = rank * rows + it / GROUPS, grp = it % GROUPS;
+    const uint32_t off = row * (C1 + C2) * 4;
+    const uint32_t o0 = off + (((2 * grp) ^ (row & 7)) << 4), o1 = off + (((2 * grp + 1) ^ (row & 7)) << 4);
+    float acc[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) acc[e] = 0.f;
+#pragma unroll 4
+    for (int p = 0; p < csize; ++p) {
+      const uint32_t base = pb::mapa_shared(stage, p);
+      const float4 a = ld_cluster_f4(base + o0), b = ld_cluster_f4(base + o1);
+      acc[0] += a.x; acc[1] += a.y; acc[2] += a.z; acc[3] += a.w;
+      acc[4] += b.x; acc[5] += b.y; acc[6] += b.z; acc[7] += b.w;
+    }
+    const bool first = grp < C1 / 8;
+    const float mul = first ? mul1 : 1.f;
+    __nv_bfloat16* dst = first ? out.p1 + (row0 + row) * out.ld1 + (long)head * C1 + grp * 8
+                               : out.p2 + (row0 + row) * out.ld2 + (long)head * C2 + (grp - C1 / 8) * 8;
+    *reinterpret_cast<uint4*>(dst) =
+        make_uint4(pb::pack_bf16x2(acc[0] * mul, acc[1] * mul), pb::pack_bf16x2(acc[2] * mul, acc[3] * mul),
+                   pb::pack_bf16x2(acc[4] * mul, acc[5] * mul), pb::pack_bf16x2(acc[6] * mul, acc[7] * mul));
+  }
+}
+// 32 columns of a row of the staging layout above
+__device__ __forceinline__ void stage_row_chunk(uint8_t* stage, int row_bytes, int row, int c32, const uint32_t* r) {
+#pragma unroll
+  for (int q = 0; q < 8; ++q)
+    *reinterpret_cast<uint4*>(stage + row * row_bytes + (((c32 * 8 + q) ^ (row & 7)) << 4)) =
+        make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+}
+
 template <int DQK, int DV, bool WIN>
 __global__ void __launch_bounds__(BW_THREADS, 1)
 flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_constant__ CUtensorMap tmX2,
                       const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
                       const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmO2,
                       const float* __restrict__ lse, const float* __restrict__ delta, int seq, int seq_k, int q_off,
-                      int hq, int hkv, float scale, int causal, int window_arg, float softcap_arg, int* status) {
+                      int hq, int hkv, float scale, int causal, int window_arg, float softcap_arg, const BwOut out, int* status) {
   const int window = WIN ? window_arg : 0;   // the instantiation without a window carries no code for it
   // softcap > 0: scores were softcap * tanh(scale * s / softcap) in the forward pass
   const float softcap = WIN ? softcap_arg : 0.f;
@@ -124,15 +178,17 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   // grid (heads * batch, row blocks): blocks are issued x-fastest, so all heads of the longest row block start
   // first and the short ones fill the tail (work per block is proportional to the number of streamed tiles)
   const int rb = blockIdx.y;
-  const int xhead = blockIdx.x % hkv;
-  const int batch = blockIdx.x / hkv;
+  const int csize = pb::cluster_nctarank(), rank = pb::cluster_ctarank();   // CTAs that share the block's steps
+  const int xhead = (blockIdx.x / csize) % hkv;
+  const int batch = blockIdx.x / csize / hkv;
   const int tok0 = batch * seq_k;
   const int toky0 = batch * seq;
   // streamed-tile schedule: the query tiles at or after this key block (query row i sits at key position q_off + i)
   const int c_start = causal ? max(0, 2 * rb - qo) : 0;
   const int c_end = window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BC + 1) : num_c;
   const int n_per_head = max(0, c_end - c_start);
-  const int n_iter = g * n_per_head;
+  const int i0 = g * n_per_head * rank / csize;           // first step of this CTA
+  const int n_iter = g * n_per_head * (rank + 1) / csize - i0;
   volatile int* abort_flag = &bars->abort_flag;
   const float sl2 = scale * 1.4426950408889634f;
 
@@ -172,8 +228,8 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
         pb::tma_load_3d(x2_smem + a * XATOM, &tmX2, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
       for (int i = 0; i < n_iter && ok; ++i) {
         const int st = i % C::NS;
-        const int yhead = xhead * g + i / n_per_head;
-        const int cs = c_start + i % n_per_head;
+        const int yhead = xhead * g + (i0 + i) / n_per_head;
+        const int cs = c_start + (i0 + i) % n_per_head;
         BW_WAIT(&bars->y_empty[st], ((i / C::NS) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
         pb::mbar_expect_tx(&bars->y_full[st], C::STAGE_BYTES);
 #pragma unroll
@@ -216,6 +272,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       // after the second GEMMs of step i (same thread: the tensor pipe keeps the order), which themselves wait for the
       // softmax threads to have replaced S of step i by P / dS.
       do {
+        if (n_iter == 0) break;
         BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_MMA);
         for (int j = 0; j < 2 && j < n_iter && ok; ++j) {
           BW_WAIT(&bars->y_full[j % C::NS], (j / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
@@ -267,9 +324,9 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
     const uint32_t lane_addr = uint32_t(wq * 32) << 16;
     const int row_g = rb * BR + row;
     bool ok = true;
+    int cs = n_iter > team ? c_start + (i0 + team) % n_per_head : 0;    // tile of the step, advanced at the end of the loop
     for (int i = team; i < n_iter && ok; i += BW_TEAMS) {
       const int st = i % C::NS;
-      const int cs = c_start + i % n_per_head;
       BW_WAIT(&bars->s_full[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_EPILOGUE);
       BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
       pb::tc_fence_after();
@@ -333,11 +390,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       pb::tc_fence_before();
       __syncwarp();
       if (lane == 0) pb::mbar_arrive(&bars->p_ready[i & 1]);   // one arrival per warp
+      cs += BW_TEAMS;
+      while (cs >= c_start + n_per_head) cs -= n_per_head;
     }
     // ---- epilogue: accumulators -> bf16 -> (dead) resident tiles -> TMA store
     do {
       if (!ok) break;
       BW_WAIT(&bars->acc_done, 0, PB_ERR_TIMEOUT_EPILOGUE);
+      BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);     // (long past, except for a CTA without a step)
       pb::tc_fence_after();
       auto drain = [&](uint32_t tcol, int ncols, uint8_t* dst) {
 #pragma unroll 1
@@ -345,6 +405,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
           uint32_t r[32];
           pb::tmem_ld_32x32b_x32(tmem_base + lane_addr + tcol + c * 32, r);
           pb::tmem_wait_ld();
+          if (n_iter == 0) {                      // nothing was accumulated: the columns are undefined
+#pragma unroll
+            for (int e = 0; e < 32; ++e) r[e] = 0u;
+          }
+          if (pb::cluster_nctarank() > 1) {
+            stage_row_chunk(smem, (DQK + DV) * 4, row, tcol / 32 + c, r);
+            continue;
+          }
           uint8_t* atom = dst + (c >> 1) * XATOM + row * 128;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -360,6 +428,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
       };
       drain(0, DQK, x1_smem);
       drain(DQK, DV, x2_smem);
+      if (pb::cluster_nctarank() > 1) break;
       pb::fence_proxy_async_smem();
       pb::named_bar_sync(1, BW_COMPUTE);
       if (threadIdx.x == 64) {
@@ -383,6 +452,11 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   if (warp == 1) {
     pb::tc_fence_after();
     pb::tmem_dealloc<1>(tmem_base, 512);
+  }
+  if (pb::cluster_nctarank() > 1) {
+    pb::cluster_sync();
+    cluster_sum_rows<DQK, DV>(smem, pb::cluster_ctarank(), pb::cluster_nctarank(), threadIdx.x, BW_THREADS, tok0 + (long)rb * BR, xhead, out, 1.f);
+    pb::cluster_sync();       // this CTA's sums may be read until here
   }
 }
 
@@ -418,6 +492,7 @@ struct BwWideCfg {
   static constexpr int NS = NS_FIT >= 4 ? 4 : NS_FIT;
   static constexpr int SMEM_BYTES = FIXED_BYTES + NS * STAGE_BYTES;
   static_assert(NS >= 2, "shared memory");
+  static_assert(ACC_COLS * 4 * BR <= FIXED_BYTES - 1536 + NS * (T1_BYTES + T2_BYTES), "sums of a shared block");
   static_assert(XA2_COL + (XA2 ? DV / 2 : 0) <= 512, "tensor memory");
 };
 constexpr int BWW_WARPS = 16;                       // softmax warps: thread = one resident row x 16 columns of each half
@@ -456,7 +531,8 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
                            const __grid_constant__ CUtensorMap tmY1, const __grid_constant__ CUtensorMap tmY2,
                            const __grid_constant__ CUtensorMap tmO1, const __grid_constant__ CUtensorMap tmO2,
                            const float* __restrict__ lse, const float* __restrict__ delta, int seq, int seq_k, int q_off,
-                           int hq, int hkv, float scale, int causal, int window_arg, float softcap_arg, int* status) {
+                           int hq, int hkv, float scale, int causal, int window_arg, float softcap_arg, const BwOut out,
+                           int* status) {
   using C = BwWideCfg<DQK, DV, MODE>;
   constexpr int BCW = C::BCW;
   constexpr bool CAP = VAR == 2;
@@ -484,8 +560,9 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   // longest row blocks first, as in the kernel above
   const int rb = (MODE == MODE_DKDV) ? blockIdx.y : (num_rb - 1 - blockIdx.y);
   const int nxh = (MODE == MODE_DKDV) ? hkv : hq;
-  const int xhead = blockIdx.x % nxh;
-  const int batch = blockIdx.x / nxh;
+  const int csize = pb::cluster_nctarank(), rank = pb::cluster_ctarank();   // CTAs that share the block's steps
+  const int xhead = (blockIdx.x / csize) % nxh;
+  const int batch = blockIdx.x / csize / nxh;
   const int tok0 = batch * seq_x;
   const int toky0 = batch * seq_y;
   const int c_start = (MODE == MODE_DKDV) ? (causal ? max(0, rb - qo) : 0)
@@ -494,7 +571,9 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
                         ? (window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BCW + 1) : num_c)
                         : (causal ? min(num_c, rb + 1 + qo) : num_c);
   const int n_per_head = max(0, c_end - c_start);
-  const int n_iter = (MODE == MODE_DKDV) ? g * n_per_head : n_per_head;
+  const int n_all = (MODE == MODE_DKDV) ? g * n_per_head : n_per_head;
+  const int i0 = n_all * rank / csize;                    // first step of this CTA
+  const int n_iter = n_all * (rank + 1) / csize - i0;
   volatile int* abort_flag = &bars->abort_flag;
   const float sl2 = scale * 1.4426950408889634f;
 
@@ -541,8 +620,8 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       for (int i = 0; i < n_iter && ok; ++i) {
         const int st = i % C::NS;
         const uint32_t par = ((i / C::NS) & 1) ^ 1;
-        const int yhead = (MODE == MODE_DKDV) ? (xhead * g + i / n_per_head) : (xhead / g);
-        const int cs = c_start + i % n_per_head;
+        const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
+        const int cs = c_start + (i0 + i) % n_per_head;
         if ((C::XA1 || C::XA2) && i == C::NS - 1) {
           BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
         }
@@ -714,9 +793,9 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         if (lane == 0) pb::mbar_arrive(&bars->xa_ready);
       } while (false);
     }
+    int cs = n_iter > 0 ? c_start + i0 % n_per_head : 0;    // tile of the step, advanced at the end of the loop
     for (int i = 0; i < n_iter && ok; ++i) {
       const int st = i % C::NS;
-      const int cs = c_start + i % n_per_head;
       if (MODE == MODE_DKDV) {
         BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
       }
@@ -815,6 +894,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         __syncwarp();
         if (lane == 0) pb::mbar_arrive(half == 0 ? &bars->pa[i & 1] : &bars->pb[i & 1]);
       }
+      if (++cs == c_end) cs = c_start;
     }
     // ---- epilogue: accumulators -> bf16 -> (dead) resident tiles -> TMA store
     do {
@@ -833,6 +913,10 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
 #pragma unroll
             for (int e = 0; e < 32; ++e) r[e] = 0u;
           }
+          if (pb::cluster_nctarank() > 1) {
+            stage_row_chunk(smem, C::ACC_COLS * 4, row, tcol / 32 + c, r);
+            continue;
+          }
           uint8_t* atom = dst + (c >> 1) * XATOM + row * 128;
 #pragma unroll
           for (int q4 = 0; q4 < 4; ++q4) {
@@ -847,6 +931,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       };
       drain(0, DQK, o1_smem, scale);
       if (MODE == MODE_DKDV) drain(DQK, DV, x2_smem, 1.f);
+      if (pb::cluster_nctarank() > 1) break;
       pb::fence_proxy_async_smem();
       pb::named_bar_sync(1, 32 * BWW_WARPS);
       if (threadIdx.x == 64) {
@@ -870,6 +955,12 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   if (warp == 1) {
     pb::tc_fence_after();
     pb::tmem_dealloc<1>(tmem_base, 512);
+  }
+  if (pb::cluster_nctarank() > 1) {
+    pb::cluster_sync();
+    cluster_sum_rows<DQK, MODE == MODE_DKDV ? DV : 0>(smem, pb::cluster_ctarank(), pb::cluster_nctarank(), threadIdx.x, BWW_THREADS, tok0 + (long)rb * BR, xhead,
+                                                      out, scale);
+    pb::cluster_sync();       // this CTA's sums may be read until here
   }
 }
 
@@ -963,6 +1054,55 @@ struct BwdArgs {
   cudaStream_t stream;
 };
 
+// How many CTAs (a cluster of 1, 2, 4 or 8) share the steps of one row block.  A pass takes the longer of its longest block
+// and its mean load per SM; a block more costs `fixed` microseconds for start and end, with a cluster more for the exchange
+// of the sums.  Few key / value heads leave long blocks and idle SMs: 4096 tokens, 32 query heads on 4 key / value heads of
+// 128 have 128 blocks of up to 256 steps but work for 114 steps per SM.  Measured (us, cluster 1 / 2 / 4 / 8), dK / dV pass:
+//   4096 x 32/4 x 128   484 / 265 / 314 / 442      1024 x 8/1 x 128   123 / 69 / 43 / 34     8192 x 1/1 x 128   126 / 72 / 61 / 129
+//   8192 x 32/8 x 128   910 / 948 / 1203 / 1736    2048 x 16/2 x 64   199 / 107 / 60 / 63    window 128, 64/8 x 64  76 / 97 / 141 / 268
+// dQ pass: 2048 x 32/8 x 128  65 / 104 / 211 / 457   8192 x 1/1 x 128  96 / 55 / 46 / 84.  The model below is within 10 % of
+// these.  Clusters of 4 and 8 do not fit every GPC: 132 and 120 CTAs in flight on 148 SMs.
+int bwd_cluster_size(int mode, int d_qk, int d_v, int batch, int seq, int seq_k, int q_off, int hq, int hkv, int causal,
+                     int window) {
+  const bool kv = mode == MODE_DKDV;
+  const int bc = kv && d_qk != d_v ? BC : BR;             // rows of a step
+  const int blocks = (kv ? seq_k : seq) / BR, tiles = (kv ? seq : seq_k) / bc;
+  double total = 0.;
+  int longest = 0;
+  for (int rb = 0; rb < blocks; ++rb) {                   // the kernels' own step ranges
+    int lo, hi;
+    if (kv) {
+      lo = causal ? (rb * BR - q_off) / bc : 0;
+      hi = window > 0 ? (rb * BR + BR + window - 2 - q_off) / bc + 1 : tiles;
+    } else {
+      lo = window > 0 ? (rb * BR + q_off - window + 1) / bc : 0;
+      hi = causal ? rb + 1 + q_off / bc : tiles;
+    }
+    lo = lo > 0 ? lo : 0;
+    hi = hi < tiles ? hi : tiles;
+    const int n = (hi > lo ? hi - lo : 0) * (kv ? hq / hkv : 1);
+    total += n;
+    longest = n > longest ? n : longest;
+  }
+  const double heads = (double)batch * (kv ? hkv : hq);
+  const double step = d_qk == 64 ? (kv ? 1.5 : 1.25) : d_qk == d_v ? (kv ? 1.95 : 1.5) : (kv ? 1.6 : 1.7);
+  static const double fixed_kv[4] = {5., 9., 14., 20.}, fixed_q[4] = {4., 8., 11., 14.}, sms[4] = {1., 1., 0.89, 0.81};
+  int best = 1;
+  double t_best = 0.;
+  for (int l = 0; l < 4; ++l) {
+    const int c = 1 << l;
+    const double fixed = (kv ? fixed_kv : fixed_q)[l];
+    const double alone = (longest + c - 1) / c * step + fixed;
+    const double mean = heads * (total * step + (double)blocks * c * fixed) / (sms[l] * pbh::sm_count());
+    const double t = alone > mean ? alone : mean;
+    if (l == 0 || t < 0.95 * t_best) {
+      best = c;
+      t_best = t;
+    }
+  }
+  return best;
+}
+
 template <int DQK, int DV>
 int launch_bwd(const BwdArgs& a) {
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
@@ -985,8 +1125,14 @@ int launch_bwd(const BwdArgs& a) {
 #undef MK
   const int var = a.softcap > 0.f ? 2 : (a.window > 0 ? 1 : 0);
   const float* lse2 = a.delta + (long)a.batch * a.hq * a.seq;
-  const dim3 grid_kv(a.hkv * a.batch, a.seq_k / BR, 1), grid_q(a.hq * a.batch, a.seq / BR, 1);
-#define PB_BWD(KERN, CFG, THREADS, GRID, X1, X2, Y1, Y2, O1, O2)                                                        \
+  auto cluster = [&](int mode) {
+    return bwd_cluster_size(mode, DQK, DV, a.batch, a.seq, a.seq_k, a.q_off, a.hq, a.hkv, a.causal, a.window);
+  };
+  const int c_kv = cluster(MODE_DKDV), c_q = cluster(MODE_DQ);
+  const dim3 grid_kv(a.hkv * a.batch * c_kv, a.seq_k / BR, 1), grid_q(a.hq * a.batch * c_q, a.seq / BR, 1);
+  const BwOut out_kv{(__nv_bfloat16*)a.dk, (__nv_bfloat16*)a.dv, a.dk_row, a.dv_row};
+  const BwOut out_q{(__nv_bfloat16*)a.dq, nullptr, a.dq_row, 0};
+#define PB_BWD(KERN, CFG, THREADS, GRID, CSIZE, OUT, X1, X2, Y1, Y2, O1, O2)                                                        \
   {                                                                                                                     \
     static bool attr_set[3] = {false, false, false};                                                                    \
     auto kern = KERN;                                                                                                   \
@@ -995,23 +1141,35 @@ int launch_bwd(const BwdArgs& a) {
       if (e != cudaSuccess) return (int)e;                                                                              \
       attr_set[var] = true;                                                                                             \
     }                                                                                                                   \
-    kern<<<GRID, THREADS, CFG::SMEM_BYTES, a.stream>>>(X1, X2, Y1, Y2, O1, O2, lse2, a.delta, a.seq, a.seq_k, a.q_off, a.hq, \
-                                                       a.hkv, a.scale, a.causal, a.window, a.softcap, a.status);        \
+    cudaLaunchConfig_t cfg = {};                                                                                        \
+    cfg.gridDim = GRID;                                                                                                 \
+    cfg.blockDim = dim3(THREADS);                                                                                       \
+    cfg.dynamicSmemBytes = CFG::SMEM_BYTES;                                                                             \
+    cfg.stream = a.stream;                                                                                              \
+    cudaLaunchAttribute attr[1];                                                                                        \
+    attr[0].id = cudaLaunchAttributeClusterDimension;                                                                   \
+    attr[0].val.clusterDim.x = CSIZE;                                                                                   \
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;                                                            \
+    cfg.attrs = attr;                                                                                                   \
+    cfg.numAttrs = CSIZE > 1 ? 1 : 0;                                                                                   \
+    cudaError_t e = cudaLaunchKernelEx(&cfg, kern, X1, X2, Y1, Y2, O1, O2, lse2, (const float*)a.delta, a.seq, a.seq_k, \
+                                       a.q_off, a.hq, a.hkv, a.scale, a.causal, a.window, a.softcap, OUT, a.status);    \
+    if (e != cudaSuccess) return (int)e;                                                                                \
   }
   if constexpr (DQK == DV) {
     using CKV = BwWideCfg<DQK, DV, MODE_DKDV>;
     PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 2>
             : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 0>),
-           CKV, BWW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
+           CKV, BWW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q64, do64, dk_m, dv_m)
   } else {
     using CKV = BwCfg<DQK, DV>;
     PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, true> : flash_attn_bwd_kernel<DQK, DV, false>), CKV,
-           BW_THREADS, grid_kv, k128, v128, q64, do64, dk_m, dv_m)
+           BW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q64, do64, dk_m, dv_m)
   }
   using CQ = BwWideCfg<DQK, DV, MODE_DQ>;
   PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 2>
           : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 0>),
-         CQ, BWW_THREADS, grid_q, q128, do128, k64, v64, dq_m, dq_m)
+         CQ, BWW_THREADS, grid_q, c_q, out_q, q128, do128, k64, v64, dq_m, dq_m)
 #undef PB_BWD
   return (int)cudaGetLastError();
 }
@@ -1036,6 +1194,12 @@ extern "C" int pb_flash_attn_bwd_cap(const void* d_o, const void* q, const void*
   if (d_qk == 192 && d_v == 128) return launch_bwd<192, 128>(a);
   if (d_qk == 64 && d_v == 64) return launch_bwd<64, 64>(a);
   return -3;
+}
+
+// CTAs per row block that pb_flash_attn_bwd_cap launches: pass 0 dK / dV, 1 dQ (host only).
+extern "C" int pb_flash_attn_bwd_cluster(int pass, int batch, int seq, int seq_k, int q_off, int hq, int hkv, int d_qk, int d_v,
+                                         int causal, int window) {
+  return bwd_cluster_size(pass, d_qk, d_v, batch, seq, seq_k, q_off, hq, hkv, causal, window);
 }
 
 extern "C" int pb_flash_attn_bwd_win(const void* d_o, const void* q, const void* k, const void* v, const void* o,
