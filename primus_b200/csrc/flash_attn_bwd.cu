@@ -217,7 +217,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       bool ok = true;
       pb::mbar_expect_tx(&bars->x_full, C::X1_BYTES + C::X2_BYTES);
 #pragma unroll
@@ -247,7 +247,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       constexpr uint32_t idesc_s = pb::make_idesc_bf16(BR, BC, 0, 0);
       constexpr uint32_t idesc_a1 = pb::make_idesc_bf16(BR, DQK, 0, 1);  // acc(DQK) += dS . Y1
       constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
@@ -608,7 +608,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       bool ok = true;
       pb::mbar_expect_tx(&bars->x_full, C::T1_BYTES + C::T2_BYTES);
 #pragma unroll
@@ -649,7 +649,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       constexpr uint32_t idesc_s = pb::make_idesc_bf16(BR, BCW, 0, 0);
       constexpr uint32_t idesc_a1 = pb::make_idesc_bf16(BR, DQK, 0, 1);  // acc(DQK) += dS . Y1
       constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2

@@ -140,7 +140,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       bool ok = true;
       pb::mbar_expect_tx(&bars->q_full, (active1 ? 2 : 1) * C::Q_BYTES);
       for (int t = 0; t < (active1 ? 2 : 1); ++t) {
@@ -167,7 +167,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       constexpr uint32_t idesc_s = pb::make_idesc_bf16(BQ, BKV, 0, 0);
       constexpr uint32_t idesc_o = pb::make_idesc_bf16(BQ, DV, 0, 1);
       bool ok = true;

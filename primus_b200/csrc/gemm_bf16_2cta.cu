@@ -151,7 +151,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -193,7 +193,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && cta == 0) {
+    if (cta == 0 && pb::elect_one()) {
       // ---------------------------------------------------------- MMA issuer (even CTA)
       constexpr uint32_t idesc = pb::make_idesc_bf16(2 * BM, BN, A_MN, B_MN);
       int stage = 0;

@@ -155,7 +155,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
 
   if (warp == 0) {
     // ---------------------------------------------------------------- TMA producer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -191,7 +191,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;

@@ -155,7 +155,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer (both CTAs)
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -190,7 +190,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && cta == 0) {
+    if (cta == 0 && pb::elect_one()) {
       // ---------------------------------------------------------- MMA issuer (even CTA)
       int stage = 0, set = 0;
       uint32_t phase = 0;

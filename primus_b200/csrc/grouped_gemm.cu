@@ -143,7 +143,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -184,7 +184,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (pb::elect_one()) {
       constexpr uint32_t idesc = pb::make_idesc_bf16(BM, BN, A_MN, B_MN);
       int stage = 0;
       uint32_t phase = 0;

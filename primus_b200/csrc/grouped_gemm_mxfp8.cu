@@ -153,7 +153,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   const uint32_t tmem_base = bars->tmem_base;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
@@ -222,7 +222,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (pb::elect_one()) {
       int stage = 0;
       uint32_t phase = 0;
       uint32_t acc_phase = 0;
