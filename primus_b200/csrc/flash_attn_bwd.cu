@@ -469,9 +469,12 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 //   * what frees a tensor-memory region is the *read* of it.  With two S buffers (64-wide heads) P and dS are packed into
 //     the step's S columns (8 + 8 of every 16) and the next dP starts as soon as this one is in registers; with one S
 //     buffer (128-wide) they are packed into the dP columns and the next S starts instead.
-// Streamed tiles sit in NS buffers of 128 rows, loaded and released by 64-row halves.  In the dQ pass of 128-wide heads the
-// resident tiles (Q, dO) move to tensor memory at the start, as A operands of the first GEMMs; their shared memory is the
-// third buffer.
+// The two streamed tiles of a step have rings of their own, NS1 and NS2 buffers of 128 rows: the tile of S is wanted a whole step before the tile of dP, and the dQ pass is done with V after dP.  In the dQ pass
+// of 128-wide heads the resident tiles (Q, dO) move to tensor memory at the start, as A operands of the first GEMMs; their
+// shared memory belongs to the rings.
+// A step of 128 x 128 x 128 holds four GEMMs of 512 clocks each in the dK / dV pass, three in the dQ pass; the passes take 2750
+// and 1960 clocks per step (3600 and 2600 with one ring of two or three buffers for both tiles: S waited for its tile).  8192 x
+// 32/8 x 128: dK / dV pass 924 -> 777 us; 4096 x 16 x 192/128: dQ pass 119 -> 101 us.
 template <int DQK, int DV, int MODE>
 struct BwWideCfg {
   static constexpr int BCW = 128;
@@ -485,14 +488,14 @@ struct BwWideCfg {
   static constexpr int XA2_COL = XA1_COL + (XA1 ? DQK / 2 : 0);
   static constexpr int T1_BYTES = BR * DQK * 2;                        // a [128, DQK] tile (X1, Y1)
   static constexpr int T2_BYTES = BR * DV * 2;                         // a [128, DV] tile (X2, Y2)
-  static constexpr int STAT_FLOATS = MODE == MODE_DKDV ? 256 : 0;      // per half: 64 lse, 64 delta
-  static constexpr int STAGE_BYTES = T1_BYTES + T2_BYTES + STAT_FLOATS * 4;
-  static constexpr int FIXED_BYTES = (XA1 ? 0 : T1_BYTES) + (XA2 ? 0 : T2_BYTES) + 1024 + 512;
-  static constexpr int NS_FIT = (232448 - FIXED_BYTES) / STAGE_BYTES;
-  static constexpr int NS = NS_FIT >= 4 ? 4 : NS_FIT;
-  static constexpr int SMEM_BYTES = FIXED_BYTES + NS * STAGE_BYTES;
-  static_assert(NS >= 2, "shared memory");
-  static_assert(ACC_COLS * 4 * BR <= FIXED_BYTES - 1536 + NS * (T1_BYTES + T2_BYTES), "sums of a shared block");
+  static constexpr int STAT = MODE == MODE_DKDV ? 128 : 0;             // statistics of a tile: lse with Y1, delta with Y2
+  static constexpr int X_BYTES = (XA1 ? 0 : T1_BYTES) + (XA2 ? 0 : T2_BYTES);
+  static constexpr int NS1 = DQK == 64 ? 4 : 3;
+  static constexpr int NS2 = DQK == 64 ? 4 : MODE == MODE_DKDV ? 2 : DQK == 128 ? 3 : 1;
+  static constexpr int TILE_BYTES = X_BYTES + NS1 * T1_BYTES + NS2 * T2_BYTES;
+  static constexpr int SMEM_BYTES = TILE_BYTES + (NS1 + NS2) * STAT * 4 + 512;
+  static_assert(SMEM_BYTES <= 232448, "shared memory");
+  static_assert(ACC_COLS * 4 * BR <= TILE_BYTES, "sums of a shared block");
   static_assert(XA2_COL + (XA2 ? DV / 2 : 0) <= 512, "tensor memory");
 };
 constexpr int BWW_WARPS = 16;                       // softmax warps: thread = one resident row x 16 columns of each half
@@ -500,8 +503,9 @@ constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
 
 struct BwWideBars {
   uint64_t x_full;
-  uint64_t y_full[4], ya_empty[4], yb_empty[4];
-  uint64_t s_full[2], dp_full;
+  uint64_t y1_full[4], y2_full[4];
+  uint64_t s_full[2];
+  uint64_t dp_full[4], done[4];   // by step: dP is there; all products of the step are.  They release the streamed tiles too
   uint64_t freed;          // the softmax threads hold S (one S buffer) or dP (two) of the step in registers
   uint64_t pa[2], pb[2];   // P / dS of half A / B are in tensor memory; by step parity, because with two S buffers a warp can
                            // be a step ahead of another
@@ -539,15 +543,16 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   const int window = VAR ? window_arg : 0;
   const float cap_a = CAP ? scale / softcap_arg : 0.f;
   const float cap_b = CAP ? softcap_arg / scale : 0.f;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* y1_smem = smem + (C::XA1 ? 0 : C::T1_BYTES) + (C::XA2 ? 0 : C::T2_BYTES);   // NS stages
-  uint8_t* y2_smem = y1_smem + C::NS * C::T1_BYTES;                                     // NS stages
-  // a resident tile that goes to tensor memory passes through the last stage's buffer before its first streamed tile
-  uint8_t* x1_smem = C::XA1 ? y1_smem + (C::NS - 1) * C::T1_BYTES : smem;
-  uint8_t* x2_smem = C::XA2 ? y2_smem + (C::NS - 1) * C::T2_BYTES : smem + (C::XA1 ? 0 : C::T1_BYTES);
-  float* stat_smem = reinterpret_cast<float*>(y2_smem + C::NS * C::T2_BYTES);   // NS x [64 lse A | 64 delta A | lse B | delta B]
-  BwWideBars* bars = reinterpret_cast<BwWideBars*>(stat_smem + C::NS * C::STAT_FLOATS);
+  extern __shared__ __align__(1024) uint8_t smem_wide[];
+  uint8_t* smem = smem_wide;
+  uint8_t* y1_smem = smem + C::X_BYTES;
+  uint8_t* y2_smem = y1_smem + C::NS1 * C::T1_BYTES;
+  // a resident tile that goes to tensor memory passes through the last buffer of a ring before its first streamed tile
+  uint8_t* x1_smem = C::XA1 ? y1_smem + (C::NS1 - 1) * C::T1_BYTES : smem;
+  uint8_t* x2_smem = C::XA2 ? y2_smem + (C::NS2 - 1) * C::T2_BYTES : smem + (C::XA1 ? 0 : C::T1_BYTES);
+  float* lse_smem = reinterpret_cast<float*>(y2_smem + C::NS2 * C::T2_BYTES);
+  float* delta_smem = lse_smem + C::NS1 * C::STAT;
+  BwWideBars* bars = reinterpret_cast<BwWideBars*>(delta_smem + C::NS2 * C::STAT);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -580,13 +585,13 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   if (threadIdx.x == 0) {
     pb::mbar_init(&bars->x_full, 1);
     for (int i = 0; i < 4; ++i) {
-      pb::mbar_init(&bars->y_full[i], 1);
-      pb::mbar_init(&bars->ya_empty[i], 1);
-      pb::mbar_init(&bars->yb_empty[i], 1);
+      pb::mbar_init(&bars->y1_full[i], 1);
+      pb::mbar_init(&bars->y2_full[i], 1);
+      pb::mbar_init(&bars->dp_full[i], 1);
+      pb::mbar_init(&bars->done[i], 1);
     }
     pb::mbar_init(&bars->s_full[0], 1);
     pb::mbar_init(&bars->s_full[1], 1);
-    pb::mbar_init(&bars->dp_full, 1);
     pb::mbar_init(&bars->freed, BWW_WARPS);
     for (int i = 0; i < 2; ++i) {
       pb::mbar_init(&bars->pa[i], BWW_WARPS);
@@ -617,34 +622,42 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
 #pragma unroll
       for (int a = 0; a < DV / 64; ++a)
         pb::tma_load_3d(x2_smem + a * XATOM, &tmX2, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
-      for (int i = 0; i < n_iter && ok; ++i) {
-        const int st = i % C::NS;
-        const uint32_t par = ((i / C::NS) & 1) ^ 1;
-        const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
-        const int cs = c_start + (i0 + i) % n_per_head;
-        if ((C::XA1 || C::XA2) && i == C::NS - 1) {
-          BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
-        }
-        for (int h = 0; h < 2 && ok; ++h) {
-          BW_WAIT(h == 0 ? &bars->ya_empty[st] : &bars->yb_empty[st], par, PB_ERR_TIMEOUT_TMA);
-          if (h == 0)
-            pb::mbar_expect_tx(&bars->y_full[st], C::STAGE_BYTES);
-          const int row = cs * BCW + h * 64;
+      auto load_y1 = [&](int i) {
+        const int st = i % C::NS1, rel = i - C::NS1;     // rel: the step that had the buffer
+        do {
+          if (C::XA1 && i == C::NS1 - 1) BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
+          if (rel >= 0) BW_WAIT(&bars->done[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
+          pb::mbar_expect_tx(&bars->y1_full[st], C::T1_BYTES + C::STAT * 4);
+          const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
+          const int row = (c_start + (i0 + i) % n_per_head) * BCW;
 #pragma unroll
           for (int a = 0; a < DQK / 64; ++a)
-            pb::tma_load_3d(y1_smem + st * C::T1_BYTES + a * XATOM + h * YATOM, &tmY1, &bars->y_full[st], a * 64, yhead,
-                            toky0 + row);
+            pb::tma_load_3d(y1_smem + st * C::T1_BYTES + a * XATOM, &tmY1, &bars->y1_full[st], a * 64, yhead, toky0 + row);
+          if (MODE == MODE_DKDV)
+            bulk_load_1d(lse_smem + st * C::STAT, lse + ((long)batch * hq + yhead) * seq + row, 512, &bars->y1_full[st]);
+        } while (false);
+      };
+      auto load_y2 = [&](int i) {
+        const int st = i % C::NS2, rel = i - C::NS2;
+        do {
+          if (C::XA2 && i == C::NS2 - 1) BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
+          // the dQ pass is done with V after dP
+          if (rel >= 0) BW_WAIT(MODE == MODE_DKDV ? &bars->done[rel & 3] : &bars->dp_full[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
+          pb::mbar_expect_tx(&bars->y2_full[st], C::T2_BYTES + C::STAT * 4);
+          const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
+          const int row = (c_start + (i0 + i) % n_per_head) * BCW;
 #pragma unroll
           for (int a = 0; a < DV / 64; ++a)
-            pb::tma_load_3d(y2_smem + st * C::T2_BYTES + a * XATOM + h * YATOM, &tmY2, &bars->y_full[st], a * 64, yhead,
-                            toky0 + row);
-          if (MODE == MODE_DKDV) {
-            const long off = ((long)batch * hq + yhead) * seq + row;
-            float* stat = stat_smem + st * C::STAT_FLOATS + h * 128;
-            bulk_load_1d(stat, lse + off, 256, &bars->y_full[st]);
-            bulk_load_1d(stat + 64, delta + off, 256, &bars->y_full[st]);
-          }
-        }
+            pb::tma_load_3d(y2_smem + st * C::T2_BYTES + a * XATOM, &tmY2, &bars->y2_full[st], a * 64, yhead, toky0 + row);
+          if (MODE == MODE_DKDV)
+            bulk_load_1d(delta_smem + st * C::STAT, delta + ((long)batch * hq + yhead) * seq + row, 512, &bars->y2_full[st]);
+        } while (false);
+      };
+      if (n_iter > 0) load_y1(0);
+      for (int i = 0; i < n_iter && ok; ++i) {      // in the order in which they are wanted and their buffers are free
+        if (C::NS2 == 1 && i + 1 < n_iter) load_y1(i + 1);
+        if (ok) load_y2(i);
+        if (C::NS2 != 1 && ok && i + 1 < n_iter) load_y1(i + 1);
       }
     }
   } else if (warp == 1) {
@@ -670,17 +683,17 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       auto issue_s = [&](int i) {
         issue_first(std::integral_constant<int, DQK>{}, std::bool_constant<C::XA1>{},
                     C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0), x1a, C::XA1_COL,
-                    pb::smem_u32(y1_smem + (i % C::NS) * C::T1_BYTES));
+                    pb::smem_u32(y1_smem + (i % C::NS1) * C::T1_BYTES));
         pb::umma_commit(&bars->s_full[C::NSB == 2 ? (i & 1) : 0]);
       };
       auto issue_dp = [&](int i) {
         issue_first(std::integral_constant<int, DV>{}, std::bool_constant<C::XA2>{}, C::DP_COL, x2a, C::XA2_COL,
-                    pb::smem_u32(y2_smem + (i % C::NS) * C::T2_BYTES));
-        pb::umma_commit(&bars->dp_full);
+                    pb::smem_u32(y2_smem + (i % C::NS2) * C::T2_BYTES));
+        pb::umma_commit(&bars->dp_full[i & 3]);
       };
       auto issue_second = [&](int i, int half) {                            // accumulators += (P, dS of the half) . Y
-        const int st = i % C::NS;
-        const uint32_t y1a = pb::smem_u32(y1_smem + st * C::T1_BYTES), y2a = pb::smem_u32(y2_smem + st * C::T2_BYTES);
+        const int st1 = i % C::NS1, st2 = i % C::NS2;
+        const uint32_t y1a = pb::smem_u32(y1_smem + st1 * C::T1_BYTES), y2a = pb::smem_u32(y2_smem + st2 * C::T2_BYTES);
         const uint32_t tp = tmem_base + (C::NSB == 2 ? C::S_COL + (i & 1) * BCW : C::DP_COL);
         if (MODE == MODE_DKDV) {
 #pragma unroll
@@ -696,7 +709,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
           pb::umma_f16_ts(tmem_base, tp + 16 * k + 8, pb::make_smem_desc(y1a + k * 2048, XATOM, 1024, 2), idesc_a1,
                           (i > 0 || k > 0) ? 1u : 0u);
         }
-        pb::umma_commit(half == 0 ? &bars->ya_empty[st] : &bars->yb_empty[st]);
+        if (half == 1) pb::umma_commit(&bars->done[i & 3]);
       };
       do {
         if (n_iter == 0) break;
@@ -704,12 +717,14 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         if (C::XA1 || C::XA2) {
           BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_MMA);
         }
-        BW_WAIT(&bars->y_full[0], 0, PB_ERR_TIMEOUT_MMA);
+        BW_WAIT(&bars->y1_full[0], 0, PB_ERR_TIMEOUT_MMA);
         pb::tc_fence_after();
         issue_s(0);
+        BW_WAIT(&bars->y2_full[0], 0, PB_ERR_TIMEOUT_MMA);
+        pb::tc_fence_after();
         issue_dp(0);
         if (C::NSB == 2 && n_iter > 1) {
-          BW_WAIT(&bars->y_full[1], 0, PB_ERR_TIMEOUT_MMA);
+          BW_WAIT(&bars->y1_full[1], 0, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
           issue_s(1);
         }
@@ -718,8 +733,10 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         // S of the next step (one S buffer) goes out at the first point at which its tile has arrived: the issuing thread
         // must not wait for a load while P / dS of this step are ready
         bool s_next = C::NSB == 2 || i + 1 >= n_iter;
-        uint64_t* y_next = &bars->y_full[(i + 1) % C::NS];
-        const uint32_t y_par = ((i + 1) / C::NS) & 1;
+        uint64_t* y_next = &bars->y1_full[(i + 1) % C::NS1];
+        const uint32_t y_par = ((i + 1) / C::NS1) & 1;
+        uint64_t* y2_next = &bars->y2_full[(i + 1) % C::NS2];
+        const uint32_t y2_par = ((i + 1) / C::NS2) & 1;
         auto try_s = [&]() {
           if (!s_next && mbar_test(y_next, y_par)) {
             pb::tc_fence_after();
@@ -729,6 +746,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         };
         if (i + 1 < n_iter) {
           BW_WAIT(&bars->freed, i & 1, PB_ERR_TIMEOUT_MMA);
+          if (C::NSB == 2) BW_WAIT(y2_next, y2_par, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
           if (C::NSB == 2) issue_dp(i + 1);
           else try_s();
@@ -746,9 +764,13 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
             pb::tc_fence_after();
             issue_s(i + 1);
           }
-          if (i + 1 < n_iter) issue_dp(i + 1);
+          if (i + 1 < n_iter) {
+            BW_WAIT(y2_next, y2_par, PB_ERR_TIMEOUT_MMA);
+            pb::tc_fence_after();
+            issue_dp(i + 1);
+          }
         } else if (i + 2 < n_iter) {
-          BW_WAIT(&bars->y_full[(i + 2) % C::NS], ((i + 2) / C::NS) & 1, PB_ERR_TIMEOUT_MMA);
+          BW_WAIT(&bars->y1_full[(i + 2) % C::NS1], ((i + 2) / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
           pb::tc_fence_after();
           issue_s(i + 2);
         }
@@ -795,9 +817,8 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
     }
     int cs = n_iter > 0 ? c_start + i0 % n_per_head : 0;    // tile of the step, advanced at the end of the loop
     for (int i = 0; i < n_iter && ok; ++i) {
-      const int st = i % C::NS;
       if (MODE == MODE_DKDV) {
-        BW_WAIT(&bars->y_full[st], (i / C::NS) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // lse / delta tile visible
+        BW_WAIT(&bars->y1_full[i % C::NS1], (i / C::NS1) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's lse is visible
       }
       const uint32_t ts = tmem_base + lane_addr + C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0) + 16 * qd;
       const uint32_t td = tmem_base + lane_addr + C::DP_COL + 16 * qd;
@@ -805,7 +826,8 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
       const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BCW + BCW - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BCW);
       const bool diag = (causal && cs_rel == rb) || (window > 0 && max_diff >= window);
-      const float* stat = stat_smem + st * C::STAT_FLOATS + 16 * qd;
+      const float* lse_t = lse_smem + (i % C::NS1) * C::STAT + 16 * qd;
+      const float* delta_t = delta_smem + (i % C::NS2) * C::STAT + 16 * qd;
       BW_WAIT(&bars->s_full[C::NSB == 2 ? (i & 1) : 0], C::NSB == 2 ? ((i >> 1) & 1) : (i & 1), PB_ERR_TIMEOUT_EPILOGUE);
       pb::tc_fence_after();
       auto masked = [&](int e) {
@@ -816,7 +838,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
       float p[32];      // CAP: tanh(scale * s / softcap) until dP is there, so that no element needs two registers
       auto probabilities = [&](int e2, float s0, float s1) {      // p[e2], p[e2 + 1] of two scores
         uint64_t l2 = row_l2;
-        if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(stat + (e2 >> 4) * 128 + (e2 & 15));
+        if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(lse_t + (e2 >> 4) * 64 + (e2 & 15));
         pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
         p[e2] = pb::fast_exp2(p[e2]);
         p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
@@ -847,7 +869,10 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
             if (masked(e)) p[e] = 0.f;
         }
       }
-      BW_WAIT(&bars->dp_full, i & 1, PB_ERR_TIMEOUT_EPILOGUE);
+      BW_WAIT(&bars->dp_full[i & 3], (i >> 2) & 1, PB_ERR_TIMEOUT_EPILOGUE);
+      if (MODE == MODE_DKDV) {
+        BW_WAIT(&bars->y2_full[i % C::NS2], (i / C::NS2) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's delta is visible
+      }
       pb::tc_fence_after();
       uint32_t dp[32];
       pb::tmem_ld_32x32b_x16(td, dp);
@@ -877,7 +902,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
             }
           }
           uint64_t dl = row_delta;
-          if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(stat + half * 128 + 64 + e2);
+          if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(delta_t + half * 64 + e2);
           const uint64_t pp = pb::pack_f32x2(p[e], p[e + 1]);
           // dS = P (dP - delta), times the score scale, which the epilogue applies
           uint64_t ds = pb::mul_f32x2(pp, pb::fma_f32x2(dl, minus_one, pb::pack_f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1]))));
@@ -1112,14 +1137,13 @@ int launch_bwd(const BwdArgs& a) {
       (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.delta + (long)a.batch * a.hq * a.seq, a.seq,
       a.hq, a.o_row, a.do_row);
   int rc;
-  CUtensorMap q128, do128, k128, v128, q64, do64, k64, v64, dq_m, dk_m, dv_m;
+  CUtensorMap q128, do128, k128, v128, q64, do64, dq_m, dk_m, dv_m;
   const long TK = (long)a.batch * a.seq_k;
 #define MK(m, p, rows, heads, d, row, br) \
   if ((rc = pbh::make_tmap_3d(&m, p, bf, 2, rows, heads, d, d, row, br, 1, 64, sw))) return rc;
   MK(q128, a.q, T, a.hq, DQK, a.q_row, 128) MK(do128, a.d_o, T, a.hq, DV, a.do_row, 128)
   MK(k128, a.k, TK, a.hkv, DQK, a.k_row, 128) MK(v128, a.v, TK, a.hkv, DV, a.v_row, 128)
   MK(q64, a.q, T, a.hq, DQK, a.q_row, 64) MK(do64, a.d_o, T, a.hq, DV, a.do_row, 64)
-  MK(k64, a.k, TK, a.hkv, DQK, a.k_row, 64) MK(v64, a.v, TK, a.hkv, DV, a.v_row, 64)
   MK(dq_m, a.dq, T, a.hq, DQK, a.dq_row, 128) MK(dk_m, a.dk, TK, a.hkv, DQK, a.dk_row, 128)
   MK(dv_m, a.dv, TK, a.hkv, DV, a.dv_row, 128)
 #undef MK
@@ -1160,7 +1184,7 @@ int launch_bwd(const BwdArgs& a) {
     using CKV = BwWideCfg<DQK, DV, MODE_DKDV>;
     PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 2>
             : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 0>),
-           CKV, BWW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q64, do64, dk_m, dv_m)
+           CKV, BWW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q128, do128, dk_m, dv_m)
   } else {
     using CKV = BwCfg<DQK, DV>;
     PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, true> : flash_attn_bwd_kernel<DQK, DV, false>), CKV,
@@ -1169,7 +1193,7 @@ int launch_bwd(const BwdArgs& a) {
   using CQ = BwWideCfg<DQK, DV, MODE_DQ>;
   PB_BWD((var == 2   ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 2>
           : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 0>),
-         CQ, BWW_THREADS, grid_q, c_q, out_q, q128, do128, k64, v64, dq_m, dq_m)
+         CQ, BWW_THREADS, grid_q, c_q, out_q, q128, do128, k128, v128, dq_m, dq_m)
 #undef PB_BWD
   return (int)cudaGetLastError();
 }
