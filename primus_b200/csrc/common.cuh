@@ -226,6 +226,32 @@ PB_DEVICE void tma_load_3d_pair(void* smem_dst, const CUtensorMap* m, uint32_t b
       "l"(reinterpret_cast<uint64_t>(m)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
+// Persistent CTAs: asks the hardware scheduler for a block of the grid that has not been launched yet; the 16-byte answer counts
+// on `bar`.  Not to be asked again after a negative answer.
+PB_DEVICE void clc_try_cancel(uint4* answer, uint64_t* bar) {
+  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
+                   smem_u32(answer)),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+// true: a block was taken over, `block` is its index
+PB_DEVICE bool clc_taken(const uint4* answer, int3& block) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
+      "ld.shared.b128 h, [%4];\n\t"
+      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t"
+      "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, h;\n\t"
+      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::z.b32.b128 %3, h;\n\t}"
+      : "=&r"(ok), "=&r"(block.x), "=&r"(block.y), "=&r"(block.z)
+      : "r"(smem_u32(answer))
+      : "memory");
+  return ok != 0;
+}
+
 // completion of all prior MMAs / copies of the pair -> the barrier at the same offset in every CTA of `mask`
 PB_DEVICE void umma_commit_2cta(uint64_t* bar, uint16_t mask) {
   asm volatile(

@@ -475,9 +475,17 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 // A step of 128 x 128 x 128 holds four GEMMs of 512 clocks each in the dK / dV pass, three in the dQ pass; the passes take 2750
 // and 1960 clocks per step (3600 and 2600 with one ring of two or three buffers for both tiles: S waited for its tile).  8192 x
 // 32/8 x 128: dK / dV pass 924 -> 777 us; 4096 x 16 x 192/128: dQ pass 119 -> 101 us.
+//
+// The CTAs are persistent where the heads have d_qk == d_v: one takes the next block from the hardware scheduler
+// (clusterlaunchcontrol.try_cancel, so that the longest blocks still start first) and loads its tiles, and issues its first
+// GEMMs, while the sums of this block leave.  A CTA of a cluster that shares a block, and the multi-latent shape, whose resident
+// tile fills the shared memory, have one block.  dQ pass, one block per CTA -> persistent, us: window of 128 at 2 x 2048 x
+// 64/8 x 64 98 -> 59 (start and end were 8500 of 11600 clocks), 2048 x 32/8 x 128 54 -> 49, 8192 x 32/8 x 128 603 -> 585.
+//   warp 0 scheduler and TMA producer; warp 1 issues the MMAs; warp 2 stores the outputs; warps 4..19 softmax and gradients
 template <int DQK, int DV, int MODE>
 struct BwWideCfg {
   static constexpr int BCW = 128;
+  static constexpr bool PERSIST = DQK == DV;
   static constexpr int ACC_COLS = (MODE == MODE_DKDV) ? DQK + DV : DQK;
   static constexpr int NSB = DQK == 64 ? 2 : 1;                        // S buffers
   static constexpr bool XA1 = MODE == MODE_DQ && DQK == 128;           // X1 (Q) in tensor memory
@@ -489,31 +497,41 @@ struct BwWideCfg {
   static constexpr int T1_BYTES = BR * DQK * 2;                        // a [128, DQK] tile (X1, Y1)
   static constexpr int T2_BYTES = BR * DV * 2;                         // a [128, DV] tile (X2, Y2)
   static constexpr int STAT = MODE == MODE_DKDV ? 128 : 0;             // statistics of a tile: lse with Y1, delta with Y2
-  static constexpr int X_BYTES = (XA1 ? 0 : T1_BYTES) + (XA2 ? 0 : T2_BYTES);
+  static constexpr int NX = DQK == 64 ? 2 : 1;                         // buffers of the resident tiles
+  // X2 of the multi-latent dQ pass goes to tensor memory by way of the V buffer
+  static constexpr bool X2_IN_RING = !PERSIST && XA2;
+  static constexpr int X_BYTES = T1_BYTES + (X2_IN_RING ? 0 : T2_BYTES);
   static constexpr int NS1 = DQK == 64 ? 4 : 3;
-  static constexpr int NS2 = DQK == 64 ? 4 : MODE == MODE_DKDV ? 2 : DQK == 128 ? 3 : 1;
-  static constexpr int TILE_BYTES = X_BYTES + NS1 * T1_BYTES + NS2 * T2_BYTES;
+  static constexpr int NS2 = DQK == 64 ? 4 : DQK == 128 ? 2 : 1;
+  static constexpr int TILE_BYTES = NX * X_BYTES + NS1 * T1_BYTES + NS2 * T2_BYTES;
   static constexpr int SMEM_BYTES = TILE_BYTES + (NS1 + NS2) * STAT * 4 + 512;
   static_assert(SMEM_BYTES <= 232448, "shared memory");
   static_assert(ACC_COLS * 4 * BR <= TILE_BYTES, "sums of a shared block");
   static_assert(XA2_COL + (XA2 ? DV / 2 : 0) <= 512, "tensor memory");
 };
 constexpr int BWW_WARPS = 16;                       // softmax warps: thread = one resident row x 16 columns of each half
-constexpr int BWW_THREADS = 64 + 32 * BWW_WARPS;
+constexpr int BWW_THREADS = 128 + 32 * BWW_WARPS;
+// registers move from warps 0..3 to the softmax warps: 64 + 4 * 104 = 5 * 96 per lane of a scheduler
+constexpr int BWW_REGS_AUX = 64, BWW_REGS_SOFTMAX = 104;
 
 struct BwWideBars {
-  uint64_t x_full;
+  uint4 next[2];           // answers of try_cancel, by block parity
+  uint64_t next_full[2], next_empty[2];
+  uint64_t x_full[2], x_empty[2];
   uint64_t y1_full[4], y2_full[4];
   uint64_t s_full[2];
   uint64_t dp_full[4], done[4];   // by step: dP is there; all products of the step are.  They release the streamed tiles too
   uint64_t freed;          // the softmax threads hold S (one S buffer) or dP (two) of the step in registers
   uint64_t pa[2], pb[2];   // P / dS of half A / B are in tensor memory; by step parity, because with two S buffers a warp can
                            // be a step ahead of another
-  uint64_t acc_done;
+  uint64_t acc_done;       // all products of the block are there
+  uint64_t acc_free;       // and have been read
+  uint64_t out_ready;      // the outputs are in shared memory
   uint64_t xa_ready;       // resident tiles copied into tensor memory
   uint32_t tmem_base;
   int abort_flag;
 };
+static_assert(sizeof(BwWideBars) <= 512, "barriers");
 
 // one look at a barrier, without waiting
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
@@ -527,6 +545,14 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+
+// in a role's lambda: a wait that runs out ends the role
+#define BWW_WAIT(bar, parity, code)            \
+  if (!bw_wait((bar), (parity), abort_flag)) { \
+    atomicCAS(status, 0, (code));              \
+    bars->abort_flag = 1;                      \
+    return false;                              \
+  }
 
 // VAR: 0 plain, 1 sliding window, 2 soft-capped scores (with or without a window); a variant carries no code of a later one
 template <int DQK, int DV, int MODE, int VAR>
@@ -545,11 +571,10 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   const float cap_b = CAP ? softcap_arg / scale : 0.f;
   extern __shared__ __align__(1024) uint8_t smem_wide[];
   uint8_t* smem = smem_wide;
-  uint8_t* y1_smem = smem + C::X_BYTES;
+  uint8_t* y1_smem = smem + C::NX * C::X_BYTES;
   uint8_t* y2_smem = y1_smem + C::NS1 * C::T1_BYTES;
-  // a resident tile that goes to tensor memory passes through the last buffer of a ring before its first streamed tile
-  uint8_t* x1_smem = C::XA1 ? y1_smem + (C::NS1 - 1) * C::T1_BYTES : smem;
-  uint8_t* x2_smem = C::XA2 ? y2_smem + (C::NS2 - 1) * C::T2_BYTES : smem + (C::XA1 ? 0 : C::T1_BYTES);
+  auto x1_smem = [&](uint32_t slot) { return smem + slot * C::X_BYTES; };
+  auto x2_smem = [&](uint32_t slot) { return C::X2_IN_RING ? y2_smem + (C::NS2 - 1) * C::T2_BYTES : smem + slot * C::X_BYTES + C::T1_BYTES; };
   float* lse_smem = reinterpret_cast<float*>(y2_smem + C::NS2 * C::T2_BYTES);
   float* delta_smem = lse_smem + C::NS1 * C::STAT;
   BwWideBars* bars = reinterpret_cast<BwWideBars*>(delta_smem + C::NS2 * C::STAT);
@@ -562,42 +587,65 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   const int num_rb = seq_x / BR;
   const int num_c = seq_y / BCW;
   const int qo = q_off / BCW;
-  // longest row blocks first, as in the kernel above
-  const int rb = (MODE == MODE_DKDV) ? blockIdx.y : (num_rb - 1 - blockIdx.y);
-  const int nxh = (MODE == MODE_DKDV) ? hkv : hq;
-  const int csize = pb::cluster_nctarank(), rank = pb::cluster_ctarank();   // CTAs that share the block's steps
-  const int xhead = (blockIdx.x / csize) % nxh;
-  const int batch = blockIdx.x / csize / nxh;
-  const int tok0 = batch * seq_x;
-  const int toky0 = batch * seq_y;
-  const int c_start = (MODE == MODE_DKDV) ? (causal ? max(0, rb - qo) : 0)
-                                          : (window > 0 ? max(0, rb * BR + q_off - window + 1) / BCW : 0);
-  const int c_end = (MODE == MODE_DKDV)
-                        ? (window > 0 ? min(num_c, (rb * BR + BR - 1 + window - 1 - q_off) / BCW + 1) : num_c)
-                        : (causal ? min(num_c, rb + 1 + qo) : num_c);
-  const int n_per_head = max(0, c_end - c_start);
-  const int n_all = (MODE == MODE_DKDV) ? g * n_per_head : n_per_head;
-  const int i0 = n_all * rank / csize;                    // first step of this CTA
-  const int n_iter = n_all * (rank + 1) / csize - i0;
+  const bool shared_block = pb::cluster_nctarank() > 1;    // the CTAs of the cluster share the steps of one block
+  const bool one_block = !C::PERSIST || shared_block;
+  struct Block {
+    int rb, xhead, batch;
+    int c_start, n_per_head;    // streamed tiles of a query head
+    int i0, n;                  // first step of this CTA and its number of steps
+  };
+  // grid (heads * cluster, batch, row blocks): longest row blocks first, as in the kernel above, and no division to find one
+  auto block_of = [&](int3 b) {
+    Block w;
+    const int csize = pb::cluster_nctarank(), rank = pb::cluster_ctarank();
+    w.rb = (MODE == MODE_DKDV) ? b.z : (num_rb - 1 - b.z);
+    w.xhead = b.x >> (__ffs(csize) - 1);                          // (csize is a power of two)
+    w.batch = b.y;
+    w.c_start = (MODE == MODE_DKDV) ? (causal ? max(0, w.rb - qo) : 0)
+                                    : (window > 0 ? max(0, w.rb * BR + q_off - window + 1) / BCW : 0);
+    const int c_end = (MODE == MODE_DKDV)
+                          ? (window > 0 ? min(num_c, (w.rb * BR + BR - 1 + window - 1 - q_off) / BCW + 1) : num_c)
+                          : (causal ? min(num_c, w.rb + 1 + qo) : num_c);
+    w.n_per_head = max(0, c_end - w.c_start);
+    const int n_all = (MODE == MODE_DKDV) ? g * w.n_per_head : w.n_per_head;
+    w.i0 = (n_all * rank) >> (__ffs(csize) - 1);
+    w.n = ((n_all * (rank + 1)) >> (__ffs(csize) - 1)) - w.i0;
+    return w;
+  };
   volatile int* abort_flag = &bars->abort_flag;
   const float sl2 = scale * 1.4426950408889634f;
+  // the block after block `item` of this CTA: waits for the scheduler's answer; false: there is none
+  auto next_block = [&](uint32_t item, int3& b) -> bool {
+    if (one_block) return false;
+    const uint32_t nx = item & 1;
+    BWW_WAIT(&bars->next_full[nx], (item >> 1) & 1, PB_ERR_TIMEOUT_MMA);
+    return pb::clc_taken(&bars->next[nx], b);
+  };
+  auto next_seen = [&](uint32_t item) {
+    pb::fence_proxy_async_smem();
+    pb::mbar_arrive(&bars->next_empty[item & 1]);
+  };
 
   if (threadIdx.x == 0) {
-    pb::mbar_init(&bars->x_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      pb::mbar_init(&bars->next_full[i], 1);
+      pb::mbar_init(&bars->next_empty[i], 2 + BWW_WARPS);   // issuer, store and softmax warps
+      pb::mbar_init(&bars->x_full[i], 1);
+      pb::mbar_init(&bars->x_empty[i], 1);
+      pb::mbar_init(&bars->s_full[i], 1);
+      pb::mbar_init(&bars->pa[i], BWW_WARPS);
+      pb::mbar_init(&bars->pb[i], BWW_WARPS);
+    }
     for (int i = 0; i < 4; ++i) {
       pb::mbar_init(&bars->y1_full[i], 1);
       pb::mbar_init(&bars->y2_full[i], 1);
       pb::mbar_init(&bars->dp_full[i], 1);
       pb::mbar_init(&bars->done[i], 1);
     }
-    pb::mbar_init(&bars->s_full[0], 1);
-    pb::mbar_init(&bars->s_full[1], 1);
     pb::mbar_init(&bars->freed, BWW_WARPS);
-    for (int i = 0; i < 2; ++i) {
-      pb::mbar_init(&bars->pa[i], BWW_WARPS);
-      pb::mbar_init(&bars->pb[i], BWW_WARPS);
-    }
     pb::mbar_init(&bars->acc_done, 1);
+    pb::mbar_init(&bars->acc_free, BWW_WARPS);
+    pb::mbar_init(&bars->out_ready, BWW_WARPS);
     pb::mbar_init(&bars->xa_ready, BWW_WARPS);
     bars->abort_flag = 0;
     pb::fence_barrier_init();
@@ -611,196 +659,240 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
-  if (warp == 0) {
-    // ------------------------------------------------------------------ producer
-    if (pb::elect_one()) {
-      bool ok = true;
-      pb::mbar_expect_tx(&bars->x_full, C::T1_BYTES + C::T2_BYTES);
+  if (warp < 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(BWW_REGS_AUX));
+    if (warp == 0 && pb::elect_one()) {
+      // ------------------------------------------------------------------ scheduler and producer
+      [&]() -> bool {
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
+        uint32_t u0 = 0;                               // steps of the blocks before
+        for (uint32_t item = 0;; ++item) {
+          const Block w = block_of(b);
+          const int tok0 = w.batch * seq_x, toky0 = w.batch * seq_y;
+          auto load_x = [&]() -> bool {
+            const uint32_t slot = item % C::NX;
+            if (C::XA1) {                              // free once copied, and the outputs of the block before have left it
+              if (item == 1) BWW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
+              if (item >= 2) BWW_WAIT(&bars->x_empty[0], item & 1, PB_ERR_TIMEOUT_TMA);
+            } else if (item >= C::NX) {                // free when the outputs of the block that had it have left it
+              BWW_WAIT(&bars->x_empty[slot], ((item / C::NX) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
+            }
+            pb::mbar_expect_tx(&bars->x_full[slot], C::T1_BYTES + C::T2_BYTES);
 #pragma unroll
-      for (int a = 0; a < DQK / 64; ++a)
-        pb::tma_load_3d(x1_smem + a * XATOM, &tmX1, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
+            for (int a = 0; a < DQK / 64; ++a)
+              pb::tma_load_3d(x1_smem(slot) + a * XATOM, &tmX1, &bars->x_full[slot], a * 64, w.xhead, tok0 + w.rb * BR);
 #pragma unroll
-      for (int a = 0; a < DV / 64; ++a)
-        pb::tma_load_3d(x2_smem + a * XATOM, &tmX2, &bars->x_full, a * 64, xhead, tok0 + rb * BR);
-      auto load_y1 = [&](int i) {
-        const int st = i % C::NS1, rel = i - C::NS1;     // rel: the step that had the buffer
-        do {
-          if (C::XA1 && i == C::NS1 - 1) BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
-          if (rel >= 0) BW_WAIT(&bars->done[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
-          pb::mbar_expect_tx(&bars->y1_full[st], C::T1_BYTES + C::STAT * 4);
-          const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
-          const int row = (c_start + (i0 + i) % n_per_head) * BCW;
+            for (int a = 0; a < DV / 64; ++a)
+              pb::tma_load_3d(x2_smem(slot) + a * XATOM, &tmX2, &bars->x_full[slot], a * 64, w.xhead, tok0 + w.rb * BR);
+            return true;
+          };
+          auto load_y1 = [&](int i) -> bool {
+            const uint32_t u = u0 + i, st = u % C::NS1, rel = u - C::NS1;     // rel: the step that had the buffer
+            if (u >= C::NS1) BWW_WAIT(&bars->done[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
+            pb::mbar_expect_tx(&bars->y1_full[st], C::T1_BYTES + C::STAT * 4);
+            const int yhead = (MODE == MODE_DKDV) ? (w.xhead * g + (w.i0 + i) / w.n_per_head) : (w.xhead / g);
+            const int row = (w.c_start + (w.i0 + i) % w.n_per_head) * BCW;
 #pragma unroll
-          for (int a = 0; a < DQK / 64; ++a)
-            pb::tma_load_3d(y1_smem + st * C::T1_BYTES + a * XATOM, &tmY1, &bars->y1_full[st], a * 64, yhead, toky0 + row);
-          if (MODE == MODE_DKDV)
-            bulk_load_1d(lse_smem + st * C::STAT, lse + ((long)batch * hq + yhead) * seq + row, 512, &bars->y1_full[st]);
-        } while (false);
-      };
-      auto load_y2 = [&](int i) {
-        const int st = i % C::NS2, rel = i - C::NS2;
-        do {
-          if (C::XA2 && i == C::NS2 - 1) BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
-          // the dQ pass is done with V after dP
-          if (rel >= 0) BW_WAIT(MODE == MODE_DKDV ? &bars->done[rel & 3] : &bars->dp_full[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
-          pb::mbar_expect_tx(&bars->y2_full[st], C::T2_BYTES + C::STAT * 4);
-          const int yhead = (MODE == MODE_DKDV) ? (xhead * g + (i0 + i) / n_per_head) : (xhead / g);
-          const int row = (c_start + (i0 + i) % n_per_head) * BCW;
+            for (int a = 0; a < DQK / 64; ++a)
+              pb::tma_load_3d(y1_smem + st * C::T1_BYTES + a * XATOM, &tmY1, &bars->y1_full[st], a * 64, yhead, toky0 + row);
+            if (MODE == MODE_DKDV)
+              bulk_load_1d(lse_smem + st * C::STAT, lse + ((long)w.batch * hq + yhead) * seq + row, 512, &bars->y1_full[st]);
+            return true;
+          };
+          auto load_y2 = [&](int i) -> bool {
+            const uint32_t u = u0 + i, st = u % C::NS2, rel = u - C::NS2;
+            if (C::X2_IN_RING && u == C::NS2 - 1) BWW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_TMA);
+            // the dQ pass is done with V after dP
+            if (u >= C::NS2)
+              BWW_WAIT(MODE == MODE_DKDV ? &bars->done[rel & 3] : &bars->dp_full[rel & 3], (rel >> 2) & 1, PB_ERR_TIMEOUT_TMA);
+            pb::mbar_expect_tx(&bars->y2_full[st], C::T2_BYTES + C::STAT * 4);
+            const int yhead = (MODE == MODE_DKDV) ? (w.xhead * g + (w.i0 + i) / w.n_per_head) : (w.xhead / g);
+            const int row = (w.c_start + (w.i0 + i) % w.n_per_head) * BCW;
 #pragma unroll
-          for (int a = 0; a < DV / 64; ++a)
-            pb::tma_load_3d(y2_smem + st * C::T2_BYTES + a * XATOM, &tmY2, &bars->y2_full[st], a * 64, yhead, toky0 + row);
-          if (MODE == MODE_DKDV)
-            bulk_load_1d(delta_smem + st * C::STAT, delta + ((long)batch * hq + yhead) * seq + row, 512, &bars->y2_full[st]);
-        } while (false);
-      };
-      if (n_iter > 0) load_y1(0);
-      for (int i = 0; i < n_iter && ok; ++i) {      // in the order in which they are wanted and their buffers are free
-        if (C::NS2 == 1 && i + 1 < n_iter) load_y1(i + 1);
-        if (ok) load_y2(i);
-        if (C::NS2 != 1 && ok && i + 1 < n_iter) load_y1(i + 1);
-      }
+            for (int a = 0; a < DV / 64; ++a)
+              pb::tma_load_3d(y2_smem + st * C::T2_BYTES + a * XATOM, &tmY2, &bars->y2_full[st], a * 64, yhead, toky0 + row);
+            if (MODE == MODE_DKDV)
+              bulk_load_1d(delta_smem + st * C::STAT, delta + ((long)w.batch * hq + yhead) * seq + row, 512,
+                           &bars->y2_full[st]);
+            return true;
+          };
+          // a resident tile whose buffer waits for the outputs of the block before does not hold up the streamed ones
+          constexpr bool X_LAST = C::PERSIST && C::NX == 1 && !C::XA1;
+          if (!X_LAST && !load_x()) return false;
+          if (w.n > 0 && !load_y1(0)) return false;
+          if (X_LAST && w.n > 0 && !load_y2(0)) return false;
+          if (X_LAST && !load_x()) return false;
+          for (int i = 0; i < w.n; ++i) {      // in the order in which they are wanted and their buffers are free
+            if (C::NS2 == 1 && i + 1 < w.n && !load_y1(i + 1)) return false;
+            if (!(X_LAST && i == 0) && !load_y2(i)) return false;
+            if (C::NS2 != 1 && i + 1 < w.n && !load_y1(i + 1)) return false;
+          }
+          if (one_block) return true;
+          u0 += w.n;
+          // ask for the next block as late as its loads allow: one taken over early is not there for a CTA that runs out first
+          const uint32_t nx = item & 1;
+          BWW_WAIT(&bars->next_empty[nx], ((item >> 1) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
+          pb::mbar_expect_tx(&bars->next_full[nx], 16);
+          pb::clc_try_cancel(&bars->next[nx], &bars->next_full[nx]);
+          if (!next_block(item, b)) return true;
+        }
+      }();
+    } else if (warp == 1 && pb::elect_one()) {
+      // ------------------------------------------------------------------ MMA issuer
+      [&]() -> bool {
+        constexpr uint32_t idesc_s = pb::make_idesc_bf16(BR, BCW, 0, 0);
+        constexpr uint32_t idesc_a1 = pb::make_idesc_bf16(BR, DQK, 0, 1);  // acc(DQK) += dS . Y1
+        constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
+        uint32_t u = 0;                                // step, counted over all blocks
+        for (uint32_t item = 0;; ++item) {
+          const int n = block_of(b).n;
+          const uint32_t slot = item % C::NX;
+          const uint32_t x1a = pb::smem_u32(x1_smem(slot)), x2a = pb::smem_u32(x2_smem(slot));
+          // X . Y^T -> 128 columns, X from shared or from tensor memory
+          auto issue_first = [&](auto dim, auto from_tmem, uint32_t tcol, uint32_t xa, uint32_t xt, uint32_t ya) {
+#pragma unroll
+            for (int k = 0; k < decltype(dim)::value / 16; ++k) {
+              const uint32_t off = (k / 4) * XATOM + (k % 4) * 32;
+              const uint64_t db = pb::make_smem_desc(ya + off, 0, 1024, 2);
+              if (decltype(from_tmem)::value)
+                pb::umma_f16_ts(tmem_base + tcol, tmem_base + xt + 8 * k, db, idesc_s, k > 0 ? 1u : 0u);
+              else
+                pb::umma_f16_ss(tmem_base + tcol, pb::make_smem_desc(xa + off, 0, 1024, 2), db, idesc_s, k > 0 ? 1u : 0u);
+            }
+          };
+          auto issue_s = [&](uint32_t v) {
+            pb::tc_fence_after();
+            issue_first(std::integral_constant<int, DQK>{}, std::bool_constant<C::XA1>{},
+                        C::S_COL + (C::NSB == 2 ? (v & 1) * BCW : 0), x1a, C::XA1_COL,
+                        pb::smem_u32(y1_smem + (v % C::NS1) * C::T1_BYTES));
+            pb::umma_commit(&bars->s_full[C::NSB == 2 ? (v & 1) : 0]);
+          };
+          auto issue_dp = [&](uint32_t v) -> bool {
+            BWW_WAIT(&bars->y2_full[v % C::NS2], (v / C::NS2) & 1, PB_ERR_TIMEOUT_MMA);
+            pb::tc_fence_after();
+            issue_first(std::integral_constant<int, DV>{}, std::bool_constant<C::XA2>{}, C::DP_COL, x2a, C::XA2_COL,
+                        pb::smem_u32(y2_smem + (v % C::NS2) * C::T2_BYTES));
+            pb::umma_commit(&bars->dp_full[v & 3]);
+            return true;
+          };
+          auto issue_second = [&](int i, int half) {                       // accumulators += (P, dS of the half) . Y
+            pb::tc_fence_after();
+            const uint32_t y1a = pb::smem_u32(y1_smem + (u % C::NS1) * C::T1_BYTES);
+            const uint32_t y2a = pb::smem_u32(y2_smem + (u % C::NS2) * C::T2_BYTES);
+            const uint32_t tp = tmem_base + (C::NSB == 2 ? C::S_COL + (u & 1) * BCW : C::DP_COL);
+            if (MODE == MODE_DKDV) {
+#pragma unroll
+              for (int kk = 0; kk < 4; ++kk) {
+                const int k = half * 4 + kk;
+                pb::umma_f16_ts(tmem_base + DQK, tp + 16 * k, pb::make_smem_desc(y2a + k * 2048, XATOM, 1024, 2), idesc_a2,
+                                (i > 0 || k > 0) ? 1u : 0u);
+              }
+            }
+#pragma unroll
+            for (int kk = 0; kk < 4; ++kk) {
+              const int k = half * 4 + kk;
+              pb::umma_f16_ts(tmem_base, tp + 16 * k + 8, pb::make_smem_desc(y1a + k * 2048, XATOM, 1024, 2), idesc_a1,
+                              (i > 0 || k > 0) ? 1u : 0u);
+            }
+          };
+          auto y1_there = [&](uint32_t v) { return mbar_test(&bars->y1_full[v % C::NS1], (v / C::NS1) & 1); };
+          // the first GEMMs of the block: the products of the block before have been issued, its last S and dP been read
+          if (C::XA1 || C::XA2) BWW_WAIT(&bars->xa_ready, item & 1, PB_ERR_TIMEOUT_MMA);
+          if (!C::XA1) BWW_WAIT(&bars->x_full[slot], (item / C::NX) & 1, PB_ERR_TIMEOUT_MMA);
+          if (n > 0) {
+            BWW_WAIT(&bars->y1_full[u % C::NS1], (u / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
+            issue_s(u);
+            if (!issue_dp(u)) return false;
+            if (C::NSB == 2 && n > 1) {
+              BWW_WAIT(&bars->y1_full[(u + 1) % C::NS1], ((u + 1) / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
+              issue_s(u + 1);
+            }
+          }
+          for (int i = 0; i < n; ++i, ++u) {
+            // S of the next step (one S buffer) goes out at the first point at which its tile has arrived: the issuing thread
+            // must not wait for a load while P / dS of this step are ready
+            bool s_next = C::NSB == 2 || i + 1 >= n;
+            auto try_s = [&]() {
+              if (!s_next && y1_there(u + 1)) {
+                issue_s(u + 1);
+                s_next = true;
+              }
+            };
+            BWW_WAIT(&bars->freed, u & 1, PB_ERR_TIMEOUT_MMA);
+            if (i + 1 < n) {
+              if (C::NSB == 2 && !issue_dp(u + 1)) return false;
+              try_s();
+            }
+            if (i == 0 && item > 0) BWW_WAIT(&bars->acc_free, (item - 1) & 1, PB_ERR_TIMEOUT_MMA);
+            BWW_WAIT(&bars->pa[u & 1], (u >> 1) & 1, PB_ERR_TIMEOUT_MMA);
+            issue_second(i, 0);
+            try_s();
+            BWW_WAIT(&bars->pb[u & 1], (u >> 1) & 1, PB_ERR_TIMEOUT_MMA);
+            issue_second(i, 1);
+            pb::umma_commit(&bars->done[u & 3]);
+            if (C::NSB == 1) {
+              if (!s_next) {
+                BWW_WAIT(&bars->y1_full[(u + 1) % C::NS1], ((u + 1) / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
+                issue_s(u + 1);
+              }
+              if (i + 1 < n && !issue_dp(u + 1)) return false;
+            } else if (i + 2 < n) {
+              BWW_WAIT(&bars->y1_full[(u + 2) % C::NS1], ((u + 2) / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
+              issue_s(u + 2);
+            }
+          }
+          pb::umma_commit(&bars->acc_done);
+          if (!next_block(item, b)) return true;
+          next_seen(item);
+        }
+      }();
+    } else if (warp == 2 && !shared_block && pb::elect_one()) {
+      // ------------------------------------------------------------------ outputs: shared -> global
+      [&]() -> bool {
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
+        for (uint32_t item = 0;; ++item) {
+          const Block w = block_of(b);
+          const uint32_t slot = item % C::NX;
+          const int row = w.batch * seq_x + w.rb * BR;
+          BWW_WAIT(&bars->out_ready, item & 1, PB_ERR_TIMEOUT_EPILOGUE);
+#pragma unroll
+          for (int a = 0; a < DQK / 64; ++a) pb::tma_store_3d(&tmO1, x1_smem(slot) + a * XATOM, a * 64, w.xhead, row);
+          if (MODE == MODE_DKDV) {
+#pragma unroll
+            for (int a = 0; a < DV / 64; ++a) pb::tma_store_3d(&tmO2, x2_smem(slot) + a * XATOM, a * 64, w.xhead, row);
+          }
+          pb::tma_store_commit();
+          pb::tma_store_wait_read<0>();
+          pb::mbar_arrive(&bars->x_empty[slot]);
+          if (!next_block(item, b)) break;
+          next_seen(item);
+        }
+        pb::tma_store_wait_all<0>();
+        return true;
+      }();
     }
-  } else if (warp == 1) {
-    // ------------------------------------------------------------------ MMA issuer
-    if (pb::elect_one()) {
-      constexpr uint32_t idesc_s = pb::make_idesc_bf16(BR, BCW, 0, 0);
-      constexpr uint32_t idesc_a1 = pb::make_idesc_bf16(BR, DQK, 0, 1);  // acc(DQK) += dS . Y1
-      constexpr uint32_t idesc_a2 = pb::make_idesc_bf16(BR, DV, 0, 1);   // acc(DV)  += P  . Y2
-      const uint32_t x1a = pb::smem_u32(x1_smem), x2a = pb::smem_u32(x2_smem);
-      bool ok = true;
-      // X . Y^T -> 128 columns, X from shared or from tensor memory
-      auto issue_first = [&](auto dim, auto from_tmem, uint32_t tcol, uint32_t xa, uint32_t xt, uint32_t ya) {
-#pragma unroll
-        for (int k = 0; k < decltype(dim)::value / 16; ++k) {
-          const uint32_t off = (k / 4) * XATOM + (k % 4) * 32;
-          const uint64_t db = pb::make_smem_desc(ya + off, 0, 1024, 2);
-          if (decltype(from_tmem)::value)
-            pb::umma_f16_ts(tmem_base + tcol, tmem_base + xt + 8 * k, db, idesc_s, k > 0 ? 1u : 0u);
-          else
-            pb::umma_f16_ss(tmem_base + tcol, pb::make_smem_desc(xa + off, 0, 1024, 2), db, idesc_s, k > 0 ? 1u : 0u);
-        }
-      };
-      auto issue_s = [&](int i) {
-        issue_first(std::integral_constant<int, DQK>{}, std::bool_constant<C::XA1>{},
-                    C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0), x1a, C::XA1_COL,
-                    pb::smem_u32(y1_smem + (i % C::NS1) * C::T1_BYTES));
-        pb::umma_commit(&bars->s_full[C::NSB == 2 ? (i & 1) : 0]);
-      };
-      auto issue_dp = [&](int i) {
-        issue_first(std::integral_constant<int, DV>{}, std::bool_constant<C::XA2>{}, C::DP_COL, x2a, C::XA2_COL,
-                    pb::smem_u32(y2_smem + (i % C::NS2) * C::T2_BYTES));
-        pb::umma_commit(&bars->dp_full[i & 3]);
-      };
-      auto issue_second = [&](int i, int half) {                            // accumulators += (P, dS of the half) . Y
-        const int st1 = i % C::NS1, st2 = i % C::NS2;
-        const uint32_t y1a = pb::smem_u32(y1_smem + st1 * C::T1_BYTES), y2a = pb::smem_u32(y2_smem + st2 * C::T2_BYTES);
-        const uint32_t tp = tmem_base + (C::NSB == 2 ? C::S_COL + (i & 1) * BCW : C::DP_COL);
-        if (MODE == MODE_DKDV) {
-#pragma unroll
-          for (int kk = 0; kk < 4; ++kk) {
-            const int k = half * 4 + kk;
-            pb::umma_f16_ts(tmem_base + DQK, tp + 16 * k, pb::make_smem_desc(y2a + k * 2048, XATOM, 1024, 2), idesc_a2,
-                            (i > 0 || k > 0) ? 1u : 0u);
-          }
-        }
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk) {
-          const int k = half * 4 + kk;
-          pb::umma_f16_ts(tmem_base, tp + 16 * k + 8, pb::make_smem_desc(y1a + k * 2048, XATOM, 1024, 2), idesc_a1,
-                          (i > 0 || k > 0) ? 1u : 0u);
-        }
-        if (half == 1) pb::umma_commit(&bars->done[i & 3]);
-      };
-      do {
-        if (n_iter == 0) break;
-        BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_MMA);
-        if (C::XA1 || C::XA2) {
-          BW_WAIT(&bars->xa_ready, 0, PB_ERR_TIMEOUT_MMA);
-        }
-        BW_WAIT(&bars->y1_full[0], 0, PB_ERR_TIMEOUT_MMA);
-        pb::tc_fence_after();
-        issue_s(0);
-        BW_WAIT(&bars->y2_full[0], 0, PB_ERR_TIMEOUT_MMA);
-        pb::tc_fence_after();
-        issue_dp(0);
-        if (C::NSB == 2 && n_iter > 1) {
-          BW_WAIT(&bars->y1_full[1], 0, PB_ERR_TIMEOUT_MMA);
-          pb::tc_fence_after();
-          issue_s(1);
-        }
-      } while (false);
-      for (int i = 0; i < n_iter && ok; ++i) {
-        // S of the next step (one S buffer) goes out at the first point at which its tile has arrived: the issuing thread
-        // must not wait for a load while P / dS of this step are ready
-        bool s_next = C::NSB == 2 || i + 1 >= n_iter;
-        uint64_t* y_next = &bars->y1_full[(i + 1) % C::NS1];
-        const uint32_t y_par = ((i + 1) / C::NS1) & 1;
-        uint64_t* y2_next = &bars->y2_full[(i + 1) % C::NS2];
-        const uint32_t y2_par = ((i + 1) / C::NS2) & 1;
-        auto try_s = [&]() {
-          if (!s_next && mbar_test(y_next, y_par)) {
-            pb::tc_fence_after();
-            issue_s(i + 1);
-            s_next = true;
-          }
-        };
-        if (i + 1 < n_iter) {
-          BW_WAIT(&bars->freed, i & 1, PB_ERR_TIMEOUT_MMA);
-          if (C::NSB == 2) BW_WAIT(y2_next, y2_par, PB_ERR_TIMEOUT_MMA);
-          pb::tc_fence_after();
-          if (C::NSB == 2) issue_dp(i + 1);
-          else try_s();
-        }
-        BW_WAIT(&bars->pa[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_MMA);
-        pb::tc_fence_after();
-        issue_second(i, 0);
-        try_s();
-        BW_WAIT(&bars->pb[i & 1], (i >> 1) & 1, PB_ERR_TIMEOUT_MMA);
-        pb::tc_fence_after();
-        issue_second(i, 1);
-        if (C::NSB == 1) {
-          if (!s_next) {
-            BW_WAIT(y_next, y_par, PB_ERR_TIMEOUT_MMA);
-            pb::tc_fence_after();
-            issue_s(i + 1);
-          }
-          if (i + 1 < n_iter) {
-            BW_WAIT(y2_next, y2_par, PB_ERR_TIMEOUT_MMA);
-            pb::tc_fence_after();
-            issue_dp(i + 1);
-          }
-        } else if (i + 2 < n_iter) {
-          BW_WAIT(&bars->y1_full[(i + 2) % C::NS1], ((i + 2) / C::NS1) & 1, PB_ERR_TIMEOUT_MMA);
-          pb::tc_fence_after();
-          issue_s(i + 2);
-        }
-      }
-      if (ok) pb::umma_commit(&bars->acc_done);
+    __syncwarp();
+    if (shared_block) {      // (in both branches: what follows them may use no more registers than these warps have)
+      pb::cluster_sync();
+      pb::cluster_sync();
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(BWW_REGS_SOFTMAX));
     // ------------------------------------------------------------------ softmax-gradient threads
-    const int wq = warp & 3;                      // TMEM lane quarter of this warp
-    const int qd = (warp - 2) >> 2;               // 16-column group of each half
-    const int row = wq * 32 + lane;
-    const uint32_t lane_addr = uint32_t(wq * 32) << 16;
-    const int row_g = rb * BR + row;
-    float lse2_row = 0.f, delta_row = 0.f;
-    if (MODE == MODE_DQ) {
-      const long off = ((long)batch * hq + xhead) * seq + row_g;
-      lse2_row = lse[off];  // negated, in log2 units
-      delta_row = delta[off];
-    }
-    const uint64_t sl2_2 = pb::pack_f32x2(sl2, sl2), minus_one = pb::pack_f32x2(-1.f, -1.f);
-    const uint64_t row_l2 = pb::pack_f32x2(lse2_row, lse2_row), row_delta = pb::pack_f32x2(delta_row, delta_row);
-    bool ok = true;
-    if (C::XA1 || C::XA2) {
+    [&]() -> bool {
+      const int wq = warp & 3;                      // TMEM lane quarter of this warp
+      const int qd = (warp - 4) >> 2;               // 16-column group of each half
+      const int row = wq * 32 + lane;
+      const uint32_t lane_addr = uint32_t(wq * 32) << 16;
+      const uint64_t sl2_2 = pb::pack_f32x2(sl2, sl2), minus_one = pb::pack_f32x2(-1.f, -1.f);
       // a thread copies 64 channels of its row of Q (groups 0, 1) or dO (groups 2, 3; 0, 1 when Q stays) from the
       // 128-byte-swizzled tile: word w of a row (elements 2w, 2w + 1) goes to column w, the layout of a TMEM A operand
-      do {
-        BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);
+      auto copy_x = [&](uint32_t item) -> bool {
+        BWW_WAIT(&bars->x_full[0], item & 1, PB_ERR_TIMEOUT_EPILOGUE);
         const bool q_part = C::XA1 && qd < 2;
         if (C::XA1 || qd < 2) {
-          const uint8_t* xs = (q_part ? x1_smem : x2_smem) + (qd & 1) * XATOM + row * 128;
+          const uint8_t* xs = (q_part ? x1_smem(0) : x2_smem(0)) + (qd & 1) * XATOM + row * 128;
           uint32_t wds[32];
 #pragma unroll
           for (int c = 0; c < 8; ++c) {
@@ -813,163 +905,195 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
         pb::tc_fence_before();
         __syncwarp();
         if (lane == 0) pb::mbar_arrive(&bars->xa_ready);
-      } while (false);
-    }
-    int cs = n_iter > 0 ? c_start + i0 % n_per_head : 0;    // tile of the step, advanced at the end of the loop
-    for (int i = 0; i < n_iter && ok; ++i) {
-      if (MODE == MODE_DKDV) {
-        BW_WAIT(&bars->y1_full[i % C::NS1], (i / C::NS1) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's lse is visible
-      }
-      const uint32_t ts = tmem_base + lane_addr + C::S_COL + (C::NSB == 2 ? (i & 1) * BCW : 0) + 16 * qd;
-      const uint32_t td = tmem_base + lane_addr + C::DP_COL + 16 * qd;
-      const uint32_t tout = C::NSB == 2 ? ts : td;
-      const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
-      const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BCW + BCW - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BCW);
-      const bool diag = (causal && cs_rel == rb) || (window > 0 && max_diff >= window);
-      const float* lse_t = lse_smem + (i % C::NS1) * C::STAT + 16 * qd;
-      const float* delta_t = delta_smem + (i % C::NS2) * C::STAT + 16 * qd;
-      BW_WAIT(&bars->s_full[C::NSB == 2 ? (i & 1) : 0], C::NSB == 2 ? ((i >> 1) & 1) : (i & 1), PB_ERR_TIMEOUT_EPILOGUE);
-      pb::tc_fence_after();
-      auto masked = [&](int e) {
-        const int col_g = cs_rel * BCW + (e >> 4) * 64 + 16 * qd + (e & 15);
-        const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
-        return diff < 0 || (window > 0 && diff >= window);
+        return true;
       };
-      float p[32];      // CAP: tanh(scale * s / softcap) until dP is there, so that no element needs two registers
-      auto probabilities = [&](int e2, float s0, float s1) {      // p[e2], p[e2 + 1] of two scores
-        uint64_t l2 = row_l2;
-        if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(lse_t + (e2 >> 4) * 64 + (e2 & 15));
-        pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
-        p[e2] = pb::fast_exp2(p[e2]);
-        p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
-      };
-      {
-        uint32_t sr[32];
-        pb::tmem_ld_32x32b_x16(ts, sr);
-        pb::tmem_ld_32x32b_x16(ts + 64, sr + 16);
-        pb::tmem_wait_ld();
-        if (C::NSB == 1) {
-          pb::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) pb::mbar_arrive(&bars->freed);
+      if ((C::XA1 || C::XA2) && !copy_x(0)) return false;
+      int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
+      uint32_t u = 0;
+      float lse2_row = 0.f, delta_row = 0.f;        // of this thread's query row, for the dQ pass
+      auto load_stats = [&]() {
+        if (MODE == MODE_DQ) {
+          const Block w = block_of(b);
+          const long off = ((long)w.batch * hq + w.xhead) * seq + w.rb * BR + row;
+          lse2_row = lse[off];  // negated, in log2 units
+          delta_row = delta[off];
         }
-#pragma unroll
-        for (int e2 = 0; e2 < 32; e2 += 2) {
-          const float s0 = __uint_as_float(sr[e2]), s1 = __uint_as_float(sr[e2 + 1]);
-          if (CAP) {
-            p[e2] = pb::fast_tanh(s0 * cap_a);
-            p[e2 + 1] = pb::fast_tanh(s1 * cap_a);
-          } else {
-            probabilities(e2, s0, s1);
+      };
+      load_stats();
+      for (uint32_t item = 0;; ++item) {
+        const Block w = block_of(b);
+        const int rb = w.rb, row_g = rb * BR + row, c_end = w.c_start + w.n_per_head;
+        const uint64_t row_l2 = pb::pack_f32x2(lse2_row, lse2_row), row_delta = pb::pack_f32x2(delta_row, delta_row);
+        int cs = w.c_start + (w.i0 > 0 && w.n > 0 ? w.i0 % w.n_per_head : 0);    // tile of the step, advanced at the end of the loop
+        for (int i = 0; i < w.n; ++i, ++u) {
+          if (MODE == MODE_DKDV) {
+            BWW_WAIT(&bars->y1_full[u % C::NS1], (u / C::NS1) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's lse is visible
           }
-        }
-        if (!CAP && diag) {
+          const uint32_t ts = tmem_base + lane_addr + C::S_COL + (C::NSB == 2 ? (u & 1) * BCW : 0) + 16 * qd;
+          const uint32_t td = tmem_base + lane_addr + C::DP_COL + 16 * qd;
+          const uint32_t tout = C::NSB == 2 ? ts : td;
+          const int cs_rel = (MODE == MODE_DKDV) ? cs + qo : cs - qo;   // streamed tile index in the stationary block's frame
+          const int max_diff = (MODE == MODE_DKDV) ? (cs_rel * BCW + BCW - 1 - rb * BR) : (rb * BR + BR - 1 - cs_rel * BCW);
+          const bool diag = (causal && cs_rel == rb) || (window > 0 && max_diff >= window);
+          const float* lse_t = lse_smem + (u % C::NS1) * C::STAT + 16 * qd;
+          const float* delta_t = delta_smem + (u % C::NS2) * C::STAT + 16 * qd;
+          BWW_WAIT(&bars->s_full[C::NSB == 2 ? (u & 1) : 0], C::NSB == 2 ? ((u >> 1) & 1) : (u & 1), PB_ERR_TIMEOUT_EPILOGUE);
+          pb::tc_fence_after();
+          auto masked = [&](int e) {
+            const int col_g = cs_rel * BCW + (e >> 4) * 64 + 16 * qd + (e & 15);
+            const int diff = (MODE == MODE_DKDV) ? (col_g - row_g) : (row_g - col_g);   // query - key position
+            return diff < 0 || (window > 0 && diff >= window);
+          };
+          float p[32];      // CAP: tanh(scale * s / softcap) until dP is there, so that no element needs two registers
+          auto probabilities = [&](int e2, float s0, float s1) {      // p[e2], p[e2 + 1] of two scores
+            uint64_t l2 = row_l2;
+            if (MODE == MODE_DKDV) l2 = *reinterpret_cast<const uint64_t*>(lse_t + (e2 >> 4) * 64 + (e2 & 15));
+            pb::unpack_f32x2(pb::fma_f32x2(pb::pack_f32x2(s0, s1), sl2_2, l2), p[e2], p[e2 + 1]);
+            p[e2] = pb::fast_exp2(p[e2]);
+            p[e2 + 1] = pb::fast_exp2(p[e2 + 1]);
+          };
+          {
+            uint32_t sr[32];
+            pb::tmem_ld_32x32b_x16(ts, sr);
+            pb::tmem_ld_32x32b_x16(ts + 64, sr + 16);
+            pb::tmem_wait_ld();
+            if (C::NSB == 1) {
+              pb::tc_fence_before();
+              __syncwarp();
+              if (lane == 0) pb::mbar_arrive(&bars->freed);
+            }
 #pragma unroll
-          for (int e = 0; e < 32; ++e)
-            if (masked(e)) p[e] = 0.f;
-        }
-      }
-      BW_WAIT(&bars->dp_full[i & 3], (i >> 2) & 1, PB_ERR_TIMEOUT_EPILOGUE);
-      if (MODE == MODE_DKDV) {
-        BW_WAIT(&bars->y2_full[i % C::NS2], (i / C::NS2) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's delta is visible
-      }
-      pb::tc_fence_after();
-      uint32_t dp[32];
-      pb::tmem_ld_32x32b_x16(td, dp);
-      pb::tmem_ld_32x32b_x16(td + 64, dp + 16);
-      pb::tmem_wait_ld();
-      if (C::NSB == 2) {
-        pb::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) pb::mbar_arrive(&bars->freed);
-      }
+            for (int e2 = 0; e2 < 32; e2 += 2) {
+              const float s0 = __uint_as_float(sr[e2]), s1 = __uint_as_float(sr[e2 + 1]);
+              if (CAP) {
+                p[e2] = pb::fast_tanh(s0 * cap_a);
+                p[e2 + 1] = pb::fast_tanh(s1 * cap_a);
+              } else {
+                probabilities(e2, s0, s1);
+              }
+            }
+            if (!CAP && diag) {
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t pk[16];                          // packed P (8), dS (8) of this thread's 16 columns
-#pragma unroll
-        for (int e2 = 0; e2 < 16; e2 += 2) {
-          const int e = half * 16 + e2;
-          float dc0 = 1.f, dc1 = 1.f;
-          if (CAP) {
-            // the score is softcap * tanh(scale * s / softcap) / scale; dc: its derivative with respect to scale * s
-            const float t0 = p[e], t1 = p[e + 1];
-            dc0 = fmaf(-t0, t0, 1.f);
-            dc1 = fmaf(-t1, t1, 1.f);
-            probabilities(e, t0 * cap_b, t1 * cap_b);
-            if (diag) {
-              if (masked(e)) p[e] = 0.f;
-              if (masked(e + 1)) p[e + 1] = 0.f;
+              for (int e = 0; e < 32; ++e)
+                if (masked(e)) p[e] = 0.f;
             }
           }
-          uint64_t dl = row_delta;
-          if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(delta_t + half * 64 + e2);
-          const uint64_t pp = pb::pack_f32x2(p[e], p[e + 1]);
-          // dS = P (dP - delta), times the score scale, which the epilogue applies
-          uint64_t ds = pb::mul_f32x2(pp, pb::fma_f32x2(dl, minus_one, pb::pack_f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1]))));
-          if (CAP) ds = pb::mul_f32x2(ds, pb::pack_f32x2(dc0, dc1));
-          float d0, d1;
-          pb::unpack_f32x2(ds, d0, d1);
-          pk[e2 / 2] = pb::pack_bf16x2(p[e], p[e + 1]);
-          pk[8 + e2 / 2] = pb::pack_bf16x2(d0, d1);
-        }
-        if (MODE == MODE_DKDV) pb::tmem_st_32x32b_x16(tout + half * 64, pk);
-        else pb::tmem_st_32x32b_x8(tout + half * 64 + 8, pk + 8);
-        pb::tmem_wait_st();
-        pb::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) pb::mbar_arrive(half == 0 ? &bars->pa[i & 1] : &bars->pb[i & 1]);
-      }
-      if (++cs == c_end) cs = c_start;
-    }
-    // ---- epilogue: accumulators -> bf16 -> (dead) resident tiles -> TMA store
-    do {
-      if (!ok) break;
-      BW_WAIT(&bars->acc_done, 0, PB_ERR_TIMEOUT_EPILOGUE);
-      BW_WAIT(&bars->x_full, 0, PB_ERR_TIMEOUT_EPILOGUE);     // (long past, except for a block without a step)
-      pb::tc_fence_after();
-      uint8_t* o1_smem = C::XA1 ? y1_smem : x1_smem;          // all tiles have been consumed
-      auto drain = [&](uint32_t tcol, int ncols, uint8_t* dst, float mul) {
-#pragma unroll 1
-        for (int c = qd; c < ncols / 32; c += 4) {
-          uint32_t r[32];
-          pb::tmem_ld_32x32b_x32(tmem_base + lane_addr + tcol + c * 32, r);
+          BWW_WAIT(&bars->dp_full[u & 3], (u >> 2) & 1, PB_ERR_TIMEOUT_EPILOGUE);
+          if (MODE == MODE_DKDV) {
+            BWW_WAIT(&bars->y2_full[u % C::NS2], (u / C::NS2) & 1, PB_ERR_TIMEOUT_EPILOGUE);  // the tile's delta is visible
+          }
+          pb::tc_fence_after();
+          uint32_t dp[32];
+          pb::tmem_ld_32x32b_x16(td, dp);
+          pb::tmem_ld_32x32b_x16(td + 64, dp + 16);
           pb::tmem_wait_ld();
-          if (n_iter == 0) {                      // nothing was accumulated: the columns are undefined
-#pragma unroll
-            for (int e = 0; e < 32; ++e) r[e] = 0u;
+          if (C::NSB == 2) {
+            pb::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) pb::mbar_arrive(&bars->freed);
           }
-          if (pb::cluster_nctarank() > 1) {
-            stage_row_chunk(smem, C::ACC_COLS * 4, row, tcol / 32 + c, r);
-            continue;
-          }
-          uint8_t* atom = dst + (c >> 1) * XATOM + row * 128;
 #pragma unroll
-          for (int q4 = 0; q4 < 4; ++q4) {
-            uint32_t w[4];
+          for (int half = 0; half < 2; ++half) {
+            uint32_t pk[16];                          // packed P (8), dS (8) of this thread's 16 columns
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-              w[u] = pb::pack_bf16x2(__uint_as_float(r[8 * q4 + 2 * u]) * mul, __uint_as_float(r[8 * q4 + 2 * u + 1]) * mul);
-            const int chunk = (c & 1) * 4 + q4;
-            *reinterpret_cast<uint4*>(atom + ((chunk ^ (row & 7)) << 4)) = make_uint4(w[0], w[1], w[2], w[3]);
+            for (int e2 = 0; e2 < 16; e2 += 2) {
+              const int e = half * 16 + e2;
+              float dc0 = 1.f, dc1 = 1.f;
+              if (CAP) {
+                // the score is softcap * tanh(scale * s / softcap) / scale; dc: its derivative with respect to scale * s
+                const float t0 = p[e], t1 = p[e + 1];
+                dc0 = fmaf(-t0, t0, 1.f);
+                dc1 = fmaf(-t1, t1, 1.f);
+                probabilities(e, t0 * cap_b, t1 * cap_b);
+                if (diag) {
+                  if (masked(e)) p[e] = 0.f;
+                  if (masked(e + 1)) p[e + 1] = 0.f;
+                }
+              }
+              uint64_t dl = row_delta;
+              if (MODE == MODE_DKDV) dl = *reinterpret_cast<const uint64_t*>(delta_t + half * 64 + e2);
+              const uint64_t pp = pb::pack_f32x2(p[e], p[e + 1]);
+              // dS = P (dP - delta), times the score scale, which the epilogue applies
+              uint64_t ds = pb::mul_f32x2(pp, pb::fma_f32x2(dl, minus_one, pb::pack_f32x2(__uint_as_float(dp[e]), __uint_as_float(dp[e + 1]))));
+              if (CAP) ds = pb::mul_f32x2(ds, pb::pack_f32x2(dc0, dc1));
+              float d0, d1;
+              pb::unpack_f32x2(ds, d0, d1);
+              pk[e2 / 2] = pb::pack_bf16x2(p[e], p[e + 1]);
+              pk[8 + e2 / 2] = pb::pack_bf16x2(d0, d1);
+            }
+            if (MODE == MODE_DKDV) pb::tmem_st_32x32b_x16(tout + half * 64, pk);
+            else pb::tmem_st_32x32b_x8(tout + half * 64 + 8, pk + 8);
+            pb::tmem_wait_st();
+            pb::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) pb::mbar_arrive(half == 0 ? &bars->pa[u & 1] : &bars->pb[u & 1]);
           }
+          if (++cs == c_end) cs = w.c_start;
         }
-      };
-      drain(0, DQK, o1_smem, scale);
-      if (MODE == MODE_DKDV) drain(DQK, DV, x2_smem, 1.f);
-      if (pb::cluster_nctarank() > 1) break;
-      pb::fence_proxy_async_smem();
-      pb::named_bar_sync(1, 32 * BWW_WARPS);
-      if (threadIdx.x == 64) {
-#pragma unroll
-        for (int a = 0; a < DQK / 64; ++a) pb::tma_store_3d(&tmO1, o1_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
-        if (MODE == MODE_DKDV) {
-#pragma unroll
-          for (int a = 0; a < DV / 64; ++a) pb::tma_store_3d(&tmO2, x2_smem + a * XATOM, a * 64, xhead, tok0 + rb * BR);
+        // ---- the block's end: what the next one's first GEMMs wait for, then accumulators -> bf16 -> (dead) resident tiles
+        const bool more = next_block(item, b);
+        if (!one_block) {
+          __syncwarp();
+          if (lane == 0) next_seen(item);
         }
-        pb::tma_store_commit();
-        pb::tma_store_wait_all<0>();
+        if (more) load_stats();
+        if (C::PERSIST && C::XA1 && more && !copy_x(item + 1)) return false;
+        const uint32_t slot = item % C::NX;
+        BWW_WAIT(&bars->acc_done, item & 1, PB_ERR_TIMEOUT_EPILOGUE);
+        // the staging tiles: the resident ones have arrived (long past, except for a block without a step); with copies in
+        // tensor memory, all warps have made those of the next block and the outputs of the block before have left
+        if (!C::XA1) BWW_WAIT(&bars->x_full[slot], (item / C::NX) & 1, PB_ERR_TIMEOUT_EPILOGUE);
+        if (C::XA1 && more) BWW_WAIT(&bars->xa_ready, (item + 1) & 1, PB_ERR_TIMEOUT_EPILOGUE);
+        if (C::XA1 && item > 0) BWW_WAIT(&bars->x_empty[0], (item - 1) & 1, PB_ERR_TIMEOUT_EPILOGUE);
+        pb::tc_fence_after();
+        auto drain = [&](uint32_t tcol, int ncols, uint8_t* dst, float mul) {
+#pragma unroll 1
+          for (int c = qd; c < ncols / 32; c += 4) {
+            uint32_t r[32];
+            pb::tmem_ld_32x32b_x32(tmem_base + lane_addr + tcol + c * 32, r);
+            pb::tmem_wait_ld();
+            if (w.n == 0) {                         // nothing was accumulated: the columns are undefined
+#pragma unroll
+              for (int e = 0; e < 32; ++e) r[e] = 0u;
+            }
+            if (shared_block) {
+              stage_row_chunk(smem, C::ACC_COLS * 4, row, tcol / 32 + c, r);
+              continue;
+            }
+            uint8_t* atom = dst + (c >> 1) * XATOM + row * 128;
+#pragma unroll
+            for (int q4 = 0; q4 < 4; ++q4) {
+              uint32_t wd[4];
+#pragma unroll
+              for (int v = 0; v < 4; ++v)
+                wd[v] = pb::pack_bf16x2(__uint_as_float(r[8 * q4 + 2 * v]) * mul, __uint_as_float(r[8 * q4 + 2 * v + 1]) * mul);
+              const int chunk = (c & 1) * 4 + q4;
+              *reinterpret_cast<uint4*>(atom + ((chunk ^ (row & 7)) << 4)) = make_uint4(wd[0], wd[1], wd[2], wd[3]);
+            }
+          }
+        };
+        drain(0, DQK, x1_smem(slot), scale);
+        if (MODE == MODE_DKDV) drain(DQK, DV, x2_smem(slot), 1.f);
+        pb::tc_fence_before();
+        pb::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          pb::mbar_arrive(&bars->acc_free);
+          if (!shared_block) pb::mbar_arrive(&bars->out_ready);
+        }
+        if (!more) return true;
       }
-    } while (false);
+    }();
+    if (shared_block) {
+      const Block w = block_of(make_int3(blockIdx.x, blockIdx.y, blockIdx.z));
+      __syncwarp();
+      pb::cluster_sync();
+      cluster_sum_rows<DQK, MODE == MODE_DKDV ? DV : 0>(smem, pb::cluster_ctarank(), pb::cluster_nctarank(), threadIdx.x - 128,
+                                                        32 * BWW_WARPS, (long)w.batch * seq_x + (long)w.rb * BR, w.xhead, out,
+                                                        scale);
+      __syncwarp();
+      pb::cluster_sync();       // this CTA's sums may be read until here
+    }
   }
 
   if (*abort_flag) {
@@ -980,12 +1104,6 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   if (warp == 1) {
     pb::tc_fence_after();
     pb::tmem_dealloc<1>(tmem_base, 512);
-  }
-  if (pb::cluster_nctarank() > 1) {
-    pb::cluster_sync();
-    cluster_sum_rows<DQK, MODE == MODE_DKDV ? DV : 0>(smem, pb::cluster_ctarank(), pb::cluster_nctarank(), threadIdx.x, BWW_THREADS, tok0 + (long)rb * BR, xhead,
-                                                      out, scale);
-    pb::cluster_sync();       // this CTA's sums may be read until here
   }
 }
 
@@ -1153,7 +1271,8 @@ int launch_bwd(const BwdArgs& a) {
     return bwd_cluster_size(mode, DQK, DV, a.batch, a.seq, a.seq_k, a.q_off, a.hq, a.hkv, a.causal, a.window);
   };
   const int c_kv = cluster(MODE_DKDV), c_q = cluster(MODE_DQ);
-  const dim3 grid_kv(a.hkv * a.batch * c_kv, a.seq_k / BR, 1), grid_q(a.hq * a.batch * c_q, a.seq / BR, 1);
+  const dim3 grid_kv = DQK == DV ? dim3(a.hkv * c_kv, a.batch, a.seq_k / BR) : dim3(a.hkv * a.batch * c_kv, a.seq_k / BR);
+  const dim3 grid_q(a.hq * c_q, a.batch, a.seq / BR);
   const BwOut out_kv{(__nv_bfloat16*)a.dk, (__nv_bfloat16*)a.dv, a.dk_row, a.dv_row};
   const BwOut out_q{(__nv_bfloat16*)a.dq, nullptr, a.dq_row, 0};
 #define PB_BWD(KERN, CFG, THREADS, GRID, CSIZE, OUT, X1, X2, Y1, Y2, O1, O2)                                                        \

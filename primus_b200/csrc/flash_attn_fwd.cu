@@ -70,31 +70,6 @@ struct FaItem {
   __device__ __forceinline__ bool has(int t, int j) const { return j >= lo[t] && j < nb[t]; }
 };
 
-__device__ __forceinline__ void try_cancel(uint4* answer, uint64_t* bar) {
-  asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];" ::"r"(
-                   pb::smem_u32(answer)),
-               "r"(pb::smem_u32(bar))
-               : "memory");
-}
-// true: a block was taken over, x / y are its index
-__device__ __forceinline__ bool taken(const uint4* answer, int& x, int& y) {
-  uint32_t ok, cx, cy;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b128 h;\n\t"
-      "ld.shared.b128 h, [%3];\n\t"
-      "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, h;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t"
-      "mov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\t"
-      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, h;\n\t"
-      "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::y.b32.b128 %2, h;\n\t}"
-      : "=r"(ok), "=r"(cx), "=r"(cy)
-      : "r"(pb::smem_u32(answer))
-      : "memory");
-  x = cx;
-  y = cy;
-  return ok != 0;
-}
-
 __device__ __forceinline__ bool fa_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   if (pb::mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
@@ -143,12 +118,12 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int num_pairs = (num_q128 + 1) / 2;
   const int n_kv = seq_k / BKV;
   volatile int* abort_flag = &bars->abort_flag;
-  // grid (heads * batch, pairs): x-fastest issue order starts all heads of the heaviest (longest KV range) pair first
-  auto item_of = [&](int bx, int by) {
+  // grid (heads, batch, pairs): x-fastest issue order starts all heads of the heaviest (longest KV range) pair first
+  auto item_of = [&](int3 b) {
     FaItem w;
-    w.qt0 = 2 * (num_pairs - 1 - by);
-    w.head = bx % hq;
-    w.batch = bx / hq;
+    w.qt0 = 2 * (num_pairs - 1 - b.z);
+    w.head = b.x;
+    w.batch = b.y;
     w.kv_head = w.head / (hq / hkv);
     const int qk0 = w.qt0 + q_off_blocks;      // key block of the first tile's diagonal
     // first key block that any row of a tile can see
@@ -162,10 +137,10 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   };
 
   // the pair after pair `item` of this CTA: waits for the scheduler's answer; false: there is none
-  auto next_item = [&](uint32_t item, int& bx, int& by) -> bool {
+  auto next_item = [&](uint32_t item, int3& b) -> bool {
     const uint32_t nx = item & 1;
     FA_WAIT(&bars->next_full[nx], (item >> 1) & 1, PB_ERR_TIMEOUT_MMA);
-    const bool more = taken(&bars->next[nx], bx, by);
+    const bool more = pb::clc_taken(&bars->next[nx], b);
     pb::fence_proxy_async_smem();
     pb::mbar_arrive(&bars->next_empty[nx]);
     return more;
@@ -209,10 +184,10 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (warp == 0 && pb::elect_one()) {
       // ------------------------------------------------------------------ scheduler and producer
       [&]() -> bool {
-        int bx = blockIdx.x, by = blockIdx.y;
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
         uint32_t kc = 0, vc = 0, qc[2] = {0, 0};       // K / V blocks and Q tiles loaded so far
         for (uint32_t item = 0;; ++item) {
-          const FaItem w = item_of(bx, by);
+          const FaItem w = item_of(b);
           const int tok0 = w.batch * seq, tokk0 = w.batch * seq_k;
           const uint32_t nx = item & 1;
           // K of a step before V of the step before: that is the order in which the issuer needs them
@@ -222,7 +197,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               // runs out of work first (2048 x 32/8 x 128: 48 us asked for at the start of a pair, 39 us here).
               FA_WAIT(&bars->next_empty[nx], ((item >> 1) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
               pb::mbar_expect_tx(&bars->next_full[nx], 16);
-              try_cancel(&bars->next[nx], &bars->next_full[nx]);
+              pb::clc_try_cancel(&bars->next[nx], &bars->next_full[nx]);
             } else {
               const uint32_t ks = kc % C::KS;
               FA_WAIT(&bars->k_empty[ks], ((kc / C::KS) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
@@ -257,7 +232,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             }
           }
           FA_WAIT(&bars->next_full[nx], (item >> 1) & 1, PB_ERR_TIMEOUT_TMA);
-          if (!taken(&bars->next[nx], bx, by)) return true;
+          if (!pb::clc_taken(&bars->next[nx], b)) return true;
         }
       }();
     } else if (warp == 1 && pb::elect_one()) {
@@ -265,9 +240,9 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       [&]() -> bool {
         constexpr uint32_t idesc = pb::make_idesc_bf16(BQ, BKV, 0, 0);
         uint32_t s_count = 0, kc = 0, qc[2] = {0, 0};  // S, K blocks and Q tiles so far
-        int bx = blockIdx.x, by = blockIdx.y;
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
         for (uint32_t item = 0;; ++item) {
-          const FaItem w = item_of(bx, by);
+          const FaItem w = item_of(b);
           for (int j = 0; j < w.n; ++j, ++kc) {
             const uint32_t ks = kc % C::KS;
             FA_WAIT(&bars->k_full[ks], (kc / C::KS) & 1, PB_ERR_TIMEOUT_MMA);
@@ -293,7 +268,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (C::STAGE && j == w.nb[t] - 1) pb::umma_commit(&bars->q_empty[t]);
             }
           }
-          if (!next_item(item, bx, by)) return true;
+          if (!next_item(item, b)) return true;
         }
       }();
     } else if (warp == 2 && pb::elect_one()) {
@@ -301,9 +276,9 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       [&]() -> bool {
         constexpr uint32_t idesc = pb::make_idesc_bf16(BQ, DV, 0, 1);
         uint32_t vc = 0, pc[2] = {0, 0}, oc[2] = {0, 0};   // V blocks so far; per tile: products, finished outputs
-        int bx = blockIdx.x, by = blockIdx.y;
+        int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
         for (uint32_t item = 0;; ++item) {
-          const FaItem w = item_of(bx, by);
+          const FaItem w = item_of(b);
           for (int j = 0; j < w.n; ++j, ++vc) {
             const uint32_t vs = vc % C::VS;
             FA_WAIT(&bars->v_full[vs], (vc / C::VS) & 1, PB_ERR_TIMEOUT_MMA);
@@ -326,7 +301,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
               if (t == 1 || !w.has(1, j)) pb::umma_commit(&bars->v_empty[vs]);
             }
           }
-          if (!next_item(item, bx, by)) return true;
+          if (!next_item(item, b)) return true;
         }
       }();
     }
@@ -343,10 +318,10 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint32_t t_o = tmem_base + lane_addr + O_COL + t * 128;
       const bool leader = (threadIdx.x & 127) == 0;
       const uint64_t scale2 = pb::pack_f32x2(scale_log2, scale_log2);
-      int bx = blockIdx.x, by = blockIdx.y;
+      int3 b = make_int3(blockIdx.x, blockIdx.y, blockIdx.z);
       uint32_t count = 0;                       // blocks of this tile so far
       for (uint32_t item = 0;; ++item) {
-        const FaItem w = item_of(bx, by);
+        const FaItem w = item_of(b);
         const int qk = w.qt0 + t + q_off_blocks;
         float m_ref = -1e30f;
         float l = 0.f;
@@ -496,7 +471,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             pb::mbar_arrive(&bars->q_empty[t]);
           }
         }
-        if (!next_item(item, bx, by)) break;
+        if (!next_item(item, b)) break;
       }
       if (leader) pb::tma_store_wait_all<0>();
       return true;
@@ -537,7 +512,7 @@ int launch_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
     if (e != cudaSuccess) return (int)e;
     attr_set[win] = true;
   }
-  dim3 grid(hq * batch, (seq / BQ + 1) / 2, 1);
+  dim3 grid(hq, batch, (seq / BQ + 1) / 2);
   kern<<<grid, FA_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, to, lse, seq, seq_k, q_off / BQ, hq, hkv,
                                                    scale * 1.4426950408889634f, causal, window, sinks, softcap, status);
   return (int)cudaGetLastError();
