@@ -1201,9 +1201,9 @@ struct BwdArgs {
 // and its mean load per SM; a block more costs `fixed` microseconds for start and end, with a cluster more for the exchange
 // of the sums.  Few key / value heads leave long blocks and idle SMs: 4096 tokens, 32 query heads on 4 key / value heads of
 // 128 have 128 blocks of up to 256 steps but work for 114 steps per SM.  Measured (us, cluster 1 / 2 / 4 / 8), dK / dV pass:
-//   4096 x 32/4 x 128   484 / 265 / 314 / 442      1024 x 8/1 x 128   123 / 69 / 43 / 34     8192 x 1/1 x 128   126 / 72 / 61 / 129
-//   8192 x 32/8 x 128   910 / 948 / 1203 / 1736    2048 x 16/2 x 64   199 / 107 / 60 / 63    window 128, 64/8 x 64  76 / 97 / 141 / 268
-// dQ pass: 2048 x 32/8 x 128  65 / 104 / 211 / 457   8192 x 1/1 x 128  96 / 55 / 46 / 84.  The model below is within 10 % of
+//   4096 x 32/4 x 128   399 / 221 / 264 / 395      1024 x 8/1 x 128   101 / 58 / 38 / 31     8192 x 1/1 x 128   104 / 62 / 56 / 123
+//   8192 x 32/8 x 128   803 / 835 / 1013 / 1511    2048 x 16/2 x 64   140 / 77 / 46 / 56     window 128, 64/8 x 64  60 / 86 / 130 / 258
+// dQ pass: 2048 x 32/8 x 128  49 / 97 / 202 / 459   8192 x 1/1 x 128  79 / 46 / 41 / 82.  The model below is within 15 % of
 // these.  Clusters of 4 and 8 do not fit every GPC: 132 and 120 CTAs in flight on 148 SMs.
 int bwd_cluster_size(int mode, int d_qk, int d_v, int batch, int seq, int seq_k, int q_off, int hq, int hkv, int causal,
                      int window) {
@@ -1228,8 +1228,8 @@ int bwd_cluster_size(int mode, int d_qk, int d_v, int batch, int seq, int seq_k,
     longest = n > longest ? n : longest;
   }
   const double heads = (double)batch * (kv ? hkv : hq);
-  const double step = d_qk == 64 ? (kv ? 1.5 : 1.25) : d_qk == d_v ? (kv ? 1.95 : 1.5) : (kv ? 1.6 : 1.7);
-  static const double fixed_kv[4] = {5., 9., 14., 20.}, fixed_q[4] = {4., 8., 11., 14.}, sms[4] = {1., 1., 0.89, 0.81};
+  const double step = d_qk == 64 ? (kv ? 1.1 : 1.) : d_qk == d_v ? (kv ? 1.55 : 1.2) : (kv ? 1.3 : 1.4);
+  static const double fixed_kv[4] = {4., 9., 14., 20.}, fixed_q[4] = {3.5, 8., 11., 14.}, sms[4] = {1., 1., 0.89, 0.81};
   int best = 1;
   double t_best = 0.;
   for (int l = 0; l < 4; ++l) {
