@@ -221,10 +221,11 @@ def _clusters(batch, seq, hq, hkv, dqk, dv, causal, window):
     # batch, seq, hq, hkv, dqk, dv, causal, window; CTAs per block of the dK / dV and the dQ pass
     ((1, 128, 1, 1, 128, 128, True, 0), (1, 1)),            # one step: nothing to share
     ((1, 640, 3, 1, 64, 64, True, 0), (2, 1)),              # step counts that the ranks cannot share evenly
-    ((1, 2048, 8, 1, 128, 128, True, 0), (8, 2)),
+    ((1, 2048, 8, 1, 128, 128, True, 0), (8, 1)),
     ((1, 4096, 2, 1, 128, 128, False, 0), (4, 2)),
-    ((2, 1152, 2, 2, 192, 128, True, 0), (4, 2)),
-    ((1, 2048, 4, 1, 64, 64, True, 1000), (4, 2)),
+    ((2, 1152, 2, 2, 192, 128, True, 0), (2, 2)),
+    ((1, 2048, 1, 1, 192, 128, True, 0), (4, 4)),
+    ((1, 2048, 4, 1, 64, 64, True, 1000), (4, 1)),
 ])
 def test_flash_attn_backward_of_shared_blocks(case, clusters):
     """Blocks whose steps several CTAs share: gradients against the fp32 reference, equal from call to call, and into strided
