@@ -13,9 +13,11 @@ from __future__ import annotations
 import argparse
 import concurrent.futures
 import os
+import platform
 import shutil
 import subprocess
 import sys
+import sysconfig
 from pathlib import Path
 
 PKG_DIR = Path(__file__).resolve().parent
@@ -23,6 +25,9 @@ CSRC = PKG_DIR / "csrc"
 LIB_DIR = PKG_DIR / "lib"
 OBJ_DIR = LIB_DIR / "obj"
 LIB_PATH = LIB_DIR / "libprimus_b200.so"
+# the launchers' Python binding; its name says which interpreter it is for
+LAUNCH_SRC = CSRC / "python" / "launch.c"
+LAUNCH_PATH = LIB_DIR / ("_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -88,7 +93,22 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
+    _build_launch(force)
     return LIB_PATH
+
+
+def _build_launch(force: bool) -> None:
+    """The launchers' binding; without Python's headers, or on another architecture, calls go through ctypes."""
+    include = Path(sysconfig.get_paths()["include"])
+    if platform.machine() != "x86_64" or not (include / "Python.h").exists():
+        print("Python headers for x86-64 not found: launchers are called through ctypes", file=sys.stderr)
+        return
+    if not force and not _needs_build(LAUNCH_SRC, LAUNCH_PATH, []):
+        return
+    cmd = ["gcc", "-O2", "-shared", "-fPIC", "-I", str(include), str(LAUNCH_SRC), "-o", str(LAUNCH_PATH)]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError(f"binding failed:\n{p.stdout}{p.stderr}")
 
 
 def main() -> None:

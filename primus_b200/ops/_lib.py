@@ -8,7 +8,10 @@ to PyTorch for CUDA tensors (``require()`` raises if the library is missing).
 from __future__ import annotations
 
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
+import sysconfig
 import threading
 from pathlib import Path
 
@@ -71,18 +74,53 @@ def _ctype(a):
     return _PTR
 
 
-# Launchers bound so far: name -> (function with its argument types set from the first call, kernels per call).  ctypes then
-# converts plain integers and floats itself; wrapping every argument of every call in a ctypes object cost more than the
-# launch for the 20-argument launchers.  A later call may bring an argument of another kind (None after an integer, a ctypes
-# integer after a plain one): ctypes refuses it before anything is called, and the launcher is bound anew.
+def _load_launch():
+    """The compiled binding beside the library, or None: calls then go through ctypes."""
+    path = LIB_PATH.parent / ("_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    if not path.exists():
+        return None
+    loader = importlib.machinery.ExtensionFileLoader("_launch", str(path))
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_launch", loader))
+    loader.exec_module(module)
+    module.init(torch.Tensor)
+    return module
+
+
+_LAUNCH = _load_launch()
+
+# Launchers bound so far: name -> (function of (arguments, stream), kernels per call).  The kinds of a launcher's arguments are
+# those of its first call; an integer in a float's place is converted.  A later call may bring an argument of another kind
+# (None after an integer, a ctypes integer after a plain one): it is refused before anything is called, and the launcher is
+# bound anew.
 _BOUND: dict = {}
+
+
+def _ctypes_launcher(fn, argtypes, stream: bool):
+    """What the compiled binding does, through ctypes: for ctypes values, and where the binding is not built."""
+    fn.restype = ctypes.c_int
+    fn.argtypes = argtypes + ([_PTR] if stream else [])
+
+    def launch(args, stream_ptr):
+        plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
+        if stream:
+            plain.append(stream_ptr)
+        try:
+            return fn(*plain)
+        except ctypes.ArgumentError:
+            return None
+
+    return launch
 
 
 def _bind(name: str, args, stream: bool):
     fn = load()["pb_" + name]       # an object of its own: argument types set here are not seen by other users
-    fn.restype = ctypes.c_int
-    fn.argtypes = [_ctype(a) for a in args] + ([_PTR] if stream else [])
-    _BOUND[name, stream] = bound = (fn, _KERNELS_PER_CALL.get(name, 1))
+    launch = None
+    if _LAUNCH is not None and all(a is None or isinstance(a, (torch.Tensor, int, float, bytes)) for a in args):
+        kinds = "".join("f" if isinstance(a, float) else "l" if isinstance(a, int) else "p" for a in args)
+        launch = _LAUNCH.bind(ctypes.cast(fn, _PTR).value, kinds.encode(), stream)
+    if launch is None:
+        launch = _ctypes_launcher(fn, [_ctype(a) for a in args], stream)
+    _BOUND[name, stream] = bound = (launch, _KERNELS_PER_CALL.get(name, 1))
     return bound
 
 
@@ -92,29 +130,31 @@ _KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "sumsq": 2, "flash_attn_bwd": 3, "quant_f
 LAUNCH_COUNT = 0
 
 
+def _bound_anew(name: str, args, stream: bool, stream_ptr: int) -> int:
+    rc = _bind(name, args, stream)[0](args, stream_ptr)
+    if rc is None:
+        raise ctypes.ArgumentError(f"pb_{name}: an argument cannot be passed: {args}")
+    return rc
+
+
 def call(name: str, *args) -> None:
     """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended."""
     global LAUNCH_COUNT
-    fn, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
+    launch, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
     LAUNCH_COUNT += kernels
-    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
-    plain.append(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))
-    try:
-        rc = fn(*plain)
-    except ctypes.ArgumentError:
-        rc = _bind(name, args, True)[0](*plain)
+    stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    rc = launch(args, stream)
+    if rc is None:
+        rc = _bound_anew(name, args, True, stream)
     if rc != 0:
         raise NativeLibraryError(f"pb_{name} failed with code {rc}")
 
 
 def call_ret(name: str, *args) -> int:
     """Invoke a host-only helper that returns a value (no stream appended)."""
-    fn, _ = _BOUND.get((name, False)) or _bind(name, args, False)
-    plain = [a.data_ptr() if isinstance(a, torch.Tensor) else a for a in args]
-    try:
-        return fn(*plain)
-    except ctypes.ArgumentError:
-        return _bind(name, args, False)[0](*plain)
+    launch, _ = _BOUND.get((name, False)) or _bind(name, args, False)
+    rc = launch(args, 0)
+    return _bound_anew(name, args, False, 0) if rc is None else rc
 
 
 class I32(int):

@@ -118,6 +118,39 @@ def test_launcher_takes_floats_after_an_integer(launchers):
     assert _lib.call_ret("first_byte", b"a") == ord("a")
 
 
+MIXED = r"""
+extern "C" int pb_mixed(const void* a, int b, float c, long d, float e, const void* f, int g, int h, float i, long j, int k, int l,
+                        float m, long n, int o, long p, void* stream) {
+  return !(a == (void*)16 && b == -3 && c == 1.5f && d == -(1L << 40) && e == -0.25f && !f && g == 7 && h == -8 && i == 3.f &&
+           j == 9 && k == 1 && l == 0 && m != m && n == 13 && o == -1 && p == (1L << 62) && stream == (void*)7);
+}
+extern "C" int pb_nine(float a, float b, float c, float d, float e, float f, float g, float h, float i, int n, void* stream) {
+  return (int)(a + b + c + d + e + f + g + h + 2 * i) + n - (int)(long)stream;
+}
+"""
+
+
+@pytest.mark.parametrize("compiled", [True, False])
+def test_launcher_arguments_keep_their_places(compiled, tmp_path, monkeypatch):
+    """Integers beyond the six registers between floats, 32-bit negatives, an integer in a float's place; more floats than
+    registers.  Through the compiled binding and through ctypes."""
+    if compiled and _lib._LAUNCH is None:
+        pytest.skip("the binding is not built")
+    monkeypatch.setattr(_lib, "_LIB", ctypes.CDLL(str(_compile(tmp_path, "mixed", MIXED, "-shared", "-fPIC"))))
+    monkeypatch.setattr(_lib, "_BOUND", {})
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 0)
+    monkeypatch.setattr(torch._C, "_cuda_getCurrentRawStream", lambda device: 7)
+    if not compiled:
+        monkeypatch.setattr(_lib, "_LAUNCH", None)
+    for i in (3.0, 3):
+        _lib.call("mixed", 16, -3, 1.5, -(1 << 40), -0.25, None, 7, -8, i, 9, True, False, float("nan"), 13, -1, 1 << 62)
+    with pytest.raises(_lib.NativeLibraryError, match="code 1"):
+        _lib.call("mixed", 16, -3, 1.5, -(1 << 40), -0.25, None, 7, -8, 4, 9, True, False, float("nan"), 13, -1, 1 << 62)
+    _lib.call("nine", *[1.0] * 8, 2.0, -5)
+    with pytest.raises(ctypes.ArgumentError):
+        _lib.call("nine", *[1.0] * 8, object(), -5)
+
+
 # Stands in for the CUDA runtime: launches are recorded as "device <d> shared <bytes>", and refused where a kernel asks for more
 # than 48 KB without having been given the attribute on that device, or when `fail_next` says so.
 RUNTIME = r"""
