@@ -532,6 +532,7 @@ qk_norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 // 128-byte reads, eight in flight) and a fixed-order tree in shared memory folds them, so the result does not depend on
 // scheduling.
 constexpr int DWR_COLS = 32, DWR_ROWS = 16;
+constexpr int DW_STORE_BF16 = 2;     // of `accumulate`: dw is a bf16 vector, and stored
 __global__ void __launch_bounds__(DWR_COLS * DWR_ROWS)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, long ld, int accumulate) {
   __shared__ float red[DWR_ROWS][DWR_COLS + 1];
@@ -549,7 +550,10 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
     if (g < step) red[g][c] += red[g + step][c];
     __syncthreads();
   }
-  if (g == 0 && h < H) dw[h] = accumulate ? dw[h] + red[0][c] : red[0][c];
+  if (g == 0 && h < H) {
+    if (accumulate == DW_STORE_BF16) reinterpret_cast<__nv_bfloat16*>(dw)[h] = __float2bfloat16(red[0][c]);
+    else dw[h] = accumulate ? dw[h] + red[0][c] : red[0][c];
+  }
 }
 
 int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
@@ -579,7 +583,7 @@ int pb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
 // Number of CTAs (= rows of the [P, H] fp32 scratch) the backward uses for a given row count.
 int pb_rmsnorm_bwd_num_partials(long rows) { return (int)(rows < BWD_MAX_PARTIALS ? (rows < 1 ? 1 : rows) : BWD_MAX_PARTIALS); }
 
-// scratch: fp32 [pb_rmsnorm_bwd_num_partials(rows), H]. dw_accumulate: 1 -> dw += result.
+// scratch: fp32 [pb_rmsnorm_bwd_num_partials(rows), H]. dw_accumulate: 1 -> dw += result; 2 -> dw is a bf16 vector, stored.
 int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
                    void* dx, float* dw, float* scratch, long rows, int H, long ldx, long lddy,
                    int dw_accumulate, cudaStream_t s) {
@@ -625,8 +629,8 @@ int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk
   const int rc = (int)cudaGetLastError();
   if (rc) return rc;                                 // no gain sums from partial rows that nothing wrote
   const int blocks = (d + DWR_COLS - 1) / DWR_COLS, threads = DWR_COLS * DWR_ROWS;
-  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate);
-  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate);
+  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate != 0);
+  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate != 0);
   return (int)cudaGetLastError();
 }
 
@@ -667,5 +671,5 @@ extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void*
     g_noalloc_scratch_ptr[dev] = p;
   }
   const int P = (int)(rows < PB_NOALLOC_MAX_PARTIALS ? rows : PB_NOALLOC_MAX_PARTIALS);
-  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate, s);
+  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate != 0, s);
 }

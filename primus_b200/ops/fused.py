@@ -90,10 +90,12 @@ class RMSNormFn(torch.autograd.Function):
                       dy2.stride(0), 1)
             dw = None
         else:
-            dwf = torch.empty(H, dtype=torch.float32, device=xin.device)
-            _lib.call("rmsnorm_bwd", dy2, xin, w, rstd, dres, dx, dwf, sc, rows, H, xin.stride(0),
-                      dy2.stride(0), 0)
-            dw = dwf.to(w.dtype)
+            # (mode 2: rounded to bf16 by the kernel)
+            half = w.dtype == torch.bfloat16
+            dw = torch.empty(H, dtype=w.dtype if half else torch.float32, device=xin.device)
+            _lib.call("rmsnorm_bwd", dy2, xin, w, rstd, dres, dx, dw, sc, rows, H, xin.stride(0),
+                      dy2.stride(0), 2 if half else 0)
+            dw = dw.to(w.dtype)
         dx = dx.view(ctx.shape)
         if ctx.has_res:
             return dx, dw, None, dx

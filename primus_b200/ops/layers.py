@@ -98,10 +98,11 @@ class NormLinearFn(torch.autograd.Function):
                       dy.stride(0), 1)
             dnw = None
         else:
-            dwf = torch.empty(H, dtype=torch.float32, device=xsum.device)
-            _lib.call("rmsnorm_bwd", dy, xsum, norm_w, rstd, dres, dx, dwf, sc, rows, H, xsum.stride(0),
-                      dy.stride(0), 0)
-            dnw = dwf.to(norm_w.dtype)
+            half = norm_w.dtype == torch.bfloat16
+            dnw = torch.empty(H, dtype=norm_w.dtype if half else torch.float32, device=xsum.device)
+            _lib.call("rmsnorm_bwd", dy, xsum, norm_w, rstd, dres, dx, dnw, sc, rows, H, xsum.stride(0),
+                      dy.stride(0), 2 if half else 0)
+            dnw = dnw.to(norm_w.dtype)
         dx = dx.view(ctx.shape)
         return dx, (dx if ctx.has_res else None), dnw, dw, None, None, None
 
