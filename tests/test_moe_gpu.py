@@ -50,6 +50,35 @@ def test_schedule_and_grouped_gemm(counts):
         assert (w.main_grad[e] - refdw).abs().max() <= 2e-3 * refdw.abs().max() + 1e-3, f"expert {e}"
 
 
+@pytest.mark.parametrize("accumulate", [True, False])
+def test_grouped_weight_gradient_on_cta_pairs(accumulate):
+    """Gradients larger than L2: rows and columns that are no multiples of a tile, experts with no tokens (untouched when the
+    gradient is added to, zero when it is stored), and the same sums from call to call."""
+    counts, N, K = [0, 130, 1, 640, 0, 257, 128, 90, 384, 12, 500, 0], 2088, 2056
+    E = len(counts)
+    assert E * N * K >= 48 << 20                                                              # what goes to CTA pairs
+    s = _sched(counts, sum(counts))
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x = torch.randn(s.rows_cap, K, device="cuda", generator=g).bfloat16()
+    dy = torch.randn(s.rows_cap, N, device="cuda", generator=g).bfloat16()
+    old = torch.randn(E, N, K, device="cuda", generator=g)
+    got = [old.clone() for _ in range(2)]
+    for t in got:
+        _lib.call("grouped_gemm", 2, dy, x, t, s.rows_cap, N, K, E, s.mblock_expert, s.row_start, s.padded, int(accumulate),
+                  _lib.status_word(x.device))
+    torch.cuda.synchronize()
+    _lib.check_status()
+    assert torch.equal(*got)
+    start, padded = s.row_start.tolist(), s.padded.tolist()
+    for e in range(E):
+        rows = slice(start[e], start[e] + padded[e])
+        ref = dy[rows].double().t() @ x[rows].double() + (old[e].double() if accumulate else 0.0)
+        # fp32 sums of up to 640 products of magnitude 1
+        assert (got[0][e].double() - ref).abs().max() <= 640 * 2.0 ** -23 * 4, f"expert {e}"
+        if not padded[e]:
+            assert torch.equal(got[0][e], old[e] if accumulate else torch.zeros_like(old[e]))
+
+
 def test_gather_combine_roundtrip():
     T, k, H, E = 300, 2, 256, 5
     x = torch.randn(T, H, device="cuda").bfloat16().requires_grad_()
