@@ -530,9 +530,12 @@ __global__ void __launch_bounds__(512) sumsq_final_kernel(const float* __restric
   }
 }
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)) * extra
-__global__ void clip_coef_kernel(const float* sumsq, float max_norm, float extra, float* coef,
-                                 float* norm_out) {
+// skip (optional): set to whether the step is left out, because the sum is not finite (check) or above `spike` (if positive).
+// In this kernel because as operations of their own the checks are eight launches for one number.
+__global__ void clip_coef_kernel(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out, int* skip,
+                                 int check, float spike) {
   const float nrm = sqrtf(sumsq[0]);
+  if (skip) skip[0] = (check && !isfinite(sumsq[0])) || (spike > 0.f && sumsq[0] > spike);
   if (norm_out) norm_out[0] = nrm;
   float c = 1.f;
   if (max_norm > 0.f) c = fminf(1.f, max_norm / (nrm + 1e-6f));
@@ -723,9 +726,9 @@ int pb_sumsq(const void* x, int is_bf16, long n, float* scratch, float* out, int
   PB_CHECK_LAUNCH();
 }
 
-int pb_clip_coef(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out,
-                 cudaStream_t s) {
-  clip_coef_kernel<<<1, 1, 0, s>>>(sumsq, max_norm, extra, coef, norm_out);
+int pb_clip_coef(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out, int* skip, int check,
+                 float spike, cudaStream_t s) {
+  clip_coef_kernel<<<1, 1, 0, s>>>(sumsq, max_norm, extra, coef, norm_out, skip, check, spike);
   PB_CHECK_LAUNCH();
 }
 

@@ -93,16 +93,20 @@ def sumsq_(x, out, accumulate=False, nonfinite=None):
     return out
 
 
-def clip_coef_(sumsq, max_norm, coef, norm_out=None, extra=1.0):
-    """coef = min(1, max_norm/(sqrt(sumsq)+1e-6)) * extra, all on device."""
+def clip_coef_(sumsq, max_norm, coef, norm_out=None, extra=1.0, skip=None, check_finite=False, spike=0.0):
+    """coef = min(1, max_norm/(sqrt(sumsq)+1e-6)) * extra, all on device.  ``skip`` (int32): set to whether ``sumsq`` is not
+    finite (``check_finite``) or above ``spike`` (if positive)."""
     if not sumsq.is_cuda:
+        if skip is not None:
+            bad = ~torch.isfinite(sumsq) if check_finite else torch.zeros_like(sumsq, dtype=torch.bool)
+            skip.copy_(bad | (sumsq > spike) if spike > 0 else bad)
         nrm = sumsq[0].sqrt()
         if norm_out is not None:
             norm_out[0] = nrm
         c = torch.clamp(max_norm / (nrm + 1e-6), max=1.0) if max_norm > 0 else torch.tensor(1.0)
         coef[0] = c * extra
         return coef
-    _lib.call("clip_coef", sumsq, float(max_norm), float(extra), coef, norm_out)
+    _lib.call("clip_coef", sumsq, float(max_norm), float(extra), coef, norm_out, skip, int(check_finite), float(spike))
     return coef
 
 

@@ -492,7 +492,6 @@ class DistributedOptimizer:
     def compute_grad_norm(self):
         """Global L2 norm of the (already reduced) gradients, left on the device."""
         self.sumsq.zero_()
-        self.skip.zero_()
         if self.sanitize_grads:
             # non-finite gradient entries become zero before the norm and the non-finite check see them: the affected
             # elements simply get no update this step (the reference's SFT gradient sanitiser,
@@ -514,14 +513,15 @@ class DistributedOptimizer:
             self.sumsq.add_(self.sumsq_part)
         self._discount_tp_duplicates()
         self._reduce_sumsq()
-        if self.check_for_nan:
-            self.skip.copy_((~torch.isfinite(self.sumsq)).to(torch.int32))
-        if self.grad_spike_threshold and self.grad_spike_threshold > 0:
-            # a gradient-norm spike is treated like a non-finite step: nothing is updated (device-side, no host sync)
-            spike = (self.sumsq > float(self.grad_spike_threshold) ** 2).to(torch.int32)
-            self.skip.copy_(torch.maximum(self.skip, spike))
-        optim_ops.clip_coef_(self.sumsq, self.clip_grad if self.clip_grad else 0.0, self.coef, self.grad_norm)
+        # a gradient-norm spike is treated like a non-finite step: nothing is updated (device-side, no host sync)
+        self._clip_and_check(self.grad_spike_threshold)
         return self.grad_norm
+
+    def _clip_and_check(self, spike_threshold=None):
+        """Clip coefficient and norm from the squared sum; ``skip`` = whether the step is left out."""
+        spike = float(spike_threshold) ** 2 if spike_threshold and spike_threshold > 0 else 0.0
+        optim_ops.clip_coef_(self.sumsq, self.clip_grad if self.clip_grad else 0.0, self.coef, self.grad_norm,
+                             skip=self.skip, check_finite=bool(self.check_for_nan), spike=spike)
 
     @staticmethod
     def _is_expert_buffer(buf) -> bool:
@@ -537,7 +537,6 @@ class DistributedOptimizer:
         # the reduce-scatter of every bucket has been issued by ``finish_grad_sync`` (or, overlapped, by the gradient
         # hooks of the last micro-batch) and left this rank's reduced shards in place
         self.sumsq.zero_()
-        self.skip.zero_()
         for st in self.state:
             buf = st["buf"]
             if not buf.symmetric:
@@ -548,9 +547,7 @@ class DistributedOptimizer:
                 buf.sym_grad.barrier(1)  # everybody has read this rank's gradients: they may be zeroed again
         self._discount_tp_duplicates()
         self._reduce_sumsq()
-        if self.check_for_nan:
-            self.skip.copy_((~torch.isfinite(self.sumsq)).to(torch.int32))
-        optim_ops.clip_coef_(self.sumsq, self.clip_grad if self.clip_grad else 0.0, self.coef, self.grad_norm)
+        self._clip_and_check()
         bc1 = 1.0 - self.betas[0] ** self.step_count
         bc2 = 1.0 - self.betas[1] ** self.step_count
         base_lr = lr
@@ -666,11 +663,7 @@ class DistributedOptimizer:
             h.wait()
         for g in self.norm_groups[1:]:
             dist.all_reduce(self.sumsq, group=g)
-        if self.check_for_nan:
-            self.skip.copy_((~torch.isfinite(self.sumsq)).to(torch.int32))
-        if self.grad_spike_threshold and self.grad_spike_threshold > 0:
-            self.skip.copy_(torch.maximum(self.skip, (self.sumsq > float(self.grad_spike_threshold) ** 2).to(torch.int32)))
-        optim_ops.clip_coef_(self.sumsq, self.clip_grad if self.clip_grad else 0.0, self.coef, self.grad_norm)
+        self._clip_and_check(self.grad_spike_threshold)
         redo = bool(self.skip.item()) or float(self.coef.item()) < 1.0      # the validation: one scalar read
         if redo:
             self.post_validation_redos += 1

@@ -143,6 +143,20 @@ def test_adamw_and_norms():
     O.sumsq_(gb, ss)
     assert abs(ss.item() - gb.float().pow(2).sum().item()) <= 1e-3 * ss.item()
 
+@pytest.mark.parametrize("total, check, spike, skip", [
+    (4.0, True, 0.0, 0), (float("inf"), True, 0.0, 1), (float("nan"), True, 0.0, 1), (float("inf"), False, 0.0, 0),
+    (4.0, False, 4.0, 0), (4.25, False, 4.0, 1), (float("nan"), False, 4.0, 0), (float("nan"), True, 4.0, 1), (9.0, True, 4.0, 1),
+])
+@pytest.mark.parametrize("device", ["cpu", "cuda"])
+def test_clip_coefficient_marks_steps_to_leave_out(device, total, check, spike, skip):
+    """A squared sum that is not finite, or above the spike limit; a mark of an earlier step is taken back."""
+    ss = torch.tensor([total], device=device)
+    coef, mark = torch.zeros(1, device=device), torch.full((1,), 1 - skip, dtype=torch.int32, device=device)
+    O.clip_coef_(ss, 1.0, coef, skip=mark, check_finite=check, spike=spike)
+    assert mark.item() == skip
+    if total == total and total < float("inf"):
+        assert abs(coef.item() - 1 / (total ** 0.5 + 1e-6)) <= 1e-6
+
 
 def test_embedding_backward_main_grad():
     V, H, T = 1000, 256, 4096
