@@ -136,6 +136,8 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 
 // ------------------------------------------------------------------ backward
 // dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x)  (+ dres when given)
+// dx2 (optional) receives dx once more: gradients of two inputs that autograd would have to copy otherwise (it keeps one tensor
+// per leaf).  16384 x 8192: a second store 41 us, the copy 83 us.
 // dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
 
 // Rows of up to 1024 channels: LPR <= 32 lanes per row, no barrier in the loop, RPG rows per group in flight.  The dw
@@ -145,7 +147,7 @@ __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                          const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                         float* __restrict__ partial, long rows, int H, long ldx, long lddy) {
+                         __nv_bfloat16* __restrict__ dx2, float* __restrict__ partial, long rows, int H, long ldx, long lddy) {
   constexpr int GROUPS = 256 / LPR;
   __shared__ float4 sums[GROUPS][LPR * VPL * 2];
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
@@ -208,7 +210,9 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
 #pragma unroll
             for (int j = 0; j < 8; ++j) o[j] += fx[j];
           }
-          reinterpret_cast<Bf8*>(dx + (row0 + r) * ldx)[lane + k * LPR] = f_to_bf8(o);
+          const Bf8 ob = f_to_bf8(o);
+          reinterpret_cast<Bf8*>(dx + (row0 + r) * ldx)[lane + k * LPR] = ob;
+          if (dx2) reinterpret_cast<Bf8*>(dx2 + (row0 + r) * ldx)[lane + k * LPR] = ob;
         }
     }
   }
@@ -238,7 +242,7 @@ __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                   float* __restrict__ partial, long rows, int H, long ldx, long lddy, int stages) {
+                   __nv_bfloat16* __restrict__ dx2, float* __restrict__ partial, long rows, int H, long ldx, long lddy, int stages) {
   extern __shared__ __align__(16) uint8_t ring_raw[];
   __shared__ float red[2][THREADS / 32];
   constexpr int OPS = RES ? 3 : 2;
@@ -323,7 +327,9 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 #pragma unroll
           for (int j = 0; j < 8; ++j) o[j] += fx[j];
         }
-        reinterpret_cast<Bf8*>(dx + row * ldx)[tid + k * THREADS] = f_to_bf8(o);
+        const Bf8 ob = f_to_bf8(o);
+        reinterpret_cast<Bf8*>(dx + row * ldx)[tid + k * THREADS] = ob;
+        if (RES && dx2) reinterpret_cast<Bf8*>(dx2 + row * ldx)[tid + k * THREADS] = ob;
       }
     rs = rs_next;
     flip ^= 1;
@@ -354,8 +360,8 @@ inline int bwd_ctas(int P, long rows, int H) {
 
 template <int VPT, int THREADS, bool RES>
 int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
-                            const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, long rows,
-                            int H, long ldx, long lddy) {
+                            const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, __nv_bfloat16* dx2,
+                            float* partial, long rows, int H, long ldx, long lddy) {
   constexpr int STAGE = (RES ? 3 : 2) * VPT * THREADS * 16;
   // four rows ahead where two CTAs of an SM then still fit into its shared memory, else two
   constexpr int STAGES = 4 * STAGE <= 100 * 1024 ? 4 : 2;
@@ -363,22 +369,23 @@ int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, cons
   static std::atomic<bool> allowed[pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, STAGES * STAGE, allowed);
   if (rc) return rc;
-  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy, STAGES);
+  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy, STAGES);
   return (int)cudaGetLastError();
 }
 
 int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
-                       const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, float* partial, long rows, int H,
-                       long ldx, long lddy) {
+                       const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, __nv_bfloat16* dx2, float* partial,
+                       long rows, int H, long ldx, long lddy) {
   const int nv = H / 8;
 #define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                         \
   {                                                                                                              \
-    rmsnorm_bwd_short_kernel<LPR, VPL, RPG><<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy); \
+    rmsnorm_bwd_short_kernel<LPR, VPL, RPG><<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, \
+                                                               lddy);                                            \
     return (int)cudaGetLastError();                                                                              \
   }
 #define PB_NORM_BWD(VPT, THREADS)                                                                                     \
-  return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy) \
-              : launch_rmsnorm_bwd_ring<VPT, THREADS, false>(P, s, dy, x, w, rstd, dres, dx, partial, rows, H, ldx, lddy)
+  return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy) \
+              : launch_rmsnorm_bwd_ring<VPT, THREADS, false>(P, s, dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy)
   const bool few = rows * nv < 148 * 512L * 4;   // (two CTAs of 256 threads per SM)
   if (nv <= 8) { if (few) PB_NORM_BWD_SHORT(8, 1, 1) else PB_NORM_BWD_SHORT(8, 1, 4) }
   if (nv <= 16) { if (few) PB_NORM_BWD_SHORT(16, 1, 1) else PB_NORM_BWD_SHORT(16, 1, 4) }
@@ -556,12 +563,13 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
   }
 }
 
-int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
                 float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
   // every one of the partial rows is fully written by its CTA before the reduction reads it
   P = bwd_ctas(P, rows, H);
   const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
-                                    (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, scratch, rows, H, ldx, lddy);
+                                    (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, rows, H,
+                                    ldx, lddy);
   if (rc) return rc;
   rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, H, dw_accumulate);
   return (int)cudaGetLastError();
@@ -589,7 +597,16 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
                    int dw_accumulate, cudaStream_t s) {
   if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L) return -2;
   if (rows == 0) return 0;
-  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dw, scratch, rows, H, ldx, lddy,
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, nullptr, dw, scratch, rows, H, ldx, lddy,
+                     dw_accumulate, s);
+}
+
+// dx is written twice, to dx and to dx2 (with dres only).
+int pb_rmsnorm_bwd_two(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
+                       float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
+  if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || !dres) return -2;
+  if (rows == 0) return 0;
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
 
@@ -671,5 +688,5 @@ extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void*
     g_noalloc_scratch_ptr[dev] = p;
   }
   const int P = (int)(rows < PB_NOALLOC_MAX_PARTIALS ? rows : PB_NOALLOC_MAX_PARTIALS);
-  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate != 0, s);
+  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, nullptr, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate != 0, s);
 }

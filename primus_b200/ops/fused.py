@@ -62,6 +62,7 @@ class RMSNormFn(torch.autograd.Function):
             _lib.call("rmsnorm_fwd", x2, None, w, y, None, rstd, rows, H, x2.stride(0), y.stride(0), float(eps))
             ctx.save_for_backward(x2, w, rstd)
         ctx.has_res = residual is not None
+        ctx.two = two_leaves(x, residual)
         ctx.shape = x.shape
         ctx.w_ref = w
         if residual is not None:
@@ -84,22 +85,36 @@ class RMSNormFn(torch.autograd.Function):
         dx = torch.empty_like(xin)
         P = _lib.call_ret("rmsnorm_bwd_num_partials", rows)
         sc = scratch(xin.device, "rmsnorm_dw", P * H)
-        main_grad = getattr(ctx.w_ref, "main_grad", None)
-        if main_grad is not None:
-            _lib.call("rmsnorm_bwd", dy2, xin, w, rstd, dres, dx, main_grad, sc, rows, H, xin.stride(0),
-                      dy2.stride(0), 1)
-            dw = None
-        else:
-            # (mode 2: rounded to bf16 by the kernel)
-            half = w.dtype == torch.bfloat16
-            dw = torch.empty(H, dtype=w.dtype if half else torch.float32, device=xin.device)
-            _lib.call("rmsnorm_bwd", dy2, xin, w, rstd, dres, dx, dw, sc, rows, H, xin.stride(0),
-                      dy2.stride(0), 2 if half else 0)
-            dw = dw.to(w.dtype)
+        dx, dx2, dw = norm_backward(dy2, xin, w, rstd, dres, dx, sc, getattr(ctx.w_ref, "main_grad", None), ctx.two)
         dx = dx.view(ctx.shape)
         if ctx.has_res:
-            return dx, dw, None, dx
+            return dx, dw, None, dx2.view(ctx.shape)
         return dx, dw, None, None
+
+
+def two_leaves(x, residual) -> bool:
+    """Whether the gradient that ``x`` and ``residual`` share has to exist twice: autograd keeps a tensor per leaf, and would
+    copy the shared one.  (Inside a model it goes on to two producers, which read it.)"""
+    return (residual is not None and residual is not x and x.is_leaf and residual.is_leaf and x.requires_grad
+            and residual.requires_grad)
+
+
+def norm_backward(dy, xin, w, rstd, dres, dx, sc, main_grad, two):
+    """(dx, the residual's gradient, dw or None when it was added to ``main_grad``); dx is shared unless ``two``."""
+    rows, H = xin.shape
+    if main_grad is not None:
+        target, mode = main_grad, 1
+    elif w.dtype == torch.bfloat16:             # rounded by the kernel
+        target, mode = torch.empty(H, dtype=w.dtype, device=xin.device), 2
+    else:
+        target, mode = torch.empty(H, dtype=torch.float32, device=xin.device), 0
+    dx2 = dx
+    if two and dres is not None:
+        dx2 = torch.empty_like(dx)
+        _lib.call("rmsnorm_bwd_two", dy, xin, w, rstd, dres, dx, dx2, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
+    else:
+        _lib.call("rmsnorm_bwd", dy, xin, w, rstd, dres, dx, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
+    return dx, dx2, None if main_grad is not None else target.to(w.dtype)
 
 
 # ``apply_layernorm_1p``: the norm weights are stored centred on zero and the norm multiplies by ``1 + weight`` (weight

@@ -49,6 +49,7 @@ class NormLinearFn(torch.autograd.Function):
         ctx.tp = (tp_group, sp)
         ctx.set_materialize_grads(False)
         ctx.has_res = residual is not None
+        ctx.two = fused.two_leaves(hidden, residual)
         ctx.shape = hidden.shape
         ctx.refs = (norm_w, weight)
         if residual is not None:
@@ -92,19 +93,9 @@ class NormLinearFn(torch.autograd.Function):
         dx = torch.empty_like(xsum)
         P = _lib.call_ret("rmsnorm_bwd_num_partials", rows)
         sc = fused.scratch(xsum.device, "rmsnorm_dw", P * H)
-        main_grad = getattr(norm_w_ref, "main_grad", None)
-        if main_grad is not None:
-            _lib.call("rmsnorm_bwd", dy, xsum, norm_w, rstd, dres, dx, main_grad, sc, rows, H, xsum.stride(0),
-                      dy.stride(0), 1)
-            dnw = None
-        else:
-            half = norm_w.dtype == torch.bfloat16
-            dnw = torch.empty(H, dtype=norm_w.dtype if half else torch.float32, device=xsum.device)
-            _lib.call("rmsnorm_bwd", dy, xsum, norm_w, rstd, dres, dx, dnw, sc, rows, H, xsum.stride(0),
-                      dy.stride(0), 2 if half else 0)
-            dnw = dnw.to(norm_w.dtype)
-        dx = dx.view(ctx.shape)
-        return dx, (dx if ctx.has_res else None), dnw, dw, None, None, None
+        dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, dx, sc, getattr(norm_w_ref, "main_grad", None), ctx.two)
+        dx, dx2 = dx.view(ctx.shape), dx2.view(ctx.shape)
+        return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
 
 
 def norm_linear(hidden, residual, norm_w, weight, eps, tp_group=None, sequence_parallel=False):

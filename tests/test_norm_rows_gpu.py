@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from primus_b200.ops import fused
+from primus_b200.ops import fused, layers
 
 from .test_kernel_edges_gpu import _close_bf16, _gen, _rms64
 
@@ -24,3 +24,30 @@ def test_norm_and_gradients(rows, H):
     _close_bf16(y.detach(), y64.detach(), "y")
     _close_bf16(leaves[0].grad, s64.grad, "dx")
     _close_bf16(leaves[1].grad, w64.grad, "dw")
+
+
+@pytest.mark.parametrize("rows, H", [(1, 8), (37, 64), (700, 520), (129, 1024), (200, 2048), (33, 4104), (40, 8192), (5, 16384)])
+@pytest.mark.parametrize("layer", [False, True])
+def test_gradients_of_two_leaves_are_two_tensors(rows, H, layer):
+    """The shared input gradient is written twice where both inputs are leaves, and equals the one that producers share."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, r, dy, ds = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(4))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    proj = (torch.randn(128, H, device="cuda", generator=g) * 0.02).bfloat16()
+
+    def grads(leaves):
+        a, b, p = x.clone().requires_grad_(), r.clone().requires_grad_(), torch.nn.Parameter(w.clone())
+        ia, ib = (a, b) if leaves else (a * 1, b * 1)
+        if layer:
+            y, s = layers.norm_linear(ia, ib, p, torch.nn.Parameter(proj.clone()), 1e-5)
+            torch.autograd.backward([y, s], [dy[:, :1].expand(rows, 128).contiguous(), ds])
+        else:
+            y, s = fused.rmsnorm(ia, p, 1e-5, ib)
+            torch.autograd.backward([y, s], [dy, ds])
+        return a.grad, b.grad, p.grad
+
+    two, shared = grads(True), grads(False)
+    assert two[0].data_ptr() != two[1].data_ptr()
+    for t, u in zip(two, shared):
+        assert torch.equal(t, u)
+    assert torch.equal(two[0], two[1])
