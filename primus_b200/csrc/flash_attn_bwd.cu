@@ -1186,7 +1186,7 @@ attn_sink_grad_kernel(const float* __restrict__ delta, const float* __restrict__
 struct BwdArgs {
   const void *d_o, *q, *k, *v, *o;
   const float* lse;
-  float* delta;
+  float *delta, *neg_lse2;
   void *dq, *dk, *dv;
   int batch, seq, seq_k, q_off, window, hq, hkv;
   float softcap;
@@ -1252,7 +1252,7 @@ int launch_bwd(const BwdArgs& a) {
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
   const long T = (long)a.batch * a.seq;
   attn_delta_kernel<DV><<<dim3((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS), DL_THREADS, 0, a.stream>>>(
-      (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.delta + (long)a.batch * a.hq * a.seq, a.seq,
+      (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.neg_lse2, a.seq,
       a.hq, a.o_row, a.do_row);
   int rc;
   CUtensorMap q128, do128, k128, v128, q64, do64, dq_m, dk_m, dv_m;
@@ -1266,7 +1266,7 @@ int launch_bwd(const BwdArgs& a) {
   MK(dv_m, a.dv, TK, a.hkv, DV, a.dv_row, 128)
 #undef MK
   const int var = a.softcap > 0.f ? 2 : (a.window > 0 ? 1 : 0);
-  const float* lse2 = a.delta + (long)a.batch * a.hq * a.seq;
+  const float* lse2 = a.neg_lse2;
   auto cluster = [&](int mode) {
     return bwd_cluster_size(mode, DQK, DV, a.batch, a.seq, a.seq_k, a.q_off, a.hq, a.hkv, a.causal, a.window);
   };
@@ -1327,16 +1327,26 @@ extern "C" int pb_flash_attn_bwd_cap(const void* d_o, const void* q, const void*
                                      long v_row, long o_row, long do_row, long dq_row, long dk_row, long dv_row,
                                      float scale, int causal, int window, float softcap, int* status,
                                      cudaStream_t stream) {
-  if (seq % 128 || seq_k % 128 || q_off % 128 || q_off < 0 || hq % hkv) return -2;
+  if (batch <= 0 || seq % 128 || seq_k % 128 || q_off % 128 || q_off < 0 || hq % hkv) return -2;
   if (causal ? (q_off + seq != seq_k) : (q_off != 0)) return -2;
   if (window < 0 || (window > 0 && (!causal || q_off != 0)) || softcap < 0.f) return -2;
   if ((q_row | k_row | v_row | o_row | do_row | dq_row | dk_row | dv_row) % 8) return -2;
-  BwdArgs a{d_o, q, k, v, o, lse, delta, dq, dk, dv, batch, seq, seq_k, q_off, window, hq, hkv, softcap, q_row, k_row,
-            v_row, o_row, do_row, dq_row, dk_row, dv_row, scale, causal, status, stream};
-  if (d_qk == 128 && d_v == 128) return launch_bwd<128, 128>(a);
-  if (d_qk == 192 && d_v == 128) return launch_bwd<192, 128>(a);
-  if (d_qk == 64 && d_v == 64) return launch_bwd<64, 64>(a);
-  return -3;
+  constexpr int MAX_BATCH = 65535;             // (sequences are the grid's second dimension)
+  float* neg_lse2 = delta + (long)batch * hq * seq;
+  for (int b = 0; b < batch; b += MAX_BATCH) {
+    const long tq = (long)b * seq, tk = (long)b * seq_k;
+    auto at = [](const void* p, long rows, long pitch) { return static_cast<const __nv_bfloat16*>(p) + rows * pitch; };
+    auto to = [](void* p, long rows, long pitch) { return static_cast<__nv_bfloat16*>(p) + rows * pitch; };
+    BwdArgs a{at(d_o, tq, do_row), at(q, tq, q_row), at(k, tk, k_row), at(v, tk, v_row), at(o, tq, o_row), lse + tq * hq,
+              delta + tq * hq, neg_lse2 + tq * hq, to(dq, tq, dq_row), to(dk, tk, dk_row), to(dv, tk, dv_row),
+              batch - b < MAX_BATCH ? batch - b : MAX_BATCH, seq, seq_k, q_off, window, hq, hkv, softcap, q_row, k_row, v_row,
+              o_row, do_row, dq_row, dk_row, dv_row, scale, causal, status, stream};
+    const int rc = d_qk == 128 && d_v == 128   ? launch_bwd<128, 128>(a)
+                   : d_qk == 192 && d_v == 128 ? launch_bwd<192, 128>(a)
+                   : d_qk == 64 && d_v == 64   ? launch_bwd<64, 64>(a) : -3;
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 // CTAs per row block that pb_flash_attn_bwd_cap launches: pass 0 dK / dV, 1 dQ (host only).

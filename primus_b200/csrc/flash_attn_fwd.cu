@@ -31,6 +31,7 @@ constexpr int BQ = 128;
 constexpr int BKV = 128;
 constexpr int ATOM_BYTES = 128 * 128;  // 128 rows x 64 bf16
 constexpr int FA_THREADS = 384;
+constexpr int MAX_GRID_Y = 65535;
 // Registers move from the producer / issuer warpgroup to the softmax warpgroups, which hold a row of S: 4 * 120 + 8 * 192 =
 // 12 * 168 per lane, the allocation of the launch.
 constexpr int FA_REGS_AUX = 120, FA_REGS_SOFTMAX = 192;
@@ -534,6 +535,18 @@ extern "C" int pb_flash_attn_fwd_cap(const void* q, const void* k, const void* v
     return -2;
   if (causal ? (q_off + seq != seq_k) : (q_off != 0)) return -2;
   if (window < 0 || (window > 0 && (!causal || q_off != 0)) || softcap < 0.f) return -2;
+  if (batch > MAX_GRID_Y) {                    // (sequences are the grid's second dimension)
+    for (int b = 0; b < batch; b += MAX_GRID_Y) {
+      const long tq = (long)b * seq, tk = (long)b * seq_k;
+      auto at = [](const void* p, long rows, long pitch) { return static_cast<const __nv_bfloat16*>(p) + rows * pitch; };
+      const int rc = pb_flash_attn_fwd_cap(at(q, tq, q_row), at(k, tk, k_row), at(v, tk, v_row),
+                                           const_cast<__nv_bfloat16*>(at(o, tq, o_row)), lse + tq * hq,
+                                           batch - b < MAX_GRID_Y ? batch - b : MAX_GRID_Y, seq, seq_k, q_off, hq, hkv, d_qk, d_v,
+                                           q_row, k_row, v_row, o_row, scale, causal, window, sinks, softcap, status, stream);
+      if (rc) return rc;
+    }
+    return 0;
+  }
   if (d_qk == 128 && d_v == 128)
     return launch_fwd<128, 128>(q, k, v, o, lse, batch, seq, seq_k, q_off, hq, hkv, q_row, k_row, v_row, o_row, scale,
                                 causal, window, sinks, softcap, status, stream);

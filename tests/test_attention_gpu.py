@@ -252,3 +252,22 @@ def test_flash_attn_backward_of_shared_blocks(case, clusters):
         assert torch.equal(a, b), name
         rel = (a.float() - r.grad).norm().item() / r.grad.norm().item()
         assert rel <= 1e-2, f"{name}: relative error {rel}"     # P, dS and the results in bf16: 2^-9 each, 3e-3 measured
+
+
+def test_flash_attn_more_sequences_than_a_grid_dimension():
+    """65537 sequences of 128 tokens: the first, those around the limit and the last, forward and backward."""
+    batch, seq, d = 65537, 128, 64
+    q, k, v = _inputs(batch, seq, 1, 1, d, d, seed=9)
+    do = torch.randn_like(q)
+    scale = 1.0 / math.sqrt(d)
+    o, lse = A.flash_attn_fwd(q, k, v, batch, True, scale)
+    grads = A.flash_attn_bwd(do, q, k, v, o, lse, batch, True, scale)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    for b in (0, 65534, 65535, 65536):
+        r = slice(b * seq, (b + 1) * seq)
+        one_o, one_lse = A.flash_attn_fwd(q[r], k[r], v[r], 1, True, scale)
+        ones = A.flash_attn_bwd(do[r], q[r], k[r], v[r], one_o, one_lse, 1, True, scale)
+        assert torch.equal(o[r], one_o) and torch.equal(lse[b], one_lse[0])
+        for a, c in zip(grads, ones):
+            assert torch.equal(a[r], c)
