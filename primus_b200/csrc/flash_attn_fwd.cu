@@ -14,7 +14,7 @@
 // as two buffers, S of a tile's next block had to wait for its P.V and with it for the exponentials: 3485 clocks per pair of
 // 128 x 128 blocks, of which the GEMMs take 2048; now 2800, with the special-function unit busy for 2048.  A pair's start and
 // end (Q, tensor memory, output: 8000 clocks of 20250 for a window of 128) pass under its neighbours' blocks.
-// Before and now, us: 8192 x 32/8 x 128 483 -> 397 (1.40 PFLOP/s, under the power cap), 2048 x 32/8 x 128 43 -> 36,
+// Before and now, us: 8192 x 32/8 x 128 483 -> 405 (1.38 PFLOP/s, under the power cap), 2048 x 32/8 x 128 43 -> 36,
 // 4096 x 16 x 192/128 83 -> 75, window of 128 at 2 x 2048 x 64/8 x 64 79 -> 52.
 // O is rescaled in tensor memory only when the running max grew by more than 2^8.
 // V is consumed straight from its [kv, d] row-major tile through an MN-major descriptor, so no
@@ -395,7 +395,8 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
             pb::tc_fence_after();
           }
           const uint64_t neg_m = pb::pack_f32x2(-m_ref, -m_ref);
-          uint64_t l2[4] = {0, 0, 0, 0};
+          // (row sums as scalars: packed additions are 1.5 % faster and, in another order, differ in the last bit)
+          float l4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int c = 0; c < 4; ++c) {
             uint32_t pk[16];
@@ -406,14 +407,12 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
                                                             __uint_as_float(sr[c * 32 + 2 * i + 1])), scale2, neg_m), e0, e1);
               e0 = pb::fast_exp2(e0);
               e1 = pb::fast_exp2(e1);
-              l2[i & 3] = pb::add_f32x2(l2[i & 3], pb::pack_f32x2(e0, e1));
+              l4[i & 3] += e0 + e1;
               pk[i] = pb::pack_bf16x2(e0, e1);
             }
             pb::tmem_st_32x32b_x16(t_p + c * 16, pk);
           }
-          float la, lb;
-          pb::unpack_f32x2(pb::add_f32x2(pb::add_f32x2(l2[0], l2[1]), pb::add_f32x2(l2[2], l2[3])), la, lb);
-          l += la + lb;
+          l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
           pb::tmem_wait_st();
           pb::tc_fence_before();
           __syncwarp();
