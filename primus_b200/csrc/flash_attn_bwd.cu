@@ -461,17 +461,18 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 }
 
 // ------------------------------------------------------------------------------------------------
-// 128-wide steps, for d_qk == d_v (64, 128) and the dQ pass of (192, 128).  A tcgen05.mma with N = 64 occupies the tensor
-// pipe about as long as one with N = 128, so the 64-row steps above pay twice for S and dP; and there the two second GEMMs of a step run only after its
-// whole softmax.  Here a step streams 128 rows, and its work is cut so that the tensor pipe always has some of it:
+// 128-wide steps, for d_qk == d_v (64, 128) and the dQ pass of (192, 128).  A tcgen05.mma with N = 64 occupies the tensor pipe for
+// three quarters of the time of one with N = 128 (48 and 64 clocks), so the 64-row steps above pay half as much again for S and
+// dP; and there the two second GEMMs of a step run only after its whole softmax.  Here a step streams 128 rows, and its work is
+// cut so that the tensor pipe always has some of it:
 //   * the softmax threads take P = exp2(S) as soon as S is there, before dP;
 //   * dS and the second GEMMs go by column halves A (64 columns) and B: the GEMMs of half A run while half B is computed;
 //   * what frees a tensor-memory region is the *read* of it.  With two S buffers (64-wide heads) P and dS are packed into
 //     the step's S columns (8 + 8 of every 16) and the next dP starts as soon as this one is in registers; with one S
 //     buffer (128-wide) they are packed into the dP columns and the next S starts instead.
-// The two streamed tiles of a step have rings of their own, NS1 and NS2 buffers of 128 rows: the tile of S is wanted a whole step before the tile of dP, and the dQ pass is done with V after dP.  In the dQ pass
-// of 128-wide heads the resident tiles (Q, dO) move to tensor memory at the start, as A operands of the first GEMMs; their
-// shared memory belongs to the rings.
+// The two streamed tiles of a step have rings of their own, NS1 and NS2 buffers of 128 rows: the tile of S is wanted a whole step
+// before the tile of dP, and the dQ pass is done with V after dP.  In the dQ pass of 128-wide heads the resident tiles (Q, dO)
+// move to tensor memory at the start of a block, as A operands of the first GEMMs; their shared memory then stages the outputs.
 // A step of 128 x 128 x 128 holds four GEMMs of 512 clocks each in the dK / dV pass, three in the dQ pass; the passes take 2750
 // and 1960 clocks per step (3600 and 2600 with one ring of two or three buffers for both tiles: S waited for its tile).  8192 x
 // 32/8 x 128: dK / dV pass 924 -> 777 us; 4096 x 16 x 192/128: dQ pass 119 -> 101 us.
