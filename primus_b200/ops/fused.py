@@ -48,13 +48,12 @@ class RMSNormFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, eps, residual):
         H = x.shape[-1]
-        x2 = x.reshape(-1, H)
+        x2, r2 = norm_inputs(x, residual)
         rows = x2.shape[0]
-        y = torch.empty_like(x2)
+        y = torch.empty(rows, H, dtype=x.dtype, device=x.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         xsum = None
         if residual is not None:
-            r2 = residual.reshape(-1, H)
             xsum = torch.empty_like(x2)
             _lib.call("rmsnorm_fwd", x2, r2, w, y, xsum, rstd, rows, H, x2.stride(0), y.stride(0), float(eps))
             ctx.save_for_backward(xsum, w, rstd)
@@ -73,19 +72,9 @@ class RMSNormFn(torch.autograd.Function):
     def backward(ctx, dy, dxsum=None):
         xin, w, rstd = ctx.saved_tensors
         H = xin.shape[-1]
-        rows = xin.shape[0]
-        dy2 = dy.reshape(-1, H)
-        if not dy2.is_contiguous():
-            dy2 = dy2.contiguous()
-        dres = None
-        if dxsum is not None:
-            dres = dxsum.reshape(-1, H)
-            if not dres.is_contiguous():
-                dres = dres.contiguous()
-        dx = torch.empty_like(xin)
-        P = _lib.call_ret("rmsnorm_bwd_num_partials", rows)
-        sc = scratch(xin.device, "rmsnorm_dw", P * H)
-        dx, dx2, dw = norm_backward(dy2, xin, w, rstd, dres, dx, sc, getattr(ctx.w_ref, "main_grad", None), ctx.two)
+        dres = None if dxsum is None else dense_rows(dxsum.reshape(-1, H))
+        dx, dx2, dw = norm_backward(dense_rows(dy.reshape(-1, H)), xin, w, rstd, dres, getattr(ctx.w_ref, "main_grad", None),
+                                    ctx.two)
         dx = dx.view(ctx.shape)
         if ctx.has_res:
             return dx, dw, None, dx2.view(ctx.shape)
@@ -99,9 +88,21 @@ def two_leaves(x, residual) -> bool:
             and residual.requires_grad)
 
 
-def norm_backward(dy, xin, w, rstd, dres, dx, sc, main_grad, two):
+def norm_inputs(x, residual):
+    """``x`` and ``residual`` as rows that the kernels can read.  A row pitch is passed for the input of a norm without residual;
+    with one, the kernel has a single pitch for both and for their sum."""
+    x2 = x.reshape(-1, x.shape[-1])
+    if residual is not None:
+        return dense_rows(x2), dense_rows(residual.reshape(-1, x.shape[-1]))
+    return (x2 if x2.stride(1) == 1 and x2.data_ptr() % 16 == 0 else dense_rows(x2)), None
+
+
+def norm_backward(dy, xin, w, rstd, dres, main_grad, two):
     """(dx, the residual's gradient, dw or None when it was added to ``main_grad``); dx is shared unless ``two``."""
+    xin = dense_rows(xin)                       # (the kernel has a single pitch for x, dres and dx)
     rows, H = xin.shape
+    dx = torch.empty_like(xin)
+    sc = scratch(xin.device, "rmsnorm_dw", _lib.call_ret("rmsnorm_bwd_num_partials", rows) * H)
     if main_grad is not None:
         target, mode = main_grad, 1
     elif w.dtype == torch.bfloat16:             # rounded by the kernel

@@ -29,12 +29,11 @@ class NormLinearFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, hidden, residual, norm_w, weight, eps, tp_group, sp):
         H = hidden.shape[-1]
-        x2 = hidden.reshape(-1, H)
+        x2, r2 = fused.norm_inputs(hidden, residual)
         rows = x2.shape[0]
-        y = torch.empty_like(x2)
+        y = torch.empty(rows, H, dtype=hidden.dtype, device=hidden.device)
         rstd = torch.empty(rows, dtype=torch.float32, device=hidden.device)
         if residual is not None:
-            r2 = residual.reshape(-1, H)
             xsum = torch.empty_like(x2)
             _lib.call("rmsnorm_fwd", x2, r2, norm_w, y, xsum, rstd, rows, H, x2.stride(0), y.stride(0), float(eps))
         else:
@@ -69,7 +68,7 @@ class NormLinearFn(torch.autograd.Function):
         if not dout2.is_contiguous():
             dout2 = dout2.contiguous()
         # recompute the normalised activations (not stored in forward)
-        y = torch.empty_like(xsum)
+        y = torch.empty(rows, H, dtype=xsum.dtype, device=xsum.device)
         _lib.call("rmsnorm_fwd", xsum, None, norm_w, y, None, None, rows, H, xsum.stride(0), y.stride(0),
                   float(ctx.eps))
         if sp:
@@ -85,15 +84,8 @@ class NormLinearFn(torch.autograd.Function):
             dy = gemm.gemm(dout2, weight, b_mn=True)
             if tp_group is not None:
                 torch.distributed.all_reduce(dy, group=tp_group)
-        dres = None
-        if dxsum is not None:
-            dres = dxsum.reshape(rows, H)
-            if not dres.is_contiguous():
-                dres = dres.contiguous()
-        dx = torch.empty_like(xsum)
-        P = _lib.call_ret("rmsnorm_bwd_num_partials", rows)
-        sc = fused.scratch(xsum.device, "rmsnorm_dw", P * H)
-        dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, dx, sc, getattr(norm_w_ref, "main_grad", None), ctx.two)
+        dres = None if dxsum is None else fused.dense_rows(dxsum.reshape(rows, H))
+        dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None), ctx.two)
         dx, dx2 = dx.view(ctx.shape), dx2.view(ctx.shape)
         return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
 

@@ -238,6 +238,85 @@ def test_gradient_of_packed_heads_is_read_from_an_aligned_start(off, rows):
     assert torch.equal(got, wide[:, 8:72]) and got.is_contiguous() and got.data_ptr() % 16 == 0
 
 
+def _norm_launchers(monkeypatch):
+    """The norm kernels' launchers in plain PyTorch: every tensor is read and written by the row pitch that the launcher gets, from
+    its own start; a pitch that leaves the tensor's memory raises, as does a start that 16-byte accesses cannot have."""
+    def at(t, rows, H, pitch):
+        assert t.data_ptr() % 16 == 0 and pitch % 8 == 0
+        return torch.as_strided(t, (rows, H), (pitch, 1))
+
+    def fwd(x, res, w, y, xsum, rstd, rows, H, ldx, ldy, eps):
+        v = at(x, rows, H, ldx)
+        if res is not None:
+            v = at(xsum, rows, H, ldx).copy_(v.float() + at(res, rows, H, ldx).float())
+        r = torch.rsqrt(v.float().pow(2).mean(1) + eps)
+        rstd.copy_(r)
+        at(y, rows, H, ldy).copy_(v.float() * r[:, None] * w.float())
+
+    def bwd(dy, x, w, rstd, dres, dx, dx2, dw, rows, H, ldx, lddy):
+        g, v, r = at(dy, rows, H, lddy).float(), at(x, rows, H, ldx).float(), rstd[:, None]
+        d = r * g * w.float() - v * r ** 3 * (g * w.float() * v).mean(1, keepdim=True)
+        if dres is not None:
+            d = d + at(dres, rows, H, ldx).float()
+        for out in (dx, dx2):
+            if out is not None:
+                at(out, rows, H, ldx).copy_(d)
+        dw.copy_((g * v * r).sum(0))
+
+    def call(name, *a):
+        if name == "rmsnorm_fwd":
+            fwd(*a)
+        elif name == "rmsnorm_bwd_two":
+            bwd(*a[:8], *a[9:13])
+        else:
+            assert name == "rmsnorm_bwd"
+            bwd(*a[:6], None, a[6], *a[8:12])
+
+    monkeypatch.setattr(_lib, "call", call)
+    monkeypatch.setattr(_lib, "call_ret", lambda name, rows: min(rows, 296))
+
+
+@pytest.mark.parametrize("residual", [None, "dense", "same pitch", "other pitch"])
+@pytest.mark.parametrize("where", ["columns", "rows", "every other row", "odd start", "one row for all"])
+def test_norm_of_rows_with_a_pitch(monkeypatch, where, residual):
+    """Inputs that are views: outputs and gradients are those of dense copies, and nothing outside the tensors is touched."""
+    _norm_launchers(monkeypatch)
+    g = torch.Generator().manual_seed(3)
+    rows, H, W = 5, 16, 48
+
+    def view(base):
+        return {"columns": base[:rows, 8:8 + H], "rows": base.reshape(-1)[H:H + rows * H].view(rows, H),
+                "every other row": base.reshape(-1, H)[:2 * rows:2], "odd start": base.reshape(-1)[4:4 + rows * H].view(rows, H),
+                "one row for all": base[:1, :H].expand(rows, H)}[where]
+
+    def wide():
+        return torch.randn(rows, W, generator=g).bfloat16()
+
+    x = view(wide())
+    r = {None: None, "dense": torch.randn(rows, H, generator=g).bfloat16(), "same pitch": view(wide()),
+         "other pitch": torch.randn(rows, 3 * H, generator=g).bfloat16()[:, H:2 * H]}[residual]
+    dy, ds = (view(wide()) for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, generator=g)).bfloat16()
+
+    def run(*ts):
+        x, r, dy, ds = (None if t is None else t.detach() for t in ts)
+        p = torch.nn.Parameter(w.clone())
+        x.requires_grad_()
+        if r is None:
+            y = fused.RMSNormFn.apply(x, p, 1e-5, None)
+            y.backward(dy)
+            return [y.detach(), x.grad, p.grad]
+        r.requires_grad_()
+        y, s = fused.RMSNormFn.apply(x, p, 1e-5, r)
+        torch.autograd.backward([y, s], [dy, ds])
+        return [y.detach(), s.detach(), x.grad, r.grad, p.grad]
+
+    got = run(x, r, dy, ds)
+    want = run(*(None if t is None else t.contiguous().clone() for t in (x, r, dy, ds)))
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("sinks", [torch.zeros(2, dtype=torch.bfloat16), torch.zeros(3), torch.zeros(4)[::2]])
 def test_attention_backward_refuses_sinks_the_kernel_cannot_read(sinks, monkeypatch):
     """The gradient kernel reads one contiguous fp32 logit per head, as the forward checks: nothing is launched for others."""

@@ -51,3 +51,33 @@ def test_gradients_of_two_leaves_are_two_tensors(rows, H, layer):
     for t, u in zip(two, shared):
         assert torch.equal(t, u)
     assert torch.equal(two[0], two[1])
+
+
+@pytest.mark.parametrize("rows, H", [(3, 64), (129, 1024), (40, 4104)])
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("layer", [False, True])
+def test_gradients_of_a_column_slice(rows, H, residual, layer):
+    """Rows with a pitch: outputs and gradients are those of a dense copy."""
+    g = torch.Generator(device="cuda").manual_seed(H)
+    wide, other = (torch.randn(rows, H + 24, device="cuda", generator=g).bfloat16() for _ in range(2))
+    dy, ds = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    proj = (torch.randn(128, H, device="cuda", generator=g) * 0.02).bfloat16()
+
+    def run(copy):
+        a, b = (t[:, 8:8 + H] for t in (wide, other))
+        a, b = (t.clone() if copy else t.detach() for t in (a, b))
+        leaves = [a.requires_grad_()] + ([b.requires_grad_()] if residual else []) + [torch.nn.Parameter(w.clone())]
+        if layer:
+            y, s = layers.norm_linear(a, b if residual else None, leaves[-1], torch.nn.Parameter(proj.clone()), 1e-5)
+            torch.autograd.backward([y, s], [dy[:, :1].expand(rows, 128).contiguous(), ds])
+        elif residual:
+            y, s = fused.rmsnorm(a, leaves[-1], 1e-5, b)
+            torch.autograd.backward([y, s], [dy, ds])
+        else:
+            y = fused.rmsnorm(a, leaves[-1], 1e-5)
+            y.backward(dy)
+        return [y.detach()] + [t.grad for t in leaves]
+
+    for t, u in zip(run(False), run(True)):
+        assert torch.equal(t, u)
