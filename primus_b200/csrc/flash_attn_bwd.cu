@@ -1278,13 +1278,9 @@ int launch_bwd(const BwdArgs& a) {
   const BwOut out_q{(__nv_bfloat16*)a.dq, nullptr, a.dq_row, 0};
 #define PB_BWD(KERN, CFG, THREADS, GRID, CSIZE, OUT, X1, X2, Y1, Y2, O1, O2)                                                        \
   {                                                                                                                     \
-    static bool attr_set[3] = {false, false, false};                                                                    \
+    static std::atomic<bool> allowed[3][pbh::MAX_DEVICES];                                                              \
     auto kern = KERN;                                                                                                   \
-    if (!attr_set[var]) {                                                                                               \
-      cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, CFG::SMEM_BYTES);         \
-      if (e != cudaSuccess) return (int)e;                                                                              \
-      attr_set[var] = true;                                                                                             \
-    }                                                                                                                   \
+    if ((rc = pbh::allow_shared_memory(kern, CFG::SMEM_BYTES, allowed[var]))) return rc;                                \
     cudaLaunchConfig_t cfg = {};                                                                                        \
     cfg.gridDim = GRID;                                                                                                 \
     cfg.blockDim = dim3(THREADS);                                                                                       \

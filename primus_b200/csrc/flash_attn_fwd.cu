@@ -506,12 +506,8 @@ int launch_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
   if ((rc = pbh::make_tmap_3d(&to, o, bf, 2, T, hq, DV, DV, o_row, BQ, 1, 64, sw))) return rc;
   const bool win = window > 0 || sinks != nullptr || softcap > 0.f;
   auto kern = win ? flash_attn_fwd_kernel<DQK, DV, true> : flash_attn_fwd_kernel<DQK, DV, false>;
-  static bool attr_set[2] = {false, false};
-  if (!attr_set[win]) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set[win] = true;
-  }
+  static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];
+  if ((rc = pbh::allow_shared_memory(kern, C::SMEM_BYTES, allowed[win]))) return rc;
   dim3 grid(hq, batch, (seq / BQ + 1) / 2);
   kern<<<grid, FA_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, to, lse, seq, seq_k, q_off / BQ, hq, hkv,
                                                    scale * 1.4426950408889634f, causal, window, sinks, softcap, status);

@@ -302,12 +302,9 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
            int* status, int max_ctas, cudaStream_t stream) {
   using C = Cfg<BN>;
   auto kern = gemm_bf16_kernel<BN, A_MN, B_MN, OUT>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, C::SMEM_BYTES, allowed);
+  if (rc) return rc;
   if (g_num_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);

@@ -325,12 +325,9 @@ template <int A_MN, int B_MN, int OUT>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, int M, int N, int K, int* status,
            int max_ctas, cudaStream_t stream, int splits = 1) {
   auto kern = gemm_bf16_2cta_kernel<A_MN, B_MN, OUT>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, SMEM_BYTES, allowed);
+  if (rc) return rc;
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = SMEM_BYTES;

@@ -330,12 +330,9 @@ template <int A_MN, int B_MN, int OUT>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, const CUtensorMap& tSA,
            const CUtensorMap& tSB, int M, int N, int K, int* status, int max_ctas, cudaStream_t stream) {
   auto kern = gemm_mxfp8_2cta_kernel<A_MN, B_MN, OUT>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, SMEM_BYTES, allowed);
+  if (rc) return rc;
   if (g_num_sms == 0) {
     int dev = 0;
     cudaGetDevice(&dev);

@@ -332,12 +332,9 @@ template <int MODE, int OUT_ADD>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, int num_m, int num_n, int num_tiles,
            int K, const int* mblock_expert, const int* row_start, const int* padded, int* status, cudaStream_t s) {
   auto kern = grouped_gemm_kernel<MODE, OUT_ADD>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, SMEM_BYTES, allowed);
+  if (rc) return rc;
   static int num_sms = 0;
   if (!num_sms) {
     int dev = 0;

@@ -360,12 +360,9 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
 template <int MODE, int OUT_ADD>
 int launch(const CUtensorMap& tA, const CUtensorMap& tB, const Args& a, cudaStream_t s) {
   auto kern = grouped_gemm_mxfp8_kernel<MODE, OUT_ADD>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set = true;
-  }
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, SMEM_BYTES, allowed);
+  if (rc) return rc;
   static int num_sms = 0;
   if (!num_sms) {
     int dev = 0;

@@ -725,14 +725,10 @@ int pb_moe_fused(int gather, int b_mn, int ep, int rank, int epoch, int comm_cta
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  static bool attr_set[2] = {false, false};
+  static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];
   auto k0 = moe_fused_kernel<0>;
   auto k1 = moe_fused_kernel<1>;
-  if (!attr_set[b_mn ? 1 : 0]) {
-    cudaError_t e = cudaFuncSetAttribute(b_mn ? k1 : k0, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES);
-    if (e != cudaSuccess) return (int)e;
-    attr_set[b_mn ? 1 : 0] = true;
-  }
+  if ((rc = pbh::allow_shared_memory(b_mn ? k1 : k0, SMEM_BYTES, allowed[b_mn ? 1 : 0]))) return rc;
   if (comm_ctas > num_sms / 2) comm_ctas = a.comm_ctas = num_sms / 2;
   const int num_n = (N + BN - 1) / BN;
   int gemm_ctas = num_sms - comm_ctas;

@@ -215,16 +215,10 @@ int pb_router_fwd(const void* logits, int in_bf16, const float* bias, int T, int
   const int blocks = (T + WARPS - 1) / WARPS;
   const size_t smem = (size_t)WARPS * 2 * E * sizeof(float);
   if (smem > 48 * 1024) {
-    static bool set_b = false, set_f = false;
-    bool& flag = in_bf16 ? set_b : set_f;
-    if (!flag) {
-      cudaError_t e = in_bf16 ? cudaFuncSetAttribute(router_fwd_kernel<__nv_bfloat16>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024)
-                              : cudaFuncSetAttribute(router_fwd_kernel<float>,
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize, 64 * 1024);
-      if (e != cudaSuccess) return (int)e;
-      flag = true;
-    }
+    static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];
+    const int rc = in_bf16 ? pbh::allow_shared_memory(router_fwd_kernel<__nv_bfloat16>, 64 * 1024, allowed[0])
+                           : pbh::allow_shared_memory(router_fwd_kernel<float>, 64 * 1024, allowed[1]);
+    if (rc) return rc;
   }
   if (in_bf16)
     router_fwd_kernel<__nv_bfloat16><<<blocks, WARPS * 32, smem, s>>>(

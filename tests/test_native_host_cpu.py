@@ -175,6 +175,15 @@ int cudaLaunchKernel(const void* f, dim3_, dim3_, void**, size_t shared, void*) 
   if (fail_next > 0 && --fail_next == 0) error = 700;
   return error;
 }
+struct Config { dim3_ grid, block; size_t shared; void *stream, *attrs; unsigned num_attrs; };
+int cudaLaunchKernelExC(const Config* c, const void* f, void** args) {
+  return cudaLaunchKernel(f, c->grid, c->block, args, c->shared, c->stream);
+}
+int cudaFree(void*) { return 0; }
+int cudaDeviceGetAttribute(int* n, int, int) { *n = 148; return 0; }
+int cudaOccupancyMaxActiveClusters(int* n, const void*, const void*) { *n = 74; return 0; }
+static int encode() { return 0; }
+int cudaGetDriverEntryPoint(const char*, void** f, unsigned long long, int* status) { *f = (void*)encode; *status = 0; return 0; }
 }
 """
 
@@ -224,6 +233,50 @@ def test_norm_backward_stops_after_a_refused_launch(tmp_path, H, residual):
     """The weight gradient is not added up from partial sums that were never written."""
     codes, launches = _norm_backward(tmp_path, 1000, H, residual, "fail=1", "device=0", "device=0")
     assert codes == [700, 0] and len(launches) == 1 + (3 if H <= 256 and residual else 2)
+
+
+TENSOR_CORES = """
+import ctypes, sys
+fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)
+lib = ctypes.CDLL(sys.argv[2])
+p, n, f = ctypes.c_void_p(4096), ctypes.c_long, ctypes.c_float
+def attention(d_qk, d_v, window, cap):
+    sizes, q, k, v, o = (1, 256, 256, 0, 2, 2, d_qk, d_v), n(2 * d_qk), n(2 * d_qk), n(2 * d_v), n(2 * d_v)
+    tail = (f(0.125), 1, window)
+    return [lambda: lib.pb_flash_attn_fwd_cap(p, p, p, p, p, *sizes, q, k, v, o, *tail, None, f(cap), p, None),
+            lambda: lib.pb_flash_attn_bwd_cap(*[p] * 10, *sizes, q, k, v, o, o, q, k, v, *tail, f(cap), p, None)]
+calls = sum((attention(*d, w, c) for d in ((64, 64), (128, 128), (192, 128)) for w, c in ((0, 0.), (128, 0.), (0, 30.))), [])
+for a_mn, b_mn in ((0, 0), (0, 1), (1, 1)):
+    for out in (0, 1, 2):
+        t = (512, 512, 512, n(512), n(512), n(512), a_mn, b_mn, out)
+        calls += [lambda t=t: lib.pb_gemm_bf16(p, p, p, *t, 128, 0, p, None),
+                  lambda t=t: lib.pb_gemm_bf16(p, p, p, *t, 256, 0, p, None),
+                  lambda t=t: lib.pb_gemm_bf16_2cta(p, p, p, *t, 0, p, None),
+                  lambda t=t: lib.pb_gemm_mxfp8(p, p, p, p, p, *t, 128, 0, p, None),
+                  lambda t=t: lib.pb_gemm_mxfp8_2cta(p, p, p, p, p, *t, 0, p, None)]
+for mode in (0, 1, 2):
+    for e in (2, 256):
+        for add in (0, 1):
+            t = (mode, (256, 512, 512, e, p, p, p, add, p, None))
+            calls += [lambda t=t: lib.pb_grouped_gemm(t[0], p, p, p, *t[1]),
+                      lambda t=t: lib.pb_grouped_gemm_mxfp8(t[0], p, p, p, p, p, *t[1])]
+calls += [lambda b=b: lib.pb_router_fwd(p, b, None, 64, 1024, 4, 0, 0, 1, 1, f(1), p, p, p, None, None) for b in (0, 1)]
+first = [call() for call in calls]
+for device in (1, 0, 3):
+    fake.fake_device(device)
+    assert [call() for call in calls] == first, device
+print(len(calls), sum(rc == 0 for rc in first), sorted(set(first)))
+"""
+
+
+@pytest.mark.skipif(not _lib.available(), reason="the native library is not built")
+def test_tensor_core_launchers_on_several_devices(tmp_path):
+    """A kernel's shared-memory limit belongs to a device: what a launcher does on the first one it does on the others."""
+    fake = _compile(tmp_path, "runtime", RUNTIME, "-shared", "-fPIC")
+    out = subprocess.run([sys.executable, "-c", TENSOR_CORES, fake, _lib.lib_path()], capture_output=True, text=True)
+    assert out.returncode == 0, out.stderr
+    total, launched = map(int, out.stdout.split()[:2])
+    assert launched == total, out.stdout
 
 
 @pytest.mark.parametrize("off,rows", [(0, 4), (1, 4), (3, 1), (8, 2)])
