@@ -136,8 +136,8 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 
 // ------------------------------------------------------------------ backward
 // dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x)  (+ dres when given)
-// dx2 (optional) receives dx once more: gradients of two inputs that autograd would have to copy otherwise (it keeps one tensor
-// per leaf).  16384 x 8192: a second store 41 us, the copy 83 us.
+// dx2 (optional) receives dx once more: first gradients of two leaves, which autograd would have to copy otherwise (a layer used
+// by itself; inside a model the two inputs are no leaves).  16384 x 8192: a second store 41 us, the copy 83 us.
 // dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
 
 // Rows of up to 1024 channels: LPR <= 32 lanes per row, no barrier in the loop, RPG rows per group in flight.  The dw

@@ -61,7 +61,6 @@ class RMSNormFn(torch.autograd.Function):
             _lib.call("rmsnorm_fwd", x2, None, w, y, None, rstd, rows, H, x2.stride(0), y.stride(0), float(eps))
             ctx.save_for_backward(x2, w, rstd)
         ctx.has_res = residual is not None
-        ctx.two = two_leaves(x, residual)
         ctx.shape = x.shape
         ctx.w_ref = w
         if residual is not None:
@@ -74,18 +73,25 @@ class RMSNormFn(torch.autograd.Function):
         H = xin.shape[-1]
         dres = None if dxsum is None else dense_rows(dxsum.reshape(-1, H))
         dx, dx2, dw = norm_backward(dense_rows(dy.reshape(-1, H)), xin, w, rstd, dres, getattr(ctx.w_ref, "main_grad", None),
-                                    ctx.two)
+                                    dres is not None and two_leaves(ctx, 0, 2))
         dx = dx.view(ctx.shape)
         if ctx.has_res:
             return dx, dw, None, dx2.view(ctx.shape)
         return dx, dw, None, None
 
 
-def two_leaves(x, residual) -> bool:
-    """Whether the gradient that ``x`` and ``residual`` share has to exist twice: autograd keeps a tensor per leaf, and would
-    copy the shared one.  (Inside a model it goes on to two producers, which read it.)"""
-    return (residual is not None and residual is not x and x.is_leaf and residual.is_leaf and x.requires_grad
-            and residual.requires_grad)
+def two_leaves(node, i, j) -> bool:
+    """Whether inputs ``i`` and ``j`` of an autograd node are two leaves that both get their first gradient from this backward
+    pass.  A shared gradient would then be copied: autograd keeps a tensor per leaf.  It copies nothing where a leaf already
+    has a gradient (the new one is added to it), where ``torch.autograd.grad`` hands the gradient out, or inside a model, where
+    it goes on to two producers, which read it: there a second one would only cost its store."""
+    nodes = [node.next_functions[k][0] for k in (i, j)]
+    if nodes[0] is nodes[1] or not all(isinstance(n, torch._C._functions.AccumulateGrad) and n.variable.grad is None for n in nodes):
+        return False
+    try:
+        return all(torch._C._will_engine_execute_node(n) for n in nodes)
+    except RuntimeError:                        # (what it answers under torch.autograd.grad)
+        return False
 
 
 def norm_inputs(x, residual):
@@ -98,7 +104,8 @@ def norm_inputs(x, residual):
 
 
 def norm_backward(dy, xin, w, rstd, dres, main_grad, two):
-    """(dx, the residual's gradient, dw or None when it was added to ``main_grad``); dx is shared unless ``two``."""
+    """(dx, the residual's gradient, dw or None when it was added to ``main_grad``); dx is shared unless ``two``
+    (with ``dres`` only)."""
     xin = dense_rows(xin)                       # (the kernel has a single pitch for x, dres and dx)
     rows, H = xin.shape
     dx = torch.empty_like(xin)
@@ -110,7 +117,7 @@ def norm_backward(dy, xin, w, rstd, dres, main_grad, two):
     else:
         target, mode = torch.empty(H, dtype=torch.float32, device=xin.device), 0
     dx2 = dx
-    if two and dres is not None:
+    if two:
         dx2 = torch.empty_like(dx)
         _lib.call("rmsnorm_bwd_two", dy, xin, w, rstd, dres, dx, dx2, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
     else:

@@ -48,7 +48,6 @@ class NormLinearFn(torch.autograd.Function):
         ctx.tp = (tp_group, sp)
         ctx.set_materialize_grads(False)
         ctx.has_res = residual is not None
-        ctx.two = fused.two_leaves(hidden, residual)
         ctx.shape = hidden.shape
         ctx.refs = (norm_w, weight)
         if residual is not None:
@@ -85,7 +84,8 @@ class NormLinearFn(torch.autograd.Function):
             if tp_group is not None:
                 torch.distributed.all_reduce(dy, group=tp_group)
         dres = None if dxsum is None else fused.dense_rows(dxsum.reshape(rows, H))
-        dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None), ctx.two)
+        dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None),
+                                            dres is not None and fused.two_leaves(ctx, 0, 1))
         dx, dx2 = dx.view(ctx.shape), dx2.view(ctx.shape)
         return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
 

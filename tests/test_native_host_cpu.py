@@ -316,7 +316,10 @@ def _norm_launchers(monkeypatch):
                 at(out, rows, H, ldx).copy_(d)
         dw.copy_((g * v * r).sum(0))
 
+    names = []
+
     def call(name, *a):
+        names.append(name)
         if name == "rmsnorm_fwd":
             fwd(*a)
         elif name == "rmsnorm_bwd_two":
@@ -327,6 +330,7 @@ def _norm_launchers(monkeypatch):
 
     monkeypatch.setattr(_lib, "call", call)
     monkeypatch.setattr(_lib, "call_ret", lambda name, rows: min(rows, 296))
+    return names
 
 
 @pytest.mark.parametrize("residual", [None, "dense", "same pitch", "other pitch"])
@@ -368,6 +372,40 @@ def test_norm_of_rows_with_a_pitch(monkeypatch, where, residual):
     want = run(*(None if t is None else t.contiguous().clone() for t in (x, r, dy, ds)))
     for a, b in zip(got, want):
         assert torch.equal(a, b)
+
+
+def test_norm_gradient_is_written_twice_only_for_first_gradients_of_two_leaves(monkeypatch):
+    """Elsewhere nothing copies the gradient that hidden and residual share, and a second store would be pure cost."""
+    names = _norm_launchers(monkeypatch)
+    g = torch.Generator().manual_seed(4)
+    x, r, dy, ds = (torch.randn(3, 16, generator=g).bfloat16() for _ in range(4))
+    w = torch.nn.Parameter(torch.ones(16, dtype=torch.bfloat16))
+    x.requires_grad_(), r.requires_grad_()
+
+    def last(step, a=x, b=r):
+        out = fused.RMSNormFn.apply(a, w, 1e-5, b)
+        got = step(out)
+        return names[-1], got
+
+    def backward(out):
+        torch.autograd.backward(out, [dy, ds])
+
+    assert last(backward)[0] == "rmsnorm_bwd_two"
+    first = x.grad.clone()
+    assert torch.equal(x.grad, r.grad) and x.grad.data_ptr() != r.grad.data_ptr()
+    assert last(backward)[0] == "rmsnorm_bwd"
+    assert torch.equal(x.grad, 2 * first) and torch.equal(r.grad, 2 * first)
+    for only in (x, r):                       # one of the two has a gradient
+        x.grad, r.grad = None, None
+        only.grad = torch.zeros_like(x)
+        assert last(backward)[0] == "rmsnorm_bwd"
+        assert torch.equal(x.grad, first) and torch.equal(r.grad, first) and x.grad.data_ptr() != r.grad.data_ptr()
+    x.grad = r.grad = None
+    name, got = last(lambda out: torch.autograd.grad(out, [x, r], [dy, ds]))
+    assert name == "rmsnorm_bwd" and torch.equal(got[0], first) and torch.equal(got[1], first)
+    assert last(backward, x * 1)[0] == "rmsnorm_bwd" and torch.equal(x.grad, first) and torch.equal(r.grad, first)
+    x.grad = r.grad = None
+    assert last(backward, x, x)[0] == "rmsnorm_bwd"
 
 
 @pytest.mark.parametrize("sinks", [torch.zeros(2, dtype=torch.bfloat16), torch.zeros(3), torch.zeros(4)[::2]])
