@@ -565,12 +565,17 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
 
 int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
                 float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
-  // every one of the partial rows is fully written by its CTA before the reduction reads it
-  P = bwd_ctas(P, rows, H);
-  const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
-                                    (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, rows, H,
-                                    ldx, lddy);
-  if (rc) return rc;
+  if (rows == 0) {                                   // nothing to add; a stored sum of no rows is zero
+    if (H == 0 || dw_accumulate == 1) return 0;
+    P = 0;
+  } else {
+    // every one of the partial rows is fully written by its CTA before the reduction reads it
+    P = bwd_ctas(P, rows, H);
+    const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
+                                      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, rows, H,
+                                      ldx, lddy);
+    if (rc) return rc;
+  }
   rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, H, dw_accumulate);
   return (int)cudaGetLastError();
 }
@@ -596,7 +601,6 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
                    void* dx, float* dw, float* scratch, long rows, int H, long ldx, long lddy,
                    int dw_accumulate, cudaStream_t s) {
   if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L) return -2;
-  if (rows == 0) return 0;
   return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, nullptr, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
@@ -605,7 +609,6 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
 int pb_rmsnorm_bwd_two(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
                        float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
   if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || !dres) return -2;
-  if (rows == 0) return 0;
   return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
@@ -675,7 +678,7 @@ extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void*
   // more than INT_MAX rows are outside the interface, as they are for pb_rmsnorm_bwd
   if (H <= 0 || H % 8 || ldx % 8 || lddy % 8 || rows < 0 || rows > 2147483647L) return PB_NOALLOC_ERR_BAD_ARG;
   if (H > PB_NOALLOC_MAX_H) return PB_NOALLOC_ERR_TOO_LARGE;  // the built-in scratch holds rows of <= 8192 floats
-  if (rows == 0) return 0;
+  if (rows == 0 && dw_accumulate) return 0;
   int dev = -1;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return (int)e;

@@ -235,6 +235,27 @@ def test_norm_backward_stops_after_a_refused_launch(tmp_path, H, residual):
     assert codes == [700, 0] and len(launches) == 1 + (3 if H <= 256 and residual else 2)
 
 
+NO_ROWS = """
+import ctypes, sys
+fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)
+lib = ctypes.CDLL(sys.argv[2])
+fake.fake_log.restype = ctypes.c_char_p
+p, n = ctypes.c_void_p(4096), ctypes.c_long
+for mode in (0, 2, 1):
+    for H in (64, 4096):
+        print(lib.pb_rmsnorm_bwd(p, p, p, p, p, p, p, p, n(0), H, n(H), n(H), mode, None),
+              lib.pb_rmsnorm_bwd_two(p, p, p, p, p, p, p, p, p, n(0), H, n(H), n(H), mode, None), fake.fake_log().count(b"device"))
+"""
+
+
+@pytest.mark.skipif(not _lib.available(), reason="the native library is not built")
+def test_norm_backward_of_no_rows_stores_the_gain_gradient(tmp_path):
+    """Stored (fp32 or bf16): the reduction alone runs, and writes zeros.  Added: nothing runs."""
+    fake = _compile(tmp_path, "runtime", RUNTIME, "-shared", "-fPIC")
+    out = subprocess.run([sys.executable, "-c", NO_ROWS, fake, _lib.lib_path()], capture_output=True, text=True, check=True).stdout
+    assert out.split("\n")[:-1] == [f"0 0 {launches}" for launches in (2, 4, 6, 8, 8, 8)]
+
+
 TENSOR_CORES = """
 import ctypes, sys
 fake = ctypes.CDLL(sys.argv[1], mode=ctypes.RTLD_GLOBAL)

@@ -81,3 +81,15 @@ def test_gradients_of_a_column_slice(rows, H, residual, layer):
 
     for t, u in zip(run(False), run(True)):
         assert torch.equal(t, u)
+
+
+@pytest.mark.parametrize("H", [64, 4096])
+def test_gain_gradient_of_no_rows_is_zero(H):
+    for _ in range(4):
+        junk = [torch.full((H,), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(8)]
+        del junk                                # what the gradient's memory held before
+        x, r = (torch.empty(0, H, device="cuda", dtype=torch.bfloat16).requires_grad_() for _ in range(2))
+        p = torch.nn.Parameter(torch.ones(H, device="cuda", dtype=torch.bfloat16))
+        y, s = fused.rmsnorm(x, p, 1e-5, r)
+        torch.autograd.backward([y, s], [torch.ones_like(y), torch.ones_like(s)])
+        assert p.grad.shape == (H,) and not p.grad.any() and x.grad.shape == (0, H)
