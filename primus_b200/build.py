@@ -2,8 +2,9 @@
 
 All device code targets sm_100a only (``-gencode arch=compute_100a,code=sm_100a``); nvcc
 cross-compiles it on hosts without a GPU.  The library exposes plain ``extern "C"`` launchers
-(raw pointers + a CUDA stream) that :mod:`primus_b200.ops._lib` binds with ctypes, so no torch
-headers are needed and a full rebuild takes seconds.
+(raw pointers + a CUDA stream) that :mod:`primus_b200.ops._lib` calls through a small CPython module
+(``csrc/python/launch.c``, compiled with gcc; ctypes without it), so no torch headers are needed and a
+full rebuild takes seconds.
 
 Run ``python -m primus_b200.build`` (add ``--force`` to rebuild everything, ``--verbose`` to see
 ptxas resource usage).
@@ -98,17 +99,24 @@ def build(force: bool = False, verbose: bool = False) -> Path:
 
 
 def _build_launch(force: bool) -> None:
-    """The launchers' binding; without Python's headers, or on another architecture, calls go through ctypes."""
+    """The launchers' binding.  Where it cannot be built (another architecture, no headers of Python, no gcc), calls go through
+    ctypes; a binding of an older source does not stay behind."""
     include = Path(sysconfig.get_paths()["include"])
-    if platform.machine() != "x86_64" or not (include / "Python.h").exists():
-        print("Python headers for x86-64 not found: launchers are called through ctypes", file=sys.stderr)
-        return
     if not force and not _needs_build(LAUNCH_SRC, LAUNCH_PATH, []):
         return
-    cmd = ["gcc", "-O2", "-shared", "-fPIC", "-I", str(include), str(LAUNCH_SRC), "-o", str(LAUNCH_PATH)]
-    p = subprocess.run(cmd, capture_output=True, text=True)
-    if p.returncode != 0:
-        raise RuntimeError(f"binding failed:\n{p.stdout}{p.stderr}")
+    if platform.machine() != "x86_64" or not (include / "Python.h").exists():
+        why = "Python headers for x86-64 not found"
+    else:
+        cmd = ["gcc", "-O2", "-shared", "-fPIC", "-I", str(include), str(LAUNCH_SRC), "-o", str(LAUNCH_PATH)]
+        try:
+            p = subprocess.run(cmd, capture_output=True, text=True)
+            if p.returncode == 0:
+                return
+            why = f"the compiled binding could not be built:\n{p.stdout}{p.stderr}"
+        except OSError as e:
+            why = f"the compiled binding could not be built ({e})"
+    LAUNCH_PATH.unlink(missing_ok=True)
+    print(f"{why}\nlaunchers are called through ctypes", file=sys.stderr)
 
 
 def main() -> None:

@@ -1,4 +1,5 @@
-"""ctypes binding of ``libprimus_b200.so`` (the sm_100a kernels under ``primus_b200/csrc``).
+"""Python binding of ``libprimus_b200.so`` (the sm_100a kernels under ``primus_b200/csrc``): the launchers are called through a
+compiled module (``csrc/python/launch.c``), or through ctypes where that is not built or does not load.
 
 The library exports ``extern "C"`` launchers that take raw device pointers and a CUDA stream.
 ``call(name, *args)`` converts torch tensors to pointers, appends nothing implicitly, and raises
@@ -13,6 +14,7 @@ import importlib.util
 import os
 import sysconfig
 import threading
+import warnings
 from pathlib import Path
 
 import torch
@@ -79,10 +81,14 @@ def _load_launch():
     path = LIB_PATH.parent / ("_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
     if not path.exists():
         return None
-    loader = importlib.machinery.ExtensionFileLoader("_launch", str(path))
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_launch", loader))
-    loader.exec_module(module)
-    module.init(torch.Tensor)
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_launch", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_launch", loader))
+        loader.exec_module(module)
+        module.init(torch.Tensor)
+    except ImportError as e:
+        warnings.warn(f"{path} does not load ({e}): launchers are called through ctypes")
+        return None
     return module
 
 

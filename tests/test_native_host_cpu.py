@@ -8,6 +8,7 @@ from pathlib import Path
 import pytest
 import torch
 
+from primus_b200 import build
 from primus_b200.ops import _lib, attention, fused
 
 ROOT = Path(__file__).resolve().parent.parent
@@ -149,6 +150,28 @@ def test_launcher_arguments_keep_their_places(compiled, tmp_path, monkeypatch):
     _lib.call("nine", *[1.0] * 8, 2.0, -5)
     with pytest.raises(ctypes.ArgumentError):
         _lib.call("nine", *[1.0] * 8, object(), -5)
+
+
+def test_binding_that_does_not_load_leaves_ctypes(tmp_path, monkeypatch):
+    monkeypatch.setattr(_lib, "LIB_PATH", tmp_path / "library.so")
+    assert _lib._load_launch() is None                                            # not built
+    (tmp_path / build.LAUNCH_PATH.name).write_bytes(b"cut off")
+    with pytest.warns(UserWarning, match="through ctypes"):
+        assert _lib._load_launch() is None
+
+
+@pytest.mark.parametrize("gcc", ["missing", "failing"])
+def test_build_without_a_working_gcc_leaves_ctypes(gcc, tmp_path, monkeypatch, capsys):
+    """The build goes on, and a binding of an older source is not left behind."""
+    stale = tmp_path / "binding.so"
+    stale.write_bytes(b"")
+    monkeypatch.setattr(build, "LAUNCH_PATH", stale)
+    monkeypatch.setenv("PATH", str(tmp_path))
+    if gcc == "failing":
+        (tmp_path / "gcc").write_text("#!/bin/sh\nexit 1\n")
+        (tmp_path / "gcc").chmod(0o755)
+    build._build_launch(force=True)
+    assert not stale.exists() and "through ctypes" in capsys.readouterr().err
 
 
 # Stands in for the CUDA runtime: launches are recorded as "device <d> shared <bytes>", and refused where a kernel asks for more
