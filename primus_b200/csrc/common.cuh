@@ -260,15 +260,6 @@ PB_DEVICE void umma_commit_2cta(uint64_t* bar, uint16_t mask) {
       "h"(mask)
       : "memory");
 }
-// D(tmem, both CTAs) (+)= A . B over a CTA pair: M = 256 (128 rows per CTA), operands at the same shared-memory offsets
-PB_DEVICE void umma_f16_ss_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
 // fp8 block-scaled MMA over a CTA pair: M = 256 (128 rows per CTA), operands at the same shared / tensor memory
 // offsets in both CTAs; issued by one thread of the even CTA.
 PB_DEVICE void umma_mxf8_ss_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,

@@ -54,6 +54,17 @@ struct Barriers {
   int abort_flag;
 };
 
+// D(tmem, both CTAs) (+)= A . B over a CTA pair: M = 256 (128 rows per CTA), operands at the same shared-memory offsets
+__device__ __forceinline__ void umma_f16_ss_2cta(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
 __device__ __forceinline__ bool wait_or_abort(uint64_t* bar, uint32_t parity, volatile int* abort_flag) {
   if (pb::mbar_try_wait(bar, parity)) return true;
   const long long t0 = clock64();
@@ -215,7 +226,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
                                      : pb::make_smem_desc(sa + k * (UMMA_K * 2), 0, 1024, 2);
             const uint64_t db = B_MN ? pb::make_smem_desc(sb + k * (UMMA_K * 128), BK * 128, 1024, 2)
                                      : pb::make_smem_desc(sb + k * (UMMA_K * 2), 0, 1024, 2);
-            pb::umma_f16_ss_2cta(d_tmem, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
+            umma_f16_ss_2cta(d_tmem, da, db, idesc, (kb > kb0 || k > 0) ? 1u : 0u);
           }
           pb::umma_commit_2cta(&bars->empty[stage], 3);
           if (++stage == STAGES) {

@@ -15,10 +15,6 @@
 // (primus/backends/megatron/core/extensions/primus_turbo.py:2103-2218).
 #include "common.cuh"
 
-// csrc/grouped_wgrad_2cta.cu
-int pb_grouped_wgrad_pair(const void* dy, const void* x, void* D, int rows_cap, int N, int K, int E, const int* row_start,
-                          const int* padded, int* status, cudaStream_t s);
-
 namespace {
 
 constexpr int BM = 128;
@@ -401,12 +397,10 @@ int pb_grouped_gemm(int mode, const void* A, const void* B, void* D, int rows_ca
                     const int* mblock_expert, const int* row_start, const int* padded, int accumulate, int* status,
                     cudaStream_t s) {
   if (rows_cap % BM || N % 8 || K % 8) return -2;
-  // Gradients added to more fp32 values than L2 holds stream them through memory, and CTA pairs keep up with that; adding to
-  // fewer in L2 does as well.  Both GEMMs of the experts, one CTA / pairs, us: 64 experts of 2048 x 768 (302 M values) with 512, 128
-  // and 2 rows each 511 / 461, 476 / 414, 475 / 372; 8 such experts (38 M) 94 / 95; 32 of 2048 x 192 (38 M) 96 / 105; 16 of
-  // 1024 x 512 (25 M) 50 / 53.
-  if (mode == G_WGRAD && accumulate && (long)E * N * K >= (48L << 20))
-    return pb_grouped_wgrad_pair(A, B, D, rows_cap, N, K, E, row_start, padded, status, s);
+  // Added gradients are reduced in L2, so that launches on several streams may add to the same ones.  Fetching the old values ahead,
+  // adding in registers and storing is faster where an expert has few rows (64 experts of 2048 x 768, both GEMMs, 128 rows each:
+  // 505 -> 425 us; 512 rows 528 -> 565 in a short run, 545 -> 512 under the power cap; 16 experts of 512 rows 141 -> 137), but two
+  // such launches lose each other's sums.
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
   CUtensorMap tA, tB, tD;
