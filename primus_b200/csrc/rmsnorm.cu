@@ -608,7 +608,7 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
 // dx is written twice, to dx and to dx2 (with dres only).
 int pb_rmsnorm_bwd_two(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
                        float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
-  if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || !dres) return -2;
+  if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || (rows && !dres)) return -2;
   return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
