@@ -212,26 +212,86 @@ def test_flash_attn_softcapped_scores(case):
         assert err <= tol, f"{name}: err {err} tol {tol}"
 
 
-def _clusters(batch, seq, hq, hkv, dqk, dv, causal, window):
+def _clusters(batch, seq, hq, hkv, dqk, dv, causal, window, q_off=0):
+    """CTAs per block of the dK / dV and of the dQ pass."""
     lib = _lib.require()
-    return [lib.pb_flash_attn_bwd_cluster(p, batch, seq, seq, 0, hq, hkv, dqk, dv, int(causal), window) for p in (0, 1)]
+    seq_k = seq + q_off
+    return [lib.pb_flash_attn_bwd_cluster(p, batch, seq, seq_k, q_off, hq, hkv, dqk, dv, int(causal), window) for p in (0, 1)]
 
 
-@pytest.mark.parametrize("case, clusters", [
-    # batch, seq, hq, hkv, dqk, dv, causal, window; CTAs per block of the dK / dV and the dQ pass
-    ((1, 128, 1, 1, 128, 128, True, 0), (1, 1)),            # one step: nothing to share
-    ((1, 640, 3, 1, 64, 64, True, 0), (2, 1)),              # step counts that the ranks cannot share evenly
-    ((1, 2048, 8, 1, 128, 128, True, 0), (8, 1)),
-    ((1, 4096, 2, 1, 128, 128, False, 0), (4, 2)),
-    ((2, 1152, 2, 2, 192, 128, True, 0), (2, 2)),
-    ((1, 2048, 1, 1, 192, 128, True, 0), (4, 4)),
-    ((1, 2048, 4, 1, 64, 64, True, 1000), (4, 1)),
+def _grads_and_reference(q, k, v, batch, causal, q_off=0, window=0, softcap=0.0, sinks=None):
+    """Outputs and gradients of the kernels (twice, equal) against the fp32 reference, in the 2-norm: P, dS and the results are
+    bf16, 2^-9 each; 3e-3 measured.  A log-sum-exp is fp32: 1e-3, and the 2^-11 that tanh.approx has of a capped score."""
+    scale = 1.0 / math.sqrt(q.shape[2])
+    o, lse = A.flash_attn_fwd(q, k, v, batch, causal, scale, q_off, window, sinks, softcap)
+    do = torch.randn_like(o)
+    grads = A.flash_attn_bwd(do, q, k, v, o, lse, batch, causal, scale, q_off=q_off, window=window, softcap=softcap, sinks=sinks)
+    o2, lse2 = A.flash_attn_fwd(q, k, v, batch, causal, scale, q_off, window, sinks, softcap)
+    again = A.flash_attn_bwd(do, q, k, v, o, lse, batch, causal, scale, q_off=q_off, window=window, softcap=softcap, sinks=sinks)
+    torch.cuda.synchronize()
+    _lib.check_status()
+    leaves = [t.detach().float().requires_grad_() for t in (q, k, v)]
+    sinks_ref = None if sinks is None else sinks.clone().requires_grad_()
+    o_ref, lse_ref = A.attention_ref(*leaves, batch, causal, None, q_off, window, sinks_ref, softcap)
+    o_ref.backward(do.float())
+    assert torch.equal(o, o2) and torch.equal(lse, lse2)
+    assert (lse - lse_ref).abs().max().item() <= 1e-3 + softcap * 2.0 ** -11
+    refs = [o_ref.detach()] + [t.grad for t in leaves] + ([] if sinks is None else [sinks_ref.grad])
+    for name, a, b, r in zip(("o", "dq", "dk", "dv", "dsinks")[:len(refs)], (o, *grads), (o, *again), refs, strict=True):
+        assert torch.equal(a, b), name
+        rel = (a.float() - r).norm().item() / r.norm().item()
+        assert rel <= 1e-2, f"{name}: relative error {rel}"
+
+
+@pytest.mark.parametrize("window, softcap, sinks, causal, q_off", [
+    (0, 0.0, False, True, 0), (0, 0.0, False, False, 0), (0, 0.0, True, True, 384), (200, 0.0, True, True, 0),
+    (128, 0.0, False, True, 0), (0, 2.0, False, True, 0), (200, 2.0, True, True, 0), (0, 2.0, False, False, 0),
 ])
-def test_flash_attn_backward_of_shared_blocks(case, clusters):
+@pytest.mark.parametrize("batch, hq, hkv, dqk, dv", [(8, 32, 16, 64, 64), (8, 32, 16, 128, 128), (16, 16, 16, 192, 128)])
+def test_flash_attn_of_more_blocks_than_sms(batch, hq, hkv, dqk, dv, window, softcap, sinks, causal, q_off):
+    """Every CTA takes several blocks, one after the other: five row blocks of 128 per head (in the forward two pairs and one tile
+    alone), blocks of one to eight steps."""
+    seq = 640
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert batch * hq * 3 >= 4 * sms and batch * hkv * 5 >= 4 * sms
+    assert _clusters(batch, seq, hq, hkv, dqk, dv, causal, window, q_off) == [1, 1]
+    q, _, _ = _inputs(batch, seq, hq, hkv, dqk, dv, seed=21)
+    _, k, v = _inputs(batch, seq + q_off, hq, hkv, dqk, dv, seed=22)
+    logits = torch.linspace(-2, 2, hq, device="cuda") if sinks else None
+    _grads_and_reference(q, k, v, batch, causal, q_off, window, softcap, logits)
+
+
+@pytest.mark.parametrize("batch, seq, hq, hkv, dqk, dv, causal, window, q_off, softcap", [
+    (1, 1024, 8, 1, 128, 128, True, 0, 3072, 0.0),          # a chunk of a longer sequence
+    (1, 1024, 8, 1, 64, 64, True, 0, 3072, 2.0),
+    (1, 512, 2, 2, 192, 128, True, 0, 3584, 0.0),
+    (1, 2048, 8, 1, 128, 128, True, 0, 0, 2.0),
+    (1, 4096, 2, 1, 64, 64, False, 0, 0, 2.0),
+    (1, 2048, 1, 1, 192, 128, True, 0, 0, 2.0),
+    (1, 2048, 4, 1, 128, 128, True, 1000, 0, 2.0),
+])
+def test_flash_attn_shared_blocks_of_chunks_and_capped_scores(batch, seq, hq, hkv, dqk, dv, causal, window, q_off, softcap):
+    assert max(_clusters(batch, seq, hq, hkv, dqk, dv, causal, window, q_off)) > 1
+    q, _, _ = _inputs(batch, seq, hq, hkv, dqk, dv, seed=23)
+    _, k, v = _inputs(batch, seq + q_off, hq, hkv, dqk, dv, seed=24)
+    _grads_and_reference(q, k, v, batch, causal, q_off, window, softcap)
+
+
+@pytest.mark.parametrize("case, shared", [
+    # batch, seq, hq, hkv, dqk, dv, causal, window; whether CTAs share the blocks of the dK / dV and of the dQ pass
+    ((1, 128, 1, 1, 128, 128, True, 0), (False, False)),    # one step: nothing to share
+    ((1, 640, 3, 1, 64, 64, True, 0), (True, False)),       # step counts that the ranks cannot share evenly
+    ((1, 2048, 8, 1, 128, 128, True, 0), (True, False)),
+    ((1, 4096, 2, 1, 128, 128, False, 0), (True, True)),
+    ((2, 1152, 2, 2, 192, 128, True, 0), (True, True)),
+    ((1, 2048, 1, 1, 192, 128, True, 0), (True, True)),
+    ((1, 2048, 4, 1, 64, 64, True, 1000), (True, False)),
+])
+def test_flash_attn_backward_of_shared_blocks(case, shared):
     """Blocks whose steps several CTAs share: gradients against the fp32 reference, equal from call to call, and into strided
     views of a packed gradient."""
     batch, seq, hq, hkv, dqk, dv, causal, window = case
-    assert tuple(_clusters(*case)) == clusters
+    assert tuple(c > 1 for c in _clusters(*case)) == shared
     q, k, v = _inputs(batch, seq, hq, hkv, dqk, dv, seed=5)
     scale = 1.0 / math.sqrt(dqk)
     o, lse = A.flash_attn_fwd(q, k, v, batch, causal, scale, window=window)
