@@ -1256,16 +1256,14 @@ int launch_bwd(const BwdArgs& a) {
       (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.neg_lse2, a.seq,
       a.hq, a.o_row, a.do_row);
   int rc;
-  CUtensorMap q128, do128, k128, v128, q64, do64, dq_m, dk_m, dv_m;
+  CUtensorMap q128, do128, k128, v128, dq_m, dk_m, dv_m;
   const long TK = (long)a.batch * a.seq_k;
 #define MK(m, p, rows, heads, d, row, br) \
   if ((rc = pbh::make_tmap_3d(&m, p, bf, 2, rows, heads, d, d, row, br, 1, 64, sw))) return rc;
   MK(q128, a.q, T, a.hq, DQK, a.q_row, 128) MK(do128, a.d_o, T, a.hq, DV, a.do_row, 128)
   MK(k128, a.k, TK, a.hkv, DQK, a.k_row, 128) MK(v128, a.v, TK, a.hkv, DV, a.v_row, 128)
-  MK(q64, a.q, T, a.hq, DQK, a.q_row, 64) MK(do64, a.d_o, T, a.hq, DV, a.do_row, 64)
   MK(dq_m, a.dq, T, a.hq, DQK, a.dq_row, 128) MK(dk_m, a.dk, TK, a.hkv, DQK, a.dk_row, 128)
   MK(dv_m, a.dv, TK, a.hkv, DV, a.dv_row, 128)
-#undef MK
   const int var = a.softcap > 0.f ? 2 : (a.window > 0 ? 1 : 0);
   const float* lse2 = a.neg_lse2;
   auto cluster = [&](int mode) {
@@ -1302,6 +1300,8 @@ int launch_bwd(const BwdArgs& a) {
             : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DKDV, 0>),
            CKV, BWW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q128, do128, dk_m, dv_m)
   } else {
+    CUtensorMap q64, do64;                     // (streamed by 64 rows)
+    MK(q64, a.q, T, a.hq, DQK, a.q_row, 64) MK(do64, a.d_o, T, a.hq, DV, a.do_row, 64)
     using CKV = BwCfg<DQK, DV>;
     PB_BWD((var ? flash_attn_bwd_kernel<DQK, DV, true> : flash_attn_bwd_kernel<DQK, DV, false>), CKV,
            BW_THREADS, grid_kv, c_kv, out_kv, k128, v128, q64, do64, dk_m, dv_m)
@@ -1311,6 +1311,7 @@ int launch_bwd(const BwdArgs& a) {
           : var == 1 ? flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 1> : flash_attn_bwd_wide_kernel<DQK, DV, MODE_DQ, 0>),
          CQ, BWW_THREADS, grid_q, c_q, out_q, q128, do128, k128, v128, dq_m, dq_m)
 #undef PB_BWD
+#undef MK
   return (int)cudaGetLastError();
 }
 
