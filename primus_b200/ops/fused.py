@@ -73,11 +73,8 @@ class RMSNormFn(torch.autograd.Function):
         H = xin.shape[-1]
         dres = None if dxsum is None else dense_rows(dxsum.reshape(-1, H))
         dx, dx2, dw = norm_backward(dense_rows(dy.reshape(-1, H)), xin, w, rstd, dres, getattr(ctx.w_ref, "main_grad", None),
-                                    dres is not None and two_leaves(ctx, 0, 2))
-        dx = dx.view(ctx.shape)
-        if ctx.has_res:
-            return dx, dw, None, dx2.view(ctx.shape)
-        return dx, dw, None, None
+                                    dres is not None and two_leaves(ctx, 0, 2), ctx.shape)
+        return dx, dw, None, (dx2 if ctx.has_res else None)
 
 
 def two_leaves(node, i, j) -> bool:
@@ -103,9 +100,10 @@ def norm_inputs(x, residual):
     return (x2 if x2.stride(1) == 1 and x2.data_ptr() % 16 == 0 else dense_rows(x2)), None
 
 
-def norm_backward(dy, xin, w, rstd, dres, main_grad, two):
-    """(dx, the residual's gradient, dw or None when it was added to ``main_grad``); dx is shared unless ``two``
-    (with ``dres`` only)."""
+def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape):
+    """(dx, the residual's gradient, dw or None when it was added to ``main_grad``).  dx is shared unless ``two`` (with ``dres``
+    only), and then one tensor object: autograd takes a gradient that nobody else holds for a leaf's own without a copy, and
+    would take two views of the same memory for two leaves."""
     xin = dense_rows(xin)                       # (the kernel has a single pitch for x, dres and dx)
     rows, H = xin.shape
     dx = torch.empty_like(xin)
@@ -116,12 +114,13 @@ def norm_backward(dy, xin, w, rstd, dres, main_grad, two):
         target, mode = torch.empty(H, dtype=w.dtype, device=xin.device), 2
     else:
         target, mode = torch.empty(H, dtype=torch.float32, device=xin.device), 0
-    dx2 = dx
     if two:
         dx2 = torch.empty_like(dx)
         _lib.call("rmsnorm_bwd_two", dy, xin, w, rstd, dres, dx, dx2, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
+        dx, dx2 = dx.view(shape), dx2.view(shape)
     else:
         _lib.call("rmsnorm_bwd", dy, xin, w, rstd, dres, dx, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
+        dx = dx2 = dx.view(shape)
     return dx, dx2, None if main_grad is not None else target.to(w.dtype)
 
 

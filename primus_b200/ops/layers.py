@@ -85,8 +85,7 @@ class NormLinearFn(torch.autograd.Function):
                 torch.distributed.all_reduce(dy, group=tp_group)
         dres = None if dxsum is None else fused.dense_rows(dxsum.reshape(rows, H))
         dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None),
-                                            dres is not None and fused.two_leaves(ctx, 0, 1))
-        dx, dx2 = dx.view(ctx.shape), dx2.view(ctx.shape)
+                                            dres is not None and fused.two_leaves(ctx, 0, 1), ctx.shape)
         return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
 
 

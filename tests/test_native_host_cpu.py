@@ -9,7 +9,7 @@ import pytest
 import torch
 
 from primus_b200 import build
-from primus_b200.ops import _lib, attention, fused
+from primus_b200.ops import _lib, attention, fused, layers
 
 ROOT = Path(__file__).resolve().parent.parent
 CSRC = ROOT / "primus_b200" / "csrc"
@@ -348,7 +348,8 @@ def _norm_launchers(monkeypatch):
         if res is not None:
             v = at(xsum, rows, H, ldx).copy_(v.float() + at(res, rows, H, ldx).float())
         r = torch.rsqrt(v.float().pow(2).mean(1) + eps)
-        rstd.copy_(r)
+        if rstd is not None:
+            rstd.copy_(r)
         at(y, rows, H, ldy).copy_(v.float() * r[:, None] * w.float())
 
     def bwd(dy, x, w, rstd, dres, dx, dx2, dw, rows, H, ldx, lddy):
@@ -451,6 +452,35 @@ def test_norm_gradient_is_written_twice_only_for_first_gradients_of_two_leaves(m
     assert last(backward, x * 1)[0] == "rmsnorm_bwd" and torch.equal(x.grad, first) and torch.equal(r.grad, first)
     x.grad = r.grad = None
     assert last(backward, x, x)[0] == "rmsnorm_bwd"
+
+
+@pytest.mark.parametrize("shape", [(6, 16), (2, 3, 16)])
+@pytest.mark.parametrize("layer", [False, True])
+@pytest.mark.parametrize("what", ["both", "first", "second"])
+@pytest.mark.parametrize("leaves", ["both", "hidden", "residual"])
+def test_leaves_of_a_norm_do_not_share_their_gradients_memory(monkeypatch, shape, layer, what, leaves):
+    """Hidden and residual get the same gradient, each in memory of its own: a second pass doubles it, and one of them can be
+    changed in place."""
+    _norm_launchers(monkeypatch)
+    g = torch.Generator().manual_seed(5)
+    x, r, dy, ds = (torch.randn(*shape, generator=g).bfloat16() for _ in range(4))
+    w = torch.nn.Parameter((1 + 0.1 * torch.randn(16, generator=g)).bfloat16())
+    p = torch.nn.Parameter(torch.randn(16, 16, generator=g).bfloat16())
+
+    def run():
+        a, b = (t if leaves in ("both", name) else t.view_as(t) for t, name in ((x, "hidden"), (r, "residual")))
+        out = layers.NormLinearFn.apply(a, b, w, p, 1e-5, None, False) if layer else fused.RMSNormFn.apply(a, w, 1e-5, b)
+        pairs = list(zip(out, (dy.reshape(out[0].shape), ds)))
+        torch.autograd.backward(*zip(*{"both": pairs, "first": pairs[:1], "second": pairs[1:]}[what]))
+
+    x.requires_grad_(), r.requires_grad_()
+    run()
+    first = [t.grad.clone() for t in (x, r)]
+    assert torch.equal(*first) and x.grad.data_ptr() != r.grad.data_ptr()
+    run()
+    assert torch.equal(x.grad, 2 * first[0]) and torch.equal(r.grad, 2 * first[1])
+    x.grad.zero_()
+    assert torch.equal(r.grad, 2 * first[1])
 
 
 @pytest.mark.parametrize("sinks", [torch.zeros(2, dtype=torch.bfloat16), torch.zeros(3), torch.zeros(4)[::2]])
