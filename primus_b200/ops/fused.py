@@ -50,7 +50,7 @@ class RMSNormFn(torch.autograd.Function):
         H = x.shape[-1]
         x2, r2 = norm_inputs(x, residual)
         rows = x2.shape[0]
-        y = torch.empty(rows, H, dtype=x.dtype, device=x.device)
+        y = torch.empty_like(x2)
         rstd = torch.empty(rows, dtype=torch.float32, device=x.device)
         xsum = None
         if residual is not None:
@@ -64,17 +64,20 @@ class RMSNormFn(torch.autograd.Function):
         ctx.shape = x.shape
         ctx.w_ref = w
         if residual is not None:
-            return y.view(x.shape), xsum.view(x.shape)
-        return y.view(x.shape)
+            return as_shape(y, x.shape), as_shape(xsum, x.shape)
+        return as_shape(y, x.shape)
 
     @staticmethod
     def backward(ctx, dy, dxsum=None):
         xin, w, rstd = ctx.saved_tensors
         H = xin.shape[-1]
-        dres = None if dxsum is None else dense_rows(dxsum.reshape(-1, H))
-        dx, dx2, dw = norm_backward(dense_rows(dy.reshape(-1, H)), xin, w, rstd, dres, getattr(ctx.w_ref, "main_grad", None),
+        dres = None if dxsum is None else dense_rows(as_rows(dxsum, H))
+        dx, dx2, dw = norm_backward(dense_rows(as_rows(dy, H)), xin, w, rstd, dres, getattr(ctx.w_ref, "main_grad", None),
                                     dres is not None and two_leaves(ctx, 0, 2), ctx.shape)
         return dx, dw, None, (dx2 if ctx.has_res else None)
+
+
+_AccumulateGrad, _will_execute = torch._C._functions.AccumulateGrad, torch._C._will_engine_execute_node
 
 
 def two_leaves(node, i, j) -> bool:
@@ -82,21 +85,34 @@ def two_leaves(node, i, j) -> bool:
     pass.  A shared gradient would then be copied: autograd keeps a tensor per leaf.  It copies nothing where a leaf already
     has a gradient (the new one is added to it), where ``torch.autograd.grad`` hands the gradient out, or inside a model, where
     it goes on to two producers, which read it: there a second one would only cost its store."""
-    nodes = [node.next_functions[k][0] for k in (i, j)]
-    if nodes[0] is nodes[1] or not all(isinstance(n, torch._C._functions.AccumulateGrad) and n.variable.grad is None for n in nodes):
+    edges = node.next_functions
+    a, b = edges[i][0], edges[j][0]
+    if type(a) is not _AccumulateGrad or type(b) is not _AccumulateGrad or a is b:
+        return False
+    if a.variable.grad is not None or b.variable.grad is not None:
         return False
     try:
-        return all(torch._C._will_engine_execute_node(n) for n in nodes)
+        return _will_execute(a) and _will_execute(b)
     except RuntimeError:                        # (what it answers under torch.autograd.grad)
         return False
+
+
+def as_rows(t, H):
+    """``t`` as [rows, H].  (A reshape that changes nothing costs 1.4 us of host time, a look at the dimensions 0.1.)"""
+    return t if t.dim() == 2 else t.reshape(-1, H)
+
+
+def as_shape(t, shape):
+    return t if t.shape == shape else t.view(shape)
 
 
 def norm_inputs(x, residual):
     """``x`` and ``residual`` as rows that the kernels can read.  A row pitch is passed for the input of a norm without residual;
     with one, the kernel has a single pitch for both and for their sum."""
-    x2 = x.reshape(-1, x.shape[-1])
+    H = x.shape[-1]
+    x2 = as_rows(x, H)
     if residual is not None:
-        return dense_rows(x2), dense_rows(residual.reshape(-1, x.shape[-1]))
+        return dense_rows(x2), dense_rows(as_rows(residual, H))
     return (x2 if x2.stride(1) == 1 and x2.data_ptr() % 16 == 0 else dense_rows(x2)), None
 
 
@@ -104,7 +120,7 @@ def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape):
     """(dx, the residual's gradient, dw or None when it was added to ``main_grad``).  dx is shared unless ``two`` (with ``dres``
     only), and then one tensor object: autograd takes a gradient that nobody else holds for a leaf's own without a copy, and
     would take two views of the same memory for two leaves."""
-    xin = dense_rows(xin)                       # (the kernel has a single pitch for x, dres and dx)
+    xin = xin.contiguous()                      # (the kernel has a single pitch for x, dres and dx)
     rows, H = xin.shape
     dx = torch.empty_like(xin)
     sc = scratch(xin.device, "rmsnorm_dw", _lib.call_ret("rmsnorm_bwd_num_partials", rows) * H)
@@ -117,10 +133,10 @@ def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape):
     if two:
         dx2 = torch.empty_like(dx)
         _lib.call("rmsnorm_bwd_two", dy, xin, w, rstd, dres, dx, dx2, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
-        dx, dx2 = dx.view(shape), dx2.view(shape)
+        dx, dx2 = as_shape(dx, shape), as_shape(dx2, shape)
     else:
         _lib.call("rmsnorm_bwd", dy, xin, w, rstd, dres, dx, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
-        dx = dx2 = dx.view(shape)
+        dx = dx2 = as_shape(dx, shape)
     return dx, dx2, None if main_grad is not None else target.to(w.dtype)
 
 
@@ -151,8 +167,9 @@ def rmsnorm(x, w, eps=1e-5, residual=None):
 def dense_rows(t):
     """``t`` itself where it is contiguous and starts on a 16-byte boundary, else a copy that does: what a kernel may read in
     16-byte vectors without a row pitch."""
-    t = t.contiguous()
-    return t if t.data_ptr() % 16 == 0 else t.clone()
+    if t.is_contiguous():
+        return t if t.data_ptr() % 16 == 0 else t.clone()
+    return t.contiguous()
 
 
 class QKNormFn(torch.autograd.Function):

@@ -31,7 +31,7 @@ class NormLinearFn(torch.autograd.Function):
         H = hidden.shape[-1]
         x2, r2 = fused.norm_inputs(hidden, residual)
         rows = x2.shape[0]
-        y = torch.empty(rows, H, dtype=hidden.dtype, device=hidden.device)
+        y = torch.empty_like(x2)
         rstd = torch.empty(rows, dtype=torch.float32, device=hidden.device)
         if residual is not None:
             xsum = torch.empty_like(x2)
@@ -51,7 +51,7 @@ class NormLinearFn(torch.autograd.Function):
         ctx.shape = hidden.shape
         ctx.refs = (norm_w, weight)
         if residual is not None:
-            return out, xsum.view(hidden.shape)
+            return out, fused.as_shape(xsum, hidden.shape)
         return out, hidden
 
     @staticmethod
@@ -67,7 +67,7 @@ class NormLinearFn(torch.autograd.Function):
         if not dout2.is_contiguous():
             dout2 = dout2.contiguous()
         # recompute the normalised activations (not stored in forward)
-        y = torch.empty(rows, H, dtype=xsum.dtype, device=xsum.device)
+        y = torch.empty_like(xsum)
         _lib.call("rmsnorm_fwd", xsum, None, norm_w, y, None, None, rows, H, xsum.stride(0), y.stride(0),
                   float(ctx.eps))
         if sp:
@@ -83,7 +83,7 @@ class NormLinearFn(torch.autograd.Function):
             dy = gemm.gemm(dout2, weight, b_mn=True)
             if tp_group is not None:
                 torch.distributed.all_reduce(dy, group=tp_group)
-        dres = None if dxsum is None else fused.dense_rows(dxsum.reshape(rows, H))
+        dres = None if dxsum is None else fused.dense_rows(fused.as_rows(dxsum, H))
         dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None),
                                             dres is not None and fused.two_leaves(ctx, 0, 1), ctx.shape)
         return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
