@@ -475,13 +475,14 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
 // move to tensor memory at the start of a block, as A operands of the first GEMMs; their shared memory then stages the outputs.
 // A step of 128 x 128 x 128 holds four GEMMs of 512 clocks each in the dK / dV pass, three in the dQ pass; the passes take 2750
 // and 1960 clocks per step (3600 and 2600 with one ring of two or three buffers for both tiles: S waited for its tile).  8192 x
-// 32/8 x 128: dK / dV pass 924 -> 777 us; 4096 x 16 x 192/128: dQ pass 119 -> 101 us.
+// 32/8 x 128: dK / dV pass 924 -> 800 us; 4096 x 16 x 192/128: dQ pass 119 -> 103 us.  Tensor pipe busy 72 % of the time in the
+// dK / dV pass at 4096 x 32/8 x 128, 68 % in the dQ pass (57 and 52 with one ring).
 //
 // The CTAs are persistent where the heads have d_qk == d_v: one takes the next block from the hardware scheduler
 // (clusterlaunchcontrol.try_cancel, so that the longest blocks still start first) and loads its tiles, and issues its first
 // GEMMs, while the sums of this block leave.  A CTA of a cluster that shares a block, and the multi-latent shape, whose resident
 // tile fills the shared memory, have one block.  dQ pass, one block per CTA -> persistent, us: window of 128 at 2 x 2048 x
-// 64/8 x 64 98 -> 59 (start and end were 8500 of 11600 clocks), 2048 x 32/8 x 128 54 -> 49, 8192 x 32/8 x 128 603 -> 585.
+// 64/8 x 64 98 -> 59 (start and end were 8500 of 11600 clocks), 2048 x 32/8 x 128 54 -> 47, 8192 x 32/8 x 128 603 -> 590.
 //   warp 0 scheduler and TMA producer; warp 1 issues the MMAs; warp 2 stores the outputs; warps 4..19 softmax and gradients
 template <int DQK, int DV, int MODE>
 struct BwWideCfg {
@@ -1205,7 +1206,8 @@ struct BwdArgs {
 //   4096 x 32/4 x 128   399 / 221 / 264 / 395      1024 x 8/1 x 128   101 / 58 / 38 / 31     8192 x 1/1 x 128   104 / 62 / 56 / 123
 //   8192 x 32/8 x 128   803 / 835 / 1013 / 1511    2048 x 16/2 x 64   140 / 77 / 46 / 56     window 128, 64/8 x 64  60 / 86 / 130 / 258
 // dQ pass: 2048 x 32/8 x 128  49 / 97 / 202 / 459   8192 x 1/1 x 128  79 / 46 / 41 / 82.  The model below is within 15 % of
-// these.  Clusters of 4 and 8 do not fit every GPC: 132 and 120 CTAs in flight on 148 SMs.
+// these but for the window (36 / 61 / 142 / 378): its blocks of few steps cost more at their start and end than `fixed` says, and
+// only the order of the choices is right there.  Clusters of 4 and 8 do not fit every GPC: 132 and 120 CTAs in flight on 148 SMs.
 int bwd_cluster_size(int mode, int d_qk, int d_v, int batch, int seq, int seq_k, int q_off, int hq, int hkv, int causal,
                      int window) {
   const bool kv = mode == MODE_DKDV;

@@ -14,8 +14,9 @@
 // as two buffers, S of a tile's next block had to wait for its P.V and with it for the exponentials: 3485 clocks per pair of
 // 128 x 128 blocks, of which the GEMMs take 2048; now 2800, with the special-function unit busy for 2048.  A pair's start and
 // end (Q, tensor memory, output: 8000 clocks of 20250 for a window of 128) pass under its neighbours' blocks.
-// Before and now, us: 8192 x 32/8 x 128 483 -> 405 (1.38 PFLOP/s, under the power cap), 2048 x 32/8 x 128 43 -> 36,
-// 4096 x 16 x 192/128 83 -> 75, window of 128 at 2 x 2048 x 64/8 x 64 79 -> 52.
+// Before and now, us (median of the kernel in a short run): 8192 x 32/8 x 128 483 -> 412 (1.33 PFLOP/s, under the power cap), 2048
+// x 32/8 x 128 43 -> 35, 4096 x 16 x 192/128 83 -> 74, window of 128 at 2 x 2048 x 64/8 x 64 79 -> 51.  Tensor pipe busy 65 % of
+// the time at 4096 x 32/8 x 128, 62 % with 192/128.
 // O is rescaled in tensor memory only when the running max grew by more than 2^8.
 // V is consumed straight from its [kv, d] row-major tile through an MN-major descriptor, so no
 // transposes are needed.  All waits are bounded.
@@ -195,7 +196,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           for (int j = 0; j <= w.n; ++j) {
             if (j == w.n) {
               // Ask for the next pair as late as its operands allow: a pair taken over early is not there for a CTA that
-              // runs out of work first (2048 x 32/8 x 128: 48 us asked for at the start of a pair, 39 us here).
+              // runs out of work first (2048 x 32/8 x 128: 48 us asked for at the start of a pair, 35 us here).
               FA_WAIT(&bars->next_empty[nx], ((item >> 1) & 1) ^ 1, PB_ERR_TIMEOUT_TMA);
               pb::mbar_expect_tx(&bars->next_full[nx], 16);
               pb::clc_try_cancel(&bars->next[nx], &bars->next_full[nx]);
