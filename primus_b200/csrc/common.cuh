@@ -402,9 +402,19 @@ PB_DEVICE void named_bar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
-// logistic function with the fast reciprocal (every SwiGLU kernel uses this one expression, so fused and un-fused
-// variants round identically)
-PB_DEVICE float fast_sigmoid(float x) { return __fdividef(1.f, 1.f + __expf(-x)); }
+PB_DEVICE float fast_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+PB_DEVICE float fast_rcp(float x) {
+  float y;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// logistic function (every SwiGLU kernel uses this one expression, so fused and un-fused variants round identically).  Flushed
+// denormals change nothing: 1 + a denormal is 1, and the reciprocal is one only where the denominator passes 2^126.
+PB_DEVICE float fast_sigmoid(float x) { return fast_rcp(1.f + fast_exp2(x * -1.4426950408889634f)); }
 PB_DEVICE uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
@@ -413,11 +423,6 @@ PB_DEVICE uint32_t pack_bf16x2(float lo, float hi) {
 PB_DEVICE float fast_tanh(float x) {
   float y;
   asm("tanh.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
-  return y;
-}
-PB_DEVICE float fast_exp2(float x) {
-  float y;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
 
@@ -437,6 +442,14 @@ PB_DEVICE uint64_t mul_f32x2(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
+}
+// fast_sigmoid of two values
+PB_DEVICE uint64_t fast_sigmoid2(uint64_t x) {
+  float a, b;
+  unpack_f32x2(mul_f32x2(x, pack_f32x2(-1.4426950408889634f, -1.4426950408889634f)), a, b);
+  const uint64_t one = pack_f32x2(1.f, 1.f);
+  unpack_f32x2(fma_f32x2(pack_f32x2(fast_exp2(a), fast_exp2(b)), one, one), a, b);
+  return pack_f32x2(fast_rcp(a), fast_rcp(b));
 }
 PB_DEVICE float warp_sum(float v) {
 #pragma unroll

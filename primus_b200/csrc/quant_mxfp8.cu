@@ -16,7 +16,7 @@
 #include <cuda_fp4.h>
 #include <cuda_fp8.h>
 
-#include "common.cuh"
+#include "vec.cuh"
 
 namespace {
 
@@ -43,15 +43,6 @@ __device__ __forceinline__ uint16_t cvt2(float a, float b) {
 // MXFP4 numerics on the FP8 data path: the block exponent leaves the block maximum at or below 6 (the largest E2M1
 // magnitude), values are rounded to E2M1 (RN-even, saturating) and stored as the E4M3 byte of the same number (every
 // E2M1 value is exact in E4M3), so the block-scaled FP8 GEMM consumes them unchanged.
-__device__ __forceinline__ int e8m0_from_amax_fp4(float amax) {
-  const float v = amax * (1.0f / 6.0f);
-  const uint32_t b = __float_as_uint(v);
-  int e = (int)((b >> 23) & 0xff);
-  if (b & 0x7fffff) e += 1;
-  if (e < 0) e = 0;
-  if (e > 254) e = 254;
-  return (amax == 0.f) ? 0 : e;
-}
 __device__ __forceinline__ uint16_t cvt2_fp4(float a, float b) {
   const uint32_t packed = (uint32_t)__nv_cvt_float2_to_fp4x2(make_float2(a, b), __NV_E2M1, cudaRoundNearest);
   // E2M1 code (sign, 3 magnitude bits: 0, 0.5, 1, 1.5, 2, 3, 4, 6) -> E4M3 byte of the same value
@@ -64,10 +55,6 @@ __device__ __forceinline__ uint16_t cvt2_fp4(float a, float b) {
 template <bool FP4>
 __device__ __forceinline__ uint16_t cvt2_sel(float a, float b) {
   return FP4 ? cvt2_fp4(a, b) : cvt2(a, b);
-}
-template <bool FP4>
-__device__ __forceinline__ int e8m0_sel(float amax) {
-  return FP4 ? e8m0_from_amax_fp4(amax) : e8m0_from_amax(amax);
 }
 
 __device__ __forceinline__ long sf_offset(int mn, int k_blk32, int k_groups) {
@@ -100,92 +87,163 @@ __device__ __forceinline__ __nv_bfloat162 as_bf2(uint32_t w) { return *reinterpr
 __device__ __forceinline__ uint32_t as_u32(__nv_bfloat162 v) { return *reinterpret_cast<uint32_t*>(&v); }
 __device__ __forceinline__ uint32_t max_pair(uint32_t a, uint32_t b) { return as_u32(__hmax2(as_bf2(a), as_bf2(b))); }
 __device__ __forceinline__ uint32_t abs_pair(uint32_t a) { return a & 0x7fff7fffu; }
+// the larger magnitudes of two pairs, with the operands' signs multiplied: a chain of them needs abs_pair at its end only
+__device__ __forceinline__ uint32_t max_mag(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("max.xorsign.abs.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 __device__ __forceinline__ float lo_f(uint32_t w) { return __uint_as_float(w << 16); }
 __device__ __forceinline__ float hi_f(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 
 // strip of 32 rows of this warp (a CTA of more than four warps has several on every strip, which share its parts)
 __device__ __forceinline__ int strip() { return (threadIdx.x >> 5) & 3; }
 
-// Quantises part `h` of this warp's strip -- 8 CG columns, held in d[CG] -- into q_row / q_col (either may be null).  CG = 8:
-// the layout above (two halves); CG = 4: quarters, lane (cg = lane & 3, sub = lane >> 2) holds rows 8 i + sub (i < 4), half
-// the registers for one more shuffle per column pair.  p: offset of the lane's first element in the [R, C] tensor.
-template <int MODE = SCALE_BLOCK32, bool FP4 = false, int CG = 8>
-__device__ __forceinline__ void quantize_half(const uint4 (&d)[CG], int h, long p, int C, uint8_t* __restrict__ q_row,
-                                              uint8_t* __restrict__ q_col, TileScales* scales, int fixed_e = 0,
-                                              const uint8_t* e_rowv = nullptr, const uint8_t* e_colv = nullptr) {
-  constexpr int SUBS = 32 / CG;
-  const int lane = threadIdx.x & 31, warp = strip();
-  const int cg = lane % CG, sub = lane / CG;
-  if (q_row) {
-    uint32_t m[CG / 2];                 // block maxima of the lane's rows 2 j, 2 j + 1
-    if (MODE == SCALE_BLOCK32) {
+// Scales of two blocks from the bf16 bits of their maxima (not NaN), both in 16-bit halves: `e` as e8m0_from_amax gives it, and
+// `inv`, 2^-(e - 127) as bf16.  In these bits 448 (fp4: 6) is an exponent field 8 (2) above that of 1 and a fraction of 0x60
+// (0x40), so that the quotient's exponent, rounded up, is the field less 8 after adding what carries a larger fraction into it.
+// With both halves at once a scale costs 4 instructions instead of 12 (8192 x 4096 in both directions 24.7 -> 23.5 us).
+struct PairScale {
+  uint32_t e, inv;
+};
+template <bool FP4>
+__device__ __forceinline__ PairScale pair_scale(uint32_t m) {
+  constexpr uint32_t OFF = FP4 ? 2 : 8, CARRY = FP4 ? 0x3f : 0x1f, TWO = 0x10001u;
+  const uint32_t t = __vmaxu2((m + CARRY * TWO) & 0x7f807f80u, ((OFF + 1) << 7) * TWO);   // (a subnormal quotient has e = 1)
+  PairScale r;
+  r.e = __vminu2((t >> 7) - OFF * TWO, m);       // zero for a block of zeros
+  r.inv = ((254 + OFF) << 7) * TWO - t;
+  const uint32_t inf = (m + 0x00800080u) & 0x80008000u;
+  if (inf) {                                     // an infinite maximum: e = 254, inv = 2^-126
+    const uint32_t mask = (inf >> 15) * 0xffffu;
+    r.e = (r.e & ~mask) | (0x00fe00feu & mask);
+    r.inv = (r.inv & ~mask) | (0x00800080u & mask);
+  }
+  return r;
+}
+
+// eight bf16 values times powers of two -> eight bytes; s[u]: the factors of the u-th pair
+template <bool FP4>
+__device__ __forceinline__ uint2 scale_cvt8(const uint64_t (&f)[4], uint64_t s0, uint64_t s1, uint64_t s2, uint64_t s3) {
+  float a, b;
+  uint32_t w[4];
+  pb::unpack_f32x2(pb::mul_f32x2(f[0], s0), a, b);
+  w[0] = cvt2_sel<FP4>(a, b);
+  pb::unpack_f32x2(pb::mul_f32x2(f[1], s1), a, b);
+  w[1] = cvt2_sel<FP4>(a, b);
+  pb::unpack_f32x2(pb::mul_f32x2(f[2], s2), a, b);
+  w[2] = cvt2_sel<FP4>(a, b);
+  pb::unpack_f32x2(pb::mul_f32x2(f[3], s3), a, b);
+  w[3] = cvt2_sel<FP4>(a, b);
+  return make_uint2(__byte_perm(w[0], w[1], 0x5410), __byte_perm(w[2], w[3], 0x5410));
+}
+
+// Quantises half `h` of this warp's strip -- 64 columns, held in d[8] -- into q_row / q_col (either may be null).  p: offset of
+// the lane's first element in the [R, C] tensor.  BOTH: neither is null, and each value is converted to fp32 once for the two,
+// at the price of registers (the plain quantiser, five CTAs per SM, spills with it: 27.6 against 23.5 us at 8192 x 4096).
+template <int MODE = SCALE_BLOCK32, bool FP4 = false, bool BOTH = false>
+__device__ __forceinline__ void quantize_half(const uint4 (&d)[8], int h, long p, int C, uint8_t* __restrict__ q_row,
+                                              uint8_t* __restrict__ q_col, TileScales* scales, int warp = strip(),
+                                              int fixed_e = 0, const uint8_t* e_rowv = nullptr,
+                                              const uint8_t* e_colv = nullptr) {
+  const int lane = threadIdx.x & 31;
+  const int cg = lane & 7, sub = lane >> 3;
+  uint32_t row_inv[4];             // of the lane's rows 2 j, 2 j + 1
+  if (BOTH || q_row) {
 #pragma unroll
-      for (int j = 0; j < CG / 2; ++j) {
+    for (int j = 0; j < 4; ++j) {
+      uint32_t e;
+      if (MODE == SCALE_BLOCK32) {
         uint32_t a[2];
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
           const uint4& v = d[2 * j + u];
-          a[u] = max_pair(max_pair(abs_pair(v.x), abs_pair(v.y)), max_pair(abs_pair(v.z), abs_pair(v.w)));
+          a[u] = max_mag(max_mag(v.x, v.y), max_mag(v.z, v.w));
         }
+        uint32_t m = max_mag(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632));
+        m = max_mag(m, __shfl_xor_sync(0xffffffffu, m, 1));
         // (a block of nothing but NaN counts as zero, as in the column direction: the maximum ignores a NaN operand)
-        m[j] = max_pair(0u, max_pair(__byte_perm(a[0], a[1], 0x5410), __byte_perm(a[0], a[1], 0x7632)));
-        m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 1));
-        m[j] = max_pair(m[j], __shfl_xor_sync(0xffffffffu, m[j], 2));
+        m = abs_pair(max_mag(0u, max_mag(m, __shfl_xor_sync(0xffffffffu, m, 2))));
+        const PairScale ps = pair_scale<FP4>(m);
+        e = ps.e;
+        row_inv[j] = ps.inv;
+      } else {
+        const int r = 8 * j + sub;
+        const int e0 = MODE == SCALE_FIXED ? fixed_e : (int)e_rowv[warp * 32 + r];
+        const int e1 = MODE == SCALE_FIXED ? fixed_e : (int)e_rowv[warp * 32 + r + 4];
+        e = (uint32_t)e0 | ((uint32_t)e1 << 16);
+        row_inv[j] = (__float_as_uint(inv_scale_from_e8m0(e0)) >> 16) | __float_as_uint(inv_scale_from_e8m0(e1));
+      }
+      if ((cg & 3) == 0) {
+        uint8_t* sf = reinterpret_cast<uint8_t*>(scales->row) + (8 * j + sub) * 16 + warp * 4 + h * 2 + (cg >> 2);
+        sf[0] = (uint8_t)e;
+        sf[64] = (uint8_t)(e >> 16);
       }
     }
+  }
+  auto unpack8 = [&](int i, uint64_t (&f)[4]) {
+    f[0] = pb::pack_f32x2(lo_f(d[i].x), hi_f(d[i].x));
+    f[1] = pb::pack_f32x2(lo_f(d[i].y), hi_f(d[i].y));
+    f[2] = pb::pack_f32x2(lo_f(d[i].z), hi_f(d[i].z));
+    f[3] = pb::pack_f32x2(lo_f(d[i].w), hi_f(d[i].w));
+  };
+  if (!BOTH && q_row) {
 #pragma unroll
-    for (int i = 0; i < CG; ++i) {
-      const int r = SUBS * i + sub;
-      const int e = MODE == SCALE_FIXED ? fixed_e
-                    : MODE == SCALE_VEC128 ? (int)e_rowv[warp * 32 + r]
-                                           : e8m0_sel<FP4>((i & 1) ? hi_f(m[i >> 1]) : lo_f(m[i >> 1]));
-      const float inv = inv_scale_from_e8m0(e);
-      const uint32_t w0 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].x) * inv, hi_f(d[i].x) * inv) |
-                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].y) * inv, hi_f(d[i].y) * inv) << 16);
-      const uint32_t w1 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].z) * inv, hi_f(d[i].z) * inv) |
-                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].w) * inv, hi_f(d[i].w) * inv) << 16);
-      *reinterpret_cast<uint2*>(q_row + p + (long)(SUBS * i) * C) = make_uint2(w0, w1);
-      if ((cg & 3) == 0) reinterpret_cast<uint8_t*>(scales->row)[r * 16 + warp * 4 + h * (CG / 4) + (cg >> 2)] = (uint8_t)e;
+    for (int i = 0; i < 8; ++i) {
+      uint64_t f[4];
+      unpack8(i, f);
+      const float inv = (i & 1) ? hi_f(row_inv[i >> 1]) : lo_f(row_inv[i >> 1]);
+      const uint64_t s = pb::pack_f32x2(inv, inv);
+      *reinterpret_cast<uint2*>(q_row + p + (long)(4 * i) * C) = scale_cvt8<FP4>(f, s, s, s, s);
     }
   }
-  if (q_col) {
-    uint32_t m[4] = {0, 0, 0, 0};       // maxima of column pairs 2 u, 2 u + 1
+  if (BOTH || q_col) {
+    uint64_t col_inv[4];                // of the column pairs 2 u, 2 u + 1
+    uint32_t m[4] = {0, 0, 0, 0}, inv[4];
+    const int c0 = h * 64 + cg * 8; // first of the lane's columns in the tile
     if (MODE == SCALE_BLOCK32) {
 #pragma unroll
-      for (int i = 0; i < CG; ++i) {
-        m[0] = max_pair(m[0], abs_pair(d[i].x));
-        m[1] = max_pair(m[1], abs_pair(d[i].y));
-        m[2] = max_pair(m[2], abs_pair(d[i].z));
-        m[3] = max_pair(m[3], abs_pair(d[i].w));
+      for (int i = 0; i < 8; ++i) {
+        m[0] = max_mag(m[0], d[i].x);
+        m[1] = max_mag(m[1], d[i].y);
+        m[2] = max_mag(m[2], d[i].z);
+        m[3] = max_mag(m[3], d[i].w);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
 #pragma unroll
-        for (int o = CG; o < 32; o <<= 1) m[u] = max_pair(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+        for (int o = 8; o < 32; o <<= 1) m[u] = max_mag(m[u], __shfl_xor_sync(0xffffffffu, m[u], o));
+        const PairScale ps = pair_scale<FP4>(abs_pair(m[u]));
+        m[u] = ps.e;
+        inv[u] = ps.inv;
+      }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int e0 = MODE == SCALE_FIXED ? fixed_e : (int)e_colv[c0 + 2 * u];
+        const int e1 = MODE == SCALE_FIXED ? fixed_e : (int)e_colv[c0 + 2 * u + 1];
+        m[u] = (uint32_t)e0 | ((uint32_t)e1 << 16);
+        inv[u] = (__float_as_uint(inv_scale_from_e8m0(e0)) >> 16) | __float_as_uint(inv_scale_from_e8m0(e1));
       }
     }
-    const int c0 = h * 8 * CG + cg * 8; // first of the lane's columns in the tile
-    float inv[8];
+    // every sub holds the 8 exponents; sub u writes those of its two columns
+    const uint32_t e = sub < 2 ? (sub == 0 ? m[0] : m[1]) : (sub == 2 ? m[2] : m[3]);
+    const int c = c0 + 2 * sub;
+    uint8_t* sf = reinterpret_cast<uint8_t*>(scales->col) + (c & 31) * 16 + (c >> 5) * 4 + warp;
+    sf[0] = (uint8_t)e;
+    sf[16] = (uint8_t)(e >> 16);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int e0 = MODE == SCALE_FIXED ? fixed_e : MODE == SCALE_VEC128 ? (int)e_colv[c0 + 2 * u] : e8m0_sel<FP4>(lo_f(m[u]));
-      const int e1 = MODE == SCALE_FIXED ? fixed_e : MODE == SCALE_VEC128 ? (int)e_colv[c0 + 2 * u + 1] : e8m0_sel<FP4>(hi_f(m[u]));
-      inv[2 * u] = inv_scale_from_e8m0(e0);
-      inv[2 * u + 1] = inv_scale_from_e8m0(e1);
-      if (sub == u) {                   // every sub holds the 8 exponents; sub u writes those of its two columns
-        const int c = c0 + 2 * u;
-        uint8_t* sf = reinterpret_cast<uint8_t*>(scales->col) + (c & 31) * 16 + (c >> 5) * 4 + warp;
-        sf[0] = (uint8_t)e0;
-        sf[16] = (uint8_t)e1;
+    for (int u = 0; u < 4; ++u) col_inv[u] = pb::pack_f32x2(lo_f(inv[u]), hi_f(inv[u]));
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      uint64_t f[4];
+      unpack8(i, f);
+      if (BOTH) {
+        const float inv = (i & 1) ? hi_f(row_inv[i >> 1]) : lo_f(row_inv[i >> 1]);
+        const uint64_t s = pb::pack_f32x2(inv, inv);
+        *reinterpret_cast<uint2*>(q_row + p + (long)(4 * i) * C) = scale_cvt8<FP4>(f, s, s, s, s);
       }
-    }
-#pragma unroll
-    for (int i = 0; i < CG; ++i) {
-      const uint32_t w0 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].x) * inv[0], hi_f(d[i].x) * inv[1]) |
-                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].y) * inv[2], hi_f(d[i].y) * inv[3]) << 16);
-      const uint32_t w1 = (uint32_t)cvt2_sel<FP4>(lo_f(d[i].z) * inv[4], hi_f(d[i].z) * inv[5]) |
-                          ((uint32_t)cvt2_sel<FP4>(lo_f(d[i].w) * inv[6], hi_f(d[i].w) * inv[7]) << 16);
-      *reinterpret_cast<uint2*>(q_col + p + (long)(SUBS * i) * C) = make_uint2(w0, w1);
+      *reinterpret_cast<uint2*>(q_col + p + (long)(4 * i) * C) = scale_cvt8<FP4>(f, col_inv[0], col_inv[1], col_inv[2], col_inv[3]);
     }
   }
 }
@@ -203,10 +261,9 @@ __device__ __forceinline__ void store_scales(const TileScales* scales, int R, in
 }
 
 // element offset of a lane: row `sub` of its warp's strip, first of its 8 columns of part 0
-template <int CG = 8>
-__device__ __forceinline__ long lane_offset(int row0, int col0, long ld) {
+__device__ __forceinline__ long lane_offset(int row0, int col0, long ld, int strip_ = strip()) {
   const int lane = threadIdx.x & 31;
-  return (long)(row0 + strip() * 32 + lane / CG) * ld + col0 + (lane % CG) * 8;
+  return (long)(row0 + strip_ * 32 + (lane >> 3)) * ld + col0 + (lane & 7) * 8;
 }
 
 __device__ __forceinline__ void load_tile(const __nv_bfloat16* __restrict__ x, long p, int C, uint4 (&d)[2][8]) {
@@ -250,7 +307,7 @@ quant_tensorwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, const
   if (a == 0.f && fallback_amax != nullptr) a = *fallback_amax;
   const int fixed_e = e8m0_from_amax(a);
 #pragma unroll
-  for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, fixed_e);
+  for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, strip(), fixed_e);
   store_scales(&scales, R, C, row0, col0, sf_row, sf_col);
 }
 
@@ -299,7 +356,7 @@ quant_blockwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_
     m = max_pair(max_pair(strip_max[0], strip_max[1]), max_pair(strip_max[2], strip_max[3]));
     const int fixed_e = e8m0_from_amax(fmaxf(lo_f(m), hi_f(m)));
 #pragma unroll
-    for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, fixed_e);
+    for (int h = 0; h < 2; ++h) quantize_half<SCALE_FIXED>(d[h], h, p + h * 64, C, q_row, q_col, &scales, strip(), fixed_e);
   } else {
     if (cg == 0) {
 #pragma unroll
@@ -335,7 +392,7 @@ quant_blockwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_
     __syncthreads();
 #pragma unroll
     for (int h = 0; h < 2; ++h)
-      quantize_half<SCALE_VEC128>(d[h], h, p + h * 64, C, q_row, q_col, &scales, 0, e_rowv, e_colv);
+      quantize_half<SCALE_VEC128>(d[h], h, p + h * 64, C, q_row, q_col, &scales, strip(), 0, e_rowv, e_colv);
   }
   store_scales(&scales, R, C, row0, col0, sf_row, sf_col);
 }
@@ -381,10 +438,11 @@ __device__ __forceinline__ uint4 bf8_pack(const float* f) {
 // SwiGLU forward fused with the quantisation of its output: h1 [T, 2I] = [gate | up] -> MXFP8 of
 // act[T, I] = silu(gate) * up (rounded to bf16 first, so the values equal quantising the un-fused kernel's output).
 // Four rows' loads in flight per lane and round keep it at 80 registers: six CTAs (24 warps) per SM hide the two special-
-// function operations per element (8192 x 14336, row direction: 107 us, 127 with the tile staged in shared memory).  WIDE: as many warps per strip as it has
-// parts, for tensors of at most a tile per SM, where a warp's parts one after the other are the time (1024 x 1408: 5.4 -> 4.9
-// us, backward 10.4 -> 7.2); with several CTAs per SM the parts' registers are better spent on more CTAs.
-template <bool WIDE>
+// function operations per element (8192 x 14336, row direction: 97 us, 6.1 TB/s; 106 with scales computed one by one and 127 with
+// the tile staged in shared memory; two fp32 operations per instruction, as in the backward, need more registers here: 115).
+// WIDE: as many warps per strip as it has parts, for tensors of at most a tile per SM, where a warp's parts one after the other
+// are the time (1024 x 1408: 5.4 -> 4.9 us); with several CTAs per SM the parts' registers are better spent on more CTAs.
+template <bool WIDE, bool CLAMP>
 __global__ void __launch_bounds__(WIDE ? 2 * QT : QT, WIDE ? 2 : 6)
 swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, float clamp, uint8_t* __restrict__ q_row,
                           uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
@@ -411,12 +469,11 @@ swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, fl
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           float gg = fg[j], uu = fu[j];
-          if (clamp > 0.f) {
+          if (CLAMP) {
             gg = fminf(gg, clamp);
             uu = fminf(fmaxf(uu, -clamp), clamp);
           }
-          const float sig = pb::fast_sigmoid(gg);
-          o[j] = gg * sig * uu * 1.f;
+          o[j] = gg * pb::fast_sigmoid(gg) * uu;
         }
         d[i0 + i] = bf8_pack(o);
       }
@@ -426,58 +483,104 @@ swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, fl
   store_scales(&scales, T, I, row0, col0, sf_row, sf_col);
 }
 
+constexpr int BWD_WARP_BYTES = 3 * 8 * 32 * 16;   // shared memory of a warp of the SwiGLU backward
+
+// Two elements of the SwiGLU backward: dgate, dup and the activation from gate, up and dact (bf16 pairs), in the order and with the
+// roundings of swiglu_bwd_kernel and swiglu_fwd_kernel (two fp32 operations an instruction).
+template <bool CLAMP>
+__device__ __forceinline__ void swiglu_bwd_pair(uint32_t gate, uint32_t up, uint32_t dact, float clamp, uint32_t& dgate, uint32_t& dup,
+                                                uint32_t& act) {
+  float g0 = lo_f(gate), g1 = hi_f(gate), u0 = lo_f(up), u1 = hi_f(up);
+  uint64_t gmask = 0, umask = 0;
+  if (CLAMP) {
+    gmask = pb::pack_f32x2(g0 > clamp ? 0.f : 1.f, g1 > clamp ? 0.f : 1.f);
+    umask = pb::pack_f32x2(u0 > clamp || u0 < -clamp ? 0.f : 1.f, u1 > clamp || u1 < -clamp ? 0.f : 1.f);
+    if (g0 > clamp) g0 = clamp;
+    if (g1 > clamp) g1 = clamp;
+    if (u0 > clamp) u0 = clamp;
+    if (u0 < -clamp) u0 = -clamp;
+    if (u1 > clamp) u1 = clamp;
+    if (u1 < -clamp) u1 = -clamp;
+  }
+  const uint64_t g = pb::pack_f32x2(g0, g1), u = pb::pack_f32x2(u0, u1), d = pb::pack_f32x2(lo_f(dact), hi_f(dact));
+  const uint64_t one = pb::pack_f32x2(1.f, 1.f), minus = pb::pack_f32x2(-1.f, -1.f);
+  const uint64_t sig = pb::fast_sigmoid2(g);
+  const uint64_t sl = pb::mul_f32x2(g, sig);
+  const uint64_t dsl = pb::mul_f32x2(sig, pb::fma_f32x2(g, pb::fma_f32x2(sig, minus, one), one));
+  uint64_t og = pb::mul_f32x2(pb::mul_f32x2(d, u), dsl), ou = pb::mul_f32x2(d, sl);
+  if (CLAMP) {
+    og = pb::mul_f32x2(og, gmask);
+    ou = pb::mul_f32x2(ou, umask);
+  }
+  float a, b;
+  pb::unpack_f32x2(og, a, b);
+  dgate = pb::pack_bf16x2(a, b);
+  pb::unpack_f32x2(ou, a, b);
+  dup = pb::pack_bf16x2(a, b);
+  pb::unpack_f32x2(pb::mul_f32x2(sl, u), a, b);
+  act = pb::pack_bf16x2(a, b);
+}
+
 // SwiGLU backward fused with the quantisation of its output: (h1 [T, 2I], dact [T, I]) -> MXFP8 (both directions) of
-// dh1 [T, 2I] = [dgate | dup].  One CTA per 128 x 128 tile of the activation, which reads gate, up and dact once.
-// A warp computes the dgate and the dup values of its strip by 32 x 32 quarters: the twelve loads of a quarter are in
-// flight per lane, and two results of 16 registers instead of 32 let five CTAs share an SM instead of three.  WIDE: as above.
-template <bool WIDE>
-__global__ void __launch_bounds__(WIDE ? 4 * QT : QT, WIDE ? 1 : 5)
+// dh1 [T, 2I] = [dgate | dup], and (optional) of the activation itself along T, the operand of the weight gradient, which
+// another pass over h1 would otherwise recompute.  One CTA per 128 x 128 tile of the activation; a warp takes 32 rows of a
+// 64-column half, with its neighbour the other half of the same rows, so that whole 128-byte lines of the results are written
+// at about the same time (quarters one after the other left half-written lines for DRAM: with more CTAs in flight twice the time).
+// gate, up and dact go to the lane's own slots of shared memory and the three results take their places there: a
+// lane holds one result at a time in registers, and 16 warps share an SM.  8192 x 14336: 238 us, and another 107 for the
+// activation, before; 194 and, with the activation, 221 now (5.8 TB/s).  What is left beside the memory is the issue of about
+// 35 instructions an element.  WIDE: as above, eight warps, one round.
+template <bool WIDE, bool CLAMP>
+__global__ void __launch_bounds__(WIDE ? 2 * QT : QT, WIDE ? 2 : 4)
 swiglu_bwd_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, const __nv_bfloat16* __restrict__ dact, int T, int I,
                               float clamp, uint8_t* __restrict__ q_row, uint8_t* __restrict__ sf_row,
-                              uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
-  __shared__ TileScales scales[2];               // of the dgate and of the dup tile
-  const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
-  const long pin = lane_offset<4>(row0, col0, 2L * I), pd = lane_offset<4>(row0, col0, I);
+                              uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col, uint8_t* __restrict__ act_col,
+                              uint8_t* __restrict__ act_sf) {
+  extern __shared__ __align__(16) uint4 slots_raw[];   // [warp][gate, up, dact][row of the lane][lane]
+  __shared__ TileScales scales[3];               // of the dgate, the dup and the activation tile
+  constexpr int WARPS = WIDE ? 8 : 4, STRIPS = WARPS / 2;
+  const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE, warp = threadIdx.x >> 5, h = warp & 1;
+  uint4 *sg = slots_raw + warp * (BWD_WARP_BYTES / 16) + (threadIdx.x & 31), *su = sg + 256, *sd = su + 256;
 #pragma unroll 1
-  for (int h = WIDE ? threadIdx.x / QT : 0; h < 4; h += WIDE ? 4 : 1) {
-    uint4 dg[4], du[4], da[4];
+  for (int st = warp >> 1; st < 4; st += STRIPS) {
+    const long o2 = lane_offset(row0, col0, 2L * I, st) + h * 64, o1 = lane_offset(row0, col0, I, st) + h * 64;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const __nv_bfloat16* g = h1 + pin + h * 32 + (long)(8 * i) * 2 * I;
-      dg[i] = *reinterpret_cast<const uint4*>(g);
-      du[i] = *reinterpret_cast<const uint4*>(g + I);
-      da[i] = *reinterpret_cast<const uint4*>(dact + pd + h * 32 + (long)(8 * i) * I);
+    for (int i = 0; i < 8; ++i) {
+      const __nv_bfloat16* g = h1 + o2 + (long)(4 * i) * 2 * I;
+      pb::cp_async_16(sg + i * 32, g);
+      pb::cp_async_16(su + i * 32, g + I);
+      pb::cp_async_16(sd + i * 32, dact + o1 + (long)(4 * i) * I);
     }
+    pb::cp_async_commit();
+    pb::cp_async_wait<0>();
+#pragma unroll 2
+    for (int i = 0; i < 8; ++i) {
+      const uint4 vg = sg[i * 32], vu = su[i * 32], vd = sd[i * 32];
+      uint32_t og[4], ou[4], oa[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float fg[8], fu[8], fd[8], og[8], ou[8];
-      bf8_unpack(dg[i], fg);
-      bf8_unpack(du[i], fu);
-      bf8_unpack(da[i], fd);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        float gg = fg[j], uu = fu[j];
-        float gmask = 1.f, umask = 1.f;
-        if (clamp > 0.f) {
-          if (gg > clamp) { gg = clamp; gmask = 0.f; }
-          if (uu > clamp) { uu = clamp; umask = 0.f; }
-          if (uu < -clamp) { uu = -clamp; umask = 0.f; }
-        }
-        const float sig = pb::fast_sigmoid(gg);
-        const float sl = gg * sig;
-        const float d = fd[j] * 1.f;
-        const float dsl = sig * (1.f + gg * (1.f - sig));
-        og[j] = d * uu * dsl * gmask;
-        ou[j] = d * sl * umask;
-      }
-      dg[i] = bf8_pack(og);
-      du[i] = bf8_pack(ou);
+      for (int j = 0; j < 4; ++j)
+        swiglu_bwd_pair<CLAMP>(reinterpret_cast<const uint32_t*>(&vg)[j], reinterpret_cast<const uint32_t*>(&vu)[j],
+                               reinterpret_cast<const uint32_t*>(&vd)[j], clamp, og[j], ou[j], oa[j]);
+      sg[i * 32] = make_uint4(og[0], og[1], og[2], og[3]);
+      su[i * 32] = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+      sd[i * 32] = make_uint4(oa[0], oa[1], oa[2], oa[3]);
     }
-    quantize_half<SCALE_BLOCK32, false, 4>(dg, h, pin + h * 32, 2 * I, q_row, q_col, &scales[0]);
-    quantize_half<SCALE_BLOCK32, false, 4>(du, h, pin + I + h * 32, 2 * I, q_row, q_col, &scales[1]);
+    uint4 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = sg[i * 32];
+    quantize_half<SCALE_BLOCK32, false, true>(v, h, o2, 2 * I, q_row, q_col, &scales[0], st);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = su[i * 32];
+    quantize_half<SCALE_BLOCK32, false, true>(v, h, o2 + I, 2 * I, q_row, q_col, &scales[1], st);
+    if (act_col) {
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[i] = sd[i * 32];
+      quantize_half(v, h, o1, I, nullptr, act_col, &scales[2], st);
+    }
   }
   store_scales(&scales[0], T, 2 * I, row0, col0, sf_row, sf_col);
   store_scales(&scales[1], T, 2 * I, row0, I + col0, sf_row, sf_col);
+  store_scales(&scales[2], T, I, row0, col0, nullptr, act_sf);
 }
 
 // value [R, C] fp8 + scales (operand layout with MN = R or C) -> fp32 [R, C]; test / debugging helper
@@ -569,22 +672,31 @@ int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row
   if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
   const dim3 grid(I / TILE, T / TILE);
   const bool wide = (long)grid.x * grid.y <= 148;
-  (wide ? swiglu_quant_mxfp8_kernel<true> : swiglu_quant_mxfp8_kernel<false>)<<<grid, wide ? 2 * QT : QT, 0, s>>>(
+  auto kern = clamp > 0.f ? (wide ? swiglu_quant_mxfp8_kernel<true, true> : swiglu_quant_mxfp8_kernel<false, true>)
+                          : (wide ? swiglu_quant_mxfp8_kernel<true, false> : swiglu_quant_mxfp8_kernel<false, false>);
+  kern<<<grid, wide ? 2 * QT : QT, 0, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
-// dh1 [T, 2I] = swiglu backward of (h1, dact) quantised to MXFP8 (outputs sized for [T, 2I]).
+// dh1 [T, 2I] = swiglu backward of (h1, dact) quantised to MXFP8 (outputs sized for [T, 2I]).  act_col / act_sf (null or both):
+// also the activation itself [T, I], quantised along T, as pb_swiglu_quant_mxfp8 gives it.
 int pb_swiglu_bwd_quant_mxfp8(const void* h1, const void* dact, int T, int I, float clamp, void* q_row, void* sf_row,
-                              void* q_col, void* sf_col, cudaStream_t s) {
-  if (T % TILE || I % TILE || T <= 0 || I <= 0) return -2;
+                              void* q_col, void* sf_col, void* act_col, void* act_sf, cudaStream_t s) {
+  if (T % TILE || I % TILE || T <= 0 || I <= 0 || !act_col != !act_sf) return -2;
   const dim3 grid(I / TILE, T / TILE);
   const bool wide = (long)grid.x * grid.y <= 148;
-  (wide ? swiglu_bwd_quant_mxfp8_kernel<true> : swiglu_bwd_quant_mxfp8_kernel<false>)<<<grid, wide ? 4 * QT : QT, 0, s>>>(
+  auto kern = clamp > 0.f ? (wide ? swiglu_bwd_quant_mxfp8_kernel<true, true> : swiglu_bwd_quant_mxfp8_kernel<false, true>)
+                          : (wide ? swiglu_bwd_quant_mxfp8_kernel<true, false> : swiglu_bwd_quant_mxfp8_kernel<false, false>);
+  const int smem = (wide ? 8 : 4) * BWD_WARP_BYTES;
+  static std::atomic<bool> allowed[4][pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, smem, allowed[wide + 2 * (clamp > 0.f)]);
+  if (rc) return rc;
+  kern<<<grid, wide ? 2 * QT : QT, smem, s>>>(
       reinterpret_cast<const __nv_bfloat16*>(h1), reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
       reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
-      reinterpret_cast<uint8_t*>(sf_col));
+      reinterpret_cast<uint8_t*>(sf_col), reinterpret_cast<uint8_t*>(act_col), reinterpret_cast<uint8_t*>(act_sf));
   return (int)cudaGetLastError();
 }
 

@@ -305,8 +305,9 @@ def swiglu_quantize_mxfp8(h1: torch.Tensor, clamp: float = 0.0, rowwise: bool = 
     return out
 
 
-def swiglu_bwd_quantize_mxfp8(h1: torch.Tensor, dact: torch.Tensor, clamp: float = 0.0) -> MXFP8Tensor:
-    """MXFP8 (both directions) of the SwiGLU input gradient ``[dgate | dup]`` [T, 2I] from ``h1`` and ``dact`` [T, I]."""
+def swiglu_bwd_quantize_mxfp8(h1: torch.Tensor, dact: torch.Tensor, clamp: float = 0.0, act: bool = False):
+    """MXFP8 (both directions) of the SwiGLU input gradient ``[dgate | dup]`` [T, 2I] from ``h1`` and ``dact`` [T, I].  ``act``:
+    returns (that, the activation itself quantised along T), which the same pass over ``h1`` gives."""
     T, I2 = h1.shape
     I = I2 // 2
     dev = h1.device
@@ -315,8 +316,13 @@ def swiglu_bwd_quantize_mxfp8(h1: torch.Tensor, dact: torch.Tensor, clamp: float
     out.sf_row = torch.empty(T * I2 // BLOCK, dtype=torch.uint8, device=dev)
     out.q_col = torch.empty(T, I2, dtype=torch.uint8, device=dev)
     out.sf_col = torch.empty(T * I2 // BLOCK, dtype=torch.uint8, device=dev)
-    _lib.call("swiglu_bwd_quant_mxfp8", h1, dact, T, I, float(clamp), out.q_row, out.sf_row, out.q_col, out.sf_col)
-    return out
+    a = MXFP8Tensor(shape=(T, I))
+    if act:
+        a.q_col = torch.empty(T, I, dtype=torch.uint8, device=dev)
+        a.sf_col = torch.empty(T * I // BLOCK, dtype=torch.uint8, device=dev)
+    _lib.call("swiglu_bwd_quant_mxfp8", h1, dact, T, I, float(clamp), out.q_row, out.sf_row, out.q_col, out.sf_col,
+              a.q_col, a.sf_col)
+    return (out, a) if act else out
 
 
 def dequantize_mxfp8(q: torch.Tensor, sf: torch.Tensor, colwise: bool) -> torch.Tensor:

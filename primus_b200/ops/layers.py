@@ -188,9 +188,24 @@ class SwiGLULinearFn(torch.autograd.Function):
             dyq_row = gemm._quantized(dout2, "row")           # quantises both directions once (backward pass)
             dyq_col = gemm._quantized(dout2, "col")
             w_ref = ctx.weight_ref
+            need_w = ctx.needs_input_grad[1]
+            wq, wsf = gemm._quantized(weight, "col")
+            dact = torch.empty(T, I, dtype=torch.bfloat16, device=x2.device)
+            fp8.launch_gemm(dyq_row[0], dyq_row[1], wq, wsf, dact, T, I, N, False, True, 0)
+            din = torch.empty_like(x2)
+            if ctx.grad_via_cache and gemm.WGRAD_STORE.current is None:   # (a deferred dW GEMM would outlive the cache entry)
+                # the gradient of h1 leaves as MXFP8 only: the bf16 tensor handed to autograd is a placeholder whose
+                # quantised copy is registered for the two GEMMs of the producing linear layer; the same pass over h1
+                # recomputes the activation for the weight gradient, column-wise
+                q = fp8.swiglu_bwd_quantize_mxfp8(x2, dact, ctx.clamp, act=need_w)
+                q, aq = q if need_w else (q, None)
+                gemm.register_quantized(din, q)
+            else:
+                _lib.call("swiglu_bwd", dact, x2, None, din, None, T, I, float(ctx.clamp), 0)
+                aq = fp8.swiglu_quantize_mxfp8(x2, ctx.clamp, False, True) if need_w else None
+            del dact
             dw = None
-            if ctx.needs_input_grad[1]:
-                aq = fp8.swiglu_quantize_mxfp8(x2, ctx.clamp, False, True)    # recomputed activation, col-wise
+            if need_w:
                 mg = getattr(w_ref, "main_grad", None)
                 tgt = mg if mg is not None else torch.empty(N, I, dtype=torch.float32, device=x2.device)
                 fp8.launch_gemm(dyq_col[0], dyq_col[1], aq.q_col, aq.sf_col, tgt, N, I, T, True, True,
@@ -202,17 +217,6 @@ class SwiGLULinearFn(torch.autograd.Function):
                     cb = getattr(w_ref, "_grad_ready_cb", None)
                     if cb is not None:
                         cb(w_ref)
-            wq, wsf = gemm._quantized(weight, "col")
-            dact = torch.empty(T, I, dtype=torch.bfloat16, device=x2.device)
-            fp8.launch_gemm(dyq_row[0], dyq_row[1], wq, wsf, dact, T, I, N, False, True, 0)
-            if ctx.grad_via_cache and gemm.WGRAD_STORE.current is None:   # (a deferred dW GEMM would outlive the cache entry)
-                # the gradient of h1 leaves as MXFP8 only: the bf16 tensor handed to autograd is a placeholder whose
-                # quantised copy is registered for the two GEMMs of the producing linear layer
-                din = torch.empty_like(x2)
-                gemm.register_quantized(din, fp8.swiglu_bwd_quantize_mxfp8(x2, dact, ctx.clamp))
-            else:
-                din = torch.empty_like(x2)
-                _lib.call("swiglu_bwd", dact, x2, None, din, None, T, I, float(ctx.clamp), 0)
             return din.view(ctx.shape), dw, None, None, None, None, None
         act = torch.empty(T, I, dtype=x2.dtype, device=x2.device)
         _lib.call("swiglu_fwd", x2, pp, act, T, I, float(ctx.clamp), ctx.kind)

@@ -49,3 +49,19 @@ def test_nan_blocks_of_the_fused_activations():
     act = torch.nn.functional.silu(gate) * up
     _check(fp8.swiglu_quantize_mxfp8(h1, rowwise=True, colwise=True), act)
     _check(fp8.swiglu_bwd_quantize_mxfp8(h1, dact), torch.cat([act, act], -1))
+
+
+@pytest.mark.parametrize("scaling", ["mxfp8", "mxfp4"])
+def test_scale_of_every_maximum(scaling):
+    """Block maxima of all bf16 magnitudes from zero over the subnormals to infinity, against the scale and bytes of the plain
+    formula, in both directions."""
+    g = torch.Generator().manual_seed(3)
+    bits = torch.arange(32768).clamp(max=0x7f80)
+    part = (bits[:, None] * torch.rand(32768, 32, generator=g)).long().clamp(max=0x7f7f)     # smaller in the order of the bits
+    part[:, 5] = bits
+    part |= torch.randint(0, 2, part.shape, generator=g) << 15
+    rows = torch.where(part > 32767, part - 65536, part).to(torch.int16).view(torch.bfloat16).view(1024, 1024)
+    for x, names in ((rows, ("q_row", "sf_row")), (rows.t().contiguous(), ("q_col", "sf_col"))):
+        got, want = fp8.quantize_mxfp8(x.cuda(), scaling=scaling), fp8.quantize_mxfp8_ref(x, scaling=scaling)
+        for n in names:
+            assert torch.equal(getattr(got, n).cpu(), getattr(want, n)), n
