@@ -138,16 +138,20 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 // dx = rstd * (dy*w) - x * rstd^3 * mean(dy*w*x)  (+ dres when given)
 // dx2 (optional) receives dx once more: first gradients of two leaves, which autograd would have to copy otherwise (a layer used
 // by itself; inside a model the two inputs are no leaves).  16384 x 8192: a second store 41 us, the copy 83 us.
+// y (optional) receives the normalised rows again, for the weight gradient of a linear layer that followed the norm and does not
+// store its input: x and rstd are here already, and a pass of its own reads x once more (8192 x 4096 with
+// residual: 54 + 31 us in two passes, 64 in one; 4096 x 2048 21 + 10 and 22).
 // dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
 
 // Rows of up to 1024 channels: LPR <= 32 lanes per row, no barrier in the loop, RPG rows per group in flight.  The dw
 // sums of a CTA's groups meet in shared memory at the end.
-template <int LPR, int VPL, int RPG>
+template <int LPR, int VPL, int RPG, bool Y>
 __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                          const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                         __nv_bfloat16* __restrict__ dx2, float* __restrict__ partial, long rows, int H, long ldx, long lddy) {
+                         __nv_bfloat16* __restrict__ dx2, __nv_bfloat16* __restrict__ y, float* __restrict__ partial, long rows,
+                         int H, long ldx, long lddy) {
   constexpr int GROUPS = 256 / LPR;
   __shared__ float4 sums[GROUPS][LPR * VPL * 2];
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
@@ -193,6 +197,11 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
             dw[k][j] += fg[j] * fx[j] * rs[r];
             dot += fg[j] * fw[j] * fx[j];
           }
+          if (Y) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) fw[j] = fx[j] * rs[r] * fw[j];
+            reinterpret_cast<Bf8*>(y + (row0 + r) * ldx)[lane + k * LPR] = f_to_bf8(fw);
+          }
         }
       dot = group_sum<LPR>(dot, nullptr);
       const float c = dot * rs[r] * rs[r] * rs[r] / H;
@@ -237,12 +246,13 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
 // of STAGES rows of its own vectors in shared memory, filled by its own 16-byte cp.async copies, so loads run several
 // rows ahead of the block reductions without holding registers; the reduction is the only barrier of a row (its slots
 // alternate).
-template <int VPT, int THREADS, bool RES>
+template <int VPT, int THREADS, bool RES, bool Y>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
-                   __nv_bfloat16* __restrict__ dx2, float* __restrict__ partial, long rows, int H, long ldx, long lddy, int stages) {
+                   __nv_bfloat16* __restrict__ dx2, __nv_bfloat16* __restrict__ y, float* __restrict__ partial, long rows, int H,
+                   long ldx, long lddy, int stages) {
   extern __shared__ __align__(16) uint8_t ring_raw[];
   __shared__ float red[2][THREADS / 32];
   constexpr int OPS = RES ? 3 : 2;
@@ -303,6 +313,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
           dw[k][j] += fg[j] * fx[j] * rs;
           dot += fg[j] * fw[j] * fx[j];
         }
+        if (Y) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) fw[j] = fx[j] * rs * fw[j];
+          reinterpret_cast<Bf8*>(y + row * ldx)[tid + k * THREADS] = f_to_bf8(fw);
+        }
       }
     dot = pb::warp_sum(dot);
     if ((tid & 31) == 0) red[flip][tid >> 5] = dot;
@@ -358,34 +373,36 @@ inline int bwd_ctas(int P, long rows, int H) {
   return (int)(n < P ? n : P);
 }
 
-template <int VPT, int THREADS, bool RES>
+template <int VPT, int THREADS, bool RES, bool Y>
 int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
                             const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, __nv_bfloat16* dx2,
-                            float* partial, long rows, int H, long ldx, long lddy) {
+                            __nv_bfloat16* y, float* partial, long rows, int H, long ldx, long lddy) {
   constexpr int STAGE = (RES ? 3 : 2) * VPT * THREADS * 16;
   // four rows ahead where two CTAs of an SM then still fit into its shared memory, else two
   constexpr int STAGES = 4 * STAGE <= 100 * 1024 ? 4 : 2;
-  auto kern = rmsnorm_bwd_kernel<VPT, THREADS, RES>;
+  auto kern = rmsnorm_bwd_kernel<VPT, THREADS, RES, Y>;
   static std::atomic<bool> allowed[pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, STAGES * STAGE, allowed);
   if (rc) return rc;
-  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy, STAGES);
+  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy, STAGES);
   return (int)cudaGetLastError();
 }
 
 int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __nv_bfloat16* x, const __nv_bfloat16* w,
-                       const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, __nv_bfloat16* dx2, float* partial,
-                       long rows, int H, long ldx, long lddy) {
+                       const float* rstd, const __nv_bfloat16* dres, __nv_bfloat16* dx, __nv_bfloat16* dx2, __nv_bfloat16* y,
+                       float* partial, long rows, int H, long ldx, long lddy) {
   const int nv = H / 8;
-#define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                         \
-  {                                                                                                              \
-    rmsnorm_bwd_short_kernel<LPR, VPL, RPG><<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, \
-                                                               lddy);                                            \
-    return (int)cudaGetLastError();                                                                              \
+#define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                               \
+  {                                                                                                                    \
+    auto kern = y ? rmsnorm_bwd_short_kernel<LPR, VPL, RPG, (LPR > 8)> : rmsnorm_bwd_short_kernel<LPR, VPL, RPG, false>; \
+    kern<<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy);                             \
+    return (int)cudaGetLastError();                                                                                    \
   }
-#define PB_NORM_BWD(VPT, THREADS)                                                                                     \
-  return dres ? launch_rmsnorm_bwd_ring<VPT, THREADS, true>(P, s, dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy) \
-              : launch_rmsnorm_bwd_ring<VPT, THREADS, false>(P, s, dy, x, w, rstd, dres, dx, dx2, partial, rows, H, ldx, lddy)
+#define PB_NORM_BWD_RING(VPT, THREADS, RES, Y) \
+  launch_rmsnorm_bwd_ring<VPT, THREADS, RES, Y>(P, s, dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy)
+#define PB_NORM_BWD(VPT, THREADS)                                                                                  \
+  return dres ? (y ? PB_NORM_BWD_RING(VPT, THREADS, true, true) : PB_NORM_BWD_RING(VPT, THREADS, true, false))     \
+              : (y ? PB_NORM_BWD_RING(VPT, THREADS, false, true) : PB_NORM_BWD_RING(VPT, THREADS, false, false))
   const bool few = rows * nv < 148 * 512L * 4;   // (two CTAs of 256 threads per SM)
   if (nv <= 8) { if (few) PB_NORM_BWD_SHORT(8, 1, 1) else PB_NORM_BWD_SHORT(8, 1, 4) }
   if (nv <= 16) { if (few) PB_NORM_BWD_SHORT(16, 1, 1) else PB_NORM_BWD_SHORT(16, 1, 4) }
@@ -399,6 +416,7 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
   if (nv <= 1024) PB_NORM_BWD(4, 256);
   PB_NORM_BWD(4, 512);
 #undef PB_NORM_BWD
+#undef PB_NORM_BWD_RING
 #undef PB_NORM_BWD_SHORT
 }
 
@@ -564,7 +582,7 @@ rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ 
 }
 
 int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
-                float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
+                void* y, float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
   if (rows == 0) {                                   // nothing to add; a stored sum of no rows is zero
     if (H == 0 || dw_accumulate == 1) return 0;
     P = 0;
@@ -572,8 +590,8 @@ int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float
     // every one of the partial rows is fully written by its CTA before the reduction reads it
     P = bwd_ctas(P, rows, H);
     const int rc = launch_rmsnorm_bwd(P, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, rstd,
-                                      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, scratch, rows, H,
-                                      ldx, lddy);
+                                      (const __nv_bfloat16*)dres, (__nv_bfloat16*)dx, (__nv_bfloat16*)dx2, (__nv_bfloat16*)y,
+                                      scratch, rows, H, ldx, lddy);
     if (rc) return rc;
   }
   rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, H, dw_accumulate);
@@ -601,7 +619,7 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
                    void* dx, float* dw, float* scratch, long rows, int H, long ldx, long lddy,
                    int dw_accumulate, cudaStream_t s) {
   if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L) return -2;
-  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, nullptr, dw, scratch, rows, H, ldx, lddy,
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, nullptr, nullptr, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
 
@@ -609,7 +627,16 @@ int pb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rs
 int pb_rmsnorm_bwd_two(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2,
                        float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
   if (H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || (rows && !dres)) return -2;
-  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, dw, scratch, rows, H, ldx, lddy,
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, nullptr, dw, scratch, rows, H, ldx,
+                     lddy, dw_accumulate, s);
+}
+
+// The same with y, the normalised rows x * rstd * w that the forward pass gave (pitch ldx; rows of more than 64 channels); dx2 may
+// be null.
+int pb_rmsnorm_bwd_y(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx, void* dx2, void* y,
+                     float* dw, float* scratch, long rows, int H, long ldx, long lddy, int dw_accumulate, cudaStream_t s) {
+  if (H <= 64 || H % 8 || ldx % 8 || lddy % 8 || H > 16384 || rows < 0 || rows > 2147483647L || (rows && dx2 && !dres)) return -2;
+  return rmsnorm_bwd(pb_rmsnorm_bwd_num_partials(rows), dy, x, w, rstd, dres, dx, dx2, y, dw, scratch, rows, H, ldx, lddy,
                      dw_accumulate, s);
 }
 
@@ -691,5 +718,5 @@ extern "C" int pb_rmsnorm_bwd_noalloc(const void* dy, const void* x, const void*
     g_noalloc_scratch_ptr[dev] = p;
   }
   const int P = (int)(rows < PB_NOALLOC_MAX_PARTIALS ? rows : PB_NOALLOC_MAX_PARTIALS);
-  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, nullptr, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate != 0, s);
+  return rmsnorm_bwd(P, dy, x, w, rstd, dres, dx, nullptr, nullptr, dw, g_noalloc_scratch_ptr[dev], rows, H, ldx, lddy, dw_accumulate != 0, s);
 }

@@ -116,10 +116,10 @@ def norm_inputs(x, residual):
     return (x2 if x2.stride(1) == 1 and x2.data_ptr() % 16 == 0 else dense_rows(x2)), None
 
 
-def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape):
+def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape, y=None):
     """(dx, the residual's gradient, dw or None when it was added to ``main_grad``).  dx is shared unless ``two`` (with ``dres``
     only), and then one tensor object: autograd takes a gradient that nobody else holds for a leaf's own without a copy, and
-    would take two views of the same memory for two leaves."""
+    would take two views of the same memory for two leaves.  ``y`` [rows, H]: receives the forward's normalised rows."""
     xin = xin.contiguous()                      # (the kernel has a single pitch for x, dres and dx)
     rows, H = xin.shape
     dx = torch.empty_like(xin)
@@ -130,7 +130,12 @@ def norm_backward(dy, xin, w, rstd, dres, main_grad, two, shape):
         target, mode = torch.empty(H, dtype=w.dtype, device=xin.device), 2
     else:
         target, mode = torch.empty(H, dtype=torch.float32, device=xin.device), 0
-    if two:
+    if y is not None:
+        dx2 = torch.empty_like(dx) if two else None
+        _lib.call("rmsnorm_bwd_y", dy, xin, w, rstd, dres, dx, dx2, y, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
+        dx = as_shape(dx, shape)
+        dx2 = as_shape(dx2, shape) if two else dx
+    elif two:
         dx2 = torch.empty_like(dx)
         _lib.call("rmsnorm_bwd_two", dy, xin, w, rstd, dres, dx, dx2, target, sc, rows, H, xin.stride(0), dy.stride(0), mode)
         dx, dx2 = as_shape(dx, shape), as_shape(dx2, shape)

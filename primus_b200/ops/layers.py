@@ -66,17 +66,22 @@ class NormLinearFn(torch.autograd.Function):
         dout2 = dout.reshape(-1, dout.shape[-1])
         if not dout2.is_contiguous():
             dout2 = dout2.contiguous()
-        # recompute the normalised activations (not stored in forward)
-        y = torch.empty_like(xsum)
-        _lib.call("rmsnorm_fwd", xsum, None, norm_w, y, None, None, rows, H, xsum.stride(0), y.stride(0),
-                  float(ctx.eps))
-        if sp:
-            if fused_tp._quantized_gather_ok(y, weight, False) and dout2.shape[1] % 128 == 0:
-                y = fused_tp.all_gather_quantized(y, tp_group, row=False, col=True)   # MXFP8: gather the quantised copy
-            else:
-                y = tp_comm.all_gather_dim0(y, tp_group)
-        dw = gemm.wgrad(dout2, y, weight_ref)
-        del y
+        # The normalised activations are not stored in forward.  The norm's backward pass reads all they are made of and writes
+        # them again, for the weight gradient after it; where they have to be gathered first, or for rows that its kernel for
+        # few channels takes, they are recomputed on their own.
+        fused_y = not sp and H > 64
+        y = torch.empty(rows, H, dtype=xsum.dtype, device=xsum.device) if fused_y else torch.empty_like(xsum)
+        dw = None
+        if not fused_y:
+            _lib.call("rmsnorm_fwd", xsum, None, norm_w, y, None, None, rows, H, xsum.stride(0), y.stride(0),
+                      float(ctx.eps))
+            if sp:
+                if fused_tp._quantized_gather_ok(y, weight, False) and dout2.shape[1] % 128 == 0:
+                    y = fused_tp.all_gather_quantized(y, tp_group, row=False, col=True)   # MXFP8: gather the quantised copy
+                else:
+                    y = tp_comm.all_gather_dim0(y, tp_group)
+            dw = gemm.wgrad(dout2, y, weight_ref)
+            del y
         if sp:
             dy = fused_tp.gemm_rs(dout2, weight, tp_group, b_mn=True, fused=fused_tp.ENABLED_RS)
         else:
@@ -85,7 +90,9 @@ class NormLinearFn(torch.autograd.Function):
                 torch.distributed.all_reduce(dy, group=tp_group)
         dres = None if dxsum is None else fused.dense_rows(fused.as_rows(dxsum, H))
         dx, dx2, dnw = fused.norm_backward(dy, xsum, norm_w, rstd, dres, getattr(norm_w_ref, "main_grad", None),
-                                            dres is not None and fused.two_leaves(ctx, 0, 1), ctx.shape)
+                                            dres is not None and fused.two_leaves(ctx, 0, 1), ctx.shape, y if fused_y else None)
+        if fused_y:
+            dw = gemm.wgrad(dout2, y, weight_ref)
         return dx, (dx2 if ctx.has_res else None), dnw, dw, None, None, None
 
 

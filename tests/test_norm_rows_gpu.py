@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from primus_b200.ops import fused, layers
+from primus_b200.ops import _lib, fused, layers
 
 from .test_kernel_edges_gpu import _close_bf16, _gen, _rms64
 
@@ -93,3 +93,23 @@ def test_gain_gradient_of_no_rows_is_zero(H):
         y, s = fused.rmsnorm(x, p, 1e-5, r)
         torch.autograd.backward([y, s], [torch.ones_like(y), torch.ones_like(s)])
         assert p.grad.shape == (H,) and not p.grad.any() and x.grad.shape == (0, H)
+
+
+@pytest.mark.parametrize("rows, H", [(1, 72), (37, 128), (700, 520), (129, 1024), (3000, 1024), (200, 2048), (33, 4104), (40, 8192),
+                                     (5, 16384)])
+@pytest.mark.parametrize("residual, two", [(False, False), (True, False), (True, True)])
+def test_backward_gives_the_normalised_rows_again(rows, H, residual, two):
+    """With ``y`` the backward writes what the forward wrote, and its gradients stay the same to the last bit."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    x, dy, ds = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(3))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+    y, rstd = torch.empty_like(x), torch.empty(rows, device="cuda")
+    _lib.call("rmsnorm_fwd", x, None, w, y, None, rstd, rows, H, H, H, 1e-5)
+    again = torch.full_like(x, float("nan"))
+    dres = ds if residual else None
+    got = fused.norm_backward(dy, x, w, rstd, dres, None, two, x.shape, again)
+    want = fused.norm_backward(dy, x, w, rstd, dres, None, two, x.shape)
+    assert torch.equal(again, y)
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
+    assert (got[0].data_ptr() != got[1].data_ptr()) == two
