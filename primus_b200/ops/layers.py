@@ -225,17 +225,15 @@ class SwiGLULinearFn(torch.autograd.Function):
                     if cb is not None:
                         cb(w_ref)
             return din.view(ctx.shape), dw, None, None, None, None, None
-        act = torch.empty(T, I, dtype=x2.dtype, device=x2.device)
-        _lib.call("swiglu_fwd", x2, pp, act, T, I, float(ctx.clamp), ctx.kind)
         if sp:
             dact, dout2 = fused_tp.ag_gemm(dout2, weight, tp_group, b_mn=True, fused=fused_tp.ENABLED, gather_col=True)
-            dw = gemm.wgrad(dout2, act, ctx.weight_ref)
         else:
-            dw = gemm.wgrad(dout2, act, ctx.weight_ref)
-            dact = gemm.gemm(dout2, weight, b_mn=True, out=act)  # reuse the activation buffer
+            dact = gemm.gemm(dout2, weight, b_mn=True)
         din = torch.empty_like(x2)
         dprobs = torch.empty(T, dtype=torch.float32, device=x2.device) if ctx.has_probs else None
-        _lib.call("swiglu_bwd", dact, x2, pp, din, dprobs, T, I, float(ctx.clamp), ctx.kind)
+        # the same pass recomputes the activation for the weight gradient, in the place of its own gradient
+        _lib.call("swiglu_bwd_act", dact, x2, pp, din, dprobs, dact, T, I, float(ctx.clamp), ctx.kind)
+        dw = gemm.wgrad(dout2, dact, ctx.weight_ref)
         dp = None
         if ctx.has_probs:
             shape, dt = ctx.probs_meta
