@@ -458,25 +458,54 @@ __global__ void adamw_kernel(float* __restrict__ master, StateT* __restrict__ m,
   }
 }
 
-// AdamW over one bucket in one launch.  The bucket is cut into ranges with their own weight-decay multiplier and learning
+// AdamW over up to ADAMW_SEGS buckets in one launch (between launches the SMs run empty, 4 us each: 126 M elements in four buckets
+// 587 us in four launches, 560 in one).  A bucket is cut into ranges with their own weight-decay multiplier and learning
 // rate (norm gains without decay between matrices with it: one launch per range left the SMs idle around every small one);
 // range r starts at starts[r] (element 0 first, all multiples of 4) and uses wd * mult[r] and lrs.v[group[r]].  A CTA takes
 // a contiguous chunk whose first range the host has looked up; its threads walk on from there, after their loads are issued.
-constexpr int ADAMW_CHUNK = 8192;
+// The chunks go from the last to the first: the gradients that the norm, just before, read last are still in L2.
+constexpr int ADAMW_CHUNK = 8192, ADAMW_SEGS = 32;
 struct AdamWRates {
   float v[4];
 };
+struct AdamWSeg {                       // a bucket; the first of its chunks in the launch
+  float* master;
+  void *m, *v;
+  const void* grad;
+  __nv_bfloat16* param_out;
+  long n;
+  const int* first;
+  const long* starts;
+  const float* mult;
+  const int* group;
+  int R;
+  unsigned chunk0;
+};
+struct AdamWSegs {
+  AdamWSeg seg[ADAMW_SEGS];
+  int count;
+};
 template <typename GradT, typename StateT>
 __global__ void __launch_bounds__(256, 5)
-adamw_ranges_kernel(float* __restrict__ master, StateT* __restrict__ m, StateT* __restrict__ v,
-                    const GradT* __restrict__ grad, __nv_bfloat16* __restrict__ param_out, long n,
-                    const int* __restrict__ first, const long* __restrict__ starts, const float* __restrict__ mult,
-                    const int* __restrict__ group, int R, AdamWRates lrs, float beta1, float beta2, float eps, float wd,
+adamw_ranges_kernel(const __grid_constant__ AdamWSegs segs, AdamWRates lrs, float beta1, float beta2, float eps, float wd,
                     float bc1, float bc2, float ic1, float ic2, const float* __restrict__ grad_scale,
                     const int* __restrict__ skip) {
   if (skip && *skip) return;
-  const long c0 = (long)blockIdx.x * ADAMW_CHUNK, c1 = min(n, c0 + ADAMW_CHUNK);
-  int r = first[blockIdx.x];
+  const unsigned chunk = gridDim.x - 1 - blockIdx.x;
+  int k = segs.count - 1;
+  while (segs.seg[k].chunk0 > chunk) --k;
+  const AdamWSeg& sg = segs.seg[k];
+  float* __restrict__ master = sg.master;
+  StateT *__restrict__ m = (StateT*)sg.m, *__restrict__ v = (StateT*)sg.v;
+  const GradT* __restrict__ grad = (const GradT*)sg.grad;
+  __nv_bfloat16* __restrict__ param_out = sg.param_out;
+  const long n = sg.n;
+  const long* __restrict__ starts = sg.starts;
+  const float* __restrict__ mult = sg.mult;
+  const int* __restrict__ group = sg.group;
+  const int R = sg.R;
+  const long c0 = (long)(chunk - sg.chunk0) * ADAMW_CHUNK, c1 = min(n, c0 + ADAMW_CHUNK);
+  int r = sg.first[chunk - sg.chunk0];
   const float gs = grad_scale ? *grad_scale : 1.f;
   long end = r + 1 < R ? starts[r + 1] : n;
   float lr = lrs.v[group[r]], rwd = wd * mult[r];
@@ -542,12 +571,20 @@ __device__ __forceinline__ void sumsq_unpack(const __nv_bfloat16* p, float (&f)[
   bf8_to_f(*reinterpret_cast<const Bf8*>(p), f);
 }
 
+constexpr int SUMSQ_SEGS = 32;
+struct SumsqSegs {                      // tensors of one launch: SUMSQ_BLOCKS blocks and partial sums each
+  const void* x[SUMSQ_SEGS];
+  long n[SUMSQ_SEGS];
+};
+
 template <typename T, bool ALIGNED>
 __global__ void __launch_bounds__(SUMSQ_BLOCK_CHAINS * sizeof(T) / 16)
-sumsq_partial_kernel(const T* __restrict__ x, long n, float* __restrict__ partial) {
+sumsq_partial_kernel(const __grid_constant__ SumsqSegs segs, float* __restrict__ partial) {
   constexpr int PER = 16 / sizeof(T), THREADS = SUMSQ_BLOCK_CHAINS / PER, LANES = 32 / PER, U = 8;
   __shared__ float red[16];
-  const long j0 = (long)blockIdx.x * SUMSQ_BLOCK_CHAINS + threadIdx.x * PER;
+  const T* __restrict__ x = (const T*)segs.x[blockIdx.x / SUMSQ_BLOCKS];
+  const long n = segs.n[blockIdx.x / SUMSQ_BLOCKS];
+  const long j0 = (long)(blockIdx.x % SUMSQ_BLOCKS) * SUMSQ_BLOCK_CHAINS + threadIdx.x * PER;
   float s[PER] = {};
   long i = j0;
   if (ALIGNED) {
@@ -590,31 +627,61 @@ sumsq_partial_kernel(const T* __restrict__ x, long n, float* __restrict__ partia
     if (threadIdx.x == 0) partial[blockIdx.x] = r;
   }
 }
-// out[0] (+)= sum(partial); nonfinite[0] |= !isfinite(sum)
-__global__ void __launch_bounds__(512) sumsq_final_kernel(const float* __restrict__ partial, int P,
-                                                         float* __restrict__ out, int accumulate,
-                                                         int* __restrict__ nonfinite) {
-  __shared__ float red[32];
-  float s = 0.f;
-  for (int i = threadIdx.x; i < P; i += blockDim.x) s += partial[i];
-  s = block_sum<512>(s, red);
-  if (threadIdx.x == 0) {
-    const float r = accumulate ? out[0] + s : s;
-    out[0] = r;
-    if (nonfinite && !isfinite(r)) *nonfinite = 1;
-  }
-}
 // coef = min(1, max_norm / (sqrt(sumsq) + 1e-6)) * extra
 // skip (optional): set to whether the step is left out, because the sum is not finite (check) or above `spike` (if positive).
-// In this kernel because as operations of their own the checks are eight launches for one number.
-__global__ void clip_coef_kernel(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out, int* skip,
-                                 int check, float spike) {
-  const float nrm = sqrtf(sumsq[0]);
-  if (skip) skip[0] = (check && !isfinite(sumsq[0])) || (spike > 0.f && sumsq[0] > spike);
-  if (norm_out) norm_out[0] = nrm;
+// In a kernel because as operations of their own the checks are eight launches for one number.
+struct ClipArgs {
+  float max_norm, extra;
+  float *coef, *norm_out;
+  int *skip, check;
+  float spike;
+};
+__device__ __forceinline__ void clip_coef(float sumsq, const ClipArgs& a) {
+  const float nrm = sqrtf(sumsq);
+  if (a.skip) a.skip[0] = (a.check && !isfinite(sumsq)) || (a.spike > 0.f && sumsq > a.spike);
+  if (a.norm_out) a.norm_out[0] = nrm;
   float c = 1.f;
-  if (max_norm > 0.f) c = fminf(1.f, max_norm / (nrm + 1e-6f));
-  coef[0] = c * extra;
+  if (a.max_norm > 0.f) c = fminf(1.f, a.max_norm / (nrm + 1e-6f));
+  a.coef[0] = c * a.extra;
+}
+__global__ void clip_coef_kernel(const float* sumsq, ClipArgs args) { clip_coef(sumsq[0], args); }
+
+// out[0] (+)= sum(partial) of each of `segs` tensors in turn; nonfinite[0] |= !isfinite(sum); with args.coef the clip
+// coefficient of that sum, where nothing else is to be added to it.
+__global__ void __launch_bounds__(512) sumsq_final_kernel(const float* __restrict__ partial, int segs,
+                                                         float* __restrict__ out, int accumulate,
+                                                         int* __restrict__ nonfinite, ClipArgs args) {
+  constexpr int B = 4;                  // tensors at a time
+  __shared__ float red[B][16], total[B];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float r = accumulate && threadIdx.x == 0 ? out[0] : 0.f;
+  for (int k0 = 0; k0 < segs; k0 += B) {
+    float s[B];
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      s[k] = 0.f;
+      if (k0 + k < segs)
+        for (int i = threadIdx.x; i < SUMSQ_BLOCKS; i += 512) s[k] += partial[(long)(k0 + k) * SUMSQ_BLOCKS + i];
+    }
+#pragma unroll
+    for (int k = 0; k < B; ++k) {
+      s[k] = pb::warp_sum(s[k]);
+      if (lane == 0) red[k][warp] = s[k];
+    }
+    __syncthreads();
+    if (warp < B) {
+      const float t = pb::warp_sum(lane < 16 ? red[warp][lane] : 0.f);
+      if (lane == 0) total[warp] = t;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+      for (int k = 0; k < B && k0 + k < segs; ++k) r += total[k];
+  }
+  if (threadIdx.x == 0) {
+    out[0] = r;
+    if (nonfinite && !isfinite(r)) *nonfinite = 1;
+    if (args.coef) clip_coef(r, args);
+  }
 }
 
 __global__ void scale_f32_kernel(float* __restrict__ x, long n, float s) {
@@ -770,29 +837,49 @@ int pb_adamw_ex(float* master, void* m, void* v, const void* grad, int grad_is_b
   PB_CHECK_LAUNCH();
 }
 
-// One bucket: ranges r = 0 .. R - 1 start at starts[r] (device, int64; starts[0] = 0, ascending multiples of 4) and use
-// weight decay wd * mult[r] and learning rate lr[group[r]] (four rates); first[c]: the range that element
-// c * pb_adamw_ranges_chunk() lies in.  param_out: bf16.
+// `count` buckets: bucket i is the eleven 64-bit values table[11 i ..] (host memory), addresses of master, m, v, grad, param_out
+// (bf16), then n, addresses of first, starts, mult and group, and R.  Its ranges r = 0 .. R - 1 start at starts[r] (device, int64;
+// starts[0] = 0, ascending multiples of 4) and use weight decay wd * mult[r] and learning rate lr[group[r]]; first[c]: the range
+// that element c * pb_adamw_ranges_chunk() lies in.  hyper (host): four learning rates, beta1, beta2, eps, wd, and the two bias
+// corrections.
 int pb_adamw_ranges_chunk() { return ADAMW_CHUNK; }
 
-int pb_adamw_ranges(float* master, void* m, void* v, const void* grad, int grad_is_bf16, int state_is_bf16,
-                    void* param_out, long n, const int* first, const long* starts, const float* mult, const int* group, int R, float lr0,
-                    float lr1, float lr2, float lr3, float beta1, float beta2, float eps, float wd, float bc1, float bc2,
+int pb_adamw_ranges(const long* table, int count, const float* hyper, int grad_is_bf16, int state_is_bf16,
                     const float* grad_scale, const int* skip, cudaStream_t s) {
-  if (n == 0) return 0;
-  if (R <= 0 || param_out == nullptr) return -2;
-  const AdamWRates lrs{{lr0, lr1, lr2, lr3}};
-  const unsigned g = (unsigned)((n + ADAMW_CHUNK - 1) / ADAMW_CHUNK);
-  __nv_bfloat16* po = (__nv_bfloat16*)param_out;
+  for (int i = 0; i < count; ++i)
+    if (table[11 * i + 5] < 0 || (table[11 * i + 5] && (table[11 * i + 10] <= 0 || !table[11 * i + 4]))) return -2;
+  const AdamWRates lrs{{hyper[0], hyper[1], hyper[2], hyper[3]}};
+  const float beta1 = hyper[4], beta2 = hyper[5], eps = hyper[6], wd = hyper[7], bc1 = hyper[8], bc2 = hyper[9];
+  for (int i = 0; i < count;) {
+    AdamWSegs segs;
+    segs.count = 0;
+    long chunks = 0;
+    for (; i < count && segs.count < ADAMW_SEGS; ++i) {
+      const long* t = table + 11 * i;
+      if (t[5] == 0) continue;
+      const long add = (t[5] + ADAMW_CHUNK - 1) / ADAMW_CHUNK;
+      if (chunks + add > 2147483647L) break;
+      segs.seg[segs.count++] = AdamWSeg{(float*)t[0], (void*)t[1], (void*)t[2], (const void*)t[3], (__nv_bfloat16*)t[4], t[5],
+                                        (const int*)t[6], (const long*)t[7], (const float*)t[8], (const int*)t[9], (int)t[10],
+                                        (unsigned)chunks};
+      chunks += add;
+    }
+    if (chunks == 0) {
+      if (i < count) return -2;                        // a bucket of more chunks than a grid has blocks
+      break;
+    }
 #define PB_ADAMW(GT, ST)                                                                                                  \
-  adamw_ranges_kernel<GT, ST><<<g, 256, 0, s>>>(master, (ST*)m, (ST*)v, (const GT*)grad, po, n, first, starts, mult, group, R, lrs, \
-                                                beta1, beta2, eps, wd, bc1, bc2, (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
-  if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
-  else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
-  else if (state_is_bf16) PB_ADAMW(float, __nv_bfloat16);
-  else PB_ADAMW(float, float);
+  adamw_ranges_kernel<GT, ST><<<(unsigned)chunks, 256, 0, s>>>(segs, lrs, beta1, beta2, eps, wd, bc1, bc2,               \
+                                                               (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
+    if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
+    else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
+    else if (state_is_bf16) PB_ADAMW(float, __nv_bfloat16);
+    else PB_ADAMW(float, float);
 #undef PB_ADAMW
-  PB_CHECK_LAUNCH();
+    const int rc = (int)cudaGetLastError();
+    if (rc) return rc;
+  }
+  return 0;
 }
 
 int pb_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf16, void* param_out,
@@ -804,23 +891,51 @@ int pb_adamw(float* master, float* m, float* v, const void* grad, int grad_is_bf
 
 int pb_sumsq_num_partials() { return SUMSQ_BLOCKS; }
 
+namespace {
+int sumsq_many(const long* table, int count, int is_bf16, float* scratch, float* out, int accumulate, int* nonfinite,
+               const ClipArgs& clip, cudaStream_t s) {
+  bool aligned = true;
+  for (int i = 0; i < count; ++i) aligned = aligned && table[2 * i] % 16 == 0;
+  for (int i = 0; i < count; i += SUMSQ_SEGS) {
+    SumsqSegs segs;
+    const int n = count - i < SUMSQ_SEGS ? count - i : SUMSQ_SEGS;
+    for (int k = 0; k < n; ++k) {
+      segs.x[k] = (const void*)table[2 * (i + k)];
+      segs.n[k] = table[2 * (i + k) + 1];
+    }
+#define PB_SUMSQ(T, A) \
+  sumsq_partial_kernel<T, A><<<n * SUMSQ_BLOCKS, SUMSQ_BLOCK_CHAINS * sizeof(T) / 16, 0, s>>>(segs, scratch + (long)i * SUMSQ_BLOCKS)
+    if (is_bf16) { if (aligned) PB_SUMSQ(__nv_bfloat16, true); else PB_SUMSQ(__nv_bfloat16, false); }
+    else { if (aligned) PB_SUMSQ(float, true); else PB_SUMSQ(float, false); }
+#undef PB_SUMSQ
+    const int rc = (int)cudaGetLastError();
+    if (rc) return rc;
+  }
+  sumsq_final_kernel<<<1, 512, 0, s>>>(scratch, count, out, accumulate, nonfinite, clip);
+  return (int)cudaGetLastError();
+}
+}  // namespace
+
 // out[0] (+)= sum(x^2). scratch: fp32 [pb_sumsq_num_partials()].
 int pb_sumsq(const void* x, int is_bf16, long n, float* scratch, float* out, int accumulate,
              int* nonfinite, cudaStream_t s) {
-  const int P = pb_sumsq_num_partials();
-  const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
-#define PB_SUMSQ(T, A) \
-  sumsq_partial_kernel<T, A><<<P, SUMSQ_BLOCK_CHAINS * sizeof(T) / 16, 0, s>>>((const T*)x, n, scratch)
-  if (is_bf16) { if (aligned) PB_SUMSQ(__nv_bfloat16, true); else PB_SUMSQ(__nv_bfloat16, false); }
-  else { if (aligned) PB_SUMSQ(float, true); else PB_SUMSQ(float, false); }
-#undef PB_SUMSQ
-  sumsq_final_kernel<<<1, 512, 0, s>>>(scratch, P, out, accumulate, nonfinite);
-  PB_CHECK_LAUNCH();
+  const long table[2] = {(long)x, n};
+  return sumsq_many(table, 1, is_bf16, scratch, out, accumulate, nonfinite, ClipArgs{}, s);
+}
+
+// out[0] (+)= the sums of squares of `count` tensors of one type, added in turn as by as many pb_sumsq calls; table (host): address
+// and number of elements of each.  scratch: fp32 [count, pb_sumsq_num_partials()].  coef (or null): then what pb_clip_coef
+// gives for out[0].  (126 M fp32 values in four tensors: 99 + 12 us in eight launches and two more for the coefficient, 88 + 6 in two.)
+int pb_grad_norm(const long* table, int count, int is_bf16, float* scratch, float* out, int accumulate, float max_norm, float extra,
+                 float* coef, float* norm_out, int* skip, int check, float spike, cudaStream_t s) {
+  if (count <= 0) return -2;
+  return sumsq_many(table, count, is_bf16, scratch, out, accumulate, nullptr,
+                    ClipArgs{max_norm, extra, coef, norm_out, skip, check, spike}, s);
 }
 
 int pb_clip_coef(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out, int* skip, int check,
                  float spike, cudaStream_t s) {
-  clip_coef_kernel<<<1, 1, 0, s>>>(sumsq, max_norm, extra, coef, norm_out, skip, check, spike);
+  clip_coef_kernel<<<1, 1, 0, s>>>(sumsq, ClipArgs{max_norm, extra, coef, norm_out, skip, check, spike});
   PB_CHECK_LAUNCH();
 }
 

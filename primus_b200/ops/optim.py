@@ -8,6 +8,8 @@ trainer_base.yaml:72-118).
 """
 from __future__ import annotations
 
+import struct
+
 import numpy as np
 import torch
 
@@ -64,18 +66,28 @@ def range_table(ranges, start: int, n: int, device):
     return t[4 * R:], t[:2 * R].view(torch.int64), t[2 * R:3 * R].view(torch.float32), t[3 * R:4 * R]
 
 
-def adamw_ranges_(master, exp_avg, exp_avg_sq, grad, param_out, table, *, lrs, beta1, beta2, eps, weight_decay, step,
-                  grad_scale=None, skip=None):
-    """:func:`adamw_step_` of a whole bucket whose ranges differ in weight decay and learning rate, in one launch (CUDA
-    tensors, bf16 ``param_out``).  ``table``: see :func:`range_table`; ``lrs``: the rates of groups 0 to 3."""
-    n = master.numel()
-    assert master.dtype == torch.float32 and master.is_contiguous() and master.data_ptr() % 16 == 0
-    assert grad.numel() == n and grad.is_contiguous() and exp_avg.dtype == exp_avg_sq.dtype
-    assert param_out.dtype == torch.bfloat16 and param_out.numel() == n and len(lrs) == 4
-    _lib.call("adamw_ranges", master, exp_avg, exp_avg_sq, grad, int(grad.dtype == torch.bfloat16),
-              int(exp_avg.dtype == torch.bfloat16), param_out, n, *table, table[1].numel(), *[float(x) for x in lrs],
-              float(beta1), float(beta2), float(eps), float(weight_decay), float(1.0 - beta1 ** step),
-              float(1.0 - beta2 ** step), grad_scale, skip)
+def adamw_ranges_(master, exp_avg, exp_avg_sq, grad, param_out, table, **hyper):
+    """:func:`adamw_step_` of a whole bucket whose ranges differ in weight decay and learning rate (CUDA tensors, bf16
+    ``param_out``).  ``table``: see :func:`range_table`; ``lrs``: the rates of groups 0 to 3."""
+    adamw_buckets_([(master, exp_avg, exp_avg_sq, grad, param_out, table)], **hyper)
+
+
+def adamw_buckets_(buckets, *, lrs, beta1, beta2, eps, weight_decay, step, grad_scale=None, skip=None):
+    """:func:`adamw_ranges_` of several buckets ``(master, exp_avg, exp_avg_sq, grad, param_out, table)``, gradients of one type
+    and moments of one type, in one launch."""
+    rows = []
+    g0, m0 = buckets[0][3], buckets[0][1]
+    for master, m, v, grad, out, (first, starts, mult, group) in buckets:
+        n = master.numel()
+        assert master.dtype == torch.float32 and master.is_contiguous() and master.data_ptr() % 16 == 0
+        assert grad.numel() == n and grad.is_contiguous() and grad.dtype == g0.dtype
+        assert m.dtype == v.dtype == m0.dtype and out.dtype == torch.bfloat16 and out.numel() == n
+        rows += [master.data_ptr(), m.data_ptr(), v.data_ptr(), grad.data_ptr(), out.data_ptr(), n, first.data_ptr(),
+                 starts.data_ptr(), mult.data_ptr(), group.data_ptr(), starts.numel()]
+    assert len(lrs) == 4
+    hyper = struct.pack("10f", *lrs, beta1, beta2, eps, weight_decay, 1.0 - beta1 ** step, 1.0 - beta2 ** step)
+    _lib.call("adamw_ranges", struct.pack(f"{len(rows)}q", *rows), len(buckets), hyper, int(g0.dtype == torch.bfloat16),
+              int(m0.dtype == torch.bfloat16), grad_scale, skip)
 
 
 def sumsq_(x, out, accumulate=False, nonfinite=None):
@@ -90,6 +102,27 @@ def sumsq_(x, out, accumulate=False, nonfinite=None):
     P = _lib.call_ret("sumsq_num_partials")
     sc = scratch(x.device, "sumsq", P)
     _lib.call("sumsq", x, int(x.dtype == torch.bfloat16), x.numel(), sc, out, int(accumulate), nonfinite)
+    return out
+
+
+def grad_norm_(xs, out, accumulate=False, clip=None):
+    """out[0] (+)= the sums of squares of the tensors ``xs``, added in turn; with ``clip``, the arguments of :func:`clip_coef_` after
+    the sum, also the clip coefficient of the result.  CUDA tensors of one type take two launches in all."""
+    if not xs or not xs[0].is_cuda or any(x.dtype != xs[0].dtype for x in xs):
+        if not accumulate:
+            out.zero_()
+        for x in xs:
+            sumsq_(x, out, accumulate=True)
+        if clip is not None:
+            clip_coef_(out, **clip)
+        return out
+    assert all(x.is_contiguous() for x in xs)
+    sc = scratch(xs[0].device, "sumsq", len(xs) * _lib.call_ret("sumsq_num_partials"))
+    c = clip or {}
+    table = struct.pack(f"{2 * len(xs)}q", *[v for x in xs for v in (x.data_ptr(), x.numel())])
+    _lib.call("grad_norm", table, len(xs), int(xs[0].dtype == torch.bfloat16), sc, out, int(accumulate),
+              float(c.get("max_norm", 0.0)), float(c.get("extra", 1.0)), c.get("coef"), c.get("norm_out"), c.get("skip"),
+              int(c.get("check_finite", False)), float(c.get("spike", 0.0)))
     return out
 
 

@@ -471,9 +471,15 @@ class DistributedOptimizer:
                 out.append((lo, hi))
         return sorted(out)
 
+    def _has_tp_duplicates(self) -> bool:
+        return self.tp_size > 1 and any(st["dup_ranges"] for st in self.state)
+
+    def _dp_reduces(self) -> bool:
+        return self.buffers[0].dp_size > 1 and self.buffers[0].use_distributed_optimizer
+
     def _discount_tp_duplicates(self):
         """sumsq -= (tp - 1) / tp * (squared sum of the tensor-parallel duplicates in the local shards)."""
-        if self.tp_size == 1 or not any(st["dup_ranges"] for st in self.state):
+        if not self._has_tp_duplicates():
             return
         self.sumsq_part.zero_()
         for st in self.state:
@@ -483,7 +489,7 @@ class DistributedOptimizer:
 
     def _reduce_sumsq(self):
         """Adds the squared sums over the ranks that hold disjoint parts of the gradients."""
-        if self.buffers[0].dp_size > 1 and self.buffers[0].use_distributed_optimizer:
+        if self._dp_reduces():
             dist.all_reduce(self.sumsq, group=self.buffers[0].dp_group)
         for g in self.norm_groups:
             dist.all_reduce(self.sumsq, group=g)
@@ -491,7 +497,6 @@ class DistributedOptimizer:
     # ------------------------------------------------------------------
     def compute_grad_norm(self):
         """Global L2 norm of the (already reduced) gradients, left on the device."""
-        self.sumsq.zero_()
         if self.sanitize_grads:
             # non-finite gradient entries become zero before the norm and the non-finite check see them: the affected
             # elements simply get no update this step (the reference's SFT gradient sanitiser,
@@ -502,13 +507,17 @@ class DistributedOptimizer:
                 torch.nan_to_num_(g, nan=0.0, posinf=0.0, neginf=0.0)
         expert_sep = self.expert_norm_group is not None and any(
             not st["buf"].use_distributed_optimizer and self._is_expert_buffer(st["buf"]) for st in self.state)
-        if expert_sep:
-            self.sumsq_part.zero_()
+        grads, experts = [], []
         for st in self.state:
             g = st["buf"].grad_data[st["s"]:st["e"]]
             sep = expert_sep and not st["buf"].use_distributed_optimizer and self._is_expert_buffer(st["buf"])
-            optim_ops.sumsq_(g, self.sumsq_part if sep else self.sumsq, accumulate=True)
+            (experts if sep else grads).append(g)
+        alone = not (expert_sep or self.norm_groups or self._dp_reduces() or self._has_tp_duplicates())
+        optim_ops.grad_norm_(grads, self.sumsq, clip=self._clip_args(self.grad_spike_threshold) if alone else None)
+        if alone:
+            return self.grad_norm
         if expert_sep:
+            optim_ops.grad_norm_(experts, self.sumsq_part)
             dist.all_reduce(self.sumsq_part, group=self.expert_norm_group)
             self.sumsq.add_(self.sumsq_part)
         self._discount_tp_duplicates()
@@ -517,11 +526,14 @@ class DistributedOptimizer:
         self._clip_and_check(self.grad_spike_threshold)
         return self.grad_norm
 
+    def _clip_args(self, spike_threshold=None):
+        spike = float(spike_threshold) ** 2 if spike_threshold and spike_threshold > 0 else 0.0
+        return dict(max_norm=self.clip_grad if self.clip_grad else 0.0, coef=self.coef, norm_out=self.grad_norm, skip=self.skip,
+                    check_finite=bool(self.check_for_nan), spike=spike)
+
     def _clip_and_check(self, spike_threshold=None):
         """Clip coefficient and norm from the squared sum; ``skip`` = whether the step is left out."""
-        spike = float(spike_threshold) ** 2 if spike_threshold and spike_threshold > 0 else 0.0
-        optim_ops.clip_coef_(self.sumsq, self.clip_grad if self.clip_grad else 0.0, self.coef, self.grad_norm,
-                             skip=self.skip, check_finite=bool(self.check_for_nan), spike=spike)
+        optim_ops.clip_coef_(self.sumsq, **self._clip_args(spike_threshold))
 
     @staticmethod
     def _is_expert_buffer(buf) -> bool:
@@ -613,15 +625,20 @@ class DistributedOptimizer:
 
     def _apply_adamw(self, lr: float, wd: float):
         base_lr = lr
+        by_type: dict = {}       # buckets that one launch can take together
+        for st in self.state:
+            if st.get("range_table") is not None:
+                by_type.setdefault((st["buf"].grad_data.dtype, st["m"].dtype), []).append(st)
+        for sts in by_type.values():
+            optim_ops.adamw_buckets_([(st["master"], st["m"], st["v"], st["buf"].grad_data[st["s"]:st["e"]],
+                                       st["buf"].param_data[st["s"]:st["e"]], st["range_table"]) for st in sts],
+                                     lrs=[self._group_lr.get(g, base_lr) for g in range(4)], beta1=self.betas[0],
+                                     beta2=self.betas[1], eps=self.eps, weight_decay=wd, step=self.step_count,
+                                     grad_scale=self.coef, skip=self.skip)
         for st in self.state:
             buf = st["buf"]
             ranges = st["wd_ranges"]
             if st.get("range_table") is not None:
-                optim_ops.adamw_ranges_(st["master"], st["m"], st["v"], buf.grad_data[st["s"]:st["e"]],
-                                        buf.param_data[st["s"]:st["e"]], st["range_table"],
-                                        lrs=[self._group_lr.get(g, base_lr) for g in range(4)], beta1=self.betas[0],
-                                        beta2=self.betas[1], eps=self.eps, weight_decay=wd, step=self.step_count,
-                                        grad_scale=self.coef, skip=self.skip)
                 continue
             for lo, hi, mult, grp in ranges:
                 lr = self._group_lr.get(grp, base_lr)
