@@ -423,132 +423,295 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
 // ------------------------------------------------------------------ per-head norms of q and k in a packed QKV tensor
 // qkv [T, (hq + 2 hkv) * d] = [q heads | k heads | v heads]: every q and k head is normalised with its own gain (wq / wk),
 // v heads are copied, and the result is packed the same way, so that nothing is sliced, copied or concatenated around the
-// norms.  A group of LPR lanes owns a head row; RPG head rows of a group are in flight.
-template <int LPR, int RPG>
-__global__ void __launch_bounds__(128)
+// norms.  ROPE: the q and k heads are then rotated (rotate-half in their first rot_dim channels, as rope_kernel does it), which as
+// passes of its own reads and writes them once more in each direction.
+// A group of LPR lanes owns a head row and a lane two 16-byte vectors of it, those that rotate with one another: no exchange but
+// the row's sum, and the pair shares its table entries, which stay for the rows of one token that a group takes in turn.  (One
+// vector per lane, twice the shuffles and three times the instructions: 4096 x 32 / 4 x 128 forward with rotation 29 us, two
+// passes 39, this 23; backward 57, 64 and 50.)
+struct Rope {
+  const int* pos;                       // row of the tables, or null: the token's number
+  const float *cos_t, *sin_t;           // [positions, rot_dim / 2]
+  int rot_dim;
+};
+struct HeadLane {                       // a lane's two vectors of a head row of d channels
+  int a, b;
+  bool ina, inb, turns;
+  template <bool ROPE>
+  static __device__ __forceinline__ HeadLane make(int lane, int d, int rot_dim) {
+    const int nv = d / 8, half8 = ROPE ? rot_dim / 16 : (nv + 1) / 2;
+    HeadLane l;
+    l.turns = ROPE && lane < half8;
+    l.a = lane < half8 ? lane : 2 * half8 + 2 * (lane - half8);
+    l.b = lane < half8 ? lane + half8 : l.a + 1;
+    l.ina = l.a < nv;
+    l.inb = l.b < nv;
+    return l;
+  }
+};
+struct HeadRow {                        // a head row; stepping to the next costs no division
+  long t;
+  int h, heads;
+  __device__ __forceinline__ HeadRow(long row, int heads_) : heads(heads_) {
+    t = row >> 32 ? row / heads_ : (long)((unsigned)row / (unsigned)heads_);
+    h = (int)(row - t * heads_);
+  }
+  __device__ __forceinline__ void next() {
+    if (++h == heads) { h = 0; ++t; }
+  }
+};
+// the entries of token t for the lane's pair
+__device__ __forceinline__ void rope_entries(const Rope& rp, long t, int lane, float (&c)[8], float (&s)[8]) {
+  const long at = ((long)(rp.pos ? rp.pos[t] : (int)t) * (rp.rot_dim / 16) + lane) * 8;
+#pragma unroll
+  for (int j = 0; j < 8; j += 4) {
+    *reinterpret_cast<float4*>(c + j) = *reinterpret_cast<const float4*>(rp.cos_t + at + j);
+    *reinterpret_cast<float4*>(s + j) = *reinterpret_cast<const float4*>(rp.sin_t + at + j);
+  }
+}
+__device__ __forceinline__ void rope_pair(Bf8& a, Bf8& b, const float (&c)[8], const float (&s)[8], float sign) {
+  float fa[8], fb[8], oa[8], ob[8];
+  bf8_to_f(a, fa);
+  bf8_to_f(b, fb);
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float sn = s[j] * sign;
+    oa[j] = fa[j] * c[j] - fb[j] * sn;
+    ob[j] = fb[j] * c[j] + fa[j] * sn;
+  }
+  a = f_to_bf8(oa);
+  b = f_to_bf8(ob);
+}
+// Neighbouring head rows, mostly of one token, that a group takes in turn.  Forward, all loaded at once: two rows and 32 warps per SM
+// 16.7 us at 4096 x 32 / 4 x 128, four rows and 16 warps 18.9.
+constexpr int QK_FWD_RUN = 2, QK_RUN = 4;
+
+template <int LPR, bool ROPE>
+__global__ void __launch_bounds__(128, 8)
 qk_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq,
                    const __nv_bfloat16* __restrict__ wk, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
-                   long rows, int hq, int hkv, int d, long ldx, long ldy, float eps) {
+                   long rows, int hq, int hkv, int d, long ldx, long ldy, float eps, Rope rp) {
   const int lane = threadIdx.x % LPR;
-  const long row0 = (blockIdx.x * (long)(128 / LPR) + threadIdx.x / LPR) * RPG;
-  const int heads = hq + 2 * hkv;
-  const bool in = lane < d / 8;
-  Bf8 v[RPG], gq, gk;
-  if (in) {
-    gq = reinterpret_cast<const Bf8*>(wq)[lane];
-    gk = reinterpret_cast<const Bf8*>(wk)[lane];
+  const long row0 = (blockIdx.x * (long)(128 / LPR) + threadIdx.x / LPR) * QK_FWD_RUN;
+  const HeadLane l = HeadLane::make<ROPE>(lane, d, rp.rot_dim);
+  const HeadRow first(row0, hq + 2 * hkv);
+  Bf8 va[QK_FWD_RUN], vb[QK_FWD_RUN];
+  HeadRow at = first;
+  float c[8], s[8];
+  if (ROPE && row0 < rows && l.turns) rope_entries(rp, at.t, lane, c, s);
+#pragma unroll
+  for (int r = 0; r < QK_FWD_RUN; ++r, at.next()) {
+    const Bf8* src = reinterpret_cast<const Bf8*>(x + at.t * ldx + (long)at.h * d);
+    if (row0 + r < rows && l.ina) va[r] = src[l.a];
+    if (row0 + r < rows && l.inb) vb[r] = src[l.b];
   }
+  at = first;
 #pragma unroll
-  for (int r = 0; r < RPG; ++r) {
-    const long row = row0 + r;
-    if (row < rows && in) v[r] = reinterpret_cast<const Bf8*>(x + row / heads * ldx + row % heads * d)[lane];
-  }
+  for (int r = 0; r < QK_FWD_RUN; ++r, at.next()) {
+    const bool live = row0 + r < rows, norm = at.h < hq + hkv;
+    if (ROPE && live && l.turns && r > 0 && at.h == 0) rope_entries(rp, at.t, lane, c, s);
+    float f[8], g[8], sa = 0.f, sb = 0.f;
+    if (live && l.ina) {
+      bf8_to_f(va[r], f);
 #pragma unroll
-  for (int r = 0; r < RPG; ++r) {
-    const long row = row0 + r, t = row / heads;
-    const int h = (int)(row - t * heads);
-    const bool live = row < rows && in;
-    float f[8], ss = 0.f;
-    if (live) {
-      bf8_to_f(v[r], f);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      for (int j = 0; j < 8; ++j) sa += f[j] * f[j];
     }
-    const float rstd = rsqrtf(group_sum<LPR>(ss, nullptr) / d + eps);
+    if (live && l.inb) {
+      bf8_to_f(vb[r], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) sb += f[j] * f[j];
+    }
+    const float rstd = rsqrtf(group_sum<LPR>(sa + sb, nullptr) / d + eps);
     if (!live) continue;
-    if (h < hq + hkv) {
-      float g[8];
-      bf8_to_f(h < hq ? gq : gk, g);
+    if (norm) {
+      const Bf8* w = reinterpret_cast<const Bf8*>(at.h < hq ? wq : wk);
+      if (l.ina) {
+        bf8_to_f(va[r], f);
+        bf8_to_f(w[l.a], g);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
-      v[r] = f_to_bf8(f);
-      if (lane == 0) rstd_out[t * (hq + hkv) + h] = rstd;
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+        va[r] = f_to_bf8(f);
+      }
+      if (l.inb) {
+        bf8_to_f(vb[r], f);
+        bf8_to_f(w[l.b], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+        vb[r] = f_to_bf8(f);
+      }
+      if (ROPE && l.turns) rope_pair(va[r], vb[r], c, s, 1.f);
+      if (lane == 0) rstd_out[at.t * (hq + hkv) + at.h] = rstd;
     }
-    reinterpret_cast<Bf8*>(y + t * ldy + (long)h * d)[lane] = v[r];
+    Bf8* dst = reinterpret_cast<Bf8*>(y + at.t * ldy + (long)at.h * d);
+    if (l.ina) dst[l.a] = va[r];
+    if (l.inb) dst[l.b] = vb[r];
   }
 }
 
-// Backward: dx of the q and k heads, the v gradient copied; gain sums per CTA in partial [gridDim.x, 2 d] (q, then k).
-template <int LPR, int RPG>
+// (two fp32 values per instruction: channel j of the lane's two vectors, so that each vector's sums keep their order)
+struct Pairs {
+  uint64_t v[8];
+};
+__device__ __forceinline__ Pairs unpack_pairs(const Bf8& a, const Bf8& b) {
+  Pairs p;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const uint32_t wa = *reinterpret_cast<const uint32_t*>(&a.v[i]), wb = *reinterpret_cast<const uint32_t*>(&b.v[i]);
+    p.v[2 * i] = pb::pack_f32x2(__uint_as_float(wa << 16), __uint_as_float(wb << 16));
+    p.v[2 * i + 1] = pb::pack_f32x2(__uint_as_float(wa & 0xffff0000u), __uint_as_float(wb & 0xffff0000u));
+  }
+  return p;
+}
+__device__ __forceinline__ void pack_pairs(const Pairs& p, Bf8& a, Bf8& b) {
+  float fa[8], fb[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) pb::unpack_f32x2(p.v[j], fa[j], fb[j]);
+  a = f_to_bf8(fa);
+  b = f_to_bf8(fb);
+}
+// the gains of the lane's channels for q or k heads
+struct HeadGains {
+  Bf8 a, b;
+  bool of_q;
+  __device__ __forceinline__ void load(const __nv_bfloat16* wq, const __nv_bfloat16* wk, bool q, const HeadLane& l) {
+    const Bf8* w = reinterpret_cast<const Bf8*>(q ? wq : wk);
+    of_q = q;
+    if (l.ina) a = w[l.a];
+    if (l.inb) b = w[l.b];
+  }
+};
+
+// Backward: dx of the q and k heads (ROPE: of gradients that are rotated back first), the v gradient copied; gain sums per CTA
+// in partial [gridDim.x, 2 d] (q, then k).  A lane's copies of its vectors run QK_STAGES rows ahead, through slots of its own in
+// shared memory (registers for as many rows left two CTAs of 256 threads per SM waiting for memory most of the time), and the
+// arithmetic runs on pairs of values, which its issue is bound by.
+constexpr int QK_STAGES = 4;
+template <int LPR, bool ROPE>
 __global__ void __launch_bounds__(256, 2)
 qk_norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                    const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
                    const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, long rows,
-                   int hq, int hkv, int d, long ldx, long lddy, long lddx) {
+                   int hq, int hkv, int d, long ldx, long lddy, long lddx, Rope rp) {
   constexpr int GROUPS = 256 / LPR;
-  __shared__ float4 sums[GROUPS][LPR * 2];
+  extern __shared__ __align__(16) uint8_t ring_raw[];
+  Bf8* slots = reinterpret_cast<Bf8*>(ring_raw) + threadIdx.x;     // [stage][dy a, dy b, x a, x b][thread]
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
+  const HeadLane l = HeadLane::make<ROPE>(lane, d, rp.rot_dim);
   const int heads = hq + 2 * hkv;
-  const bool in = lane < d / 8;
-  Bf8 gq, gk;
-  float dw[2][8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) dw[0][j] = dw[1][j] = 0.f;
-  if (in) {
-    gq = reinterpret_cast<const Bf8*>(wq)[lane];
-    gk = reinterpret_cast<const Bf8*>(wk)[lane];
-  }
-  const long stride = (long)gridDim.x * GROUPS * RPG;
-  for (long base = (long)blockIdx.x * GROUPS * RPG; base < rows; base += stride) {
-    const long row0 = base + grp * RPG;
-    Bf8 vx[RPG], vg[RPG];
-    float rs[RPG];
-#pragma unroll
-    for (int r = 0; r < RPG; ++r) {
-      const long row = row0 + r, t = row / heads;
-      const int h = (int)(row - t * heads);
-      rs[r] = 0.f;
-      if (row < rows && in) {
-        vg[r] = reinterpret_cast<const Bf8*>(dy + t * lddy + (long)h * d)[lane];
-        if (h < hq + hkv) {
-          vx[r] = reinterpret_cast<const Bf8*>(x + t * ldx + (long)h * d)[lane];
-          rs[r] = rstd[t * (hq + hkv) + h];
-        }
+  const long runs = (rows + QK_RUN - 1) / QK_RUN, step = (long)gridDim.x * GROUPS;
+  Pairs dw[2] = {};                      // gain sums of the lane's channels: q heads, k heads
+
+  // the row after the last one fetched: run `frun`, `fr` rows into it
+  long frun = (long)blockIdx.x * GROUPS + grp;
+  int fr = 0;
+  HeadRow fat(frun * QK_RUN, heads);
+  auto fetch = [&](int st) {
+    if (frun < runs && frun * QK_RUN + fr < rows) {
+      Bf8* sl = slots + st * 4 * 256;
+      const Bf8* g = reinterpret_cast<const Bf8*>(dy + fat.t * lddy + (long)fat.h * d);
+      if (l.ina) pb::cp_async_16(sl, g + l.a);
+      if (l.inb) pb::cp_async_16(sl + 256, g + l.b);
+      if (fat.h < hq + hkv) {
+        const Bf8* v = reinterpret_cast<const Bf8*>(x + fat.t * ldx + (long)fat.h * d);
+        if (l.ina) pb::cp_async_16(sl + 512, v + l.a);
+        if (l.inb) pb::cp_async_16(sl + 768, v + l.b);
       }
     }
+    pb::cp_async_commit();               // also when empty: the wait below counts groups
+    fat.next();
+    if (++fr == QK_RUN) {
+      fr = 0;
+      frun += step;
+      fat = HeadRow(frun * QK_RUN, heads);
+    }
+  };
 #pragma unroll
-    for (int r = 0; r < RPG; ++r) {
-      const long row = row0 + r, t = row / heads;
-      const int h = (int)(row - t * heads);
-      const bool live = row < rows && in, norm = live && h < hq + hkv;
-      float fx[8], fg[8], dot = 0.f;
+  for (int st = 0; st < QK_STAGES; ++st) fetch(st);
+  HeadGains w{};
+  w.load(wq, wk, true, l);
+  // the loop bound is the CTA's first run: all lanes of a warp make the same number of turns (shuffles inside)
+  for (long base = (long)blockIdx.x * GROUPS; base < runs; base += step) {
+    const long row0 = (base + grp) * QK_RUN;
+    HeadRow at(row0, heads);
+    float c[8], s[8], rs_run[QK_RUN];
+    if (ROPE && row0 < rows && l.turns) rope_entries(rp, at.t, lane, c, s);
+#pragma unroll
+    for (int r = 0; r < QK_RUN; ++r) {
+      const int h = at.h + r < heads ? at.h + r : at.h + r - heads;          // (a run of more than two tokens: below)
+      const long t = at.h + r < heads ? at.t : at.t + 1;
+      rs_run[r] = heads >= QK_RUN && row0 + r < rows && h < hq + hkv ? rstd[t * (hq + hkv) + h] : 0.f;
+    }
+#pragma unroll
+    for (int r = 0; r < QK_RUN; ++r, at.next()) {
+      static_assert(QK_RUN == QK_STAGES, "row r of a run is in slot r");
+      const int h = at.h;
+      const bool live = row0 + r < rows, norm = live && h < hq + hkv;
+      float rs = rs_run[r];
+      if (heads < QK_RUN) rs = norm ? rstd[at.t * (hq + hkv) + h] : 0.f;
+      if (ROPE && live && l.turns && r > 0 && h == 0) rope_entries(rp, at.t, lane, c, s);
+      if (norm && (h < hq) != w.of_q) w.load(wq, wk, h < hq, l);
+      pb::cp_async_wait<QK_STAGES - 1>();
+      const Bf8* sl = slots + r * 4 * 256;
+      Bf8 ga{}, gb{}, xa{}, xb{};
+      if (live && l.ina) ga = sl[0];
+      if (live && l.inb) gb = sl[256];
+      if (norm && l.ina) xa = sl[512];
+      if (norm && l.inb) xb = sl[768];
+      if (ROPE && norm && l.turns) rope_pair(ga, gb, c, s, -1.f);
+      const Pairs fx = unpack_pairs(xa, xb);
+      Pairs fg = unpack_pairs(ga, gb);
+      uint64_t dots = 0;
       if (norm) {
-        float fw[8];
-        bf8_to_f(vx[r], fx);
-        bf8_to_f(vg[r], fg);
-        bf8_to_f(h < hq ? gq : gk, fw);
-        const float sq = h < hq ? rs[r] : 0.f, sk = h < hq ? 0.f : rs[r];
+        const Pairs fw = unpack_pairs(w.a, w.b);
+        const uint64_t rr = pb::pack_f32x2(rs, rs);
+        auto products = [&](Pairs& sum) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) sum.v[j] = pb::fma_f32x2(pb::mul_f32x2(fg.v[j], fx.v[j]), rr, sum.v[j]);
+        };
+        if (h < hq) products(dw[0]);
+        else products(dw[1]);
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          dw[0][j] += fg[j] * fx[j] * sq;
-          dw[1][j] += fg[j] * fx[j] * sk;
-          fg[j] *= fw[j];
-          dot += fg[j] * fx[j];
+          fg.v[j] = pb::mul_f32x2(fg.v[j], fw.v[j]);
+          dots = pb::fma_f32x2(fg.v[j], fx.v[j], dots);
         }
       }
-      dot = group_sum<LPR>(dot, nullptr);
+      float da, db;
+      pb::unpack_f32x2(dots, da, db);
+      const float dot = group_sum<LPR>(da + db, nullptr);
       if (norm) {
-        const float c = dot * rs[r] * rs[r] * rs[r] / d;
+        const float k = dot * rs * rs * rs / d;
+        const uint64_t rr = pb::pack_f32x2(rs, rs), nk = pb::pack_f32x2(-k, -k);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) fg[j] = fg[j] * rs[r] - fx[j] * c;
-        vg[r] = f_to_bf8(fg);
+        for (int j = 0; j < 8; ++j) fg.v[j] = pb::fma_f32x2(fg.v[j], rr, pb::mul_f32x2(fx.v[j], nk));
+        pack_pairs(fg, ga, gb);
       }
-      if (live) reinterpret_cast<Bf8*>(dx + t * lddx + (long)h * d)[lane] = vg[r];
+      if (live) {
+        Bf8* dst = reinterpret_cast<Bf8*>(dx + at.t * lddx + (long)h * d);
+        if (l.ina) dst[l.a] = ga;
+        if (l.inb) dst[l.b] = gb;
+      }
+      fetch(r);                          // (the slot's values are in registers: the lane's own, used above)
     }
   }
+  pb::cp_async_wait<0>();
+  // sums of the CTA's groups, through the ring's memory: GROUPS x d floats fit into it
+  float* sums = reinterpret_cast<float*>(ring_raw);
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     __syncthreads();
-    sums[grp][lane * 2] = make_float4(dw[w][0], dw[w][1], dw[w][2], dw[w][3]);
-    sums[grp][lane * 2 + 1] = make_float4(dw[w][4], dw[w][5], dw[w][6], dw[w][7]);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      float a, b;
+      pb::unpack_f32x2(dw[w].v[j], a, b);
+      if (l.ina) sums[grp * d + l.a * 8 + j] = a;
+      if (l.inb) sums[grp * d + l.b * 8 + j] = b;
+    }
     __syncthreads();
-    for (int i = threadIdx.x; i < d / 4; i += 256) {
-      float4 t = sums[0][i];
-      for (int g = 1; g < GROUPS; ++g) {
-        const float4 u = sums[g][i];
-        t.x += u.x; t.y += u.y; t.z += u.z; t.w += u.w;
-      }
-      reinterpret_cast<float4*>(partial + (long)blockIdx.x * 2 * d + w * d)[i] = t;
+    for (int i = threadIdx.x; i < d; i += 256) {
+      float t = sums[i];
+      for (int g = 1; g < GROUPS; ++g) t += sums[g * d + i];
+      partial[(long)blockIdx.x * 2 * d + w * d + i] = t;
     }
   }
 }
@@ -640,38 +803,57 @@ int pb_rmsnorm_bwd_y(const void* dy, const void* x, const void* w, const float* 
                      dw_accumulate, s);
 }
 
-// y = qkv with RMSNorm over every q head (gain wq) and k head (gain wk); rstd: fp32 [T, hq + hkv].
-int pb_qk_norm_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, long T, int hq, int hkv, int d,
-                   long ldx, long ldy, float eps, cudaStream_t s) {
+// y = qkv with RMSNorm over every q head (gain wq) and k head (gain wk); rstd: fp32 [T, hq + hkv].  cos_t (or null): the normalised
+// heads are rotated in their first rot_dim channels by the tables' entries [positions, rot_dim / 2] of pos[t] (null: t).
+int pb_qk_norm_rope_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, long T, int hq, int hkv, int d,
+                        long ldx, long ldy, float eps, const int* pos, const float* cos_t, const float* sin_t, int rot_dim,
+                        cudaStream_t s) {
   if (d % 8 || d <= 0 || d > 256 || ldx % 8 || ldy % 8) return -2;
+  if (cos_t && (rot_dim % 16 || rot_dim <= 0 || rot_dim > d)) return -2;
   const long rows = T * (hq + 2 * hkv);
   if (rows == 0) return 0;
 #define PB_QK_FWD(LPR)                                                                                                  \
-  qk_norm_fwd_kernel<LPR, 4><<<(unsigned)((rows + 128 / LPR * 4 - 1) / (128 / LPR * 4)), 128, 0, s>>>(                  \
-      (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, (__nv_bfloat16*)y, rstd, rows, hq, hkv, \
-      d, ldx, ldy, eps)
-  if (d <= 64) PB_QK_FWD(8);
-  else if (d <= 128) PB_QK_FWD(16);
-  else PB_QK_FWD(32);
+  {                                                                                                                     \
+    auto kern = cos_t ? qk_norm_fwd_kernel<LPR, true> : qk_norm_fwd_kernel<LPR, false>;                                 \
+    kern<<<(unsigned)((rows + 128 / LPR * QK_FWD_RUN - 1) / (128 / LPR * QK_FWD_RUN)), 128, 0, s>>>(                            \
+        (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, (__nv_bfloat16*)y, rstd, rows, hq, \
+        hkv, d, ldx, ldy, eps, Rope{pos, cos_t, sin_t, rot_dim});                                                       \
+  }
+  if (d <= 64) PB_QK_FWD(4)
+  else if (d <= 128) PB_QK_FWD(8)
+  else PB_QK_FWD(16)
 #undef PB_QK_FWD
   return (int)cudaGetLastError();
 }
+int pb_qk_norm_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, long T, int hq, int hkv, int d,
+                   long ldx, long ldy, float eps, cudaStream_t s) {
+  return pb_qk_norm_rope_fwd(x, wq, wk, y, rstd, T, hq, hkv, d, ldx, ldy, eps, nullptr, nullptr, nullptr, 0, s);
+}
 
-// scratch: fp32 [pb_rmsnorm_bwd_num_partials(T), 2 d]; dwq / dwk: fp32 [d], dw_accumulate: += instead of =.
-int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq,
-                   float* dwk, float* scratch, long T, int hq, int hkv, int d, long ldx, long lddy, long lddx,
-                   int dw_accumulate, cudaStream_t s) {
+// scratch: fp32 [pb_rmsnorm_bwd_num_partials(T), 2 d]; dwq / dwk: fp32 [d], dw_accumulate: += instead of =.  cos_t (or null), pos,
+// sin_t, rot_dim: as the forward was called.
+int pb_qk_norm_rope_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq,
+                        float* dwk, float* scratch, long T, int hq, int hkv, int d, long ldx, long lddy, long lddx,
+                        int dw_accumulate, const int* pos, const float* cos_t, const float* sin_t, int rot_dim, cudaStream_t s) {
   if (d % 8 || d <= 0 || d > 256 || ldx % 8 || lddy % 8 || lddx % 8) return -2;
+  if (cos_t && (rot_dim % 16 || rot_dim <= 0 || rot_dim > d)) return -2;
   const long rows = T * (hq + 2 * hkv);
   if (rows == 0) return 0;
   const int P = pb_rmsnorm_bwd_num_partials(T);
-#define PB_QK_BWD(LPR)                                                                                            \
-  qk_norm_bwd_kernel<LPR, 4><<<P, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x,                 \
-                                               (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, rstd,          \
-                                               (__nv_bfloat16*)dx, scratch, rows, hq, hkv, d, ldx, lddy, lddx)
-  if (d <= 64) PB_QK_BWD(8);
-  else if (d <= 128) PB_QK_BWD(16);
-  else PB_QK_BWD(32);
+  const int ring = QK_STAGES * 4 * 256 * (int)sizeof(Bf8);
+#define PB_QK_BWD(LPR)                                                                                              \
+  {                                                                                                                 \
+    auto kern = cos_t ? qk_norm_bwd_kernel<LPR, true> : qk_norm_bwd_kernel<LPR, false>;                             \
+    static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];                                                          \
+    const int rc = pbh::allow_shared_memory(kern, ring, allowed[cos_t != nullptr]);                                 \
+    if (rc) return rc;                                                                                              \
+    kern<<<P, 256, ring, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,             \
+                           (const __nv_bfloat16*)wk, rstd, (__nv_bfloat16*)dx, scratch, rows, hq, hkv, d, ldx, lddy, \
+                           lddx, Rope{pos, cos_t, sin_t, rot_dim});                                                 \
+  }
+  if (d <= 64) PB_QK_BWD(4)
+  else if (d <= 128) PB_QK_BWD(8)
+  else PB_QK_BWD(16)
 #undef PB_QK_BWD
   const int rc = (int)cudaGetLastError();
   if (rc) return rc;                                 // no gain sums from partial rows that nothing wrote
@@ -679,6 +861,12 @@ int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk
   rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate != 0);
   rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate != 0);
   return (int)cudaGetLastError();
+}
+int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq,
+                   float* dwk, float* scratch, long T, int hq, int hkv, int d, long ldx, long lddy, long lddx,
+                   int dw_accumulate, cudaStream_t s) {
+  return pb_qk_norm_rope_bwd(dy, x, wq, wk, rstd, dx, dwq, dwk, scratch, T, hq, hkv, d, ldx, lddy, lddx, dw_accumulate, nullptr,
+                             nullptr, nullptr, 0, s);
 }
 
 }  // extern "C"

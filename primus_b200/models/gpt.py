@@ -21,7 +21,7 @@ from typing import Optional
 import torch
 import torch.nn as nn
 
-from ..ops import fused, gemm, layers
+from ..ops import attention, fused, gemm, layers
 from ..parallel import random as prandom
 from ..parallel import state as ps
 from ..parallel import tensor_parallel as tpc
@@ -105,9 +105,17 @@ class SelfAttention(nn.Module):
         d = cfg.kv_channels
         if cfg.add_qkv_bias:
             qkv = qkv + self.linear_qkv.bias
-        if cfg.qk_layernorm:
-            qkv = self._qk_norm(qkv, d)
         cos, sin, pos = rope[:3]
+        if cfg.qk_layernorm:
+            rotated = None
+            if st.cp == 1 and not layers.SEQ_SPLIT.active and attention.kernel_supports(d, d):
+                # (the other branches below rotate with positions of their own)
+                rotated = fused.qk_norm_rope(qkv, self.q_layernorm.weight, self.k_layernorm.weight, self.hq, self.hkv, d,
+                                             cfg.norm_epsilon, cos, sin, pos, int(d * cfg.rotary_percent))
+            if rotated is not None:
+                qkv, cos, sin, pos = rotated, None, None, None
+            else:
+                qkv = self._qk_norm(qkv, d)
         segments = rope[3] if len(rope) > 3 else None
         scale = cfg.attention_softmax_scale
         if st.cp > 1 and (self.window or self.has_sinks or segments or cfg.attn_logit_softcapping):

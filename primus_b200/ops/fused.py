@@ -178,45 +178,62 @@ def dense_rows(t):
 
 
 class QKNormFn(torch.autograd.Function):
-    """RMSNorm of every q and k head inside a packed [T, (hq + 2 hkv) d] projection output; v passes through."""
+    """RMSNorm of every q and k head inside a packed [T, (hq + 2 hkv) d] projection output, rotated afterwards where ``cos`` is
+    given; v passes through."""
 
     @staticmethod
-    def forward(ctx, qkv, wq, wk, hq, hkv, d, eps):
+    def forward(ctx, qkv, wq, wk, hq, hkv, d, eps, cos=None, sin=None, pos=None, rot_dim=0):
         T = qkv.shape[0]
         out = torch.empty(T, (hq + 2 * hkv) * d, dtype=qkv.dtype, device=qkv.device)
         rstd = torch.empty(T, hq + hkv, dtype=torch.float32, device=qkv.device)
-        _lib.call("qk_norm_fwd", qkv, wq, wk, out, rstd, T, hq, hkv, d, qkv.stride(0), out.stride(0), float(eps))
-        ctx.save_for_backward(qkv, wq, wk, rstd)
-        ctx.dims = (hq, hkv, d)
+        _lib.call("qk_norm_rope_fwd", qkv, wq, wk, out, rstd, T, hq, hkv, d, qkv.stride(0), out.stride(0), float(eps),
+                  pos, cos, sin, rot_dim)
+        ctx.save_for_backward(qkv, wq, wk, rstd, cos, sin, pos)
+        ctx.dims = (hq, hkv, d, rot_dim)
         ctx.w_refs = (wq, wk)
         return out
 
     @staticmethod
     def backward(ctx, dy):
-        qkv, wq, wk, rstd = ctx.saved_tensors
-        hq, hkv, d = ctx.dims
+        qkv, wq, wk, rstd, cos, sin, pos = ctx.saved_tensors
+        hq, hkv, d, rot_dim = ctx.dims
         T = qkv.shape[0]
         dy = dense_rows(dy)
         dx = torch.empty(T, (hq + 2 * hkv) * d, dtype=qkv.dtype, device=qkv.device)
         main = [getattr(w, "main_grad", None) for w in ctx.w_refs]
         dw = [g if g is not None else torch.zeros(d, dtype=torch.float32, device=qkv.device) for g in main]
         P = _lib.call_ret("rmsnorm_bwd_num_partials", T)
-        _lib.call("qk_norm_bwd", dy, qkv, wq, wk, rstd, dx, dw[0], dw[1], scratch(qkv.device, "qk_norm_dw", P * 2 * d),
-                  T, hq, hkv, d, qkv.stride(0), dy.stride(0), dx.stride(0), 1)
+        _lib.call("qk_norm_rope_bwd", dy, qkv, wq, wk, rstd, dx, dw[0], dw[1], scratch(qkv.device, "qk_norm_dw", P * 2 * d),
+                  T, hq, hkv, d, qkv.stride(0), dy.stride(0), dx.stride(0), 1, pos, cos, sin, rot_dim)
         dwq, dwk = (None if g is not None else t.to(w.dtype) for g, t, w in zip(main, dw, (wq, wk)))
-        return dx, dwq, dwk, None, None, None, None
+        return dx, dwq, dwk, *[None] * 8
+
+
+def _qk_norm_kernel(qkv, d) -> bool:
+    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and d % 8 == 0 and d <= 256
+            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
 
 
 def qk_norm(qkv, wq, wk, hq, hkv, d, eps=1e-5):
     """Per-head RMSNorm of the q heads (gain ``wq`` [d]) and k heads (``wk``) of a packed tensor
     ``[q heads | k heads | v heads]`` [T, (hq + 2 hkv) d]; the v heads are unchanged."""
     T = qkv.shape[0]
-    if (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and d % 8 == 0 and d <= 256
-            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0):
+    if _qk_norm_kernel(qkv, d):
         return QKNormFn.apply(qkv, gamma(wq), gamma(wk), hq, hkv, d, eps)
     q = rmsnorm(qkv[:, : hq * d].reshape(T * hq, d), wq, eps).reshape(T, hq * d)
     k = rmsnorm(qkv[:, hq * d: (hq + hkv) * d].reshape(T * hkv, d), wk, eps).reshape(T, hkv * d)
     return torch.cat([q, k, qkv[:, (hq + hkv) * d:]], dim=1)
+
+
+def qk_norm_rope(qkv, wq, wk, hq, hkv, d, eps, cos, sin, pos, rot_dim):
+    """:func:`qk_norm` and the rotary embedding of its q and k heads in one pass each way; None where the kernel does not take
+    the tensors (the caller then norms, and rotates where it did)."""
+    tables = [t for t in (cos, sin, pos) if t is not None]
+    if (cos is None or not _qk_norm_kernel(qkv, d) or rot_dim % 16 or not 0 < rot_dim <= d
+            or any(not t.is_contiguous() or t.data_ptr() % 16 or t.device != qkv.device for t in tables)
+            or cos.dtype != torch.float32 or sin.dtype != torch.float32 or (pos is not None and pos.dtype != torch.int32)):
+        return None
+    return QKNormFn.apply(qkv, gamma(wq), gamma(wk), hq, hkv, d, eps, cos, sin, pos, rot_dim)
 
 
 # ----------------------------------------------------------------------------------------------
