@@ -10,6 +10,11 @@
 //   p *= scaling_factor;  counts[e] += 1 for every selected expert.
 // `full` (fp32 [T, E]) is written for the load-balancing losses and the backward.
 //
+// Tokens are counted per CTA in shared memory and added once per expert: 32768 atomics on 64 counters of two cache lines were most of
+// the kernel (4096 tokens, 64 experts, eight each: 22 us, now 11).  The usual load-balancing loss, coeff * E * sum_e f_e P_e with
+// f_e = counts[e] / (T k) and P_e the mean of full[:, e], comes from the same scores: every CTA leaves the sums of its tokens, and
+// aux_loss_kernel adds them in a fixed order; its gradient joins the router's backward.
+//
 // Replaces `fused_group_topk_routing_with_aux_score` and the router's softmax / top-k op chain
 // (primus/backends/megatron/core/transformer/moe/router.py:24-134).
 #include "common.cuh"
@@ -42,17 +47,14 @@ __device__ __forceinline__ float to_f<float>(float x) { return x; }
 template <>
 __device__ __forceinline__ float to_f<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
 
+// One token: everything but the counts.  sel_i: the expert that lane j < k selected.
 template <typename TIn>
-__global__ void __launch_bounds__(WARPS * 32)
-router_fwd_kernel(const TIn* __restrict__ logits, const float* __restrict__ bias, int T, int E, int k, int sigmoid,
-                  int pre_softmax, int num_groups, int group_topk, float scale, float* __restrict__ probs,
-                  int* __restrict__ idx, float* __restrict__ full, int* __restrict__ counts) {
-  extern __shared__ float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int t = blockIdx.x * WARPS + warp;
-  if (t >= T) return;
-  float* sc = smem + warp * 2 * E;  // [0,E): full scores, [E,2E): selection scores
-  float* ch = sc + E;
+__device__ __forceinline__ int route_token(const TIn* __restrict__ logits, const float* __restrict__ bias, int t, int E, int k,
+                                           int sigmoid, int pre_softmax, int num_groups, int group_topk, float scale,
+                                           float* __restrict__ probs, int* __restrict__ idx, long* __restrict__ idx64,
+                                           float* __restrict__ full, float* sc, float* ch) {
+  // sc [0,E): full scores; ch [0,E): selection scores
+  const int lane = threadIdx.x & 31;
   const TIn* lrow = logits + (long)t * E;
 
   float m = -INFINITY;
@@ -147,28 +149,101 @@ router_fwd_kernel(const TIn* __restrict__ logits, const float* __restrict__ bias
   if (act) {
     probs[(long)t * k + lane] = sel_p * scale;
     idx[(long)t * k + lane] = sel_i;
-    if (counts) atomicAdd(counts + sel_i, 1);
+    if (idx64) idx64[(long)t * k + lane] = sel_i;
+  }
+  return sel_i;
+}
+
+// counts (or null): [E], added to; score_sums (or null): [gridDim.x, E], the sums of full over the CTA's tokens.
+template <typename TIn>
+__global__ void __launch_bounds__(WARPS * 32)
+router_fwd_kernel(const TIn* __restrict__ logits, const float* __restrict__ bias, int T, int E, int k, int sigmoid,
+                  int pre_softmax, int num_groups, int group_topk, float scale, float* __restrict__ probs,
+                  int* __restrict__ idx, long* __restrict__ idx64, float* __restrict__ full, int* __restrict__ counts,
+                  float* __restrict__ score_sums) {
+  extern __shared__ float smem[];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int t = blockIdx.x * WARPS + warp;
+  float* sc = smem + warp * 2 * E;
+  int* hist = reinterpret_cast<int*>(smem + WARPS * 2 * E);
+  for (int e = threadIdx.x; e < E; e += WARPS * 32) hist[e] = 0;
+  __syncthreads();
+  if (t < T) {
+    const int sel = route_token<TIn>(logits, bias, t, E, k, sigmoid, pre_softmax, num_groups, group_topk, scale, probs, idx, idx64,
+                                     full, sc, sc + E);
+    if (lane < k) atomicAdd(hist + sel, 1);
+  }
+  __syncthreads();
+  const int tokens = min(WARPS, T - blockIdx.x * WARPS);
+  for (int e = threadIdx.x; e < E; e += WARPS * 32) {
+    if (counts && hist[e]) atomicAdd(counts + e, hist[e]);
+    if (score_sums) {
+      float s = 0.f;
+      for (int w = 0; w < tokens; ++w) s += smem[w * 2 * E + e];
+      score_sums[(long)blockIdx.x * E + e] = s;
+    }
   }
 }
 
-// dlogits [T, E] fp32 from dprobs [T, k], dfull [T, E] (may be null), saved full / idx / probs.
+// aux = factor * sum_e counts[e] / (T k) * (sum over `blocks` rows of score_sums[:, e]) / T.  A CTA owns 32 experts, its 16 thread
+// rows every 16th row of sums; the last CTA to finish (`done`, zero before) adds the CTAs' terms in their order.
+constexpr int AUX_COLS = 32, AUX_ROWS = 16;
+__global__ void __launch_bounds__(AUX_COLS * AUX_ROWS)
+aux_loss_kernel(const float* __restrict__ score_sums, const int* __restrict__ counts, int blocks, int T, int E, int k, float factor,
+                int* __restrict__ done, volatile float* __restrict__ terms, float* __restrict__ aux) {
+  __shared__ float red[AUX_ROWS][AUX_COLS + 1];
+  const int c = threadIdx.x % AUX_COLS, g = threadIdx.x / AUX_COLS, e = blockIdx.x * AUX_COLS + c;
+  float s = 0.f;
+  if (e < E) {
+#pragma unroll 8
+    for (int b = g; b < blocks; b += AUX_ROWS) s += score_sums[(long)b * E + e];
+  }
+  red[g][c] = s;
+  __syncthreads();
+#pragma unroll
+  for (int step = AUX_ROWS / 2; step > 0; step >>= 1) {
+    if (g < step) red[g][c] += red[g + step][c];
+    __syncthreads();
+  }
+  if (threadIdx.x >= 32) return;
+  float term = e < E ? (float)counts[e] / ((float)T * (float)k) * (red[0][c] / (float)T) : 0.f;
+  term = pb::warp_sum(term);
+  if (threadIdx.x != 0) return;
+  terms[blockIdx.x] = term;
+  __threadfence();
+  if (atomicAdd(done, 1) != (int)gridDim.x - 1) return;
+  __threadfence();
+  float total = 0.f;
+  for (int i = 0; i < (int)gridDim.x; ++i) total += terms[i];
+  aux[0] = factor * total;
+}
+
+// dlogits [T, E] from dprobs [T, k], dfull [T, E] (may be null), saved full / idx / probs.  daux (or null): the gradient of the
+// load-balancing loss, whose own with respect to full[t, e] is aux_factor * f_e / T.
+template <typename TOut>
 __global__ void __launch_bounds__(WARPS * 32)
 router_bwd_kernel(const float* __restrict__ dprobs, const float* __restrict__ dfull, const float* __restrict__ full,
                   const int* __restrict__ idx, const float* __restrict__ probs, int T, int E, int k, int sigmoid,
-                  int pre_softmax, float scale, float* __restrict__ dlogits) {
+                  int pre_softmax, float scale, const float* __restrict__ daux, const int* __restrict__ counts, float aux_factor,
+                  TOut* __restrict__ dlogits) {
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * WARPS + warp;
   if (t >= T) return;
   float* g = smem + warp * E;  // gradient w.r.t. the full scores
-  for (int e = lane; e < E; e += 32) g[e] = dfull ? dfull[(long)t * E + e] : 0.f;
+  const float da = daux ? *daux * aux_factor : 0.f;
+  for (int e = lane; e < E; e += 32) {
+    float d = dfull ? dfull[(long)t * E + e] : 0.f;
+    if (daux) d += da * ((float)counts[e] / ((float)T * (float)k)) / (float)T;
+    g[e] = d;
+  }
   __syncwarp();
   const bool act = lane < k;
   const int my_i = act ? idx[(long)t * k + lane] : 0;
   const float dp = act ? dprobs[(long)t * k + lane] * scale : 0.f;   // gradient w.r.t. the unscaled probability
   const float p = act ? probs[(long)t * k + lane] / scale : 0.f;
   const float* frow = full + (long)t * E;
-  float* drow = dlogits + (long)t * E;
+  TOut* drow = dlogits + (long)t * E;
   if (!sigmoid) {
     float extra = 0.f;  // direct logit gradient of the selected entries (post-softmax normalisation)
     if (pre_softmax) {
@@ -185,7 +260,7 @@ router_bwd_kernel(const float* __restrict__ dprobs, const float* __restrict__ df
     __syncwarp();
     if (!pre_softmax && act) g[my_i] += extra;
     __syncwarp();
-    for (int e = lane; e < E; e += 32) drow[e] = g[e];
+    for (int e = lane; e < E; e += 32) drow[e] = (TOut)g[e];
   } else {
     const float f = act ? frow[my_i] : 0.f;
     float df = dp;
@@ -198,7 +273,7 @@ router_bwd_kernel(const float* __restrict__ dprobs, const float* __restrict__ df
     __syncwarp();
     for (int e = lane; e < E; e += 32) {
       const float fe = frow[e];
-      drow[e] = g[e] * fe * (1.f - fe);
+      drow[e] = (TOut)(g[e] * fe * (1.f - fe));
     }
   }
 }
@@ -207,36 +282,68 @@ router_bwd_kernel(const float* __restrict__ dprobs, const float* __restrict__ df
 
 extern "C" {
 
-// logits: [T, E] bf16 (in_bf16 != 0) or fp32.  bias: fp32 [E] or null.  counts: int [E] accumulated (may be null).
-int pb_router_fwd(const void* logits, int in_bf16, const float* bias, int T, int E, int k, int sigmoid, int pre_softmax,
-                  int num_groups, int group_topk, float scale, float* probs, int* idx, float* full, int* counts,
-                  cudaStream_t s) {
+// logits: [T, E] bf16 (in_bf16 != 0) or fp32.  bias: fp32 [E] or null.  idx64 (or null): idx as 64-bit values.  counts: int [E]
+// accumulated (may be null).  score_sums (or null): fp32 [ceil(T / 8), E].
+static int router_fwd(const void* logits, int in_bf16, const float* bias, int T, int E, int k, int sigmoid, int pre_softmax,
+                      int num_groups, int group_topk, float scale, float* probs, int* idx, long* idx64, float* full, int* counts,
+                      float* score_sums, cudaStream_t s) {
   if (E > 1024 || k > 32 || k < 1 || k > E || (num_groups > 1 && (E % num_groups || num_groups > 64))) return -2;
   const int blocks = (T + WARPS - 1) / WARPS;
-  const size_t smem = (size_t)WARPS * 2 * E * sizeof(float);
+  const size_t smem = (size_t)(WARPS * 2 + 1) * E * sizeof(float);
   if (smem > 48 * 1024) {
     static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];
-    const int rc = in_bf16 ? pbh::allow_shared_memory(router_fwd_kernel<__nv_bfloat16>, 64 * 1024, allowed[0])
-                           : pbh::allow_shared_memory(router_fwd_kernel<float>, 64 * 1024, allowed[1]);
+    const int rc = in_bf16 ? pbh::allow_shared_memory(router_fwd_kernel<__nv_bfloat16>, 68 * 1024, allowed[0])
+                           : pbh::allow_shared_memory(router_fwd_kernel<float>, 68 * 1024, allowed[1]);
     if (rc) return rc;
   }
   if (in_bf16)
     router_fwd_kernel<__nv_bfloat16><<<blocks, WARPS * 32, smem, s>>>(
         reinterpret_cast<const __nv_bfloat16*>(logits), bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk,
-        scale, probs, idx, full, counts);
+        scale, probs, idx, idx64, full, counts, score_sums);
   else
     router_fwd_kernel<float><<<blocks, WARPS * 32, smem, s>>>(reinterpret_cast<const float*>(logits), bias, T, E, k,
                                                               sigmoid, pre_softmax, num_groups, group_topk, scale, probs,
-                                                              idx, full, counts);
+                                                              idx, idx64, full, counts, score_sums);
+  return (int)cudaGetLastError();
+}
+int pb_router_fwd(const void* logits, int in_bf16, const float* bias, int T, int E, int k, int sigmoid, int pre_softmax,
+                  int num_groups, int group_topk, float scale, float* probs, int* idx, float* full, int* counts,
+                  cudaStream_t s) {
+  return router_fwd(logits, in_bf16, bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk, scale, probs, idx, nullptr, full,
+                    counts, nullptr, s);
+}
+
+// pb_router_fwd with counts stored instead of added, and 64-bit copies of the indices.  ws: 32-bit words, E counts and 33 more.
+// aux (or null): fp32, receives aux_factor * sum_e f_e P_e; score_sums: fp32 [ceil(T / 8), E], its scratch.
+int pb_moe_route(const void* logits, int in_bf16, const float* bias, int T, int E, int k, int sigmoid, int pre_softmax,
+                 int num_groups, int group_topk, float scale, float* probs, int* idx, long* idx64, float* full, int* ws,
+                 float* aux, float* score_sums, float aux_factor, cudaStream_t s) {
+  if (E > 1024 || E < 1) return -2;
+  const cudaError_t e = cudaMemsetAsync(ws, 0, (size_t)(E + 1) * sizeof(int), s);
+  if (e != cudaSuccess) return (int)e;
+  if (T == 0) return aux ? (int)cudaMemsetAsync(aux, 0xff, sizeof(float), s) : 0;      // the mean of nothing
+  const int rc = router_fwd(logits, in_bf16, bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk, scale, probs, idx, idx64, full,
+                            ws, aux ? score_sums : nullptr, s);
+  if (rc || !aux) return rc;
+  aux_loss_kernel<<<(E + AUX_COLS - 1) / AUX_COLS, AUX_COLS * AUX_ROWS, 0, s>>>(
+      score_sums, ws, (T + WARPS - 1) / WARPS, T, E, k, aux_factor, ws + E, reinterpret_cast<float*>(ws + E + 1), aux);
   return (int)cudaGetLastError();
 }
 
+// dlogits: bf16 (out_bf16 != 0) or fp32.  daux (or null), counts and aux_factor: as the loss of pb_moe_route was made.
 int pb_router_bwd(const float* dprobs, const float* dfull, const float* full, const int* idx, const float* probs, int T,
-                  int E, int k, int sigmoid, int pre_softmax, float scale, float* dlogits, cudaStream_t s) {
+                  int E, int k, int sigmoid, int pre_softmax, float scale, const float* daux, const int* counts, float aux_factor,
+                  int out_bf16, void* dlogits, cudaStream_t s) {
   if (E > 1024 || k > 32) return -2;
+  if (T == 0) return 0;
   const int blocks = (T + WARPS - 1) / WARPS;
-  router_bwd_kernel<<<blocks, WARPS * 32, (size_t)WARPS * E * sizeof(float), s>>>(
-      dprobs, dfull, full, idx, probs, T, E, k, sigmoid, pre_softmax, scale, dlogits);
+  const size_t smem = (size_t)WARPS * E * sizeof(float);
+  if (out_bf16)
+    router_bwd_kernel<__nv_bfloat16><<<blocks, WARPS * 32, smem, s>>>(dprobs, dfull, full, idx, probs, T, E, k, sigmoid, pre_softmax,
+                                                                      scale, daux, counts, aux_factor, (__nv_bfloat16*)dlogits);
+  else
+    router_bwd_kernel<float><<<blocks, WARPS * 32, smem, s>>>(dprobs, dfull, full, idx, probs, T, E, k, sigmoid, pre_softmax, scale,
+                                                              daux, counts, aux_factor, (float*)dlogits);
   return (int)cudaGetLastError();
 }
 

@@ -32,7 +32,7 @@ class AuxLossScaler(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (aux,) = ctx.saved_tensors
-        return g, torch.ones_like(aux) * AuxLossScaler.scale
+        return g, torch.full_like(aux, float(AuxLossScaler.scale))
 
 
 class _TokenIds:
@@ -140,10 +140,15 @@ class MoELayer(nn.Module):
             if ids is None or ids.numel() != y.shape[0]:
                 raise RuntimeError("hash-routed MoE layer: the token ids of the micro-batch are not available")
             fixed = self.router.tid2eid[ids.long()]
-        probs, idx, full, counts = moe_ops.router_scores(
+        balance = bool(cfg.moe_aux_loss_coeff and cfg.moe_router_load_balancing_type in ("aux_loss", "seq_aux_loss")
+                       and torch.is_grad_enabled())
+        # the loss over all tokens at once comes out of the fused router
+        in_router = balance and cfg.moe_router_load_balancing_type == "aux_loss" and not cfg.moe_router_force_load_balancing and \
+            moe_ops.router_takes(logits, cfg.moe_router_topk, cfg.moe_router_score_function, fixed)
+        probs, idx, full, counts, *in_router = moe_ops.router_scores(
             logits, cfg.moe_router_topk, cfg.moe_router_score_function, cfg.moe_router_pre_softmax, bias,
             cfg.moe_router_topk_scaling_factor, cfg.moe_router_num_groups, cfg.moe_router_group_topk,
-            return_counts=True, fixed_idx=fixed)
+            return_counts=True, fixed_idx=fixed, aux_coeff=cfg.moe_aux_loss_coeff if in_router else None)
         if cfg.moe_router_force_load_balancing:
             T = y.shape[0]
             k = cfg.moe_router_topk
@@ -158,13 +163,14 @@ class MoELayer(nn.Module):
                 self.router.local_margin_histogram += margin_histogram(
                     full.detach(), bias, cfg.moe_router_topk, cfg.quantile_balancing_num_bins,
                     cfg.quantile_balancing_margin_min, cfg.quantile_balancing_margin_max)
-        aux = None
-        if cfg.moe_aux_loss_coeff and cfg.moe_router_load_balancing_type in ("aux_loss", "seq_aux_loss") \
-                and torch.is_grad_enabled():
-            seq = cfg.seq_length if cfg.moe_router_load_balancing_type == "seq_aux_loss" and \
-                y.shape[0] % cfg.seq_length == 0 else None
-            aux = moe_ops.load_balancing_loss(full, idx, cfg.num_experts, cfg.moe_router_topk,
-                                              cfg.moe_aux_loss_coeff, seq, counts)
+        if balance:
+            if in_router:
+                aux = in_router[0]
+            else:
+                seq = cfg.seq_length if cfg.moe_router_load_balancing_type == "seq_aux_loss" and \
+                    y.shape[0] % cfg.seq_length == 0 else None
+                aux = moe_ops.load_balancing_loss(full, idx, cfg.num_experts, cfg.moe_router_topk,
+                                                  cfg.moe_aux_loss_coeff, seq, counts)
             probs = AuxLossScaler.apply(probs, aux)
             self.last_aux_loss = aux.detach()
         return probs, idx, counts
@@ -246,14 +252,10 @@ class MoELayer(nn.Module):
 
     # ------------------------------------------------------------------ single rank
     def _forward_local(self, y, probs, flat_e, counts, T, k):
-        rows_cap = moe_ops.rows_capacity(T * k, self.e_local)
-        sched = moe_ops.build_schedule(counts.to(torch.int32), rows_cap)
-        src, pos, src_token = moe_ops.token_maps(flat_e, sched, k)
-        inv_pos = pos.view(T, k)
-        x_perm = moe_ops.gather_rows(y, src_token, inv_pos)
-        probs_perm = moe_ops.permute_probs(probs, src, pos)
+        sched, pos, src_token, probs_perm = moe_ops.local_plan(probs, flat_e.view(T, k), counts, k)
+        x_perm = moe_ops.gather_rows(y, src_token, pos)
         out_perm = self.experts_forward(x_perm, probs_perm, sched)
-        return moe_ops.combine_rows(out_perm, inv_pos, src_token)
+        return moe_ops.combine_rows(out_perm, pos, src_token)
 
     # ------------------------------------------------------------------ fused dispatch / combine (symmetric memory)
     def _forward_fused(self, y, probs, idx, T, k):

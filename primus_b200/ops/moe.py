@@ -28,10 +28,10 @@ BLOCK_ROWS = 128
 # Router
 class RouterFn(torch.autograd.Function):
     """Fused router (``csrc/router.cu``): logits [T, E] -> (probs [T, k] fp32, idx [T, k] int64, full [T, E] fp32,
-    counts [E] int32)."""
+    counts [E] int32, aux).  ``aux``: the load-balancing loss with the coefficient ``aux_coeff`` (None: None)."""
 
     @staticmethod
-    def forward(ctx, logits, bias, topk, sigmoid, pre_softmax, num_groups, group_topk, scale):
+    def forward(ctx, logits, bias, topk, sigmoid, pre_softmax, num_groups, group_topk, scale, aux_coeff=None):
         T, E = logits.shape
         dev = logits.device
         lg = logits.contiguous()
@@ -39,48 +39,67 @@ class RouterFn(torch.autograd.Function):
             lg = lg.float()
         probs = torch.empty(T, topk, dtype=torch.float32, device=dev)
         idx = torch.empty(T, topk, dtype=torch.int32, device=dev)
+        idx64 = torch.empty(T, topk, dtype=torch.int64, device=dev)
         full = torch.empty(T, E, dtype=torch.float32, device=dev)
-        counts = torch.zeros(E, dtype=torch.int32, device=dev)
+        ws = torch.empty(E + 33, dtype=torch.int32, device=dev)
         b = bias.float().contiguous() if bias is not None else None
-        _lib.call("router_fwd", lg, int(lg.dtype == torch.bfloat16), b, T, E, topk, int(sigmoid), int(pre_softmax),
-                  int(num_groups or 0), int(group_topk or 0), float(scale), probs, idx, full, counts)
-        ctx.save_for_backward(full, idx, probs)
-        ctx.cfg = (topk, int(sigmoid), int(pre_softmax), float(scale), logits.dtype)
-        idx64 = idx.long()
+        aux = sums = None
+        factor = 0.0
+        if aux_coeff is not None:
+            aux = torch.empty((), dtype=torch.float32, device=dev)
+            sums = torch.empty(-(-T // 8), E, dtype=torch.float32, device=dev)
+            factor = float(aux_coeff) * E
+        _lib.call("moe_route", lg, int(lg.dtype == torch.bfloat16), b, T, E, topk, int(sigmoid), int(pre_softmax),
+                  int(num_groups or 0), int(group_topk or 0), float(scale), probs, idx, idx64, full, ws, aux, sums, factor)
+        counts = ws[:E]
+        ctx.save_for_backward(full, idx, probs, counts)
+        ctx.cfg = (topk, int(sigmoid), int(pre_softmax), float(scale), logits.dtype, factor)
         ctx.mark_non_differentiable(idx64, counts)
-        return probs, idx64, full, counts
+        ctx.set_materialize_grads(False)
+        return probs, idx64, full, counts, aux
 
     @staticmethod
-    def backward(ctx, dprobs, _didx, dfull, _dcounts):
-        full, idx, probs = ctx.saved_tensors
-        topk, sigmoid, pre_softmax, scale, dt = ctx.cfg
+    def backward(ctx, dprobs, _didx, dfull, _dcounts, daux):
+        full, idx, probs, counts = ctx.saved_tensors
+        topk, sigmoid, pre_softmax, scale, dt, factor = ctx.cfg
         T, E = full.shape
-        dlogits = torch.empty(T, E, dtype=torch.float32, device=full.device)
+        out_bf16 = dt == torch.bfloat16
+        dlogits = torch.empty(T, E, dtype=torch.bfloat16 if out_bf16 else torch.float32, device=full.device)
         dp = dprobs.float().contiguous() if dprobs is not None else torch.zeros_like(probs)
         df = dfull.float().contiguous() if dfull is not None else None
-        _lib.call("router_bwd", dp, df, full, idx, probs, T, E, topk, sigmoid, pre_softmax, scale, dlogits)
-        return dlogits.to(dt), None, None, None, None, None, None, None
+        _lib.call("router_bwd", dp, df, full, idx, probs, T, E, topk, sigmoid, pre_softmax, scale, daux, counts, factor,
+                  int(out_bf16), dlogits)
+        return dlogits.to(dt), *[None] * 8
+
+
+def router_takes(logits, topk: int, score_function: str = "softmax", fixed_idx=None) -> bool:
+    """Whether :func:`router_scores` runs on the fused kernel."""
+    return logits.is_cuda and logits.shape[1] <= 1024 and topk <= 32 and fixed_idx is None and score_function != "sqrtsoftplus"
 
 
 def router_scores(logits: torch.Tensor, topk: int, score_function: str = "softmax", pre_softmax: bool = False,
                   expert_bias: Optional[torch.Tensor] = None, scaling_factor: Optional[float] = None,
                   num_groups: Optional[int] = None, group_topk: Optional[int] = None, return_counts: bool = False,
-                  fixed_idx: Optional[torch.Tensor] = None):
+                  fixed_idx: Optional[torch.Tensor] = None, aux_coeff: Optional[float] = None):
     """Returns (probs [T, k] fp32, idx [T, k] int64, full scores [T, E] fp32 used by the aux losses) and, with
-    ``return_counts``, the per-expert token counts (int32 [E]).  ``score_function`` "sqrtsoftplus" (DeepSeek-V4:
+    ``return_counts``, the per-expert token counts (int32 [E]), and with ``aux_coeff`` last the loss that
+    :func:`load_balancing_loss` gives for it.  ``score_function`` "sqrtsoftplus" (DeepSeek-V4:
     ``sqrt(softplus(logit))``, handled like sigmoid scores) and ``fixed_idx`` (hash routing: the experts are given, only
     the weights come from the scores) run as composed PyTorch operations on every device."""
     if score_function not in ("softmax", "sigmoid", "sqrtsoftplus"):
         raise ValueError(f"unknown moe_router_score_function {score_function!r}")
-    if logits.is_cuda and logits.shape[1] <= 1024 and topk <= 32 and fixed_idx is None and score_function != "sqrtsoftplus":
-        probs, idx, full, counts = RouterFn.apply(logits, expert_bias, topk, score_function == "sigmoid", pre_softmax,
-                                                  num_groups, group_topk, scaling_factor or 1.0)
-        return (probs, idx, full, counts) if return_counts else (probs, idx, full)
+    if router_takes(logits, topk, score_function, fixed_idx):
+        probs, idx, full, counts, aux = RouterFn.apply(logits, expert_bias, topk, score_function == "sigmoid", pre_softmax,
+                                                       num_groups, group_topk, scaling_factor or 1.0, aux_coeff)
+        out = (probs, idx, full, counts) if return_counts else (probs, idx, full)
+        return out if aux_coeff is None else (*out, aux)
     out = router_scores_ref(logits, topk, score_function, pre_softmax, expert_bias, scaling_factor, num_groups,
                             group_topk, fixed_idx)
+    counts = None
     if return_counts:
-        return (*out, torch.bincount(out[1].reshape(-1), minlength=logits.shape[1]).to(torch.int32))
-    return out
+        counts = torch.bincount(out[1].reshape(-1), minlength=logits.shape[1]).to(torch.int32)
+    extra = [] if aux_coeff is None else [load_balancing_loss(out[2], out[1], logits.shape[1], topk, aux_coeff, counts=counts)]
+    return (*out, *([counts] if return_counts else []), *extra)
 
 
 def router_scores_ref(logits: torch.Tensor, topk: int, score_function: str = "softmax", pre_softmax: bool = False,
@@ -240,6 +259,49 @@ class PermuteProbsFn(torch.autograd.Function):
         d = torch.empty(pos.numel(), dtype=torch.float32, device=dout.device)
         _lib.call("gather_f32", dout.float().contiguous(), pos, d, pos.numel())
         return d, None, None
+
+
+class LocalPlanFn(torch.autograd.Function):
+    """The layout of one rank's own copies in one launch (``csrc/moe_permute.cu``): (probabilities of the padded rows, pos [T, k],
+    src_token, padded, row_start, mblock_expert, total)."""
+
+    @staticmethod
+    def forward(ctx, probs, idx, counts, topk, rows_cap):
+        E, R, max_mb, dev = counts.numel(), idx.numel(), rows_cap // BLOCK_ROWS, probs.device
+        ints = torch.empty(R + 2 * rows_cap + max_mb + 2 * E + 1, dtype=torch.int32, device=dev)
+        pos, src, src_token, mblock, row_start, padded, total = ints.split([R, rows_cap, rows_cap, max_mb, E, E, 1])
+        out = torch.empty(rows_cap, dtype=torch.float32, device=dev)
+        _lib.call("moe_local_plan", idx, counts, probs, R, topk, E, rows_cap, max_mb, padded, row_start, mblock, total, src,
+                  src_token, pos, out)
+        pos = pos.view(-1, topk)
+        ctx.save_for_backward(pos)
+        ctx.shape = probs.shape
+        ctx.mark_non_differentiable(pos, src_token, padded, row_start, mblock, total)
+        ctx.set_materialize_grads(False)
+        return out, pos, src_token, padded, row_start, mblock, total
+
+    @staticmethod
+    def backward(ctx, dout, *_):
+        (pos,) = ctx.saved_tensors
+        if dout is None:
+            return (None,) * 5
+        d = torch.empty(ctx.shape, dtype=torch.float32, device=dout.device)
+        _lib.call("gather_f32", dout.float().contiguous(), pos, d, pos.numel())
+        return d, None, None, None, None
+
+
+def local_plan(probs, idx, counts, topk: int):
+    """(schedule, pos [T, k], src_token, routing probabilities of the padded rows) of the copies that ``idx`` [T, k] sends to the
+    ``counts.numel()`` experts of one rank."""
+    E = counts.numel()
+    rows_cap = rows_capacity(idx.numel(), E)
+    if idx.is_cuda and E <= 1024:
+        perm, pos, src_token, padded, row_start, mblock, total = LocalPlanFn.apply(
+            probs.reshape(-1, topk).float().contiguous(), idx.long().contiguous(), counts.to(torch.int32).contiguous(), topk, rows_cap)
+        return Schedule(counts, padded, row_start, mblock, total, rows_cap), pos, src_token, perm
+    sched = build_schedule(counts.to(torch.int32), rows_cap)
+    src, pos, src_token = token_maps(idx.reshape(-1), sched, topk)
+    return sched, pos.view(-1, topk), src_token, permute_probs(probs, src, pos)
 
 
 def permute_probs(probs, src, pos):
