@@ -358,7 +358,7 @@ def main() -> int:
     if rank == 0:
         sampler.start()
     # ---------------------------------------------------------------- device-timed region
-    launches0 = _lib.LAUNCH_COUNT
+    launches0 = _lib.launch_count()
     ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     barrier()
     ev0.record()
@@ -367,7 +367,7 @@ def main() -> int:
     ev1.record()
     barrier()
     ms = ev0.elapsed_time(ev1)
-    launches = _lib.LAUNCH_COUNT - launches0
+    launches = _lib.launch_count() - launches0
     h2d = trainer.stager.h2d_bytes_last_step
     # ---------------------------------------------------------------- end-to-end region
     e2e_ms = None

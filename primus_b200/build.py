@@ -3,8 +3,8 @@
 All device code targets sm_100a only (``-gencode arch=compute_100a,code=sm_100a``); nvcc
 cross-compiles it on hosts without a GPU.  The library exposes plain ``extern "C"`` launchers
 (raw pointers + a CUDA stream) that :mod:`primus_b200.ops._lib` calls through a small CPython module
-(``csrc/python/launch.c``, compiled with gcc; ctypes without it), so no torch headers are needed and a
-full rebuild takes seconds.
+(``csrc/python/launch.c``, compiled with gcc; ctypes without it), so a rebuild of the kernels takes seconds and no torch headers.
+Those are needed by one module alone, the C++ autograd nodes of the common layers (``csrc/python/nodes.cpp``).
 
 Run ``python -m primus_b200.build`` (add ``--force`` to rebuild everything, ``--verbose`` to see
 ptxas resource usage).
@@ -29,6 +29,9 @@ LIB_PATH = LIB_DIR / "libprimus_b200.so"
 # the launchers' Python binding; its name says which interpreter it is for
 LAUNCH_SRC = CSRC / "python" / "launch.c"
 LAUNCH_PATH = LIB_DIR / ("_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+# autograd nodes of the common layers (torch headers: half a minute)
+NODES_SRC = CSRC / "python" / "nodes.cpp"
+NODES_PATH = LIB_DIR / ("_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -95,6 +98,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if p.returncode != 0:
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
     _build_launch(force)
+    _build_nodes(force)
     return LIB_PATH
 
 
@@ -117,6 +121,33 @@ def _build_launch(force: bool) -> None:
             why = f"the compiled binding could not be built ({e})"
     LAUNCH_PATH.unlink(missing_ok=True)
     print(f"{why}\nlaunchers are called through ctypes", file=sys.stderr)
+
+
+def _build_nodes(force: bool) -> None:
+    """The C++ autograd nodes.  Where they cannot be built, the layers run as Python functions; a module of an older source does
+    not stay behind."""
+    if not force and not _needs_build(NODES_SRC, NODES_PATH, []):
+        return
+    NODES_PATH.unlink(missing_ok=True)
+    if platform.machine() != "x86_64":
+        why = "not x86-64"
+    else:
+        import torch
+
+        root, cuda = Path(torch.__file__).parent, Path(find_nvcc()).parent.parent
+        includes = [root / "include", root / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
+        cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_nodes",
+               f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-I{i}" for i in includes], str(NODES_SRC),
+               "-o", str(NODES_PATH), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+        try:
+            p = subprocess.run(cmd, capture_output=True, text=True)
+            if p.returncode == 0:
+                return
+            why = f"{p.stdout}{p.stderr}"
+        except OSError as e:
+            why = str(e)
+    NODES_PATH.unlink(missing_ok=True)
+    print(f"the autograd nodes could not be built:\n{why}\nlayers run as Python functions", file=sys.stderr)
 
 
 def main() -> None:

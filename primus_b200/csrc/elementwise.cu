@@ -378,6 +378,16 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ lab
   }
 }
 
+// out[0] = sum of x[i] * w[i], in a fixed order (the loss of a micro-batch from its tokens')
+__global__ void __launch_bounds__(1024)
+weighted_sum_kernel(const float* __restrict__ x, const float* __restrict__ w, long n, float* __restrict__ out) {
+  __shared__ float red[32];
+  float s = 0.f;
+  for (long i = threadIdx.x; i < n; i += 1024) s += x[i] * w[i];
+  s = block_sum<1024>(s, red);
+  if (threadIdx.x == 0) out[0] = s;
+}
+
 // ------------------------------------------------------------------ optimizer / flat-buffer helpers
 // AdamW over a flat shard. grads are multiplied by *grad_scale (device scalar: clip coefficient x
 // 1/loss-scale). When *skip != 0 (non-finite gradients found) nothing is updated.
@@ -816,6 +826,11 @@ int pb_ce_fused(void* logits, const long* labels, const float* gscale, float* lo
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
   ce_fused_kernel<<<(unsigned)rows, CE_THREADS, 0, s>>>((__nv_bfloat16*)logits, labels, gscale, loss, V, ld);
+  PB_CHECK_LAUNCH();
+}
+
+int pb_weighted_sum(const float* x, const float* w, float* out, long n, cudaStream_t s) {
+  weighted_sum_kernel<<<1, 1024, 0, s>>>(x, w, n, out);
   PB_CHECK_LAUNCH();
 }
 

@@ -12,6 +12,7 @@ import ctypes
 import importlib.machinery
 import importlib.util
 import os
+import sys
 import sysconfig
 import threading
 import warnings
@@ -131,7 +132,7 @@ def _bind(name: str, args, stream: bool):
 
 
 # Number of device kernels each launcher enqueues (default 1); used for the launch counter below.
-_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "rmsnorm_bwd_two": 2, "rmsnorm_bwd_y": 2, "sumsq": 2, "grad_norm": 2, "flash_attn_bwd": 3, "quant_fp8_tensorwise": 2,
+_KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "rmsnorm_bwd_two": 2, "rmsnorm_bwd_y": 2, "sumsq": 2, "grad_norm": 2, "flash_attn_bwd": 3, "flash_attn_bwd_cap": 3, "quant_fp8_tensorwise": 2,
                      "quant_fp8_delayed": 2, "gemm_bf16_splitk": 2, "qk_norm_bwd": 3, "qk_norm_rope_bwd": 3}
 LAUNCH_COUNT = 0
 
@@ -161,6 +162,53 @@ def call_ret(name: str, *args) -> int:
     launch, _ = _BOUND.get((name, False)) or _bind(name, args, False)
     rc = launch(args, 0)
     return _bound_anew(name, args, False, 0) if rc is None else rc
+
+
+def _load_nodes():
+    """The C++ autograd nodes beside the library, or None: the layers then run as Python functions."""
+    path = LIB_PATH.parent / ("_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
+    if not path.exists() or not available() or not torch.cuda.is_available():
+        return None
+    from . import autotune, gemm
+
+    try:
+        loader = importlib.machinery.ExtensionFileLoader("_nodes", str(path))
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_nodes", loader))
+        loader.exec_module(module)
+        if torch.__version__.split("+")[0] != module.torch_version:
+            raise ImportError(f"built for torch {module.torch_version}")
+        load()
+        module.init(str(lib_path()), sys.modules[__name__], gemm, autotune)
+    except (ImportError, RuntimeError) as e:
+        warnings.warn(f"{path} does not load ({e}): layers run as Python functions")
+        return None
+    return module
+
+
+_NODES: list = []       # [the module, or None]
+
+
+_PLAIN = (torch.Tensor, torch.nn.Parameter)
+_functorch = torch._C._are_functorch_transforms_active
+
+
+def nodes(*tensors):
+    """The C++ autograd nodes where they take these tensors (bf16 on the GPU, no subclass, no function transform at work; None among
+    them counts as taken), else None."""
+    if not _NODES:
+        _NODES.append(_load_nodes())
+    n = _NODES[0]
+    if n is None or _functorch():
+        return None
+    for t in tensors:
+        if t is not None and (type(t) not in _PLAIN or t.dtype is not torch.bfloat16 or not t.is_cuda):
+            return None
+    return n
+
+
+def launch_count() -> int:
+    """Kernels launched so far, from Python and by the C++ nodes."""
+    return LAUNCH_COUNT + (_NODES[0].launches() if _NODES and _NODES[0] is not None else 0)
 
 
 class I32(int):

@@ -165,4 +165,9 @@ def flash_attention(q, k, v, batch: int = 1, causal: bool = True, scale: float |
         return attention_ref(q, k, v, batch, causal, scale, q_off, window, sinks, softcap)[0]
     if not q.is_cuda:
         return attention_ref(q, k, v, batch, causal, scale, q_off, window, sinks, softcap)[0]
+    n = _lib.nodes(q, k, v)
+    if n is not None:
+        if sinks is not None:
+            _check_sinks(sinks, q.shape[1])
+        return n.flash_attention(q, k, v, batch, causal, scale, int(q_off), int(window or 0), sinks, float(softcap or 0.0))
     return FlashAttnFn.apply(q, k, v, batch, causal, scale, q_off, window, sinks, softcap)

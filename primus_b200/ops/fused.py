@@ -166,6 +166,9 @@ def rmsnorm(x, w, eps=1e-5, residual=None):
     w = gamma(w)
     if not x.is_cuda:
         return rmsnorm_ref(x, w, eps, residual)
+    n = _lib.nodes(x, w, residual)
+    if n is not None:
+        return n.rmsnorm(x, w, eps, residual)
     return RMSNormFn.apply(x, w, eps, residual)
 
 
@@ -219,7 +222,11 @@ def qk_norm(qkv, wq, wk, hq, hkv, d, eps=1e-5):
     ``[q heads | k heads | v heads]`` [T, (hq + 2 hkv) d]; the v heads are unchanged."""
     T = qkv.shape[0]
     if _qk_norm_kernel(qkv, d):
-        return QKNormFn.apply(qkv, gamma(wq), gamma(wk), hq, hkv, d, eps)
+        wq, wk = gamma(wq), gamma(wk)
+        n = _lib.nodes(qkv, wq, wk)
+        if n is not None:
+            return n.qk_norm(qkv, wq, wk, hq, hkv, d, eps, None, None, None, 0)
+        return QKNormFn.apply(qkv, wq, wk, hq, hkv, d, eps)
     q = rmsnorm(qkv[:, : hq * d].reshape(T * hq, d), wq, eps).reshape(T, hq * d)
     k = rmsnorm(qkv[:, hq * d: (hq + hkv) * d].reshape(T * hkv, d), wk, eps).reshape(T, hkv * d)
     return torch.cat([q, k, qkv[:, (hq + hkv) * d:]], dim=1)
@@ -233,7 +240,11 @@ def qk_norm_rope(qkv, wq, wk, hq, hkv, d, eps, cos, sin, pos, rot_dim):
             or any(not t.is_contiguous() or t.data_ptr() % 16 or t.device != qkv.device for t in tables)
             or cos.dtype != torch.float32 or sin.dtype != torch.float32 or (pos is not None and pos.dtype != torch.int32)):
         return None
-    return QKNormFn.apply(qkv, gamma(wq), gamma(wk), hq, hkv, d, eps, cos, sin, pos, rot_dim)
+    wq, wk = gamma(wq), gamma(wk)
+    n = _lib.nodes(qkv, wq, wk)
+    if n is not None:
+        return n.qk_norm(qkv, wq, wk, hq, hkv, d, eps, cos, sin, pos, rot_dim)
+    return QKNormFn.apply(qkv, wq, wk, hq, hkv, d, eps, cos, sin, pos, rot_dim)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -391,6 +402,9 @@ def swiglu(x, probs=None, clamp=0.0, act="silu"):
     (primus/backends/megatron/core/extensions/primus_turbo.py:1954-1980)."""
     if not x.is_cuda or GATE_KINDS[act] == 2:
         return swiglu_ref(x, probs, clamp, act)
+    n = _lib.nodes(x)
+    if n is not None and (probs is None or type(probs) is torch.Tensor):
+        return n.swiglu(x, probs, float(clamp), GATE_KINDS[act])
     return SwiGLUFn.apply(x, probs, clamp, act)
 
 
@@ -531,6 +545,11 @@ def cross_entropy(logits, labels, vocab_start=0, group=None, weights=None, unit_
     if not logits.is_cuda:
         loss = cross_entropy_ref(logits, labels, vocab_start, group if _dist_group_active(group) else None)
         return (loss * weights.reshape(loss.shape).float()).sum() if weights is not None else loss
+    if not _dist_group_active(group) and labels.dtype == torch.int64 and labels.is_cuda and type(labels) is torch.Tensor \
+            and (weights is None or weights.is_cuda):
+        n = _lib.nodes(logits)
+        if n is not None:
+            return n.cross_entropy(logits, labels, weights, bool(unit_upstream))
     return CrossEntropyFn.apply(logits, labels, vocab_start, group, weights, unit_upstream)
 
 
@@ -580,4 +599,8 @@ class EmbeddingFn(torch.autograd.Function):
 def embedding(tokens, weight, vocab_start=0, partial=False):
     """``partial``: the weight holds the vocabulary slice starting at ``vocab_start`` (vocab-parallel);
     tokens outside the slice produce zero rows (summed across the TP group by the caller)."""
+    if not partial and not vocab_start and tokens.dtype == torch.int64 and tokens.is_cuda and type(tokens) is torch.Tensor:
+        n = _lib.nodes(weight)
+        if n is not None:
+            return n.embedding(tokens, weight)
     return EmbeddingFn.apply(tokens, weight, vocab_start, partial)

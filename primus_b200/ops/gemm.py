@@ -370,6 +370,9 @@ def wgrad(dy2: torch.Tensor, x2: torch.Tensor, weight: torch.Tensor):
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    n = _lib.nodes(x, weight)
+    if n is not None and n.plain_gemms():
+        return n.linear(x, weight)
     return LinearFn.apply(x, weight)
 
 

@@ -114,6 +114,10 @@ def norm_linear(hidden, residual, norm_w, weight, eps, tp_group=None, sequence_p
         elif tp_group is not None:
             y = tp_comm.copy_to_tp(y, tp_group)
         return gemm.linear(y, weight), xsum
+    if tp_group is None:
+        n = _lib.nodes(hidden, residual, norm_w, weight)
+        if n is not None and n.plain_gemms():
+            return n.norm_linear(hidden, residual, norm_w, weight, eps)
     return NormLinearFn.apply(hidden, residual, norm_w, weight, eps, tp_group, sp)
 
 
@@ -253,6 +257,10 @@ def swiglu_linear(h1, weight, probs=None, clamp=0.0, tp_group=None, sequence_par
         if sp:
             return tp_comm.reduce_scatter_seq(out, tp_group)
         return tp_comm.all_reduce(out, tp_group) if tp_group is not None else out
+    if tp_group is None and probs is None:
+        n = _lib.nodes(h1, weight)
+        if n is not None and n.plain_gemms():
+            return n.swiglu_linear(h1, weight, float(clamp), fused.GATE_KINDS[act])
     return SwiGLULinearFn.apply(h1, weight, probs, clamp, tp_group, sp, act)
 
 
@@ -374,6 +382,13 @@ def rope_attention(qkv, cos, sin, pos, batch, hq, hkv, d, rot_dim=None, causal=T
         else:
             o = attention.attention_ref(q, k, v, batch, causal, scale, 0, window, sinks, softcap)[0]
         return o.reshape(T, hq * d)
+    if not segments:
+        n = _lib.nodes(qkv)
+        if n is not None:
+            if sinks is not None:
+                attention._check_sinks(sinks, hq)
+            return n.rope_attention(qkv, cos, sin, pos, batch, hq, hkv, d, rot_dim, causal, scale, int(window or 0), sinks,
+                                    float(softcap or 0.0))
     return RopeAttentionFn.apply(qkv, cos, sin, pos, batch, hq, hkv, d, rot_dim, causal, scale, window, sinks, segments,
                                  softcap or 0.0)
 

@@ -89,8 +89,13 @@ def router_scores(logits: torch.Tensor, topk: int, score_function: str = "softma
     if score_function not in ("softmax", "sigmoid", "sqrtsoftplus"):
         raise ValueError(f"unknown moe_router_score_function {score_function!r}")
     if router_takes(logits, topk, score_function, fixed_idx):
-        probs, idx, full, counts, aux = RouterFn.apply(logits, expert_bias, topk, score_function == "sigmoid", pre_softmax,
-                                                       num_groups, group_topk, scaling_factor or 1.0, aux_coeff)
+        n = _lib.nodes(logits)
+        args = (logits, expert_bias, topk, score_function == "sigmoid", bool(pre_softmax))
+        if n is not None:
+            probs, idx, full, counts, aux = n.router(*args, int(num_groups or 0), int(group_topk or 0), float(scaling_factor or 1.0),
+                                                     aux_coeff)
+        else:
+            probs, idx, full, counts, aux = RouterFn.apply(*args, num_groups, group_topk, scaling_factor or 1.0, aux_coeff)
         out = (probs, idx, full, counts) if return_counts else (probs, idx, full)
         return out if aux_coeff is None else (*out, aux)
     out = router_scores_ref(logits, topk, score_function, pre_softmax, expert_bias, scaling_factor, num_groups,
@@ -296,7 +301,8 @@ def local_plan(probs, idx, counts, topk: int):
     E = counts.numel()
     rows_cap = rows_capacity(idx.numel(), E)
     if idx.is_cuda and E <= 1024:
-        perm, pos, src_token, padded, row_start, mblock, total = LocalPlanFn.apply(
+        n = _lib.nodes()
+        perm, pos, src_token, padded, row_start, mblock, total = (LocalPlanFn.apply if n is None else n.local_plan)(
             probs.reshape(-1, topk).float().contiguous(), idx.long().contiguous(), counts.to(torch.int32).contiguous(), topk, rows_cap)
         return Schedule(counts, padded, row_start, mblock, total, rows_cap), pos, src_token, perm
     sched = build_schedule(counts.to(torch.int32), rows_cap)
@@ -366,7 +372,8 @@ def gather_rows(x, src, inv_pos):
         m = src >= 0
         out[m] = x[src[m].long()]
         return out
-    return GatherRowsFn.apply(x, src, inv_pos, None)
+    n = _lib.nodes(x)
+    return GatherRowsFn.apply(x, src, inv_pos, None) if n is None else n.gather_rows(x, src, inv_pos)
 
 
 def combine_rows(y, pos, src_token):
@@ -376,7 +383,8 @@ def combine_rows(y, pos, src_token):
         g = y[pos.clamp_min(0).long().reshape(-1)].view(T, k, -1)
         g = g * (pos >= 0).unsqueeze(-1).to(g.dtype)
         return g.sum(1)
-    return CombineRowsFn.apply(y, pos, src_token)
+    n = _lib.nodes(y)
+    return CombineRowsFn.apply(y, pos, src_token) if n is None else n.combine_rows(y, pos, src_token)
 
 
 # ----------------------------------------------------------------------------------------------
@@ -499,6 +507,11 @@ class GroupedLinearFn(torch.autograd.Function):
 def grouped_linear(x, w, sched: Schedule):
     if not x.is_cuda:
         return _GroupedRefFn.apply(x, w, sched)
+    from . import gemm
+
+    n = _lib.nodes(x, w)
+    if n is not None and gemm.fp8_recipe() is None:
+        return n.grouped_linear(x, w, sched.mblock_expert, sched.row_start, sched.padded)
     return GroupedLinearFn.apply(x, w, sched)
 
 
