@@ -111,6 +111,106 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
+// Many long rows: CTAs that stay, THREADS threads a row, whose loads run `stages` rows ahead of the row sums through the threads' own
+// slots of shared memory, as in the backward; a CTA per row spends its life waiting for its loads, then for its sum (16384 x
+// 8192 with residual 183 us, this 172, without 121 and 89; 8192 x 4096 50 and 46, 30 and 23; 1300 x 8192 19 and 14).  Sums in the
+// order of the kernel above.  (Three rows ahead or eight CTAs per SM are no faster: 8192 x 5120 63 us against 56.)
+constexpr int FWD_STAGES = 2, FWD_CTAS = 4;
+inline bool fwd_ring(long rows, int H) { return H > 2048 && rows >= 148 * 8; }
+template <int VPT, int THREADS, bool RES>
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_fwd_ring_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
+                        const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
+                        __nv_bfloat16* __restrict__ xsum, float* __restrict__ rstd_out, long rows, int H, long ldx,
+                        long ldy, float eps) {
+  extern __shared__ __align__(16) uint8_t ring_raw[];
+  __shared__ float red[2][THREADS / 32];
+  constexpr int OPS = RES ? 2 : 1;
+  Bf8* ring = reinterpret_cast<Bf8*>(ring_raw) + threadIdx.x;      // [stage][operand][k][thread]
+  const int tid = threadIdx.x, nv = H / 8;
+  auto fetch = [&](long row, int st) {
+    if (row < rows) {
+      Bf8* slot = ring + st * (OPS * VPT * THREADS);
+#pragma unroll
+      for (int k = 0; k < VPT; ++k) {
+        const int i = tid + k * THREADS;
+        if (i < nv) {
+          pb::cp_async_16(slot + k * THREADS, reinterpret_cast<const Bf8*>(x + row * ldx) + i);
+          if (RES) pb::cp_async_16(slot + (VPT + k) * THREADS, reinterpret_cast<const Bf8*>(res + row * ldx) + i);
+        }
+      }
+    }
+    pb::cp_async_commit();   // also when empty: the wait below counts groups
+  };
+  long row = blockIdx.x;
+#pragma unroll
+  for (int st = 0; st < FWD_STAGES; ++st) fetch(row + (long)st * gridDim.x, st);
+  Bf8 wv[VPT];
+#pragma unroll
+  for (int k = 0; k < VPT; ++k)
+    if (tid + k * THREADS < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[tid + k * THREADS];
+  int st = 0, flip = 0;
+  for (; row < rows; row += gridDim.x, flip ^= 1) {
+    pb::cp_async_wait<FWD_STAGES - 1>();
+    const Bf8* slot = ring + st * (OPS * VPT * THREADS);
+    Bf8 v[VPT];
+    float ss = 0.f;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (tid + k * THREADS < nv) {
+        float f[8];
+        v[k] = slot[k * THREADS];
+        bf8_to_f(v[k], f);
+        if (RES) {
+          float g[8];
+          bf8_to_f(slot[(VPT + k) * THREADS], g);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) f[j] += g[j];
+          v[k] = f_to_bf8(f);  // normalise exactly what later layers will read
+          reinterpret_cast<Bf8*>(xsum + row * ldx)[tid + k * THREADS] = v[k];
+          bf8_to_f(v[k], f);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+      }
+    ss = pb::warp_sum(ss);
+    if ((tid & 31) == 0) red[flip][tid >> 5] = ss;
+    __syncthreads();           // (the slots of `red` alternate: one barrier a row)
+    fetch(row + (long)FWD_STAGES * gridDim.x, st);   // the slot's values are in registers
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < THREADS / 32; ++i) ss += red[flip][i];
+    const float rstd = rsqrtf(ss / H + eps);
+    if (tid == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int k = 0; k < VPT; ++k)
+      if (tid + k * THREADS < nv) {
+        float f[8], g[8];
+        bf8_to_f(v[k], f);
+        bf8_to_f(wv[k], g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * rstd * g[j];
+        reinterpret_cast<Bf8*>(y + row * ldy)[tid + k * THREADS] = f_to_bf8(f);
+      }
+    if (++st == FWD_STAGES) st = 0;
+  }
+}
+
+template <int VPT, int THREADS, bool RES>
+int launch_rmsnorm_fwd_ring(cudaStream_t s, const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
+                            __nv_bfloat16* xsum, float* rstd, long rows, int H, long ldx, long ldy, float eps) {
+  constexpr int BYTES = FWD_STAGES * (RES ? 2 : 1) * VPT * THREADS * 16;
+  constexpr int PER_SM = 220 * 1024 / BYTES;
+  static_assert(PER_SM >= 1, "shared memory");
+  auto kern = rmsnorm_fwd_ring_kernel<VPT, THREADS, RES>;
+  static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+  const int rc = pbh::allow_shared_memory(kern, BYTES, allowed);
+  if (rc) return rc;
+  kern<<<(unsigned)(pbh::sm_count() * (PER_SM < FWD_CTAS ? PER_SM : FWD_CTAS)), THREADS, BYTES, s>>>(x, res, w, y, xsum, rstd, rows, H, ldx,
+                                                                                                      ldy, eps);
+  return 0;
+}
+
 template <typename... Args>
 void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
   const int nv = H / 8;
@@ -769,6 +869,17 @@ int pb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
                    long rows, int H, long ldx, long ldy, float eps, cudaStream_t s) {
   if (H % 8 || ldx % 8 || ldy % 8 || H > 16384) return -2;
   if (rows == 0) return 0;
+  if (fwd_ring(rows, H)) {
+#define PB_NORM_FWD_RING(VPT, THREADS, RES)                                                                                  \
+  launch_rmsnorm_fwd_ring<VPT, THREADS, RES>(s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, \
+                                             (__nv_bfloat16*)y, (__nv_bfloat16*)xsum, rstd, rows, H, ldx, ldy, eps)
+    int rc;
+    if (H <= 4096) rc = res ? PB_NORM_FWD_RING(4, 128, true) : PB_NORM_FWD_RING(4, 128, false);
+    else if (H <= 8192) rc = res ? PB_NORM_FWD_RING(4, 256, true) : PB_NORM_FWD_RING(4, 256, false);
+    else rc = res ? PB_NORM_FWD_RING(8, 256, true) : PB_NORM_FWD_RING(8, 256, false);
+#undef PB_NORM_FWD_RING
+    return rc ? rc : (int)cudaGetLastError();
+  }
   launch_rmsnorm_fwd(rows, H, s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w,
                      (__nv_bfloat16*)y, (__nv_bfloat16*)xsum, rstd, rows, H, ldx, ldy, eps);
   return (int)cudaGetLastError();

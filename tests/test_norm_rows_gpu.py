@@ -113,3 +113,25 @@ def test_backward_gives_the_normalised_rows_again(rows, H, residual, two):
     for a, b in zip(got, want):
         assert torch.equal(a, b)
     assert (got[0].data_ptr() != got[1].data_ptr()) == two
+
+
+@pytest.mark.parametrize("rows", [1183, 1184, 1185, 2400])
+@pytest.mark.parametrize("H", [2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("residual", [False, True])
+def test_forward_around_the_rows_that_ctas_stay_for(rows, H, residual):
+    """The kernel of many rows gives the bits of the one for few (the same rows in two halves)."""
+    g = _gen(rows + H)
+    x, r = (torch.randn(rows, H, device="cuda", generator=g).bfloat16() for _ in range(2))
+    w = (1 + 0.1 * torch.randn(H, device="cuda", generator=g)).bfloat16()
+
+    def run(a, b):
+        y, s, rstd = torch.empty_like(a), torch.empty_like(a), torch.empty(a.shape[0], device="cuda")
+        _lib.call("rmsnorm_fwd", a, b if residual else None, w, y, s if residual else None, rstd, a.shape[0], H, H, H, 1e-5)
+        return (y, s, rstd) if residual else (y, rstd)
+
+    whole = run(x, r)
+    halves = [run(x[i:i + 600].contiguous(), r[i:i + 600].contiguous()) for i in range(0, rows, 600)]
+    for i, t in enumerate(whole):
+        assert torch.equal(t, torch.cat([h[i] for h in halves])), i
+    s64 = (x + r if residual else x).double()
+    _close_bf16(whole[0], _rms64(s64, w.double()), "y")
