@@ -58,6 +58,7 @@ template <int ROPE_HEADS>
 __global__ void __launch_bounds__(256)
 rope_kernel(__nv_bfloat16* __restrict__ x, const int* __restrict__ pos, const float* __restrict__ cos_t,
             const float* __restrict__ sin_t, long T, int heads, int d, int rot_dim, long ld, float sign) {
+  PB_GRID_WAIT();
   const int half = rot_dim / 2;
   const int vec_per_head = half / 8;
   const int per_token = vec_per_head * ((heads + ROPE_HEADS - 1) / ROPE_HEADS);
@@ -189,6 +190,7 @@ template <int KIND, bool CLAMP>
 __global__ void __launch_bounds__(256)
 swiglu_fwd_kernel(const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs, __nv_bfloat16* __restrict__ out, long T,
                   int I, float clamp, int dt, int dv) {
+  PB_GRID_WAIT();
   for (VecWalk w(I / 8); w.t < T; w.next(dt, dv)) {
     const Bf8* row = reinterpret_cast<const Bf8*>(in + w.t * 2L * I) + w.v;
     Bf8 o;
@@ -203,6 +205,7 @@ template <int KIND, bool CLAMP>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
                   __nv_bfloat16* __restrict__ din, __nv_bfloat16* act, long T, int I, float clamp, int dt, int dv) {
+  PB_GRID_WAIT();
   VecWalk w(I / 8);
   while (w.t < T) {
     Bf8 g[2], u[2], d[2];
@@ -240,6 +243,7 @@ template <int KIND, bool CLAMP>
 __global__ void __launch_bounds__(256)
 swiglu_bwd_probs_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* __restrict__ in, const float* __restrict__ probs,
                         __nv_bfloat16* __restrict__ din, __nv_bfloat16* act, float* __restrict__ dprobs, long T, int I, float clamp) {
+  PB_GRID_WAIT();
   const int vpr = I / 8, lane = threadIdx.x & 31;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
   for (long t = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5; t < T; t += num_warps) {
@@ -336,6 +340,7 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ labe
 __global__ void __launch_bounds__(CE_THREADS)
 ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ labels,
                 const float* __restrict__ gscale, float* __restrict__ loss, int V, long ld) {
+  PB_GRID_WAIT();
   __shared__ float red[32];
   const long row = blockIdx.x;
   Bf8* lr = reinterpret_cast<Bf8*>(logits + row * ld);
@@ -381,6 +386,7 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ lab
 // out[0] = sum of x[i] * w[i], in a fixed order (the loss of a micro-batch from its tokens')
 __global__ void __launch_bounds__(1024)
 weighted_sum_kernel(const float* __restrict__ x, const float* __restrict__ w, long n, float* __restrict__ out) {
+  PB_GRID_WAIT();
   __shared__ float red[32];
   float s = 0.f;
   for (long i = threadIdx.x; i < n; i += 1024) s += x[i] * w[i];
@@ -500,6 +506,7 @@ __global__ void __launch_bounds__(256, 5)
 adamw_ranges_kernel(const __grid_constant__ AdamWSegs segs, AdamWRates lrs, float beta1, float beta2, float eps, float wd,
                     float bc1, float bc2, float ic1, float ic2, const float* __restrict__ grad_scale,
                     const int* __restrict__ skip) {
+  PB_GRID_WAIT();
   if (skip && *skip) return;
   const unsigned chunk = gridDim.x - 1 - blockIdx.x;
   int k = segs.count - 1;
@@ -590,6 +597,7 @@ struct SumsqSegs {                      // tensors of one launch: SUMSQ_BLOCKS b
 template <typename T, bool ALIGNED>
 __global__ void __launch_bounds__(SUMSQ_BLOCK_CHAINS * sizeof(T) / 16)
 sumsq_partial_kernel(const __grid_constant__ SumsqSegs segs, float* __restrict__ partial) {
+  PB_GRID_WAIT();
   constexpr int PER = 16 / sizeof(T), THREADS = SUMSQ_BLOCK_CHAINS / PER, LANES = 32 / PER, U = 8;
   __shared__ float red[16];
   const T* __restrict__ x = (const T*)segs.x[blockIdx.x / SUMSQ_BLOCKS];
@@ -654,13 +662,16 @@ __device__ __forceinline__ void clip_coef(float sumsq, const ClipArgs& a) {
   if (a.max_norm > 0.f) c = fminf(1.f, a.max_norm / (nrm + 1e-6f));
   a.coef[0] = c * a.extra;
 }
-__global__ void clip_coef_kernel(const float* sumsq, ClipArgs args) { clip_coef(sumsq[0], args); }
+__global__ void clip_coef_kernel(const float* sumsq, ClipArgs args) {
+  PB_GRID_WAIT();
+  clip_coef(sumsq[0], args); }
 
 // out[0] (+)= sum(partial) of each of `segs` tensors in turn; nonfinite[0] |= !isfinite(sum); with args.coef the clip
 // coefficient of that sum, where nothing else is to be added to it.
 __global__ void __launch_bounds__(512) sumsq_final_kernel(const float* __restrict__ partial, int segs,
                                                          float* __restrict__ out, int accumulate,
                                                          int* __restrict__ nonfinite, ClipArgs args) {
+  PB_GRID_WAIT();
   constexpr int B = 4;                  // tensors at a time
   __shared__ float red[B][16], total[B];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -710,6 +721,7 @@ __global__ void add_bf16_into_f32_kernel(float* __restrict__ dst, const __nv_bfl
 // embedding backward: dW[token[t], :] += dy[t, :]  (fp32 atomics)
 __global__ void embedding_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const long* __restrict__ tokens,
                                      float* __restrict__ dw, long T, int H, int vocab_start, int vocab) {
+  PB_GRID_WAIT();
   const long total = T * (H / 2);
   for (long idx = blockIdx.x * (long)blockDim.x + threadIdx.x; idx < total;
        idx += (long)gridDim.x * blockDim.x) {
@@ -744,10 +756,12 @@ int pb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, lon
   if (one <= 0) return 0;
   const float sign = backward ? -1.f : 1.f;
   if (four >= 148 * 1024L)
-    rope_kernel<4><<<(unsigned)((four + 255) / 256), 256, 0, s>>>((__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads, d, rot_dim,
+    pbh::launch_dependent(rope_kernel<4>, (unsigned)((four + 255) / 256), 256, 0, s, (__nv_bfloat16*)x, pos, cos_t, sin_t, T,
+        heads, d, rot_dim,
                                                                  ld, sign);
   else
-    rope_kernel<1><<<(unsigned)((one + 255) / 256), 256, 0, s>>>((__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads, d, rot_dim,
+    pbh::launch_dependent(rope_kernel<1>, (unsigned)((one + 255) / 256), 256, 0, s, (__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads,
+        d, rot_dim,
                                                                 ld, sign);
   PB_CHECK_LAUNCH();
 }
@@ -776,7 +790,8 @@ int pb_swiglu_fwd(const void* in, const float* probs, void* out, long T, int I, 
   if (T == 0 || I == 0) return 0;
   const int blocks = grid_for(T * (I / 8), 256), step = blocks * 256;
   auto kern = PB_SWIGLU_KERNEL(swiglu_fwd_kernel);
-  kern<<<blocks, 256, 0, s>>>((const __nv_bfloat16*)in, probs, (__nv_bfloat16*)out, T, I, clamp, step / (I / 8), step % (I / 8));
+  pbh::launch_dependent(kern, blocks, 256, 0, s, (const __nv_bfloat16*)in, probs, (__nv_bfloat16*)out, T, I, clamp, step / (I / 8),
+      step % (I / 8));
   PB_CHECK_LAUNCH();
 }
 
@@ -787,12 +802,14 @@ int pb_swiglu_bwd_act(const void* dy, const void* in, const float* probs, void* 
   if (T == 0) return 0;
   if (dprobs) {
     auto kern = PB_SWIGLU_KERNEL(swiglu_bwd_probs_kernel);
-    kern<<<grid_for(T * 32, 256), 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs, (__nv_bfloat16*)din,
+    pbh::launch_dependent(kern, grid_for(T * 32, 256), 256, 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs,
+        (__nv_bfloat16*)din,
                                                (__nv_bfloat16*)act, dprobs, T, I, clamp);
   } else if (I > 0) {
     const int blocks = grid_for(T * (I / 8), 512, 148 * 8), step = blocks * 256;
     auto kern = PB_SWIGLU_KERNEL(swiglu_bwd_kernel);
-    kern<<<blocks, 256, 0, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs, (__nv_bfloat16*)din, (__nv_bfloat16*)act,
+    pbh::launch_dependent(kern, blocks, 256, 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs, (__nv_bfloat16*)din,
+        (__nv_bfloat16*)act,
                                 T, I, clamp, step / (I / 8), step % (I / 8));
   }
   PB_CHECK_LAUNCH();
@@ -825,12 +842,12 @@ int pb_ce_fused(void* logits, const long* labels, const float* gscale, float* lo
                 long ld, cudaStream_t s) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  ce_fused_kernel<<<(unsigned)rows, CE_THREADS, 0, s>>>((__nv_bfloat16*)logits, labels, gscale, loss, V, ld);
+  pbh::launch_dependent(ce_fused_kernel, (unsigned)rows, CE_THREADS, 0, s, (__nv_bfloat16*)logits, labels, gscale, loss, V, ld);
   PB_CHECK_LAUNCH();
 }
 
 int pb_weighted_sum(const float* x, const float* w, float* out, long n, cudaStream_t s) {
-  weighted_sum_kernel<<<1, 1024, 0, s>>>(x, w, n, out);
+  pbh::launch_dependent(weighted_sum_kernel, 1, 1024, 0, s, x, w, n, out);
   PB_CHECK_LAUNCH();
 }
 
@@ -884,7 +901,7 @@ int pb_adamw_ranges(const long* table, int count, const float* hyper, int grad_i
       break;
     }
 #define PB_ADAMW(GT, ST)                                                                                                  \
-  adamw_ranges_kernel<GT, ST><<<(unsigned)chunks, 256, 0, s>>>(segs, lrs, beta1, beta2, eps, wd, bc1, bc2,               \
+  pbh::launch_dependent(adamw_ranges_kernel<GT, ST>, (unsigned)chunks, 256, 0, s, segs, lrs, beta1, beta2, eps, wd, bc1, bc2, \
                                                                (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
     if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
     else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
@@ -919,14 +936,15 @@ int sumsq_many(const long* table, int count, int is_bf16, float* scratch, float*
       segs.n[k] = table[2 * (i + k) + 1];
     }
 #define PB_SUMSQ(T, A) \
-  sumsq_partial_kernel<T, A><<<n * SUMSQ_BLOCKS, SUMSQ_BLOCK_CHAINS * sizeof(T) / 16, 0, s>>>(segs, scratch + (long)i * SUMSQ_BLOCKS)
+  pbh::launch_dependent(sumsq_partial_kernel<T, A>, n * SUMSQ_BLOCKS, SUMSQ_BLOCK_CHAINS * sizeof(T) / 16, 0, s, segs, \
+      scratch + (long)i * SUMSQ_BLOCKS)
     if (is_bf16) { if (aligned) PB_SUMSQ(__nv_bfloat16, true); else PB_SUMSQ(__nv_bfloat16, false); }
     else { if (aligned) PB_SUMSQ(float, true); else PB_SUMSQ(float, false); }
 #undef PB_SUMSQ
     const int rc = (int)cudaGetLastError();
     if (rc) return rc;
   }
-  sumsq_final_kernel<<<1, 512, 0, s>>>(scratch, count, out, accumulate, nonfinite, clip);
+  pbh::launch_dependent(sumsq_final_kernel, 1, 512, 0, s, scratch, count, out, accumulate, nonfinite, clip);
   return (int)cudaGetLastError();
 }
 }  // namespace
@@ -950,7 +968,7 @@ int pb_grad_norm(const long* table, int count, int is_bf16, float* scratch, floa
 
 int pb_clip_coef(const float* sumsq, float max_norm, float extra, float* coef, float* norm_out, int* skip, int check,
                  float spike, cudaStream_t s) {
-  clip_coef_kernel<<<1, 1, 0, s>>>(sumsq, ClipArgs{max_norm, extra, coef, norm_out, skip, check, spike});
+  pbh::launch_dependent(clip_coef_kernel, 1, 1, 0, s, sumsq, ClipArgs{max_norm, extra, coef, norm_out, skip, check, spike});
   PB_CHECK_LAUNCH();
 }
 
@@ -973,7 +991,7 @@ int pb_embedding_bwd(const void* dy, const long* tokens, float* dw, long T, int 
                      int vocab, cudaStream_t s) {
   if (H % 2) return -2;
   if (T == 0) return 0;
-  embedding_bwd_kernel<<<grid_for(T * (H / 2), 256), 256, 0, s>>>((const __nv_bfloat16*)dy, tokens, dw, T, H,
+  pbh::launch_dependent(embedding_bwd_kernel, grid_for(T * (H / 2), 256), 256, 0, s, (const __nv_bfloat16*)dy, tokens, dw, T, H,
                                                                  vocab_start, vocab);
   PB_CHECK_LAUNCH();
 }
@@ -997,6 +1015,7 @@ template <int ROWS, int VECS>
 __global__ void __launch_bounds__(256)
 moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restrict__ src, const float* __restrict__ scale,
                        __nv_bfloat16* __restrict__ out, long R, int H, const int* __restrict__ limit_rows) {
+  PB_GRID_WAIT();
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1046,6 +1065,7 @@ moe_gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const int* __restric
 template <int COPIES, int ROWS, int VECS, int CTAS>
 __global__ void __launch_bounds__(256, CTAS)
 moe_combine_all_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, __nv_bfloat16* __restrict__ out, long T, int H) {
+  PB_GRID_WAIT();
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1090,6 +1110,7 @@ template <int COPIES, int ROWS, int VECS>
 __global__ void __launch_bounds__(256)
 moe_combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos, __nv_bfloat16* __restrict__ out,
                         long T, int topk, int H) {
+  PB_GRID_WAIT();
   const int lane = threadIdx.x & 31;
   const long warp_global = (blockIdx.x * (long)blockDim.x + threadIdx.x) >> 5;
   const long num_warps = ((long)gridDim.x * blockDim.x) >> 5;
@@ -1145,7 +1166,8 @@ extern "C" int pb_moe_gather_rows(const void* x, const int* src, const float* sc
   if (H % 8) return -2;
   if (R == 0) return 0;
 #define PB_GATHER(ROWS, VECS)                                                                                        \
-  moe_gather_rows_kernel<ROWS, VECS><<<moe_grid((R + ROWS - 1) / ROWS), 256, 0, s>>>((const __nv_bfloat16*)x, src, scale, \
+  pbh::launch_dependent(moe_gather_rows_kernel<ROWS, VECS>, moe_grid((R + ROWS - 1) / ROWS), 256, 0, s, (const __nv_bfloat16*)x, \
+      src, scale, \
                                                                                      (__nv_bfloat16*)out, R, H, limit_rows)
   // (us, B200, before and now: 4096 tokens of 2048, 64 experts, eight copies 51 -> 43; 65536 of 256, two copies 44 -> 22)
   if (H <= 256 && R >= 8192) PB_GATHER(4, 1); else PB_GATHER(1, 2);
@@ -1158,10 +1180,10 @@ extern "C" int pb_moe_combine_rows(const void* y, const int* pos, void* out, lon
   if (H % 8) return -2;
   if (T == 0) return 0;
 #define PB_COMBINE_ALL(COPIES, ROWS, VECS, CTAS)                                                  \
-  moe_combine_all_kernel<COPIES, ROWS, VECS, CTAS><<<moe_grid((T + ROWS - 1) / ROWS), 256, 0, s>>>( \
+  pbh::launch_dependent(moe_combine_all_kernel<COPIES, ROWS, VECS, CTAS>, moe_grid((T + ROWS - 1) / ROWS), 256, 0, s, \
       (const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T, H)
 #define PB_COMBINE(COPIES, ROWS, VECS)                                                            \
-  moe_combine_rows_kernel<COPIES, ROWS, VECS><<<moe_grid((T + ROWS - 1) / ROWS), 256, 0, s>>>(    \
+  pbh::launch_dependent(moe_combine_rows_kernel<COPIES, ROWS, VECS>, moe_grid((T + ROWS - 1) / ROWS), 256, 0, s, \
       (const __nv_bfloat16*)y, pos, (__nv_bfloat16*)out, T, topk, H)
   // (us, B200, before and now: 16384 tokens of 2048, one copy 31 -> 24; 65536 of 256, two copies 35 -> 17; 4096 of 2048,
   // eight copies 35 -> 29).  Fewer than 148 x 16 warps leave the SMs short of loads unless each asks for more of them: 1024

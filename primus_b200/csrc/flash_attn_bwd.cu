@@ -211,6 +211,7 @@ flash_attn_bwd_kernel(const __grid_constant__ CUtensorMap tmX1, const __grid_con
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   const uint32_t tmem_sbuf = tmem_base + C::ACC_COLS;  // [S 64][S 64][dP 64]
@@ -658,6 +659,7 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -1118,6 +1120,8 @@ __global__ void __launch_bounds__(DL_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ neg_lse2, int seq, int hq,
                   long o_row, long do_row) {
+  pb::grid_release();
+  PB_GRID_WAIT();
   constexpr int LANES = DV / 8;
   constexpr int GROUPS = DL_THREADS / LANES;
   constexpr int ITERS = DL_POS * DL_HEADS / GROUPS;
@@ -1168,6 +1172,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
 __global__ void __launch_bounds__(1024)
 attn_sink_grad_kernel(const float* __restrict__ delta, const float* __restrict__ lse, const float* __restrict__ sinks,
                       float* __restrict__ dsinks, int batch, int seq, int hq) {
+  PB_GRID_WAIT();
   __shared__ float red[32];
   const int h = blockIdx.x;
   const float sink = sinks[h];
@@ -1254,8 +1259,8 @@ int launch_bwd(const BwdArgs& a) {
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
   const long T = (long)a.batch * a.seq;
-  attn_delta_kernel<DV><<<dim3((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS), DL_THREADS, 0, a.stream>>>(
-      (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.neg_lse2, a.seq,
+  pbh::launch_dependent(attn_delta_kernel<DV>, dim3((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS), DL_THREADS, 0,
+      a.stream, (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.neg_lse2, a.seq,
       a.hq, a.o_row, a.do_row);
   int rc;
   CUtensorMap q128, do128, k128, v128, dq_m, dk_m, dv_m;
@@ -1286,12 +1291,14 @@ int launch_bwd(const BwdArgs& a) {
     cfg.blockDim = dim3(THREADS);                                                                                       \
     cfg.dynamicSmemBytes = CFG::SMEM_BYTES;                                                                             \
     cfg.stream = a.stream;                                                                                              \
-    cudaLaunchAttribute attr[1];                                                                                        \
-    attr[0].id = cudaLaunchAttributeClusterDimension;                                                                   \
-    attr[0].val.clusterDim.x = CSIZE;                                                                                   \
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;                                                            \
+    cudaLaunchAttribute attr[2];                                                                                        \
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;     /* (pb::grid_wait) */                          \
+    attr[0].val.programmaticStreamSerializationAllowed = 1;                                                             \
+    attr[1].id = cudaLaunchAttributeClusterDimension;                                                                   \
+    attr[1].val.clusterDim.x = CSIZE;                                                                                   \
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;                                                            \
     cfg.attrs = attr;                                                                                                   \
-    cfg.numAttrs = CSIZE > 1 ? 1 : 0;                                                                                   \
+    cfg.numAttrs = CSIZE > 1 ? 2 : 1;                                                                                   \
     cudaError_t e = cudaLaunchKernelEx(&cfg, kern, X1, X2, Y1, Y2, O1, O2, lse2, (const float*)a.delta, a.seq, a.seq_k, \
                                        a.q_off, a.hq, a.hkv, a.scale, a.causal, a.window, a.softcap, OUT, a.status);    \
     if (e != cudaSuccess) return (int)e;                                                                                \
@@ -1388,6 +1395,6 @@ extern "C" int pb_flash_attn_bwd(const void* d_o, const void* q, const void* k, 
 extern "C" int pb_attn_sink_grad(const float* delta, const float* lse, const float* sinks, float* dsinks, int batch, int seq,
                                  int hq, cudaStream_t stream) {
   if (hq <= 0) return 0;
-  attn_sink_grad_kernel<<<hq, 1024, 0, stream>>>(delta, lse, sinks, dsinks, batch, seq, hq);
+  pbh::launch_dependent(attn_sink_grad_kernel, hq, 1024, 0, stream, delta, lse, sinks, dsinks, batch, seq, hq);
   return (int)cudaGetLastError();
 }

@@ -177,6 +177,7 @@ flash_attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
   constexpr uint32_t P_COL = 128, O_COL = 256;      // S [0, 128)  P_t [128 + 64 t, +64)  O_t [256 + 128 t, +DV)
@@ -510,7 +511,7 @@ int launch_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
   static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];
   if ((rc = pbh::allow_shared_memory(kern, C::SMEM_BYTES, allowed[win]))) return rc;
   dim3 grid(hq, batch, (seq / BQ + 1) / 2);
-  kern<<<grid, FA_THREADS, C::SMEM_BYTES, stream>>>(tq, tk, tv, to, lse, seq, seq_k, q_off / BQ, hq, hkv,
+  pbh::launch_dependent(kern, grid, FA_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, to, lse, seq, seq_k, q_off / BQ, hq, hkv,
                                                    scale * 1.4426950408889634f, causal, window, sinks, softcap, status);
   return (int)cudaGetLastError();
 }

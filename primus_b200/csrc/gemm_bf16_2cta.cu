@@ -146,6 +146,7 @@ gemm_bf16_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_cons
   pb::tc_fence_before();
   __syncthreads();
   pb::cluster_sync();          // barriers of both CTAs are initialised before any remote arrive / multicast commit
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -342,7 +343,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = SMEM_BYTES;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -370,6 +371,9 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   if (pairs < 1) pairs = 1;
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.stream = stream;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // (pb::grid_wait)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return (int)cudaLaunchKernelEx(&cfg, kern, tA, tB, tD, M, N, K, splits, kb_per_split, status);
 }
 
@@ -377,6 +381,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
 template <int OUT>
 __global__ void __launch_bounds__(256)
 splitk_reduce_kernel(const float* __restrict__ ws, void* __restrict__ out, int M, int N, long ldd, int splits, long part) {
+  PB_GRID_WAIT();
   const int nv = N / 4;
   const long i = blockIdx.x * 256L + threadIdx.x;
   const long m = i / nv;
@@ -475,8 +480,10 @@ extern "C" int pb_gemm_bf16_splitk(const void* A, const void* B, void* D, float*
   else rc = launch<1, 0, OUT_F32>(tA, tB, tD, M, N, K, status, 0, stream, splits);
   if (rc) return rc;
   const unsigned blocks = (unsigned)(((long)M * (N / 4) + 255) / 256);
-  if (out_mode == OUT_BF16) splitk_reduce_kernel<OUT_BF16><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
-  else if (out_mode == OUT_F32) splitk_reduce_kernel<OUT_F32><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
-  else splitk_reduce_kernel<OUT_F32_ADD><<<blocks, 256, 0, stream>>>(ws, D, M, N, ldd, splits, rows * N);
+  if (out_mode == OUT_BF16) pbh::launch_dependent(splitk_reduce_kernel<OUT_BF16>, blocks, 256, 0, stream, ws, D, M, N, ldd, splits,
+      rows * N);
+  else if (out_mode == OUT_F32) pbh::launch_dependent(splitk_reduce_kernel<OUT_F32>, blocks, 256, 0, stream, ws, D, M, N, ldd,
+      splits, rows * N);
+  else pbh::launch_dependent(splitk_reduce_kernel<OUT_F32_ADD>, blocks, 256, 0, stream, ws, D, M, N, ldd, splits, rows * N);
   return (int)cudaGetLastError();
 }

@@ -150,6 +150,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -428,7 +429,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   int ctas = g_num_sms;
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   if (tiles < ctas) ctas = tiles;
-  kern<<<ctas, NUM_THREADS, C::SMEM_BYTES, stream>>>(tA, tB, tD, reinterpret_cast<const uint8_t*>(sfa),
+  pbh::launch_dependent(kern, ctas, NUM_THREADS, C::SMEM_BYTES, stream, tA, tB, tD, reinterpret_cast<const uint8_t*>(sfa),
                                                      reinterpret_cast<const uint8_t*>(sfb), M, N, K, status);
   return (int)cudaGetLastError();
 }

@@ -150,6 +150,7 @@ gemm_mxfp8_2cta_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_con
   pb::tc_fence_before();
   __syncthreads();
   pb::cluster_sync();          // barriers of both CTAs are initialised before any remote arrive / multicast commit
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -342,7 +343,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(NUM_THREADS, 1, 1);
   cfg.dynamicSmemBytes = SMEM_BYTES;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
@@ -368,6 +369,9 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   if (pairs < 1) pairs = 1;
   cfg.gridDim = dim3(2 * pairs, 1, 1);
   cfg.stream = stream;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;     // (pb::grid_wait)
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   return (int)cudaLaunchKernelEx(&cfg, kern, tA, tB, tD, tSA, tSB, M, N, K, status);
 }
 

@@ -139,6 +139,7 @@ grouped_gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -338,7 +339,8 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const int ctas = num_tiles < num_sms ? num_tiles : num_sms;
-  kern<<<ctas, NUM_THREADS, SMEM_BYTES, s>>>(tA, tB, tD, num_m, num_n, num_tiles, K, mblock_expert, row_start, padded,
+  pbh::launch_dependent(kern, ctas, NUM_THREADS, SMEM_BYTES, s, tA, tB, tD, num_m, num_n, num_tiles, K, mblock_expert, row_start,
+      padded,
                                             status);
   return (int)cudaGetLastError();
 }
@@ -349,6 +351,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
 __global__ void build_schedule_kernel(const int* __restrict__ counts, int E, int max_mblocks, int* __restrict__ padded,
                                       int* __restrict__ row_start, int* __restrict__ mblock_expert,
                                       int* __restrict__ total_rows) {
+  PB_GRID_WAIT();
   __shared__ int s_start[1025];
   if (threadIdx.x == 0) {
     int acc = 0;
@@ -385,7 +388,7 @@ extern "C" {
 int pb_moe_build_schedule(const int* counts, int E, int max_mblocks, int* padded, int* row_start, int* mblock_expert,
                           int* total_rows, cudaStream_t s) {
   if (E > 1024) return -2;
-  build_schedule_kernel<<<1, 256, 0, s>>>(counts, E, max_mblocks, padded, row_start, mblock_expert, total_rows);
+  pbh::launch_dependent(build_schedule_kernel, 1, 256, 0, s, counts, E, max_mblocks, padded, row_start, mblock_expert, total_rows);
   return (int)cudaGetLastError();
 }
 

@@ -149,6 +149,7 @@ grouped_gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_
   }
   pb::tc_fence_before();
   __syncthreads();
+  PB_GRID_WAIT();
   pb::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
 
@@ -370,7 +371,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const Args& a, cudaStre
     cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const int ctas = a.num_tiles < num_sms ? a.num_tiles : num_sms;
-  kern<<<ctas, NUM_THREADS, SMEM_BYTES, s>>>(tA, tB, a);
+  pbh::launch_dependent(kern, ctas, NUM_THREADS, SMEM_BYTES, s, tA, tB, a);
   return (int)cudaGetLastError();
 }
 

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(MAP_THREADS)
 moe_permutation_maps_kernel(const long* __restrict__ expert, int R, int topk, int E, const int* __restrict__ row_start,
                             const int* __restrict__ padded, int rows_cap, int* src,
                             int* __restrict__ src_token, int* __restrict__ pos, LocalPlan plan) {
+  PB_GRID_WAIT();
   __shared__ int warp_sums[2][MAP_THREADS / 32];
   const int e = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int start, pad;
@@ -111,6 +112,7 @@ moe_permutation_maps_kernel(const long* __restrict__ expert, int R, int topk, in
 
 // out[i] = idx[i] >= 0 ? x[idx[i]] : 0
 __global__ void gather_f32_kernel(const float* __restrict__ x, const int* __restrict__ idx, float* __restrict__ out, long n) {
+  PB_GRID_WAIT();
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) {
     const int j = idx[i];
     out[i] = j >= 0 ? x[j] : 0.f;
@@ -126,7 +128,8 @@ extern "C" {
 int pb_moe_permutation_maps(const long* expert, long R, int topk, int E, const int* row_start, const int* padded,
                             int rows_cap, int* src, int* src_token, int* pos, cudaStream_t s) {
   if (E <= 0 || topk <= 0 || R < 0 || R > 2147483647L - 2 * MAP_THREADS * MAP_ITEMS) return -2;
-  moe_permutation_maps_kernel<false><<<E, MAP_THREADS, 0, s>>>(expert, (int)R, topk, E, row_start, padded, rows_cap, src, src_token,
+  pbh::launch_dependent(moe_permutation_maps_kernel<false>, E, MAP_THREADS, 0, s, expert, (int)R, topk, E, row_start, padded,
+      rows_cap, src, src_token,
                                                               pos, LocalPlan{});
   return (int)cudaGetLastError();
 }
@@ -137,8 +140,8 @@ int pb_moe_local_plan(const long* expert, const int* counts, const float* probs,
                       int* padded, int* row_start, int* mblock_expert, int* total, int* src, int* src_token, int* pos, float* probs_perm,
                       cudaStream_t s) {
   if (E <= 0 || E > 1024 || topk <= 0 || R < 0 || R > 2147483647L - 2 * MAP_THREADS * MAP_ITEMS) return -2;
-  moe_permutation_maps_kernel<true><<<E, MAP_THREADS, 0, s>>>(
-      expert, (int)R, topk, E, nullptr, nullptr, rows_cap, src, src_token, pos,
+  pbh::launch_dependent(moe_permutation_maps_kernel<true>, E, MAP_THREADS, 0, s, expert, (int)R, topk, E, nullptr, nullptr,
+      rows_cap, src, src_token, pos,
       LocalPlan{counts, probs, padded, row_start, mblock_expert, total, probs_perm, max_mblocks});
   return (int)cudaGetLastError();
 }
@@ -146,7 +149,7 @@ int pb_moe_local_plan(const long* expert, const int* counts, const float* probs,
 int pb_gather_f32(const float* x, const int* idx, float* out, long n, cudaStream_t s) {
   if (n == 0) return 0;
   const long blocks = (n + 255) / 256;
-  gather_f32_kernel<<<(unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, s>>>(x, idx, out, n);
+  pbh::launch_dependent(gather_f32_kernel, (unsigned)(blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, s, x, idx, out, n);
   return (int)cudaGetLastError();
 }
 

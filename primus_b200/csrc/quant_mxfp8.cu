@@ -277,6 +277,8 @@ template <bool FP4>
 __global__ void __launch_bounds__(QT, 5)
 quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_t* __restrict__ q_row,
                    uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
+  pb::grid_release();
+  PB_GRID_WAIT();
   __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
   const long p = lane_offset(row0, col0, C);
@@ -296,6 +298,7 @@ __global__ void __launch_bounds__(QT, 5)
 quant_tensorwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, const float* __restrict__ tensor_amax,
                         const float* __restrict__ fallback_amax, uint8_t* __restrict__ q_row,
                         uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
+  PB_GRID_WAIT();
   __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
   const long p = lane_offset(row0, col0, C);
@@ -321,6 +324,7 @@ template <bool TILEWISE>
 __global__ void __launch_bounds__(QT, 4)
 quant_blockwise_kernel(const __nv_bfloat16* __restrict__ x, int R, int C, uint8_t* __restrict__ q_row,
                        uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
+  PB_GRID_WAIT();
   __shared__ TileScales scales;
   __shared__ uint8_t e_rowv[TILE], e_colv[TILE];
   __shared__ uint32_t col_max[4][TILE / 2];      // per warp strip: maxima of column pairs
@@ -446,6 +450,7 @@ template <bool WIDE, bool CLAMP>
 __global__ void __launch_bounds__(WIDE ? 2 * QT : QT, WIDE ? 2 : 6)
 swiglu_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, int T, int I, float clamp, uint8_t* __restrict__ q_row,
                           uint8_t* __restrict__ sf_row, uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col) {
+  PB_GRID_WAIT();
   __shared__ TileScales scales;
   const int row0 = blockIdx.y * TILE, col0 = blockIdx.x * TILE;
   const long pin = lane_offset(row0, col0, 2L * I), p = lane_offset(row0, col0, I);
@@ -536,6 +541,7 @@ swiglu_bwd_quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ h1, const __nv_b
                               float clamp, uint8_t* __restrict__ q_row, uint8_t* __restrict__ sf_row,
                               uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col, uint8_t* __restrict__ act_col,
                               uint8_t* __restrict__ act_sf) {
+  PB_GRID_WAIT();
   extern __shared__ __align__(16) uint4 slots_raw[];   // [warp][gate, up, dact][row of the lane][lane]
   __shared__ TileScales scales[3];               // of the dgate, the dup and the activation tile
   constexpr int WARPS = WIDE ? 8 : 4, STRIPS = WARPS / 2;
@@ -604,7 +610,7 @@ extern "C" {
 int pb_quant_mxfp8(const void* x, int R, int C, void* q_row, void* sf_row, void* q_col, void* sf_col, cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
   dim3 grid(C / TILE, R / TILE);
-  quant_mxfp8_kernel<false><<<grid, QT, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), R, C,
+  pbh::launch_dependent(quant_mxfp8_kernel<false>, grid, QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R, C,
                                                 reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row),
                                                 reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
@@ -615,8 +621,8 @@ int pb_quant_mxfp8(const void* x, int R, int C, void* q_row, void* sf_row, void*
 int pb_quant_mxfp4_as_fp8(const void* x, int R, int C, void* q_row, void* sf_row, void* q_col, void* sf_col,
                           cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
-  quant_mxfp8_kernel<true><<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), R, C, reinterpret_cast<uint8_t*>(q_row),
+  pbh::launch_dependent(quant_mxfp8_kernel<true>, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
+      C, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
@@ -630,8 +636,8 @@ int pb_quant_fp8_tensorwise(const void* x, int R, int C, float* amax, void* q_ro
   const long n8 = (long)R * C / 8;
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax);
-  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), R, C, amax, nullptr, reinterpret_cast<uint8_t*>(q_row),
+  pbh::launch_dependent(quant_tensorwise_kernel, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
+      C, amax, nullptr, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
@@ -646,8 +652,8 @@ int pb_quant_fp8_delayed(const void* x, int R, int C, float* amax_now, const flo
   const long n8 = (long)R * C / 8;
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax_now);
-  quant_tensorwise_kernel<<<dim3(C / TILE, R / TILE), QT, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(x), R, C, scale_amax, amax_now, reinterpret_cast<uint8_t*>(q_row),
+  pbh::launch_dependent(quant_tensorwise_kernel, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
+      C, scale_amax, amax_now, reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
@@ -661,8 +667,8 @@ int pb_quant_fp8_blockwise(const void* x, int R, int C, int tilewise, void* q_ro
   const __nv_bfloat16* xp = reinterpret_cast<const __nv_bfloat16*>(x);
   uint8_t *qr = reinterpret_cast<uint8_t*>(q_row), *sr = reinterpret_cast<uint8_t*>(sf_row);
   uint8_t *qc = reinterpret_cast<uint8_t*>(q_col), *sc = reinterpret_cast<uint8_t*>(sf_col);
-  if (tilewise) quant_blockwise_kernel<true><<<grid, QT, 0, s>>>(xp, R, C, qr, sr, qc, sc);
-  else quant_blockwise_kernel<false><<<grid, QT, 0, s>>>(xp, R, C, qr, sr, qc, sc);
+  if (tilewise) pbh::launch_dependent(quant_blockwise_kernel<true>, grid, QT, 0, s, xp, R, C, qr, sr, qc, sc);
+  else pbh::launch_dependent(quant_blockwise_kernel<false>, grid, QT, 0, s, xp, R, C, qr, sr, qc, sc);
   return (int)cudaGetLastError();
 }
 
@@ -674,8 +680,8 @@ int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row
   const bool wide = (long)grid.x * grid.y <= 148;
   auto kern = clamp > 0.f ? (wide ? swiglu_quant_mxfp8_kernel<true, true> : swiglu_quant_mxfp8_kernel<false, true>)
                           : (wide ? swiglu_quant_mxfp8_kernel<true, false> : swiglu_quant_mxfp8_kernel<false, false>);
-  kern<<<grid, wide ? 2 * QT : QT, 0, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp, reinterpret_cast<uint8_t*>(q_row),
+  pbh::launch_dependent(kern, grid, wide ? 2 * QT : QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp,
+      reinterpret_cast<uint8_t*>(q_row),
       reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
@@ -693,8 +699,8 @@ int pb_swiglu_bwd_quant_mxfp8(const void* h1, const void* dact, int T, int I, fl
   static std::atomic<bool> allowed[4][pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, smem, allowed[wide + 2 * (clamp > 0.f)]);
   if (rc) return rc;
-  kern<<<grid, wide ? 2 * QT : QT, smem, s>>>(
-      reinterpret_cast<const __nv_bfloat16*>(h1), reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
+  pbh::launch_dependent(kern, grid, wide ? 2 * QT : QT, smem, s, reinterpret_cast<const __nv_bfloat16*>(h1),
+      reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
       reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
       reinterpret_cast<uint8_t*>(sf_col), reinterpret_cast<uint8_t*>(act_col), reinterpret_cast<uint8_t*>(act_sf));
   return (int)cudaGetLastError();

@@ -44,6 +44,7 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
                    const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                    __nv_bfloat16* __restrict__ xsum, float* __restrict__ rstd_out, long rows, int H, long ldx,
                    long ldy, float eps) {
+  PB_GRID_WAIT();
   __shared__ float red[THREADS / 32];
   const int lane = threadIdx.x % LPR;
   const long row0 = (blockIdx.x * (long)(THREADS / LPR) + threadIdx.x / LPR) * RPG;
@@ -123,6 +124,7 @@ rmsnorm_fwd_ring_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
                         const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ y,
                         __nv_bfloat16* __restrict__ xsum, float* __restrict__ rstd_out, long rows, int H, long ldx,
                         long ldy, float eps) {
+  PB_GRID_WAIT();
   extern __shared__ __align__(16) uint8_t ring_raw[];
   __shared__ float red[2][THREADS / 32];
   constexpr int OPS = RES ? 2 : 1;
@@ -206,8 +208,9 @@ int launch_rmsnorm_fwd_ring(cudaStream_t s, const __nv_bfloat16* x, const __nv_b
   static std::atomic<bool> allowed[pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, BYTES, allowed);
   if (rc) return rc;
-  kern<<<(unsigned)(pbh::sm_count() * (PER_SM < FWD_CTAS ? PER_SM : FWD_CTAS)), THREADS, BYTES, s>>>(x, res, w, y, xsum, rstd, rows, H, ldx,
-                                                                                                      ldy, eps);
+  pbh::launch_dependent(kern, (unsigned)(pbh::sm_count() * (PER_SM < FWD_CTAS ? PER_SM : FWD_CTAS)), THREADS, BYTES, s, x, res, w,
+      y,
+                        xsum, rstd, rows, H, ldx, ldy, eps);
   return 0;
 }
 
@@ -215,8 +218,8 @@ template <typename... Args>
 void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
   const int nv = H / 8;
 #define PB_NORM_FWD(LPR, VPL, RPG, THREADS)                                                             \
-  rmsnorm_fwd_kernel<LPR, VPL, RPG, THREADS>                                                            \
-      <<<(unsigned)((rows + (THREADS / LPR) * RPG - 1) / ((THREADS / LPR) * RPG)), THREADS, 0, s>>>(args...)
+  pbh::launch_dependent(rmsnorm_fwd_kernel<LPR, VPL, RPG, THREADS>, \
+      (unsigned)((rows + (THREADS / LPR) * RPG - 1) / ((THREADS / LPR) * RPG)), THREADS, 0, s, args...)
   // Few rows do not fill the SMs with four rows (or two, or a row per warp) per group: spread them (768 rows of 256: 3.0 -> 2.2
   // us).  The lines lie where both forms take the same time; 64 lanes of four vectors hold for 1032 to 2048 channels at any
   // number of rows (500 rows of 2048 3.2 us, with 256 lanes of one vector 3.5), 256 lanes of eight above 8192 (4096 rows of
@@ -252,6 +255,7 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
                          const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                          __nv_bfloat16* __restrict__ dx2, __nv_bfloat16* __restrict__ y, float* __restrict__ partial, long rows,
                          int H, long ldx, long lddy) {
+  PB_GRID_WAIT();
   constexpr int GROUPS = 256 / LPR;
   __shared__ float4 sums[GROUPS][LPR * VPL * 2];
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
@@ -353,6 +357,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ dres, __nv_bfloat16* __restrict__ dx,
                    __nv_bfloat16* __restrict__ dx2, __nv_bfloat16* __restrict__ y, float* __restrict__ partial, long rows, int H,
                    long ldx, long lddy, int stages) {
+  PB_GRID_WAIT();
   extern __shared__ __align__(16) uint8_t ring_raw[];
   __shared__ float red[2][THREADS / 32];
   constexpr int OPS = RES ? 3 : 2;
@@ -484,7 +489,7 @@ int launch_rmsnorm_bwd_ring(int P, cudaStream_t s, const __nv_bfloat16* dy, cons
   static std::atomic<bool> allowed[pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, STAGES * STAGE, allowed);
   if (rc) return rc;
-  kern<<<P, THREADS, STAGES * STAGE, s>>>(dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy, STAGES);
+  pbh::launch_dependent(kern, P, THREADS, STAGES * STAGE, s, dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy, STAGES);
   return (int)cudaGetLastError();
 }
 
@@ -495,7 +500,7 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
 #define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                               \
   {                                                                                                                    \
     auto kern = y ? rmsnorm_bwd_short_kernel<LPR, VPL, RPG, (LPR > 8)> : rmsnorm_bwd_short_kernel<LPR, VPL, RPG, false>; \
-    kern<<<P, 256, 0, s>>>(dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy);                             \
+    pbh::launch_dependent(kern, P, 256, 0, s, dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy);                   \
     return (int)cudaGetLastError();                                                                                    \
   }
 #define PB_NORM_BWD_RING(VPT, THREADS, RES, Y) \
@@ -591,6 +596,7 @@ __global__ void __launch_bounds__(128, 8)
 qk_norm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ wq,
                    const __nv_bfloat16* __restrict__ wk, __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_out,
                    long rows, int hq, int hkv, int d, long ldx, long ldy, float eps, Rope rp) {
+  PB_GRID_WAIT();
   const int lane = threadIdx.x % LPR;
   const long row0 = (blockIdx.x * (long)(128 / LPR) + threadIdx.x / LPR) * QK_FWD_RUN;
   const HeadLane l = HeadLane::make<ROPE>(lane, d, rp.rot_dim);
@@ -692,6 +698,7 @@ qk_norm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
                    const __nv_bfloat16* __restrict__ wq, const __nv_bfloat16* __restrict__ wk,
                    const float* __restrict__ rstd, __nv_bfloat16* __restrict__ dx, float* __restrict__ partial, long rows,
                    int hq, int hkv, int d, long ldx, long lddy, long lddx, Rope rp) {
+  PB_GRID_WAIT();
   constexpr int GROUPS = 256 / LPR;
   extern __shared__ __align__(16) uint8_t ring_raw[];
   Bf8* slots = reinterpret_cast<Bf8*>(ring_raw) + threadIdx.x;     // [stage][dy a, dy b, x a, x b][thread]
@@ -823,6 +830,7 @@ constexpr int DWR_COLS = 32, DWR_ROWS = 16;
 constexpr int DW_STORE_BF16 = 2;     // of `accumulate`: dw is a bf16 vector, and stored
 __global__ void __launch_bounds__(DWR_COLS * DWR_ROWS)
 rmsnorm_dw_reduce_kernel(const float* __restrict__ partial, float* __restrict__ dw, int P, int H, long ld, int accumulate) {
+  PB_GRID_WAIT();
   __shared__ float red[DWR_ROWS][DWR_COLS + 1];
   const int c = threadIdx.x % DWR_COLS, g = threadIdx.x / DWR_COLS;
   const int h = blockIdx.x * DWR_COLS + c;
@@ -857,7 +865,8 @@ int rmsnorm_bwd(int P, const void* dy, const void* x, const void* w, const float
                                       scratch, rows, H, ldx, lddy);
     if (rc) return rc;
   }
-  rmsnorm_dw_reduce_kernel<<<(H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s>>>(scratch, dw, P, H, H, dw_accumulate);
+  pbh::launch_dependent(rmsnorm_dw_reduce_kernel, (H + DWR_COLS - 1) / DWR_COLS, DWR_COLS * DWR_ROWS, 0, s, scratch, dw, P, H, H,
+      dw_accumulate);
   return (int)cudaGetLastError();
 }
 
@@ -926,7 +935,7 @@ int pb_qk_norm_rope_fwd(const void* x, const void* wq, const void* wk, void* y, 
 #define PB_QK_FWD(LPR)                                                                                                  \
   {                                                                                                                     \
     auto kern = cos_t ? qk_norm_fwd_kernel<LPR, true> : qk_norm_fwd_kernel<LPR, false>;                                 \
-    kern<<<(unsigned)((rows + 128 / LPR * QK_FWD_RUN - 1) / (128 / LPR * QK_FWD_RUN)), 128, 0, s>>>(                            \
+    pbh::launch_dependent(kern, (unsigned)((rows + 128 / LPR * QK_FWD_RUN - 1) / (128 / LPR * QK_FWD_RUN)), 128, 0, s, \
         (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, (const __nv_bfloat16*)wk, (__nv_bfloat16*)y, rstd, rows, hq, \
         hkv, d, ldx, ldy, eps, Rope{pos, cos_t, sin_t, rot_dim});                                                       \
   }
@@ -958,7 +967,7 @@ int pb_qk_norm_rope_bwd(const void* dy, const void* x, const void* wq, const voi
     static std::atomic<bool> allowed[2][pbh::MAX_DEVICES];                                                          \
     const int rc = pbh::allow_shared_memory(kern, ring, allowed[cos_t != nullptr]);                                 \
     if (rc) return rc;                                                                                              \
-    kern<<<P, 256, ring, s>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq,             \
+    pbh::launch_dependent(kern, P, 256, ring, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)x, (const __nv_bfloat16*)wq, \
                            (const __nv_bfloat16*)wk, rstd, (__nv_bfloat16*)dx, scratch, rows, hq, hkv, d, ldx, lddy, \
                            lddx, Rope{pos, cos_t, sin_t, rot_dim});                                                 \
   }
@@ -969,8 +978,8 @@ int pb_qk_norm_rope_bwd(const void* dy, const void* x, const void* wq, const voi
   const int rc = (int)cudaGetLastError();
   if (rc) return rc;                                 // no gain sums from partial rows that nothing wrote
   const int blocks = (d + DWR_COLS - 1) / DWR_COLS, threads = DWR_COLS * DWR_ROWS;
-  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch, dwq, P, d, 2 * d, dw_accumulate != 0);
-  rmsnorm_dw_reduce_kernel<<<blocks, threads, 0, s>>>(scratch + d, dwk, P, d, 2 * d, dw_accumulate != 0);
+  pbh::launch_dependent(rmsnorm_dw_reduce_kernel, blocks, threads, 0, s, scratch, dwq, P, d, 2 * d, dw_accumulate != 0);
+  pbh::launch_dependent(rmsnorm_dw_reduce_kernel, blocks, threads, 0, s, scratch + d, dwk, P, d, 2 * d, dw_accumulate != 0);
   return (int)cudaGetLastError();
 }
 int pb_qk_norm_bwd(const void* dy, const void* x, const void* wq, const void* wk, const float* rstd, void* dx, float* dwq,

@@ -161,6 +161,7 @@ router_fwd_kernel(const TIn* __restrict__ logits, const float* __restrict__ bias
                   int pre_softmax, int num_groups, int group_topk, float scale, float* __restrict__ probs,
                   int* __restrict__ idx, long* __restrict__ idx64, float* __restrict__ full, int* __restrict__ counts,
                   float* __restrict__ score_sums) {
+  PB_GRID_WAIT();
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * WARPS + warp;
@@ -191,6 +192,7 @@ constexpr int AUX_COLS = 32, AUX_ROWS = 16;
 __global__ void __launch_bounds__(AUX_COLS * AUX_ROWS)
 aux_loss_kernel(const float* __restrict__ score_sums, const int* __restrict__ counts, int blocks, int T, int E, int k, float factor,
                 int* __restrict__ done, volatile float* __restrict__ terms, float* __restrict__ aux) {
+  PB_GRID_WAIT();
   __shared__ float red[AUX_ROWS][AUX_COLS + 1];
   const int c = threadIdx.x % AUX_COLS, g = threadIdx.x / AUX_COLS, e = blockIdx.x * AUX_COLS + c;
   float s = 0.f;
@@ -226,6 +228,7 @@ router_bwd_kernel(const float* __restrict__ dprobs, const float* __restrict__ df
                   const int* __restrict__ idx, const float* __restrict__ probs, int T, int E, int k, int sigmoid,
                   int pre_softmax, float scale, const float* __restrict__ daux, const int* __restrict__ counts, float aux_factor,
                   TOut* __restrict__ dlogits) {
+  PB_GRID_WAIT();
   extern __shared__ float smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * WARPS + warp;
@@ -297,11 +300,12 @@ static int router_fwd(const void* logits, int in_bf16, const float* bias, int T,
     if (rc) return rc;
   }
   if (in_bf16)
-    router_fwd_kernel<__nv_bfloat16><<<blocks, WARPS * 32, smem, s>>>(
+    pbh::launch_dependent(router_fwd_kernel<__nv_bfloat16>, blocks, WARPS * 32, smem, s,
         reinterpret_cast<const __nv_bfloat16*>(logits), bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk,
         scale, probs, idx, idx64, full, counts, score_sums);
   else
-    router_fwd_kernel<float><<<blocks, WARPS * 32, smem, s>>>(reinterpret_cast<const float*>(logits), bias, T, E, k,
+    pbh::launch_dependent(router_fwd_kernel<float>, blocks, WARPS * 32, smem, s, reinterpret_cast<const float*>(logits), bias, T,
+        E, k,
                                                               sigmoid, pre_softmax, num_groups, group_topk, scale, probs,
                                                               idx, idx64, full, counts, score_sums);
   return (int)cudaGetLastError();
@@ -325,8 +329,8 @@ int pb_moe_route(const void* logits, int in_bf16, const float* bias, int T, int 
   const int rc = router_fwd(logits, in_bf16, bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk, scale, probs, idx, idx64, full,
                             ws, aux ? score_sums : nullptr, s);
   if (rc || !aux) return rc;
-  aux_loss_kernel<<<(E + AUX_COLS - 1) / AUX_COLS, AUX_COLS * AUX_ROWS, 0, s>>>(
-      score_sums, ws, (T + WARPS - 1) / WARPS, T, E, k, aux_factor, ws + E, reinterpret_cast<float*>(ws + E + 1), aux);
+  pbh::launch_dependent(aux_loss_kernel, (E + AUX_COLS - 1) / AUX_COLS, AUX_COLS * AUX_ROWS, 0, s, score_sums, ws,
+      (T + WARPS - 1) / WARPS, T, E, k, aux_factor, ws + E, reinterpret_cast<float*>(ws + E + 1), aux);
   return (int)cudaGetLastError();
 }
 
@@ -339,10 +343,12 @@ int pb_router_bwd(const float* dprobs, const float* dfull, const float* full, co
   const int blocks = (T + WARPS - 1) / WARPS;
   const size_t smem = (size_t)WARPS * E * sizeof(float);
   if (out_bf16)
-    router_bwd_kernel<__nv_bfloat16><<<blocks, WARPS * 32, smem, s>>>(dprobs, dfull, full, idx, probs, T, E, k, sigmoid, pre_softmax,
+    pbh::launch_dependent(router_bwd_kernel<__nv_bfloat16>, blocks, WARPS * 32, smem, s, dprobs, dfull, full, idx, probs, T, E, k,
+        sigmoid, pre_softmax,
                                                                       scale, daux, counts, aux_factor, (__nv_bfloat16*)dlogits);
   else
-    router_bwd_kernel<float><<<blocks, WARPS * 32, smem, s>>>(dprobs, dfull, full, idx, probs, T, E, k, sigmoid, pre_softmax, scale,
+    pbh::launch_dependent(router_bwd_kernel<float>, blocks, WARPS * 32, smem, s, dprobs, dfull, full, idx, probs, T, E, k, sigmoid,
+        pre_softmax, scale,
                                                               daux, counts, aux_factor, (float*)dlogits);
   return (int)cudaGetLastError();
 }
