@@ -336,51 +336,113 @@ ce_grad_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ labe
   }
 }
 
-// Single-rank fused form: loss[row] = lse - target, gradient written in place.
-__global__ void __launch_bounds__(CE_THREADS)
-ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ labels,
-                const float* __restrict__ gscale, float* __restrict__ loss, int V, long ld) {
+// Single-rank fused form: loss[row] = lse - target, gradient written in place.  A CTA takes a row, sums it and reads it again.
+// What bounded it was instructions (80 % of the issue slots at 1480 x 128256, half of the memory's rate), so two values go into one
+// packed operation wherever there is one, the exponentials' care for denormals is left to vectors that have any, and the target
+// to its owner before and after the loop.  Then it is the memory, twice the logits as long as the second reading comes from L2:
+//   HOLD = 0: four rows per SM under way, which have to fit into L2;
+//   HOLD > 0: two, of whose vectors a thread keeps its first HOLD (all there: V >= 8 THREADS HOLD) in shared memory, and results
+//   leave by stores that make way in L2.
+// us, before and now: 4096 x 128256 494 -> 358, 1024 x 202048 226 -> 176, 4096 x 50304 223 -> 153, 4096 x 32000 153 -> 94, 768 x
+// 32000 39 -> 27, 20000 x 1000 173 -> 75.  (A CTA per SM that stays, with its row and the next ones' start in a ring of
+// asynchronous copies: 450 us for the first, as its SM moves nothing between sums and gradient.)
+constexpr int CE_HOLD = 6;
+template <int THREADS, int CTAS, int HOLD, int U>
+__global__ void __launch_bounds__(THREADS, CTAS)
+ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ labels, const float* __restrict__ gscale,
+                float* __restrict__ loss, int V, long ld) {
   PB_GRID_WAIT();
-  __shared__ float red[32];
+  extern __shared__ __align__(16) uint8_t held_raw[];
+  __shared__ float2 red[THREADS / 32];
+  constexpr float LOG2E = 1.4426950408889634f;
+  const int tid = threadIdx.x, nv = V / 8;
   const long row = blockIdx.x;
-  Bf8* lr = reinterpret_cast<Bf8*>(logits + row * ld);
-  const int nv = V / 8;
-  float m = -INFINITY, s = 0.f;
-  for (int i = threadIdx.x; i < nv; i += CE_THREADS) {
-    float f[8];
-    bf8_to_f(lr[i], f);
-    float lm = f[0];
-#pragma unroll
-    for (int j = 1; j < 8; ++j) lm = fmaxf(lm, f[j]);
+  uint4* held = reinterpret_cast<uint4*>(held_raw) + tid;                // [HOLD][thread]
+  uint4* lr = reinterpret_cast<uint4*>(logits + row * ld);
+  const uint64_t one2 = pb::pack_f32x2(1.f, 1.f), log2e2 = pb::pack_f32x2(LOG2E, LOG2E);
+  // (f + neg) log2(e) of a word's two values
+  auto scaled = [&](uint32_t w, uint64_t neg) {
+    const uint64_t f = pb::pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+    return pb::mul_f32x2(pb::fma_f32x2(f, one2, neg), log2e2);
+  };
+  float m = -3.402823466e38f;    // (finite: nothing but -inf so far adds 0, not a NaN)
+  uint64_t s2 = 0;               // sums of the even and the odd values' exp(f - m)
+  auto sum = [&](const uint4 v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    const float lm = pb::max_bf16x2(pb::max2_bf16x2(pb::max2_bf16x2(w[0], w[1]), pb::max2_bf16x2(w[2], w[3])));
     if (lm > m) {
-      s *= __expf(m - lm);
+      const float c = pb::fast_exp2((m - lm) * LOG2E);
+      s2 = pb::mul_f32x2(s2, pb::pack_f32x2(c, c));
       m = lm;
     }
+    const uint64_t neg = pb::pack_f32x2(-m, -m);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) s += __expf(f[j] - m);
-  }
-  const float gm = block_max<CE_THREADS>(m, red);
-  s = (m == -INFINITY) ? 0.f : s * __expf(m - gm);
-  s = block_sum<CE_THREADS>(s, red);
-  const float l = gm + __logf(s);
-  const long lab = labels[row];
-  if (threadIdx.x == 0) {
-    const float t = (lab >= 0 && lab < V) ? __bfloat162float(logits[row * ld + lab]) : l;
-    loss[row] = l - t;
-  }
-  __syncthreads();  // the target logit must be read before it is overwritten
-  const float sc = gscale[row];
-  for (int i = threadIdx.x; i < nv; i += CE_THREADS) {
-    float f[8];
-    bf8_to_f(lr[i], f);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float p = __expf(f[j] - l);
-      if ((long)i * 8 + j == lab) p -= 1.f;
-      f[j] = p * sc;
+    for (int q = 0; q < 4; ++q) {
+      float a, b;
+      pb::unpack_f32x2(scaled(w[q], neg), a, b);
+      s2 = pb::fma_f32x2(pb::pack_f32x2(pb::fast_exp2(a), pb::fast_exp2(b)), one2, s2);
     }
-    lr[i] = f_to_bf8(f);
+  };
+  int i = tid;
+#pragma unroll 1
+  for (int h = 0; h < HOLD; h += U) {
+    uint4 v[U];
+#pragma unroll
+    for (int k = 0; k < U; ++k) v[k] = __ldcs(lr + i + k * THREADS);
+#pragma unroll
+    for (int k = 0; k < U; ++k) {
+      held[(h + k) * THREADS] = v[k];
+      sum(v[k]);
+    }
+    i += U * THREADS;
   }
+  for (; i < nv; i += THREADS) sum(lr[i]);
+  const long lab = labels[row];
+  const float sc = gscale[row];
+  float s, s1;
+  pb::unpack_f32x2(s2, s, s1);
+  const float wm = pb::warp_max(m);
+  s = pb::warp_sum((s + s1) * pb::fast_exp2((m - wm) * LOG2E));
+  if ((tid & 31) == 0) red[tid >> 5] = make_float2(wm, s);
+  __syncthreads();
+  const float2 r = red[tid & (THREADS / 32 - 1)];
+  const float gm = pb::warp_max(r.x);
+  s = r.y * pb::fast_exp2((r.x - gm) * LOG2E);
+  const float l = gm + __logf(pb::warp_sum((tid & 31) < THREADS / 32 ? s : 0.f));
+  // the target's logit belongs to the thread that will write its vector
+  const bool has_label = lab >= 0 && lab < V, own_label = has_label && tid == (int)(lab / 8) % THREADS;
+  float t = l;
+  if (own_label) t = __bfloat162float(logits[row * ld + lab]);
+  if (has_label ? own_label : tid == 0) loss[row] = l - t;
+  const uint64_t neg = pb::pack_f32x2(-l, -l), sc2 = pb::pack_f32x2(sc, sc);
+  const float low = l - 86.f;    // exp(-86) is a normal number
+  auto grad = [&](const uint4 v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+    float p[8];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pb::unpack_f32x2(scaled(w[q], neg), p[2 * q], p[2 * q + 1]);
+    if (pb::min_bf16x2(pb::min2_bf16x2(pb::min2_bf16x2(w[0], w[1]), pb::min2_bf16x2(w[2], w[3]))) > low) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) p[j] = pb::fast_exp2(p[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) asm("ex2.approx.f32 %0, %0;" : "+f"(p[j]));
+    }
+    uint32_t g[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float a, b;
+      pb::unpack_f32x2(pb::mul_f32x2(pb::pack_f32x2(p[2 * q], p[2 * q + 1]), sc2), a, b);
+      g[q] = pb::pack_bf16x2(a, b);
+    }
+    if (HOLD) __stcs(lr + i, make_uint4(g[0], g[1], g[2], g[3]));
+    else lr[i] = make_uint4(g[0], g[1], g[2], g[3]);
+  };
+  i = tid;
+#pragma unroll 2
+  for (int h = 0; h < HOLD; ++h, i += THREADS) grad(held[h * THREADS]);
+  for (; i < nv; i += THREADS) grad(HOLD ? __ldcs(lr + i) : lr[i]);
+  if (own_label) logits[row * ld + lab] = __float2bfloat16_rn((__expf(t - l) - 1.f) * sc);
 }
 
 // out[0] = sum of x[i] * w[i], in a fixed order (the loss of a micro-batch from its tokens')
@@ -842,7 +904,17 @@ int pb_ce_fused(void* logits, const long* labels, const float* gscale, float* lo
                 long ld, cudaStream_t s) {
   if (V % 8 || ld % 8) return -2;
   if (rows == 0) return 0;
-  pbh::launch_dependent(ce_fused_kernel, (unsigned)rows, CE_THREADS, 0, s, (__nv_bfloat16*)logits, labels, gscale, loss, V, ld);
+  __nv_bfloat16* l = (__nv_bfloat16*)logits;
+  // (us, four rows and two: V = 32000 94 and 123, 50304 153 and 165, 65536 209 and 204, 81920 277 and 235, 128256 480 and 358)
+  if (V <= 57344) {
+    pbh::launch_dependent(ce_fused_kernel<512, 4, 0, 1>, (unsigned)rows, 512, 0, s, l, labels, gscale, loss, V, ld);
+  } else {
+    static std::atomic<bool> allowed[pbh::MAX_DEVICES];
+    auto kern = ce_fused_kernel<1024, 2, CE_HOLD, 3>;
+    constexpr int BYTES = CE_HOLD * 1024 * 16;
+    if (int rc = pbh::allow_shared_memory(kern, BYTES, allowed)) return rc;
+    pbh::launch_dependent(kern, (unsigned)rows, 1024, BYTES, s, l, labels, gscale, loss, V, ld);
+  }
   PB_CHECK_LAUNCH();
 }
 

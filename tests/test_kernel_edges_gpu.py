@@ -213,3 +213,35 @@ def test_cross_entropy_masked_and_ragged(V):
     loss.sum().backward()
     assert (loss.double() - loss64).abs().max() <= 1e-5 * (1 + loss64.abs().max())
     _close_bf16(xl.grad, ref.grad, "dlogits")
+
+
+@pytest.mark.parametrize("V", [8, 4096, 57344, 57352, 131072])
+@pytest.mark.parametrize("pad", [0, 24])
+def test_cross_entropy_rows_with_pitch_spread_and_start_masks(V, pad):
+    """The edges between the variants; rows with a pitch, a mask in front, probabilities that are no normal numbers, labels out of
+    range (no target: loss 0, gradient the softmax)."""
+    g = _gen(V + pad)
+    T = 6
+    x = (torch.randn(T, V + pad, device="cuda", generator=g) * 4).bfloat16()
+    x[1, : V - 3] = float("-inf")
+    x[2, ::3] -= 95.0
+    x[3, 1:V] -= 300.0
+    lab = torch.randint(0, V, (T,), device="cuda", generator=g)
+    lab[0], lab[1], lab[4], lab[5] = 0, V - 1, -100, V
+    scale = torch.rand(T, device="cuda", generator=g) + 0.5
+    want = x.clone()
+    lse = torch.logsumexp(x[:, :V].double(), 1)
+    p = (x[:, :V].double() - lse[:, None]).exp()
+    rows = torch.arange(4, device="cuda")
+    loss64 = torch.zeros(T, device="cuda", dtype=torch.float64)
+    loss64[:4] = lse[:4] - x[rows, lab[:4]].double()
+    p[rows, lab[:4]] -= 1
+    want[:, :V] = (p * scale.double()[:, None]).bfloat16()
+    loss = torch.empty(T, device="cuda")
+    _lib.call("ce_fused", x, lab, scale, loss, T, V, x.stride(0))
+    assert torch.equal(x[:, V:], want[:, V:])
+    # fp32 sums of 8 to 131072 terms in pairs of chains and trees: a few 2^-24 of the sum, and of the log-sum-exp itself
+    assert (loss.double() - loss64).abs().max() <= 1e-5 * (1 + lse.abs().max())
+    # exponents of up to 2^-16 absolute at |f - lse| of 300, one rounding to bf16; below 2^-126 an exponential has 2^-149 at best
+    err = (x[:, :V].double() - want[:, :V].double()).abs()
+    assert (err <= 2.0 ** -7 * want[:, :V].double().abs() + 2.0 ** -22 * (lab < V)[:, None] + 2.0 ** -133).all()
