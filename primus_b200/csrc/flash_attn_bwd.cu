@@ -1123,8 +1123,11 @@ flash_attn_bwd_wide_kernel(const __grid_constant__ CUtensorMap tmX1, const __gri
 // delta[b, h, s] = sum_d dO * O ;  neg_lse2 = -lse * log2(e) (the addend of the main kernels' exponent).
 // A CTA takes 32 positions x 8 heads.  DV / 8 lanes share a (position, head) row, neighbouring rows of the same position
 // are neighbours in memory, so a warp reads whole 128-byte lines; the 32 sums of a head then leave as one 128-byte line.
+// What bounds it are the loads in flight: of U rows per thread, few where many CTAs share an SM (more of them fit by their registers),
+// many where there are at most two CTAs per SM.  us, four rows before and now: 8192 x 32 x 128 31.5 -> 26.3, 4096 x 64 x 64 16.2 ->
+// 11.8, both with two; 4096 x 16 x 128 12.2 -> 10.3, 1024 x 16 x 128 7.5 -> 6.4, with eight (with two 13.7 for the former).
 constexpr int DL_POS = 32, DL_HEADS = 8, DL_THREADS = 256;
-template <int DV>
+template <int DV, int U>
 __global__ void __launch_bounds__(DL_THREADS)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   const float* __restrict__ lse, float* __restrict__ delta, float* __restrict__ neg_lse2, int seq, int hq,
@@ -1139,10 +1142,10 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
   const int h0 = blockIdx.y * DL_HEADS;
   const int lane = threadIdx.x % LANES, grp = threadIdx.x / LANES;
 #pragma unroll 1
-  for (int i0 = 0; i0 < ITERS; i0 += 4) {
-    uint4 x[4], y[4];
+  for (int i0 = 0; i0 < ITERS; i0 += U) {
+    uint4 x[U], y[U];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < U; ++i) {
       const int item = (i0 + i) * GROUPS + grp, p = item / DL_HEADS, h = h0 + item % DL_HEADS;
       x[i] = y[i] = make_uint4(0, 0, 0, 0);
       if (h < hq) {
@@ -1151,7 +1154,7 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
       }
     }
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < U; ++i) {
       const int item = (i0 + i) * GROUPS + grp;
       const __nv_bfloat162* xa = reinterpret_cast<const __nv_bfloat162*>(&x[i]);
       const __nv_bfloat162* ya = reinterpret_cast<const __nv_bfloat162*>(&y[i]);
@@ -1268,9 +1271,10 @@ int launch_bwd(const BwdArgs& a) {
   const auto bf = CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
   const auto sw = CU_TENSOR_MAP_SWIZZLE_128B;
   const long T = (long)a.batch * a.seq;
-  pbh::launch_dependent(attn_delta_kernel<DV>, dim3((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS), DL_THREADS, 0,
-      a.stream, (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse, a.delta, a.neg_lse2, a.seq,
-      a.hq, a.o_row, a.do_row);
+  const dim3 grid_delta((unsigned)(T / DL_POS), (a.hq + DL_HEADS - 1) / DL_HEADS);
+  auto delta_kern = (long)grid_delta.x * grid_delta.y > 148 * 2 ? attn_delta_kernel<DV, 2> : attn_delta_kernel<DV, 8>;
+  pbh::launch_dependent(delta_kern, grid_delta, DL_THREADS, 0, a.stream, (const __nv_bfloat16*)a.o, (const __nv_bfloat16*)a.d_o, a.lse,
+                        a.delta, a.neg_lse2, a.seq, a.hq, a.o_row, a.do_row);
   int rc;
   CUtensorMap q128, do128, k128, v128, dq_m, dk_m, dv_m;
   const long TK = (long)a.batch * a.seq_k;
