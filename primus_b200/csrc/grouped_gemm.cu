@@ -73,7 +73,10 @@ struct Tile {
 //                   group before the next: the CTAs in flight then share a few experts' weights and their rows, which are
 //                   read from memory once.  (Running over all row blocks of a column block first re-read the activations,
 //                   150 MB at 36k rows of 2048, from memory once per column block.)
-// MODE wgrad      : tiles = E x num_m x num_n over D[e][N_out, K_out]
+// MODE wgrad      : tiles = E x num_m x num_n over D[e][N_out, K_out], n fastest: what bounds it is the fp32 gradient's way to memory
+//                   and back, which then runs along its rows, and a wave needs fewer operand columns (both of an accumulating layer,
+//                   us, m and n fastest: 64 experts of 2048 x 768, 512 rows each 504 and 494; 32 of 4096 x 1536, 256 rows 1000 and
+//                   957; 8 of 2048 x 4096, 1024 rows 456 and 445; 16 of 2048 x 1408, 2048 rows 498 and 496).
 template <int MODE>
 __device__ __forceinline__ Tile get_tile(int tile, int num_m, int num_n, int K, const int* __restrict__ mblock_expert,
                                          const int* __restrict__ row_start, const int* __restrict__ padded) {
@@ -95,8 +98,8 @@ __device__ __forceinline__ Tile get_tile(int tile, int num_m, int num_n, int K, 
     const int e = tile / per_e;
     const int r = tile - e * per_e;
     t.expert = e;
-    t.m0 = (r % num_m) * BM;
-    t.n0 = (r / num_m) * BN;
+    t.m0 = (r / num_n) * BM;
+    t.n0 = (r % num_n) * BN;
     t.k_begin = row_start[e] / BK;
     t.k_blocks = padded[e] / BK;
     t.valid = 1;  // experts without tokens still run the epilogue with an untouched (zero) accumulator
