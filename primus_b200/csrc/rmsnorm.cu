@@ -116,8 +116,12 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
 // slots of shared memory, as in the backward; a CTA per row spends its life waiting for its loads, then for its sum (16384 x
 // 8192 with residual 183 us, this 172, without 121 and 89; 8192 x 4096 50 and 46, 30 and 23; 1300 x 8192 19 and 14).  Sums in the
 // order of the kernel above.  (Three rows ahead or eight CTAs per SM are no faster: 8192 x 5120 63 us against 56.)
-constexpr int FWD_STAGES = 2, FWD_CTAS = 4;
-inline bool fwd_ring(long rows, int H) { return H > 2048 && rows >= 148 * 8; }
+// Rows of up to 2048 want twice the CTAs, pay from 16 rows per SM on and without residual: 4096 x 2048 14.3 -> 12.3 us, 16384 x 2048
+// 34.8 -> 28.7, 8192 x 1536 18.5 -> 15.4, 2000 x 2048 9.2 -> 10.2; with residual 52.2 -> 53.2 and 24.6 -> 24.6.
+constexpr int FWD_STAGES = 2;
+inline bool fwd_ring(long rows, int H, bool residual) {
+  return H > 2048 ? rows >= 148 * 8 : H > 1024 && !residual && rows >= 148 * 16;
+}
 template <int VPT, int THREADS, bool RES>
 __global__ void __launch_bounds__(THREADS)
 rmsnorm_fwd_ring_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ res,
@@ -198,7 +202,7 @@ rmsnorm_fwd_ring_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
   }
 }
 
-template <int VPT, int THREADS, bool RES>
+template <int VPT, int THREADS, int CTAS, bool RES>
 int launch_rmsnorm_fwd_ring(cudaStream_t s, const __nv_bfloat16* x, const __nv_bfloat16* res, const __nv_bfloat16* w, __nv_bfloat16* y,
                             __nv_bfloat16* xsum, float* rstd, long rows, int H, long ldx, long ldy, float eps) {
   constexpr int BYTES = FWD_STAGES * (RES ? 2 : 1) * VPT * THREADS * 16;
@@ -208,9 +212,8 @@ int launch_rmsnorm_fwd_ring(cudaStream_t s, const __nv_bfloat16* x, const __nv_b
   static std::atomic<bool> allowed[pbh::MAX_DEVICES];
   const int rc = pbh::allow_shared_memory(kern, BYTES, allowed);
   if (rc) return rc;
-  pbh::launch_dependent(kern, (unsigned)(pbh::sm_count() * (PER_SM < FWD_CTAS ? PER_SM : FWD_CTAS)), THREADS, BYTES, s, x, res, w,
-      y,
-                        xsum, rstd, rows, H, ldx, ldy, eps);
+  pbh::launch_dependent(kern, (unsigned)(pbh::sm_count() * (PER_SM < CTAS ? PER_SM : CTAS)), THREADS, BYTES, s, x, res, w, y, xsum,
+                        rstd, rows, H, ldx, ldy, eps);
   return 0;
 }
 
@@ -878,14 +881,15 @@ int pb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void*
                    long rows, int H, long ldx, long ldy, float eps, cudaStream_t s) {
   if (H % 8 || ldx % 8 || ldy % 8 || H > 16384) return -2;
   if (rows == 0) return 0;
-  if (fwd_ring(rows, H)) {
-#define PB_NORM_FWD_RING(VPT, THREADS, RES)                                                                                  \
-  launch_rmsnorm_fwd_ring<VPT, THREADS, RES>(s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, \
-                                             (__nv_bfloat16*)y, (__nv_bfloat16*)xsum, rstd, rows, H, ldx, ldy, eps)
-    int rc;
-    if (H <= 4096) rc = res ? PB_NORM_FWD_RING(4, 128, true) : PB_NORM_FWD_RING(4, 128, false);
-    else if (H <= 8192) rc = res ? PB_NORM_FWD_RING(4, 256, true) : PB_NORM_FWD_RING(4, 256, false);
-    else rc = res ? PB_NORM_FWD_RING(8, 256, true) : PB_NORM_FWD_RING(8, 256, false);
+  if (fwd_ring(rows, H, res)) {
+#define PB_NORM_FWD_RING(VPT, THREADS, CTAS)                                                                     \
+  (res ? launch_rmsnorm_fwd_ring<VPT, THREADS, CTAS, true> : launch_rmsnorm_fwd_ring<VPT, THREADS, CTAS, false>) \
+  (s, (const __nv_bfloat16*)x, (const __nv_bfloat16*)res, (const __nv_bfloat16*)w, (__nv_bfloat16*)y,            \
+   (__nv_bfloat16*)xsum, rstd, rows, H, ldx, ldy, eps)
+    const int rc = H <= 2048   ? launch_rmsnorm_fwd_ring<4, 64, 8, false>(s, (const __nv_bfloat16*)x, nullptr, (const __nv_bfloat16*)w,
+                                                                         (__nv_bfloat16*)y, nullptr, rstd, rows, H, ldx, ldy, eps)
+                   : H <= 4096 ? PB_NORM_FWD_RING(4, 128, 4)
+                   : H <= 8192 ? PB_NORM_FWD_RING(4, 256, 4) : PB_NORM_FWD_RING(8, 256, 4);
 #undef PB_NORM_FWD_RING
     return rc ? rc : (int)cudaGetLastError();
   }

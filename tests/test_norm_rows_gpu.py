@@ -115,8 +115,8 @@ def test_backward_gives_the_normalised_rows_again(rows, H, residual, two):
     assert (got[0].data_ptr() != got[1].data_ptr()) == two
 
 
-@pytest.mark.parametrize("rows", [1183, 1184, 1185, 2400])
-@pytest.mark.parametrize("H", [2048, 2056, 4096, 4104, 8192, 8200, 16384])
+@pytest.mark.parametrize("rows", [1183, 1184, 1185, 2367, 2368, 2400])
+@pytest.mark.parametrize("H", [1024, 1032, 1544, 2048, 2056, 4096, 4104, 8192, 8200, 16384])
 @pytest.mark.parametrize("residual", [False, True])
 def test_forward_around_the_rows_that_ctas_stay_for(rows, H, residual):
     """The kernel of many rows gives the bits of the one for few (the same rows in two halves)."""
