@@ -408,7 +408,8 @@ ce_fused_kernel(__nv_bfloat16* __restrict__ logits, const long* __restrict__ lab
   const float2 r = red[tid & (THREADS / 32 - 1)];
   const float gm = pb::warp_max(r.x);
   s = r.y * pb::fast_exp2((r.x - gm) * LOG2E);
-  const float l = gm + __logf(pb::warp_sum((tid & 31) < THREADS / 32 ? s : 0.f));
+  // (logf: mean error of the loss against 64 bits 3.0e-7 at 512 x 8192, 2.8e-7 at 128 x 128256; with __logf 3.6e-7 and 4.0e-7)
+  const float l = gm + logf(pb::warp_sum((tid & 31) < THREADS / 32 ? s : 0.f));
   // the target's logit belongs to the thread that will write its vector
   const bool has_label = lab >= 0 && lab < V, own_label = has_label && tid == (int)(lab / 8) % THREADS;
   float t = l;
