@@ -349,10 +349,23 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
   }
 }
 
+// word j of a vector as two fp32 values and back
+__device__ __forceinline__ uint64_t widen(const Bf8& b, int j) {
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&b.v[j]);
+  return pb::pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ void narrow(uint64_t f, Bf8& b, int j) {
+  float lo, hi;
+  pb::unpack_f32x2(f, lo, hi);
+  b.v[j] = __floats2bfloat162_rn(lo, hi);
+}
+
 // Longer rows: one CTA per row, persistent over rows blockIdx.x, blockIdx.x + gridDim.x, ...  Every thread keeps a ring
 // of STAGES rows of its own vectors in shared memory, filled by its own 16-byte cp.async copies, so loads run several
 // rows ahead of the block reductions without holding registers; the reduction is the only barrier of a row (its slots
-// alternate).
+// alternate).  Two channels share an fp32 instruction but for the row sum, whose order stands, and the residual, whose packed
+// addend would spill: us with single values and now, 16384 x 8192 with residual 175 -> 165, 8192 x 4096 52.2 -> 50.2 and 44 -> 42
+// without, 16384 x 2048 without 50 -> 46.
 template <int VPT, int THREADS, bool RES, bool Y>
 __global__ void __launch_bounds__(THREADS, THREADS == 256 ? 2 : 1)
 rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
@@ -368,11 +381,11 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   const int tid = threadIdx.x;
   const int nv = H / 8;
   Bf8 wv[VPT];
-  float dw[VPT][8];
+  uint64_t dw[VPT][4];
 #pragma unroll
   for (int k = 0; k < VPT; ++k) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
+    for (int j = 0; j < 4; ++j) dw[k][j] = 0;
     if (tid + k * THREADS < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[tid + k * THREADS];
   }
   auto fetch = [&](long row, int st) {
@@ -405,6 +418,7 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
     wait_oldest();
     const Bf8* slot = ring + (long)st * OPS * VPT * THREADS + tid;
     Bf8 vx[VPT], vg[VPT], vr[VPT];
+    const uint64_t rs2 = pb::pack_f32x2(rs, rs);
     float dot = 0.f;
 #pragma unroll
     for (int k = 0; k < VPT; ++k)
@@ -412,20 +426,19 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
         vx[k] = slot[k * THREADS];
         vg[k] = slot[(VPT + k) * THREADS];
         if (RES) vr[k] = slot[(2 * VPT + k) * THREADS];
-        float fx[8], fg[8], fw[8];
-        bf8_to_f(vx[k], fx);
-        bf8_to_f(vg[k], fg);
-        bf8_to_f(wv[k], fw);
+        Bf8 yv;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          dw[k][j] += fg[j] * fx[j] * rs;
-          dot += fg[j] * fw[j] * fx[j];
+        for (int j = 0; j < 4; ++j) {
+          const uint64_t px = widen(vx[k], j), pg = widen(vg[k], j), pw = widen(wv[k], j);
+          dw[k][j] = pb::fma_f32x2(pb::mul_f32x2(pg, px), rs2, dw[k][j]);
+          float x0, x1, d0, d1;
+          pb::unpack_f32x2(px, x0, x1);
+          pb::unpack_f32x2(pb::mul_f32x2(pg, pw), d0, d1);
+          dot = fmaf(d0, x0, dot);
+          dot = fmaf(d1, x1, dot);
+          if (Y) narrow(pb::mul_f32x2(pb::mul_f32x2(px, rs2), pw), yv, j);
         }
-        if (Y) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) fw[j] = fx[j] * rs * fw[j];
-          reinterpret_cast<Bf8*>(y + row * ldx)[tid + k * THREADS] = f_to_bf8(fw);
-        }
+        if (Y) reinterpret_cast<Bf8*>(y + row * ldx)[tid + k * THREADS] = yv;
       }
     dot = pb::warp_sum(dot);
     if ((tid & 31) == 0) red[flip][tid >> 5] = dot;
@@ -436,21 +449,19 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
 #pragma unroll
     for (int i = 0; i < THREADS / 32; ++i) dot += red[flip][i];
     const float c = dot * rs * rs * rs / H;
+    const uint64_t c2 = pb::pack_f32x2(-c, -c);
 #pragma unroll
     for (int k = 0; k < VPT; ++k)
       if (tid + k * THREADS < nv) {
-        float fx[8], fg[8], fw[8], o[8];
-        bf8_to_f(vx[k], fx);
-        bf8_to_f(vg[k], fg);
-        bf8_to_f(wv[k], fw);
+        Bf8 ob;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) o[j] = fg[j] * fw[j] * rs - fx[j] * c;
-        if (RES) {
-          bf8_to_f(vr[k], fx);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] += fx[j];
+        for (int j = 0; j < 4; ++j) {
+          const uint64_t gw = pb::mul_f32x2(widen(vg[k], j), widen(wv[k], j)), px = widen(vx[k], j);
+          float o0, o1, r0 = 0.f, r1 = 0.f;
+          pb::unpack_f32x2(pb::fma_f32x2(gw, rs2, pb::mul_f32x2(px, c2)), o0, o1);
+          if (RES) pb::unpack_f32x2(widen(vr[k], j), r0, r1);
+          ob.v[j] = RES ? __floats2bfloat162_rn(o0 + r0, o1 + r1) : __floats2bfloat162_rn(o0, o1);
         }
-        const Bf8 ob = f_to_bf8(o);
         reinterpret_cast<Bf8*>(dx + row * ldx)[tid + k * THREADS] = ob;
         if (RES && dx2) reinterpret_cast<Bf8*>(dx2 + row * ldx)[tid + k * THREADS] = ob;
       }
@@ -462,8 +473,13 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __
   for (int k = 0; k < VPT; ++k)
     if (tid + k * THREADS < nv) {
       float4* p = reinterpret_cast<float4*>(partial + (long)blockIdx.x * H + (long)(tid + k * THREADS) * 8);
-      p[0] = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
-      p[1] = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        float4 v;
+        pb::unpack_f32x2(dw[k][2 * q], v.x, v.y);
+        pb::unpack_f32x2(dw[k][2 * q + 1], v.z, v.w);
+        p[q] = v;
+      }
     }
 }
 
