@@ -249,9 +249,40 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 // residual: 54 + 31 us in two passes, 64 in one; 4096 x 2048 21 + 10 and 22).
 // dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
 
+// word j of a vector as two fp32 values and back
+__device__ __forceinline__ uint64_t widen(const Bf8& b, int j) {
+  const uint32_t w = *reinterpret_cast<const uint32_t*>(&b.v[j]);
+  return pb::pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
+}
+__device__ __forceinline__ void narrow(uint64_t f, Bf8& b, int j) {
+  float lo, hi;
+  pb::unpack_f32x2(f, lo, hi);
+  b.v[j] = __floats2bfloat162_rn(lo, hi);
+}
+
 // Rows of up to 1024 channels: LPR <= 32 lanes per row, no barrier in the loop, RPG rows per group in flight.  The dw
 // sums of a CTA's groups meet in shared memory at the end.
-template <int LPR, int VPL, int RPG, bool Y>
+// PACKED: two channels per fp32 instruction (the same bits; us without and with: 262144 x 192 91 -> 83, 262144 x 128 52 -> 48, 32768 x 512
+// with residual 33.8 -> 31.7, 32768 x 1024 52 -> 46).  Rows of more than 512 with a residual hold too much for register pairs: 16384 x
+// 1024 36 -> 40.
+template <bool PACKED>
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  if (PACKED) return pb::mul_f32x2(a, b);
+  float a0, a1, b0, b1;
+  pb::unpack_f32x2(a, a0, a1);
+  pb::unpack_f32x2(b, b0, b1);
+  return pb::pack_f32x2(a0 * b0, a1 * b1);
+}
+template <bool PACKED>
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  if (PACKED) return pb::fma_f32x2(a, b, c);
+  float a0, a1, b0, b1, c0, c1;
+  pb::unpack_f32x2(a, a0, a1);
+  pb::unpack_f32x2(b, b0, b1);
+  pb::unpack_f32x2(c, c0, c1);
+  return pb::pack_f32x2(fmaf(a0, b0, c0), fmaf(a1, b1, c1));
+}
+template <int LPR, int VPL, int RPG, bool Y, bool PACKED>
 __global__ void __launch_bounds__(256, 2)
 rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ x,
                          const __nv_bfloat16* __restrict__ w, const float* __restrict__ rstd,
@@ -264,11 +295,11 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
   const int lane = threadIdx.x % LPR, grp = threadIdx.x / LPR;
   const int nv = H / 8;
   Bf8 wv[VPL];
-  float dw[VPL][8];
+  uint64_t dw[VPL][4];
 #pragma unroll
   for (int k = 0; k < VPL; ++k) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) dw[k][j] = 0.f;
+    for (int j = 0; j < 4; ++j) dw[k][j] = 0;
     if (lane + k * LPR < nv) wv[k] = reinterpret_cast<const Bf8*>(w)[lane + k * LPR];
   }
   const long stride = (long)gridDim.x * GROUPS * RPG;
@@ -291,42 +322,43 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
     }
 #pragma unroll
     for (int r = 0; r < RPG; ++r) {
+      const uint64_t rs2 = pb::pack_f32x2(rs[r], rs[r]);
       float dot = 0.f;
 #pragma unroll
       for (int k = 0; k < VPL; ++k)
         if (row0 + r < rows && lane + k * LPR < nv) {
-          float fx[8], fg[8], fw[8];
-          bf8_to_f(vx[r][k], fx);
-          bf8_to_f(vg[r][k], fg);
-          bf8_to_f(wv[k], fw);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            dw[k][j] += fg[j] * fx[j] * rs[r];
-            dot += fg[j] * fw[j] * fx[j];
-          }
-          if (Y) {
-#pragma unroll
-            for (int j = 0; j < 8; ++j) fw[j] = fx[j] * rs[r] * fw[j];
-            reinterpret_cast<Bf8*>(y + (row0 + r) * ldx)[lane + k * LPR] = f_to_bf8(fw);
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t px = widen(vx[r][k], j), pg = widen(vg[r][k], j), pw = widen(wv[k], j);
+            dw[k][j] = fma2<PACKED>(mul2<PACKED>(pg, px), rs2, dw[k][j]);
+            float x0, x1, d0, d1;
+            pb::unpack_f32x2(px, x0, x1);
+            pb::unpack_f32x2(mul2<PACKED>(pg, pw), d0, d1);
+            dot = fmaf(d0, x0, dot);
+            dot = fmaf(d1, x1, dot);
           }
         }
       dot = group_sum<LPR>(dot, nullptr);
       const float c = dot * rs[r] * rs[r] * rs[r] / H;
+      const uint64_t c2 = pb::pack_f32x2(-c, -c);
 #pragma unroll
       for (int k = 0; k < VPL; ++k)
         if (row0 + r < rows && lane + k * LPR < nv) {
-          float fx[8], fg[8], fw[8], o[8];
-          bf8_to_f(vx[r][k], fx);
-          bf8_to_f(vg[r][k], fg);
-          bf8_to_f(wv[k], fw);
+          Bf8 ob, yv;
 #pragma unroll
-          for (int j = 0; j < 8; ++j) o[j] = fg[j] * fw[j] * rs[r] - fx[j] * c;
-          if (dres) {
-            bf8_to_f(vr[r][k], fx);
-#pragma unroll
-            for (int j = 0; j < 8; ++j) o[j] += fx[j];
+          for (int j = 0; j < 4; ++j) {
+            const uint64_t px = widen(vx[r][k], j), pw = widen(wv[k], j);
+            float o0, o1, r0 = 0.f, r1 = 0.f;
+            pb::unpack_f32x2(fma2<PACKED>(mul2<PACKED>(widen(vg[r][k], j), pw), rs2, mul2<PACKED>(px, c2)), o0, o1);
+            if (Y) narrow(mul2<PACKED>(mul2<PACKED>(px, rs2), pw), yv, j);
+            if (dres) {
+              pb::unpack_f32x2(widen(vr[r][k], j), r0, r1);
+              o0 += r0;
+              o1 += r1;
+            }
+            ob.v[j] = __floats2bfloat162_rn(o0, o1);
           }
-          const Bf8 ob = f_to_bf8(o);
+          if (Y) reinterpret_cast<Bf8*>(y + (row0 + r) * ldx)[lane + k * LPR] = yv;
           reinterpret_cast<Bf8*>(dx + (row0 + r) * ldx)[lane + k * LPR] = ob;
           if (dx2) reinterpret_cast<Bf8*>(dx2 + (row0 + r) * ldx)[lane + k * LPR] = ob;
         }
@@ -334,8 +366,13 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
   }
 #pragma unroll
   for (int k = 0; k < VPL; ++k) {
-    sums[grp][(lane + k * LPR) * 2] = make_float4(dw[k][0], dw[k][1], dw[k][2], dw[k][3]);
-    sums[grp][(lane + k * LPR) * 2 + 1] = make_float4(dw[k][4], dw[k][5], dw[k][6], dw[k][7]);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      float4 v;
+      pb::unpack_f32x2(dw[k][2 * q], v.x, v.y);
+      pb::unpack_f32x2(dw[k][2 * q + 1], v.z, v.w);
+      sums[grp][(lane + k * LPR) * 2 + q] = v;
+    }
   }
   __syncthreads();
   for (int i = threadIdx.x; i < nv * 2; i += 256) {
@@ -347,17 +384,6 @@ rmsnorm_bwd_short_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat
     }
     reinterpret_cast<float4*>(partial + (long)blockIdx.x * H)[i] = t;
   }
-}
-
-// word j of a vector as two fp32 values and back
-__device__ __forceinline__ uint64_t widen(const Bf8& b, int j) {
-  const uint32_t w = *reinterpret_cast<const uint32_t*>(&b.v[j]);
-  return pb::pack_f32x2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
-}
-__device__ __forceinline__ void narrow(uint64_t f, Bf8& b, int j) {
-  float lo, hi;
-  pb::unpack_f32x2(f, lo, hi);
-  b.v[j] = __floats2bfloat162_rn(lo, hi);
 }
 
 // Longer rows: one CTA per row, persistent over rows blockIdx.x, blockIdx.x + gridDim.x, ...  Every thread keeps a ring
@@ -518,7 +544,11 @@ int launch_rmsnorm_bwd(int P, cudaStream_t s, const __nv_bfloat16* dy, const __n
   const int nv = H / 8;
 #define PB_NORM_BWD_SHORT(LPR, VPL, RPG)                                                                               \
   {                                                                                                                    \
-    auto kern = y ? rmsnorm_bwd_short_kernel<LPR, VPL, RPG, (LPR > 8)> : rmsnorm_bwd_short_kernel<LPR, VPL, RPG, false>; \
+    auto kern = VPL == 4 && dres                                                                                       \
+                    ? (y ? rmsnorm_bwd_short_kernel<LPR, VPL, RPG, (LPR > 8), VPL != 4>                                \
+                         : rmsnorm_bwd_short_kernel<LPR, VPL, RPG, false, VPL != 4>)                                   \
+                    : (y ? rmsnorm_bwd_short_kernel<LPR, VPL, RPG, (LPR > 8), true>                                    \
+                         : rmsnorm_bwd_short_kernel<LPR, VPL, RPG, false, true>);                                      \
     pbh::launch_dependent(kern, P, 256, 0, s, dy, x, w, rstd, dres, dx, dx2, y, partial, rows, H, ldx, lddy);                   \
     return (int)cudaGetLastError();                                                                                    \
   }
