@@ -409,9 +409,12 @@ PB_DEVICE void named_bar_sync(int id, int nthreads) {
 // The rules that keep stream order:
 //   - every thread of such a kernel passes grid_wait before it touches memory that others write or read: it returns when the
 //     kernel in front has ended, and with it, as that one waited too, all before it;
+//     The one exception is the dQ pass of the attention backward, which needs nothing of the dK / dV pass in front of it, only
+//     what that one waited for before its release, and waits at its end;
 //   - grid_release lets the kernel behind start once every CTA of this one has called it or ended; without it that one starts
 //     as the last CTAs end.  It pays where a kernel's CTAs are many and short (the quantiser, the row sums of the attention
-//     backward).  Called by every kernel it cost more than it gave, as the CTAs that wait take room that others would fill:
+//     backward) and in front of the dQ pass.  Called by every kernel it cost more than it gave, as the CTAs that wait take room
+//     that others would fill:
 //     the windowed attention 184 -> 188 us, 192 / 128-wide heads 343 -> 350, RMSNorm of 16384 x 8192 380 -> 400.
 // Kernels that wait for other CTAs, flags or ranks are launched the ordinary way, and so are those behind a memset.
 PB_DEVICE void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }

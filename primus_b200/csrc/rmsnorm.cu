@@ -246,7 +246,7 @@ void launch_rmsnorm_fwd(long rows, int H, cudaStream_t s, Args... args) {
 // by itself; inside a model the two inputs are no leaves).  16384 x 8192: a second store 41 us, the copy 83 us.
 // y (optional) receives the normalised rows again, for the weight gradient of a linear layer that followed the norm and does not
 // store its input: x and rstd are here already, and a pass of its own reads x once more (8192 x 4096 with
-// residual: 54 + 31 us in two passes, 64 in one; 4096 x 2048 21 + 10 and 22).
+// residual: 50 + 23 us in two passes, 58 in one; 4096 x 2048 21 + 12 and 23).
 // dw partial sums per CTA go to `partial` [gridDim.x, H]; rmsnorm_dw_reduce_kernel folds them.
 
 // word j of a vector as two fp32 values and back
