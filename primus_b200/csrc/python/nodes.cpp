@@ -428,11 +428,14 @@ struct SwiGLULinear : Function<SwiGLULinear> {
 };
 
 // ------------------------------------------------------------------ attention
-void check_view(const Tensor& t, long d) {     // (attention._check_view, and its class of error)
-  if (t.dim() == 3 && t.stride(2) == 1 && t.stride(1) == d && aligned(t)) return;
+[[noreturn]] void refuse(PyObject* error, const char* why) {
   py::gil_scoped_acquire gil;
-  PyErr_SetString(PyExc_AssertionError, "heads must be contiguous [.., H, D] views");
+  PyErr_SetString(error, why);
   throw py::error_already_set();
+}
+void check_view(const Tensor& t, long d) {     // (attention._check_view, and its class of error)
+  if (t.dim() != 3 || t.stride(2) != 1 || t.stride(1) != d || !aligned(t))
+    refuse(PyExc_AssertionError, "heads must be contiguous [.., H, D] views");
 }
 
 struct AttnArgs {
@@ -503,6 +506,11 @@ struct FlashAttention : Function<FlashAttention> {
   }
 };
 
+// What heads() takes for granted (the Python function's slices and views refuse the rest)
+void check_packed(const Tensor& qkv, long hq, long hkv, long d) {
+  if (qkv.dim() != 2 || qkv.size(1) != (hq + 2 * hkv) * d) refuse(PyExc_RuntimeError, "packed heads must be [T, (Hq + 2 Hkv) D]");
+  if (qkv.stride(1) != 1 || !aligned(qkv)) refuse(PyExc_AssertionError, "packed heads must be contiguous rows");
+}
 // q, k and v heads inside a packed [T, (hq + 2 hkv) d] tensor
 std::tuple<Tensor, Tensor, Tensor> heads(const Tensor& qkv, long hq, long hkv, long d) {
   const long T = qkv.size(0), ld = qkv.stride(0);
@@ -516,6 +524,7 @@ struct RopeAttention : Function<RopeAttention> {
                         double softcap) {
     const Tensor sinks = given(sinks_), cos = given(cos_), sin = given(sin_), pos = given(pos_);
     const AttnArgs a{batch, causal, scale, 0, window, softcap};
+    check_packed(qkv, hq, hkv, d);
     const auto [q, k, v] = heads(qkv, hq, hkv, d);
     // (in place: the projection's output has no other consumer; q and k heads are neighbours)
     if (cos.defined())

@@ -1,0 +1,35 @@
+"""Calls that the Python functions of the layers refuse are refused by the C++ autograd nodes too, with the same class of error and
+before anything is launched.  Here the module is called by itself, on tensors of the host: no case gets as far as a launch."""
+import pytest
+import torch
+
+from primus_b200.ops import _lib, layers
+
+
+@pytest.fixture(scope="module")
+def nodes():
+    with pytest.MonkeyPatch.context() as m:
+        m.setattr(torch.cuda, "is_available", lambda: True)
+        module = _lib._load_nodes()
+    if module is None:
+        pytest.skip("the autograd nodes are not built")
+    return module
+
+
+def _zeros(*shape):
+    return torch.zeros(*shape, dtype=torch.bfloat16)
+
+
+ROPE_ARGS = (None, None, None, 1, 4, 2, 64, 64, True, 0.125)      # no rotation, 4 query and 2 key / value heads of 64
+
+
+@pytest.mark.parametrize("qkv,error", [(lambda: _zeros(128, 520), RuntimeError),                  # 8 heads and 8 columns more
+                                       (lambda: _zeros(128, 512)[:, :448], RuntimeError),         # a head less, of a wider buffer
+                                       (lambda: _zeros(128, 1024)[:, ::2], AssertionError),       # every other column
+                                       (lambda: _zeros(2, 64, 512), RuntimeError)])
+def test_rope_attention_of_other_layouts(nodes, monkeypatch, qkv, error):
+    with pytest.raises(error, match="heads"):
+        nodes.rope_attention(qkv(), *ROPE_ARGS, 0, None, 0.0)
+    monkeypatch.setattr(_lib, "call", lambda *a: None)             # (the Python function, whose launches do nothing)
+    with pytest.raises(error):
+        layers.RopeAttentionFn.apply(qkv(), *ROPE_ARGS)
