@@ -617,6 +617,8 @@ struct CrossEntropy : Function<CrossEntropy> {
     const long V = logits.size(-1);
     const Tensor l2 = as_rows(logits, V), lab = labels.reshape({-1}).contiguous();
     const long rows = l2.size(0);
+    TORCH_CHECK(lab.numel() == rows && (!weights || weights->numel() == rows), "cross entropy of ", rows, " rows: ", lab.numel(), " labels, ",
+                weights ? weights->numel() : rows, " weights");
     const Tensor scale = weights ? weights->reshape({-1}).to(at::kFloat).contiguous() : at::ones({rows}, logits.options().dtype(at::kFloat));
     const Tensor loss = empty({rows}, logits, at::kFloat);
     launch("ce_fused", 1, ptr(l2), ptr(lab), ptr(scale), ptr(loss), rows, V, l2.stride(0));

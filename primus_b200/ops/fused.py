@@ -504,6 +504,8 @@ class CrossEntropyFn(torch.autograd.Function):
         l2 = logits.reshape(-1, V)
         rows = l2.shape[0]
         lab = labels.reshape(-1).contiguous()
+        if lab.numel() != rows or (weights is not None and weights.numel() != rows):     # (the kernels read one of each per row)
+            raise RuntimeError(f"cross entropy of {rows} rows: {lab.numel()} labels, {rows if weights is None else weights.numel()} weights")
         gsc = (weights.reshape(-1).float().contiguous() if weights is not None
                else torch.ones(rows, dtype=torch.float32, device=logits.device))
         loss = torch.empty(rows, dtype=torch.float32, device=logits.device)

@@ -3,7 +3,7 @@ before anything is launched.  Here the module is called by itself, on tensors of
 import pytest
 import torch
 
-from primus_b200.ops import _lib, layers
+from primus_b200.ops import _lib, fused, layers
 
 
 @pytest.fixture(scope="module")
@@ -33,3 +33,17 @@ def test_rope_attention_of_other_layouts(nodes, monkeypatch, qkv, error):
     monkeypatch.setattr(_lib, "call", lambda *a: None)             # (the Python function, whose launches do nothing)
     with pytest.raises(error):
         layers.RopeAttentionFn.apply(qkv(), *ROPE_ARGS)
+
+
+@pytest.mark.parametrize("labels,weights", [(30, 29), (30, 31), (30, 1), (30, 0), (29, 30), (1, 30), (29, 29), (31, None), (29, None)])
+def test_cross_entropy_of_other_lengths(nodes, monkeypatch, labels, weights):
+    logits, labels = _zeros(2, 15, 64), torch.zeros(labels, dtype=torch.int64)
+    weights = None if weights is None else torch.ones(weights)
+    launched = []
+    monkeypatch.setattr(_lib, "call", lambda *a: launched.append(a))
+    for call in (nodes.cross_entropy, lambda x, l, w, unit: fused.CrossEntropyFn.apply(x, l, 0, None, w, unit)):
+        with pytest.raises(RuntimeError, match="30 rows"):
+            call(logits, labels, weights, False)
+    assert not launched
+    with pytest.raises(RuntimeError):                              # the reference of the host's tensors
+        fused.cross_entropy(logits, labels, weights=weights)
