@@ -445,6 +445,10 @@ struct AttnArgs {
   long q_off, window;
   double softcap;
 };
+AttnArgs attn_args(long batch, bool causal, double scale, long q_off, long window, double softcap) {
+  if (batch == 0) refuse(PyExc_ZeroDivisionError, "attention of rows that belong to no sequence");    // (as T // batch does)
+  return {batch, causal, scale, q_off, window, softcap};
+}
 void save_args(AutogradContext* ctx, const AttnArgs& a) {
   ctx->saved_data["args"] = std::vector<int64_t>{a.batch, a.causal, a.q_off, a.window};
   ctx->saved_data["fargs"] = std::vector<double>{a.scale, a.softcap};
@@ -489,7 +493,7 @@ struct FlashAttention : Function<FlashAttention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Opt& sinks_, int64_t batch,
                         bool causal, double scale, int64_t q_off, int64_t window, double softcap) {
     const Tensor sinks = given(sinks_);
-    const AttnArgs a{batch, causal, scale, q_off, window, softcap};
+    const AttnArgs a = attn_args(batch, causal, scale, q_off, window, softcap);
     const auto [o, lse] = attn_forward(q, k, v, sinks, a);
     ctx->save_for_backward({q, k, v, o, lse, sinks});
     save_args(ctx, a);
@@ -523,7 +527,7 @@ struct RopeAttention : Function<RopeAttention> {
                         int64_t batch, int64_t hq, int64_t hkv, int64_t d, int64_t rot_dim, bool causal, double scale, int64_t window,
                         double softcap) {
     const Tensor sinks = given(sinks_), cos = given(cos_), sin = given(sin_), pos = given(pos_);
-    const AttnArgs a{batch, causal, scale, 0, window, softcap};
+    const AttnArgs a = attn_args(batch, causal, scale, 0, window, softcap);
     check_packed(qkv, hq, hkv, d);
     const auto [q, k, v] = heads(qkv, hq, hkv, d);
     // (in place: the projection's output has no other consumer; q and k heads are neighbours)
