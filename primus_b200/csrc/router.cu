@@ -117,22 +117,25 @@ __device__ __forceinline__ int route_token(const TIn* __restrict__ logits, const
     __syncwarp();
   }
 
+  // Every lane proposes the best of its experts that are still free, the first of them if none has a score (NaN and -inf count as
+  // none: a diverged row, or fewer eligible experts than k).  As k <= E, one always is free: the k selections are distinct experts
+  // whatever the row holds, and scores that are no numbers go on into the probabilities.
   float sel_p = 0.f;   // lane j < k keeps the j-th selection
   int sel_i = 0;
+  unsigned taken = 0;  // bit n: expert lane + 32 n
   for (int j = 0; j < k; ++j) {
     float v = -INFINITY;
     int i = 0x7fffffff;
-    for (int e = lane; e < E; e += 32) {
+    for (int e = lane, n = 0; e < E; e += 32, ++n) {
       const float c = ch[e];
-      if (c > v) { v = c; i = e; }
+      if (!((taken >> n) & 1u) && (c > v || i == 0x7fffffff)) { v = fmaxf(c, -INFINITY); i = e; }
     }
-    const ArgMax am = warp_argmax(v, i);
+    i = warp_argmax(v, i).i;
     if (lane == j) {
-      sel_i = am.i;
-      sel_p = (!sigmoid && !pre_softmax) ? am.v : sc[am.i];
+      sel_i = i;
+      sel_p = (!sigmoid && !pre_softmax) ? ch[i] : sc[i];
     }
-    if (lane == (am.i & 31)) ch[am.i] = -INFINITY;
-    __syncwarp();
+    if (lane == (i & 31)) taken |= 1u << (i >> 5);
   }
   const bool act = lane < k;
   if (!sigmoid && !pre_softmax) {
