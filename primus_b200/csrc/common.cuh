@@ -416,7 +416,9 @@ PB_DEVICE void named_bar_sync(int id, int nthreads) {
 //     backward) and in front of the dQ pass.  Called by every kernel it cost more than it gave, as the CTAs that wait take room
 //     that others would fill:
 //     the windowed attention 184 -> 188 us, 192 / 128-wide heads 343 -> 350, RMSNorm of 16384 x 8192 380 -> 400.
-// Kernels that wait for other CTAs, flags or ranks are launched the ordinary way, and so are those behind a memset.
+// Kernels that wait for other CTAs, flags or ranks are launched the ordinary way.  A memset or a copy in front asks for no early
+// start, so that the kernel behind it starts after its end, dependent launch or not (the router behind the zeros of its counts,
+// and whatever follows torch's zeros and copies).
 PB_DEVICE void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // (The result is always true.  What follows hangs on it, so that no load through a pointer that is never written here, which a
 // compiler may take for constant, moves up before the wait.)

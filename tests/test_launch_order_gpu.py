@@ -1,5 +1,7 @@
 """Kernels that may start before the one in front of them has ended: a chain of launches gives the same bits as the same chain with
-the device idle between any two of them, in a stream and as a captured graph."""
+the device idle between any two of them, in a stream, as a captured graph, and in several streams at once."""
+import threading
+
 import pytest
 import torch
 
@@ -18,7 +20,7 @@ def _chain(T, H, step):
     x, w1, w2, wn = rnd(T, H), rnd(2 * H, H) / H ** 0.5, rnd(H, H) / H ** 0.5, 1 + 0.1 * rnd(H)
     heads = H // 64
     cos, sin = fused.rope_tables(T, 64, 1e4, "cuda")
-    wr = rnd(8, H) / H ** 0.5
+    wr, we = rnd(8, H) / H ** 0.5, rnd(8, H, H) / H ** 0.5
 
     def run():
         y, outs = x.clone(), []
@@ -43,9 +45,18 @@ def _chain(T, H, step):
             step()
             logits = gemm.gemm(z, wr)
             step()
-            probs, idx, counts = moe.router_scores(logits.float(), 2)[:3]
+            # (counts that are added to memory set to zero just before, and everything that follows from them)
+            probs, idx, full, counts, aux = moe.router_scores(logits, 2, return_counts=True, aux_coeff=0.1)
             step()
-            outs += [dq, dk, dv, probs]
+            sched, pos, src_token, perm = moe.local_plan(probs, idx, counts, 2)
+            step()
+            rows = moe.gather_rows(z, src_token, pos)
+            step()
+            e = moe.grouped_linear(rows, we, sched)
+            step()
+            m = moe.combine_rows(e, pos, src_token)
+            step()
+            outs += [dq, dk, dv, probs, idx, full, counts, aux, pos, src_token, perm, m]
             y = z
             y.add_(dv.view(T, H))
             step()
@@ -71,3 +82,29 @@ def test_chain_in_stream_order(T, H):
             graph.replay()
             for a, b in zip(got, want):
                 assert torch.equal(a, b)
+
+
+def test_chains_on_several_streams():
+    """Each thread's chain runs on a stream of its own, beside the others'."""
+    shapes = [(1024, 512), (2048, 256), (128, 2048)]
+    with torch.no_grad():
+        runs = [_chain(T, H, lambda: None) for T, H in shapes]
+        wants = [_chain(T, H, torch.cuda.synchronize)() for T, H in shapes]
+    torch.cuda.synchronize()
+    streams, got = [torch.cuda.Stream() for _ in shapes], [None] * len(shapes)
+    start = threading.Barrier(len(shapes))
+
+    def work(i):
+        with torch.no_grad(), torch.cuda.stream(streams[i]):
+            start.wait(60)
+            for _ in range(4):
+                got[i] = runs[i]()
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(len(shapes))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    for outs, want in zip(got, wants):
+        assert len(outs) == len(want) and all(torch.equal(a, b) for a, b in zip(outs, want))
