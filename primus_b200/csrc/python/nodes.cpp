@@ -64,24 +64,27 @@ std::enable_if_t<std::is_integral_v<T>, long> as_arg(T v) { return (long)v; }
 inline float as_arg(float v) { return v; }
 inline void* as_arg(void* v) { return v; }
 
+void* symbol(const char* name) {        // pb_<name>
+  static std::mutex m;
+  static std::map<std::string, void*> known;
+  std::lock_guard<std::mutex> g(m);
+  void*& f = known[name];
+  if (!f) f = dlsym(library, (std::string("pb_") + name).c_str());
+  if (!f) throw LaunchError(std::string("pb_") + name + " not found");
+  return f;
+}
+
 // pb_<name>(args..., stream); `kernels`: how many it launches
 template <typename... A>
 void launch(const char* name, int kernels, A... a) {
   using Fn = int (*)(decltype(as_arg(a))..., void*);
-  static std::mutex m;
-  static std::map<std::string, void*> known;
-  void* fn;
-  {
-    std::lock_guard<std::mutex> g(m);
-    void*& f = known[name];
-    if (!f) f = dlsym(library, (std::string("pb_") + name).c_str());
-    fn = f;
-  }
-  if (!fn) throw LaunchError(std::string("pb_") + name + " not found");
-  const int rc = reinterpret_cast<Fn>(fn)(as_arg(a)..., stream());
+  const int rc = reinterpret_cast<Fn>(symbol(name))(as_arg(a)..., stream());
   launches.fetch_add(kernels, std::memory_order_relaxed);
   if (rc) throw LaunchError(std::string("pb_") + name + " failed with code " + std::to_string(rc));
 }
+
+// rows of partial sums that the norms' backward passes write for so many rows, as the library has it
+long partial_rows(long rows) { return reinterpret_cast<int (*)(long)>(symbol("rmsnorm_bwd_num_partials"))(rows); }
 
 // the device's status word, which ops/_lib.py owns
 int* status_word(const Tensor& like) {
@@ -255,7 +258,7 @@ NormGrads norm_backward(const Tensor& dy, const Tensor& xin_, const Tensor& w, c
   }
   g.dx = at::empty_like(xin);
   if (two) g.dx2 = at::empty_like(xin);
-  const Tensor partial = empty({std::max(1L, std::min(rows, 296L)) * H}, xin, at::kFloat);   // (BWD_MAX_PARTIALS rows at most)
+  const Tensor partial = empty({partial_rows(rows) * H}, xin, at::kFloat);
   const long ldx = xin.stride(0), ldy = dy.stride(0);
   if (y.defined())
     launch("rmsnorm_bwd_y", 2, ptr(dy), ptr(xin), ptr(w), ptr(rstd), ptr(dres), ptr(g.dx), ptr(g.dx2), ptr(y), ptr(target), ptr(partial),
@@ -582,7 +585,7 @@ struct QKNorm : Function<QKNorm> {
       Tensor target[2] = {main_grad_of(kept(ctx, "wq")), main_grad_of(kept(ctx, "wk"))}, dw[2];
       for (int i = 0; i < 2; ++i)
         if (!target[i].defined()) target[i] = dw[i] = at::zeros({d}, qkv.options().dtype(at::kFloat));
-      const Tensor partial = empty({std::max(1L, std::min(T, 296L)) * 2 * d}, qkv, at::kFloat);
+      const Tensor partial = empty({partial_rows(T) * 2 * d}, qkv, at::kFloat);
       launch("qk_norm_rope_bwd", 3, ptr(dy), ptr(qkv), ptr(wq), ptr(wk), ptr(s[3]), ptr(dx), ptr(target[0]), ptr(target[1]), ptr(partial), T,
              (int)hq, (int)hkv, (int)d, (long)qkv.stride(0), (long)dy.stride(0), (long)dx.stride(0), 1, ptr(s[6]), ptr(s[4]), ptr(s[5]),
              (int)dims[3]);
@@ -857,6 +860,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("launches", [] { return launches.load(); });
   m.def("plain_gemms", [] { return plain_gemms(); });
+  m.def("partial_rows", &partial_rows);
   m.def("rmsnorm", [](const Tensor& x, const Tensor& w, double eps, const Opt& residual) -> py::object {
     auto r = RMSNorm::apply(x, w, residual, eps);
     if (r.size() == 1) return py::cast(r[0]);

@@ -1,5 +1,6 @@
 """Calls that the Python functions of the layers refuse are refused by the C++ autograd nodes too, with the same class of error and
-before anything is launched.  Here the module is called by itself, on tensors of the host: no case gets as far as a launch."""
+before anything is launched, and what the module has from the library is what the library says.  Here the module is called by itself,
+on tensors of the host: no case gets as far as a launch."""
 import os
 
 import pytest
@@ -73,3 +74,8 @@ def test_attention_of_no_sequences(nodes, monkeypatch):
                  lambda: attention.FlashAttnFn.apply(q, q, q, 0, True, 0.125),
                  lambda: nodes.rope_attention(qkv, *rope, 0, None, 0.0), lambda: layers.RopeAttentionFn.apply(qkv, *rope)):
         assert _refused_in_child(call, ZeroDivisionError)
+
+
+@pytest.mark.parametrize("rows", [0, 1, 295, 296, 297, 100000])
+def test_partial_sums_have_the_librarys_size(nodes, rows):
+    assert nodes.partial_rows(rows) == _lib.call_ret("rmsnorm_bwd_num_partials", rows)
