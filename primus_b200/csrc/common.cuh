@@ -556,10 +556,14 @@ int allow_shared_memory(Kernel kern, int bytes, std::atomic<bool> (&done)[MAX_DE
   return (int)e;
 }
 
+template <typename T>
+struct Same {
+  using type = T;
+};
 // kern<<<grid, block, shared, s>>>(args...) that may start before the kernel in front of it has ended: kern has to wait for that
-// itself (pb::grid_wait).  Errors are left to cudaGetLastError, as by the ordinary launch.
-template <typename... P, typename... A>
-void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t s, A... args) {
+// itself (pb::grid_wait).  Errors are left to cudaGetLastError, and arguments converted, as by the ordinary launch.
+template <typename... P>
+void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t s, typename Same<P>::type... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -570,7 +574,7 @@ void launch_dependent(void (*kern)(P...), dim3 grid, dim3 block, size_t shared, 
   cfg.stream = s;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+  cudaLaunchKernelEx(&cfg, kern, args...);
 }
 
 inline EncodeTiledFn get_encode_fn() {
