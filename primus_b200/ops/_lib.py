@@ -144,11 +144,12 @@ def _bound_anew(name: str, args, stream: bool, stream_ptr: int) -> int:
     return rc
 
 
-def call(name: str, *args) -> None:
-    """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended."""
+def call(name: str, *args, more: int = 0) -> None:
+    """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended.  ``more``: kernels that it enqueues with
+    these arguments beyond the usual number."""
     global LAUNCH_COUNT
     launch, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
-    LAUNCH_COUNT += kernels
+    LAUNCH_COUNT += kernels + more
     stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     rc = launch(args, stream)
     if rc is None:

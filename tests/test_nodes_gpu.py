@@ -298,3 +298,17 @@ def test_errors_keep_their_class():
     o = gemm.linear(torch.randn(8, 64, device="cuda").bfloat16().requires_grad_(), p)
     with pytest.raises(KeyError, match="from the callback"):
         o.backward(torch.ones_like(o))
+
+
+@pytest.mark.parametrize("coeff", [None, 0.1])
+def test_router_launches_are_counted_alike(monkeypatch, coeff):
+    from primus_b200.ops import moe
+
+    logits, counts = _randn(_gen(15), 64, 8), []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(_lib, "_NODES", [None])
+        before = _lib.launch_count()
+        moe.router_scores(logits, 2, aux_coeff=coeff)
+        counts.append(_lib.launch_count() - before)
+    assert counts == [1 if coeff is None else 2] * 2
