@@ -4,7 +4,8 @@ All device code targets sm_100a only (``-gencode arch=compute_100a,code=sm_100a`
 cross-compiles it on hosts without a GPU.  The library exposes plain ``extern "C"`` launchers
 (raw pointers + a CUDA stream) that :mod:`primus_b200.ops._lib` calls through a small CPython module
 (``csrc/python/launch.c``, compiled with gcc; ctypes without it), so a rebuild of the kernels takes seconds and no torch headers.
-Those are needed by one module alone, the C++ autograd nodes of the common layers (``csrc/python/nodes.cpp``).
+Those are needed by one module alone, the C++ autograd nodes of the common layers (``csrc/python/nodes.cpp``), which is compiled
+beside the kernels.
 
 Run ``python -m primus_b200.build`` (add ``--force`` to rebuild everything, ``--verbose`` to see
 ptxas resource usage).
@@ -13,8 +14,11 @@ from __future__ import annotations
 
 import argparse
 import concurrent.futures
+import hashlib
+import importlib.util
 import os
 import platform
+import re
 import shutil
 import subprocess
 import sys
@@ -31,7 +35,6 @@ LAUNCH_SRC = CSRC / "python" / "launch.c"
 LAUNCH_PATH = LIB_DIR / ("_launch" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 # autograd nodes of the common layers (torch headers: half a minute)
 NODES_SRC = CSRC / "python" / "nodes.cpp"
-NODES_PATH = LIB_DIR / ("_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -40,6 +43,29 @@ NVCC_FLAGS = [
     "-Xcompiler", "-fPIC",
     "-Xcompiler", "-fvisibility=default",
 ]
+
+
+def nodes_name(torch_version: str, abi: str) -> str:
+    """File name of the autograd nodes: which torch they were compiled for, which launchers they call and which interpreter they
+    are for, so that nothing else is ever loaded."""
+    return f"_nodes-torch{torch_version}-{abi}{sysconfig.get_config_var('EXT_SUFFIX') or '.so'}"
+
+
+def launcher_abi() -> str:
+    """What the launchers' declarations hash to.  The library answers with it to ``pb_abi``."""
+    declarations = []
+    for src in _sources():
+        declarations += re.findall(r"^(?:extern\s+\"C\"\s+)?(\w[\w\s*]*?\bpb_\w+\s*\([^)]*\))\s*\{", src.read_text(), re.M)
+    return hashlib.sha256("\n".join(sorted(" ".join(d.split()) for d in declarations)).encode()).hexdigest()[:12]
+
+
+def _torch_version() -> str:
+    """Without importing it; empty where there is none."""
+    spec = importlib.util.find_spec("torch")
+    if spec is None or not spec.submodule_search_locations:
+        return ""
+    text = (Path(spec.submodule_search_locations[0]) / "version.py").read_text()
+    return re.search(r"""^__version__\s*=\s*['"]([^'"]+)""", text, re.M).group(1)
 
 
 def find_nvcc() -> str:
@@ -72,12 +98,25 @@ def _compile_one(nvcc: str, src: Path, obj: Path, verbose: bool) -> tuple[Path, 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compile out-of-date sources and link the shared library. Returns the library path."""
+    with concurrent.futures.ThreadPoolExecutor(1) as beside:
+        nodes = beside.submit(_build_nodes, force)
+        _build_library(force, verbose)
+        _build_launch(force)
+        nodes.result()
+    return LIB_PATH
+
+
+def _build_library(force: bool, verbose: bool) -> None:
     nvcc = find_nvcc()
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    abi = OBJ_DIR / "abi.cpp"
+    text = f'extern "C" const char* pb_abi() {{ return "{launcher_abi()}"; }}\n'
+    if not abi.exists() or abi.read_text() != text:
+        abi.write_text(text)
     headers = sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h"))
     jobs = []
     objs = []
-    for src in _sources():
+    for src in [*_sources(), abi]:
         obj = OBJ_DIR / (src.name + ".o")
         objs.append(obj)
         if force or _needs_build(src, obj, headers):
@@ -97,9 +136,6 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError(f"link failed:\n{p.stdout}{p.stderr}")
-    _build_launch(force)
-    _build_nodes(force)
-    return LIB_PATH
 
 
 def _build_launch(force: bool) -> None:
@@ -124,21 +160,27 @@ def _build_launch(force: bool) -> None:
 
 
 def _build_nodes(force: bool) -> None:
-    """The C++ autograd nodes.  Where they cannot be built, the layers run as Python functions; a module of an older source does
-    not stay behind."""
-    if not force and not _needs_build(NODES_SRC, NODES_PATH, []):
+    """The C++ autograd nodes.  Where they cannot be built, the layers run as Python functions; a module of an older source, of
+    another torch or for other launchers does not stay behind."""
+    version = _torch_version()
+    path = LIB_DIR / nodes_name(version, launcher_abi())
+    for other in LIB_DIR.glob("_nodes*" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so")):
+        if other != path:
+            other.unlink(missing_ok=True)
+    if not force and not _needs_build(NODES_SRC, path, []):
         return
-    NODES_PATH.unlink(missing_ok=True)
-    if platform.machine() != "x86_64":
-        why = "not x86-64"
+    path.unlink(missing_ok=True)
+    if platform.machine() != "x86_64" or not version:
+        why = "x86-64 and torch are needed"
     else:
         import torch
 
+        LIB_DIR.mkdir(parents=True, exist_ok=True)
         root, cuda = Path(torch.__file__).parent, Path(find_nvcc()).parent.parent
         includes = [root / "include", root / "include/torch/csrc/api/include", cuda / "include", sysconfig.get_paths()["include"]]
         cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", "-DTORCH_EXTENSION_NAME=_nodes",
                f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}", *[f"-I{i}" for i in includes], str(NODES_SRC),
-               "-o", str(NODES_PATH), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+               "-o", str(path), f"-L{root / 'lib'}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
         try:
             p = subprocess.run(cmd, capture_output=True, text=True)
             if p.returncode == 0:
@@ -146,7 +188,7 @@ def _build_nodes(force: bool) -> None:
             why = f"{p.stdout}{p.stderr}"
         except OSError as e:
             why = str(e)
-    NODES_PATH.unlink(missing_ok=True)
+    path.unlink(missing_ok=True)
     print(f"the autograd nodes could not be built:\n{why}\nlayers run as Python functions", file=sys.stderr)
 
 

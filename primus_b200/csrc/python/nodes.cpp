@@ -849,7 +849,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       PyErr_SetString(lib_module->attr("NativeLibraryError").ptr(), e.what());
     }
   });
-  m.attr("torch_version") = TORCH_VERSION;
   m.def("init", [](const std::string& path, py::object lib, py::object gemm_mod, py::object autotune_mod) {
     library = dlopen(path.c_str(), RTLD_NOW | RTLD_GLOBAL);
     if (!library) throw std::runtime_error(dlerror());

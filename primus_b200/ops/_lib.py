@@ -166,9 +166,23 @@ def call_ret(name: str, *args) -> int:
 
 
 def _load_nodes():
-    """The C++ autograd nodes beside the library, or None: the layers then run as Python functions."""
-    path = LIB_PATH.parent / ("_nodes" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))
-    if not path.exists() or not available() or not torch.cuda.is_available():
+    """The C++ autograd nodes beside the library, or None: the layers then run as Python functions.  The file's name says which
+    torch and which launchers a module was compiled for; none of another name is opened."""
+    from ..build import nodes_name
+
+    if not available() or not torch.cuda.is_available():
+        return None
+    try:
+        answer = load().pb_abi
+        answer.restype = ctypes.c_char_p
+        path = LIB_PATH.parent / nodes_name(torch.__version__, answer().decode())
+    except AttributeError:                      # a library without an answer: an older one
+        path = LIB_PATH.parent / "none"
+    if not path.exists():
+        others = sorted(p.name for p in LIB_PATH.parent.glob("_nodes*"))
+        if others:
+            warnings.warn(f"{', '.join(others)}: not for torch {torch.__version__} and the launchers of {lib_path()} "
+                          "(python -m primus_b200.build); layers run as Python functions")
         return None
     from . import autotune, gemm
 
@@ -176,9 +190,6 @@ def _load_nodes():
         loader = importlib.machinery.ExtensionFileLoader("_nodes", str(path))
         module = importlib.util.module_from_spec(importlib.util.spec_from_loader("_nodes", loader))
         loader.exec_module(module)
-        if torch.__version__.split("+")[0] != module.torch_version:
-            raise ImportError(f"built for torch {module.torch_version}")
-        load()
         module.init(str(lib_path()), sys.modules[__name__], gemm, autotune)
     except (ImportError, RuntimeError) as e:
         warnings.warn(f"{path} does not load ({e}): layers run as Python functions")
