@@ -995,10 +995,6 @@ int pb_qk_norm_rope_fwd(const void* x, const void* wq, const void* wk, void* y, 
 #undef PB_QK_FWD
   return (int)cudaGetLastError();
 }
-int pb_qk_norm_fwd(const void* x, const void* wq, const void* wk, void* y, float* rstd, long T, int hq, int hkv, int d,
-                   long ldx, long ldy, float eps, cudaStream_t s) {
-  return pb_qk_norm_rope_fwd(x, wq, wk, y, rstd, T, hq, hkv, d, ldx, ldy, eps, nullptr, nullptr, nullptr, 0, s);
-}
 
 // scratch: fp32 [pb_rmsnorm_bwd_num_partials(T), 2 d]; dwq / dwk: fp32 [d], dw_accumulate: += instead of =.  cos_t (or null), pos,
 // sin_t, rot_dim: as the forward was called.

@@ -1,1 +1,1 @@
-extern "C" const char* pb_abi() { return "1404724f9e58"; }
+extern "C" const char* pb_abi() { return "cc65064b7c93"; }

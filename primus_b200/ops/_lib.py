@@ -133,7 +133,7 @@ def _bind(name: str, args, stream: bool):
 
 # Number of device kernels each launcher enqueues (default 1); used for the launch counter below.
 _KERNELS_PER_CALL = {"rmsnorm_bwd": 2, "rmsnorm_bwd_two": 2, "rmsnorm_bwd_y": 2, "sumsq": 2, "grad_norm": 2, "flash_attn_bwd": 3, "flash_attn_bwd_cap": 3, "quant_fp8_tensorwise": 2,
-                     "quant_fp8_delayed": 2, "gemm_bf16_splitk": 2, "qk_norm_bwd": 3, "qk_norm_rope_bwd": 3}
+                     "quant_fp8_delayed": 2, "gemm_bf16_splitk": 2, "qk_norm_rope_bwd": 3}
 LAUNCH_COUNT = 0
 
 
