@@ -144,10 +144,21 @@ def _bound_anew(name: str, args, stream: bool, stream_ptr: int) -> int:
     return rc
 
 
+_tracing = torch._C._is_tracing
+
+
+def _refuse_trace():
+    """While torch.jit.trace records, sizes are tensors, whose addresses a launcher would take for numbers, and the trace would
+    return memory that no kernel has written."""
+    raise NativeLibraryError("the kernels cannot be recorded by torch.jit.trace")
+
+
 def call(name: str, *args, more: int = 0) -> None:
     """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended.  ``more``: kernels that it enqueues with
     these arguments beyond the usual number."""
     global LAUNCH_COUNT
+    if _tracing():
+        _refuse_trace()
     launch, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
     LAUNCH_COUNT += kernels + more
     stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
@@ -209,6 +220,8 @@ def nodes(*tensors):
     them counts as taken), else None."""
     if not _NODES:
         _NODES.append(_load_nodes())
+    if _tracing():
+        _refuse_trace()
     n = _NODES[0]
     if n is None or _functorch():
         return None
