@@ -367,6 +367,12 @@ struct NormLinear : Function<NormLinear> {
 };
 
 // ------------------------------------------------------------------ linear, SwiGLU
+// channels of one half of [gate | up]
+long half_of(long I2) {
+  TORCH_CHECK(I2 % 2 == 0, "gated rows of ", I2, " values have no two halves");
+  return I2 / 2;
+}
+
 struct Linear : Function<Linear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& weight) {
     const Tensor x2 = as_rows(x, x.size(-1));
@@ -398,7 +404,7 @@ struct Linear : Function<Linear> {
 
 struct SwiGLULinear : Function<SwiGLULinear> {
   static Tensor forward(AutogradContext* ctx, const Tensor& h1, const Tensor& weight, double clamp, int64_t kind) {
-    const long I2 = h1.size(-1), I = I2 / 2;
+    const long I2 = h1.size(-1), I = half_of(I2);
     const Tensor x2 = as_rows(h1, I2);
     const long T = x2.size(0);
     const Tensor act = empty({T, I}, h1, at::kBFloat16);
@@ -804,7 +810,7 @@ struct GroupedLinear : Function<GroupedLinear> {
 
 struct SwiGLU : Function<SwiGLU> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Opt& probs_, double clamp, int64_t kind) {
-    const long I2 = x.size(-1), I = I2 / 2;
+    const long I2 = x.size(-1), I = half_of(I2);
     const Tensor x2 = as_rows(x, I2);
     Tensor probs;
     if (probs_) probs = probs_->reshape({-1}).to(at::kFloat).contiguous();

@@ -142,6 +142,8 @@ class SwiGLULinearFn(torch.autograd.Function):
     def forward(ctx, h1, weight, probs, clamp, tp_group, sp, act="silu"):
         ctx.kind = fused.GATE_KINDS[act]
         I2 = h1.shape[-1]
+        if I2 % 2:
+            raise RuntimeError(f"gated rows of {I2} values have no two halves")
         I = I2 // 2
         x2 = h1.reshape(-1, I2)
         T = x2.shape[0]

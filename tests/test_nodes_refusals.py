@@ -64,3 +64,17 @@ def test_attention_of_no_sequences(nodes, monkeypatch):
 @pytest.mark.parametrize("rows", [0, 1, 295, 296, 297, 100000])
 def test_partial_sums_have_the_librarys_size(nodes, rows):
     assert nodes.partial_rows(rows) == _lib.call_ret("rmsnorm_bwd_num_partials", rows)
+
+
+@pytest.mark.parametrize("layer", ["swiglu", "swiglu_linear"])
+@pytest.mark.parametrize("rows", [64, 16])
+def test_gated_rows_of_odd_width(nodes, monkeypatch, layer, rows):
+    x, w = _zeros(rows, 17), _zeros(24, 8)
+    monkeypatch.setattr(_lib, "call", lambda *a, **k: None)
+    monkeypatch.setattr(layers.gemm, "gemm", lambda a, b, **k: _zeros(rows, 24))
+    calls = [lambda: nodes.swiglu(x, None, 0.0, 0), lambda: fused.SwiGLUFn.apply(x, None, 0.0)]
+    if layer == "swiglu_linear":
+        calls = [lambda: nodes.swiglu_linear(x, w, 0.0, 0), lambda: layers.SwiGLULinearFn.apply(x, w, None, 0.0, None, False)]
+    for call in calls:
+        with pytest.raises(RuntimeError, match="shape|halves"):
+            call()
