@@ -443,7 +443,8 @@ struct SwiGLULinear : Function<SwiGLULinear> {
   throw py::error_already_set();
 }
 void check_view(const Tensor& t, long d) {     // (attention._check_view, and its class of error)
-  if (t.dim() != 3 || t.stride(2) != 1 || t.stride(1) != d || !aligned(t))
+  if (t.dim() < 3) refuse(PyExc_IndexError, "heads must be [T, H, D]");
+  if (t.stride(2) != 1 || t.stride(1) != d || !aligned(t))
     refuse(PyExc_AssertionError, "heads must be contiguous [.., H, D] views");
 }
 
@@ -502,6 +503,7 @@ struct FlashAttention : Function<FlashAttention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Opt& sinks_, int64_t batch,
                         bool causal, double scale, int64_t q_off, int64_t window, double softcap) {
     const Tensor sinks = given(sinks_);
+    if (q.dim() != 3) refuse(PyExc_ValueError, "queries must be [T, H, D]");
     const AttnArgs a = attn_args(batch, causal, scale, q_off, window, softcap);
     const auto [o, lse] = attn_forward(q, k, v, sinks, a);
     ctx->save_for_backward({q, k, v, o, lse, sinks});

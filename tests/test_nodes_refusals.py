@@ -78,3 +78,17 @@ def test_gated_rows_of_odd_width(nodes, monkeypatch, layer, rows):
     for call in calls:
         with pytest.raises(RuntimeError, match="shape|halves"):
             call()
+
+
+@pytest.mark.parametrize("which", range(3))
+@pytest.mark.parametrize("shape", [(128, 64), (1, 128, 2, 64)])
+def test_attention_of_other_dimensions(nodes, monkeypatch, which, shape):
+    monkeypatch.setattr(_lib, "call", lambda *a, **k: None)
+    qkv = [_zeros(128, 2, 64) for _ in range(3)]
+    qkv[which] = _zeros(*shape)
+    errors = []
+    for call in (lambda: nodes.flash_attention(*qkv, 1, True, 0.125, 0, 0, None, 0.0), lambda: attention.FlashAttnFn.apply(*qkv, 1, True, 0.125)):
+        with pytest.raises((ValueError, IndexError, AssertionError)) as e:
+            call()
+        errors.append(e.type)
+    assert errors[0] is errors[1]
