@@ -212,16 +212,17 @@ class QKNormFn(torch.autograd.Function):
         return dx, dwq, dwk, *[None] * 8
 
 
-def _qk_norm_kernel(qkv, d) -> bool:
-    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.stride(1) == 1 and d % 8 == 0 and d <= 256
-            and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
+def _qk_norm_kernel(qkv, heads, d) -> bool:
+    """Whether the kernel can read ``heads`` heads in every row of this tensor."""
+    return (qkv.is_cuda and qkv.dtype == torch.bfloat16 and qkv.shape[1] >= heads * d and qkv.stride(1) == 1 and d % 8 == 0
+            and d <= 256 and qkv.stride(0) % 8 == 0 and qkv.data_ptr() % 16 == 0)
 
 
 def qk_norm(qkv, wq, wk, hq, hkv, d, eps=1e-5):
     """Per-head RMSNorm of the q heads (gain ``wq`` [d]) and k heads (``wk``) of a packed tensor
     ``[q heads | k heads | v heads]`` [T, (hq + 2 hkv) d]; the v heads are unchanged."""
     T = qkv.shape[0]
-    if _qk_norm_kernel(qkv, d):
+    if _qk_norm_kernel(qkv, hq + 2 * hkv, d):
         wq, wk = gamma(wq), gamma(wk)
         n = _lib.nodes(qkv, wq, wk)
         if n is not None:
@@ -236,7 +237,7 @@ def qk_norm_rope(qkv, wq, wk, hq, hkv, d, eps, cos, sin, pos, rot_dim):
     """:func:`qk_norm` and the rotary embedding of its q and k heads in one pass each way; None where the kernel does not take
     the tensors (the caller then norms, and rotates where it did)."""
     tables = [t for t in (cos, sin, pos) if t is not None]
-    if (cos is None or not _qk_norm_kernel(qkv, d) or rot_dim % 16 or not 0 < rot_dim <= d
+    if (cos is None or not _qk_norm_kernel(qkv, hq + 2 * hkv, d) or rot_dim % 16 or not 0 < rot_dim <= d
             or any(not t.is_contiguous() or t.data_ptr() % 16 or t.device != qkv.device for t in tables)
             or cos.dtype != torch.float32 or sin.dtype != torch.float32 or (pos is not None and pos.dtype != torch.int32)):
         return None

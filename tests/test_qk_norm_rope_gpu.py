@@ -66,3 +66,13 @@ def test_tables_the_kernel_cannot_read_are_left_to_the_two_passes():
         a = dict(cos=cos, sin=sin, pos=None, rot_dim=64)
         a.update(bad)
         assert fused.qk_norm_rope(x, w, w, 2, 1, 64, 1e-5, **a) is None
+
+
+@pytest.mark.parametrize("columns", [3 * 64, 64])
+def test_rows_of_fewer_heads_are_not_read_past_their_end(columns):
+    x = torch.zeros(4, 8 * 64, device="cuda").bfloat16()[:, :columns]        # (of 2 query and 2 + 2 key / value heads)
+    w = torch.ones(64, device="cuda").bfloat16()
+    with pytest.raises(RuntimeError):
+        fused.qk_norm(x, w, w, 2, 2, 64)
+    cos, sin = fused.rope_tables(8, 64, 1e4, "cuda")
+    assert fused.qk_norm_rope(x, w, w, 2, 2, 64, 1e-5, cos, sin, None, 64) is None
