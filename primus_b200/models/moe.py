@@ -32,7 +32,10 @@ class AuxLossScaler(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         (aux,) = ctx.saved_tensors
-        return g, torch.full_like(aux, float(AuxLossScaler.scale))
+        scale = AuxLossScaler.scale
+        if isinstance(scale, torch.Tensor):     # (a loss scale that lives on the device stays there)
+            return g, torch.ones_like(aux) * scale
+        return g, torch.full_like(aux, scale)
 
 
 class _TokenIds:
