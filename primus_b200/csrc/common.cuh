@@ -456,7 +456,7 @@ PB_DEVICE float fast_tanh(float x) {
   return y;
 }
 
-// two fp32 values per instruction (sm_100: fma / add / mul on 64-bit register pairs, each rounded as the scalar form)
+// two bf16 values per instruction
 PB_DEVICE uint32_t max2_bf16x2(uint32_t a, uint32_t b) {   // (a NaN yields to a number, as in fmaxf)
   asm("max.bf16x2 %0, %0, %1;" : "+r"(a) : "r"(b));
   return a;
@@ -467,6 +467,7 @@ PB_DEVICE uint32_t min2_bf16x2(uint32_t a, uint32_t b) {
 }
 PB_DEVICE float max_bf16x2(uint32_t v) { return fmaxf(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
 PB_DEVICE float min_bf16x2(uint32_t v) { return fminf(__uint_as_float(v << 16), __uint_as_float(v & 0xffff0000u)); }
+// two fp32 values per instruction (sm_100: fma / add / mul on 64-bit register pairs, each rounded as the scalar form)
 PB_DEVICE uint64_t pack_f32x2(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));

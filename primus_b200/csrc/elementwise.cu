@@ -727,7 +727,8 @@ __device__ __forceinline__ void clip_coef(float sumsq, const ClipArgs& a) {
 }
 __global__ void clip_coef_kernel(const float* sumsq, ClipArgs args) {
   PB_GRID_WAIT();
-  clip_coef(sumsq[0], args); }
+  clip_coef(sumsq[0], args);
+}
 
 // out[0] (+)= sum(partial) of each of `segs` tensors in turn; nonfinite[0] |= !isfinite(sum); with args.coef the clip
 // coefficient of that sum, where nothing else is to be added to it.
@@ -819,13 +820,11 @@ int pb_rope(void* x, const int* pos, const float* cos_t, const float* sin_t, lon
   if (one <= 0) return 0;
   const float sign = backward ? -1.f : 1.f;
   if (four >= 148 * 1024L)
-    pbh::launch_dependent(rope_kernel<4>, (unsigned)((four + 255) / 256), 256, 0, s, (__nv_bfloat16*)x, pos, cos_t, sin_t, T,
-        heads, d, rot_dim,
-                                                                 ld, sign);
+    pbh::launch_dependent(rope_kernel<4>, (unsigned)((four + 255) / 256), 256, 0, s, (__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads,
+        d, rot_dim, ld, sign);
   else
     pbh::launch_dependent(rope_kernel<1>, (unsigned)((one + 255) / 256), 256, 0, s, (__nv_bfloat16*)x, pos, cos_t, sin_t, T, heads,
-        d, rot_dim,
-                                                                ld, sign);
+        d, rot_dim, ld, sign);
   PB_CHECK_LAUNCH();
 }
 
@@ -866,14 +865,12 @@ int pb_swiglu_bwd_act(const void* dy, const void* in, const float* probs, void* 
   if (dprobs) {
     auto kern = PB_SWIGLU_KERNEL(swiglu_bwd_probs_kernel);
     pbh::launch_dependent(kern, grid_for(T * 32, 256), 256, 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs,
-        (__nv_bfloat16*)din,
-                                               (__nv_bfloat16*)act, dprobs, T, I, clamp);
+        (__nv_bfloat16*)din, (__nv_bfloat16*)act, dprobs, T, I, clamp);
   } else if (I > 0) {
     const int blocks = grid_for(T * (I / 8), 512, 148 * 8), step = blocks * 256;
     auto kern = PB_SWIGLU_KERNEL(swiglu_bwd_kernel);
     pbh::launch_dependent(kern, blocks, 256, 0, s, (const __nv_bfloat16*)dy, (const __nv_bfloat16*)in, probs, (__nv_bfloat16*)din,
-        (__nv_bfloat16*)act,
-                                T, I, clamp, step / (I / 8), step % (I / 8));
+        (__nv_bfloat16*)act, T, I, clamp, step / (I / 8), step % (I / 8));
   }
   PB_CHECK_LAUNCH();
 }
@@ -973,9 +970,9 @@ int pb_adamw_ranges(const long* table, int count, const float* hyper, int grad_i
       if (i < count) return -2;                        // a bucket of more chunks than a grid has blocks
       break;
     }
-#define PB_ADAMW(GT, ST)                                                                                                  \
+#define PB_ADAMW(GT, ST)                                                                                                      \
   pbh::launch_dependent(adamw_ranges_kernel<GT, ST>, (unsigned)chunks, 256, 0, s, segs, lrs, beta1, beta2, eps, wd, bc1, bc2, \
-                                                               (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
+      (float)(1.0 / bc1), (float)(1.0 / bc2), grad_scale, skip)
     if (grad_is_bf16 && state_is_bf16) PB_ADAMW(__nv_bfloat16, __nv_bfloat16);
     else if (grad_is_bf16) PB_ADAMW(__nv_bfloat16, float);
     else if (state_is_bf16) PB_ADAMW(float, __nv_bfloat16);
@@ -1065,7 +1062,7 @@ int pb_embedding_bwd(const void* dy, const long* tokens, float* dw, long T, int 
   if (H % 2) return -2;
   if (T == 0) return 0;
   pbh::launch_dependent(embedding_bwd_kernel, grid_for(T * (H / 2), 256), 256, 0, s, (const __nv_bfloat16*)dy, tokens, dw, T, H,
-                                                                 vocab_start, vocab);
+      vocab_start, vocab);
   PB_CHECK_LAUNCH();
 }
 
@@ -1238,10 +1235,9 @@ extern "C" int pb_moe_gather_rows(const void* x, const int* src, const float* sc
                                   const int* limit_rows, cudaStream_t s) {
   if (H % 8) return -2;
   if (R == 0) return 0;
-#define PB_GATHER(ROWS, VECS)                                                                                        \
-  pbh::launch_dependent(moe_gather_rows_kernel<ROWS, VECS>, moe_grid((R + ROWS - 1) / ROWS), 256, 0, s, (const __nv_bfloat16*)x, \
-      src, scale, \
-                                                                                     (__nv_bfloat16*)out, R, H, limit_rows)
+#define PB_GATHER(ROWS, VECS)                                                                           \
+  pbh::launch_dependent(moe_gather_rows_kernel<ROWS, VECS>, moe_grid((R + ROWS - 1) / ROWS), 256, 0, s, \
+      (const __nv_bfloat16*)x, src, scale, (__nv_bfloat16*)out, R, H, limit_rows)
   // (us, B200, before and now: 4096 tokens of 2048, 64 experts, eight copies 51 -> 43; 65536 of 256, two copies 44 -> 22)
   if (H <= 256 && R >= 8192) PB_GATHER(4, 1); else PB_GATHER(1, 2);
 #undef PB_GATHER

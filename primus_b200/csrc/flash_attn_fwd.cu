@@ -512,7 +512,7 @@ int launch_fwd(const void* q, const void* k, const void* v, void* o, float* lse,
   if ((rc = pbh::allow_shared_memory(kern, C::SMEM_BYTES, allowed[win]))) return rc;
   dim3 grid(hq, batch, (seq / BQ + 1) / 2);
   pbh::launch_dependent(kern, grid, FA_THREADS, C::SMEM_BYTES, stream, tq, tk, tv, to, lse, seq, seq_k, q_off / BQ, hq, hkv,
-                                                   scale * 1.4426950408889634f, causal, window, sinks, softcap, status);
+      scale * 1.4426950408889634f, causal, window, sinks, softcap, status);
   return (int)cudaGetLastError();
 }
 

@@ -430,7 +430,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   if (max_ctas > 0 && max_ctas < ctas) ctas = max_ctas;
   if (tiles < ctas) ctas = tiles;
   pbh::launch_dependent(kern, ctas, NUM_THREADS, C::SMEM_BYTES, stream, tA, tB, tD, reinterpret_cast<const uint8_t*>(sfa),
-                                                     reinterpret_cast<const uint8_t*>(sfb), M, N, K, status);
+      reinterpret_cast<const uint8_t*>(sfb), M, N, K, status);
   return (int)cudaGetLastError();
 }
 

@@ -343,8 +343,7 @@ int launch(const CUtensorMap& tA, const CUtensorMap& tB, const CUtensorMap& tD, 
   }
   const int ctas = num_tiles < num_sms ? num_tiles : num_sms;
   pbh::launch_dependent(kern, ctas, NUM_THREADS, SMEM_BYTES, s, tA, tB, tD, num_m, num_n, num_tiles, K, mblock_expert, row_start,
-      padded,
-                                            status);
+      padded, status);
   return (int)cudaGetLastError();
 }
 

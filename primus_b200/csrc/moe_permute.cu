@@ -129,8 +129,7 @@ int pb_moe_permutation_maps(const long* expert, long R, int topk, int E, const i
                             int rows_cap, int* src, int* src_token, int* pos, cudaStream_t s) {
   if (E <= 0 || topk <= 0 || R < 0 || R > 2147483647L - 2 * MAP_THREADS * MAP_ITEMS) return -2;
   pbh::launch_dependent(moe_permutation_maps_kernel<false>, E, MAP_THREADS, 0, s, expert, (int)R, topk, E, row_start, padded,
-      rows_cap, src, src_token,
-                                                              pos, LocalPlan{});
+      rows_cap, src, src_token, pos, LocalPlan{});
   return (int)cudaGetLastError();
 }
 
@@ -141,8 +140,7 @@ int pb_moe_local_plan(const long* expert, const int* counts, const float* probs,
                       cudaStream_t s) {
   if (E <= 0 || E > 1024 || topk <= 0 || R < 0 || R > 2147483647L - 2 * MAP_THREADS * MAP_ITEMS) return -2;
   pbh::launch_dependent(moe_permutation_maps_kernel<true>, E, MAP_THREADS, 0, s, expert, (int)R, topk, E, nullptr, nullptr,
-      rows_cap, src, src_token, pos,
-      LocalPlan{counts, probs, padded, row_start, mblock_expert, total, probs_perm, max_mblocks});
+      rows_cap, src, src_token, pos, LocalPlan{counts, probs, padded, row_start, mblock_expert, total, probs_perm, max_mblocks});
   return (int)cudaGetLastError();
 }
 

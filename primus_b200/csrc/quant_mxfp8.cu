@@ -611,8 +611,8 @@ int pb_quant_mxfp8(const void* x, int R, int C, void* q_row, void* sf_row, void*
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
   dim3 grid(C / TILE, R / TILE);
   pbh::launch_dependent(quant_mxfp8_kernel<false>, grid, QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R, C,
-                                                reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row),
-                                                reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
+      reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
+      reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
@@ -622,8 +622,8 @@ int pb_quant_mxfp4_as_fp8(const void* x, int R, int C, void* q_row, void* sf_row
                           cudaStream_t s) {
   if (R % TILE || C % TILE || R <= 0 || C <= 0) return -2;
   pbh::launch_dependent(quant_mxfp8_kernel<true>, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
-      C, reinterpret_cast<uint8_t*>(q_row),
-      reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
+      C, reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
+      reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
@@ -637,8 +637,8 @@ int pb_quant_fp8_tensorwise(const void* x, int R, int C, float* amax, void* q_ro
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax);
   pbh::launch_dependent(quant_tensorwise_kernel, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
-      C, amax, nullptr, reinterpret_cast<uint8_t*>(q_row),
-      reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
+      C, amax, nullptr, reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
+      reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
@@ -653,8 +653,8 @@ int pb_quant_fp8_delayed(const void* x, int R, int C, float* amax_now, const flo
   const int blocks = (int)((n8 + 2047) / 2048 < 1184 ? (n8 + 2047) / 2048 : 1184);
   amax_bf16_kernel<<<blocks, 256, 0, s>>>(reinterpret_cast<const __nv_bfloat16*>(x), n8, amax_now);
   pbh::launch_dependent(quant_tensorwise_kernel, dim3(C / TILE, R / TILE), QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(x), R,
-      C, scale_amax, amax_now, reinterpret_cast<uint8_t*>(q_row),
-      reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
+      C, scale_amax, amax_now, reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row),
+      reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
@@ -681,8 +681,8 @@ int pb_swiglu_quant_mxfp8(const void* h1, int T, int I, float clamp, void* q_row
   auto kern = clamp > 0.f ? (wide ? swiglu_quant_mxfp8_kernel<true, true> : swiglu_quant_mxfp8_kernel<false, true>)
                           : (wide ? swiglu_quant_mxfp8_kernel<true, false> : swiglu_quant_mxfp8_kernel<false, false>);
   pbh::launch_dependent(kern, grid, wide ? 2 * QT : QT, 0, s, reinterpret_cast<const __nv_bfloat16*>(h1), T, I, clamp,
-      reinterpret_cast<uint8_t*>(q_row),
-      reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col));
+      reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
+      reinterpret_cast<uint8_t*>(sf_col));
   return (int)cudaGetLastError();
 }
 
@@ -700,9 +700,9 @@ int pb_swiglu_bwd_quant_mxfp8(const void* h1, const void* dact, int T, int I, fl
   const int rc = pbh::allow_shared_memory(kern, smem, allowed[wide + 2 * (clamp > 0.f)]);
   if (rc) return rc;
   pbh::launch_dependent(kern, grid, wide ? 2 * QT : QT, smem, s, reinterpret_cast<const __nv_bfloat16*>(h1),
-      reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp,
-      reinterpret_cast<uint8_t*>(q_row), reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col),
-      reinterpret_cast<uint8_t*>(sf_col), reinterpret_cast<uint8_t*>(act_col), reinterpret_cast<uint8_t*>(act_sf));
+      reinterpret_cast<const __nv_bfloat16*>(dact), T, I, clamp, reinterpret_cast<uint8_t*>(q_row),
+      reinterpret_cast<uint8_t*>(sf_row), reinterpret_cast<uint8_t*>(q_col), reinterpret_cast<uint8_t*>(sf_col),
+      reinterpret_cast<uint8_t*>(act_col), reinterpret_cast<uint8_t*>(act_sf));
   return (int)cudaGetLastError();
 }
 

@@ -307,10 +307,8 @@ static int router_fwd(const void* logits, int in_bf16, const float* bias, int T,
         reinterpret_cast<const __nv_bfloat16*>(logits), bias, T, E, k, sigmoid, pre_softmax, num_groups, group_topk,
         scale, probs, idx, idx64, full, counts, score_sums);
   else
-    pbh::launch_dependent(router_fwd_kernel<float>, blocks, WARPS * 32, smem, s, reinterpret_cast<const float*>(logits), bias, T,
-        E, k,
-                                                              sigmoid, pre_softmax, num_groups, group_topk, scale, probs,
-                                                              idx, idx64, full, counts, score_sums);
+    pbh::launch_dependent(router_fwd_kernel<float>, blocks, WARPS * 32, smem, s, reinterpret_cast<const float*>(logits), bias, T, E,
+        k, sigmoid, pre_softmax, num_groups, group_topk, scale, probs, idx, idx64, full, counts, score_sums);
   return (int)cudaGetLastError();
 }
 int pb_router_fwd(const void* logits, int in_bf16, const float* bias, int T, int E, int k, int sigmoid, int pre_softmax,
@@ -347,12 +345,10 @@ int pb_router_bwd(const float* dprobs, const float* dfull, const float* full, co
   const size_t smem = (size_t)WARPS * E * sizeof(float);
   if (out_bf16)
     pbh::launch_dependent(router_bwd_kernel<__nv_bfloat16>, blocks, WARPS * 32, smem, s, dprobs, dfull, full, idx, probs, T, E, k,
-        sigmoid, pre_softmax,
-                                                                      scale, daux, counts, aux_factor, (__nv_bfloat16*)dlogits);
+        sigmoid, pre_softmax, scale, daux, counts, aux_factor, (__nv_bfloat16*)dlogits);
   else
     pbh::launch_dependent(router_bwd_kernel<float>, blocks, WARPS * 32, smem, s, dprobs, dfull, full, idx, probs, T, E, k, sigmoid,
-        pre_softmax, scale,
-                                                              daux, counts, aux_factor, (float*)dlogits);
+        pre_softmax, scale, daux, counts, aux_factor, (float*)dlogits);
   return (int)cudaGetLastError();
 }
 
