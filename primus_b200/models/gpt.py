@@ -146,9 +146,11 @@ class SelfAttention(nn.Module):
                                                     rot_dim=int(d * cfg.rotary_percent), causal=True, scale=scale)
         else:
             sinks = self.core_attention.softmax_offset.float() if self.has_sinks else None
+            # the kernels rotate q and k in place: what runs once more in the backward pass works on a copy
+            own = cos is not None and qkv.is_cuda and selectively_recomputed(cfg, "core_attn")
             ctx_out = selective_checkpoint(
                 cfg, "core_attn",
-                lambda t: layers.rope_attention(t, cos, sin, pos, batch, self.hq, self.hkv, d,
+                lambda t: layers.rope_attention(t.clone() if own else t, cos, sin, pos, batch, self.hq, self.hkv, d,
                                                 rot_dim=int(d * cfg.rotary_percent), causal=True, scale=scale,
                                                 window=self.window, sinks=sinks, segments=segments,
                                                 softcap=cfg.attn_logit_softcapping or 0.0), qkv)
@@ -703,12 +705,16 @@ def _run_layer(layer, hidden, residual, rope, batch, cfg):
     return layer(hidden, residual, rope, batch)
 
 
+def selectively_recomputed(cfg, module: str) -> bool:
+    return cfg.recompute_granularity == "selective" and torch.is_grad_enabled() and \
+        module in (cfg.recompute_modules or ["core_attn"])
+
+
 def selective_checkpoint(cfg, module: str, fn, *args):
     """``recompute_granularity: selective``: run ``fn(*args)`` under activation checkpointing when ``module`` is in
     ``recompute_modules`` (default: the core attention only, whose saved output and statistics are then rebuilt from
     q / k / v in the backward pass)."""
-    if cfg.recompute_granularity == "selective" and torch.is_grad_enabled() and \
-            module in (cfg.recompute_modules or ["core_attn"]):
+    if selectively_recomputed(cfg, module):
         return prandom.checkpoint(fn, *args)
     return fn(*args)
 
