@@ -108,3 +108,42 @@ def test_chains_on_several_streams():
     torch.cuda.synchronize()
     for outs, want in zip(got, wants):
         assert len(outs) == len(want) and all(torch.equal(a, b) for a, b in zip(outs, want))
+
+
+def test_chains_that_fork_and_join():
+    """Two chains between an event that both wait for and a kernel that waits for both, in streams and as a graph."""
+    runs = [_chain(256, 512, lambda: None), _chain(512, 512, lambda: None)]
+    w = torch.ones(512, device="cuda").bfloat16()
+    x = torch.randn(256, 512, device="cuda", generator=torch.Generator(device="cuda").manual_seed(1)).bfloat16()
+    side = torch.cuda.Stream()
+
+    def work(step):
+        with torch.no_grad():
+            first = fused.rmsnorm(x, w)
+            step()
+            side.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(side):
+                b = runs[1]()
+                second = fused.rmsnorm(first, w)
+            step()
+            a = runs[0]()
+            step()
+            torch.cuda.current_stream().wait_stream(side)
+            last = fused.rmsnorm(a[-1], w, residual=second)[0]      # (launched dependent, behind two kernels)
+            step()
+        return a + b + [second, last]
+
+    want = [t.clone() for t in work(torch.cuda.synchronize)]
+    torch.cuda.synchronize()
+    for a, b in zip(work(lambda: None), want):
+        assert torch.equal(a, b)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = work(lambda: None)
+    for _ in range(3):
+        for t in got:
+            t.zero_()
+        graph.replay()
+        for a, b in zip(got, want):
+            assert torch.equal(a, b)
