@@ -55,6 +55,16 @@ variable_list guarded(F f) {
   }
 }
 
+// An argument that the Python function refuses, with the class of error that it raises.
+[[noreturn]] void refuse(PyObject* error, const char* why) {
+  py::gil_scoped_acquire gil;
+  PyErr_SetString(error, why);
+  throw py::error_already_set();
+}
+void check_dims(const Tensor& t, long dims, const char* what) {      // (where it unpacks the shape)
+  if (t.dim() != dims) refuse(PyExc_ValueError, what);
+}
+
 void* stream() { return c10::cuda::getCurrentCUDAStream().stream(); }
 void* ptr(const Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
@@ -437,11 +447,6 @@ struct SwiGLULinear : Function<SwiGLULinear> {
 };
 
 // ------------------------------------------------------------------ attention
-[[noreturn]] void refuse(PyObject* error, const char* why) {
-  py::gil_scoped_acquire gil;
-  PyErr_SetString(error, why);
-  throw py::error_already_set();
-}
 void check_view(const Tensor& t, long d) {     // (attention._check_view, and its class of error)
   if (t.dim() < 3) refuse(PyExc_IndexError, "heads must be [T, H, D]");
   if (t.stride(2) != 1 || t.stride(1) != d || !aligned(t))
@@ -503,7 +508,7 @@ struct FlashAttention : Function<FlashAttention> {
   static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, const Opt& sinks_, int64_t batch,
                         bool causal, double scale, int64_t q_off, int64_t window, double softcap) {
     const Tensor sinks = given(sinks_);
-    if (q.dim() != 3) refuse(PyExc_ValueError, "queries must be [T, H, D]");
+    check_dims(q, 3, "queries must be [T, H, D]");
     const AttnArgs a = attn_args(batch, causal, scale, q_off, window, softcap);
     const auto [o, lse] = attn_forward(q, k, v, sinks, a);
     ctx->save_for_backward({q, k, v, o, lse, sinks});
@@ -660,6 +665,7 @@ struct CrossEntropy : Function<CrossEntropy> {
 struct Router : Function<Router> {
   static variable_list forward(AutogradContext* ctx, const Tensor& logits_, const Opt& bias_, int64_t topk, bool sigmoid, bool pre_softmax,
                                int64_t groups, int64_t group_topk, double scale, const std::optional<double>& aux_coeff) {
+    check_dims(logits_, 2, "logits must be [T, E]");
     const Tensor logits = logits_.contiguous();
     const long T = logits.size(0), E = logits.size(1);
     Tensor bias, aux, sums;
@@ -755,6 +761,7 @@ struct GatherRows : Function<GatherRows> {
 };
 struct CombineRows : Function<CombineRows> {
   static Tensor forward(AutogradContext* ctx, const Tensor& y, const Tensor& pos, const Tensor& src_token) {
+    check_dims(pos, 2, "positions must be [T, k]");
     ctx->save_for_backward({src_token});
     return combine(y, pos.contiguous(), pos.size(0), pos.size(1));
   }
@@ -774,6 +781,7 @@ struct GroupedLinear : Function<GroupedLinear> {
   }
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const Tensor& mblock, const Tensor& row_start,
                         const Tensor& padded) {
+    check_dims(w, 3, "weights must be [E, N, K]");
     const long E = w.size(0), N = w.size(1), K = w.size(2);
     const Tensor out = empty({x.size(0), N}, x, at::kBFloat16);
     run(0, x, w, out, x.size(0), N, K, E, mblock, row_start, padded, false);

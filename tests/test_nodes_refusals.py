@@ -4,7 +4,7 @@ on tensors of the host: no case gets as far as a launch."""
 import pytest
 import torch
 
-from primus_b200.ops import _lib, attention, fused, layers
+from primus_b200.ops import _lib, attention, fused, layers, moe
 
 
 @pytest.fixture(scope="module")
@@ -92,3 +92,25 @@ def test_attention_of_other_dimensions(nodes, monkeypatch, which, shape):
             call()
         errors.append(e.type)
     assert errors[0] is errors[1]
+
+
+@pytest.mark.parametrize("which", ["router", "router 1", "pos", "pos 1", "weight", "weight 2"])
+def test_moe_tensors_of_other_dimensions(nodes, monkeypatch, which):
+    """Logits [T, E], positions [T, k], weights [E, N, K]: the Python functions unpack these shapes."""
+    monkeypatch.setattr(_lib, "call", lambda *a, **k: None)
+    ints = torch.zeros(2, 3, 4, dtype=torch.int32)
+    sched = moe.Schedule(*[ints] * 5, rows_cap=8)
+    x = _zeros(8, 16)
+    calls = {
+        "router": [(f, _zeros(2, 3, 8)) for f in (nodes.router, moe.RouterFn.apply)],
+        "router 1": [(f, _zeros(8)) for f in (nodes.router, moe.RouterFn.apply)],
+        "pos": [(lambda p, f=f: f(x, p, ints), ints) for f in (nodes.combine_rows, moe.CombineRowsFn.apply)],
+        "pos 1": [(lambda p, f=f: f(x, p, ints), ints[0, 0]) for f in (nodes.combine_rows, moe.CombineRowsFn.apply)],
+        "weight": [(lambda w: nodes.grouped_linear(x, w, ints, ints, ints), _zeros(1, 2, 16, 16)),
+                   (lambda w: moe.GroupedLinearFn.apply(x, w, sched), _zeros(1, 2, 16, 16))],
+        "weight 2": [(lambda w: nodes.grouped_linear(x, w, ints, ints, ints), _zeros(16, 16)),
+                     (lambda w: moe.GroupedLinearFn.apply(x, w, sched), _zeros(16, 16))],
+    }[which]
+    for call, t in calls:
+        with pytest.raises(ValueError):
+            call(t, None, 2, False, False, 0, 0, 1.0, None) if which.startswith("router") else call(t)
