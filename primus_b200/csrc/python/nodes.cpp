@@ -94,7 +94,10 @@ void launch(const char* name, int kernels, A... a) {
 }
 
 // rows of partial sums that the norms' backward passes write for so many rows, as the library has it
-long partial_rows(long rows) { return reinterpret_cast<int (*)(long)>(symbol("rmsnorm_bwd_num_partials"))(rows); }
+long partial_rows(long rows) {
+  static const auto f = reinterpret_cast<int (*)(long)>(symbol("rmsnorm_bwd_num_partials"));
+  return f(rows);
+}
 
 // the device's status word, which ops/_lib.py owns
 int* status_word(const Tensor& like) {

@@ -119,7 +119,13 @@ def _ctypes_launcher(fn, argtypes, stream: bool):
     return launch
 
 
+_tracing = torch._C._is_tracing
+
+
 def _bind(name: str, args, stream: bool):
+    if _tracing() and any(isinstance(a, torch.Tensor) and not a.dim() and not a.is_cuda for a in args):
+        # (what a recorded shape consists of: its address would travel in the number's place)
+        raise NativeLibraryError(f"pb_{name}: sizes are tensors while torch.jit.trace records")
     fn = load()["pb_" + name]       # an object of its own: argument types set here are not seen by other users
     launch = None
     if _LAUNCH is not None and all(a is None or isinstance(a, (torch.Tensor, int, float, bytes)) for a in args):
@@ -144,23 +150,11 @@ def _bound_anew(name: str, args, stream: bool, stream_ptr: int) -> int:
     return rc
 
 
-_tracing = torch._C._is_tracing
-
-
-def _refuse_trace():
-    """While torch.jit.trace records, sizes are tensors, whose addresses a launcher would take for numbers, and the trace would
-    return memory that no kernel has written."""
-    raise NativeLibraryError("the kernels cannot be recorded by torch.jit.trace")
-
-
-def call(name: str, *args, more: int = 0) -> None:
-    """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended.  ``more``: kernels that it enqueues with
-    these arguments beyond the usual number."""
+def call(name: str, *args) -> None:
+    """Invoke ``pb_<name>`` with converted arguments; the current CUDA stream is appended."""
     global LAUNCH_COUNT
-    if _tracing():
-        _refuse_trace()
     launch, kernels = _BOUND.get((name, True)) or _bind(name, args, True)
-    LAUNCH_COUNT += kernels + more
+    LAUNCH_COUNT += kernels
     stream = torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
     rc = launch(args, stream)
     if rc is None:
@@ -216,14 +210,12 @@ _functorch = torch._C._are_functorch_transforms_active
 
 
 def nodes(*tensors):
-    """The C++ autograd nodes where they take these tensors (bf16 on the GPU, no subclass, no function transform at work; None among
-    them counts as taken), else None."""
+    """The C++ autograd nodes where they take these tensors (bf16 on the GPU, no subclass, no function transform or trace at work; None
+    among them counts as taken), else None."""
     if not _NODES:
         _NODES.append(_load_nodes())
-    if _tracing():
-        _refuse_trace()
     n = _NODES[0]
-    if n is None or _functorch():
+    if n is None or _functorch() or _tracing():
         return None
     for t in tensors:
         if t is not None and (type(t) not in _PLAIN or t.dtype is not torch.bfloat16 or not t.is_cuda):

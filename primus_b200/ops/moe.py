@@ -50,8 +50,8 @@ class RouterFn(torch.autograd.Function):
             sums = torch.empty(-(-T // 8), E, dtype=torch.float32, device=dev)
             factor = float(aux_coeff) * E
         _lib.call("moe_route", lg, int(lg.dtype == torch.bfloat16), b, T, E, topk, int(sigmoid), int(pre_softmax),
-                  int(num_groups or 0), int(group_topk or 0), float(scale), probs, idx, idx64, full, ws, aux, sums, factor,
-                  more=int(aux is not None))
+                  int(num_groups or 0), int(group_topk or 0), float(scale), probs, idx, idx64, full, ws, aux, sums, factor)
+        _lib.LAUNCH_COUNT += aux is not None       # (the loss has a kernel of its own)
         counts = ws[:E]
         ctx.save_for_backward(full, idx, probs, counts)
         ctx.cfg = (topk, int(sigmoid), int(pre_softmax), float(scale), logits.dtype, factor)
